@@ -743,14 +743,8 @@ template <int BITS, int MODE>
 int launch_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     const size_t smem = (size_t)kStages * kStageBytes + (size_t)kWSlots * kWSlotBytes + 1024;
     a.wait_limit_ns = g_wait_limit_ns, a.test_skip_slot = g_test_skip_slot;
-    // Tile-blocked activations have a kernel of their own (grouped_tc_tiled.cu), whose work item is 128 weight rows x up
-    // to 192 or 256 tokens.  It wins wherever experts hold many tokens, and for every short contraction (its two
-    // accumulators hide the epilogue); a long contraction over experts of a few dozen tokens each is better served by
-    // this file's 256 rows per item, since an item costs the same whatever its token count.
-    if (a.x_kind == 3) {
-        const int64_t per_expert = a.dense_M > 0 ? a.dense_M : a.L.S / a.E;
-        if (a.K < 2048 || per_expert >= 160) return launch_tiled_tc<BITS, MODE>(fn, a, G, st);
-    }
+    // Tile-blocked activations have a kernel of their own (grouped_tc_tiled.cu).
+    if (a.x_kind == 3) return launch_tiled_tc<BITS, MODE>(fn, a, G, st);
     CUtensorMap wmap;
     if (int rc = weight_tensor_map(fn, a.q, a.E * a.N, BITS == 4 ? a.K / 2 : a.K, &wmap)) return rc;
     auto go = [&](auto kern) -> int {

@@ -4,38 +4,40 @@
 // activations arrive in that form.  Numerics as in grouped_tc.cu (kernels/moe_grouped.hpp:29-38,
 // kernels/wmma_gemm.hpp:116-129): F16 operands, weights code * scale + min with one rounding, FP32 accumulation.
 //
-// Why a second kernel.  A k-block of a work item costs about the same whatever the number of tokens it meets: the
-// dequantization, the MMA issue and the hand-overs between them are per k-block.  grouped_tc.cu's item is 256 weight
-// rows x up to 128 tokens.  Here an item is 128 weight rows (ONE accumulator, a row per tensor-memory lane) x up to 192
-// or 256 tokens, so an expert with many tokens has its weights dequantized once per 192 / 256 of them, and the tensor
-// memory that the second row half would take holds more pipeline stages or a second accumulator instead:
-//   TILE = 256 (long contractions, K >= 2048: gate/up): one accumulator, six stages, three producer warps and two
-//              epilogue warps a quadrant;
-//   TILE = 192 (short contractions: a down projection is 16 k-blocks): two accumulators - the epilogue of one item runs
-//              under the mainloop of the next, which matters most when the mainloop is short - four stages, two
-//              producer warps a quadrant.
-// The pack cuts both tile lists.  Experts of a few dozen tokens gain nothing from the wider tile and lose the 256 rows per
-// item, so the launcher in grouped_tc.cu keeps long contractions over such experts on its own kernel.
+// Work item: 128 weight rows (a row per tensor-memory lane) x up to 128 tokens of one expert.  k advances in steps of 128.
 //
-// SwiGLU: gate row j and up row j are rows of the same accumulator now, so they cannot share a lane.  An item holds 64
+// What bounds it (B200, SM cycles per step, the pieces measured alone): the MMAs take max(305, 4 n) for n tokens (below 76
+// tokens reading the A operand bounds them); dequantizing 128 x 128 codes and storing them to tensor memory takes the sixteen
+// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 660 a step for 15 tokens
+// and 840 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions.
+//   * One thread issues everything tensor-core: its loop runs under ONE elect.sync, with the base of tensor memory a constant
+//     (all of it is allocated).  12 cycles an MMA; with elect.sync inside each MMA's instruction group and the base read from
+//     shared memory an MMA cost its warp 90, which was the bound of the loop this one replaces (1400 a step).
+//   * A commit and the next stage's wait cost ~250 whatever lies between: steps of 128 k, eight MMAs.
+//   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 162 instructions a warp and step, not 290.
+//   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
+//     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
+// A wider token tile would not be cheaper: it shares a dequantization that is no longer the bound, and 128 columns leave tensor
+// memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column stages of A.
+// Measured, 512 experts, d = 4096, I = 1024, Q4: gate/up + SwiGLU 1052 -> 579 us at 777 tokens (15 an expert), 1132 -> 771 at
+// 4096 (80 an expert), 3034 -> 2477 at 16384 (Zipf-popular experts); down 820 -> 330, 861 -> 460, 1997 -> 1750 (Q8).
+//
+// SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up
 // rows of the same h columns, and the epilogue pairs them with one shuffle per value: of the 32 tokens of a pass the gate
 // lane finishes the first 16, the up lane the other 16.
 //
 // Operands as in grouped_tc.cu: A (weights) dequantized in registers and stored to tensor memory by the producer warps
-// (the [tmem] form of tcgen05.mma), B (activations) one cp.async.bulk per k-block into a 128-byte-swizzled K-major
-// tile, packed codes by 2-D tensor copies (64 bytes x 64 rows a box, two boxes a ring slot).  Tensor memory: the
-// accumulator(s) first, then one 32-column A stage per pipeline stage.
+// (the [tmem] form of tcgen05.mma), B (activations) two cp.async.bulk per step (one per 64-k sub-tile) into
+// 128-byte-swizzled K-major tiles, packed codes by 2-D tensor copies (128 codes x 64 rows a box, two boxes a ring slot).
 //
-// One persistent CTA per SM.  Warps: the epilogue first (one per lane quadrant; two per quadrant, each taking half of the
-// columns, where there is a single accumulator whose epilogue the MMA warp has to wait for, and in the hyper-connection up
-// mix, whose epilogue carries the arithmetic of the stream combine - see TcHcUp), then MMA issue, activation
-// copies, the ring of weight codes and one idle warp, then the
-// weight producers (a lane quadrant's warps take every second or third k-block each).  A producer hands its k-block
-// over before it waits for anything its next one needs.  Every wait is bounded: past the limit the CTA raises its abort
-// flag, records {2, item, role} in the status words, drains the tensor pipe and frees its tensor memory before
-// returning.  The tensor copies read this GPU's own weight array only, each into the shared memory of the one CTA that
-// issues it.
+// One persistent CTA per SM.  Warps: the epilogue first (one per lane quadrant; two in the hyper-connection up mix, whose
+// epilogue carries the arithmetic of the stream combine - see TcHcUp), then MMA issue, activation copies, the ring of weight
+// codes and the item ring, then four sets of four weight producers (a lane quadrant's warps take every fourth step each).  All lanes
+// of a producer warp wait on its barriers themselves: a poll by one lane and a reconvergence after it cost more than 32
+// lanes reading the same word.  Every wait is bounded: past the limit the CTA raises its abort flag, records
+// {2, item, role} in the status words, drains the tensor pipe and frees its tensor memory before returning.  The tensor
+// copies read this GPU's own weight array only, each into the shared memory of the one CTA that issues it.
 
 #include "grouped_tc.cuh"
 
@@ -44,42 +46,43 @@
 namespace sxb {
 namespace {
 
-constexpr int kBK = 64;              // k per stage: one 128-byte swizzle line of F16
+constexpr int kTile = 128;           // tokens per item at most = columns of an accumulator
+constexpr int kSubK = 64;            // k of one 128-byte swizzle line of F16
+constexpr int kBK = 2 * kSubK;       // k per stage
 constexpr int kRows = 128;           // weight rows per item = tensor-memory lanes
-constexpr int kAStageCols = kBK / 2; // 64 F16 of one weight row per lane
+constexpr int kSubBytes = kTile * 128;      // activation tile of 64 k
+constexpr int kStageBytes = 2 * kSubBytes;  // of a stage
+constexpr int kAStageCols = kBK / 2; // 128 F16 of one weight row per lane
+constexpr int kAccs = 2;
 constexpr int kTmemCols = 512;
-// TILE = tokens per item at most = columns of an accumulator.  Tensor memory holds two accumulators when they fit beside at
-// least four A stages (an item's epilogue then runs under the next item's mainloop), else one; the rest is A stages, as
-// many as the activation tiles of as many k-blocks fit in shared memory.
-// HC: the shape of the hyper-connection up mix (kTcHcUp), whose epilogue does the arithmetic of the stream combine and is
-// what its items wait for: a second set of epilogue warps, and a shorter ring of codes (its contractions are a few
-// k-blocks) to leave their staging buffers room in shared memory.
-template <int TILE, bool HC = false>
+
+// HC: the hyper-connection up mix (kTcHcUp), whose contraction is short and whose epilogue needs registers and shared memory:
+// half the producers, stages and ring slots.
+// A set of four producer warps (one per lane quadrant) owns one stage, and its own ring slots: it meets every barrier it
+// waits on again only after it has seen that barrier's previous phase end, so watching the parity is enough.
+template <int BITS, bool HC>
 struct Shape {
-    static constexpr int kAccs = 2 * TILE + 4 * kAStageCols <= kTmemCols ? 2 : 1;
-    static constexpr int kStageBytes = TILE * kBK * 2;  // the activation tile of one k-block
-    static constexpr int kByTmem = (kTmemCols - kAccs * TILE) / kAStageCols, kBySmem = TILE > 192 ? 6 : 8;
-    static constexpr int kStages = kByTmem < kBySmem ? kByTmem : kBySmem;
-    static constexpr int kWSlots = TILE > 192 ? 4 : HC ? 6 : 8;  // ring slots of packed codes (8 KB each)
-    // Producer warps per lane quadrant: they take every kWays-th k-block each.
-    static constexpr int kWays = TILE > 192 ? 3 : 2;
-    // Epilogue warps per lane quadrant: a single accumulator's epilogue is exposed (the MMA warp waits for it), so its
-    // columns are split between two sets of warps; with two accumulators one set keeps up.
-    static constexpr int kEpiSets = kAccs == 1 || HC ? 2 : 1;
-    // warps: epilogue | MMA issue, activation copies, ring of weight codes, one idle | producers
+    static constexpr int kWays = HC ? 2 : 4;  // producer sets
+    static constexpr int kStages = kWays;
+    static constexpr int kSlotBytes = kRows * kBK * BITS / 8;  // a ring slot: the packed codes of a step, 8 or 16 KB
+    static constexpr int kWSlots = kWays * (BITS == 4 ? 2 : 1) * (HC ? 2 : 1);
+    static constexpr int kEpiSets = HC ? 2 : 1;  // epilogue warps per lane quadrant
     static constexpr int kEpiWarps = 4 * kEpiSets, kMmaWarp = kEpiWarps, kBCopyWarp = kEpiWarps + 1, kWCopyWarp = kEpiWarps + 2,
-                         kFirstAWarp = kEpiWarps + 4;
+                         kItemWarp = kEpiWarps + 3, kFirstAWarp = kEpiWarps + 4;
     static constexpr int kThreads = 32 * (kFirstAWarp + 4 * kWays);
-    static_assert(TILE % (32 * kEpiSets) == 0 || kEpiSets == 1, "an epilogue set takes whole passes of 32 columns");
-    static_assert(TILE % 16 == 0 && TILE <= 256 && kStages > kWays && kStages >= 3, "tile size / pipeline depth");
-    static_assert(kStageBytes % 1024 == 0, "operand tiles start on the swizzle pattern's 1024-byte period");
+    static constexpr int kItemReaders = kEpiWarps + 3 + 4 * kWays;  // warps that read every item from the item ring
+    static_assert(kAccs * kTile + kStages * kAStageCols <= kTmemCols, "tensor memory");
+    static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
-constexpr int kWSlotBytes = kRows * 64;  // 64 bytes (128 Q4 or 64 Q8 codes) of each of the item's rows
+constexpr int kItemRing = 4;
 // kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
 constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
+// The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).
+__device__ inline float unscale(float scale) { return __int_as_float(((127 + 24 + 127) << 23) - __float_as_int(scale)); }
+
 struct Item {
-    int bucket, start, cnt;  // expert (bucket E = invalid ids), first position in slots[], tokens of the item
+    int bucket, start, cnt;  // expert (bucket E = invalid ids, -1 = no more items), first position in slots[], tokens of the item
     int rb;                  // row block
 };
 
@@ -87,15 +90,7 @@ template <int MODE>
 __device__ inline int row_blocks(const TcArgs &a) {
     return MODE == kTcSwiglu ? (int)((a.N / 2 + kRows / 2 - 1) / (kRows / 2)) : (int)((a.N + kRows - 1) / kRows);
 }
-template <int TILE>
-__device__ inline int tile_count(const TcArgs &a) {
-    static_assert(TILE == kTcTileA || TILE == kTcTileB, "the pack cuts tiles of these two sizes");
-    if (a.dense_M > 0) return (int)((a.dense_M + TILE - 1) / TILE);
-    return a.ws[TILE == kTcTileA ? a.L.tta_n : a.L.ttb_n];
-}
-template <int TILE>
 __device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
-    constexpr int kTile = TILE;
     Item it;
     const int tile = item / rbs;
     it.rb = item % rbs;
@@ -104,39 +99,34 @@ __device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
         it.cnt = (int)min((int64_t)kTile, a.dense_M - it.start);
         return it;
     }
-    it.bucket = a.ws[(TILE == kTcTileA ? a.L.tta_bucket : a.L.ttb_bucket) + tile];
-    it.start = a.ws[(TILE == kTcTileA ? a.L.tta_start : a.L.ttb_start) + tile];
+    it.bucket = a.ws[a.L.t128_bucket + tile];
+    it.start = a.ws[a.L.t128_start + tile];
     it.cnt = min(kTile, a.ws[a.L.offsets + it.bucket + 1] - it.start);
     return it;
 }
-// Next item of this CTA (stride gridDim.x) at or after `item` whose bucket is a real expert.
-template <int TILE>
-__device__ inline int next_valid_item(const TcArgs &a, int item, int n_items, int rbs) {
-    if (a.dense_M > 0) return item;
-    const int64_t tb = TILE == kTcTileA ? a.L.tta_bucket : a.L.ttb_bucket;
-    while (item < n_items && a.ws[tb + item / rbs] >= a.E) item += gridDim.x;
-    return item;
-}
 
-template <int BITS, int G, int MODE, int TILE>
-__global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
+template <int BITS, int G, int MODE>
+__global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     tiled_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap wmap) {
-    using S = Shape<TILE, MODE == kTcHcUp>;
-    constexpr int kTile = TILE, kAccs = S::kAccs, kStages = S::kStages, kStageBytes = S::kStageBytes, kWSlots = S::kWSlots, kWays = S::kWays,
-                  kEpiSets = S::kEpiSets, kEpiWarps = S::kEpiWarps, kMmaWarp = S::kMmaWarp, kBCopyWarp = S::kBCopyWarp,
-                  kWCopyWarp = S::kWCopyWarp, kFirstAWarp = S::kFirstAWarp;
+    using S = Shape<BITS, MODE == kTcHcUp>;
+    constexpr int kStages = S::kStages, kWSlots = S::kWSlots, kSlotBytes = S::kSlotBytes, kWays = S::kWays, kEpiSets = S::kEpiSets,
+                  kEpiWarps = S::kEpiWarps, kMmaWarp = S::kMmaWarp, kBCopyWarp = S::kBCopyWarp, kWCopyWarp = S::kWCopyWarp,
+                  kItemWarp = S::kItemWarp, kFirstAWarp = S::kFirstAWarp;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     // 1024-byte alignment of the operand tiles (the swizzle pattern repeats every 1024 bytes).
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[2], acc_empty[2], drain_bar;
+    __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[kAccs], acc_empty[kAccs], drain_bar;
     __shared__ uint64_t w_full[kWSlots], w_empty[kWSlots];
+    __shared__ uint64_t item_full[kItemRing], item_empty[kItemRing];
+    __shared__ __align__(16) Item item_ring[kItemRing];
+    __shared__ float row_scale[kItemRing][kRows];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int K = (int)a.K, n_kb = K / kBK, groups = K / G;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int n_steps = (int)a.K / kBK, groups = (int)a.K / G;
     const int rbs = row_blocks<MODE>(a);
-    const int n_items = tile_count<TILE>(a) * rbs;
+    const int n_items = (a.dense_M > 0 ? (int)((a.dense_M + kTile - 1) / kTile) : a.ws[3]) * rbs;
     // slot (row of the output / of h) at position pos of the slot order; a dense projection's rows are in their own order
     auto slot_at = [&](int pos) -> int { return a.dense_M > 0 ? pos : a.ws[a.L.slots + pos]; };
     volatile int *abort_v = &abort_flag;
@@ -145,7 +135,8 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
         for (int s = 0; s < kStages; ++s) mbar_init(&full_bar[s], 4 + 1), mbar_init(&empty_bar[s], 1);
         for (int h = 0; h < kAccs; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kEpiWarps);
         mbar_init(&drain_bar, 1);
-        for (int s = 0; s < kWSlots; ++s) mbar_init(&w_full[s], 1), mbar_init(&w_empty[s], BITS == 4 ? 8 : 4);
+        for (int s = 0; s < kWSlots; ++s) mbar_init(&w_full[s], 1), mbar_init(&w_empty[s], 4);
+        for (int s = 0; s < kItemRing; ++s) mbar_init(&item_full[s], 1), mbar_init(&item_empty[s], S::kItemReaders);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -156,7 +147,6 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = tmem_base_smem;
 
     auto raise_abort = [&](int item, int role) {
         if (atomicExch(&abort_flag, 1) == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) {
@@ -164,58 +154,80 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
             a.status[2] = (uint32_t)role;
         }
     };
+    // All 512 columns are this CTA's, so they start at column 0, and the code below says so with constants.
+    if (tmem_base_smem != 0 && threadIdx.x == 0) raise_abort(0, 0);
+    __syncthreads();
+    const bool run = tmem_base_smem == 0;
 
-    constexpr int kKbPerSlot = BITS == 4 ? 2 : 1;  // k-blocks per 64 bytes of packed codes
-    const int n_slots = (n_kb + kKbPerSlot - 1) / kKbPerSlot;
-    const uint32_t w_base = smem_u32(smem + kStages * kStageBytes);
+    const uint32_t b_base = smem_u32(smem), w_base = b_base + (uint32_t)(kStages * kStageBytes);
     uint32_t issued = 0;  // ring slots issued by this thread (the ring's thread only)
 
-    if (warp >= kFirstAWarp && (warp - kFirstAWarp) >> 2 < n_kb) {
+    // Item number i of this CTA, from the item ring.  read_item: a whole warp; read_item_one: a single thread.
+    const Item no_item{-1, 0, 0, 0};
+    auto read_item_one = [&](int i) -> Item {
+        if (!mbar_wait(&item_full[i % kItemRing], (uint32_t)(i / kItemRing) & 1u, abort_v, a.wait_limit_ns)) {
+            raise_abort(blockIdx.x + i * gridDim.x, 8);
+            return no_item;
+        }
+        const Item it = item_ring[i % kItemRing];
+        mbar_arrive(&item_empty[i % kItemRing]);
+        return it;
+    };
+    auto read_item = [&](int i, int p, float &scale) -> Item {  // scale: the power of two of tensor-memory lane p (row_scale)
+        const bool ok = mbar_wait(&item_full[i % kItemRing], (uint32_t)(i / kItemRing) & 1u, abort_v, a.wait_limit_ns);
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 8);
+            return no_item;
+        }
+        const Item it = item_ring[i % kItemRing];
+        scale = row_scale[i % kItemRing][p];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&item_empty[i % kItemRing]);
+        return it;
+    };
+
+    // The row of the stacked weight in tensor-memory lane p of an item, -1 past the end of the expert.
+    auto row_of = [&](const Item &it, int p) -> int64_t {
+        if (MODE == kTcSwiglu) {
+            const int64_t I = a.N / 2, j = (int64_t)it.rb * (kRows / 2) + (p >> 5) * 16 + (p & 15);
+            return j < I ? (int64_t)it.bucket * a.N + ((p & 16) ? I + j : j) : -1;
+        }
+        const int64_t rr = (int64_t)it.rb * kRows + p;
+        return rr < a.N ? (int64_t)it.bucket * a.N + rr : -1;
+    };
+
+    if (!run) {
+    } else if (warp >= kFirstAWarp) {
         // ===================== A producers: weights =====================
         // A thread writes one weight row into its own tensor-memory lane; a warp may only touch the lane quadrant
-        // warp % 4.  The kWays warps of a quadrant take every kWays-th k-block each, so that while one is in its chain of
-        // barrier polls and hand-over the others have the arithmetic pipes, and a warp's fixed per-k-block latencies are
-        // paid once per kWays k-blocks of the pipeline.
-        const int a_par = (warp - kFirstAWarp) >> 2, a_quad = warp & 3;  // a_par: which of every kWays k-blocks
+        // warp % 4.  Step number cnt of the CTA, counted across its items, belongs to set cnt % kWays, which works in stage
+        // number `set`; the sets are out of step with one another, so that while one waits for a barrier or for its stores
+        // the others have the arithmetic pipes.
+        const int set = (warp - kFirstAWarp) >> 2, a_quad = warp & 3;
         const int p0 = a_quad * 32 + lane;  // tensor-memory lane = row of the item
         // row of the ring slot that holds this lane's codes: the SwiGLU form's slot is [64 gate rows | 64 up rows]
         const int srow = MODE == kTcSwiglu ? (lane >> 4) * (kRows / 2) + a_quad * 16 + (lane & 15) : p0;
-        constexpr int kKbPerChunk = G / 8;  // k-blocks covered by eight scale groups (one 16-byte load)
-        static_assert(kWays <= kKbPerChunk, "a warp's consecutive k-blocks never skip a chunk of scale groups");
-        constexpr int kGroupsPerKb = G >= kBK ? 1 : kBK / G;
-        constexpr int kCodeRegs = BITS == 4 ? 2 : 4;  // 16-byte chunks of codes per row and k-block
+        constexpr int kStepsPerChunk = 8 * G / kBK;  // steps covered by eight scale groups (one 16-byte load)
+        constexpr int kGroupsPerStep = kBK / G;
+        constexpr int kCodeRegs = kBK * BITS / 128;  // 16-byte chunks of codes per row and step
+        constexpr int kWordsPerChunk = BITS == 4 ? 4 : 2;  // runs of eight codes in one of them
+        constexpr int kSlotsPerSet = kWSlots / kWays;
         const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
-        // this thread's 64 bytes inside a slot; 16-byte chunks swizzled (64-byte mode)
-        const uint32_t my_w = (uint32_t)(srow * 64), my_sw = (uint32_t)((srow >> 1) & 3);
+        // this thread's row inside the set's first slot; its 16-byte chunks are swizzled (64-byte mode for Q4's 64-byte rows,
+        // 128-byte for Q8's)
+        const uint32_t my_w = w_base + (uint32_t)(set * kSlotBytes + srow * (kBK * BITS / 8)), my_sw = (uint32_t)(BITS == 4 ? (srow >> 1) & 3 : srow & 7);
+        const uint32_t a_addr = ((uint32_t)(a_quad * 32) << 16) + (uint32_t)(kAccs * kTile + set * kAStageCols);
 
-        struct Row {
-            int64_t wrow;  // row of the stacked weight
-            bool valid;
-        };
-        auto row_of = [&](int item) {
-            Row r{0, false};
-            if (item >= n_items) return r;
-            const Item it = item_info<TILE>(a, item, rbs);
-            if (MODE == kTcSwiglu) {
-                const int64_t I = a.N / 2, j = (int64_t)it.rb * (kRows / 2) + a_quad * 16 + (lane & 15);
-                r.valid = j < I;
-                r.wrow = (int64_t)it.bucket * a.N + ((lane >> 4) ? I + j : j);
-            } else {
-                const int64_t rr = (int64_t)it.rb * kRows + p0;
-                r.valid = rr < a.N;
-                r.wrow = (int64_t)it.bucket * a.N + rr;
-            }
-            return r;
-        };
-        // Scales and mins of eight consecutive groups of a row (BF16 bits), fetched one chunk ahead of use.
+        // Scales and mins of eight consecutive groups of a row (BF16 bits), fetched one chunk ahead of use.  A row past the
+        // end of the expert gets zeros: its operand row is then zero whatever codes its lane reads.
         struct ScaleChunk {
             uint4 s, m;
         };
-        auto load_scales = [&](const Row &r, int chunk) {
+        auto load_scales = [&](int64_t wrow, int chunk) {
             ScaleChunk c{make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-            if (!r.valid) return c;
+            if (wrow < 0) return c;
             const int g0 = chunk * 8;
-            const uint16_t *sp = a.scale + r.wrow * groups + g0, *mp = a.minv + r.wrow * groups + g0;
+            const uint16_t *sp = a.scale + wrow * groups + g0, *mp = a.minv + wrow * groups + g0;
             if (vec_scales) {
                 c.s = __ldg(reinterpret_cast<const uint4 *>(sp)), c.m = __ldg(reinterpret_cast<const uint4 *>(mp));
             } else {
@@ -231,202 +243,254 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
             const uint32_t w = (g & 4) ? ((g & 2) ? v.w : v.z) : ((g & 2) ? v.y : v.x);
             return (uint16_t)((g & 1) ? (w >> 16) : (w & 0xffffu));
         };
-        // lane 0: the codes of slot number wc have landed and the stage of k-block number cnt is free
-        auto poll = [&](uint32_t wc, uint32_t cnt, int it_for_status) {
-            if (!mbar_wait(&w_full[wc % kWSlots], (wc / kWSlots) & 1u, abort_v, a.wait_limit_ns)) {
-                raise_abort(it_for_status, 7);
-                return;
-            }
-            if (!mbar_wait(&empty_bar[cnt % kStages], ((cnt / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) raise_abort(it_for_status, 1);
-        };
 
-        // This warp's k-blocks of an item: kb = a_par, a_par + kWays, ...; k-block kb lives in slot kb / kKbPerSlot.  The
-        // stores' source registers must stay untouched until tcgen05.wait::st.
-        int item = next_valid_item<TILE>(a, blockIdx.x, n_items, rbs);
-        uint32_t kb_base = 0, w_base_count = 0;  // k-blocks / slots of the items before this one
-        Row row = row_of(item);
         ScaleChunk sc_cur = {}, sc_nxt = {};
-        if (item < n_items) sc_nxt = load_scales(row, 0);
-        if (item < n_items && lane == 0) poll((uint32_t)(a_par / kKbPerSlot), (uint32_t)a_par, item);
-        __syncwarp();
+        int nxt_item = -1, nxt_chunk = -1;  // what sc_nxt holds
+        uint32_t j = 0;                     // steps this set has done
+        int st = set;                       // the set's next step, relative to the item at hand
         bool live = true;
-        while (item < n_items && live && !*abort_v) {
-            const int next = next_valid_item<TILE>(a, item + gridDim.x, n_items, rbs);
-            const Row next_row = row_of(next);
+        float nxt_scale = 1.f;
+        Item nxt = read_item(0, p0, nxt_scale);
+        for (int i = 0; nxt.bucket >= 0 && live; ++i) {
+            const Item it = nxt;
+            const float scale = nxt_scale, scale_min = scale * 0x1p-24f;
+            nxt = read_item(i + 1, p0, nxt_scale);
+            if (it.bucket >= a.E) continue;
             int cur_chunk = -1;
-            for (int kb = a_par; kb < n_kb; kb += kWays) {
-                const uint32_t cnt = kb_base + (uint32_t)kb, wc = w_base_count + (uint32_t)(kb / kKbPerSlot);
-                const int stage = cnt % kStages, slot = wc % kWSlots;
-                if (kb / kKbPerChunk != cur_chunk) {  // this warp's first k-block in a chunk of eight scale groups
-                    cur_chunk = kb / kKbPerChunk;
-                    sc_cur = sc_nxt;
-                    int nkb = kb + kWays;  // this warp's first k-block past the chunk (kWays <= kKbPerChunk: no chunk is skipped)
-                    while (nkb / kKbPerChunk == cur_chunk) nkb += kWays;
-                    if (nkb < n_kb) sc_nxt = load_scales(row, nkb / kKbPerChunk);
-                    else if (next < n_items) sc_nxt = load_scales(next_row, 0);
+            for (; st < n_steps; st += kWays, ++j) {
+                const int chunk = st / kStepsPerChunk;
+                if (chunk != cur_chunk) {
+                    if (nxt_item == i && nxt_chunk == chunk) sc_cur = sc_nxt;
+                    else sc_cur = load_scales(row_of(it, p0), chunk);
+                    cur_chunk = chunk;
+                    // the set's first step past this chunk: in this item, or in the next one
+                    int nst = st + ((min((chunk + 1) * kStepsPerChunk, n_steps) - st + kWays - 1) & ~(kWays - 1));
+                    if (nst < n_steps) {
+                        nxt_item = i, nxt_chunk = nst / kStepsPerChunk;
+                        sc_nxt = load_scales(row_of(it, p0), nxt_chunk);
+                    } else if (nst -= n_steps; nxt.bucket >= 0 && nxt.bucket < a.E && nst < n_steps) {
+                        nxt_item = i + 1, nxt_chunk = nst / kStepsPerChunk;
+                        sc_nxt = load_scales(row_of(nxt, p0), nxt_chunk);
+                    }
                 }
-                // this k-block's codes of the row (Q4: half of the slot's 64 bytes of a row; Q8: all of them)
+                const uint32_t slot = set + (kSlotsPerSet > 1 ? (j % kSlotsPerSet) * kWays : 0);
+                bool ok = mbar_wait(&w_full[slot], (j / kSlotsPerSet) & 1u, abort_v, a.wait_limit_ns);
+                if (!ok && lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 7);
                 uint4 code[kCodeRegs];
 #pragma unroll
-                for (int c = 0; c < kCodeRegs; ++c) {
-                    const uint32_t chunk = (uint32_t)((BITS == 4 ? (kb & 1) * 2 : 0) + c);
-                    code[c] = ld_shared_v4(w_base + (uint32_t)(slot * kWSlotBytes) + my_w + ((chunk ^ my_sw) << 4));
-                    if (!row.valid) code[c] = make_uint4(0u, 0u, 0u, 0u);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
-                __half2 s2[kGroupsPerKb], s16[kGroupsPerKb], m2[kGroupsPerKb];
+                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(my_w + (slot - set) * (uint32_t)kSlotBytes + (((uint32_t)c ^ my_sw) << 4));
+                __half2 s2[kGroupsPerStep], s16[kGroupsPerStep], m2[kGroupsPerStep];
 #pragma unroll
-                for (int gi = 0; gi < kGroupsPerKb; ++gi) {
-                    const int g = ((kb * kBK) / G + gi) & 7;  // group inside the chunk of eight
+                for (int gi = 0; gi < kGroupsPerStep; ++gi) {
+                    const int g = (st * kGroupsPerStep + gi) & 7;  // group inside the chunk of eight
                     const float sf = bf16_bits_to_f32(pick16(sc_cur.s, g)), mf = bf16_bits_to_f32(pick16(sc_cur.m, g));
-                    s2[gi] = __float2half2_rn(sf), s16[gi] = __float2half2_rn(sf * 0.0625f), m2[gi] = __float2half2_rn(mf);
+                    s2[gi] = __float2half2_rn(sf * scale), m2[gi] = __float2half2_rn(mf * scale_min);
+                    s16[gi] = __hmul2(s2[gi], __float2half2_rn(0.0625f));
                 }
-                const uint32_t a_addr = tmem_base + ((uint32_t)(a_quad * 32) << 16) + (uint32_t)(kAccs * kTile + stage * kAStageCols);
-                // the row: 64 codes -> 64 F16 = 32 tensor-memory columns of this lane, two stores of 16
+                // 32 codes of the row -> 32 F16 = 16 tensor-memory columns of this lane
+                auto quarter = [&](int hc, uint4 (&d)[4]) {
 #pragma unroll
-                for (int hc = 0; hc < 2; ++hc) {
-                    uint4 d[4];
-                    if (BITS == 4) {
-                        const uint4 v = code[hc];  // 32 codes
-                        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) {
-                            const int gi = kGroupsPerKb == 1 ? 0 : ((hc * 4 + cc) * 8) / G;
-                            d[cc] = dequant_q4_word(w4[cc], s2[gi], s16[gi], m2[gi]);
-                        }
-                    } else {
-                        const uint4 v0 = code[hc * 2], v1 = code[hc * 2 + 1];  // 2 x 16 codes
-                        const uint32_t w8[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-#pragma unroll
-                        for (int cc = 0; cc < 4; ++cc) {
-                            const int gi = kGroupsPerKb == 1 ? 0 : ((hc * 4 + cc) * 8) / G;
-                            d[cc] = dequant_q8_words(w8[2 * cc], w8[2 * cc + 1], s2[gi], m2[gi]);
-                        }
+                    for (int cc = 0; cc < 4; ++cc) {
+                        const int gi = ((hc * 4 + cc) * 8) / G;
+                        const uint4 v = code[(hc * 4 + cc) / kWordsPerChunk];
+                        if (BITS == 4) d[cc] = dequant_q4_scaled(cc == 0 ? v.x : cc == 1 ? v.y : cc == 2 ? v.z : v.w, s2[gi], s16[gi], m2[gi]);
+                        else d[cc] = (cc & 1) ? dequant_q8_scaled(v.z, v.w, s2[gi], m2[gi]) : dequant_q8_scaled(v.x, v.y, s2[gi], m2[gi]);
                     }
-                    tc_st16(a_addr + hc * 16, d);
+                };
+                uint4 d[4];
+                quarter(0, d);
+                if (ok && !mbar_wait(&empty_bar[set], (j & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 1);
+                    ok = false;
                 }
-                // Under the stores: a look (never a wait) at what this warp's next k-block needs - its codes landed, its
-                // stage free.  The k-block in hand is handed over BEFORE any wait for those: a producer that waited for a
-                // free stage while holding back a finished k-block would tie the MMA warp's progress to its own.
-                uint32_t nwc = 0, ncnt = 0;
-                int nitem = -1;  // -1: this warp has no further k-block
-                if (kb + kWays < n_kb) nwc = w_base_count + (uint32_t)((kb + kWays) / kKbPerSlot), ncnt = cnt + kWays, nitem = item;
-                else if (next < n_items) nwc = w_base_count + (uint32_t)(n_slots + a_par / kKbPerSlot), ncnt = kb_base + (uint32_t)(n_kb + a_par), nitem = next;
-                bool seen = true;
-                if (lane == 0 && nitem >= 0)
-                    seen = mbar_test_wait(&w_full[nwc % kWSlots], (nwc / kWSlots) & 1u) &&
-                           mbar_test_wait(&empty_bar[ncnt % kStages], ((ncnt / kStages) & 1u) ^ 1u);
-                __syncwarp();
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();  // orders the stores before the MMA warp's reads across the barrier
-                __syncwarp();
-                tc_fence_after();   // and the next k-block's stores after the MMAs that freed its stage
-                if (lane == 0) {
-                    mbar_arrive(&full_bar[stage]);
-                    if (!seen) poll(nwc, ncnt, nitem);
-                }
-                __syncwarp();
-                if (*abort_v) {
+                // reconverges the warp; a wait that gave up in any lane ends the warp's work
+                if (!__all_sync(0xffffffffu, ok)) {
                     live = false;
                     break;
                 }
+                tc_fence_after();  // the stores below come after the MMAs that freed the stage
+                if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
+                tc_st16(a_addr, d);
+#pragma unroll
+                for (int hc = 1; hc < 4; ++hc) {
+                    quarter(hc, d);
+                    tc_st16(a_addr + hc * 16, d);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full_bar[set]);
             }
-            kb_base += (uint32_t)n_kb, w_base_count += (uint32_t)n_slots;
-            item = next;
-            row = next_row;
+            st -= n_steps;
+        }
+    } else if (warp == kItemWarp) {
+        // ===================== the item ring =====================
+        // One warp looks the CTA's items up ahead of everyone else: the other roles read an item's description from shared
+        // memory instead of each walking two dependent loads of the grouping workspace per item.  It also finds each
+        // row's power of two (dequant_q4_scaled) from the row's scales and mins, four rows a lane; those lines are then in
+        // L2 when the producers want them.
+        const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
+        Item nxt = blockIdx.x < n_items ? item_info(a, blockIdx.x, rbs) : no_item;
+        for (int i = 0;; ++i) {
+            const Item it = nxt;
+            const int item = blockIdx.x + i * gridDim.x;
+            nxt = item + (int)gridDim.x < n_items ? item_info(a, item + gridDim.x, rbs) : no_item;
+            uint32_t smax[4] = {0u, 0u, 0u, 0u}, mmax[4] = {0u, 0u, 0u, 0u};  // two 16-bit maxima of the BF16 magnitudes
+            if (it.bucket >= 0 && it.bucket < a.E) {
+                int64_t at[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int64_t wrow = row_of(it, r * 32 + lane);
+                    at[r] = (wrow < 0 ? row_of(it, 0) : wrow) * groups;  // lanes past the expert's end look at a row that exists
+                }
+                if (vec_scales) {
+#pragma unroll 2
+                    for (int g = 0; g < groups; g += 8) {
+                        uint4 sv[4], mv[4];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            sv[r] = __ldg(reinterpret_cast<const uint4 *>(a.scale + at[r] + g));
+                            mv[r] = __ldg(reinterpret_cast<const uint4 *>(a.minv + at[r] + g));
+                        }
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            const uint32_t sw[4] = {sv[r].x, sv[r].y, sv[r].z, sv[r].w}, mw[4] = {mv[r].x, mv[r].y, mv[r].z, mv[r].w};
+#pragma unroll
+                            for (int c = 0; c < 4; ++c)
+                                smax[r] = __vmaxu2(smax[r], sw[c] & 0x7fff7fffu), mmax[r] = __vmaxu2(mmax[r], mw[c] & 0x7fff7fffu);
+                        }
+                    }
+                } else {
+                    for (int g = 0; g < groups; ++g)
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            smax[r] = max(smax[r], (uint32_t)__ldg(a.scale + at[r] + g) & 0x7fffu);
+                            mmax[r] = max(mmax[r], (uint32_t)__ldg(a.minv + at[r] + g) & 0x7fffu);
+                        }
+                }
+            }
+            if (i >= kItemRing) {
+                const bool ok = mbar_wait(&item_empty[i % kItemRing], ((uint32_t)(i / kItemRing) & 1u) ^ 1u, abort_v, a.wait_limit_ns);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) raise_abort(item, 9);
+                    break;
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                // exponent e of the largest scale, or of the largest min less 8 where that is more: 2^(14 - e) takes every scale
+                // below 2^15 and every min, after its further 2^-24, below 1/2
+                const int es = (int)(max(smax[r] >> 16, smax[r] & 0xffffu) >> 7), em = (int)(max(mmax[r] >> 16, mmax[r] & 0xffffu) >> 7) - 8;
+                const int e = min(max(max(es, em), 127 - 24), 127 + 15);
+                row_scale[i % kItemRing][r * 32 + lane] = __int_as_float((127 + 14 + 127 - e) << 23);
+            }
+            if (lane == 0) item_ring[i % kItemRing] = it;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&item_full[i % kItemRing]);
+            if (it.bucket < 0) break;
         }
     } else if (warp == kWCopyWarp) {
         // ===================== the ring of weight codes =====================
         // One thread keeps the ring as far ahead as free slots allow: per slot two boxes of 64 rows (the SwiGLU form: the
         // gate rows and, I rows further, their up rows; otherwise 128 consecutive rows).
-        if (lane == 0) {
-            int is_item = next_valid_item<TILE>(a, blockIdx.x, n_items, rbs), is_slot = 0, y0 = 0, y1 = 0;
-            while (is_item < n_items && !*abort_v) {
-                const int slot = issued % kWSlots;
-                if (issued >= (uint32_t)kWSlots && !mbar_wait(&w_empty[slot], ((issued / kWSlots) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
-                    raise_abort(is_item, 6);
-                    break;
-                }
-                if (is_slot == 0) {
-                    const Item it = item_info<TILE>(a, is_item, rbs);
-                    if (MODE == kTcSwiglu) y0 = (int)(it.bucket * a.N + it.rb * (kRows / 2)), y1 = y0 + (int)(a.N / 2);
-                    else y0 = (int)(it.bucket * a.N + (int64_t)it.rb * kRows), y1 = y0 + kRows / 2;
-                }
-                const uint32_t dst = w_base + (uint32_t)(slot * kWSlotBytes);
-                // test hook: CTA 0 leaves one slot unfilled (neither the byte count nor the copies), so that its consumers'
-                // wait runs out at the launch's limit and the abort path is exercised without anything faulting
-                if (!(blockIdx.x == 0 && (int)issued == a.test_skip_slot)) {
-                    mbar_expect_tx(&w_full[slot], (uint32_t)kWSlotBytes);
-                    tma_load_2d(dst, &wmap, is_slot * 64, y0, &w_full[slot]);
-                    tma_load_2d(dst + kWSlotBytes / 2, &wmap, is_slot * 64, y1, &w_full[slot]);
-                }
-                ++issued;
-                if (++is_slot == n_slots) is_slot = 0, is_item = next_valid_item<TILE>(a, is_item + gridDim.x, n_items, rbs);
-            }
-        }
-    } else if (warp == kBCopyWarp) {
-        // ===================== activations =====================
-        // One thread, one bulk copy per k-block: the tile of (item, k-block) is one contiguous run of cnt * 128 bytes;
-        // completion is counted in bytes on the stage's barrier, and every free stage is refilled at once.
-        if (lane == 0) {
-            uint32_t it_count = 0;
-            for (int item = next_valid_item<TILE>(a, blockIdx.x, n_items, rbs); item < n_items && !*abort_v;
-                 item = next_valid_item<TILE>(a, item + gridDim.x, n_items, rbs)) {
-                const Item it = item_info<TILE>(a, item, rbs);
-                const uint32_t bytes = (uint32_t)it.cnt * 128u;
-                const unsigned char *src = reinterpret_cast<const unsigned char *>(a.x) + (int64_t)it.start * 128;
-                for (int kb = 0; kb < n_kb; ++kb, ++it_count) {
-                    const int stage = it_count % kStages;
-                    if (!mbar_wait(&empty_bar[stage], ((it_count / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
-                        raise_abort(item, 5);
+        if (elect_one()) {
+            bool ok = true;
+            for (int i = 0; ok; ++i) {
+                const Item it = read_item_one(i);
+                if (it.bucket < 0) break;
+                if (it.bucket >= a.E) continue;
+                int y0, y1;
+                if (MODE == kTcSwiglu) y0 = (int)(it.bucket * a.N + it.rb * (kRows / 2)), y1 = y0 + (int)(a.N / 2);
+                else y0 = (int)(it.bucket * a.N + (int64_t)it.rb * kRows), y1 = y0 + kRows / 2;
+                for (int step = 0; step < n_steps; ++step) {
+                    const uint32_t slot = issued % kWSlots;
+                    if (issued >= (uint32_t)kWSlots && !mbar_wait(&w_empty[slot], ((issued / kWSlots) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                        raise_abort(blockIdx.x + i * gridDim.x, 6);
+                        ok = false;
                         break;
                     }
-                    mbar_expect_tx(&full_bar[stage], bytes);
-                    bulk_g2s(smem_u32(smem + stage * kStageBytes), src + (int64_t)kb * a.L.S * 128, bytes, &full_bar[stage]);
+                    const uint32_t dst = w_base + slot * (uint32_t)kSlotBytes;
+                    // test hook: CTA 0 leaves one slot unfilled (neither the byte count nor the copies), so that its consumers'
+                    // wait runs out at the launch's limit and the abort path is exercised without anything faulting
+                    if (!(blockIdx.x == 0 && (int)issued == a.test_skip_slot)) {
+                        mbar_expect_tx(&w_full[slot], (uint32_t)kSlotBytes);
+                        tma_load_2d(dst, &wmap, step * (kBK * BITS / 8), y0, &w_full[slot]);
+                        tma_load_2d(dst + kSlotBytes / 2, &wmap, step * (kBK * BITS / 8), y1, &w_full[slot]);
+                    }
+                    ++issued;
                 }
             }
         }
-    } else if (warp == kMmaWarp) {
-        // ===================== MMA issue =====================
-        // The whole warp runs the loop with warp-uniform operands and elect.sync picks the issuing lane (always the same
-        // one for a full mask), which keeps descriptors and addresses out of per-thread registers.
-        uint32_t it_count = 0, acc_count = 0;
-        bool ready = false;  // the probe issued with the previous k-block already saw this one's operands
-        for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x) {
-            const Item it = item_info<TILE>(a, item, rbs);
-            if (it.bucket >= a.E) continue;
-            const uint32_t half = acc_count % kAccs, acc_phase = (acc_count / kAccs) & 1u;  // the accumulators take turns
-            ++acc_count;
-            if (lane == 0 && !mbar_wait(&acc_empty[half], acc_phase ^ 1u, abort_v, a.wait_limit_ns)) raise_abort(item, 2);
-            __syncwarp();
-            if (*abort_v) break;
-            tc_fence_after();
-            const int n_cols = (it.cnt + 15) & ~15;
-            const uint32_t idesc = instr_desc(n_cols);
-            const uint32_t d = tmem_base + half * (uint32_t)kTile;
-            for (int kb = 0; kb < n_kb; ++kb, ++it_count) {
-                const int stage = it_count % kStages;
-                const uint32_t phase = (it_count / kStages) & 1u;
-                bool failed = false;
-                if (lane == 0 && !ready && !mbar_wait(&full_bar[stage], phase, abort_v, a.wait_limit_ns)) raise_abort(item, 3), failed = true;
-                // One vote reconverges the warp and tells it whether lane 0's wait gave up (a wait gives up when its
-                // limit runs out or once another warp has raised the abort flag); the item loop re-reads the flag.
-                if (__any_sync(0xffffffffu, failed)) break;
-                tc_fence_after();
-                const uint64_t b_desc = smem_desc(smem_u32(smem + stage * kStageBytes));
-                const uint32_t at = tmem_base + (uint32_t)(kAccs * kTile + stage * kAStageCols);
-                static_assert(kBK / 16 == 4, "tc_kblock_ts issues four MMAs");
-                // the stage is freed when these MMAs have read it; the last k-block hands the accumulator to the epilogue
-                const bool last = kb == n_kb - 1;
-                ready = tc_kblock_ts(d, at, b_desc, idesc, kb != 0, &empty_bar[stage], last ? &acc_full[half] : nullptr,
-                                     &full_bar[(it_count + 1) % kStages], ((it_count + 1) / kStages) & 1u);
+        __syncwarp();
+    } else if (warp == kBCopyWarp) {
+        // ===================== activations =====================
+        // One thread, two bulk copies per step: the tile of (item, 64 k) is one contiguous run of cnt * 128 bytes;
+        // completion is counted in bytes on the stage's barrier, and every free stage is refilled at once.
+        if (elect_one()) {
+            uint32_t count = 0;
+            bool ok = true;
+            const int64_t line = a.L.S * 128;  // bytes from one 64-k sub-tile to the next
+            for (int i = 0; ok; ++i) {
+                const Item it = read_item_one(i);
+                if (it.bucket < 0) break;
+                if (it.bucket >= a.E) continue;
+                const uint32_t bytes = (uint32_t)it.cnt * 128u;
+                const unsigned char *src = reinterpret_cast<const unsigned char *>(a.x) + (int64_t)it.start * 128;
+                for (int st = 0; st < n_steps; ++st, ++count, src += 2 * line) {
+                    const uint32_t stage = count % kStages;
+                    if (!mbar_wait(&empty_bar[stage], ((count / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                        raise_abort(blockIdx.x + i * gridDim.x, 5);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t dst = b_base + stage * (uint32_t)kStageBytes;
+                    mbar_expect_tx(&full_bar[stage], 2 * bytes);
+                    bulk_g2s(dst, src, bytes, &full_bar[stage]);
+                    bulk_g2s(dst + kSubBytes, src + line, bytes, &full_bar[stage]);
+                }
             }
         }
-        // Drain: every MMA issued by this CTA has completed before tensor memory is released.
-        // (this wait does not give up when the CTA is aborting: tensor memory must not be released under an MMA)
-        tc_commit(&drain_bar);
-        if (lane == 0) mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        // ===================== MMA issue =====================
+        if (elect_one()) {
+            uint32_t count = 0, acc_count = 0;
+            bool ok = true;
+            for (int i = 0; ok; ++i) {
+                const Item it = read_item_one(i);
+                if (it.bucket < 0) break;
+                if (it.bucket >= a.E) continue;
+                const uint32_t idesc = instr_desc((it.cnt + 15) & ~15);
+                const uint32_t half = acc_count & 1u;  // the accumulators take turns
+                if (!mbar_wait(&acc_empty[half], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                    raise_abort(blockIdx.x + i * gridDim.x, 2);
+                    break;
+                }
+                ++acc_count;
+                tc_fence_after();
+                const uint32_t d = half * (uint32_t)kTile;
+                for (int st = 0; st < n_steps; ++st, ++count) {
+                    const uint32_t stage = count % kStages;
+                    if (!mbar_wait(&full_bar[stage], (count / kStages) & 1u, abort_v, a.wait_limit_ns)) {
+                        raise_abort(blockIdx.x + i * gridDim.x, 3);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t b_desc = smem_desc(b_base + stage * (uint32_t)kStageBytes);
+                    const uint32_t at = (uint32_t)(kAccs * kTile) + stage * (uint32_t)kAStageCols;
+#pragma unroll
+                    for (int j = 0; j < kBK / 16; ++j)  // k = 16 an instruction: 8 columns of A, 32 bytes along B's swizzled line
+                        tc_mma_f16_ts_one(d, at + 8 * j, b_desc + (j >> 2) * (kSubBytes >> 4) + 2 * (j & 3), idesc, (st | j) != 0);
+                    tc_commit_one(&empty_bar[stage]);  // the stage is free when these MMAs have read it
+                }
+                if (ok) tc_commit_one(&acc_full[half]);
+            }
+            // Drain: every MMA issued by this CTA has completed before tensor memory is released.
+            // (this wait does not give up when the CTA is aborting: tensor memory must not be released under an MMA)
+            tc_commit_one(&drain_bar);
+            mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
+        }
         __syncwarp();
     } else if (MODE == kTcHcUp && warp < kEpiWarps) {
         // ===================== epilogue of the hyper-connection up mix =====================
@@ -446,9 +510,9 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
                 uint32_t acc_count = 0, pass_count = 0;
                 const int quad = warp & 3, s = lane & 3, jj = lane >> 2;
                 const int col_lo = (warp >> 2) * (kTile / kEpiSets);
-                const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+                const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
                 const int64_t row_bytes = 4 * hc.d * es;  // a token's four streams
-                unsigned char *my_buf = smem + kStages * kStageBytes + kWSlots * kWSlotBytes + warp * (2 * kHcUpBufBytes);
+                unsigned char *my_buf = smem + kStages * kStageBytes + kWSlots * kSlotBytes + warp * (2 * kHcUpBufBytes);
                 // Copy number k of a pass: piece p = 32 k + lane of the pass's [token][stream][part] order, i.e. token
                 // k * (8 / parts) + tok_l, stream str_l, part part_l with parts = seg / 16.
                 constexpr int kParts = seg / 16, kTokStep = 8 / kParts;
@@ -464,12 +528,15 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
                     cp_async_commit();
                 };
                 auto col_hi_of = [&](const Item &it) { return min(it.cnt, col_lo + kTile / kEpiSets); };
-                if (blockIdx.x < n_items) {
-                    const Item it0 = item_info<TILE>(a, blockIdx.x, rbs);
-                    issue(it0, col_lo, col_hi_of(it0), my_buf);
-                }
-                for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x) {
-                    const Item it = item_info<TILE>(a, item, rbs);
+                float itn_scale = 1.f;
+                Item itn = read_item(0, quad * 32 + lane, itn_scale);
+                if (itn.bucket >= 0) issue(itn, col_lo, col_hi_of(itn), my_buf);
+                for (int i = 0; itn.bucket >= 0; ++i) {
+                    const Item it = itn;
+                    // sigmoid(z) = 1 / (1 + 2^(-z log2 e)), with the row's power of two taken out of z on the way
+                    const float nz = -1.44269504f * unscale(itn_scale);
+                    itn = read_item(i + 1, quad * 32 + lane, itn_scale);
+                    const int item = blockIdx.x + i * gridDim.x;
                     const int64_t j = (int64_t)it.rb * 32 + quad * 8 + jj;
                     const float nwp = 1.0f + __ldg(hc.norm_w + (int64_t)s * hc.d + j);
                     const int col_hi = col_hi_of(it);
@@ -487,8 +554,7 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
                         __syncwarp();  // every lane has finished reading the buffer that the next copies overwrite
                         if (c0 + 32 < col_hi) {
                             issue(it, c0 + 32, col_hi, nxt);
-                        } else if (item + (int)gridDim.x < n_items) {
-                            const Item itn = item_info<TILE>(a, item + gridDim.x, rbs);
+                        } else if (itn.bucket >= 0) {
                             issue(itn, col_lo, col_hi_of(itn), nxt);
                         } else {
                             cp_async_commit();
@@ -521,7 +587,7 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
                             for (int hf = 0; hf < 2; ++hf) {
                                 const int tt = t + 16 * hf;
                                 const float z = hf ? vb[t] : va[t];
-                                const float c = __fdividef(load_as_f32(xs_, tt * 32) * ivs[tt * 4] * nwp, 1.0f + __expf(-z));
+                                const float c = __fdividef(load_as_f32(xs_, tt * 32) * ivs[tt * 4] * nwp, 1.0f + exp2_fast(z * nz));
                                 if (hf) vb[t] = c;
                                 else va[t] = c;
                             }
@@ -549,103 +615,104 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
         }
     } else if (warp < kEpiWarps) {
         // ===================== epilogue =====================
-        // Lane = weight row: 32 tokens at a time from tensor memory into registers (two loads of 16 columns), then one
-        // store per token straight to global memory - for a fixed token a warp's rows are contiguous bytes.  Tensor
-        // memory goes back to the MMA warp as soon as the item's last columns are in registers.  What depends on the
-        // token - the output row of its slot, or its line in the tile-blocked h - is computed by lane t for token t of
-        // the pass and handed round by shuffles.
+        // Lane = weight row: 16 tokens at a time from tensor memory into registers (two loads of 8 columns: a longer pass
+        // would be more code than the instruction caches hold beside the producers'), then one store per token straight
+        // to global memory - for a fixed token a warp's rows are contiguous bytes.  Tensor memory goes back to the MMA
+        // thread as soon as the item's last columns are in registers.  What depends on the token - the output row of its slot - is
+        // computed by lane t for token t of the pass and handed round by shuffles; a line of the tile-blocked h follows from
+        // the token's position.
         uint32_t acc_count = 0;
         const int64_t I = a.N / 2;
         const bool tiled_out = MODE == kTcSwiglu && a.out_f16 >= 3;
         const bool h_as_f16 = a.out_f16 != 0, q4_order = a.out_f16 == 2 || a.out_f16 == 3;
-        const int quad = warp & 3;                         // the lane quadrant this warp may read
-        const int col_lo = (warp >> 2) * (kTile / kEpiSets);  // this warp's set takes the columns [col_lo, col_lo + kTile / kEpiSets)
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
+        const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;  // warp = the lane quadrant it may read
         const int up_lane = lane >> 4;  // SwiGLU: lanes 16-31 hold the up rows of the h columns of lanes 0-15
-        for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x) {
-            const Item it = item_info<TILE>(a, item, rbs);
+        for (int i = 0;; ++i) {
+            float scale = 1.f;
+            const Item it = read_item(i, warp * 32 + lane, scale);
+            if (it.bucket < 0) break;
+            const float back = unscale(scale);  // undoes the row's power of two
             const bool valid = it.bucket < a.E;
             // per-thread constants of the item: byte offset of this thread's element inside a token's output row / line
             int64_t elem_off;
             uint32_t xor_chunk = 0;  // tile-blocked h: 16-byte chunk of the line, before the per-token swizzle
             bool row_ok;
             if (MODE == kTcSwiglu) {
-                const int64_t j = (int64_t)it.rb * (kRows / 2) + quad * 16 + (lane & 15);  // h column
+                const int64_t j = (int64_t)it.rb * (kRows / 2) + warp * 16 + (lane & 15);  // h column
                 const int j7 = (int)(j & 7), pos = q4_order ? (((j7 & 3) << 1) | (j7 >> 2)) : j7;  // [0 4 1 5 2 6 3 7]
                 row_ok = j < I;
-                if (tiled_out) elem_off = (j >> 6) * a.L.S * 128 + pos * 2, xor_chunk = (uint32_t)((j & 63) >> 3);
+                if (tiled_out) elem_off = (j >> 6) * a.L.S * 128 + pos * 2 + (int64_t)(it.start + 8 * up_lane) * 128, xor_chunk = (uint32_t)((j & 63) >> 3);
                 else elem_off = ((j & ~(int64_t)7) + pos) * 2;
             } else {
-                const int64_t r = (int64_t)it.rb * kRows + quad * 32 + lane;
+                const int64_t r = (int64_t)it.rb * kRows + warp * 32 + lane;
                 row_ok = r < a.N;
                 elem_off = r * (MODE == kTcPartial ? 4 : 2);
             }
-            // Slot of token n of the item (fetched one pass ahead; nothing may depend on the loaded value before the next
-            // pass, or the in-order issue would stall this pass's stores behind it).
+            // Slot of token n of the item (lanes 0-15 and again 16-31; fetched one pass ahead: nothing may depend on the loaded
+            // value before the next pass, or the in-order issue would stall this pass's stores behind it).
             auto token_slot = [&](int n) -> int { return (tiled_out || n >= it.cnt) ? 0 : slot_at(it.start + n); };
-            // Offset of a token's output row / line, in 16-byte units.
-            auto token_off = [&](int n, int slot) -> uint32_t {
-                if (tiled_out) return (uint32_t)(it.start + n) * 8u;
+            // Offset of a token's output row, in 16-byte units.
+            auto token_off = [&](int slot) -> uint32_t {
                 return (uint32_t)(((int64_t)slot * (MODE == kTcSwiglu ? I * 2 : a.N * (MODE == kTcPartial ? 4 : 2))) >> 4);
             };
-            const int col_hi = min(it.cnt, col_lo + kTile / kEpiSets);  // this set's tokens: [col_lo, col_hi)
-            int slot_nxt = token_slot(col_lo + lane);
+            int slot_nxt = token_slot(lane & 15);
             uint32_t half = 0;
             if (valid) {
-                half = acc_count % kAccs;
-                const uint32_t acc_phase = (acc_count / kAccs) & 1u;
+                half = acc_count & 1u;
+                const uint32_t acc_phase = (acc_count >> 1) & 1u;
                 ++acc_count;
-                if (lane == 0 && !mbar_wait(&acc_full[half], acc_phase, abort_v, a.wait_limit_ns)) raise_abort(item, 4);
-                __syncwarp();
-                if (*abort_v) break;
+                const bool ok = mbar_wait(&acc_full[half], acc_phase, abort_v, a.wait_limit_ns);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 4);
+                    break;
+                }
                 tc_fence_after();
-                if (col_lo >= col_hi && lane == 0) mbar_arrive(&acc_empty[half]);  // none of the item's tokens are this set's
             }
             unsigned char *out = static_cast<unsigned char *>(a.out) + elem_off;
-            for (int c0 = col_lo; c0 < col_hi; c0 += 32) {
-                float va[16], vb[16];  // this row's accumulators of tokens c0 .. c0 + 15 and c0 + 16 .. c0 + 31
+            for (int c0 = 0; c0 < it.cnt; c0 += 16) {
+                float va[8], vb[8];  // this row's accumulators of tokens c0 .. c0 + 7 and c0 + 8 .. c0 + 15
                 if (valid) {
-                    const uint32_t col = lane_addr + half * (uint32_t)kTile + (uint32_t)c0;
-                    tc_ld16x2(col, col + 16u, va, vb);
-                    if (c0 + 32 >= col_hi) {  // this set's last columns are out: its share of the accumulator is free
+                    tc_ld8x2(lane_addr + half * (uint32_t)kTile + (uint32_t)c0, va, vb);
+                    if (c0 + 16 >= it.cnt) {  // the last columns are out: this warp's share of the accumulator is free
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[half]);
                     }
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) va[t] *= back, vb[t] *= back;
                 } else {
 #pragma unroll
-                    for (int t = 0; t < 16; ++t) va[t] = vb[t] = qnan_f32();
+                    for (int t = 0; t < 8; ++t) va[t] = vb[t] = qnan_f32();
                 }
-                const uint32_t off_cur = token_off(c0 + lane, slot_nxt);
-                if (c0 + 32 < col_hi) slot_nxt = token_slot(c0 + 32 + lane);
-                const int live = it.cnt - c0;  // tokens of this pass; the columns past them are computed and dropped
+                const uint32_t off_cur = token_off(slot_nxt);
+                if (c0 + 16 < it.cnt) slot_nxt = token_slot(c0 + 16 + (lane & 15));
+                const int live = row_ok ? it.cnt - c0 : 0;  // tokens of this pass; the columns past them are computed and dropped
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
+                for (int t = 0; t < 8; ++t) {
                     if (MODE == kTcSwiglu) {
-                        // the gate lane finishes token c0 + t, its up lane token c0 + 16 + t: each sends the other the
+                        // the gate lane finishes token c0 + t, its up lane token c0 + 8 + t: each sends the other the
                         // value that one needs (kernels/moe_grouped.hip:508-524: from the FP32 accumulators, rounded once)
-                        const float mine = up_lane ? va[t] : vb[t], theirs = __shfl_xor_sync(0xffffffffu, mine, 16);
+                        const float theirs = __shfl_xor_sync(0xffffffffu, up_lane ? va[t] : vb[t], 16);
                         const float g = up_lane ? theirs : va[t], u = up_lane ? vb[t] : theirs;
-                        // a token's line of the tile-blocked h follows from its position; otherwise its slot's row was
-                        // looked up by lane (t or t + 16) of this pass
-                        const int64_t off = tiled_out ? (int64_t)(it.start + c0 + t + 16 * up_lane) << 7
-                                                      : (int64_t)__shfl_sync(0xffffffffu, off_cur, t + (lane & 16)) << 4;
                         const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(silu_fast(g) * u));
                         const uint16_t hv = h_as_f16 ? __half_as_ushort(__float2half_rn(bf16_bits_to_f32(b))) : b;
-                        const uint32_t sw = tiled_out ? ((xor_chunk ^ (uint32_t)(t & 7)) << 4) : 0u;
-                        if (row_ok && t + 16 * up_lane < live) *reinterpret_cast<uint16_t *>(out + off + sw) = hv;
+                        unsigned char *p = out;
+                        if (tiled_out) p += t * 128 + ((xor_chunk ^ (uint32_t)t) << 4);
+                        else p += (int64_t)__shfl_sync(0xffffffffu, off_cur, t + 8 * up_lane) << 4;
+                        if (t + 8 * up_lane < live) *reinterpret_cast<uint16_t *>(p) = hv;
                     } else {
                         const int64_t off_a = (int64_t)__shfl_sync(0xffffffffu, off_cur, t) << 4;
-                        const int64_t off_b = (int64_t)__shfl_sync(0xffffffffu, off_cur, t + 16) << 4;
+                        const int64_t off_b = (int64_t)__shfl_sync(0xffffffffu, off_cur, t + 8) << 4;
                         if (MODE == kTcPartial) {
-                            if (row_ok && t < live) *reinterpret_cast<float *>(out + off_a) = va[t];
-                            if (row_ok && t + 16 < live) *reinterpret_cast<float *>(out + off_b) = vb[t];
+                            if (t < live) *reinterpret_cast<float *>(out + off_a) = va[t];
+                            if (t + 8 < live) *reinterpret_cast<float *>(out + off_b) = vb[t];
                         } else {  // BF16 rows: the plain gather's y, or the per-slot dots as kernels/moe_grouped.hip:47-57 stores them
-                            if (row_ok && t < live) *reinterpret_cast<uint16_t *>(out + off_a) = __bfloat16_as_ushort(__float2bfloat16_rn(va[t]));
-                            if (row_ok && t + 16 < live) *reinterpret_cast<uint16_t *>(out + off_b) = __bfloat16_as_ushort(__float2bfloat16_rn(vb[t]));
+                            if (t < live) *reinterpret_cast<uint16_t *>(out + off_a) = __bfloat16_as_ushort(__float2bfloat16_rn(va[t]));
+                            if (t + 8 < live) *reinterpret_cast<uint16_t *>(out + off_b) = __bfloat16_as_ushort(__float2bfloat16_rn(vb[t]));
                         }
                     }
                 }
+                if (tiled_out) out += 16 * 128;
             }
         }
     }
@@ -660,55 +727,41 @@ __global__ void __launch_bounds__((Shape<TILE, MODE == kTcHcUp>::kThreads), 1)
             if (blockIdx.x == 0 && (int)last == a.test_skip_slot) continue;  // the test hook's slot was never filled
             mbar_wait(&w_full[sl], (last / kWSlots) & 1u, nullptr, 1000000ull);
         }
-        if (warp == kBCopyWarp && lane == 0)
+        if (warp == kBCopyWarp)
             for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 50000ull;) {}
     }
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_smem), "r"(kTmemCols) : "memory");
     }
 }
 
 }  // namespace
 
-// Two boxes of 64 bytes x 64 rows fill a ring slot; 16-byte chunks swizzled in the 64-byte mode so that the producers'
-// 16-byte reads of consecutive rows hit every bank once.
+// Two boxes of 128 codes x 64 rows fill a ring slot; 16-byte chunks swizzled in the mode of the box's row length so that the
+// producers' 16-byte reads of consecutive rows hit every bank once.
 template <int BITS, int MODE>
 int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     SXB_CHECK(a.x_kind == 3, fn, ": the tiled tcgen05 kernel takes tile-blocked activations only");
+    using S = Shape<BITS, MODE == kTcHcUp>;
+    const uint64_t row_bytes = (uint64_t)(BITS == 4 ? a.K / 2 : a.K);
     CUtensorMap wmap;
-    if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)(BITS == 4 ? a.K / 2 : a.K), (uint64_t)(a.E * a.N),
-                               (uint64_t)(BITS == 4 ? a.K / 2 : a.K), 64u, (uint32_t)(kRows / 2), CU_TENSOR_MAP_SWIZZLE_64B, &wmap))
+    if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)(a.E * a.N), row_bytes, (uint32_t)(kBK * BITS / 8),
+                               (uint32_t)(kRows / 2), BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
         return rc;
-    // A long contraction (gate/up: d = 4096 is 64 k-blocks) takes the wider tile; a short one (down: I = 1024 is 16 k-blocks)
-    // the narrower, double-buffered one: there the epilogue weighs as much as the mainloop.
-    // (the up mix of the hyper-connections contracts over its rank, at most 1024: it has the narrower form only)
-    const bool wide = MODE != kTcHcUp && a.K >= 2048;
-    using SB = Shape<kTcTileB>;
-    using SA = Shape<kTcTileA, MODE == kTcHcUp>;
-    const size_t smem = (wide ? (size_t)SB::kStages * SB::kStageBytes + (size_t)SB::kWSlots * kWSlotBytes
-                              : (size_t)SA::kStages * SA::kStageBytes + (size_t)SA::kWSlots * kWSlotBytes) + 1024 +
-                        (MODE == kTcHcUp ? (size_t)SA::kEpiWarps * 2 * kHcUpBufBytes : 0);
+    const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + 1024 +
+                        (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
     auto go = [&](auto kern) -> int {
         SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
-        kern<<<(unsigned)sm_count(), wide ? SB::kThreads : SA::kThreads, smem, st>>>(a, wmap);
+        kern<<<(unsigned)sm_count(), S::kThreads, smem, st>>>(a, wmap);
         return SXB_OK;
     };
-    if constexpr (MODE != kTcHcUp) {
-        if (wide) {
-            switch (G) {
-                case 32: return go(tiled_tc_kernel<BITS, 32, MODE, kTcTileB>);
-                case 64: return go(tiled_tc_kernel<BITS, 64, MODE, kTcTileB>);
-                default: return go(tiled_tc_kernel<BITS, 128, MODE, kTcTileB>);
-            }
-        }
-    }
     switch (G) {
-        case 32: return go(tiled_tc_kernel<BITS, 32, MODE, kTcTileA>);
-        case 64: return go(tiled_tc_kernel<BITS, 64, MODE, kTcTileA>);
-        default: return go(tiled_tc_kernel<BITS, 128, MODE, kTcTileA>);
+        case 32: return go(tiled_tc_kernel<BITS, 32, MODE>);
+        case 64: return go(tiled_tc_kernel<BITS, 64, MODE>);
+        default: return go(tiled_tc_kernel<BITS, 128, MODE>);
     }
 }
 

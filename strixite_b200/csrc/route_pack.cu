@@ -330,9 +330,11 @@ int tc_status_error(const char *what, const uint32_t e[3]) {
                                   "the epilogue waiting for the accumulators",
                                   "the activation copy thread waiting for a free operand stage",
                                   "the weight-code copy thread waiting for a free ring slot",
-                                  "a weight producer waiting for its packed codes"};
+                                  "a weight producer waiting for its packed codes",
+                                  "a warp waiting for the description of its next work item",
+                                  "the work-item thread waiting for room in its ring"};
     last_error() = cat(what ? what : "", ": a tcgen05 kernel gave up a wait at work item ", e[1], " (",
-                       roles[e[2] >= 1 && e[2] <= 7 ? e[2] : 0], "); its outputs are incomplete");
+                       roles[e[2] >= 1 && e[2] <= 9 ? e[2] : 0], "); its outputs are incomplete");
     return SXB_ERR_DATA;
 }
 }  // namespace sxb

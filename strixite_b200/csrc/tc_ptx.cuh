@@ -54,14 +54,39 @@ __device__ inline unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
+// The same, the thread suspended by the hardware for up to `ns` while the phase has not completed.
+__device__ inline bool mbar_try_wait_for(uint64_t *bar, uint32_t parity, uint32_t ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait.  False when the CTA is aborting or the limit ran out (then the caller raises the abort itself).
-// The common case must stay cheap: the first polls touch nothing but the barrier; the abort flag and the (slow to read)
-// global timer are consulted only once a wait has lasted thousands of polls.
+// A waiting warp must not take issue slots from the working ones: the wait suspends for 10 us at a time, and the abort flag
+// and the (slow to read) global timer are looked at in between.  (Without the time hint the polls of the waiting warps were
+// 40 % of the instructions that the tiled tcgen05 kernel issued, at two thirds of the issue slots busy.)
 __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, unsigned long long limit_ns) {
+    if (mbar_try_wait(bar, parity)) return true;
     unsigned long long t0 = 0;
-    for (uint32_t spins = 0;; ++spins) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spins & 4095u) == 4095u) {
+    while (!mbar_try_wait_for(bar, parity, 10000u)) {
+        if (abort_flag != nullptr && *abort_flag) return false;
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > limit_ns) return false;
+    }
+    return true;
+}
+// The same for a single thread that everyone else waits for: no suspension, so no time is lost waking up.
+__device__ inline bool mbar_spin(uint64_t *bar, uint32_t parity, volatile int *abort_flag, unsigned long long limit_ns) {
+    unsigned long long t0 = 0;
+    for (uint32_t spins = 1;; ++spins) {
+        if (mbar_test_wait(bar, parity)) return true;
+        if ((spins & 1023u) == 0u) {
             if (abort_flag != nullptr && *abort_flag) return false;
             const unsigned long long now = global_ns();
             if (t0 == 0) t0 = now;
@@ -98,6 +123,25 @@ __device__ inline void tc_ld16x2(uint32_t taddr0, uint32_t taddr1, float (&v0)[1
 #pragma unroll
     for (int i = 0; i < 16; ++i) v0[i] = __uint_as_float(r[i]), v1[i] = __uint_as_float(q[i]);
 }
+// 2 x 8 consecutive columns of this thread's TMEM lane.
+__device__ inline void tc_ld8x2(uint32_t taddr, float (&v0)[8], float (&v1)[8]) {
+    uint32_t r[8], q[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
+                 : "r"(taddr + 8));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v0[i] = __uint_as_float(r[i]), v1[i] = __uint_as_float(q[i]);
+}
+// 2^v on the special-function unit.
+__device__ inline float exp2_fast(float v) {
+    float r;
+    asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
 // silu on the special-function unit: ex2 and a reciprocal, a few ulp of FP32 - far inside the BF16 rounding that follows.
 __device__ inline float silu_fast(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 
@@ -119,6 +163,25 @@ __device__ inline void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t 
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// The same for a loop that runs under ONE election: elect_one() picks a lane of the converged warp, and that lane alone runs
+// the loop with these.  An MMA then costs its issuer 12 cycles; with the election inside each instruction group, 40 to 90.
+__device__ inline bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ inline void tc_mma_f16_ts_one(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        : "memory");
+}
+__device__ inline void tc_commit_one(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // One k-block of an accumulator as one instruction group: a non-blocking probe of the NEXT k-block's "operands ready"
