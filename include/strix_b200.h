@@ -13,7 +13,10 @@
  * Ownership, as in the reference (kernels/moe_grouped.hpp:84-87, runtime/qwen4exp.cpp:1092-1101): the caller owns
  * every buffer - weights, activations, ids / coef, the grouping workspace, the combine's `partial`, the error
  * words.  Unless a declaration says otherwise, no entry point allocates, frees or synchronizes; all work is enqueued
- * on the caller's stream.  Exceptions: sxb_check_*_error (a blocking 12-byte copy, as the reference's).
+ * on the caller's stream.  Exceptions: sxb_check_*_error (a blocking 12-byte copy, as the reference's), and the WMMA_F16
+ * entries given row-major activations (BF16, or F16 other than SXB_ACT_F16_TILED): they write the tile-blocked form into
+ * stream-ordered scratch of the library, which keeps at most 1 GiB of it per device between calls (sxb_release_scratch gives
+ * that back).  The ..._noalloc entries never do.
  *
  * Error words (`err`): >= 3 zeroed uint32 on the device, zeroed by the caller at session start.  A data error on the
  * device sets err[0] = 1, err[1], err[2] (first writer wins), poisons the affected outputs with NaN and never reads
@@ -105,6 +108,9 @@ typedef struct SxbMoeSharedAdd {
 const char *sxb_last_error(void);
 /* "strix_b200 <version> sm_100a" */
 const char *sxb_version(void);
+
+/* Returns the current device's idle scratch memory (see "Ownership") to the device. */
+int sxb_release_scratch(void);
 
 /* ---- Router ------------------------------------------------------------------------------------------------ */
 

@@ -53,6 +53,7 @@ SA = C.POINTER(SxbMoeSharedAdd)
 SIGNATURES = {
     "sxb_last_error": (cp, []),
     "sxb_version": (cp, []),
+    "sxb_release_scratch": (C.c_int, []),
     "sxb_moe_router": (C.c_int, [vp, i64, i64, i64, i64, vp, i64, i32, vp, vp, C.c_int, vp, vp]),
     "sxb_check_router_error": (C.c_int, [vp, cp]),
     "sxb_report_router_error": (C.c_int, [C.POINTER(u32), cp]),

@@ -39,6 +39,7 @@
 // The tensor copies read this GPU's own weight array only, each into the shared memory of the one CTA that issues it.
 
 #include "grouped_tc.cuh"
+#include "scratch.cuh"
 
 namespace sxb {
 namespace {
@@ -666,24 +667,29 @@ __global__ void __launch_bounds__(256) stage_f16_kernel(const uint4 *__restrict_
         xh[i] = b_chunk<BITS>(x[i], false);
 }
 
-// x [M, K] BF16 -> the tile-blocked F16 form (tiled_offset) for the tiles of a grouping workspace: row pos of the
-// slot order holds the activation row of token slots[pos] / A, converted, in the operand's k order, swizzled for its place
-// in its tile.  One CTA per tile at a time.
-template <int BITS>
+// x -> the tile-blocked F16 form (tiled_offset) for the tiles of a grouping workspace: position pos of the slot order holds
+// the activation row of its slot (row slots[pos] / row_div), as F16 in the operand's k order, swizzled for its place in its
+// tile.  KIND: x is BF16 (0), F16 in natural k order (1) or F16 in this operand's order (2).  HBM-bound; a CTA takes a
+// quarter of a tile at a time (32 rows), because a small batch has a handful of tiles only: whole tiles left a 1001-row
+// dense projection to eight CTAs.
+constexpr int kStageRows = 32;
+template <int BITS, int KIND>
 __global__ void __launch_bounds__(256) stage_tiles_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ ws,
-                                                          RouteWords L, int64_t A, int64_t K, unsigned char *__restrict__ xs) {
+                                                          RouteWords L, int64_t row_div, int64_t K, unsigned char *__restrict__ xs) {
     // ws == nullptr: a dense projection's rows, in their own order (L.S rows, tile t = rows 128 t ..)
+    constexpr int kParts = kMaxTileTokens / kStageRows;
     const int n_tiles = ws ? ws[3] : (int)((L.S + kMaxTileTokens - 1) / kMaxTileTokens), chunks_per_row = (int)(K / 8);
-    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    for (int part = blockIdx.x; part < n_tiles * kParts; part += gridDim.x) {
+        const int tile = part / kParts, n0 = (part % kParts) * kStageRows;
         const int bucket = ws ? ws[L.t128_bucket + tile] : 0, start = ws ? ws[L.t128_start + tile] : tile * kMaxTileTokens;
         const int cnt = ws ? min(kMaxTileTokens, ws[L.offsets + bucket + 1] - start) : (int)min((int64_t)kMaxTileTokens, L.S - start);
         if (bucket >= L.E) continue;
         // a warp takes one row at a time: its 32 lanes read 512 contiguous bytes of the token's activations per step,
         // four steps in flight
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-        for (int n = warp; n < cnt; n += warps) {
-            const int64_t tok = ws ? ws[L.slots + start + n] / A : start + n;
-            const uint4 *src = reinterpret_cast<const uint4 *>(x + tok * K);
+        for (int n = n0 + warp; n < min(cnt, n0 + kStageRows); n += warps) {
+            const int64_t row = ws ? ws[L.slots + start + n] / row_div : start + n;
+            const uint4 *src = reinterpret_cast<const uint4 *>(x + row * K);
             for (int k8 = lane; k8 < chunks_per_row; k8 += 128) {
                 uint4 v[4];
 #pragma unroll
@@ -693,11 +699,20 @@ __global__ void __launch_bounds__(256) stage_tiles_kernel(const uint16_t *__rest
                 for (int u = 0; u < 4; ++u) {
                     const int kk = k8 + 32 * u;
                     if (kk < chunks_per_row)
-                        *reinterpret_cast<uint4 *>(xs + tiled_offset(L.S, kk >> 3, start + n, n, kk & 7)) = b_chunk<BITS>(v[u], false);
+                        *reinterpret_cast<uint4 *>(xs + tiled_offset(L.S, kk >> 3, start + n, n, kk & 7)) = KIND == 2 ? v[u] : b_chunk<BITS>(v[u], KIND == 1);
                 }
             }
         }
     }
+}
+template <int BITS>
+void launch_stage_tiles(const void *x, int kind, const void *ws, const RouteWords &L, int64_t row_div, int64_t K, void *xs, cudaStream_t st) {
+    const int64_t tiles = ws ? L.T128max : (L.S + kMaxTileTokens - 1) / kMaxTileTokens;
+    const unsigned blocks = (unsigned)std::min<int64_t>(tiles * (kMaxTileTokens / kStageRows), (int64_t)sm_count() * 8);
+    auto go = [&](auto kern) { kern<<<blocks, 256, 0, st>>>((const uint16_t *)x, (const int32_t *)ws, L, row_div, K, (unsigned char *)xs); };
+    if (kind == 0) go(stage_tiles_kernel<BITS, 0>);
+    else if (kind == 1) go(stage_tiles_kernel<BITS, 1>);
+    else go(stage_tiles_kernel<BITS, 2>);
 }
 
 int check_tc(const char *fn, const void *x, const SxbQView *w, int64_t E, const void *ws, size_t ws_bytes, int64_t M,
@@ -743,8 +758,22 @@ template <int BITS, int MODE>
 int launch_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     const size_t smem = (size_t)kStages * kStageBytes + (size_t)kWSlots * kWSlotBytes + 1024;
     a.wait_limit_ns = g_wait_limit_ns, a.test_skip_slot = g_test_skip_slot;
-    // Tile-blocked activations have a kernel of their own (grouped_tc_tiled.cu).
+    // Tile-blocked activations have a kernel of their own (grouped_tc_tiled.cu), and any other form is brought into that one
+    // first, in stream-ordered scratch: a pass over the activations (14 us for the 12000 slots x 4096 of a 1200-token
+    // prefill) against two warps that convert or gather them for every row block of the weight again (a 1200-token layer with
+    // BF16 activations: 6.9 + 3.5 ms in this file's kernel).  Without scratch (out of memory, allocation-free entry points)
+    // this file's kernel takes the activations as they are.
     if (a.x_kind == 3) return launch_tiled_tc<BITS, MODE>(fn, a, G, st);
+    StreamScratch staged;
+    if (staged.get((size_t)a.L.S * (size_t)a.K * 2, st)) {
+        const bool by_slot = MODE == kTcPartial || MODE == kTcPartialBf16;
+        // F16 in natural order is the order of a Q8 operand
+        const int kind = a.x_kind == 1 && BITS == 8 ? 2 : a.x_kind;
+        launch_stage_tiles<BITS>(a.x, kind, a.ws, a.L, by_slot ? 1 : a.A, a.K, staged.ptr(), st);
+        SXB_CHECK_LAUNCH(fn, " staging ", a.L.S, " rows of ", a.K);
+        a.x = static_cast<const uint16_t *>(staged.ptr()), a.x_kind = 3;
+        return launch_tiled_tc<BITS, MODE>(fn, a, G, st);
+    }
     CUtensorMap wmap;
     if (int rc = weight_tensor_map(fn, a.q, a.E * a.N, BITS == 4 ? a.K / 2 : a.K, &wmap)) return rc;
     auto go = [&](auto kern) -> int {
@@ -972,14 +1001,10 @@ extern "C" int sxb_stage_f16_tiles(const void *x, const void *ws, size_t ws_byte
     SXB_CHECK(ws == nullptr || ws_bytes >= (size_t)route_words(M, A, E).total * 4, "stage_f16_tiles: workspace of ", ws_bytes,
               " bytes, needs ", route_words(M, A, E).total * 4);
     SXB_CHECK(aligned16(x) && aligned16(xs), "stage_f16_tiles: x and xs must be 16-byte aligned");
-    RouteWords L = route_words(M, A, E);
-    const int64_t tiles = ws ? L.T128max : (M + kMaxTileTokens - 1) / kMaxTileTokens;
-    const unsigned blocks = (unsigned)std::min<int64_t>(tiles, (int64_t)sm_count() * 4);
+    const RouteWords L = route_words(M, A, E);
     auto st = static_cast<cudaStream_t>(stream);
-    if (bits == 4)
-        stage_tiles_kernel<4><<<blocks, 256, 0, st>>>((const uint16_t *)x, (const int32_t *)ws, L, A, K, (unsigned char *)xs);
-    else
-        stage_tiles_kernel<8><<<blocks, 256, 0, st>>>((const uint16_t *)x, (const int32_t *)ws, L, A, K, (unsigned char *)xs);
+    if (bits == 4) launch_stage_tiles<4>(x, 0, ws, L, A, K, xs, st);
+    else launch_stage_tiles<8>(x, 0, ws, L, A, K, xs, st);
     SXB_CHECK_LAUNCH("stage_f16_tiles M=", M, " A=", A, " K=", K, " bits=", bits);
     return SXB_OK;
 }

@@ -27,6 +27,7 @@
 //   * Nothing here calls cudaMalloc, cudaFree or an allocating library routine.
 
 #include "experts.cuh"
+#include "scratch.cuh"
 
 #include <mutex>
 
@@ -73,5 +74,6 @@ extern "C" int sxb_linear_q4_experts_combine_grouped_noalloc(const void *h, cons
     float *partial = nullptr;
     if (int rc = partial_scratch(&partial)) return rc;
     // from here on the caller-scratch entry point's own code: the same checks (pointers, dtypes, overlaps), the same kernels
+    const NoScratch no_scratch;
     return combine_grouped<4>(fn, h, w, E, ids, coef, ws, ws_bytes, partial, M, A, y, act, out_act, math, stream, shared, h_f16, E, 0);
 }
