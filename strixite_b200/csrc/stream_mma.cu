@@ -12,14 +12,18 @@
 //   * a warp owns 16 weight rows; lane (g = lane / 4, c = lane % 4) streams rows g and g + 8 with one 16-byte
 //     `ld.global.nc` each per step, the four lanes of a quad covering 64 contiguous bytes of a row, which for the
 //     served formats (Q4 G = 128, Q8 G = 64) is exactly one quantization group;
-//   * nibbles become BF16 pairs in registers with a shift, a `lop3` and a packed subtract per pair:
-//     (w >> 4s) & 0x000F000F | 0x43004300 is the pair (128 + code, 128 + code') exactly, minus (128, 128) the codes;
-//     a Q8 byte is split into its two nibbles and the high one meets 16 * x;
+//   * codes become F16 pairs in registers: a code n in the low mantissa bits of an F16 whose exponent field is zero IS the
+//     subnormal n * 2^-24 (n * 2^-20 four bits further up), so eight nibbles take a shift and four masks of the half-rate
+//     integer pipe, four bytes two byte permutes, and a packed multiply by a power of two makes a pair of normal numbers.
+//     (With BF16 operands, whose seven mantissa bits hold a nibble in one place only, a pair took a shift and a lop3, and a
+//     Q8 code the pairs of its two nibbles.)  The activations come as F16 too, each token's times the power of two that takes
+//     its largest magnitude to 2^15 .. 2^16: BF16's eight significant bits survive for everything within 2^-32 of the largest,
+//     and what lies below is rounded at 2^-40 of it, far under the rounding of an FP32 sum that contains it;
 //   * the activations of the tile's <= 8 tokens sit in shared memory already permuted into `mma.m16n8k16` B-fragment
 //     order, so a lane fetches its fragments with conflict-free 16-byte loads; k is permuted consistently on both
 //     operands, which a dot product does not notice;
 //   * per step: D = sum over the quad's codes of q * x on the tensor cores (exact products, FP32 sums), then
-//     acc += s * D + m * sum(x) in FP32.
+//     acc += s * D + m * sum(x) in FP32; the token's power of two comes off the finished dot.
 // Work is cut into units of 16 rows x one tile of <= 8 tokens of one expert; CTAs take contiguous ranges of units so
 // a CTA restages activations only when it crosses into another tile, and every touched expert's weights are read
 // once per tile (once in total when an expert has <= 8 tokens, the decode case).
@@ -35,6 +39,7 @@ namespace {
 constexpr int kThreads = 256;      // small launches: two CTAs of eight warps an SM
 constexpr int kBigThreads = 512;   // launches with work for every SM: one CTA of sixteen warps, units handed out on demand
 constexpr int kTileTokens = 8;
+constexpr int kPerTokenPasses = 8;  // tiles of eight slots of a token at most (A <= 64)
 constexpr int kPrefetch = 4;  // steps of weights in flight per warp beyond the one being consumed
 constexpr int64_t kMaxK = 1 << 24;
 constexpr int64_t kMaxN = 0x7fffffff;
@@ -71,40 +76,59 @@ template <> __device__ inline void load_codes<1>(uint32_t (&w)[1], const uint8_t
 }
 
 // D = A * B (no accumulator input: the zero operand needs no registers set up).
-__device__ inline void mma_bf16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+__device__ inline void mma_f16_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
-__device__ inline void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+__device__ inline void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Nibbles s and s + 4 of w as the BF16 pair (n_s, n_{s+4}): `(w >> 4s) & 0x000F000F | 0x43004300` is the pair
-// (128 + n_s, 128 + n_{s+4}) exactly (BF16 keeps 8 significant bits), and one packed subtract removes the 128s.
-template <int S> __device__ inline uint32_t nibble_pair(uint32_t w) {
-    uint32_t v = ((w >> (4 * S)) & 0x000F000Fu) | 0x43004300u, r;
-    asm("sub.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0x43004300u));
+// d (+)= the products of eight codes of weight rows a and b with one staged unit of activations.  Q4: word w0; Q8: words w0,
+// w1.  Codes as F16 subnormals (the header of this file): a mask for nibbles 0, 4 and 1, 5 of a word, the same two masks for
+// nibbles 2, 6 and 3, 7 eight bits further down; a byte permute for a pair of Q8 codes.  A packed multiply then makes them the
+// normal numbers n * 2^-9: with subnormal operands the tensor cores lose the sum some of its low bits (3.4e-5 of the RMS on a
+// 64-long dot).
+__device__ inline uint32_t times_h2(uint32_t v, uint32_t f) {
+    uint32_t r;
+    asm("mul.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(f));
     return r;
 }
-
-// Nibbles s and s + 4 of w as the BF16 pair (16 + n_s, 16 + n_{s+4}): the nibble lands in the top four of the seven
-// mantissa bits of 16.0 (0x4180), whose steps are 1/8, so the value is 16 + n exactly - a shift and a lop3, no subtract.
-// The 16s are taken out after the contraction: sum((16 + n) x) = sum(n x) + 16 sum(x), and sum(x) of the group is at hand
-// for the min term anyway.
-template <int S> __device__ inline uint32_t nibble_pair16(uint32_t w) {
-    const uint32_t sh = S == 0 ? (w << 3) : (w >> (4 * S - 3));
-    return (sh & 0x00780078u) | 0x41804180u;
+template <int BITS, bool FIRST>
+__device__ inline void unit_mma(float (&d)[4], uint32_t a_w0, uint32_t a_w1, uint32_t b_w0, uint32_t b_w1, const uint4 &bx) {
+    constexpr uint32_t k2p15 = 0x78007800u, k2p11 = 0x68006800u;  // packed 2^15 and 2^11
+    uint32_t pa[4], pb[4];
+    if (BITS == 4) {
+        const uint32_t a8 = a_w0 >> 8, b8 = b_w0 >> 8;
+        pa[0] = times_h2(a_w0 & 0x000F000Fu, k2p15), pa[1] = times_h2(a_w0 & 0x00F000F0u, k2p11);
+        pa[2] = times_h2(a8 & 0x000F000Fu, k2p15), pa[3] = times_h2(a8 & 0x00F000F0u, k2p11);
+        pb[0] = times_h2(b_w0 & 0x000F000Fu, k2p15), pb[1] = times_h2(b_w0 & 0x00F000F0u, k2p11);
+        pb[2] = times_h2(b8 & 0x000F000Fu, k2p15), pb[3] = times_h2(b8 & 0x00F000F0u, k2p11);
+    } else {
+        pa[0] = times_h2(__byte_perm(a_w0, 0u, 0x4140), k2p15), pa[1] = times_h2(__byte_perm(a_w0, 0u, 0x4342), k2p15);
+        pa[2] = times_h2(__byte_perm(a_w1, 0u, 0x4140), k2p15), pa[3] = times_h2(__byte_perm(a_w1, 0u, 0x4342), k2p15);
+        pb[0] = times_h2(__byte_perm(b_w0, 0u, 0x4140), k2p15), pb[1] = times_h2(__byte_perm(b_w0, 0u, 0x4342), k2p15);
+        pb[2] = times_h2(__byte_perm(b_w1, 0u, 0x4140), k2p15), pb[3] = times_h2(__byte_perm(b_w1, 0u, 0x4342), k2p15);
+    }
+    if (FIRST) mma_f16_first(d, pa[0], pb[0], pa[1], pb[1], bx.x, bx.y);
+    else mma_f16(d, pa[0], pb[0], pa[1], pb[1], bx.x, bx.y);
+    mma_f16(d, pa[2], pb[2], pa[3], pb[3], bx.z, bx.w);
 }
 
-__device__ inline uint32_t times16(uint32_t bf16x2) {
-    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162 *>(&bf16x2);
-    v = __hmul2(v, __float2bfloat162_rn(16.f));
-    return *reinterpret_cast<uint32_t *>(&v);
+__device__ inline float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // e in -126 .. 127
+
+// The exponent e of a token's scale 2^e from the largest magnitude of its activations (BF16 bits without the sign): 2^15 <= max
+// * 2^e < 65504, where the clamp to exponents that FP32 can hold allows it.
+__device__ inline int token_exponent(uint32_t max_bits) { return min(max(142 - (int)(max_bits >> 7), -112), 126); }
+// A dot of the staged operands back to its value: v * 2^(9 - e), in two factors that meet no range limit the result does not.
+__device__ inline float unscaled(float v, int e) {
+    const int t = 9 - e, h = t >> 1;
+    return v * pow2f(h) * pow2f(t - h);
 }
 
 struct StreamArgs {
@@ -123,14 +147,52 @@ struct StreamArgs {
 
 template <typename T> __device__ inline void store_out(T *p, int64_t i, float v) { store_from_f32(p, i, v); }
 
-// Stages up to 8 activation rows (rows[n] < 0 = none, zeros) into fragment order at xs / xsum.  All threads of the CTA.
+// Stages up to 8 activation rows (rows[n] < 0 = none, zeros) as F16 in fragment order at xs, every row times its power of two
+// 2^e (token_exponent; max_bits[n] comes in as zero and leaves as the row's largest magnitude), and at xsum the sums of every
+// (step, token) times 2^(e - 9), the factor that the dots with the codes carry.  All threads of the CTA.
 template <int BITS, int G>
-__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum) {
+__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, uint32_t *max_bits) {
     using geo = Geo<BITS, G>;
     constexpr int UNITS = geo::kUnits, KI = geo::kStepCodes, CPL = geo::kCodesPerLane;
     const int units_per_row = K / 8, steps = K / KI;
-    // 8 consecutive k of token n (16 bytes) -> one unit, permuted to match the nibble pairs of the weights.  Four loads a
-    // thread are issued before the first is used (see the note on batches below).
+    // sum(x) of every (step, token), in a fixed order, and the largest magnitude of every token.  blockDim is a multiple of
+    // eight, so a thread meets one token only.
+    uint32_t top = 0u;
+    for (int idx = threadIdx.x; idx < steps * kTileTokens; idx += blockDim.x) {
+        const int step = idx / kTileTokens, n = idx % kTileTokens;
+        const int64_t row = rows[n];
+        float sum = 0.f;
+        if (row >= 0) {
+            // the loads of a batch are independent of one another: under a streaming kernel's load an L2 round trip is
+            // thousands of cycles, and one load at a time made staging a tenth of a decode kernel's time
+            const uint4 *p = reinterpret_cast<const uint4 *>(x + row * K + (int64_t)step * KI);
+            constexpr int kBatch = KI / 8 < 8 ? KI / 8 : 8;
+            for (int i0 = 0; i0 < KI / 8; i0 += kBatch) {
+                uint4 u[kBatch];
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) u[i] = p[i0 + i];
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) {
+                    const uint32_t w4[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        sum += __uint_as_float(w4[j] << 16), sum += __uint_as_float(w4[j] & 0xffff0000u);
+                        top = __vmaxu2(top, w4[j] & 0x7fff7fffu);
+                    }
+                }
+            }
+        }
+        xsum[idx] = sum;
+    }
+    top = max(top >> 16, top & 0xffffu);
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 8));
+    top = max(top, __shfl_xor_sync(0xffffffffu, top, 16));
+    if ((threadIdx.x & 31) < kTileTokens) atomicMax(&max_bits[threadIdx.x & 7], top);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < steps * kTileTokens; idx += blockDim.x)  // each thread the sums it wrote
+        xsum[idx] = xsum[idx] * pow2f(token_exponent(max_bits[idx % kTileTokens])) * 0x1p-9f;
+    // 8 consecutive k of token n (16 bytes) -> one unit, permuted to match the pairs of codes.  Four loads a thread are issued
+    // before the first is used (see the note on batches above).
     const int n_units = kTileTokens * units_per_row, stride = (int)blockDim.x;
     for (int base = threadIdx.x; base < n_units; base += 4 * stride) {
         uint4 src[4];
@@ -149,53 +211,30 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             if (idx >= n_units) break;
             const int n = idx / units_per_row, k = (idx % units_per_row) * 8;
             const int step = k / KI, rem = k % KI, cc = rem / CPL, v = (rem % CPL) / 8;
+            const float f = pow2f(token_exponent(max_bits[n]));
+            const uint32_t w4[4] = {src[j].x, src[j].y, src[j].z, src[j].w};
+            float lo[4], hi[4];  // elements 2 i and 2 i + 1
+#pragma unroll
+            for (int i = 0; i < 4; ++i) lo[i] = __uint_as_float(w4[i] << 16) * f, hi[i] = __uint_as_float(w4[i] & 0xffff0000u) * f;
+            auto pack = [](float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t *>(&h); };
             uint4 dst;
             if (BITS == 4) {  // [x0 x4 | x1 x5 | x2 x6 | x3 x7]
-                dst.x = __byte_perm(src[j].x, src[j].z, 0x5410), dst.y = __byte_perm(src[j].x, src[j].z, 0x7632);
-                dst.z = __byte_perm(src[j].y, src[j].w, 0x5410), dst.w = __byte_perm(src[j].y, src[j].w, 0x7632);
-            } else {  // [x0 x2 | x1 x3 | x4 x6 | x5 x7]
-                dst.x = __byte_perm(src[j].x, src[j].y, 0x5410), dst.y = __byte_perm(src[j].x, src[j].y, 0x7632);
-                dst.z = __byte_perm(src[j].z, src[j].w, 0x5410), dst.w = __byte_perm(src[j].z, src[j].w, 0x7632);
+                dst.x = pack(lo[0], lo[2]), dst.y = pack(hi[0], hi[2]), dst.z = pack(lo[1], lo[3]), dst.w = pack(hi[1], hi[3]);
+            } else {  // natural order
+                dst.x = pack(lo[0], hi[0]), dst.y = pack(lo[1], hi[1]), dst.z = pack(lo[2], hi[2]), dst.w = pack(lo[3], hi[3]);
             }
             xs[(step * UNITS + v) * 32 + n * 4 + cc] = dst;
         }
-    }
-    // sum(x) of every (step, token), in a fixed order.
-    for (int idx = threadIdx.x; idx < steps * kTileTokens; idx += blockDim.x) {
-        const int step = idx / kTileTokens, n = idx % kTileTokens;
-        const int64_t row = rows[n];
-        float sum = 0.f;
-        if (row >= 0) {
-            // the loads of a batch are independent of one another: under a streaming kernel's load an L2 round trip is
-            // thousands of cycles, and one load at a time made staging a tenth of a decode kernel's time
-            const uint4 *p = reinterpret_cast<const uint4 *>(x + row * K + (int64_t)step * KI);
-            constexpr int kBatch = KI / 8 < 8 ? KI / 8 : 8;
-            for (int i0 = 0; i0 < KI / 8; i0 += kBatch) {
-                uint4 u[kBatch];
-#pragma unroll
-                for (int i = 0; i < kBatch; ++i) u[i] = p[i0 + i];
-#pragma unroll
-                for (int i = 0; i < kBatch; ++i) {
-                    const uint32_t w4[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) sum += __uint_as_float(w4[j] << 16), sum += __uint_as_float(w4[j] & 0xffff0000u);
-                }
-            }
-        }
-        xsum[idx] = sum;
     }
 }
 
 // One warp: the dots of weight rows rowa / rowb (lane quad g streams both) with the staged tokens.
 // acc[0], acc[1] = row a x tokens 2c, 2c+1;  acc[2], acc[3] = row b x the same tokens.
-// VEC: a step is one quantization group and the row has a multiple of four groups, so the scales and mins of the four
-// steps of a prefetch block are one aligned 8-byte load each (four loads a block instead of sixteen 2-byte ones).
-template <int BITS, int G, bool VEC>
+template <int BITS, int G>
 __device__ inline void rows_dot_impl(float (&acc)[4], const StreamArgs &a, int64_t rowa, int64_t rowb, bool va, bool vb,
                                      const uint4 *xs, const float *xsum, int lane) {
     using geo = Geo<BITS, G>;
     constexpr int W = geo::kWords, UNITS = geo::kUnits, KI = geo::kStepCodes;
-    static_assert(kPrefetch == 4, "the vector scale path loads four groups at a time");
     const int K = (int)a.K, steps = K / KI, groups = K / G, c = lane & 3;
     const int64_t row_bytes = BITS == 4 ? a.K / 2 : a.K;
     const uint8_t *pa = a.q + rowa * row_bytes + c * geo::kLoadBytes;
@@ -204,33 +243,20 @@ __device__ inline void rows_dot_impl(float (&acc)[4], const StreamArgs &a, int64
     const uint16_t *sb = a.scale + rowb * groups, *mb = a.minv + rowb * groups;
 
     uint32_t wa[kPrefetch][W], wb[kPrefetch][W];
-    uint16_t qs[VEC ? 1 : kPrefetch][4];
-    uint2 qv[2][4];  // VEC: {scale a, min a, scale b, min b} of the block in use and of the next one
+    uint16_t qs[kPrefetch][4];  // scale a, min a, scale b, min b
     auto fetch = [&](int slot, int step) {
         const bool in = step < steps;
         load_codes<W>(wa[slot], pa + (int64_t)step * 4 * geo::kLoadBytes, in && va);
         load_codes<W>(wb[slot], pb + (int64_t)step * 4 * geo::kLoadBytes, in && vb);
-        if (!VEC) {
-            const int grp = step / geo::kStepsPerGroup;
-            qs[slot][0] = in && va ? __ldg(sa + grp) : (uint16_t)0;
-            qs[slot][1] = in && va ? __ldg(ma + grp) : (uint16_t)0;
-            qs[slot][2] = in && vb ? __ldg(sb + grp) : (uint16_t)0;
-            qs[slot][3] = in && vb ? __ldg(mb + grp) : (uint16_t)0;
-        }
+        const int grp = step / geo::kStepsPerGroup;
+        qs[slot][0] = in && va ? __ldg(sa + grp) : (uint16_t)0;
+        qs[slot][1] = in && va ? __ldg(ma + grp) : (uint16_t)0;
+        qs[slot][2] = in && vb ? __ldg(sb + grp) : (uint16_t)0;
+        qs[slot][3] = in && vb ? __ldg(mb + grp) : (uint16_t)0;
     };
-    auto fetch_scales = [&](uint2 (&dst)[4], int step0) {  // VEC: the four groups step0 .. step0 + 3
-        const bool in = step0 < steps;
-        const uint2 z = make_uint2(0u, 0u);
-        dst[0] = in && va ? __ldg(reinterpret_cast<const uint2 *>(sa + step0)) : z;
-        dst[1] = in && va ? __ldg(reinterpret_cast<const uint2 *>(ma + step0)) : z;
-        dst[2] = in && vb ? __ldg(reinterpret_cast<const uint2 *>(sb + step0)) : z;
-        dst[3] = in && vb ? __ldg(reinterpret_cast<const uint2 *>(mb + step0)) : z;
-    };
-    if (VEC) fetch_scales(qv[0], 0);
 #pragma unroll
     for (int p = 0; p < kPrefetch; ++p) fetch(p, p);
     for (int step0 = 0; step0 < steps; step0 += kPrefetch) {
-        if (VEC) fetch_scales(qv[1], step0 + kPrefetch);
 #pragma unroll
         for (int p = 0; p < kPrefetch; ++p) {
             const int step = step0 + p;
@@ -240,42 +266,18 @@ __device__ inline void rows_dot_impl(float (&acc)[4], const StreamArgs &a, int64
 #pragma unroll
                 for (int v = 0; v < UNITS; ++v) {
                     const uint4 bx = xu[v * 32];
-                    if (BITS == 4) {
-                        const uint32_t x0 = wa[p][v], x1 = wb[p][v];
-                        mma_bf16(d, nibble_pair16<0>(x0), nibble_pair16<0>(x1), nibble_pair16<1>(x0), nibble_pair16<1>(x1), bx.x, bx.y);
-                        mma_bf16(d, nibble_pair16<2>(x0), nibble_pair16<2>(x1), nibble_pair16<3>(x0), nibble_pair16<3>(x1), bx.z, bx.w);
-                    } else {
-                        const uint32_t bw[4] = {bx.x, bx.y, bx.z, bx.w};
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const uint32_t x0 = wa[p][2 * v + h], x1 = wb[p][2 * v + h];
-                            mma_bf16(d, nibble_pair<0>(x0), nibble_pair<0>(x1), nibble_pair<1>(x0), nibble_pair<1>(x1),
-                                     bw[2 * h], times16(bw[2 * h]));
-                            mma_bf16(d, nibble_pair<2>(x0), nibble_pair<2>(x1), nibble_pair<3>(x0), nibble_pair<3>(x1),
-                                     bw[2 * h + 1], times16(bw[2 * h + 1]));
-                        }
-                    }
+                    if (BITS == 4) unit_mma<4, false>(d, wa[p][v], 0u, wb[p][v], 0u, bx);
+                    else unit_mma<8, false>(d, wa[p][2 * v], wa[p][2 * v + 1], wb[p][2 * v], wb[p][2 * v + 1], bx);
                 }
                 const float2 xs2 = *reinterpret_cast<const float2 *>(xsum + step * kTileTokens + 2 * c);
-                uint16_t q4[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    if (VEC) q4[i] = (uint16_t)((p < 2 ? qv[0][i].x : qv[0][i].y) >> (16 * (p & 1)));
-                    else q4[i] = qs[p][i];
-                }
-                const float s_a = bf16_bits_to_f32(q4[0]), s_b = bf16_bits_to_f32(q4[2]);
-                float m_a = bf16_bits_to_f32(q4[1]), m_b = bf16_bits_to_f32(q4[3]);
-                if (BITS == 4) m_a = fmaf(-16.f, s_a, m_a), m_b = fmaf(-16.f, s_b, m_b);  // the 16s of nibble_pair16
+                const float s_a = bf16_bits_to_f32(qs[p][0]), s_b = bf16_bits_to_f32(qs[p][2]);
+                const float m_a = bf16_bits_to_f32(qs[p][1]), m_b = bf16_bits_to_f32(qs[p][3]);
                 acc[0] = fmaf(s_a, d[0], fmaf(m_a, xs2.x, acc[0]));
                 acc[1] = fmaf(s_a, d[1], fmaf(m_a, xs2.y, acc[1]));
                 acc[2] = fmaf(s_b, d[2], fmaf(m_b, xs2.x, acc[2]));
                 acc[3] = fmaf(s_b, d[3], fmaf(m_b, xs2.y, acc[3]));
             }
             fetch(p, step + kPrefetch);  // refill the slot just consumed
-        }
-        if (VEC) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) qv[0][i] = qv[1][i];
         }
     }
 }
@@ -312,31 +314,15 @@ __device__ inline void rows_dot_fast(float (&acc)[4], const StreamArgs &a, int64
 #pragma unroll
         for (int v = 0; v < UNITS; ++v) {
             const uint4 bx = xu[(p * UNITS + v) * 32];
-            if (BITS == 4) {
-                const uint32_t x0 = wa[p][v], x1 = wb[p][v];
-                if (v == 0) mma_bf16_first(d, nibble_pair16<0>(x0), nibble_pair16<0>(x1), nibble_pair16<1>(x0), nibble_pair16<1>(x1), bx.x, bx.y);
-                else mma_bf16(d, nibble_pair16<0>(x0), nibble_pair16<0>(x1), nibble_pair16<1>(x0), nibble_pair16<1>(x1), bx.x, bx.y);
-                mma_bf16(d, nibble_pair16<2>(x0), nibble_pair16<2>(x1), nibble_pair16<3>(x0), nibble_pair16<3>(x1), bx.z, bx.w);
-            } else {
-                const uint32_t bw[4] = {bx.x, bx.y, bx.z, bx.w};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint32_t x0 = wa[p][2 * v + h], x1 = wb[p][2 * v + h];
-                    if (v == 0 && h == 0)
-                        mma_bf16_first(d, nibble_pair<0>(x0), nibble_pair<0>(x1), nibble_pair<1>(x0), nibble_pair<1>(x1), bw[0], times16(bw[0]));
-                    else
-                        mma_bf16(d, nibble_pair<0>(x0), nibble_pair<0>(x1), nibble_pair<1>(x0), nibble_pair<1>(x1), bw[2 * h], times16(bw[2 * h]));
-                    mma_bf16(d, nibble_pair<2>(x0), nibble_pair<2>(x1), nibble_pair<3>(x0), nibble_pair<3>(x1), bw[2 * h + 1],
-                             times16(bw[2 * h + 1]));
-                }
-            }
+            const int i0 = BITS == 4 ? v : 2 * v, i1 = BITS == 4 ? v : 2 * v + 1;
+            if (v == 0) unit_mma<BITS, true>(d, wa[p][i0], wa[p][i1], wb[p][i0], wb[p][i1], bx);
+            else unit_mma<BITS, false>(d, wa[p][i0], wa[p][i1], wb[p][i0], wb[p][i1], bx);
         }
         const float2 xs2 = *reinterpret_cast<const float2 *>(xq + p * kTileTokens);
         // BF16 bits -> FP32: the upper half of the word as it is, the lower half shifted up
         auto f32_of = [&](const uint2 &q) { const uint32_t w = p < 2 ? q.x : q.y; return __uint_as_float((p & 1) ? (w & 0xffff0000u) : (w << 16)); };
         const float s_a = f32_of(qv[0]), s_b = f32_of(qv[2]);
-        float m_a = f32_of(qv[1]), m_b = f32_of(qv[3]);
-        if (BITS == 4) m_a = fmaf(-16.f, s_a, m_a), m_b = fmaf(-16.f, s_b, m_b);  // the 16s of nibble_pair16
+        const float m_a = f32_of(qv[1]), m_b = f32_of(qv[3]);
         acc[0] = fmaf(s_a, d[0], fmaf(m_a, xs2.x, acc[0]));
         acc[1] = fmaf(s_a, d[1], fmaf(m_a, xs2.y, acc[1]));
         acc[2] = fmaf(s_b, d[2], fmaf(m_b, xs2.x, acc[2]));
@@ -374,7 +360,7 @@ __device__ inline void rows_dot(float (&acc)[4], const StreamArgs &a, int64_t ro
         const int64_t any = va ? rowa : vb ? rowb : 0;
         rows_dot_fast<BITS, G>(acc, a, va ? rowa : any, vb ? rowb : any, xs, xsum, lane);
     } else {
-        rows_dot_impl<BITS, G, false>(acc, a, rowa, rowb, va, vb, xs, xsum, lane);
+        rows_dot_impl<BITS, G>(acc, a, rowa, rowb, va, vb, xs, xsum, lane);
     }
 }
 
@@ -387,6 +373,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
     const size_t pass_bytes = (size_t)steps * geo::kUnits * 512 + (size_t)steps * kTileTokens * 4;
     __shared__ int64_t s_row[kTileTokens];  // activation row of each token of the tile, -1 = none
     __shared__ int64_t s_out[kTileTokens];  // output row (slot, or token for dense)
+    __shared__ uint32_t s_max[kPerTokenPasses][kTileTokens];  // largest magnitude of each token's activations (stage_tile)
     __shared__ int s_bucket, s_cnt;
     __shared__ int s_next;  // the next unit of the CTA's run that no warp has taken yet
 
@@ -440,10 +427,11 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 if (threadIdx.x < kTileTokens) {
                     const int k = p * kTileTokens + threadIdx.x;
                     s_row[threadIdx.x] = k < a.A ? m * a.A + k : -1;
+                    s_max[p][threadIdx.x] = 0u;
                 }
                 __syncthreads();
                 stage_tile<BITS, G>(a.x, K, s_row, reinterpret_cast<uint4 *>(smem + p * pass_bytes),
-                                    reinterpret_cast<float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512));
+                                    reinterpret_cast<float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512), s_max[p]);
             }
             __syncthreads();
             for (int64_t unit = lo + warp; unit < hi; unit += kWarps) {
@@ -460,8 +448,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                                       lane);
                     if (c == col / 2) {  // the lane of the quad that holds this slot's column
                         const float cf = a.coef[m * a.A + k];
-                        ta = fmaf(cf, col & 1 ? acc[1] : acc[0], ta);
-                        tb = fmaf(cf, col & 1 ? acc[3] : acc[2], tb);
+                        const int e = token_exponent(s_max[p][col]);
+                        ta = fmaf(cf, unscaled(col & 1 ? acc[1] : acc[0], e), ta);
+                        tb = fmaf(cf, unscaled(col & 1 ? acc[3] : acc[2], e), tb);
                     }
                 }
                 // the four lanes of a quad hold the partial sums of slots {0,1}, {2,3}, {4,5}, {6,7} (mod 8)
@@ -501,14 +490,14 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 if (n == 0) s_bucket = 0, s_cnt = (int)min((int64_t)kTileTokens, a.M - tile * kTileTokens);
                 if (m < a.M) row = orow = m;
             }
-            s_row[n] = row, s_out[n] = orow;
+            s_row[n] = row, s_out[n] = orow, s_max[0][n] = 0u;
         }
         __syncthreads();
         const int bucket = s_bucket, cnt = s_cnt;
         const bool valid = bucket < a.E;  // bucket E: slots with an id outside [0, E) - their outputs become NaN
         uint4 *xs = reinterpret_cast<uint4 *>(smem);
         float *xsum = reinterpret_cast<float *>(smem + (size_t)steps * geo::kUnits * 512);
-        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum);
+        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum, s_max[0]);
         if (threadIdx.x == 0) s_next = 0;
         __syncthreads();
 
@@ -540,15 +529,17 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 const int n = 2 * c + t;
                 if (n >= cnt) continue;
                 const int64_t orow = s_out[n];
+                const int e = token_exponent(s_max[0][n]);
+                const float dot_a = unscaled(acc[t], e), dot_b = unscaled(acc[2 + t], e);
                 if (MODE == kSwiglu) {
                     if (!va) continue;
                     // kernels/linear_q4.hip:272-274: g, u as stored, h = stored(stored(silu(g)) * u)
-                    const float gg = as_stored_bf16(acc[t]), uu = as_stored_bf16(acc[2 + t]);
+                    const float gg = as_stored_bf16(dot_a), uu = as_stored_bf16(dot_b);
                     const float hv = as_stored_bf16(silu_f32(gg)) * uu;
                     store_out(out, orow * I + ra, valid ? hv : qnan_f32());
                 } else {
-                    if (va) store_out(out, orow * a.N + ra, valid ? acc[t] : qnan_f32());
-                    if (vb) store_out(out, orow * a.N + rb, valid ? acc[2 + t] : qnan_f32());
+                    if (va) store_out(out, orow * a.N + ra, valid ? dot_a : qnan_f32());
+                    if (vb) store_out(out, orow * a.N + rb, valid ? dot_b : qnan_f32());
                 }
             }
         }

@@ -68,6 +68,34 @@ def test_linear_dense(cuda, oracle, bits, G, M, N, Kd):
     assert_bf16_close(bits_of(ybf), refbf, oracle, "linear bf16")
 
 
+@pytest.mark.parametrize("bits,G,Kd", [(4, 128, 4096), (4, 128, 128), (4, 32, 160), (8, 64, 1024), (8, 128, 384)])
+def test_linear_activation_range(cuda, oracle, bits, G, Kd):
+    """The streaming kernel holds activations as F16 times a power of two a token: tokens of every magnitude that BF16 has,
+    values far below a token's largest, zeros and subnormals.  Bound: FP32 sums of the K / 16 products' blocks and the K / G
+    groups, in absolute values, whose roundings (2^-23 each, truncating adds) bound any order's error; infinities and NaN reach
+    every output of their token and of no other."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(Kd + bits)
+    mags = [0, 2.0 ** -133, 2.0 ** -126, 2.0 ** -60, 1.0, 2.0 ** 16, 2.0 ** 60, 2.0 ** 100, 0, 1.0, 1.0, 1.0]
+    x = rng.standard_normal((len(mags), Kd)) * np.array(mags)[:, None]
+    x[8, 5] = 1.5                                            # one value alone
+    x[9] *= 2.0 ** rng.integers(-40, 41, Kd)                 # eighty binades inside one token
+    xb = oracle.f32_to_bf16(x.astype(np.float32))
+    xb[10, 3], xb[11, Kd - 1] = 0x7F80, 0x7FC0               # +inf, NaN
+    w = oracle.quantize(random_weights(rng, 48, Kd), G, bits)
+    y = torch.empty((len(mags), 48), dtype=torch.float32, device=cuda)
+    K.linear_qw(bf16_tensor(xb, cuda), upload(w, cuda), y, len(mags), K.Act.BF16, out_act=K.Act.F32)
+    torch.cuda.synchronize()
+    got = y.cpu().numpy().astype(np.float64)
+    assert not np.isfinite(got[10:]).any()
+    xf = oracle.bf16_to_f32(xb[:10]).astype(np.float64)
+    s, m = (np.repeat(oracle.bf16_to_f32(v).astype(np.float64).reshape(48, Kd // G), G, axis=1) for v in (w.scale, w.minv))
+    codes = oracle.codes_of(w).astype(np.float64)
+    want = xf @ (codes * s + m).T
+    bound = (Kd / 8 + 3 * Kd / G + 4) * 2.0 ** -23 * (np.abs(xf) @ (codes * np.abs(s) + np.abs(m)).T) + 2.0 ** -149
+    assert np.all(np.abs(got[:10] - want) <= bound), np.max(np.abs(got[:10] - want) / bound, axis=1)
+
+
 @pytest.mark.parametrize("rows,I", [(1, 8), (5, 1000), (160, 1024), (3, 7)])
 def test_swiglu(cuda, oracle, rows, I):
     from strixite_b200 import kernels as K
