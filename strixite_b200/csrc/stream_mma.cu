@@ -143,76 +143,100 @@ struct StreamArgs {
     const float *coef;   // kPerToken
     void *out;
     uint32_t *err;
+    int chunks, split;   // see chunk_count: chunks of a contraction; warps that share a unit (1 .. chunks)
 };
+
+// Dense projections: a row's contraction is summed in `chunks` chunks of whole blocks, and the chunks' sums are added as a
+// binary tree over their order.  Warps that share a unit take a power of two of neighbouring chunks each, i.e. a node of that tree, so a result does
+// not depend on how many share it - which follows from the launch's size, and a row must not notice the rest of its batch.
+// The routed forms have units enough from the first tokens on, and the chunks would cost them 6 % (150 tokens x 10 experts,
+// 4096 x 2048 Q4: 415 -> 441 us).
+constexpr int kMaxChunks = 8, kTreeLevels = 3;
+inline int chunk_count(int64_t blocks) {
+    int n = kMaxChunks;
+    while (n > 1 && (blocks % n != 0 || blocks / n < 2)) n /= 2;
+    return n;
+}
+// Node number i joins the tree: v becomes its sum with the left-hand nodes that were waiting for it in this thread's slots, a
+// level of them kBigThreads apart.  Returns the slot where it would wait itself (past the last one when the tree is complete).
+__device__ inline float4 *tree_join(float4 *level, int i, float (&v)[4]) {
+    for (; i & 1; i >>= 1, level += kBigThreads) {
+        const float4 l = *level;
+        v[0] = l.x + v[0], v[1] = l.y + v[1], v[2] = l.z + v[2], v[3] = l.w + v[3];
+    }
+    return level;
+}
+__device__ inline void tree_push(float4 *level, int i, float (&v)[4]) {
+    level = tree_join(level, i, v);
+    *level = make_float4(v[0], v[1], v[2], v[3]);
+}
 
 template <typename T> __device__ inline void store_out(T *p, int64_t i, float v) { store_from_f32(p, i, v); }
 
-// Stages up to 8 activation rows (rows[n] < 0 = none, zeros) as F16 in fragment order at xs, every row times its power of two
+// Stages up to 8 activation rows (rows[n] < 0 = none) as F16 in fragment order at xs, every row times its power of two
 // 2^e (token_exponent; max_bits[n] comes in as zero and leaves as the row's largest magnitude), and at xsum the sums of every
 // (step, token) times 2^(e - 9), the factor that the dots with the codes carry.  All threads of the CTA.
 template <int BITS, int G>
 __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, uint32_t *max_bits) {
     using geo = Geo<BITS, G>;
     constexpr int UNITS = geo::kUnits, KI = geo::kStepCodes, CPL = geo::kCodesPerLane;
-    const int units_per_row = K / 8, steps = K / KI;
-    // sum(x) of every (step, token), in a fixed order, and the largest magnitude of every token.  blockDim is a multiple of
-    // eight, so a thread meets one token only.
+    constexpr int kStepLanes = KI / 8;  // lanes that hold one step of one token: 4, 8 or 16
+    constexpr int kBatch = 8;           // 16-byte loads a lane has in flight
+    // A token is staged by every eighth warp, so that what belongs to the token is the same for a whole warp (dealing 16-byte
+    // units out over the CTA cost two divisions a unit and an atomic a step: 150 tokens x 10 experts, 4096 x 2048 Q4, 415 ->
+    // 442 us).  Eight loads in flight: under a streaming kernel's load an L2 round trip is thousands of cycles.
+    const int lane = threadIdx.x & 31, n = (threadIdx.x >> 5) & (kTileTokens - 1), share = threadIdx.x >> 8, stride = (int)blockDim.x / kTileTokens;
+    const int units = K / 8;
+    const int64_t row = rows[n];
+    const uint4 *src = reinterpret_cast<const uint4 *>(x + row * K);
+    uint4 v[kBatch];
+    auto load = [&](int base) {
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+            if (base + j * stride < units) v[j] = src[base + j * stride];
+    };
     uint32_t top = 0u;
-    for (int idx = threadIdx.x; idx < steps * kTileTokens; idx += blockDim.x) {
-        const int step = idx / kTileTokens, n = idx % kTileTokens;
-        const int64_t row = rows[n];
-        float sum = 0.f;
-        if (row >= 0) {
-            // the loads of a batch are independent of one another: under a streaming kernel's load an L2 round trip is
-            // thousands of cycles, and one load at a time made staging a tenth of a decode kernel's time
-            const uint4 *p = reinterpret_cast<const uint4 *>(x + row * K + (int64_t)step * KI);
-            constexpr int kBatch = KI / 8 < 8 ? KI / 8 : 8;
-            for (int i0 = 0; i0 < KI / 8; i0 += kBatch) {
-                uint4 u[kBatch];
+    if (row >= 0) {
+        // sum(x) of every step: eight values a lane, then a butterfly over the step's lanes
+        for (int base = share * 32 + lane; base - lane < units; base += kBatch * stride) {
+            load(base);
 #pragma unroll
-                for (int i = 0; i < kBatch; ++i) u[i] = p[i0 + i];
+            for (int j = 0; j < kBatch; ++j) {
+                const int u = base + j * stride;
+                if (u - lane >= units) break;
+                float sum = 0.f;
+                if (u < units) {
+                    const uint32_t w4[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
-                for (int i = 0; i < kBatch; ++i) {
-                    const uint32_t w4[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        sum += __uint_as_float(w4[j] << 16), sum += __uint_as_float(w4[j] & 0xffff0000u);
-                        top = __vmaxu2(top, w4[j] & 0x7fff7fffu);
+                    for (int i = 0; i < 4; ++i) {
+                        sum += __uint_as_float(w4[i] << 16), sum += __uint_as_float(w4[i] & 0xffff0000u);
+                        top = __vmaxu2(top, w4[i] & 0x7fff7fffu);
                     }
                 }
+#pragma unroll
+                for (int o = kStepLanes / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (lane % kStepLanes == 0 && u < units) xsum[u / kStepLanes * kTileTokens + n] = sum;
             }
         }
-        xsum[idx] = sum;
+        top = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xffffu));
+        if (lane == 0) atomicMax(&max_bits[n], top);
     }
-    top = max(top >> 16, top & 0xffffu);
-    top = max(top, __shfl_xor_sync(0xffffffffu, top, 8));
-    top = max(top, __shfl_xor_sync(0xffffffffu, top, 16));
-    if ((threadIdx.x & 31) < kTileTokens) atomicMax(&max_bits[threadIdx.x & 7], top);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < steps * kTileTokens; idx += blockDim.x)  // each thread the sums it wrote
-        xsum[idx] = xsum[idx] * pow2f(token_exponent(max_bits[idx % kTileTokens])) * 0x1p-9f;
-    // 8 consecutive k of token n (16 bytes) -> one unit, permuted to match the pairs of codes.  Four loads a thread are issued
-    // before the first is used (see the note on batches above).
-    const int n_units = kTileTokens * units_per_row, stride = (int)blockDim.x;
-    for (int base = threadIdx.x; base < n_units; base += 4 * stride) {
-        uint4 src[4];
+    // absent tokens' columns keep whatever the memory held: a column of the products depends on its own token only, and theirs
+    // are dropped
+    if (row < 0) return;
+    const float f = pow2f(token_exponent(max_bits[n]));
+    // One batch holds the row up to 4096 k at 512 threads; a longer one is read again.
+    const bool held = units <= kBatch * stride;
+    for (int base = share * 32 + lane; base < units; base += kBatch * stride) {
+        if (!held) load(base);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int idx = base + j * stride;
-            src[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (idx < n_units) {
-                const int64_t row = rows[idx / units_per_row];
-                if (row >= 0) src[j] = *reinterpret_cast<const uint4 *>(x + row * K + (idx % units_per_row) * 8);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int idx = base + j * stride;
-            if (idx >= n_units) break;
-            const int n = idx / units_per_row, k = (idx % units_per_row) * 8;
-            const int step = k / KI, rem = k % KI, cc = rem / CPL, v = (rem % CPL) / 8;
-            const float f = pow2f(token_exponent(max_bits[n]));
-            const uint32_t w4[4] = {src[j].x, src[j].y, src[j].z, src[j].w};
+        for (int j = 0; j < kBatch; ++j) {
+            const int u = base + j * stride, k = u * 8;
+            if (u >= units) break;
+            if (u % kStepLanes == 0) xsum[u / kStepLanes * kTileTokens + n] *= f * 0x1p-9f;
+            const int step = k / KI, rem = k % KI, cc = rem / CPL, part = (rem % CPL) / 8;
+            const uint32_t w4[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
             float lo[4], hi[4];  // elements 2 i and 2 i + 1
 #pragma unroll
             for (int i = 0; i < 4; ++i) lo[i] = __uint_as_float(w4[i] << 16) * f, hi[i] = __uint_as_float(w4[i] & 0xffff0000u) * f;
@@ -223,7 +247,7 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             } else {  // natural order
                 dst.x = pack(lo[0], hi[0]), dst.y = pack(lo[1], hi[1]), dst.z = pack(lo[2], hi[2]), dst.w = pack(lo[3], hi[3]);
             }
-            xs[(step * UNITS + v) * 32 + n * 4 + cc] = dst;
+            xs[(step * UNITS + part) * 32 + n * 4 + cc] = dst;
         }
     }
 }
@@ -287,20 +311,21 @@ __device__ inline void rows_dot_impl(float (&acc)[4], const StreamArgs &a, int64
 // the end of the expert is replaced by a row that exists; its sums are dropped by the caller), pointers advance by
 // increments, the last block is peeled so nothing is fetched past the end of a row, and a step's first MMA takes a
 // zero accumulator operand instead of cleared registers.
-template <int BITS, int G>
+// TREE: the contraction in chunks (chunk_count), this warp's part of it only; otherwise one running sum.
+template <int BITS, int G, bool TREE>
 __device__ inline void rows_dot_fast(float (&acc)[4], const StreamArgs &a, int64_t rowa, int64_t rowb, const uint4 *xs,
-                                     const float *xsum, int lane) {
+                                     const float *xsum, int lane, int part, float4 *tree) {
     using geo = Geo<BITS, G>;
     constexpr int W = geo::kWords, UNITS = geo::kUnits, KI = geo::kStepCodes;
     constexpr int kBlockBytes = kPrefetch * 4 * geo::kLoadBytes;  // bytes of one row consumed per block of four steps
-    const int K = (int)a.K, blocks = K / (KI * kPrefetch), groups = K / G, c = lane & 3;
-    const int64_t row_bytes = BITS == 4 ? a.K / 2 : a.K;
-    const uint8_t *pa = a.q + rowa * row_bytes + c * geo::kLoadBytes;
-    const uint8_t *pb = a.q + rowb * row_bytes + c * geo::kLoadBytes;
-    const uint2 *sa = reinterpret_cast<const uint2 *>(a.scale + rowa * groups), *ma = reinterpret_cast<const uint2 *>(a.minv + rowa * groups);
-    const uint2 *sb = reinterpret_cast<const uint2 *>(a.scale + rowb * groups), *mb = reinterpret_cast<const uint2 *>(a.minv + rowb * groups);
-    const uint4 *xu = xs + lane;
-    const float *xq = xsum + 2 * c;
+    const int K = (int)a.K, blocks = K / (KI * kPrefetch) / (TREE ? a.split : 1), groups = K / G, c = lane & 3;
+    const int first = TREE ? part * blocks : 0, per_chunk = TREE ? K / (KI * kPrefetch) / a.chunks : 0;
+    const int64_t row_bytes = BITS == 4 ? a.K / 2 : a.K, at = first * kBlockBytes + c * geo::kLoadBytes;
+    const uint8_t *pa = a.q + rowa * row_bytes + at, *pb = a.q + rowb * row_bytes + at;
+    const uint2 *sa = reinterpret_cast<const uint2 *>(a.scale + rowa * groups) + first, *ma = reinterpret_cast<const uint2 *>(a.minv + rowa * groups) + first;
+    const uint2 *sb = reinterpret_cast<const uint2 *>(a.scale + rowb * groups) + first, *mb = reinterpret_cast<const uint2 *>(a.minv + rowb * groups) + first;
+    const uint4 *xu = xs + lane + first * (kPrefetch * UNITS * 32);
+    const float *xq = xsum + 2 * c + first * (kPrefetch * kTileTokens);
 
     uint32_t wa[kPrefetch][W], wb[kPrefetch][W];
     uint2 qv[4], qn[4];  // {scale a, min a, scale b, min b} of the block in use / of the next one
@@ -332,6 +357,7 @@ __device__ inline void rows_dot_fast(float (&acc)[4], const StreamArgs &a, int64
     fetch_scales(qv);
 #pragma unroll
     for (int p = 0; p < kPrefetch; ++p) fetch_codes(p);
+    int chunk = 0, left = per_chunk;
     for (int b = 1; b < blocks; ++b) {  // consume block b - 1, fetching block b into the registers it frees
         pa += kBlockBytes, pb += kBlockBytes, ++sa, ++ma, ++sb, ++mb;
         fetch_scales(qn);
@@ -343,22 +369,30 @@ __device__ inline void rows_dot_fast(float (&acc)[4], const StreamArgs &a, int64
 #pragma unroll
         for (int i = 0; i < 4; ++i) qv[i] = qn[i];
         xu += kPrefetch * UNITS * 32, xq += kPrefetch * kTileTokens;
+        if (TREE && --left == 0) {
+            tree_push(tree, chunk++, acc);
+            acc[0] = acc[1] = acc[2] = acc[3] = 0.f, left = per_chunk;
+        }
     }
 #pragma unroll
     for (int p = 0; p < kPrefetch; ++p) consume(p);
+    if (TREE && chunk > 0) tree_join(tree, chunk, acc);
 }
 
-template <int BITS, int G>
+// Whether a row's scales and mins are whole aligned 8-byte loads of four groups.
+__host__ __device__ inline bool vector_scales(const StreamArgs &a, int G) {
+    return (a.K / G) % 4 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 7) == 0;
+}
+
+// The dots of this warp's part of the contraction (part 0 of 1: all of it).  tree: the thread's slots, kBigThreads apart.
+template <int BITS, int G, bool TREE>
 __device__ inline void rows_dot(float (&acc)[4], const StreamArgs &a, int64_t rowa, int64_t rowb, bool va, bool vb,
-                                const uint4 *xs, const float *xsum, int lane) {
+                                const uint4 *xs, const float *xsum, int lane, int part, float4 *tree) {
     using geo = Geo<BITS, G>;
-    const int groups = (int)(a.K / G);
-    const bool vec = geo::kStepsPerGroup == 1 && groups % 4 == 0 &&
-                     ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 7) == 0;
-    if (vec && geo::kStepsPerGroup == 1) {
+    if (geo::kStepsPerGroup == 1 && vector_scales(a, G)) {
         // rows past the end of the expert: stream a row that exists instead (the caller drops their sums)
         const int64_t any = va ? rowa : vb ? rowb : 0;
-        rows_dot_fast<BITS, G>(acc, a, va ? rowa : any, vb ? rowb : any, xs, xsum, lane);
+        rows_dot_fast<BITS, G, TREE>(acc, a, va ? rowa : any, vb ? rowb : any, xs, xsum, lane, part, tree);
     } else {
         rows_dot_impl<BITS, G>(acc, a, rowa, rowb, va, vb, xs, xsum, lane);
     }
@@ -376,6 +410,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
     __shared__ uint32_t s_max[kPerTokenPasses][kTileTokens];  // largest magnitude of each token's activations (stage_tile)
     __shared__ int s_bucket, s_cnt;
     __shared__ int s_next;  // the next unit of the CTA's run that no warp has taken yet
+    constexpr bool kTree = SRC == kDense;
+    __shared__ float4 s_tree[kTree ? kTreeLevels * kBigThreads : 1];  // tree_push; its last level also hands parts' sums over
+    const int split = kTree ? a.split : 1;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const int64_t I = a.N / 2;
@@ -392,7 +429,8 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
     // idle; inside a run the warps take units on demand either way.
     const int64_t nb = gridDim.x;
     int64_t cpt = max((int64_t)1, nb / max(n_tiles, (int64_t)1));
-    const int64_t chunk = ((units_per_tile + cpt - 1) / cpt + kWarps - 1) / kWarps * kWarps;
+    const int n_groups = kWarps / split;  // a group of `split` warps takes a unit at a time
+    const int64_t chunk = ((units_per_tile + cpt - 1) / cpt + n_groups - 1) / n_groups * n_groups;
     cpt = (units_per_tile + chunk - 1) / chunk;
     const int64_t n_chunks = n_tiles * cpt;
     const bool aligned = ((n_chunks + nb - 1) / nb) * chunk * 100 <= ((total + nb - 1) / nb) * 115;
@@ -443,9 +481,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                     const int p = k / kTileTokens, col = k % kTileTokens;
                     const int64_t base = (int64_t)a.ids[m * a.A + k] * a.N;
                     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                    rows_dot<BITS, G>(acc, a, base + ra, base + rb, va, vb, reinterpret_cast<const uint4 *>(smem + p * pass_bytes),
+                    rows_dot<BITS, G, false>(acc, a, base + ra, base + rb, va, vb, reinterpret_cast<const uint4 *>(smem + p * pass_bytes),
                                       reinterpret_cast<const float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512),
-                                      lane);
+                                      lane, 0, nullptr);
                     if (c == col / 2) {  // the lane of the quad that holds this slot's column
                         const float cf = a.coef[m * a.A + k];
                         const int e = token_exponent(s_max[p][col]);
@@ -497,23 +535,10 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
         const bool valid = bucket < a.E;  // bucket E: slots with an id outside [0, E) - their outputs become NaN
         uint4 *xs = reinterpret_cast<uint4 *>(smem);
         float *xsum = reinterpret_cast<float *>(smem + (size_t)steps * geo::kUnits * 512);
-        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum, s_max[0]);
-        if (threadIdx.x == 0) s_next = 0;
-        __syncthreads();
-
-        // Warps take units on demand: two warps of an SM do not stream at the same rate (measured: the units of one of two
-        // co-resident CTAs took 2.5 times as long as the other's while both were alive), and a fixed deal leaves the fast ones
-        // idle at the end.  A unit's result does not depend on which warp computes it.
-        for (;;) {
-            int taken = 0;
-            if (lane == 0) taken = atomicAdd(&s_next, 1);
-            taken = __shfl_sync(0xffffffffu, taken, 0);
-            const int64_t unit = lo + taken;
-            if (unit >= hi) break;
+        const int part = warp & (split - 1), group = warp / split;
+        // The two weight rows of a unit that this lane streams, as rows inside the expert.
+        auto rows_of = [&](int64_t unit, int64_t &ra, int64_t &rb, bool &va, bool &vb) {
             const int64_t u = unit - tile * units_per_tile;
-            // The two weight rows this lane streams, as rows inside the expert, and where their results go.
-            int64_t ra, rb;
-            bool va, vb;
             if (MODE == kSwiglu) {
                 ra = u * 8 + g, rb = I + u * 8 + g;
                 va = vb = u * 8 + g < I;
@@ -521,8 +546,58 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 ra = u * 16 + g, rb = ra + 8;
                 va = ra < a.N, vb = rb < a.N;
             }
+        };
+        if (kTree && valid && lo + group < hi) {
+            // The codes of the warp's first unit are asked for, into L2, before the staging below goes to memory itself.
+            int64_t ra, rb;
+            bool va, vb;
+            rows_of(lo + group, ra, rb, va, vb);
+            const int64_t row_bytes = BITS == 4 ? a.K / 2 : a.K;
+            const uint8_t *base = a.q + (int64_t)bucket * a.N * row_bytes;
+            for (int64_t at = row_bytes * part / split + c * 128; at < row_bytes * (part + 1) / split; at += 512) {
+                if (va) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + ra * row_bytes + at));
+                if (vb) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + rb * row_bytes + at));
+            }
+        }
+        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum, s_max[0]);
+        if (threadIdx.x == 0) s_next = 0;
+        __syncthreads();
+
+        // split == 1: warps take units on demand.  Two warps of an SM do not stream at the same rate (measured: the units of one
+        // of two co-resident CTAs took 2.5 times as long as the other's while both were alive), and a fixed deal leaves the
+        // fast ones idle at the end.  A unit's result does not depend on which warp computes it.
+        // split > 1 (few units): `split` warps share a unit, each a run of its contraction's chunks, and the first adds the parts.
+        int round = 0;
+        auto next_unit = [&]() -> int64_t {
+            if (kTree && split > 1) return lo + group + (int64_t)round * n_groups;
+            int taken = 0;
+            if (lane == 0) taken = atomicAdd(&s_next, 1);
+            return lo + __shfl_sync(0xffffffffu, taken, 0);
+        };
+        auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(32 * split) : "memory"); };
+        for (int64_t unit; (unit = next_unit()) < hi; ++round) {
+            int64_t ra, rb;
+            bool va, vb;
+            rows_of(unit, ra, rb, va, vb);
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            if (valid) rows_dot<BITS, G>(acc, a, (int64_t)bucket * a.N + ra, (int64_t)bucket * a.N + rb, va, vb, xs, xsum, lane);
+            if (valid) rows_dot<BITS, G, kTree>(acc, a, (int64_t)bucket * a.N + ra, (int64_t)bucket * a.N + rb, va, vb, xs, xsum, lane, part, s_tree + threadIdx.x);
+            if (kTree && split > 1) {
+                // a warp that shares a unit has at most half its chunks, so the last level of its own tree is free for this
+                float4 *parts = s_tree + (kTreeLevels - 1) * kBigThreads + threadIdx.x;
+                if (part != 0) *parts = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                group_sync();
+                if (part == 0) {
+                    tree_push(s_tree + threadIdx.x, 0, acc);
+                    for (int p = 1; p < split; ++p) {
+                        const float4 v = parts[32 * p];
+                        acc[0] = v.x, acc[1] = v.y, acc[2] = v.z, acc[3] = v.w;
+                        if (p + 1 < split) tree_push(s_tree + threadIdx.x, p, acc);
+                        else tree_join(s_tree + threadIdx.x, p, acc);
+                    }
+                }
+                group_sync();
+                if (part != 0) continue;
+            }
             // Epilogue.  Lane (g, c) holds rows ra / rb for tokens 2c and 2c + 1.
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
@@ -660,14 +735,26 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     auto kern = stream_kernel<BITS, G, MODE, SRC, TOUT>;
     SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn,
              ": reserving shared memory");
+    // A dense projection of few units for the machine's warps: up to eight warps share one, as long as that gives a warp at most two and a half
+    // parts in turn.  A warp alone walks K / (4 * kStepCodes) blocks one after another, each a round trip to memory (2048 x 4096
+    // Q8, one token: 39 us with 128 warps at work).
+    const int64_t machine_warps = (int64_t)sm_count() * (kBigThreads / 32);
+    StreamArgs args = a;
+    args.chunks = SRC == kDense && geo::kStepsPerGroup == 1 && vector_scales(a, G) ? chunk_count(steps / kPrefetch) : 1, args.split = 1;
+    if (SRC == kDense)
+        while (args.split * 2 <= args.chunks && est_units * args.split * 4 <= machine_warps * 5) args.split *= 2;
+    if (args.split > 1) {
+        kern<<<(unsigned)std::min<int64_t>(sm_count(), est_units), kBigThreads, smem, st>>>(args);
+        return SXB_OK;
+    }
     // One CTA of sixteen warps an SM when there are several units for every warp of the machine; otherwise CTAs of eight
     // warps, two an SM where their shared memory allows, and never more CTAs than one per unit and warp.
-    const bool big = est_units >= (int64_t)sm_count() * (kBigThreads / 32) * 2;
+    const bool big = est_units >= machine_warps * 2;
     const int threads = big ? kBigThreads : kThreads, warps = threads / 32;
     const int per_sm = big || smem > 100 * 1024 ? 1 : 2;
     int64_t grid = (int64_t)sm_count() * per_sm;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (est_units + warps - 1) / warps));
-    kern<<<(unsigned)grid, threads, smem, st>>>(a);
+    kern<<<(unsigned)grid, threads, smem, st>>>(args);
     return SXB_OK;
 }
 

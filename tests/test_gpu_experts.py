@@ -96,6 +96,26 @@ def test_linear_activation_range(cuda, oracle, bits, G, Kd):
     assert np.all(np.abs(got[:10] - want) <= bound), np.max(np.abs(got[:10] - want) / bound, axis=1)
 
 
+@pytest.mark.parametrize("bits,G,Kd", [(4, 128, 1024), (4, 128, 2048), (8, 64, 2048), (8, 64, 640)])
+def test_linear_row_does_not_depend_on_launch(cuda, oracle, bits, G, Kd):
+    """One warp a unit of 16 rows, or two, four or eight, by the launch's size: a token's row is the same, bit for bit, alone, in
+    launches around each of those limits, and in one that keeps every warp of the machine busy."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(Kd)
+    w = upload(oracle.quantize(random_weights(rng, 4808, Kd), G, bits), cuda)
+    x = torch.randn((136, Kd), device=cuda).to(torch.bfloat16)
+    x[0] *= 3.0
+    rows = []
+    for N, M in [(24, 1), (4808, 1), (4808, 3), (4808, 16), (4808, 17), (4808, 72), (4808, 80), (4808, 136)]:
+        y = torch.full((M, N), float("nan"), dtype=torch.float32, device=cuda)
+        K.linear_qw(x, w.rows(0, N), y, M, K.Act.BF16, out_act=K.Act.F32)
+        torch.cuda.synchronize()
+        assert torch.isfinite(y).all()
+        rows.append(y)
+    for y in rows:
+        assert torch.equal(y[0, :24], rows[0][0]) and torch.equal(y, rows[-1][:y.shape[0], :y.shape[1]])
+
+
 @pytest.mark.parametrize("rows,I", [(1, 8), (5, 1000), (160, 1024), (3, 7)])
 def test_swiglu(cuda, oracle, rows, I):
     from strixite_b200 import kernels as K
