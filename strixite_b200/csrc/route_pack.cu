@@ -20,132 +20,182 @@ namespace {
 
 constexpr int kPackThreads = 1024;
 constexpr int kSmallSlots = 2048;
-constexpr int kSegWarps = 8;  // warps (segments) per CTA in the histogram / scatter launches
+constexpr int kSegWarps = 4;  // warps (segments) per CTA in the histogram / scatter launches
 
 __device__ inline int bucket_of(int32_t id, int e_lo, int E_local) {
     const int b = id - e_lo;
     return (b < 0 || b >= E_local) ? E_local : b;
 }
 
-// Exclusive scan of v over the CTA's kPackThreads threads; *total = the sum.  buf: 33 ints of shared memory.
-__device__ inline int cta_exclusive_scan(int v, int *buf, int *total) {
+// Exclusive scan of v over the CTA's kPackThreads threads; *total = the sum.  buf: 33 words of shared memory.
+__device__ inline uint64_t cta_exclusive_scan(uint64_t v, uint64_t *buf, uint64_t *total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
+    uint64_t incl = v;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, off);
+        const uint64_t t = __shfl_up_sync(0xffffffffu, incl, off);
         if (lane >= off) incl += t;
     }
     if (lane == 31) buf[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        int w = buf[lane], wi = w;
+        const uint64_t w = buf[lane];
+        uint64_t wi = w;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, wi, off);
+            const uint64_t t = __shfl_up_sync(0xffffffffu, wi, off);
             if (lane >= off) wi += t;
         }
         buf[lane] = wi - w;
         if (lane == 31) buf[32] = wi;
     }
     __syncthreads();
-    const int excl = incl - v + buf[warp];
     *total = buf[32];
-    __syncthreads();
-    return excl;
+    return incl - v + buf[warp];
 }
 
-// Writes offsets, the header and the four tile lists from per-bucket counts (thread b owns bucket b).
-// tile_first: 4 * 1025 ints of shared memory.
-__device__ void emit_layout(int count, const RouteWords &L, int32_t *ws, int *scanbuf, int *tile_first, bool ep) {
+// Where every bucket's slots and tiles begin.  first[i]: the bucket's first tile in list i; entry E + 1 = the total.
+constexpr int kTileLists = 4;
+__device__ constexpr int kTileRows[kTileLists] = {8, 128, kTcTileA, kTcTileB};
+struct Layout {
+    int start[kMoeMaxExperts + 1];
+    int first[kTileLists][kMoeMaxExperts + 2];
+    uint64_t scan[2][33];
+};
+
+// Per-bucket counts (thread b owns bucket b) -> sm, and offsets and header of the workspace.  Ends with a barrier.
+// Two scans for all five sums, a sum in 21 bits (at most 2^20 slots): slots, 8-slot and 128-slot tiles; the other two lists.
+__device__ void scan_layout(int count, const RouteWords &L, int32_t *ws, Layout &sm, bool ep) {
     const int b = threadIdx.x, E = (int)L.E;
-    const bool owner = b <= E;
     // Tiles are cut for buckets 0..E-1, and for the overflow bucket E only outside expert-parallel mode (there its
     // slots are invalid ids whose outputs must become NaN; in EP mode they belong to other ranks and are skipped).
-    const bool tiled = owner && (b < E || !ep);
-    int total_slots, n8, n128, nta, ntb;
-    const int start = cta_exclusive_scan(owner ? count : 0, scanbuf, &total_slots);
-    const int t8 = tiled ? (count + 7) / 8 : 0, t128 = tiled ? (count + 127) / 128 : 0;
-    const int first8 = cta_exclusive_scan(t8, scanbuf, &n8);
-    const int first128 = cta_exclusive_scan(t128, scanbuf, &n128);
-    const int firstta = cta_exclusive_scan(tiled ? (count + kTcTileA - 1) / kTcTileA : 0, scanbuf, &nta);
-    const int firsttb = cta_exclusive_scan(tiled ? (count + kTcTileB - 1) / kTcTileB : 0, scanbuf, &ntb);
-    int32_t *offsets = ws + L.offsets;
-    if (owner) offsets[b] = start;
-    if (b <= E + 1) {  // first tile of each bucket; entry E + 1 = the total
-        tile_first[b] = b <= E ? first8 : n8;
-        tile_first[1025 + b] = b <= E ? first128 : n128;
-        tile_first[2050 + b] = b <= E ? firstta : nta;
-        tile_first[3075 + b] = b <= E ? firsttb : ntb;
+    const bool tiled = b < E || (b == E && !ep);
+    if (b > E) count = 0;
+    auto tiles = [&](int rows) { return (uint64_t)(tiled ? (count + rows - 1) / rows : 0); };
+    uint64_t total0, total1;
+    const uint64_t sum0 = cta_exclusive_scan((uint64_t)count | (tiles(8) << 21) | (tiles(128) << 42), sm.scan[0], &total0);
+    const uint64_t sum1 = cta_exclusive_scan(tiles(kTcTileA) | (tiles(kTcTileB) << 21), sm.scan[1], &total1);
+    const int mask = (1 << 21) - 1;
+    auto store = [&](int at, uint64_t s0, uint64_t s1) {
+        sm.first[0][at] = (int)(s0 >> 21) & mask, sm.first[1][at] = (int)(s0 >> 42);
+        sm.first[2][at] = (int)s1 & mask, sm.first[3][at] = (int)(s1 >> 21) & mask;
+    };
+    if (b <= E) {
+        sm.start[b] = (int)sum0 & mask;
+        ws[L.offsets + b] = (int)sum0 & mask;
+        store(b, sum0, sum1);
     }
     if (b == 0) {
-        offsets[E + 1] = total_slots;
-        ws[0] = n8, ws[1] = (int32_t)L.S, ws[2] = E, ws[3] = n128, ws[4] = ep ? 1 : 0, ws[5] = 0, ws[6] = 0, ws[7] = 0;
-        ws[L.tta_n] = nta, ws[L.ttb_n] = ntb;
+        store(E + 1, total0, total1);
+        ws[L.offsets + E + 1] = (int)total0 & mask;
+        ws[0] = (int)(total0 >> 21) & mask, ws[1] = (int32_t)L.S, ws[2] = E, ws[3] = (int)(total0 >> 42), ws[4] = ep ? 1 : 0;
+        ws[5] = 0, ws[6] = 0, ws[7] = 0;
+        ws[L.tta_n] = (int)total1 & mask, ws[L.ttb_n] = (int)(total1 >> 21) & mask;
     }
     __syncthreads();
-    // Tiles in parallel: tile t belongs to the last bucket whose first tile is <= t.
-    for (int pass = 0; pass < 4; ++pass) {
-        const int *first = tile_first + pass * 1025;
-        const int n = pass == 0 ? n8 : pass == 1 ? n128 : pass == 2 ? nta : ntb;
-        const int rows = pass == 0 ? 8 : pass == 1 ? 128 : pass == 2 ? kTcTileA : kTcTileB;
-        int32_t *tb = ws + (pass == 0 ? L.t8_bucket : pass == 1 ? L.t128_bucket : pass == 2 ? L.tta_bucket : L.ttb_bucket);
-        int32_t *ts = ws + (pass == 0 ? L.t8_start : pass == 1 ? L.t128_start : pass == 2 ? L.tta_start : L.ttb_start);
-        for (int t = threadIdx.x; t < n; t += kPackThreads) {
+}
+
+// Tiles t0, t0 + stride, ... of every list: a tile belongs to the last bucket whose first tile is not past it (empty buckets
+// never win).
+__device__ void emit_tiles(const RouteWords &L, int32_t *ws, const Layout &sm, int t0, int stride) {
+    const int E = (int)L.E;
+    const int64_t bucket_at[kTileLists] = {L.t8_bucket, L.t128_bucket, L.tta_bucket, L.ttb_bucket};
+    const int64_t start_at[kTileLists] = {L.t8_start, L.t128_start, L.tta_start, L.ttb_start};
+#pragma unroll
+    for (int list = 0; list < kTileLists; ++list) {
+        const int *first = sm.first[list];
+        for (int t = t0; t < first[E + 1]; t += stride) {
             int lo = 0, hi = E + 1;  // invariant: first[lo] <= t < first[hi]
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
                 if (first[mid] <= t) lo = mid;
                 else hi = mid;
             }
-            // lo is the last bucket whose first tile is <= t; empty buckets (first[b] == first[b + 1]) never win
-            tb[t] = lo;
-            ts[t] = offsets[lo] + (t - first[lo]) * rows;
+            ws[bucket_at[list] + t] = lo;
+            ws[start_at[list] + t] = sm.start[lo] + (t - first[lo]) * kTileRows[list];
         }
     }
 }
 
-// One warp places the slots [s0, s1) in order: rank inside a round from match.any, bucket cursors in shared memory.
+// One warp places the slots [s0, s1), at most kSegSlots of them, in order: rank inside a round from match.any, bucket cursors
+// in shared memory.  All ids are asked for before the first is used (with a load a round a round took 1100 cycles).
 __device__ inline void warp_place(const int32_t *ids, int s0, int s1, int e_lo, int E_local, int *cursor, int32_t *slots) {
+    constexpr int kRounds = kSegSlots / 32;
     const int lane = threadIdx.x & 31;
-    for (int base = s0; base < s1; base += 32) {
-        const int s = base + lane;
+    int id[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) id[r] = s0 + r * 32 + lane < s1 ? ids[s0 + r * 32 + lane] : 0;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int s = s0 + r * 32 + lane;
+        if (s0 + r * 32 >= s1) break;
         const bool live = s < s1;
-        const int b = live ? bucket_of(ids[s], e_lo, E_local) : -1 - lane;  // dead lanes match nobody
+        const int b = live ? bucket_of(id[r], e_lo, E_local) : -1 - lane;  // dead lanes match nobody
         const unsigned peers = __match_any_sync(0xffffffffu, b);
-        if (live) {
-            const int rank = __popc(peers & ((1u << lane) - 1u));
-            const int at = cursor[b];
-            slots[at + rank] = s;
-            __syncwarp(peers);
-            if (rank == 0) cursor[b] = at + __popc(peers);
-        }
+        const int rank = __popc(peers & ((1u << lane) - 1u)), at = live ? cursor[b] : 0;
+        if (live) slots[at + rank] = s;
+        __syncwarp();  // of the whole warp: one per group of peers ran them one after another
+        if (live && rank == 0) cursor[b] = at + __popc(peers);
         __syncwarp();
     }
 }
 
-// The whole pack of a small batch by one CTA of kPackThreads threads.
+// The whole pack of a small batch by one CTA of kPackThreads threads.  Eight warps take a run of slots each, in slot order; a
+// slot's rank among its warp's slots of the same bucket comes from match.any and the warp's own counts, and a bucket's base for
+// each warp from a prefix over the warps' counts: no warp waits for another (one warp placing 1500 slots, 32 a round, was most
+// of an 87 us launch).
+constexpr int kPlaceWarps = 8, kPlaceRounds = kSmallSlots / (32 * kPlaceWarps);
 __device__ void pack_small_body(const int32_t *__restrict__ ids, const RouteWords &L, int E_total, int e_lo, bool ep, int32_t *ws,
                                 uint32_t *err) {
-    __shared__ int cnt[kPackThreads], scanbuf[33], tile_first[4 * 1025];
+    __shared__ Layout sm;
+    __shared__ uint16_t counts[kPlaceWarps][kPackThreads];
     __shared__ int first_bad;
-    const int t = threadIdx.x, S = (int)L.S, E = (int)L.E;
-    cnt[t] = 0;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, S = (int)L.S, E = (int)L.E;
+    for (int i = t; i < kPlaceWarps * kPackThreads / 2; i += kPackThreads) reinterpret_cast<uint32_t *>(counts)[i] = 0u;
     if (t == 0) first_bad = 0x7fffffff;
     __syncthreads();
-    for (int s = t; s < S; s += kPackThreads) {
-        const int32_t id = ids[s];
-        atomicAdd(&cnt[bucket_of(id, e_lo, E)], 1);  // counts do not depend on the order of arrival
-        if (id < 0 || id >= E_total) atomicMin(&first_bad, s);
+    const int rounds = (S + 32 * kPlaceWarps - 1) / (32 * kPlaceWarps);  // of each warp: 1 .. kPlaceRounds
+    int bucket[kPlaceRounds], rank[kPlaceRounds];
+    if (warp < kPlaceWarps) {
+        int32_t id[kPlaceRounds];
+#pragma unroll
+        for (int r = 0; r < kPlaceRounds; ++r) {
+            const int s = (warp * rounds + r) * 32 + lane;
+            id[r] = r < rounds && s < S ? ids[s] : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < kPlaceRounds; ++r) {
+            const int s = (warp * rounds + r) * 32 + lane;
+            const bool live = r < rounds && s < S;
+            bucket[r] = live ? bucket_of(id[r], e_lo, E) : -1 - lane;  // dead lanes match nobody
+            if (live && (id[r] < 0 || id[r] >= E_total)) atomicMin(&first_bad, s);
+            if (r >= rounds) continue;
+            const unsigned peers = __match_any_sync(0xffffffffu, bucket[r]);
+            const int before = live ? counts[warp][bucket[r]] : 0, mine = __popc(peers & ((1u << lane) - 1u));
+            rank[r] = before + mine;
+            __syncwarp();
+            if (live && mine == 0) counts[warp][bucket[r]] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
     }
     __syncthreads();
     if (t == 0 && first_bad != 0x7fffffff) raise_error(err, (uint32_t)ids[first_bad], (uint32_t)first_bad);
-    const int count = t <= E ? cnt[t] : 0;
-    emit_layout(count, L, ws, scanbuf, tile_first, ep);
-    __syncthreads();
-    if (t <= E) cnt[t] = ws[L.offsets + t];  // cnt becomes the bucket cursors
-    __syncthreads();
-    if (t < 32) warp_place(ids, 0, S, e_lo, E, cnt, ws + L.slots);
+    int count = 0;
+    if (t <= E) {
+#pragma unroll
+        for (int w = 0; w < kPlaceWarps; ++w) {
+            const int c = counts[w][t];
+            counts[w][t] = (uint16_t)count;  // the warp's base inside the bucket
+            count += c;
+        }
+    }
+    scan_layout(count, L, ws, sm, ep);
+    if (warp < kPlaceWarps) {
+#pragma unroll
+        for (int r = 0; r < kPlaceRounds; ++r)
+            if (bucket[r] >= 0) ws[L.slots + sm.start[bucket[r]] + counts[warp][bucket[r]] + rank[r]] = (warp * rounds + r) * 32 + lane;
+    }
+    emit_tiles(L, ws, sm, t, kPackThreads);
 }
 
 __global__ void __launch_bounds__(kPackThreads)
@@ -198,7 +248,7 @@ __global__ void __launch_bounds__(32 * kSegWarps)
 // the bucket); totals -> offsets, header, tile lists; the first invalid slot -> err.
 __global__ void __launch_bounds__(kPackThreads)
     pack_scan_kernel(const int32_t *__restrict__ ids, RouteWords L, bool ep, int32_t *ws, uint32_t *err) {
-    __shared__ int scanbuf[33], tile_first[4 * 1025];
+    __shared__ Layout sm;
     const int b = threadIdx.x, E = (int)L.E;
     int total = 0;
     if (b <= E) {
@@ -206,10 +256,16 @@ __global__ void __launch_bounds__(kPackThreads)
         // read-modify-writes over 160 segments was most of this launch)
         int32_t *col = ws + L.scratch + b;
         const int64_t stride = E + 1;
-        for (int seg0 = 0; seg0 < L.nseg; seg0 += 16) {
-            int c[16];
+        int c[16], nxt[16];
+        auto fetch = [&](int seg0) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) c[i] = seg0 + i < L.nseg ? col[(int64_t)(seg0 + i) * stride] : 0;
+            for (int i = 0; i < 16; ++i) nxt[i] = seg0 + i < L.nseg ? col[(int64_t)(seg0 + i) * stride] : 0;
+        };
+        fetch(0);
+        for (int seg0 = 0; seg0 < L.nseg; seg0 += 16) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) c[i] = nxt[i];
+            fetch(seg0 + 16);  // the next chunk's loads before this chunk's stores, which they do not depend on
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 if (seg0 + i < L.nseg) col[(int64_t)(seg0 + i) * stride] = total;
@@ -227,21 +283,31 @@ __global__ void __launch_bounds__(kPackThreads)
         for (int w = 1; w < 32; ++w) bad = min(bad, bad_w[w]);
         if (bad != 0x7fffffff) raise_error(err, (uint32_t)ids[bad], (uint32_t)bad);
     }
-    emit_layout(total, L, ws, scanbuf, tile_first, ep);
+    scan_layout(total, L, ws, sm, ep);
+    // the tile lists are the last launch's work, whose CTAs share it
+    for (int i = b; i < kTileLists * (E + 2); i += kPackThreads) ws[L.first + i] = sm.first[i / (E + 2)][i % (E + 2)];
 }
 
-// Launch 3: every warp places its segment, starting each bucket at offsets[b] + the segment's base.
+// Launch 3: every warp places its segment, starting each bucket at offsets[b] + the segment's base; the CTAs then share the
+// tile lists, whose length grows with the slots (written by the one CTA of launch 2 they were most of its 39 us at 16384
+// tokens).
 __global__ void __launch_bounds__(32 * kSegWarps)
     pack_scatter_kernel(const int32_t *__restrict__ ids, RouteWords L, int e_lo, int32_t *ws) {
     __shared__ int cursor[kSegWarps][1024];
+    __shared__ Layout sm;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, E = (int)L.E, S = (int)L.S;
     const int seg = blockIdx.x * kSegWarps + warp;
-    if (seg >= L.nseg) return;
-    const int32_t *base = ws + L.scratch + (int64_t)seg * (E + 1);
-    for (int b = lane; b <= E; b += 32) cursor[warp][b] = ws[L.offsets + b] + base[b];
-    __syncwarp();
-    const int s0 = seg * kSegSlots;
-    warp_place(ids, s0, min(S, s0 + kSegSlots), e_lo, E, cursor[warp], ws + L.slots);
+    for (int b = threadIdx.x; b <= E; b += 32 * kSegWarps) sm.start[b] = ws[L.offsets + b];
+    for (int i = threadIdx.x; i < kTileLists * (E + 2); i += 32 * kSegWarps) sm.first[i / (E + 2)][i % (E + 2)] = ws[L.first + i];
+    __syncthreads();
+    if (seg < L.nseg) {
+        const int32_t *base = ws + L.scratch + (int64_t)seg * (E + 1);
+        for (int b = lane; b <= E; b += 32) cursor[warp][b] = sm.start[b] + base[b];
+        __syncwarp();
+        const int s0 = seg * kSegSlots;
+        warp_place(ids, s0, min(S, s0 + kSegSlots), e_lo, E, cursor[warp], ws + L.slots);
+    }
+    emit_tiles(L, ws, sm, blockIdx.x * 32 * kSegWarps + threadIdx.x, gridDim.x * 32 * kSegWarps);
 }
 
 int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo,
@@ -272,12 +338,15 @@ int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64
 // The workspace of a regular grouping, written without ids: S = M * E slots, slot m * E + b in bucket b for every m, so that
 // bucket b holds M slots in ascending order.  CTA 0 writes offsets, header and tile lists; every CTA writes slots.
 __global__ void __launch_bounds__(kPackThreads) regular_routes_kernel(RouteWords L, int per_bucket, int32_t *ws) {
-    __shared__ int scanbuf[33], tile_first[4 * 1025];
+    __shared__ Layout sm;
     const int E = (int)L.E;
     int32_t *slots = ws + L.slots;
     for (int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; pos < L.S; pos += (int64_t)gridDim.x * blockDim.x)
         slots[pos] = (int32_t)((pos % per_bucket) * E + pos / per_bucket);
-    if (blockIdx.x == 0) emit_layout((int)threadIdx.x < E ? per_bucket : 0, L, ws, scanbuf, tile_first, false);
+    if (blockIdx.x == 0) {
+        scan_layout((int)threadIdx.x < E ? per_bucket : 0, L, ws, sm, false);
+        emit_tiles(L, ws, sm, threadIdx.x, kPackThreads);
+    }
 }
 
 }  // namespace
@@ -306,7 +375,8 @@ RouteWords route_words(int64_t M, int64_t A, int64_t E) {
     L.segbad = L.t128_start + L.T128max;
     L.scratch = L.segbad + L.nseg;
     L.TtAmax = L.S / kTcTileA + E + 2, L.TtBmax = L.S / kTcTileB + E + 2;
-    L.tta_n = L.scratch + L.nseg * (E + 1);
+    L.first = L.scratch + L.nseg * (E + 1);
+    L.tta_n = L.first + (L.nseg ? kTileLists * (E + 2) : 0);
     L.tta_bucket = L.tta_n + 1;
     L.tta_start = L.tta_bucket + L.TtAmax;
     L.ttb_n = L.tta_start + L.TtAmax;
@@ -395,6 +465,14 @@ int sxb_moe_route_small(const float *logits, int64_t ld, int64_t M, int64_t E_to
     SXB_CHECK(ws_bytes >= (size_t)L.total * 4, fn, ": workspace of ", ws_bytes, " bytes, needs ", L.total * 4);
     auto st = static_cast<cudaStream_t>(stream);
     auto *w = static_cast<int32_t *>(ws);
+    // One CTA routes 32 tokens at a time, so from there on the router has a launch of its own, with a warp a token over the
+    // machine (150 tokens x 512 experts, top-10: 87 us as one launch).
+    if (M > kPackThreads / 32) {
+        if (int rc = sxb_moe_router(logits, ld, M, E_total, k, nullptr, 1, 0, ids, coef, SXB_ACT_F32, router_err, stream)) return rc;
+        pack_small_kernel<<<1, kPackThreads, 0, st>>>(ids, L, (int)E_total, (int)e_lo, ep, w, expert_err);
+        SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
+        return SXB_OK;
+    }
 #define SXB_ROUTE_SMALL(NV) \
     route_small_kernel<NV><<<1, kPackThreads, 0, st>>>(logits, ld, (int)M, (int)E_total, (int)k, ids, coef, L, (int)e_lo, ep, w, router_err, expert_err)
     if (E_total <= 128) SXB_ROUTE_SMALL(4);

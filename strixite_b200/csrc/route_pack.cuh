@@ -20,11 +20,12 @@ constexpr int kTcTileA = 192, kTcTileB = 256;
 //   slots [S]: slot index s = m * A + a, ascending inside a bucket
 //   t8_bucket / t8_start [T8max]: tiles of up to 8 slots (the streaming kernels); t128_*: up to 128 (tcgen05)
 //   segbad [nseg], scratch [nseg][E + 1]: the multi-CTA pack's per-segment first invalid slot and histograms
+//   first [4][E + 2], multi-CTA pack only: every bucket's first tile in the four lists, then the list's length
 //   tta [1 + 2 * TtAmax], ttb [1 + 2 * TtBmax]: a count, then bucket / start of tiles of up to kTcTileA and kTcTileB slots
 //                    (the tcgen05 kernel for tile-blocked activations: a work item is 128 weight rows x one such tile)
 struct RouteWords {
     int64_t S, E, T8max, T128max, TtAmax, TtBmax, nseg;
-    int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, tta_n, tta_bucket, tta_start, ttb_n, ttb_bucket, ttb_start, total;
+    int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, first, tta_n, tta_bucket, tta_start, ttb_n, ttb_bucket, ttb_start, total;
 };
 RouteWords route_words(int64_t M, int64_t A, int64_t E);
 // The workspace (route_words(M * E, 1, E)) of the grouping in which slot m * E + b belongs to bucket b, for all m < M: what

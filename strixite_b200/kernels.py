@@ -312,7 +312,8 @@ def moe_group_routes(ids, M, A, E, ws, ws_bytes, err, stream=None):
 
 
 def moe_route_small(logits, ld, M, E_total, k, e_lo, E_local, ids, coef, ws, ws_bytes, router_err, expert_err, stream=None):
-    """moe_router + moe_group_routes[_ep] as one launch of one CTA (M * k <= 2048 slots)."""
+    """moe_router + moe_group_routes[_ep] (M * k <= 2048 slots): one launch of one CTA up to 32 tokens, two above."""
+    _count(1 if M > 32 else 0)
     _check(_lib.load().sxb_moe_route_small(_ptr(logits), ld, M, E_total, k, e_lo, E_local, _ptr(ids), _ptr(coef), _ptr(ws),
                                            ws_bytes, _ptr(router_err), _ptr(expert_err), _stream(stream)))
 

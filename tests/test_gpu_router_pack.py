@@ -185,6 +185,13 @@ def test_pack_bit_exact(cuda, oracle, M, A, E):
         check_tiles(ws, L, offsets, E, rows, L[f"tile{rows}_n"], f"tile{rows}_bucket", f"tile{rows}_start")
 
 
+@pytest.mark.parametrize("M,A,E", [(1, 1, 1), (31, 1, 1), (257, 1, 3), (32, 64, 1023), (683, 3, 40), (1024, 4, 700), (2051, 5, 1023)])
+def test_pack_edges(cuda, oracle, M, A, E):
+    """Where the one-CTA pack's warps meet (a round or a run partly filled, 2048 slots exactly, every bucket count) and the
+    smallest and fullest launches of the other form."""
+    test_pack_bit_exact(cuda, oracle, M, A, E)
+
+
 def test_pack_golden(cuda, golden):
     from strixite_b200 import kernels as K
     ws, err, L = pack_on_gpu(K, golden["pack.ids"], 16, cuda)
