@@ -667,49 +667,72 @@ __global__ void __launch_bounds__(256) stage_f16_kernel(const uint4 *__restrict_
         xh[i] = b_chunk<BITS>(x[i], false);
 }
 
-// x -> the tile-blocked F16 form (tiled_offset) for the tiles of a grouping workspace: position pos of the slot order holds
-// the activation row of its slot (row slots[pos] / row_div), as F16 in the operand's k order, swizzled for its place in its
-// tile.  KIND: x is BF16 (0), F16 in natural k order (1) or F16 in this operand's order (2).  HBM-bound; a CTA takes a
-// quarter of a tile at a time (32 rows), because a small batch has a handful of tiles only: whole tiles left a 1001-row
-// dense projection to eight CTAs.
-constexpr int kStageRows = 32;
+// x -> the tile-blocked F16 form (tiled_offset) of a grouping workspace's slot order: position pos holds the activation row of
+// its slot (row slots[pos] / row_div), as F16 in the operand's k order, swizzled for its place in its tile (the place modulo 8,
+// i.e. the distance from the start of its expert's run: tiles are 128 positions).  KIND: x is BF16 (0), F16 in natural k order
+// (1) or F16 in this operand's order (2).
+// Memory-bound.  A CTA takes 32 neighbouring positions and blocks_per 64-k blocks, a warp a 64-k block at a time: four rows a
+// load, so that the 32 rows' 128-byte lines of the block are 4 KB written in one go, and eight loads in flight a lane.  Work is
+// cut by position and not by tile, and the k range too while there are few positions: a batch of 777 tokens is 512 tiles of 15
+// rows, and dealt out by quarter tiles it kept a quarter of the CTAs at work.
+constexpr int kStageRows = 32, kStageWarps = 8;
 template <int BITS, int KIND>
-__global__ void __launch_bounds__(256) stage_tiles_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ ws,
-                                                          RouteWords L, int64_t row_div, int64_t K, unsigned char *__restrict__ xs) {
-    // ws == nullptr: a dense projection's rows, in their own order (L.S rows, tile t = rows 128 t ..)
-    constexpr int kParts = kMaxTileTokens / kStageRows;
-    const int n_tiles = ws ? ws[3] : (int)((L.S + kMaxTileTokens - 1) / kMaxTileTokens), chunks_per_row = (int)(K / 8);
-    for (int part = blockIdx.x; part < n_tiles * kParts; part += gridDim.x) {
-        const int tile = part / kParts, n0 = (part % kParts) * kStageRows;
-        const int bucket = ws ? ws[L.t128_bucket + tile] : 0, start = ws ? ws[L.t128_start + tile] : tile * kMaxTileTokens;
-        const int cnt = ws ? min(kMaxTileTokens, ws[L.offsets + bucket + 1] - start) : (int)min((int64_t)kMaxTileTokens, L.S - start);
-        if (bucket >= L.E) continue;
-        // a warp takes one row at a time: its 32 lanes read 512 contiguous bytes of the token's activations per step,
-        // four steps in flight
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-        for (int n = n0 + warp; n < min(cnt, n0 + kStageRows); n += warps) {
-            const int64_t row = ws ? ws[L.slots + start + n] / row_div : start + n;
-            const uint4 *src = reinterpret_cast<const uint4 *>(x + row * K);
-            for (int k8 = lane; k8 < chunks_per_row; k8 += 128) {
-                uint4 v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (k8 + 32 * u < chunks_per_row) v[u] = src[k8 + 32 * u];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int kk = k8 + 32 * u;
-                    if (kk < chunks_per_row)
-                        *reinterpret_cast<uint4 *>(xs + tiled_offset(L.S, kk >> 3, start + n, n, kk & 7)) = KIND == 2 ? v[u] : b_chunk<BITS>(v[u], KIND == 1);
-                }
+__global__ void __launch_bounds__(32 * kStageWarps) stage_tiles_kernel(const uint16_t *__restrict__ x, const int32_t *__restrict__ ws,
+                                                                       RouteWords L, int64_t row_div, int64_t K, int blocks_per,
+                                                                       unsigned char *__restrict__ xs) {
+    // ws == nullptr: a dense projection's rows in their own order
+    __shared__ int first[kMoeMaxExperts + 1];  // first[b]: where bucket b's positions begin
+    __shared__ int64_t s_row[kStageRows];      // activation row, -1 = none
+    __shared__ int s_place[kStageRows];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x, E = (int)L.E;
+    const int64_t pos0 = (int64_t)blockIdx.x * kStageRows;
+    int slot = 0;
+    if (ws) {
+        if (t < kStageRows && pos0 + t < L.S) slot = ws[L.slots + pos0 + t];
+        for (int b = t; b <= E; b += 32 * kStageWarps) first[b] = ws[L.offsets + b];
+        __syncthreads();
+    }
+    if (t < kStageRows) {
+        const int64_t pos = pos0 + t;
+        int64_t row = pos < L.S ? pos : -1;
+        int place = (int)(pos & 7);
+        if (ws && row >= 0) {  // the last bucket that begins at or before pos; empty ones never win
+            int lo = 0, hi = E + 1;
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (first[mid] <= (int)pos) lo = mid;
+                else hi = mid;
             }
+            row = lo < E ? slot / row_div : -1;
+            place = ((int)pos - first[lo]) & 7;
+        }
+        s_row[t] = row, s_place[t] = place;
+    }
+    __syncthreads();
+    const int n_kb = (int)(K / 64), kb1 = min(n_kb, ((int)blockIdx.y + 1) * blocks_per), c = lane & 7;
+    for (int kb = (int)blockIdx.y * blocks_per + warp; kb < kb1; kb += kStageWarps) {
+        uint4 v[kStageRows / 4];
+#pragma unroll
+        for (int i = 0; i < kStageRows / 4; ++i) {
+            const int64_t row = s_row[4 * i + (lane >> 3)];
+            if (row >= 0) v[i] = __ldg(reinterpret_cast<const uint4 *>(x + row * K + (int64_t)kb * 64) + c);
+        }
+#pragma unroll
+        for (int i = 0; i < kStageRows / 4; ++i) {
+            const int r = 4 * i + (lane >> 3);
+            if (s_row[r] >= 0)
+                *reinterpret_cast<uint4 *>(xs + tiled_offset(L.S, kb, pos0 + r, s_place[r], c)) = KIND == 2 ? v[i] : b_chunk<BITS>(v[i], KIND == 1);
         }
     }
 }
 template <int BITS>
 void launch_stage_tiles(const void *x, int kind, const void *ws, const RouteWords &L, int64_t row_div, int64_t K, void *xs, cudaStream_t st) {
-    const int64_t tiles = ws ? L.T128max : (L.S + kMaxTileTokens - 1) / kMaxTileTokens;
-    const unsigned blocks = (unsigned)std::min<int64_t>(tiles * (kMaxTileTokens / kStageRows), (int64_t)sm_count() * 8);
-    auto go = [&](auto kern) { kern<<<blocks, 256, 0, st>>>((const uint16_t *)x, (const int32_t *)ws, L, row_div, K, (unsigned char *)xs); };
+    const int64_t parts = (L.S + kStageRows - 1) / kStageRows, n_kb = K / 64;
+    // k blocks a CTA takes: a multiple of its warps, fewer while that leaves less than eight CTAs an SM
+    int64_t per = (n_kb + kStageWarps - 1) / kStageWarps * kStageWarps;
+    while (per > kStageWarps && parts * ((n_kb + per - 1) / per) < (int64_t)sm_count() * 8) per = (per / 2 + kStageWarps - 1) / kStageWarps * kStageWarps;
+    const dim3 grid((unsigned)parts, (unsigned)((n_kb + per - 1) / per));
+    auto go = [&](auto kern) { kern<<<grid, 32 * kStageWarps, 0, st>>>((const uint16_t *)x, (const int32_t *)ws, L, row_div, K, (int)per, (unsigned char *)xs); };
     if (kind == 0) go(stage_tiles_kernel<BITS, 0>);
     else if (kind == 1) go(stage_tiles_kernel<BITS, 1>);
     else go(stage_tiles_kernel<BITS, 2>);
