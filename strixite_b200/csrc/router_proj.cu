@@ -163,14 +163,13 @@ struct GemmArgs {
 __device__ inline uint32_t instr_desc_bf16(int n_cols) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n_cols >> 3) << 17) | ((128u >> 4) << 24);
 }
-// D[tmem] (+)= A[smem] * B[smem].  Whole-warp call, one elected lane issues (as tc_commit).
-__device__ inline void tc_mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem], issued by one thread.
+__device__ inline void tc_mma_f16_ss_one(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
+        "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
 __device__ inline void tc_ld16(uint32_t taddr, float (&v)[16]) {
@@ -245,39 +244,44 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
     } else if (warp == 1) {
         // ===================== MMA issue =====================
-        uint32_t count = 0, acc_count = 0;
-        const uint32_t idesc = instr_desc_bf16(kTile);
-        for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x, ++acc_count) {
-            const uint32_t buf = acc_count & 1u;
-            if (lane == 0 && acc_count >= 2 && !mbar_wait(&acc_empty[buf], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns))
-                raise_abort(item, 2);
-            __syncwarp();
-            if (*abort_v) break;
-            tc_fence_after();
-            const uint32_t d = tmem_base + buf * (uint32_t)kTile;
-            bool failed = false;
-            for (int kb = 0; kb < n_kb; ++kb, ++count) {
-                const int stage = count % a.stages;
-                if (lane == 0 && !mbar_wait(&full_bar[stage], (count / a.stages) & 1u, abort_v, a.wait_limit_ns))
-                    raise_abort(item, 3), failed = true;
-                if (__any_sync(0xffffffffu, failed)) break;
-                tc_fence_after();
-                const uint32_t base = smem_u32(smem + stage * stage_bytes);
-                const uint64_t b_desc = smem_desc(base);
-                for (int p = 0; p < a.planes; ++p) {
-                    const uint64_t a_desc = smem_desc(base + (uint32_t)((1 + p) * kOperandBytes));
-#pragma unroll
-                    for (int j = 0; j < kGemmBK / 16; ++j)  // k = 16 an instruction: 32 bytes further along the swizzled line
-                        tc_mma_f16_ss(d, a_desc + 2 * j, b_desc + 2 * j, idesc, (kb | p | j) != 0);
+        // One thread runs the whole loop: an MMA costs it 12 cycles, against 40 to 90 with the election inside each MMA's
+        // instruction group, which at twelve MMAs a k-block (three planes) was more than their time on the tensor cores.
+        if (elect_one()) {
+            uint32_t count = 0, acc_count = 0;
+            const uint32_t idesc = instr_desc_bf16(kTile);
+            bool ok = true;
+            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++acc_count) {
+                const uint32_t buf = acc_count & 1u;
+                if (!mbar_wait(&acc_empty[buf], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                    raise_abort(item, 2);
+                    break;
                 }
-                tc_commit(&empty_bar[stage]);  // the stage is free once these MMAs have read it
+                tc_fence_after();
+                const uint32_t d = tmem_base + buf * (uint32_t)kTile;
+                for (int kb = 0; kb < n_kb; ++kb, ++count) {
+                    const int stage = count % a.stages;
+                    if (!mbar_wait(&full_bar[stage], (count / a.stages) & 1u, abort_v, a.wait_limit_ns)) {
+                        raise_abort(item, 3);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t base = smem_u32(smem + stage * stage_bytes);
+                    const uint64_t b_desc = smem_desc(base);
+                    for (int p = 0; p < a.planes; ++p) {
+                        const uint64_t a_desc = smem_desc(base + (uint32_t)((1 + p) * kOperandBytes));
+#pragma unroll
+                        for (int j = 0; j < kGemmBK / 16; ++j)  // k = 16 an instruction: 32 bytes further along the swizzled line
+                            tc_mma_f16_ss_one(d, a_desc + 2 * j, b_desc + 2 * j, idesc, (kb | p | j) != 0);
+                    }
+                    tc_commit_one(&empty_bar[stage]);  // the stage is free once these MMAs have read it
+                }
+                if (ok) tc_commit_one(&acc_full[buf]);
             }
-            if (__any_sync(0xffffffffu, failed)) break;
-            tc_commit(&acc_full[buf]);
+            // every MMA of this CTA has completed before tensor memory is released (not given up while aborting)
+            tc_commit_one(&drain_bar);
+            mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
         }
-        // every MMA of this CTA has completed before tensor memory is released (not given up while aborting)
-        tc_commit(&drain_bar);
-        if (lane == 0) mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
         __syncwarp();
     } else {
         // ===================== epilogue =====================
