@@ -422,6 +422,9 @@ typedef struct SxbMoeLayerArgs {
     uint32_t *router_err, *expert_err; /* >= 3 words each, zeroed by the caller at session start */
 } SxbMoeLayerArgs;
 int sxb_moe_layer(const SxbMoeLayerArgs *args, sxb_stream_t stream);
+/* The same with the shared expert's launches of the streaming path on a second stream, started behind what `stream` holds and
+ * waited for before the combine: nothing is left running on `side` that `stream` has not been made to wait for. */
+int sxb_moe_layer_two_streams(const SxbMoeLayerArgs *args, sxb_stream_t stream, sxb_stream_t side);
 
 /* ---- Expert parallelism (no counterpart in the reference, which drives one GPU) ------------------------------- */
 

@@ -73,6 +73,7 @@ SIGNATURES = {
     "sxb_report_expert_error": (C.c_int, [C.POINTER(u32), cp]),
     "sxb_quantize": (C.c_int, [vp, i64, i64, i64, C.c_int, vp, vp, vp, vp, vp]),
     "sxb_moe_layer": (C.c_int, [C.POINTER(SxbMoeLayerArgs), vp]),
+    "sxb_moe_layer_two_streams": (C.c_int, [C.POINTER(SxbMoeLayerArgs), vp, vp]),
     "sxb_set_wait_limit": (C.c_int, [C.c_uint64]),
     "sxb_test_skip_ring_slot": (C.c_int, [C.c_int]),
     "sxb_check_dense_status": (C.c_int, [cp]),

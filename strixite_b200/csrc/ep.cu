@@ -277,7 +277,7 @@ int sxb_moe_layer_ep(SxbEp *ep, const SxbMoeLayerArgs *a, sxb_stream_t stream) {
     PeerOut peer{};
     if (ep->return_path == 0) {
         b.y = ep->y_part, b.out_act = SXB_ACT_F32;
-        if (int rc = moe_layer_impl(&b, stream, nullptr)) return rc;
+        if (int rc = moe_layer_impl(&b, stream, nullptr, stream)) return rc;
         mark(ep, 3, st);
         // 4. reduce-scatter of the partial rows
         float *dst = a->out_act == SXB_ACT_F32 ? static_cast<float *>(a->y) : ep->y_part + (size_t)ep->rank * t * d;  // in place is allowed
@@ -293,7 +293,7 @@ int sxb_moe_layer_ep(SxbEp *ep, const SxbMoeLayerArgs *a, sxb_stream_t stream) {
         for (int r = 0; r < ep->world; ++r) peer.base[r] = ep->peer_recv[r];
         peer.world = ep->world, peer.rank = ep->rank, peer.t = t, peer.f16 = ep->return_path == 2;
         b.y = nullptr, b.out_act = SXB_ACT_F32;
-        if (int rc = moe_layer_impl(&b, stream, &peer)) return rc;
+        if (int rc = moe_layer_impl(&b, stream, &peer, stream)) return rc;
         mark(ep, 3, st);
         // 4. every rank has stored its pieces (stream order + the collective) before anybody reads its receive buffer
         SXB_NCCL(nc.AllReduce(ep->flag, ep->flag + 32, 1, kNcclInt32, kNcclSum, ep->comm, st), "all-reduce after the peer stores");

@@ -37,7 +37,7 @@ int combine_grouped(const char *fn, const void *h, const SxbQView *w, int64_t E_
                     int math, sxb_stream_t stream, const SxbMoeSharedAdd *shared, int h_f16, int64_t E_total, int64_t e_lo,
                     const PeerOut *peer = nullptr);
 // layer.cu: sxb_moe_layer; with `peer` the combine's rows go to their owners' receive buffers instead of y.
-int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut *peer);
+int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut *peer, sxb_stream_t side);
 
 // grouped_tc.cu - tcgen05 kernels (F16 operands, FP32 accumulation in tensor memory).
 template <int BITS>

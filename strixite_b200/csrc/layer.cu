@@ -36,7 +36,44 @@ int combine_ep(int bits, const void *h, const SxbQView *w, int64_t E, int64_t E_
 
 }  // namespace
 
-int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut *peer) {
+namespace {
+// Work on a second stream between two points of the caller's: fork() lets it start behind what the caller's stream holds,
+// join() - or the end of the scope, whatever was refused in between - makes the caller's stream wait for it.
+class SideWork {
+  public:
+    SideWork(cudaStream_t main, cudaStream_t side) : main_(main), side_(side) {}
+    SideWork(const SideWork &) = delete;
+    SideWork &operator=(const SideWork &) = delete;
+    ~SideWork() { join(); }
+    cudaError_t fork() {
+        const cudaError_t rc = order(main_, side_);
+        open_ = rc == cudaSuccess;
+        return rc;
+    }
+    cudaError_t join() {
+        if (!open_) return cudaSuccess;
+        open_ = false;
+        return order(side_, main_);
+    }
+
+  private:
+    static cudaError_t order(cudaStream_t first, cudaStream_t second) {
+        cudaEvent_t ev;
+        cudaError_t rc = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        if (rc != cudaSuccess) return rc;
+        rc = cudaEventRecord(ev, first);
+        if (rc == cudaSuccess) rc = cudaStreamWaitEvent(second, ev, 0);
+        cudaEventDestroy(ev);  // the runtime keeps it until the wait has passed
+        return rc;
+    }
+    cudaStream_t main_, side_;
+    bool open_ = false;
+};
+}  // namespace
+
+// side: the stream for the shared expert's small launches on the streaming kernels (they leave most SMs idle on their own), the
+// caller's stream itself = in order.
+int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut *peer, sxb_stream_t side) {
     const char *fn = "moe_layer";
     SXB_CHECK(a != nullptr, fn, ": null argument block");
     SXB_CHECK(a->gate_up != nullptr && a->down != nullptr, fn, ": null weight view");
@@ -79,13 +116,15 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
     }
 
     // the shared expert as dense projections (runtime/qwen4exp.cpp:3163-3168), in y's dtype
+    SideWork beside(st, static_cast<cudaStream_t>(side));
     if (shared) {
         SXB_CHECK(a->sh_h != nullptr && a->sh_y != nullptr, fn, ": null shared-expert buffer");
         if (!tc) {
             SXB_CHECK(a->sh_gu != nullptr, fn, ": null shared-expert buffer sh_gu");
-            if (int rc = linear_dense(a->shared_bits, a->x, a->shared_gate_up, a->sh_gu, M, SXB_ACT_BF16, SXB_ACT_BF16, stream)) return rc;
-            if (int rc = sxb_swiglu(a->sh_gu, a->sh_h, M, I, SXB_ACT_BF16, stream)) return rc;
-            if (int rc = linear_dense(a->shared_bits, a->sh_h, a->shared_down, a->sh_y, M, SXB_ACT_BF16, a->out_act, stream)) return rc;
+            if (side != stream) SXB_CUDA(beside.fork(), fn, ": starting the shared expert's stream");
+            if (int rc = linear_dense(a->shared_bits, a->x, a->shared_gate_up, a->sh_gu, M, SXB_ACT_BF16, SXB_ACT_BF16, side)) return rc;
+            if (int rc = sxb_swiglu(a->sh_gu, a->sh_h, M, I, SXB_ACT_BF16, side)) return rc;
+            if (int rc = linear_dense(a->shared_bits, a->sh_h, a->shared_down, a->sh_y, M, SXB_ACT_BF16, a->out_act, side)) return rc;
         } else {
             // dense projections on the tcgen05 kernel (kernels/linear_wmma.hip:69-113), SwiGLU fused into the first;
             // a wait that ran out is recorded in the routed experts' workspace header, like theirs
@@ -125,6 +164,7 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
     if (ep)
         return combine_ep(a->down_bits, a->h, a->down, E, a->E_total, a->e_lo, a->ids, a->coef, a->ws, a->ws_bytes, a->partial, M, A,
                           a->y, a->out_act, math, stream, hf, peer);
+    SXB_CUDA(beside.join(), fn, ": waiting for the shared expert's stream");
     SxbMoeSharedAdd sh{};
     if (shared) {
         sh.s = a->sh_y, sh.gate_logit = a->logits + a->E_total, sh.gate_ld = a->logits_ld, sh.gate_index = (uint32_t)a->E_total;
@@ -136,4 +176,7 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
 
 }  // namespace sxb
 
-extern "C" int sxb_moe_layer(const SxbMoeLayerArgs *a, sxb_stream_t stream) { return sxb::moe_layer_impl(a, stream, nullptr); }
+extern "C" int sxb_moe_layer(const SxbMoeLayerArgs *a, sxb_stream_t stream) { return sxb::moe_layer_impl(a, stream, nullptr, stream); }
+extern "C" int sxb_moe_layer_two_streams(const SxbMoeLayerArgs *a, sxb_stream_t stream, sxb_stream_t side) {
+    return sxb::moe_layer_impl(a, stream, nullptr, side);
+}

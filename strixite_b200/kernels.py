@@ -471,14 +471,20 @@ def _layer_args(x, logits, y, gate_up, down, E, A, ids, coef, ws, ws_bytes, h, p
 
 def moe_layer(x, logits, y, gate_up: QDeviceView, down: QDeviceView, E, A, ids, coef, ws, ws_bytes, h, partial, router_err,
               expert_err, xs=None, math=None, E_total=None, e_lo=0, shared_gate_up: Optional[QDeviceView] = None,
-              shared_down: Optional[QDeviceView] = None, sh_gu=None, sh_h=None, sh_y=None, sh_xs=None, stream=None):
+              shared_down: Optional[QDeviceView] = None, sh_gu=None, sh_h=None, sh_y=None, sh_xs=None, stream=None, side=None):
     """sxb_moe_layer: router, grouping, gate/up + SwiGLU, down + combine (+ shared expert) enqueued by one C call.
     x [M, d] BF16, logits [M, ld] FP32 (None: ids / coef already hold the routes), y [M, d] BF16 or FP32; the rest are the
-    caller's work buffers."""
+    caller's work buffers.  side: a second stream for the shared expert's launches on the streaming path."""
     a, keep = _layer_args(x, logits, y, gate_up, down, E, A, ids, coef, ws, ws_bytes, h, partial, router_err, expert_err, xs, math,
                           E_total, e_lo, shared_gate_up, shared_down, sh_gu, sh_h, sh_y, sh_xs)
-    _count(8)
-    _check(_lib.load().sxb_moe_layer(C.byref(a), _stream(stream)))
+    M, small = x.shape[0], x.shape[0] * A <= 2048
+    merged = logits is not None and small and M <= 32  # router and pack in one launch
+    tc = (M >= 256) if math is None else int(math) >= int(MoeMath.WmmaF16)
+    _count(int(logits is not None) + (1 if small else 3) - int(merged) + int(tc) + (3 if shared_gate_up is not None else 0) + 2)
+    if side is None:
+        _check(_lib.load().sxb_moe_layer(C.byref(a), _stream(stream)))
+    else:
+        _check(_lib.load().sxb_moe_layer_two_streams(C.byref(a), _stream(stream), _stream(side)))
 
 
 # ---- expert parallelism over the C ABI (no counterpart in the reference) ------------------------------------------

@@ -62,6 +62,10 @@ class MoeBuffers:
             self.sh_y = torch.empty((T, d), dtype=torch.bfloat16, device=dev)
             self.sh_y32 = torch.empty((T, d), dtype=torch.float32, device=dev)
 
+    def make_side_stream(self, device):
+        self.side_stream = torch.cuda.Stream(device=device)
+        self.ev_fork, self.ev_join = torch.cuda.Event(), torch.cuda.Event()
+
 
 class MoeLayer:
     """One MoE sublayer.  E_total / e_lo: expert-parallel ranks hold experts [e_lo, e_lo + E_local) of E_total in their
@@ -176,8 +180,26 @@ class MoeLayer:
         T = x.shape[0]
         assert T <= self.buf.max_tokens and x.dtype == torch.bfloat16 and logits.dtype == torch.float32
         math = self.math_for(T, math)
+        w = self.w
+        if not self.ep and not K_is_f16(math) and (w.shared_gate_up is None or w.shared_gate_up.bits == w.shared_down.bits):
+            return self._forward_streaming(x, logits, y, math)
         packed = self.route(logits, T)
         return self.run_experts(x, T, y, math, logits, packed=packed)
+
+    def _forward_streaming(self, x, logits, y, math):
+        """The decode step as one library call: the launches of route() and run_experts(), in their order and on their two
+        streams.  At a few tokens a step is shorter on the GPU than its eight calls from Python (one token: 112 us)."""
+        b, w = self.buf, self.w
+        side = None
+        if w.shared_gate_up is not None:
+            if b.side_stream is None:
+                b.make_side_stream(x.device)
+            side = b.side_stream
+        sh = {} if side is None else dict(shared_gate_up=w.shared_gate_up, shared_down=w.shared_down, sh_gu=b.sh_gu, sh_h=b.sh_h,
+                                          sh_y=b.sh_y32 if y.dtype == torch.float32 else b.sh_y)
+        K.moe_layer(x, logits, y, w.gate_up, w.down, self.E, self.k, b.ids, b.coef, b.ws, b.ws_bytes, b.h, b.partial, b.router_err,
+                    b.expert_err, math=math, side=side, **sh)
+        return y
 
     def run_experts(self, x: torch.Tensor, T: int, y: torch.Tensor, math: MoeMath, logits: torch.Tensor, events=None,
                     packed: bool = False):
@@ -199,8 +221,7 @@ class MoeLayer:
         # streaming (they leave most SMs idle on their own) and are joined just before the combine that adds them.
         cur = torch.cuda.current_stream()
         if b.side_stream is None:
-            b.side_stream = torch.cuda.Stream(device=x.device)
-            b.ev_fork, b.ev_join = torch.cuda.Event(), torch.cuda.Event()
+            b.make_side_stream(x.device)
         b.ev_fork.record(cur)
         b.side_stream.wait_event(b.ev_fork)
         with torch.cuda.stream(b.side_stream):

@@ -83,6 +83,36 @@ def test_layer_rows_do_not_depend_on_batch(cuda):
         start += n
 
 
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 33, 230])
+def test_forward_equals_its_launchers(cuda, T, out):
+    """The one-call decode step (also on a stream of its own, where its second stream has to follow it) gives what the launchers
+    give call by call, bit for bit."""
+    from strixite_b200 import workloads as W
+    from strixite_b200.kernels import MoeMath
+    from strixite_b200.layer import MoeBuffers, MoeLayer
+    from dataclasses import replace
+    cfg = replace(W.CONFIGS["c1"], T=T, E=64, name="forward")
+    w = W.make_layer_weights(cfg, 0, cuda)
+    x = W.activations(cfg, 0, cuda)
+    logits = W.router_logits(x, W.router_weight(cfg, 0, cuda), W.expert_bias(cfg, 0, cuda))
+    ys = []
+    for one_call in (False, True, True):
+        layer = MoeLayer(w, cfg.E, cfg.k, MoeBuffers(T, cfg.d, cfg.I, cfg.E, cfg.k, cuda, cfg.shared))
+        y = torch.empty((T, cfg.d), dtype=out, device=cuda)
+        stream = torch.cuda.Stream() if len(ys) == 2 else torch.cuda.current_stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            if one_call:
+                layer.forward(x, logits, y, math=MoeMath.F32)
+            else:
+                layer.run_experts(x, T, y, MoeMath.F32, logits, packed=layer.route(logits, T))
+        torch.cuda.synchronize()
+        layer.check_errors("forward")
+        ys.append(y)
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+
+
 def edge_rows(buf, cfg):
     """Token rows that sit at the edges of the pack: the first and the last slot of the fullest and of the emptiest
     non-empty expert, and the first slot of a partly filled 128-slot tile."""
