@@ -1,5 +1,5 @@
 // Shared by the two tcgen05 expert kernels (grouped_tc.cu: activations gathered per tile, any layout; grouped_tc_tiled.cu:
-// tile-blocked activations, one dequantization of the weights shared by up to 256 tokens): launch arguments, output modes,
+// tile-blocked activations): launch arguments, output modes,
 // and the dequantization of packed codes to the F16 operand.
 #pragma once
 

@@ -24,8 +24,8 @@
 //
 // SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up
-// rows of the same h columns, and the epilogue pairs them with one shuffle per value: of the 32 tokens of a pass the gate
-// lane finishes the first 16, the up lane the other 16.
+// rows of the same h columns, and the epilogue pairs them with one shuffle per value: of the 16 tokens of a pass the gate
+// lane finishes the first 8, the up lane the other 8.
 //
 // Operands as in grouped_tc.cu: A (weights) dequantized in registers and stored to tensor memory by the producer warps
 // (the [tmem] form of tcgen05.mma), B (activations) two cp.async.bulk per step (one per 64-k sub-tile) into
@@ -65,7 +65,7 @@ struct Shape {
     static constexpr int kWays = HC ? 2 : 4;  // producer sets
     static constexpr int kStages = kWays;
     static constexpr int kSlotBytes = kRows * kBK * BITS / 8;  // a ring slot: the packed codes of a step, 8 or 16 KB
-    static constexpr int kWSlots = kWays * (BITS == 4 ? 2 : 1) * (HC ? 2 : 1);
+    static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 4 ? 3 : 1);  // what shared memory holds beside the stages (Q4, 8 -> 12 slots: 583 -> 572 us at 777 tokens)
     static constexpr int kEpiSets = HC ? 2 : 1;  // epilogue warps per lane quadrant
     static constexpr int kEpiWarps = 4 * kEpiSets, kMmaWarp = kEpiWarps, kBCopyWarp = kEpiWarps + 1, kWCopyWarp = kEpiWarps + 2,
                          kItemWarp = kEpiWarps + 3, kFirstAWarp = kEpiWarps + 4;
@@ -74,7 +74,7 @@ struct Shape {
     static_assert(kAccs * kTile + kStages * kAStageCols <= kTmemCols, "tensor memory");
     static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
-constexpr int kItemRing = 4;
+constexpr int kItemRing = 2;
 // kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
 constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
