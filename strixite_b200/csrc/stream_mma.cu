@@ -622,6 +622,49 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
     }
 }
 
+// v = four columns of token m, from n on: sum_a fma(coef[m, a], partial[m*A + a, n]) in slot order; NaN for a token with an id
+// outside [0, E_total).  Slots of experts outside [e_lo, e_lo + E_local) - other ranks' in expert-parallel runs - are skipped.
+// PBF16: the per-slot dots are BF16 bits, N * 2 bytes a slot (kernels/moe_grouped.hip:47-57), read from the same buffer.
+// Memory-bound: five slots' loads are issued before the first is added (one slot at a time, its load
+// behind its id's: 159 -> 146 us at 4096 tokens x 10 slots x 4096, 509 -> 477 at 16384).
+template <bool PBF16>
+__device__ inline void combine_slots(float (&v)[4], const float *__restrict__ partial, const int32_t *__restrict__ ids,
+                                     const float *__restrict__ coef, int64_t m, int64_t n, int64_t A, int64_t E_total, int64_t e_lo,
+                                     int64_t E_local, int64_t N) {
+    constexpr int kAhead = 5;
+    bool ok = true;
+    v[0] = v[1] = v[2] = v[3] = 0.f;
+    for (int64_t k0 = 0; k0 < A; k0 += kAhead) {
+        float4 p[kAhead];
+        float cf[kAhead];
+        bool use[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int64_t slot = m * A + k0 + u;
+            const bool in = k0 + u < A;
+            const int32_t id = in ? __ldg(ids + slot) : 0;
+            ok = ok && (!in || (id >= 0 && id < E_total));
+            use[u] = in && id >= e_lo && id < e_lo + E_local;
+            cf[u] = use[u] ? __ldg(coef + slot) : 0.f;
+            if (!use[u]) continue;
+            if constexpr (PBF16) {
+                const uint2 b = __ldg(reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(partial) + slot * N + n));
+                p[u].x = __uint_as_float(b.x << 16), p[u].y = __uint_as_float(b.x & 0xffff0000u);
+                p[u].z = __uint_as_float(b.y << 16), p[u].w = __uint_as_float(b.y & 0xffff0000u);
+            } else {
+                p[u] = __ldg(reinterpret_cast<const float4 *>(partial + slot * N + n));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (!use[u]) continue;
+            v[0] = fmaf(cf[u], p[u].x, v[0]), v[1] = fmaf(cf[u], p[u].y, v[1]);
+            v[2] = fmaf(cf[u], p[u].z, v[2]), v[3] = fmaf(cf[u], p[u].w, v[3]);
+        }
+    }
+    if (!ok) v[0] = v[1] = v[2] = v[3] = qnan_f32();
+}
+
 // y[m, n] = sum_a fma(coef[m, a], partial[m*A + a, n]) in slot order, one rounding (kernels/moe_grouped.hip:948-984).
 // Four columns a thread.  A token with an id outside [0, E_total) gets a NaN row.  Slots of experts outside
 // [e_lo, e_lo + E_local) - other ranks' in expert-parallel runs - are skipped.  SH folds the shared expert's gated add:
@@ -636,24 +679,8 @@ __global__ void __launch_bounds__(256)
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= M * N) return;
     const int64_t m = i / N, n = i % N;  // N % 4 == 0: the four columns lie in one row
-    bool ok = true;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int64_t k = 0; k < A; ++k) {
-        const int32_t id = ids[m * A + k];
-        ok = ok && id >= 0 && id < E_total;
-        if (id < e_lo || id >= e_lo + E_local) continue;
-        const float cf = coef[m * A + k];
-        float4 p;
-        if constexpr (PBF16) {
-            const uint2 b = *reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(partial) + (m * A + k) * N + n);
-            p.x = __uint_as_float(b.x << 16), p.y = __uint_as_float(b.x & 0xffff0000u);
-            p.z = __uint_as_float(b.y << 16), p.w = __uint_as_float(b.y & 0xffff0000u);
-        } else {
-            p = *reinterpret_cast<const float4 *>(partial + (m * A + k) * N + n);
-        }
-        v[0] = fmaf(cf, p.x, v[0]), v[1] = fmaf(cf, p.y, v[1]), v[2] = fmaf(cf, p.z, v[2]), v[3] = fmaf(cf, p.w, v[3]);
-    }
-    if (!ok) v[0] = v[1] = v[2] = v[3] = qnan_f32();
+    float v[4];
+    combine_slots<PBF16>(v, partial, ids, coef, m, n, A, E_total, e_lo, E_local, N);
     if constexpr (SH) {
         const float gl = gate_logit[m * gate_ld];
         const bool gok = isfinite(gl);
@@ -675,24 +702,8 @@ __global__ void __launch_bounds__(256)
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= M * N) return;
     const int64_t m = i / N, n = i % N;
-    bool ok = true;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int64_t k = 0; k < A; ++k) {
-        const int32_t id = ids[m * A + k];
-        ok = ok && id >= 0 && id < E_total;
-        if (id < e_lo || id >= e_lo + E_local) continue;
-        const float cf = coef[m * A + k];
-        float4 p;
-        if constexpr (PBF16) {
-            const uint2 b = *reinterpret_cast<const uint2 *>(reinterpret_cast<const uint16_t *>(partial) + (m * A + k) * N + n);
-            p.x = __uint_as_float(b.x << 16), p.y = __uint_as_float(b.x & 0xffff0000u);
-            p.z = __uint_as_float(b.y << 16), p.w = __uint_as_float(b.y & 0xffff0000u);
-        } else {
-            p = *reinterpret_cast<const float4 *>(partial + (m * A + k) * N + n);
-        }
-        v[0] = fmaf(cf, p.x, v[0]), v[1] = fmaf(cf, p.y, v[1]), v[2] = fmaf(cf, p.z, v[2]), v[3] = fmaf(cf, p.w, v[3]);
-    }
-    if (!ok) v[0] = v[1] = v[2] = v[3] = qnan_f32();
+    float v[4];
+    combine_slots<PBF16>(v, partial, ids, coef, m, n, A, E_total, e_lo, E_local, N);
     const int owner = (int)(m / peer.t);
     const int64_t at = (((int64_t)peer.rank * peer.t + m % peer.t) * N + n);
     if constexpr (OUT_F16) {
