@@ -1,6 +1,5 @@
 // Shared by the two tcgen05 expert kernels (grouped_tc.cu: activations gathered per tile, any layout; grouped_tc_tiled.cu:
-// tile-blocked activations): launch arguments, output modes,
-// and the dequantization of packed codes to the F16 operand.
+// tile-blocked activations): launch arguments, output modes, and the dequantization of packed codes to the F16 operand.
 #pragma once
 
 #include "experts.cuh"

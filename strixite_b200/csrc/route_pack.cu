@@ -6,9 +6,9 @@
 // Here the sort is stable - inside a bucket, slots ascend - so the whole workspace is a pure function of ids and can
 // be compared word for word with a CPU counting sort.  Ranks inside a bucket come from `match.any` warp votes, never
 // from the arrival order of atomics.
-//   S <= kSmallSlots: one CTA does everything (decode: S = 160 is five warp rounds).
-//   larger S: three launches - per-warp-segment histograms, one CTA that scans them into bucket offsets / per-segment
-//   bases / tile lists, and a scatter in which every warp places its own segment in order.
+//   S <= kSmallSlots: one CTA does everything, eight of its warps a run of slots each.
+//   larger S: three launches - per-warp-segment histograms, one CTA that scans them into bucket offsets and per-segment
+//   bases, and a scatter in which every warp places its own segment in order and the CTAs share the tile lists.
 
 #include "route_pack.cuh"
 

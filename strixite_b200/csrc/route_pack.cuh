@@ -8,9 +8,7 @@ namespace sxb {
 constexpr int64_t kMoeMaxExperts = 1023;   // E + 1 buckets fit one 1024-thread CTA (kernels/moe_grouped.hpp:43)
 constexpr int64_t kMoeMaxSlots = 1 << 20;  // kernels/moe_grouped.hpp:44
 constexpr int kSegSlots = 1024;            // slots one warp places in the multi-CTA pack
-// Tokens per work item of the tcgen05 kernel for tile-blocked activations (multiples of 16): the narrower tile has two
-// accumulators in tensor memory (short contractions, where an item's epilogue must run under the next item's mainloop),
-// the wider one has one (long contractions, where sharing a dequantization between more tokens pays more).
+// Rows of the two wider tile lists that close the workspace; the kernels here walk the lists of 8 and 128.
 constexpr int kTcTileA = 192, kTcTileB = 256;
 
 // Word (int32) offsets into the workspace.
@@ -22,7 +20,6 @@ constexpr int kTcTileA = 192, kTcTileB = 256;
 //   segbad [nseg], scratch [nseg][E + 1]: the multi-CTA pack's per-segment first invalid slot and histograms
 //   first [4][E + 2], multi-CTA pack only: every bucket's first tile in the four lists, then the list's length
 //   tta [1 + 2 * TtAmax], ttb [1 + 2 * TtBmax]: a count, then bucket / start of tiles of up to kTcTileA and kTcTileB slots
-//                    (the tcgen05 kernel for tile-blocked activations: a work item is 128 weight rows x one such tile)
 struct RouteWords {
     int64_t S, E, T8max, T128max, TtAmax, TtBmax, nseg;
     int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, first, tta_n, tta_bucket, tta_start, ttb_n, ttb_bucket, ttb_start, total;

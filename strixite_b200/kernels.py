@@ -289,7 +289,7 @@ def moe_route_workspace_bytes(M, A, E) -> int:
     return n
 
 
-TC_TILES = (192, 256)  # tokens per work item of the tcgen05 kernel for tile-blocked activations (route_pack.cuh)
+TC_TILES = (192, 256)  # rows of the two wider tile lists that close the workspace (route_pack.cuh)
 
 
 def route_layout(M, A, E) -> dict:
