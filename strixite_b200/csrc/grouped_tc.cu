@@ -320,12 +320,12 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
                 if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    __half2 s2[kGroupsPerKb], s16[kGroupsPerKb], m2[kGroupsPerKb];
+                    __half2 s2[kGroupsPerKb], m2[kGroupsPerKb];
 #pragma unroll
                     for (int gi = 0; gi < kGroupsPerKb; ++gi) {
                         const int g = ((kb * kBK) / G + gi) & 7;  // group inside the chunk of eight
                         const float sf = bf16_bits_to_f32(pick16(sc_cur[h].s, g)), mf = bf16_bits_to_f32(pick16(sc_cur[h].m, g));
-                        s2[gi] = __float2half2_rn(sf), s16[gi] = __float2half2_rn(sf * 0.0625f), m2[gi] = __float2half2_rn(mf);
+                        s2[gi] = __float2half2_rn(sf), m2[gi] = __float2half2_rn(mf);
                     }
                     const uint32_t a_addr = tmem_base + ((uint32_t)(a_quad * 32) << 16) +
                                             (uint32_t)(kAStageCol0 + stage * kAStageCols + h * (kBK / 2));
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
 #pragma unroll
                             for (int cc = 0; cc < 4; ++cc) {
                                 const int gi = kGroupsPerKb == 1 ? 0 : ((hc * 4 + cc) * 8) / G;
-                                d[cc] = dequant_q4_word(w4[cc], s2[gi], s16[gi], m2[gi]);
+                                d[cc] = dequant_q4_word(w4[cc], s2[gi], m2[gi]);
                             }
                         } else {
                             const uint4 v0 = code[h][hc * 2], v1 = code[h][hc * 2 + 1];  // 2 x 16 codes

@@ -48,17 +48,18 @@ struct TcArgs {
 
 // Eight weights = one 16-byte chunk of the A line, from one word of Q4 codes or two words of Q8 codes.
 // w = code * s + m with one F16 rounding (kernels/wmma_gemm.hpp:116-129).
-__device__ inline uint4 dequant_q4_word(uint32_t w, __half2 s, __half2 s16, __half2 m) {
-    const __half2 k1024 = __float2half2_rn(1024.f);
+__device__ inline uint4 dequant_q4_word(uint32_t w, __half2 s, __half2 m) {
+    const __half2 k1024 = __float2half2_rn(1024.f), k16th = __float2half2_rn(0.0625f);
     const uint32_t w8 = w >> 8;
-    // (w & 0x000F000F) | 0x64006400 = (1024 + n0, 1024 + n4); the 0x00F0 nibbles give 1024 + 16 n and meet s / 16
+    // (w & 0x000F000F) | 0x64006400 = (1024 + n0, 1024 + n4); the 0x00F0 nibbles give 1024 + 16 n.  The sixteenth goes to the code,
+    // where it is exact: s / 16 would be an F16 subnormal from s < 2^-10 on, and short of bits from 2^-13 on.
     const __half2 p0 = __hsub2(u32_as_h2((w & 0x000F000Fu) | 0x64006400u), k1024);
-    const __half2 p1 = __hsub2(u32_as_h2((w & 0x00F000F0u) | 0x64006400u), k1024);
+    const __half2 p1 = __hmul2(__hsub2(u32_as_h2((w & 0x00F000F0u) | 0x64006400u), k1024), k16th);
     const __half2 p2 = __hsub2(u32_as_h2((w8 & 0x000F000Fu) | 0x64006400u), k1024);
-    const __half2 p3 = __hsub2(u32_as_h2((w8 & 0x00F000F0u) | 0x64006400u), k1024);
+    const __half2 p3 = __hmul2(__hsub2(u32_as_h2((w8 & 0x00F000F0u) | 0x64006400u), k1024), k16th);
     uint4 d;
-    d.x = h2_as_u32(__hfma2(p0, s, m)), d.y = h2_as_u32(__hfma2(p1, s16, m));
-    d.z = h2_as_u32(__hfma2(p2, s, m)), d.w = h2_as_u32(__hfma2(p3, s16, m));
+    d.x = h2_as_u32(__hfma2(p0, s, m)), d.y = h2_as_u32(__hfma2(p1, s, m));
+    d.z = h2_as_u32(__hfma2(p2, s, m)), d.w = h2_as_u32(__hfma2(p3, s, m));
     return d;
 }
 __device__ inline uint4 dequant_q8_words(uint32_t w0, uint32_t w1, __half2 s, __half2 m) {
@@ -78,8 +79,8 @@ __device__ inline uint4 dequant_q8_words(uint32_t w0, uint32_t w1, __half2 s, __
 // with their factors, s16 = s / 16.  Nine instructions per eight codes instead of eighteen (adding the 0x6400 and taking the
 // 1024 off again): a 128 x 128 block took its four warps 202 SM cycles instead of 337.
 // Rounding: s * 2^k < 2^15 for the row's largest s, so the row's largest weights lie between 2^-9 and 1/2 and keep their
-// eleven bits; weights 2^10 times smaller than those fall below 2^-14 and are rounded at 2^-25, i.e. still finer than the
-// rounding of the large ones.
+// eleven bits; those of a group whose scale is 2^7 or more below the largest can lose bits to F16's subnormals, so rows with
+// such groups go without a power of two (kScaleSpread in grouped_tc_tiled.cu).
 __device__ inline uint4 dequant_q4_scaled(uint32_t w, __half2 s, __half2 s16, __half2 m) {
     const uint32_t w8 = w >> 8;
     uint4 d;

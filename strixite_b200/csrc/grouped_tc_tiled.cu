@@ -78,13 +78,23 @@ constexpr int kItemRing = 2;
 // kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
 constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
-// The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).
-__device__ inline float unscale(float scale) { return __int_as_float(((127 + 24 + 127) << 23) - __float_as_int(scale)); }
+// The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).  Rows at natural magnitude: scale = -2^24.
+constexpr float kNatural = -0x1p24f;
+__device__ inline float unscale(float scale) { return __int_as_float(((127 + 24 + 127) << 23) - __float_as_int(fabsf(scale))); }
 
 struct Item {
     int bucket, start, cnt;  // expert (bucket E = invalid ids, -1 = no more items), first position in slots[], tokens of the item
     int rb;                  // row block
 };
+
+// A row's common power of two is set by its largest group, and weights far below that one's lose bits (dequant_q4_scaled).  With e
+// the largest exponent among a row's groups (of the scale, or of the min less 8) and every other group's at most kScaleSpread
+// below, nothing is lost: a code's step is a BF16 of eight bits and at least 2^-16, so its last bit is at least 2^-23, above the
+// last place of an F16 subnormal, 2^-24.  A quadrant of an item with a row spread wider - columns that a quantizer scaled up on
+// purpose - takes its weights at their natural magnitude (dequant_q4_word), unless the common power makes them no smaller than that
+// (scales below 2^-9).  Error of the small columns' dots against 64 bits, Q4, groups 2^7 / 2^10 / 2^12 apart: 5.6e-4 / 9.2e-3 /
+// 3.4e-2 with the common power of two, 2e-5 at any distance without.  The test for it costs gate/up at 777 tokens 553 -> 560 us.
+constexpr int kScaleSpread = 6;
 
 template <int MODE>
 __device__ inline int row_blocks(const TcArgs &a) {
@@ -103,6 +113,38 @@ __device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
     it.start = a.ws[a.L.t128_start + tile];
     it.cnt = min(kTile, a.ws[a.L.offsets + it.bucket + 1] - it.start);
     return it;
+}
+
+// The sixteen BF16 halves' g-th, of eight groups.
+__device__ inline uint16_t pick16(const uint4 &v, int g) {
+    const uint32_t w = (g & 4) ? ((g & 2) ? v.w : v.z) : ((g & 2) ? v.y : v.x);
+    return (uint16_t)((g & 1) ? (w >> 16) : (w & 0xffffu));
+}
+
+// A producer lane's step of a quadrant at natural magnitude (kScaleSpread): its row's codes at `src` of shared memory (16-byte chunks
+// swizzled by sw) with the groups from g0 on of s and m -> tensor memory.  A call: rare, and inlined its registers would be the
+// common step's.
+template <int BITS, int G>
+__device__ __noinline__ void natural_step(uint32_t src, uint32_t sw, uint32_t a_addr, uint4 s, uint4 m, int g0) {
+    constexpr int kChunkCodes = BITS == 4 ? 32 : 16, kChunks = 32 / kChunkCodes;
+#pragma unroll 1
+    for (int hc = 0; hc < 4; ++hc) {
+        uint4 d[4];
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            const uint4 v = ld_shared_v4(src + ((uint32_t)(hc * kChunks + c) ^ sw) * 16u);
+            const int g = (g0 + hc * 32 / G) & 7;  // 32 codes lie in one group
+            const __half2 s2 = __float2half2_rn(bf16_bits_to_f32(pick16(s, g))), m2 = __float2half2_rn(bf16_bits_to_f32(pick16(m, g)));
+            if (BITS == 4) {
+                d[0] = dequant_q4_word(v.x, s2, m2), d[1] = dequant_q4_word(v.y, s2, m2);
+                d[2] = dequant_q4_word(v.z, s2, m2), d[3] = dequant_q4_word(v.w, s2, m2);
+            } else {
+                d[2 * c] = dequant_q8_words(v.x, v.y, s2, m2), d[2 * c + 1] = dequant_q8_words(v.z, v.w, s2, m2);
+            }
+        }
+        tc_st16(a_addr + hc * 16, d);
+    }
+    __syncwarp();
 }
 
 template <int BITS, int G, int MODE>
@@ -239,11 +281,6 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
             }
             return c;
         };
-        auto pick16 = [](const uint4 &v, int g) {
-            const uint32_t w = (g & 4) ? ((g & 2) ? v.w : v.z) : ((g & 2) ? v.y : v.x);
-            return (uint16_t)((g & 1) ? (w >> 16) : (w & 0xffffu));
-        };
-
         ScaleChunk sc_cur = {}, sc_nxt = {};
         int nxt_item = -1, nxt_chunk = -1;  // what sc_nxt holds
         uint32_t j = 0;                     // steps this set has done
@@ -276,9 +313,10 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 const uint32_t slot = set + (kSlotsPerSet > 1 ? (j % kSlotsPerSet) * kWays : 0);
                 bool ok = mbar_wait(&w_full[slot], (j / kSlotsPerSet) & 1u, abort_v, a.wait_limit_ns);
                 if (!ok && lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 7);
+                const uint32_t src = my_w + (slot - set) * (uint32_t)kSlotBytes;
                 uint4 code[kCodeRegs];
 #pragma unroll
-                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(my_w + (slot - set) * (uint32_t)kSlotBytes + (((uint32_t)c ^ my_sw) << 4));
+                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(src + (((uint32_t)c ^ my_sw) << 4));
                 __half2 s2[kGroupsPerStep], s16[kGroupsPerStep], m2[kGroupsPerStep];
 #pragma unroll
                 for (int gi = 0; gi < kGroupsPerStep; ++gi) {
@@ -309,12 +347,17 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                     break;
                 }
                 tc_fence_after();  // the stores below come after the MMAs that freed the stage
-                if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
-                tc_st16(a_addr, d);
+                if (scale > 0.f) {
+                    if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
+                    tc_st16(a_addr, d);
 #pragma unroll
-                for (int hc = 1; hc < 4; ++hc) {
-                    quarter(hc, d);
-                    tc_st16(a_addr + hc * 16, d);
+                    for (int hc = 1; hc < 4; ++hc) {
+                        quarter(hc, d);
+                        tc_st16(a_addr + hc * 16, d);
+                    }
+                } else {
+                    natural_step<BITS, G>(src, my_sw, a_addr, sc_cur.s, sc_cur.m, (st * kGroupsPerStep) & 7);
+                    if (lane == 0) mbar_arrive(&w_empty[slot]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
@@ -327,15 +370,23 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         // ===================== the item ring =====================
         // One warp looks the CTA's items up ahead of everyone else: the other roles read an item's description from shared
         // memory instead of each walking two dependent loads of the grouping workspace per item.  It also finds each
-        // row's power of two (dequant_q4_scaled) from the row's scales and mins, four rows a lane; those lines are then in
-        // L2 when the producers want them.
+        // row's power of two (dequant_q4_scaled) from the row's scales and mins, four rows a lane, and whether one suits the rows of
+        // a tensor-memory quadrant at all (kScaleSpread); those lines are then in L2 when the producers want them.  Where
+        // contractions are short this is the longest chain of an item: its instructions count.
         const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
+        const bool pair_scales = groups % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 3) == 0;
         Item nxt = blockIdx.x < n_items ? item_info(a, blockIdx.x, rbs) : no_item;
         for (int i = 0;; ++i) {
             const Item it = nxt;
             const int item = blockIdx.x + i * gridDim.x;
             nxt = item + (int)gridDim.x < n_items ? item_info(a, item + gridDim.x, rbs) : no_item;
-            uint32_t smax[4] = {0u, 0u, 0u, 0u}, mmax[4] = {0u, 0u, 0u, 0u};  // two 16-bit maxima of the BF16 magnitudes
+            // Of every group v = max(|scale| * 2^8, |min|) as BF16 bits, 0x400 = an empty group; two 16-bit maxima of v, and signed
+            // minima of v + 0x7bff, in which an empty group's is the largest.  Five instructions for two groups.
+            uint32_t top[4] = {0u, 0u, 0u, 0u}, low[4] = {0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu};
+            auto take = [&](int r, uint32_t s, uint32_t m) {
+                const uint32_t v = __viaddmax_u16x2(s & 0x7fff7fffu, 0x04000400u, m & 0x7fff7fffu);
+                top[r] = __vmaxu2(top[r], v), low[r] = __viaddmin_s16x2(v, 0x7bff7bffu, low[r]);
+            };
             if (it.bucket >= 0 && it.bucket < a.E) {
                 int64_t at[4];
 #pragma unroll
@@ -353,20 +404,19 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                             mv[r] = __ldg(reinterpret_cast<const uint4 *>(a.minv + at[r] + g));
                         }
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const uint32_t sw[4] = {sv[r].x, sv[r].y, sv[r].z, sv[r].w}, mw[4] = {mv[r].x, mv[r].y, mv[r].z, mv[r].w};
-#pragma unroll
-                            for (int c = 0; c < 4; ++c)
-                                smax[r] = __vmaxu2(smax[r], sw[c] & 0x7fff7fffu), mmax[r] = __vmaxu2(mmax[r], mw[c] & 0x7fff7fffu);
-                        }
+                        for (int r = 0; r < 4; ++r)
+                            take(r, sv[r].x, mv[r].x), take(r, sv[r].y, mv[r].y), take(r, sv[r].z, mv[r].z), take(r, sv[r].w, mv[r].w);
                     }
+                } else if (pair_scales) {
+#pragma unroll 2
+                    for (int g = 0; g < groups; g += 2)
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            take(r, __ldg(reinterpret_cast<const uint32_t *>(a.scale + at[r] + g)), __ldg(reinterpret_cast<const uint32_t *>(a.minv + at[r] + g)));
                 } else {
                     for (int g = 0; g < groups; ++g)
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            smax[r] = max(smax[r], (uint32_t)__ldg(a.scale + at[r] + g) & 0x7fffu);
-                            mmax[r] = max(mmax[r], (uint32_t)__ldg(a.minv + at[r] + g) & 0x7fffu);
-                        }
+                        for (int r = 0; r < 4; ++r) take(r, __ldg(a.scale + at[r] + g), __ldg(a.minv + at[r] + g));
                 }
             }
             if (i >= kItemRing) {
@@ -378,11 +428,12 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
             }
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                // exponent e of the largest scale, or of the largest min less 8 where that is more: 2^(14 - e) takes every scale
-                // below 2^15 and every min, after its further 2^-24, below 1/2
-                const int es = (int)(max(smax[r] >> 16, smax[r] & 0xffffu) >> 7), em = (int)(max(mmax[r] >> 16, mmax[r] & 0xffffu) >> 7) - 8;
-                const int e = min(max(max(es, em), 127 - 24), 127 + 15);
-                row_scale[i % kItemRing][r * 32 + lane] = __int_as_float((127 + 14 + 127 - e) << 23);
+                // e: the exponent of the row's largest scale (or min less 8), kept where 2^(14 - e) is a float; that power takes every
+                // scale below 2^15 and every min, after its further 2^-24, below 1/2.  e_low: the smallest group's.
+                const int hi = (int)max(top[r] >> 16, top[r] & 0xffffu), lo = min((int)low[r] >> 16, (int)(int16_t)low[r]);
+                const int e = min(max((hi >> 7) - 8, 127 - 24), 127 + 15), e_low = (((lo - 0x7bff) & 0xffff) >> 7) - 8;
+                const bool spread = __any_sync(0xffffffffu, e > 127 - 10 && lo != 0x7fff && e_low < e - kScaleSpread);
+                row_scale[i % kItemRing][r * 32 + lane] = spread ? kNatural : __int_as_float((127 + 14 + 127 - e) << 23);
             }
             if (lane == 0) item_ring[i % kItemRing] = it;
             __syncwarp();

@@ -228,6 +228,39 @@ def test_dense_tcgen05_partial_row_blocks(cuda, oracle, bits, G, M, N, K):
     assert torch.equal(ybf, y32[:M].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("spread", [0, 6, 7, 9, 12])
+@pytest.mark.parametrize("bits,G,K", [(4, 128, 1024), (8, 64, 1024), (4, 32, 384), (8, 128, 640)])
+def test_dense_tcgen05_spread_scales(cuda, oracle, bits, G, K, spread):
+    """Rows whose groups' scales lie up to 2^spread apart, against activations that meet the small groups only (large weight
+    columns and small activations, as activation-scaling quantizers make them).  Row blocks of every kind: all rows spread, one
+    row of a block, rows of small weights throughout, a constant group, an all-zero group.  The dots are no further from 64 bits than
+    with every weight rounded once to F16 at its natural magnitude (2e-6: FP32 sums)."""
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(bits + K + spread)
+    N, M = 400, 40
+    W = random_weights(rng, N, K)
+    W[:128, K // 2:] *= 2.0 ** spread
+    W[130, K // 2:] *= 2.0 ** spread
+    W[256:384] *= 2.0 ** -spread
+    W[256:384, K // 2:] *= 2.0 ** spread
+    W[3, :G], W[4, :G], W[131, :G] = 0.0, 0.01, 0.0
+    wq = oracle.quantize(W, G, bits)
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    x[:, K // 2:] = 0.0
+    xb = oracle.f32_to_bf16(x)
+    y = torch.empty((M, N), dtype=torch.float32, device=cuda)
+    Kn.linear_qw_wmma(bf16_tensor(xb, cuda), upload(wq, cuda), y, M, Kn.Act.BF16, Kn.Act.F32)
+    torch.cuda.synchronize()
+    Kn.check_dense_status("spread scales")
+    exact = oracle.bf16_to_f32(xb).astype(np.float64) @ oracle.affine_weights(wq).T
+    natural = oracle.linear_q(xb, wq, out_act=oracle.F32, w_f16=True)
+    got = y.cpu().numpy()
+    for lo, hi in ((0, 128), (128, 256), (256, 384), (384, 400)):
+        size = np.linalg.norm(exact[:, lo:hi])
+        off, off_natural = (np.linalg.norm(v[:, lo:hi] - exact[:, lo:hi]) / size for v in (got, natural))
+        assert off <= 1.05 * off_natural + 2e-6, (lo, hi, off, off_natural)
+
+
 @pytest.mark.parametrize("bits,G", [(4, 128), (8, 64)])
 def test_fp32_activations(cuda, oracle, bits, G):
     """Act::F32 into the dense, per-slot and grouped entry points (kernels/linear_q4.hpp:26-30): FP32 in, FP32 out,
