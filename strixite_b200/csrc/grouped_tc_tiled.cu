@@ -93,7 +93,7 @@ struct Item {
 // last place of an F16 subnormal, 2^-24.  A quadrant of an item with a row spread wider - columns that a quantizer scaled up on
 // purpose - takes its weights at their natural magnitude (dequant_q4_word), unless the common power makes them no smaller than that
 // (scales below 2^-9).  Error of the small columns' dots against 64 bits, Q4, groups 2^7 / 2^10 / 2^12 apart: 5.6e-4 / 9.2e-3 /
-// 3.4e-2 with the common power of two, 2e-5 at any distance without.  The test for it costs gate/up at 777 tokens 553 -> 560 us.
+// 3.4e-2 with the common power of two, 2e-5 at any distance without.
 constexpr int kScaleSpread = 6;
 
 template <int MODE>
@@ -122,10 +122,10 @@ __device__ inline uint16_t pick16(const uint4 &v, int g) {
 }
 
 // A producer lane's step of a quadrant at natural magnitude (kScaleSpread): its row's codes at `src` of shared memory (16-byte chunks
-// swizzled by sw) with the groups from g0 on of s and m -> tensor memory.  A call: rare, and inlined its registers would be the
-// common step's.
+// swizzled by sw) with the groups from g0 on of s and m -> tensor memory.  Rare, so it is short rather than fast: a quarter at a time,
+// read again from shared memory (as a call, or unrolled, it cost the common step registers: 2000 x 8192 x 4096 Q8 133 us, not 129).
 template <int BITS, int G>
-__device__ __noinline__ void natural_step(uint32_t src, uint32_t sw, uint32_t a_addr, uint4 s, uint4 m, int g0) {
+__device__ __forceinline__ void natural_step(uint32_t src, uint32_t sw, uint32_t a_addr, uint4 s, uint4 m, int g0) {
     constexpr int kChunkCodes = BITS == 4 ? 32 : 16, kChunks = 32 / kChunkCodes;
 #pragma unroll 1
     for (int hc = 0; hc < 4; ++hc) {
