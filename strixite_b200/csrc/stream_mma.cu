@@ -17,8 +17,12 @@
 //     integer pipe, four bytes two byte permutes, and a packed multiply by a power of two makes a pair of normal numbers.
 //     (With BF16 operands, whose seven mantissa bits hold a nibble in one place only, a pair took a shift and a lop3, and a
 //     Q8 code the pairs of its two nibbles.)  The activations come as F16 too, each token's times the power of two that takes
-//     its largest magnitude to 2^15 .. 2^16: BF16's eight significant bits survive for everything within 2^-32 of the largest,
-//     and what lies below is rounded at 2^-40 of it, far under the rounding of an FP32 sum that contains it;
+//     its largest magnitude to 2^15 .. 2^16: everything down to 2^-29 of the largest is a normal F16, BF16's eight significant
+//     bits exactly.  What is smaller is rounded at 2^-40 of the largest, which shows where the large values meet weights of exactly
+//     zero (code and min) and the small ones are the dot.  Q8 keeps those: they are left out of the F16 operand and added to the
+//     finished dots in FP32, and a token with more than kLowMax of them takes BF16 operands, codes and all (rows_dot_wide).  Q4
+//     has no such form (it costs 1.5 to 3 % of a decode step): it rounds at 2^-40, where its codes as BF16 pairs 16 + n, with 16
+//     sum(x) taken off again, lost what lay below 2^-24;
 //   * the activations of the tile's <= 8 tokens sit in shared memory already permuted into `mma.m16n8k16` B-fragment
 //     order, so a lane fetches its fragments with conflict-free 16-byte loads; k is permuted consistently on both
 //     operands, which a dot product does not notice;
@@ -122,6 +126,31 @@ __device__ inline void unit_mma(float (&d)[4], uint32_t a_w0, uint32_t a_w1, uin
 
 __device__ inline float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // e in -126 .. 127
 
+__device__ inline void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// What stage_tile finds out about a token of the tile.
+template <int BITS> constexpr bool kKeepLow = BITS == 8;  // see the head of this file
+constexpr int kLowMax = 4;
+struct Low {
+    int k;
+    float x;
+};
+struct Token {
+    uint32_t top;  // largest magnitude of its activations, BF16 bits
+    int low;       // the smallest that is not zero, as a signed 16-bit value with 0x7fff added (0x7fff: all are zero)
+    int exp;       // e of the power 2^e that its dots carry beside the codes' 2^-9 (unscaled); 9 = none
+    int n_low;     // activations too small for F16 beside the largest; more than kLowMax: the token is staged as BF16
+    int n_list[2];  // the first kLowMax of them at most, ascending k, by each of the (one or two) warps that stage the token
+    Low list[2][kLowMax];
+};
+__device__ inline void clear_token(Token &t) { t.top = 0u, t.low = 0x7fff, t.exp = 9, t.n_low = 0, t.n_list[0] = t.n_list[1] = 0; }
+__device__ inline bool too_small(float scaled) { return fabsf(scaled) < 0x1p-14f; }
+
 // The exponent e of a token's scale 2^e from the largest magnitude of its activations (BF16 bits without the sign): 2^15 <= max
 // * 2^e < 65504, where the clamp to exponents that FP32 can hold allows it.
 __device__ inline int token_exponent(uint32_t max_bits) { return min(max(142 - (int)(max_bits >> 7), -112), 126); }
@@ -174,10 +203,11 @@ __device__ inline void tree_push(float4 *level, int i, float (&v)[4]) {
 template <typename T> __device__ inline void store_out(T *p, int64_t i, float v) { store_from_f32(p, i, v); }
 
 // Stages up to 8 activation rows (rows[n] < 0 = none) as F16 in fragment order at xs, every row times its power of two
-// 2^e (token_exponent; max_bits[n] comes in as zero and leaves as the row's largest magnitude), and at xsum the sums of every
-// (step, token) times 2^(e - 9), the factor that the dots with the codes carry.  All threads of the CTA.
+// 2^e (token_exponent), and at xsum the sums of every (step, token) times 2^(e - 9), the factor that the dots with the codes carry.
+// kKeepLow: activations that would be subnormal are staged as zeros and listed in tok[n], which comes in cleared; *any_low = 1 where
+// there are any.  All threads of the CTA; the caller synchronizes before it reads those.
 template <int BITS, int G>
-__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, uint32_t *max_bits) {
+__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok, int *any_low) {
     using geo = Geo<BITS, G>;
     constexpr int UNITS = geo::kUnits, KI = geo::kStepCodes, CPL = geo::kCodesPerLane;
     constexpr int kStepLanes = KI / 8;  // lanes that hold one step of one token: 4, 8 or 16
@@ -195,7 +225,7 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
         for (int j = 0; j < kBatch; ++j)
             if (base + j * stride < units) v[j] = src[base + j * stride];
     };
-    uint32_t top = 0u;
+    uint32_t top = 0u, low2 = 0x7fff7fffu;
     if (row >= 0) {
         // sum(x) of every step: eight values a lane, then a butterfly over the step's lanes
         for (int base = share * 32 + lane; base - lane < units; base += kBatch * stride) {
@@ -210,7 +240,9 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         sum += __uint_as_float(w4[i] << 16), sum += __uint_as_float(w4[i] & 0xffff0000u);
-                        top = __vmaxu2(top, w4[i] & 0x7fff7fffu);
+                        const uint32_t mag = w4[i] & 0x7fff7fffu;
+                        top = __vmaxu2(top, mag);
+                        if (kKeepLow<BITS>) low2 = __viaddmin_s16x2(mag, 0x7fff7fffu, low2);
                     }
                 }
 #pragma unroll
@@ -219,13 +251,47 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             }
         }
         top = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xffffu));
-        if (lane == 0) atomicMax(&max_bits[n], top);
+        if (lane == 0) atomicMax(&tok[n].top, top);
+        if (kKeepLow<BITS>) {
+            const int low = __reduce_min_sync(0xffffffffu, min((int)low2 >> 16, (int)(int16_t)low2));
+            if (lane == 0) atomicMin(&tok[n].low, low);
+        }
     }
     __syncthreads();
     // absent tokens' columns keep whatever the memory held: a column of the products depends on its own token only, and theirs
     // are dropped
     if (row < 0) return;
-    const float f = pow2f(token_exponent(max_bits[n]));
+    const int e = token_exponent(tok[n].top), smallest = kKeepLow<BITS> ? tok[n].low : 0x7fff;
+    const float f = pow2f(e);
+    const bool low = smallest != 0x7fff && too_small(__uint_as_float((uint32_t)((smallest - 0x7fff) & 0xffff) << 16) * f);
+    if (lane == 0 && share == 0) tok[n].exp = e;
+    if (low) {
+        int found = 0;
+        for (int first = share * 32; first < units; first += stride) {
+            const int u = first + lane;
+            const uint4 q = u < units ? src[u] : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+            uint32_t mine = 0u;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float x = __uint_as_float((i & 1) ? w4[i >> 1] & 0xffff0000u : w4[i >> 1] << 16);
+                if (x != 0.f && too_small(x * f)) mine |= 1u << i;
+            }
+            for (uint32_t who = __ballot_sync(0xffffffffu, mine != 0u); who != 0u; who &= who - 1) {
+                const int l = __ffs(who) - 1;
+                const uint32_t theirs = __shfl_sync(0xffffffffu, mine, l);
+                if (lane == l) {
+                    int at = found;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (((mine >> i) & 1u) && at < kLowMax)
+                            tok[n].list[share][at++] = Low{u * 8 + i, __uint_as_float((i & 1) ? w4[i >> 1] & 0xffff0000u : w4[i >> 1] << 16)};
+                }
+                found += __popc(theirs);
+            }
+        }
+        if (lane == 0 && found > 0) tok[n].n_list[share] = min(found, kLowMax), atomicAdd(&tok[n].n_low, found), *any_low = 1;
+    }
     // One batch holds the row up to 4096 k at 512 threads; a longer one is read again.
     const bool held = units <= kBatch * stride;
     for (int base = share * 32 + lane; base < units; base += kBatch * stride) {
@@ -241,6 +307,10 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
 #pragma unroll
             for (int i = 0; i < 4; ++i) lo[i] = __uint_as_float(w4[i] << 16) * f, hi[i] = __uint_as_float(w4[i] & 0xffff0000u) * f;
             auto pack = [](float a, float b) { const __half2 h = __floats2half2_rn(a, b); return *reinterpret_cast<const uint32_t *>(&h); };
+            if (low) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) lo[i] = too_small(lo[i]) ? 0.f : lo[i], hi[i] = too_small(hi[i]) ? 0.f : hi[i];
+            }
             uint4 dst;
             if (BITS == 4) {  // [x0 x4 | x1 x5 | x2 x6 | x3 x7]
                 dst.x = pack(lo[0], lo[2]), dst.y = pack(hi[0], hi[2]), dst.z = pack(lo[1], lo[3]), dst.w = pack(hi[1], hi[3]);
@@ -250,6 +320,91 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             xs[(step * UNITS + part) * 32 + n * 4 + cc] = dst;
         }
     }
+}
+
+// Stages the tile's tokens with more than kLowMax small activations again, as BF16 in natural order, and their sums as they are.
+template <int BITS, int G>
+__device__ __noinline__ void stage_wide(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok) {
+    using geo = Geo<BITS, G>;
+    constexpr int KI = geo::kStepCodes;
+    for (int n = 0; n < kTileTokens; ++n) {
+        if (tok[n].n_low <= kLowMax) continue;
+        const uint4 *src = reinterpret_cast<const uint4 *>(x + rows[n] * K);
+        if (threadIdx.x == 0) tok[n].exp = 9;
+        for (int u = threadIdx.x; u < K / 8; u += blockDim.x) {
+            const int step = u * 8 / KI, rem = u * 8 % KI;
+            xs[(step * geo::kUnits + rem % geo::kCodesPerLane / 8) * 32 + n * 4 + rem / geo::kCodesPerLane] = src[u];
+        }
+        for (int step = threadIdx.x; step < K / KI; step += blockDim.x) {
+            float sum = 0.f;
+            for (int i = 0; i < KI; ++i) sum += bf16_bits_to_f32(x[rows[n] * K + (int64_t)step * KI + i]);
+            xsum[step * kTileTokens + n] = sum;
+        }
+    }
+}
+// After stage_tile and a barrier, where some token has small activations.
+template <int BITS, int G>
+__device__ inline void finish_staging(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok) {
+    bool again = false;
+    for (int n = 0; n < kTileTokens; ++n) again = again || tok[n].n_low > kLowMax;
+    if (again) stage_wide<BITS, G>(x, K, rows, xs, xsum, tok);
+    __syncthreads();
+}
+
+// What a token's listed activations add to its dot with weight row `row`, in ascending k (the mins' part is in xsum).
+template <int BITS, int G>
+__device__ __noinline__ float low_dot(const uint8_t *q, const uint16_t *scale, int K, int64_t row, const Token &tok) {
+    float sum = 0.f;
+    for (int i = 0, j = 0; i < tok.n_list[0] || j < tok.n_list[1];) {
+        const bool first = j >= tok.n_list[1] || (i < tok.n_list[0] && tok.list[0][i].k < tok.list[1][j].k);
+        const Low l = first ? tok.list[0][i++] : tok.list[1][j++];
+        const uint8_t byte = BITS == 4 ? q[row * (K / 2) + l.k / 2] : q[row * K + l.k];
+        const int code = BITS == 4 ? (byte >> (4 * (l.k & 1))) & 15 : byte;
+        sum = fmaf(bf16_bits_to_f32(scale[row * (K / G) + l.k / G]), (float)code * l.x, sum);
+    }
+    return sum;
+}
+
+// The dots of weight rows rowa / rowb with the tokens that are staged as BF16 (the other tokens' sums are meaningless): codes as BF16
+// too, exact products at any distance.  acc as below.  The whole contraction in order, whatever warps share it otherwise; rare, so
+// short rather than fast.
+template <int BITS, int G>
+__device__ __noinline__ float4 rows_dot_wide(const uint8_t *q, const uint16_t *scale, const uint16_t *minv, int K, int64_t rowa, int64_t rowb,
+                                             bool va, bool vb, const uint4 *xs, const float *xsum) {
+    using geo = Geo<BITS, G>;
+    constexpr int W = geo::kWords;
+    const int lane = threadIdx.x & 31, c = lane & 3, steps = K / geo::kStepCodes, groups = K / G;
+    const int64_t row_bytes = BITS == 4 ? K / 2 : K;
+    const uint8_t *pa = q + rowa * row_bytes + c * geo::kLoadBytes, *pb = q + rowb * row_bytes + c * geo::kLoadBytes;
+    auto pair = [](uint32_t w0, uint32_t w1, int i) -> uint32_t {  // codes 2 i and 2 i + 1 of eight
+        const uint32_t w = BITS == 4 || i < 2 ? w0 : w1;
+        const uint32_t lo = BITS == 4 ? (w >> (8 * i)) & 15u : (w >> (16 * (i & 1))) & 255u;
+        const uint32_t hi = BITS == 4 ? (w >> (8 * i + 4)) & 15u : (w >> (16 * (i & 1) + 8)) & 255u;
+        const __nv_bfloat162 p = __floats2bfloat162_rn((float)lo, (float)hi);  // eight significant bits: exact
+        return *reinterpret_cast<const uint32_t *>(&p);
+    };
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int step = 0; step < steps; ++step) {
+        uint32_t wa[W], wb[W];
+        load_codes<W>(wa, pa + (int64_t)step * 4 * geo::kLoadBytes, va);
+        load_codes<W>(wb, pb + (int64_t)step * 4 * geo::kLoadBytes, vb);
+        const int64_t ga = rowa * groups + step / geo::kStepsPerGroup, gb = rowb * groups + step / geo::kStepsPerGroup;
+        const float s_a = va ? bf16_bits_to_f32(__ldg(scale + ga)) : 0.f, m_a = va ? bf16_bits_to_f32(__ldg(minv + ga)) : 0.f;
+        const float s_b = vb ? bf16_bits_to_f32(__ldg(scale + gb)) : 0.f, m_b = vb ? bf16_bits_to_f32(__ldg(minv + gb)) : 0.f;
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int v = 0; v < geo::kUnits; ++v) {
+            const uint4 bx = xs[(step * geo::kUnits + v) * 32 + lane];
+            const int i0 = BITS == 4 ? v : 2 * v, i1 = BITS == 4 ? v : 2 * v + 1;
+            mma_bf16(d, pair(wa[i0], wa[i1], 0), pair(wb[i0], wb[i1], 0), pair(wa[i0], wa[i1], 1), pair(wb[i0], wb[i1], 1), bx.x, bx.y);
+            mma_bf16(d, pair(wa[i0], wa[i1], 2), pair(wb[i0], wb[i1], 2), pair(wa[i0], wa[i1], 3), pair(wb[i0], wb[i1], 3), bx.z, bx.w);
+        }
+        const float2 xs2 = *reinterpret_cast<const float2 *>(xsum + step * kTileTokens + 2 * c);
+        acc.x = fmaf(s_a, d[0], fmaf(m_a, xs2.x, acc.x)), acc.y = fmaf(s_a, d[1], fmaf(m_a, xs2.y, acc.y));
+        acc.z = fmaf(s_b, d[2], fmaf(m_b, xs2.x, acc.z)), acc.w = fmaf(s_b, d[3], fmaf(m_b, xs2.y, acc.w));
+    }
+    return acc;
 }
 
 // One warp: the dots of weight rows rowa / rowb (lane quad g streams both) with the staged tokens.
@@ -407,7 +562,8 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
     const size_t pass_bytes = (size_t)steps * geo::kUnits * 512 + (size_t)steps * kTileTokens * 4;
     __shared__ int64_t s_row[kTileTokens];  // activation row of each token of the tile, -1 = none
     __shared__ int64_t s_out[kTileTokens];  // output row (slot, or token for dense)
-    __shared__ uint32_t s_max[kPerTokenPasses][kTileTokens];  // largest magnitude of each token's activations (stage_tile)
+    __shared__ Token s_tok[SRC == kPerToken ? kPerTokenPasses : 1][kTileTokens];
+    __shared__ int s_low[SRC == kPerToken ? kPerTokenPasses : 1];  // some token of the tile has activations too small for F16
     __shared__ int s_bucket, s_cnt;
     __shared__ int s_next;  // the next unit of the CTA's run that no warp has taken yet
     constexpr bool kTree = SRC == kDense;
@@ -465,11 +621,16 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 if (threadIdx.x < kTileTokens) {
                     const int k = p * kTileTokens + threadIdx.x;
                     s_row[threadIdx.x] = k < a.A ? m * a.A + k : -1;
-                    s_max[p][threadIdx.x] = 0u;
+                    clear_token(s_tok[p][threadIdx.x]);
+                    if (threadIdx.x == 0) s_low[p] = 0;
                 }
                 __syncthreads();
                 stage_tile<BITS, G>(a.x, K, s_row, reinterpret_cast<uint4 *>(smem + p * pass_bytes),
-                                    reinterpret_cast<float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512), s_max[p]);
+                                    reinterpret_cast<float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512), s_tok[p], &s_low[p]);
+                __syncthreads();
+                if (kKeepLow<BITS> && s_low[p])
+                    finish_staging<BITS, G>(a.x, K, s_row, reinterpret_cast<uint4 *>(smem + p * pass_bytes),
+                                            reinterpret_cast<float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512), s_tok[p]);
             }
             __syncthreads();
             for (int64_t unit = lo + warp; unit < hi; unit += kWarps) {
@@ -481,14 +642,24 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                     const int p = k / kTileTokens, col = k % kTileTokens;
                     const int64_t base = (int64_t)a.ids[m * a.A + k] * a.N;
                     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-                    rows_dot<BITS, G, false>(acc, a, base + ra, base + rb, va, vb, reinterpret_cast<const uint4 *>(smem + p * pass_bytes),
-                                      reinterpret_cast<const float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512),
-                                      lane, 0, nullptr);
+                    const uint4 *xs = reinterpret_cast<const uint4 *>(smem + p * pass_bytes);
+                    const float *xsum = reinterpret_cast<const float *>(smem + p * pass_bytes + (size_t)steps * geo::kUnits * 512);
+                    const Token &tok = s_tok[p][col];
+                    if (kKeepLow<BITS> && tok.n_low > kLowMax) {
+                        const float4 w = rows_dot_wide<BITS, G>(a.q, a.scale, a.minv, K, base + ra, base + rb, va, vb, xs, xsum);
+                        acc[0] = w.x, acc[1] = w.y, acc[2] = w.z, acc[3] = w.w;
+                    } else {
+                        rows_dot<BITS, G, false>(acc, a, base + ra, base + rb, va, vb, xs, xsum, lane, 0, nullptr);
+                    }
                     if (c == col / 2) {  // the lane of the quad that holds this slot's column
                         const float cf = a.coef[m * a.A + k];
-                        const int e = token_exponent(s_max[p][col]);
-                        ta = fmaf(cf, unscaled(col & 1 ? acc[1] : acc[0], e), ta);
-                        tb = fmaf(cf, unscaled(col & 1 ? acc[3] : acc[2], e), tb);
+                        float da = unscaled(col & 1 ? acc[1] : acc[0], tok.exp), db = unscaled(col & 1 ? acc[3] : acc[2], tok.exp);
+                        if (kKeepLow<BITS> && tok.n_low > 0 && tok.n_low <= kLowMax) {
+                            if (va) da += low_dot<BITS, G>(a.q, a.scale, K, base + ra, tok);
+                            if (vb) db += low_dot<BITS, G>(a.q, a.scale, K, base + rb, tok);
+                        }
+                        ta = fmaf(cf, da, ta);
+                        tb = fmaf(cf, db, tb);
                     }
                 }
                 // the four lanes of a quad hold the partial sums of slots {0,1}, {2,3}, {4,5}, {6,7} (mod 8)
@@ -528,7 +699,8 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 if (n == 0) s_bucket = 0, s_cnt = (int)min((int64_t)kTileTokens, a.M - tile * kTileTokens);
                 if (m < a.M) row = orow = m;
             }
-            s_row[n] = row, s_out[n] = orow, s_max[0][n] = 0u;
+            s_row[n] = row, s_out[n] = orow, clear_token(s_tok[0][n]);
+            if (n == 0) s_low[0] = 0;
         }
         __syncthreads();
         const int bucket = s_bucket, cnt = s_cnt;
@@ -559,9 +731,10 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 if (vb) asm volatile("prefetch.global.L2 [%0];" ::"l"(base + rb * row_bytes + at));
             }
         }
-        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum, s_max[0]);
+        if (valid) stage_tile<BITS, G>(a.x, K, s_row, xs, xsum, s_tok[0], &s_low[0]);
         if (threadIdx.x == 0) s_next = 0;
         __syncthreads();
+        if (kKeepLow<BITS> && s_low[0]) finish_staging<BITS, G>(a.x, K, s_row, xs, xsum, s_tok[0]);
 
         // split == 1: warps take units on demand.  Two warps of an SM do not stream at the same rate (measured: the units of one
         // of two co-resident CTAs took 2.5 times as long as the other's while both were alive), and a fixed deal leaves the
@@ -598,14 +771,28 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 group_sync();
                 if (part != 0) continue;
             }
+            const int64_t row0 = (int64_t)bucket * a.N;
+            const bool any_low = kKeepLow<BITS> && valid && s_low[0] != 0;
+            if (any_low) {
+                bool wide[2] = {s_tok[0][2 * c].n_low > kLowMax, s_tok[0][2 * c + 1].n_low > kLowMax};
+                if (__any_sync(0xffffffffu, wide[0] || wide[1])) {
+                    const float4 w = rows_dot_wide<BITS, G>(a.q, a.scale, a.minv, K, row0 + ra, row0 + rb, va, vb, xs, xsum);
+                    if (wide[0]) acc[0] = w.x, acc[2] = w.z;
+                    if (wide[1]) acc[1] = w.y, acc[3] = w.w;
+                }
+            }
             // Epilogue.  Lane (g, c) holds rows ra / rb for tokens 2c and 2c + 1.
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
                 const int n = 2 * c + t;
                 if (n >= cnt) continue;
                 const int64_t orow = s_out[n];
-                const int e = token_exponent(s_max[0][n]);
-                const float dot_a = unscaled(acc[t], e), dot_b = unscaled(acc[2 + t], e);
+                const Token &tok = s_tok[0][n];
+                float dot_a = unscaled(acc[t], tok.exp), dot_b = unscaled(acc[2 + t], tok.exp);
+                if (any_low && tok.n_low > 0 && tok.n_low <= kLowMax) {
+                    if (va) dot_a += low_dot<BITS, G>(a.q, a.scale, K, row0 + ra, tok);
+                    if (vb) dot_b += low_dot<BITS, G>(a.q, a.scale, K, row0 + rb, tok);
+                }
                 if (MODE == kSwiglu) {
                     if (!va) continue;
                     // kernels/linear_q4.hip:272-274: g, u as stored, h = stored(stored(silu(g)) * u)

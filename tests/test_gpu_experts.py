@@ -96,6 +96,72 @@ def test_linear_activation_range(cuda, oracle, bits, G, Kd):
     assert np.all(np.abs(got[:10] - want) <= bound), np.max(np.abs(got[:10] - want) / bound, axis=1)
 
 
+@pytest.mark.parametrize("far", [28, 31, 40, 80])
+@pytest.mark.parametrize("bits,G,Kd", [(8, 64, 1024), (8, 128, 384), (8, 32, 160)])
+def test_large_activation_against_zero_weights(cuda, oracle, bits, G, Kd, far):
+    """A token's largest value, 2^far times the others, meets weights that are exactly zero (code 0, min 0): the dot is that of the
+    small values, and none of their bits may go.  Dense (a unit shared between warps, and not), grouped and per-slot forms; the
+    tokens beside it in its tile give the same bits as without it.  Bound: FP32 sums in absolute values, as in
+    test_linear_activation_range."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(Kd + bits + far)
+    N, E, M, A, at = 4832, 8, 40, 4, 34
+    w = oracle.quantize(np.abs(random_weights(rng, N, Kd)), G, bits)
+    w.minv[:, at // G], w.q[:, at] = 0, 0
+    x = rng.standard_normal((M, Kd)).astype(np.float32)
+    plain = oracle.f32_to_bf16(x)
+    x[::3, at] = 2.0 ** far
+    x[6, np.arange(Kd) % 37 != 5] = 0.0  # a few small values only
+    x[6, at] = 2.0 ** far
+    xb = oracle.f32_to_bf16(x)
+    wd, xd, pd = upload(w, cuda), bf16_tensor(xb, cuda), bf16_tensor(plain, cuda)
+    s, m = (np.repeat(oracle.bf16_to_f32(v).astype(np.float64).reshape(N, Kd // G), G, axis=1) for v in (w.scale, w.minv))
+    xf, affine, size = oracle.bf16_to_f32(xb).astype(np.float64), oracle.affine_weights(w), oracle.codes_of(w) * np.abs(s) + np.abs(m)
+    want, bound = xf @ affine.T, (Kd / 8 + 3 * Kd / G + 4) * 2.0 ** -23 * (np.abs(xf) @ size.T) + 2.0 ** -149
+    others = [t for t in range(M) if t % 3]
+
+    def check(got, cols, what, plain_got):
+        assert np.all(np.abs(got.astype(np.float64) - want[:, :cols]) <= bound[:, :cols]), what
+        assert np.array_equal(got[others], plain_got[others]), what
+
+    for cols in (24, N):
+        y, yp = (torch.empty((M, cols), dtype=torch.float32, device=cuda) for _ in range(2))
+        K.linear_qw(xd, wd.rows(0, cols), y, M, K.Act.BF16, out_act=K.Act.F32)
+        K.linear_qw(pd, wd.rows(0, cols), yp, M, K.Act.BF16, out_act=K.Act.F32)
+        torch.cuda.synchronize()
+        check(y.cpu().numpy(), cols, f"dense {cols}", yp.cpu().numpy())
+    # experts: the rows [E, N / E] of the same weight; every slot of token t holds x[t], so the combines' dots are x @ w^T again
+    n = N // E
+    ids = np.stack([rng.permutation(E)[:A] for _ in range(M)]).astype(np.int32)
+    idd = torch.from_numpy(ids).to(cuda)
+    one = torch.zeros((M, A), dtype=torch.float32, device=cuda)
+    one[:, 1] = 1.0
+    err = torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = K.moe_route_workspace_bytes(M, A, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    K.moe_group_routes(idd, M, A, E, ws, nbytes, err)
+    partial = torch.empty((M * A, n), dtype=torch.float32, device=cuda)
+    rows = ids[:, 1, None] * n + np.arange(n)  # the weight rows of slot 1
+    want, bound = np.take_along_axis(want, rows, 1), np.take_along_axis(bound, rows, 1)
+    got = {}
+    for src in (xd, pd):
+        h = src[:, None].expand(M, A, Kd).contiguous()
+        y1, y2 = (torch.empty((M, n), dtype=torch.float32, device=cuda) for _ in range(2))
+        K.linear_qw_experts_combine(h, wd, E, idd, one, M, A, y1, K.Act.BF16, err, out_act=K.Act.F32)
+        K.linear_qw_experts_combine_grouped(h.view(M * A, Kd), wd, E, idd, one, ws, nbytes, partial, M, A, y2, K.Act.BF16, K.MoeMath.F32,
+                                            out_act=K.Act.F32)
+        torch.cuda.synchronize()
+        for name, y in (("per slot", y1), ("grouped", y2)):
+            got.setdefault(name, []).append(y.cpu().numpy())
+    for name, (y, yp) in got.items():
+        check(y, n, name, yp)
+    g = torch.empty((M * A, n), dtype=torch.bfloat16, device=cuda)
+    K.linear_qw_experts_gather_grouped(xd, wd, E, ws, nbytes, M, A, g, K.Act.BF16, K.MoeMath.F32)
+    torch.cuda.synchronize()
+    assert torch.equal(g.view(M, A, n)[:, 1], torch.from_numpy(got["grouped"][0]).to(cuda).to(torch.bfloat16))
+    assert int(err[0]) == 0
+
+
 @pytest.mark.parametrize("bits,G,Kd", [(4, 128, 1024), (4, 128, 2048), (8, 64, 2048), (8, 64, 640)])
 def test_linear_row_does_not_depend_on_launch(cuda, oracle, bits, G, Kd):
     """One warp a unit of 16 rows, or two, four or eight, by the launch's size: a token's row is the same, bit for bit, alone, in
