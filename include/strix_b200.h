@@ -14,9 +14,13 @@
  * every buffer - weights, activations, ids / coef, the grouping workspace, the combine's `partial`, the error
  * words.  Unless a declaration says otherwise, no entry point allocates, frees or synchronizes; all work is enqueued
  * on the caller's stream.  Exceptions: sxb_check_*_error (a blocking 12-byte copy, as the reference's), and the WMMA_F16
- * entries given row-major activations (BF16, or F16 other than SXB_ACT_F16_TILED): they write the tile-blocked form into
- * stream-ordered scratch of the library, which keeps at most 1 GiB of it per device between calls (sxb_release_scratch gives
- * that back).  The ..._noalloc entries never do.
+ * entries given row-major activations (BF16, or F16 other than SXB_ACT_F16_TILED): they write the tile-blocked form, two
+ * bytes an activation of every slot, into stream-ordered scratch of the library, which keeps at most 1 GiB of it per device
+ * between calls (sxb_release_scratch gives that back; a call that needs more returns the rest at the next synchronization).
+ * Without scratch - out of device memory, on a capturing stream, in the ..._noalloc entries - they read the activations as
+ * they are, several times slower (a 1200-token layer 11 ms, not 1.3), and a weight's one rounding to F16 may fall elsewhere
+ * where it is subnormal (|w| < 2^-14), so the two ways may differ in the last bits there.  A graph that wants the speed
+ * stages its activations itself: sxb_stage_f16_tiles into memory of its own, then SXB_ACT_F16_TILED.
  *
  * Error words (`err`): >= 3 zeroed uint32 on the device, zeroed by the caller at session start.  A data error on the
  * device sets err[0] = 1, err[1], err[2] (first writer wins), poisons the affected outputs with NaN and never reads

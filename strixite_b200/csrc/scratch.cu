@@ -40,6 +40,14 @@ cudaMemPool_t pool() {
 
 bool StreamScratch::get(size_t bytes, cudaStream_t stream) {
     if (g_refuse > 0 || p_ != nullptr) return false;
+    // Not under capture: the allocation would be a node of the graph, which then can no longer be cloned, be a child of another or
+    // have two executable instances, and whose memory is neither bounded by this pool nor given back by sxb_release_scratch.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return false;
     cudaMemPool_t from = pool();
     if (from == nullptr || cudaMallocFromPoolAsync(&p_, bytes, from, stream) != cudaSuccess) {
         p_ = nullptr;

@@ -3,8 +3,8 @@
 // until the work enqueued before its release has run.
 //
 // The memory comes from a pool of this library's own, one per device, through the runtime's stream-ordered allocator: an
-// allocation is ordered on the stream it is made on, so calls from several threads and streams never share live memory, and
-// it may be captured into a graph.  The pool keeps at most kKeepBytes between calls; what lies above that goes back to the
+// allocation is ordered on the stream it is made on, so calls from several threads and streams never share live memory.
+// A captured call gets none (scratch.cu).  The pool keeps at most kKeepBytes between calls; what lies above that goes back to the
 // device at the next synchronization, all of it with sxb_release_scratch.
 #pragma once
 
@@ -18,7 +18,7 @@ class StreamScratch {
     StreamScratch(const StreamScratch &) = delete;
     StreamScratch &operator=(const StreamScratch &) = delete;
     ~StreamScratch();  // enqueues the release on the stream of the allocation
-    // False when there is none to be had (out of memory, or inside a NoScratch): no error is left behind.
+    // False when there is none to be had (out of memory, a capturing stream, inside a NoScratch): no error is left behind.
     bool get(size_t bytes, cudaStream_t stream);
     void *ptr() const { return p_; }
 

@@ -28,3 +28,26 @@ def bf16_ulps(a_bits: np.ndarray, b_bits: np.ndarray) -> np.ndarray:
 
 def random_weights(rng, n, k, std=0.02):
     return (rng.standard_normal((n, k)) * std).astype(np.float32)
+
+
+def capture_calls(monkeypatch) -> list:
+    """From here on every call of the tensor-core launchers is a CUDA graph of its own, captured and replayed.  A captured call gets
+    no scratch, so row-major activations take the kernel that reads them as they are."""
+    from strixite_b200 import kernels as K
+    graphs = []
+
+    def replayed(fn):
+        def call(*args, **kw):
+            graph = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph):
+                fn(*args, **kw)
+            graph.replay()
+            torch.cuda.synchronize()
+            graphs.append(graph)
+        return call
+
+    for name in ("linear_qw_wmma", "linear_qw_wmma_swiglu", "linear_qw_experts_gather_grouped", "linear_qw_experts_gather_grouped_swiglu",
+                 "linear_qw_experts_combine_grouped"):
+        monkeypatch.setattr(K, name, replayed(getattr(K, name)))
+    return graphs

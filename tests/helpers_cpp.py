@@ -20,3 +20,11 @@ def build_call_block(out_dir: pathlib.Path) -> pathlib.Path:
                     str(ROOT / "tests" / "cpp" / "call_block.cpp"), "-o", str(exe), f"-L{lib_dir}", "-lstrix_b200",
                     f"-L{cuda / 'lib64'}", "-lcudart", f"-Wl,-rpath,{lib_dir}", f"-Wl,-rpath,{cuda / 'lib64'}"], check=True)
     return exe
+
+
+def build_scratch_fake(out_dir: pathlib.Path) -> pathlib.Path:
+    """tests/cpp/scratch_fake.cpp: csrc/scratch.cu with a fake of the runtime in place of the CUDA library."""
+    exe = pathlib.Path(out_dir) / "scratch_fake"
+    subprocess.run(["g++", "-std=c++17", "-x", "c++", "-w", f"-I{ROOT / 'include'}", f"-I{ROOT / 'strixite_b200' / 'csrc'}",
+                    f"-I{cuda_home() / 'include'}", str(ROOT / "tests" / "cpp" / "scratch_fake.cpp"), "-pthread", "-o", str(exe)], check=True)
+    return exe

@@ -50,6 +50,13 @@ def test_cxx_host_links_against_the_library(lib, tmp_path):
     assert exe.exists()
 
 
+def test_scratch_pool_against_a_fake_runtime(tmp_path):
+    """csrc/scratch.cu: no scratch (and no pool) for captured calls, a failed allocation leaves no error, one pool per device, memory freed on its stream, NoScratch per thread."""
+    from helpers_cpp import build_scratch_fake
+    res = subprocess.run([str(build_scratch_fake(tmp_path))], capture_output=True, text=True, timeout=60)
+    assert res.returncode == 0 and "FAIL" not in res.stdout, res.stdout + res.stderr
+
+
 def test_preconditions_fail_before_any_launch(lib):
     from strixite_b200 import kernels as K
     with pytest.raises(K.Error, match="null pointer"):

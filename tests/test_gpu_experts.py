@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bf16_tensor, bf16_ulps, bits_of, download, max_abs_over_rms, random_weights, upload
+from helpers import bf16_tensor, bf16_ulps, bits_of, capture_calls, download, max_abs_over_rms, random_weights, upload
 
 pytestmark = pytest.mark.gpu
 
@@ -459,3 +459,101 @@ def test_grouped_experts_tcgen05(cuda, oracle, bits, G, M, A, E, I, d):
         # a dot on a BF16 rounding boundary falls either way (one ulp = 2^-8 of the dot, times its coefficient): over M * d
         # outputs the largest such flip reaches ~1e-2 of the RMS, which is why this library's default keeps the dots in FP32
         assert max_abs_over_rms(yb.cpu().numpy()[rows], y_ref_b[rows]) < 2e-2
+
+
+@pytest.mark.parametrize("bits,G", [(4, 128), (8, 64), (4, 32)])
+@pytest.mark.parametrize("M,A,E,I,d", [(40, 2, 4, 128, 256), (300, 2, 8, 128, 256)])
+def test_grouped_experts_tcgen05_captured(cuda, oracle, monkeypatch, bits, G, M, A, E, I, d):
+    """All grouped forms (gather, SwiGLU, per-slot dots; BF16, F16 and staged activations; an invalid id) without scratch."""
+    capture_calls(monkeypatch)
+    test_grouped_experts_tcgen05(cuda, oracle, bits, G, M, A, E, I, d)
+
+
+def node_types(graph):
+    """The CUgraphNodeType of every node of a captured graph."""
+    import ctypes as C
+    drv, n = C.CDLL("libcuda.so.1"), C.c_size_t()
+    g = C.c_void_p(graph.raw_cuda_graph())
+    assert drv.cuGraphGetNodes(g, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert drv.cuGraphGetNodes(g, nodes, C.byref(n)) == 0
+    types = []
+    for node in nodes:
+        t = C.c_int()
+        assert drv.cuGraphNodeGetType(C.c_void_p(node), C.byref(t)) == 0
+        types.append(t.value)
+    return types
+
+
+def test_captured_calls_allocate_nothing(cuda, oracle):
+    """A graph of row-major tensor-core calls holds kernels only (a memory node would forbid cloning and nesting it); replays follow
+    the inputs, also with eager calls of the same entry on another stream between them."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(4)
+    M, N, Kd = 150, 272, 512
+    w = oracle.quantize(random_weights(rng, N, Kd), 64, 8)
+    wd = upload(w, cuda)
+    xs = [oracle.f32_to_bf16(rng.standard_normal((M, Kd)).astype(np.float32)) for _ in range(2)]
+    want = [oracle.linear_q(x, w, out_act=oracle.F32, w_f16=True) for x in xs]
+    x, y = bf16_tensor(xs[0], cuda).clone(), torch.empty((M, N), dtype=torch.float32, device=cuda)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        K.linear_qw_wmma(x, wd, y, M, K.Act.BF16, K.Act.F32)
+    assert set(node_types(graph)) == {0}  # CU_GRAPH_NODE_TYPE_KERNEL
+    graph.instantiate()
+    side = torch.cuda.Stream()
+    for i in (0, 1, 0):
+        x.copy_(bf16_tensor(xs[i], cuda))
+        y.fill_(float("nan"))
+        other = torch.empty_like(y)
+        torch.cuda.synchronize()
+        graph.replay()
+        with torch.cuda.stream(side):
+            K.linear_qw_wmma(x, wd, other, M, K.Act.BF16, K.Act.F32)
+        torch.cuda.synchronize()
+        K.check_dense_status("captured")
+        for got in (y, other):
+            assert max_abs_over_rms(got.cpu().numpy(), want[i]) <= 2e-5
+
+
+def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
+    """Two threads, each on a stream of its own, call a row-major form over and over with inputs of their own, while a third gives the
+    pool's idle memory back: every result is its own input's."""
+    import threading
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(8)
+    Kd, N = 512, 256
+    w = upload(oracle.quantize(random_weights(rng, N, Kd), 128, 4), cuda)
+    jobs, bad = [], []
+    for t, M in enumerate((700, 130)):
+        x = torch.randn((M, Kd), device=cuda).to(torch.bfloat16)
+        want = torch.empty((M, N), dtype=torch.float32, device=cuda)
+        K.linear_qw_wmma(x, w, want, M, K.Act.BF16, K.Act.F32)
+        jobs.append((x, want, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    done = threading.Event()
+
+    def work(x, want, stream):
+        with torch.cuda.stream(stream):
+            ys = [torch.empty_like(want) for _ in range(4)]
+            for _ in range(25):
+                for y in ys:
+                    K.linear_qw_wmma(x, w, y, x.shape[0], K.Act.BF16, K.Act.F32)
+                stream.synchronize()
+                bad.extend(1 for y in ys if not torch.equal(y, want))
+
+    def release():
+        while not done.wait(0.002):
+            bad.extend([lib.sxb_last_error()] if lib.sxb_release_scratch() else [])
+
+    threads = [threading.Thread(target=work, args=j) for j in jobs]
+    extra = threading.Thread(target=release)
+    for t in threads + [extra]:
+        t.start()
+    for t in threads:
+        t.join()
+    done.set()
+    extra.join()
+    torch.cuda.synchronize()
+    K.check_dense_status("two streams")
+    assert not bad and lib.sxb_release_scratch() == 0

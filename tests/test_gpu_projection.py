@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bf16_tensor, bits_of, max_abs_over_rms, random_weights, upload
+from helpers import bf16_tensor, bits_of, capture_calls, max_abs_over_rms, random_weights, upload
 
 pytestmark = pytest.mark.gpu
 
@@ -394,3 +394,15 @@ def test_a_wait_that_runs_out_ends_the_kernel_with_a_status(cuda, oracle, lib, t
     Kn.check_dense_status("after")
     want = oracle.linear_q(xb, wq, out_act=oracle.F32, w_f16=True)
     assert max_abs_over_rms(y2.cpu().numpy(), want) <= 2e-5
+
+
+def test_dense_tcgen05_captured(cuda, oracle, lib, monkeypatch):
+    """The dense forms, spread scales and a wait that runs out, on the kernel that captured calls take (no scratch)."""
+    graphs = capture_calls(monkeypatch)
+    test_dense_tcgen05_projections(cuda, oracle, 8, 64, 300, 2048, 1024)
+    test_dense_tcgen05_projections(cuda, oracle, 4, 128, 129, 512, 2048)
+    for spread in (0, 7, 12):
+        test_dense_tcgen05_spread_scales(cuda, oracle, 4, 128, 1024, spread)
+        test_dense_tcgen05_spread_scales(cuda, oracle, 8, 64, 1024, spread)
+    test_a_wait_that_runs_out_ends_the_kernel_with_a_status(cuda, oracle, lib, False)
+    assert graphs
