@@ -40,6 +40,9 @@ cudaMemPool_t pool() {
 
 bool StreamScratch::get(size_t bytes, cudaStream_t stream) {
     if (g_refuse > 0 || p_ != nullptr) return false;
+    // An error that the caller's earlier calls left pending is for the next launch check to report: nothing here may replace or
+    // clear it.  Past this line a pending error is this function's own.
+    if (cudaPeekAtLastError() != cudaSuccess) return false;
     // Not under capture: the allocation would be a node of the graph, which then can no longer be cloned, be a child of another or
     // have two executable instances, and whose memory is neither bounded by this pool nor given back by sxb_release_scratch.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;

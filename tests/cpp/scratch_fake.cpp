@@ -69,7 +69,18 @@ int main() {
         StreamScratch m;
         check("none where the capture state cannot be told, and no error left", !m.get(100, s) && g_last == cudaSuccess && g_allocs == 0);
     }
-    g_query_fails = false, g_alloc_fails = true;
+    g_query_fails = false, g_last = cudaErrorInvalidValue;
+    {
+        StreamScratch m;
+        m.get(100, s);
+        check("a caller's pending error is still pending", g_last == cudaErrorInvalidValue);
+    }
+    g_last = cudaErrorInvalidValue, g_alloc_fails = true;
+    {
+        StreamScratch m;
+        check("also where the allocation fails", !m.get(100, s) && g_last == cudaErrorInvalidValue);
+    }
+    g_last = cudaSuccess;
     {
         StreamScratch m;
         check("an allocation that fails leaves no error behind", !m.get(100, s) && m.ptr() == nullptr && g_last == cudaSuccess);

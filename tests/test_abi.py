@@ -51,7 +51,8 @@ def test_cxx_host_links_against_the_library(lib, tmp_path):
 
 
 def test_scratch_pool_against_a_fake_runtime(tmp_path):
-    """csrc/scratch.cu: no scratch (and no pool) for captured calls, a failed allocation leaves no error, one pool per device, memory freed on its stream, NoScratch per thread."""
+    """csrc/scratch.cu: no scratch (and no pool) for captured calls, a caller's pending CUDA error is left pending, a failed
+    allocation leaves none, one pool per device, memory freed on its stream, NoScratch per thread."""
     from helpers_cpp import build_scratch_fake
     res = subprocess.run([str(build_scratch_fake(tmp_path))], capture_output=True, text=True, timeout=60)
     assert res.returncode == 0 and "FAIL" not in res.stdout, res.stdout + res.stderr
