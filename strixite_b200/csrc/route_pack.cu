@@ -55,16 +55,16 @@ __device__ inline uint64_t cta_exclusive_scan(uint64_t v, uint64_t *buf, uint64_
 }
 
 // Where every bucket's slots and tiles begin.  first[i]: the bucket's first tile in list i; entry E + 1 = the total.
-constexpr int kTileLists = 4;
-__device__ constexpr int kTileRows[kTileLists] = {8, 128, kTcTileA, kTcTileB};
+constexpr int kTileLists = 2;
+__device__ constexpr int kTileRows[kTileLists] = {8, 128};
 struct Layout {
     int start[kMoeMaxExperts + 1];
     int first[kTileLists][kMoeMaxExperts + 2];
-    uint64_t scan[2][33];
+    uint64_t scan[33];
 };
 
 // Per-bucket counts (thread b owns bucket b) -> sm, and offsets and header of the workspace.  Ends with a barrier.
-// Two scans for all five sums, a sum in 21 bits (at most 2^20 slots): slots, 8-slot and 128-slot tiles; the other two lists.
+// One scan for the three sums, each in 21 bits (at most 2^20 slots): slots, 8-slot and 128-slot tiles.
 __device__ void scan_layout(int count, const RouteWords &L, int32_t *ws, Layout &sm, bool ep) {
     const int b = threadIdx.x, E = (int)L.E;
     // Tiles are cut for buckets 0..E-1, and for the overflow bucket E only outside expert-parallel mode (there its
@@ -72,25 +72,20 @@ __device__ void scan_layout(int count, const RouteWords &L, int32_t *ws, Layout 
     const bool tiled = b < E || (b == E && !ep);
     if (b > E) count = 0;
     auto tiles = [&](int rows) { return (uint64_t)(tiled ? (count + rows - 1) / rows : 0); };
-    uint64_t total0, total1;
-    const uint64_t sum0 = cta_exclusive_scan((uint64_t)count | (tiles(8) << 21) | (tiles(128) << 42), sm.scan[0], &total0);
-    const uint64_t sum1 = cta_exclusive_scan(tiles(kTcTileA) | (tiles(kTcTileB) << 21), sm.scan[1], &total1);
+    uint64_t total;
+    const uint64_t sum = cta_exclusive_scan((uint64_t)count | (tiles(8) << 21) | (tiles(128) << 42), sm.scan, &total);
     const int mask = (1 << 21) - 1;
-    auto store = [&](int at, uint64_t s0, uint64_t s1) {
-        sm.first[0][at] = (int)(s0 >> 21) & mask, sm.first[1][at] = (int)(s0 >> 42);
-        sm.first[2][at] = (int)s1 & mask, sm.first[3][at] = (int)(s1 >> 21) & mask;
-    };
+    auto store = [&](int at, uint64_t s) { sm.first[0][at] = (int)(s >> 21) & mask, sm.first[1][at] = (int)(s >> 42); };
     if (b <= E) {
-        sm.start[b] = (int)sum0 & mask;
-        ws[L.offsets + b] = (int)sum0 & mask;
-        store(b, sum0, sum1);
+        sm.start[b] = (int)sum & mask;
+        ws[L.offsets + b] = (int)sum & mask;
+        store(b, sum);
     }
     if (b == 0) {
-        store(E + 1, total0, total1);
-        ws[L.offsets + E + 1] = (int)total0 & mask;
-        ws[0] = (int)(total0 >> 21) & mask, ws[1] = (int32_t)L.S, ws[2] = E, ws[3] = (int)(total0 >> 42), ws[4] = ep ? 1 : 0;
+        store(E + 1, total);
+        ws[L.offsets + E + 1] = (int)total & mask;
+        ws[0] = (int)(total >> 21) & mask, ws[1] = (int32_t)L.S, ws[2] = E, ws[3] = (int)(total >> 42), ws[4] = ep ? 1 : 0;
         ws[5] = 0, ws[6] = 0, ws[7] = 0;
-        ws[L.tta_n] = (int)total1 & mask, ws[L.ttb_n] = (int)(total1 >> 21) & mask;
     }
     __syncthreads();
 }
@@ -99,8 +94,8 @@ __device__ void scan_layout(int count, const RouteWords &L, int32_t *ws, Layout 
 // never win).
 __device__ void emit_tiles(const RouteWords &L, int32_t *ws, const Layout &sm, int t0, int stride) {
     const int E = (int)L.E;
-    const int64_t bucket_at[kTileLists] = {L.t8_bucket, L.t128_bucket, L.tta_bucket, L.ttb_bucket};
-    const int64_t start_at[kTileLists] = {L.t8_start, L.t128_start, L.tta_start, L.ttb_start};
+    const int64_t bucket_at[kTileLists] = {L.t8_bucket, L.t128_bucket};
+    const int64_t start_at[kTileLists] = {L.t8_start, L.t128_start};
 #pragma unroll
     for (int list = 0; list < kTileLists; ++list) {
         const int *first = sm.first[list];
@@ -374,15 +369,8 @@ RouteWords route_words(int64_t M, int64_t A, int64_t E) {
     L.t128_start = L.t128_bucket + L.T128max;
     L.segbad = L.t128_start + L.T128max;
     L.scratch = L.segbad + L.nseg;
-    L.TtAmax = L.S / kTcTileA + E + 2, L.TtBmax = L.S / kTcTileB + E + 2;
     L.first = L.scratch + L.nseg * (E + 1);
-    L.tta_n = L.first + (L.nseg ? kTileLists * (E + 2) : 0);
-    L.tta_bucket = L.tta_n + 1;
-    L.tta_start = L.tta_bucket + L.TtAmax;
-    L.ttb_n = L.tta_start + L.TtAmax;
-    L.ttb_bucket = L.ttb_n + 1;
-    L.ttb_start = L.ttb_bucket + L.TtBmax;
-    L.total = L.ttb_start + L.TtBmax;
+    L.total = L.first + (L.nseg ? kTileLists * (E + 2) : 0);
     return L;
 }
 

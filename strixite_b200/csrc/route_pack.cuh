@@ -8,8 +8,6 @@ namespace sxb {
 constexpr int64_t kMoeMaxExperts = 1023;   // E + 1 buckets fit one 1024-thread CTA (kernels/moe_grouped.hpp:43)
 constexpr int64_t kMoeMaxSlots = 1 << 20;  // kernels/moe_grouped.hpp:44
 constexpr int kSegSlots = 1024;            // slots one warp places in the multi-CTA pack
-// Rows of the two wider tile lists that close the workspace; the kernels here walk the lists of 8 and 128.
-constexpr int kTcTileA = 192, kTcTileB = 256;
 
 // Word (int32) offsets into the workspace.
 //   header [8]: n_tiles8, S, E, n_tiles128, ep_mode, 0, 0, 0
@@ -18,11 +16,10 @@ constexpr int kTcTileA = 192, kTcTileB = 256;
 //   slots [S]: slot index s = m * A + a, ascending inside a bucket
 //   t8_bucket / t8_start [T8max]: tiles of up to 8 slots (the streaming kernels); t128_*: up to 128 (tcgen05)
 //   segbad [nseg], scratch [nseg][E + 1]: the multi-CTA pack's per-segment first invalid slot and histograms
-//   first [4][E + 2], multi-CTA pack only: every bucket's first tile in the four lists, then the list's length
-//   tta [1 + 2 * TtAmax], ttb [1 + 2 * TtBmax]: a count, then bucket / start of tiles of up to kTcTileA and kTcTileB slots
+//   first [2][E + 2], multi-CTA pack only: every bucket's first tile in the two lists, then the list's length
 struct RouteWords {
-    int64_t S, E, T8max, T128max, TtAmax, TtBmax, nseg;
-    int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, first, tta_n, tta_bucket, tta_start, ttb_n, ttb_bucket, ttb_start, total;
+    int64_t S, E, T8max, T128max, nseg;
+    int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, first, total;
 };
 RouteWords route_words(int64_t M, int64_t A, int64_t E);
 // The workspace (route_words(M * E, 1, E)) of the grouping in which slot m * E + b belongs to bucket b, for all m < M: what

@@ -37,24 +37,12 @@ __device__ inline bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Non-blocking: has the phase of this parity completed?  (try_wait may suspend the thread for a while; this never does.)
-__device__ inline bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 __device__ inline unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-// The same, the thread suspended by the hardware for up to `ns` while the phase has not completed.
+// The same as mbar_try_wait, the thread suspended by the hardware for up to `ns` while the phase has not completed.
 __device__ inline bool mbar_try_wait_for(uint64_t *bar, uint32_t parity, uint32_t ns) {
     uint32_t ok;
     asm volatile(
@@ -80,19 +68,6 @@ __device__ inline bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *a
         else if (now - t0 > limit_ns) return false;
     }
     return true;
-}
-// The same for a single thread that everyone else waits for: no suspension, so no time is lost waking up.
-__device__ inline bool mbar_spin(uint64_t *bar, uint32_t parity, volatile int *abort_flag, unsigned long long limit_ns) {
-    unsigned long long t0 = 0;
-    for (uint32_t spins = 1;; ++spins) {
-        if (mbar_test_wait(bar, parity)) return true;
-        if ((spins & 1023u) == 0u) {
-            if (abort_flag != nullptr && *abort_flag) return false;
-            const unsigned long long now = global_ns();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > limit_ns) return false;
-        }
-    }
 }
 __device__ inline void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ inline void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -153,20 +128,9 @@ __device__ inline void tc_st16(uint32_t taddr, const uint4 (&d)[4]) {
         "r"(d[2].y), "r"(d[2].z), "r"(d[2].w), "r"(d[3].x), "r"(d[3].y), "r"(d[3].z), "r"(d[3].w)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]: the A operand (128 rows x 16 k of F16, two per 32-bit column) read from tensor memory.
-// Whole-warp call, one elected lane issues (see tc_commit).
-__device__ inline void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "elect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// The same for a loop that runs under ONE election: elect_one() picks a lane of the converged warp, and that lane alone runs
-// the loop with these.  An MMA then costs its issuer 12 cycles; with the election inside each instruction group, 40 to 90.
+// D[tmem] (+)= A[tmem] * B[smem], the A operand (128 rows x 16 k of F16, two per 32-bit column) read from tensor memory, for
+// a loop that runs under ONE election: elect_one() picks a lane of the converged warp, and that lane alone runs the loop with
+// these.  An MMA then costs its issuer 12 cycles; with the election inside each instruction group, 40 to 90.
 __device__ inline bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
