@@ -15,9 +15,9 @@
 // Operands.  A (weights) is read by the MMA from TENSOR MEMORY (the [tmem] form of tcgen05.mma): the producer threads
 // dequantize in registers and tcgen05.st the F16 rows straight into their own TMEM lanes, which needs no proxy fence
 // (shared-memory operands written by threads do, and that fence cost more than the dequantization).  B (activations)
-// is a K-major, 128-byte-swizzled tile in shared memory; with "tile-blocked" activations (sxb_stage_f16_tiles, or the
-// h this kernel's own SwiGLU form writes) the tile of a k-block is ONE contiguous run in global memory and arrives by
-// one cp.async.bulk.  The packed codes come by 2-D tensor copies (64 bytes x 128 rows a box) into a ring in shared
+// is a K-major, 128-byte-swizzled tile in shared memory, gathered row by row (activations in the tile-blocked form go to
+// grouped_tc_tiled.cu, and so do row-major ones where there is scratch to bring them into that form: launch_tc).  The packed
+// codes come by 2-D tensor copies (64 bytes x 128 rows a box) into a ring in shared
 // memory.  Tensor memory: columns 0-255 the two accumulators, 256-511 four stages of the A operand.
 //
 // One persistent CTA per SM, 16 warps:
@@ -30,8 +30,7 @@
 //               dequantizes the rows of BOTH accumulators on its lane: lop3 / packed-half arithmetic on 64 codes a
 //               row and k-block.  Within every 8 consecutive k both operands use the order [0 4 1 5 2 6 3 7] (Q4),
 //               the order in which a nibble pair falls out of one lop3, so no element moves after dequantization
-//   warps 14-15 activation producers (one thread issues the bulk copies of tile-blocked activations; the other warp's
-//               lane 0 then runs the ring of weight codes; otherwise both warps gather and convert rows)
+//   warps 14-15 activation producers: gather rows and convert them
 // Stages are handed over with mbarriers (producers -> MMA: arrive after tcgen05.wait::st; copies: complete_tx bytes;
 // MMA -> producers and MMA -> epilogue: tcgen05.commit).  Every wait is bounded: past the limit the CTA raises its abort
 // flag, records {2, item, role} in the status words, drains the tensor pipe and frees its tensor memory before returning.
@@ -148,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
     volatile int *abort_v = &abort_flag;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) mbar_init(&full_bar[s], kAWarps / 2 + (a.x_kind == 3 ? 1 : kBWarps)), mbar_init(&empty_bar[s], kMmaWarps);
+        for (int s = 0; s < kStages; ++s) mbar_init(&full_bar[s], kAWarps / 2 + kBWarps), mbar_init(&empty_bar[s], kMmaWarps);
         mbar_init(&acc_full[0], kMmaWarps), mbar_init(&acc_empty[0], kEpiWarps);
         mbar_init(&drain_bar, kMmaWarps);
         for (int s = 0; s < kWSlots; ++s) mbar_init(&w_full[s], 1), mbar_init(&w_empty[s], BITS == 4 ? kAWarps : kAWarps / 2);
@@ -171,14 +170,12 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
         }
     };
 
-    // The ring of weight-code slots is filled by ONE thread.  With tile-blocked activations the second B warp has nothing
-    // else to do and its lane 0 runs the ring as far ahead as free slots allow.  Otherwise lane 0 of the first A warp tops
+    // The ring of weight-code slots is filled by ONE thread: lane 0 of the first A warp tops
     // the ring up before it consumes slot number j, to slot j + kWSlots - 1, which reuses the buffer of slot j - 1 -
     // released by every A warp as soon as the warp has its codes in registers, so that wait is short.
     constexpr int kKbPerSlot = BITS == 4 ? 2 : 1;  // k-blocks per 64 bytes of packed codes
     const int n_slots = (n_kb + kKbPerSlot - 1) / kKbPerSlot;
     const uint32_t w_base = smem_u32(smem + kStages * kStageBytes);
-    const bool own_w_thread = a.x_kind == 3;
     int is_item = next_valid_item<MODE>(a, blockIdx.x, n_items, rbs), is_slot = 0, is_y0 = 0, is_y1 = 0;
     uint32_t issued = 0;
     auto issue_one = [&]() -> bool {
@@ -275,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
         };
         // lane 0: the codes of slot number wc have landed and the stage of k-block number cnt is free
         auto poll = [&](uint32_t wc, uint32_t cnt, int it_for_status) {
-            if (!own_w_thread && warp == kFirstAWarp) top_up(wc);
+            if (warp == kFirstAWarp) top_up(wc);
             if (!mbar_wait(&w_full[wc % kWSlots], (wc / kWSlots) & 1u, abort_v, a.wait_limit_ns)) raise_abort(it_for_status, 7);
             else if (!mbar_wait(&empty_bar[cnt % kStages], ((cnt / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) raise_abort(it_for_status, 1);
         };
@@ -383,31 +380,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
         // ===================== B producers: activations =====================
         // B warp w owns tokens [64 w, 64 w + 64) of the tile; lane l copies 16-byte chunk c = l % 8 of tokens
         // 64 w + l / 8 + 4 i (i < 16), every k-block, so eight lanes cover one 128-byte line of one activation row.
-        if (a.x_kind == 3) {
-            if (warp == kFirstBWarp + 1 && lane == 0)
-                while (is_item < n_items && !*abort_v)
-                    if (!issue_one()) break;
-            // Tile-blocked activations: one thread, one bulk copy per k-block, completion counted in bytes on the
-            // stage's barrier; every free stage is refilled at once, so kStages k-blocks are in flight.
-            if (warp == kFirstBWarp && lane == 0) {
-                uint32_t it_count = 0;
-                for (int item = next_valid_item<MODE>(a, blockIdx.x, n_items, rbs); item < n_items && !*abort_v;
-                     item = next_valid_item<MODE>(a, item + gridDim.x, n_items, rbs)) {
-                    const ItemInfo it = item_info<MODE>(a, item, rbs);
-                    const uint32_t bytes = (uint32_t)it.cnt * 128u;
-                    const unsigned char *src = reinterpret_cast<const unsigned char *>(a.x) + (int64_t)it.start * 128;
-                    for (int kb = 0; kb < n_kb; ++kb, ++it_count) {
-                        const int stage = it_count % kStages;
-                        if (!mbar_wait(&empty_bar[stage], ((it_count / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
-                            raise_abort(item, 5);
-                            break;
-                        }
-                        mbar_expect_tx(&full_bar[stage], bytes);
-                        bulk_g2s(smem_u32(smem + stage * kStageBytes), src + (int64_t)kb * a.L.S * 128, bytes, &full_bar[stage]);
-                    }
-                }
-            }
-        } else {
         const int bw = warp - kFirstBWarp, c = lane & 7, rg = lane >> 3;
         constexpr int kRowsPerWarp = kMaxTileTokens / kBWarps, kRowsPerLane = kRowsPerWarp / 4;  // 64, 16
         int64_t *row_off = b_row_off[bw];  // element offset of every owned token's activation row (this warp only)
@@ -486,7 +458,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
                 }
             }
             it_count += n_kb;
-        }
         }
     } else if (warp >= kMmaWarp) {
         // ===================== MMA issue =====================
@@ -639,8 +610,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
     }
 
     // An aborting CTA must not return under copies it issued into its own shared memory (which may go to the next CTA):
-    // the thread that ran the ring of weight codes waits, bounded, for the last fill of every slot; the activation copies
-    // complete on barriers that also count thread arrivals, so their issuer lets a generous time pass instead.
+    // the thread that ran the ring of weight codes waits, bounded, for the last fill of every slot.
     if (*abort_v) {
         for (int sl = 0; sl < kWSlots && issued > 0; ++sl) {
             if (issued <= (uint32_t)sl) continue;
@@ -648,8 +618,6 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
             if (blockIdx.x == 0 && (int)last == a.test_skip_slot) continue;  // the test hook's slot was never filled
             mbar_wait(&w_full[sl], (last / kWSlots) & 1u, nullptr, 1000000ull);
         }
-        if (warp == kFirstBWarp && lane == 0 && a.x_kind == 3)
-            for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 50000ull;) {}
     }
     tc_fence_before();
     __syncthreads();
@@ -782,10 +750,10 @@ int launch_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     const size_t smem = (size_t)kStages * kStageBytes + (size_t)kWSlots * kWSlotBytes + 1024;
     a.wait_limit_ns = g_wait_limit_ns, a.test_skip_slot = g_test_skip_slot;
     // Tile-blocked activations have a kernel of their own (grouped_tc_tiled.cu), and any other form is brought into that one
-    // first, in stream-ordered scratch: a pass over the activations (14 us for the 12000 slots x 4096 of a 1200-token
+    // first, in stream-ordered scratch: a pass over the activations (25 us for the 12000 slots x 4096 of a 1200-token
     // prefill) against two warps that convert or gather them for every row block of the weight again (a 1200-token layer with
-    // BF16 activations: 6.9 + 3.5 ms in this file's kernel).  Without scratch (out of memory, allocation-free entry points)
-    // this file's kernel takes the activations as they are.
+    // BF16 activations: 6.9 + 3.5 ms in this file's kernel).  Without scratch (out of memory, a capturing stream,
+    // allocation-free entry points) this file's kernel takes the activations as they are.
     if (a.x_kind == 3) return launch_tiled_tc<BITS, MODE>(fn, a, G, st);
     StreamScratch staged;
     if (staged.get((size_t)a.L.S * (size_t)a.K * 2, st)) {
