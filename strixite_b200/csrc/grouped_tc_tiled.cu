@@ -80,7 +80,9 @@ constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
 // The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).  Rows at natural magnitude: scale = -2^24.
 constexpr float kNatural = -0x1p24f;
-__device__ inline float unscale(float scale) { return __int_as_float(((127 + 24 + 127) << 23) - __float_as_int(fabsf(scale))); }
+__host__ __device__ constexpr uint32_t unscale_bits(uint32_t scale_bits) { return ((127u + 24u + 127u) << 23) - scale_bits; }  // past int
+static_assert(unscale_bits((127u + 24u) << 23) == 127u << 23 && unscale_bits((127u - 1u) << 23) == (127u + 25u) << 23, "2^(24 - k)");
+__device__ inline float unscale(float scale) { return __uint_as_float(unscale_bits(__float_as_uint(fabsf(scale)))); }
 
 struct Item {
     int bucket, start, cnt;  // expert (bucket E = invalid ids, -1 = no more items), first position in slots[], tokens of the item
