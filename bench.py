@@ -64,7 +64,7 @@ def parse():
     ap.add_argument("--placement", default="balanced", choices=["balanced", "contiguous"],
                     help="expert-parallel runs: experts dealt to ranks by calibrated load, or expert e on rank e // (E / N)")
     ap.add_argument("--stage", default="tiles", choices=["tiles", "rows"],
-                    help="tcgen05 gate/up activations: gathered once into the tile-blocked form, or converted once and gathered per tile")
+                    help="tcgen05 gate/up activations: handed over in the tile-blocked form, or as F16 rows that the library brings into it (a pass more)")
     ap.add_argument("--math", default="", help="tcgen05 numerics: wmma_f16 (BF16 per-slot dots, the reference's) or wmma_f16_f32p")
     return ap.parse_args()
 
@@ -491,10 +491,8 @@ def roofline_tensor(cfg, res, peaks, world):
     # codes + scales / mins + tile-blocked activations, a ratio of 1.00; the same sum for this launch, times that ratio.
     ly = res["stack"].layers[0]
     traffic = 1.003 * (ly.w.gate_up.bytes() + cfg.T * cfg.k / world / micro * cfg.d * 2)
-    # which tcgen05 kernel serves gate/up (launch_tc in csrc/grouped_tc.cu): tile-blocked activations and >= 160 slots an expert
-    # on average go to the 128-row x 256-token kernel, fewer stay on the 256-row x 128-token one
-    name = "tiled_tc_kernel" if cfg.T * cfg.k / world / micro / (cfg.E / world) >= 160 else "grouped_tc_kernel"
-    return dict(bound="tensor", kernel=name + "<gate_up+swiglu>", achieved=achieved, peak=peak, unit="TFLOP/s",
+    # the layer hands gate/up tile-blocked activations, which the tiled kernel alone takes (launch_tc in csrc/grouped_tc.cu)
+    return dict(bound="tensor", kernel="tiled_tc_kernel<gate_up+swiglu>", achieved=achieved, peak=peak, unit="TFLOP/s",
                 frac=achieved / peak, peak_source=peaks["source"] + " (sustained bf16)",
                 frac_of_burst=achieved / peaks["tflops_burst"], peak_burst=peaks["tflops_burst"], traffic=traffic,
                 traffic_source="dram bytes of an ncu capture of a reduced case, scaled by algorithmic bytes",
