@@ -266,10 +266,10 @@ int sxb_linear_q4(const void *x, const SxbQView *w, void *y, int64_t M, int act,
 int sxb_linear_q8(const void *x, const SxbQView *w, void *y, int64_t M, int act, int out_act, sxb_stream_t stream);
 
 /* kernels/linear_wmma.hpp:23,26  linear_q4_wmma / linear_q8_wmma: the multi-token dense projection on the tensor cores,
- * here the tcgen05 grouped kernel run as one group with the result written by its epilogue (no pack, no scratch).
+ * here the tcgen05 grouped kernel run as one group with the result written by its epilogue (no pack).
  * Numerics of this library's WMMA_F16 path: x as F16, weights f16(code * scale + min), FP32 accumulation, one rounding.
  * act SXB_ACT_BF16, or SXB_ACT_F16_TILED for x staged by sxb_stage_f16_tiles with a null workspace; out_act BF16 or F32.
- * K % 128 == 0, N % 16 == 0. */
+ * K % 128 == 0, N % 8 == 0 (the SwiGLU form: N % 16 == 0). */
 int sxb_linear_q4_wmma(const void *x, const SxbQView *w, void *y, int64_t M, int act, int out_act, sxb_stream_t stream);
 int sxb_linear_q8_wmma(const void *x, const SxbQView *w, void *y, int64_t M, int act, int out_act, sxb_stream_t stream);
 /* No counterpart in the reference (which runs linear_q8_wmma, then swiglu): w = [gate | up] rows, h [M, N/2] =

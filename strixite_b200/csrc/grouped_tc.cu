@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_tc_kernel(const TcArgs a,
                 else elem_off = ((j & ~(int64_t)7) + pos) * 2;
             } else {
                 const int64_t r = (int64_t)it.rb * kAThreads + r_loc;
-                row_ok = r < a.N;  // N is a multiple of 16: the second accumulator's row r + 128 is checked on its own
+                row_ok = r < a.N;  // the second accumulator's row r + 128 is checked on its own
                 elem_off = r * (MODE == kTcPartial ? 4 : 2);
             }
             const bool row1_ok = MODE != kTcSwiglu && (int64_t)it.rb * kAThreads + 128 + r_loc < a.N;
@@ -867,7 +867,9 @@ int tc_dense(const char *fn, const void *x, const SxbQView *w, void *y, int64_t 
     SXB_CHECK(w->G == 32 || w->G == 64 || w->G == 128, fn, ": group size ", w->G, " unsupported (32, 64 or 128)");
     SXB_CHECK(w->K >= 128 && w->K % 128 == 0 && w->K <= (1 << 24), fn, ": K = ", w->K, ", the tcgen05 kernels need a multiple of 128");
     SXB_CHECK(M >= 1 && M <= kMoeMaxSlots, fn, ": M (rows of x) = ", M, ", expected 1..", kMoeMaxSlots);
-    SXB_CHECK(w->N >= 16 && w->N % 16 == 0 && w->N <= 0x7fffffff, fn, ": N = ", w->N, " must be a multiple of 16");
+    // rows of y begin on 16-byte boundaries; the SwiGLU form stores 8 h columns at a time
+    SXB_CHECK(w->N >= 16 && w->N % (out_kind == 2 ? 16 : 8) == 0 && w->N <= 0x7fffffff, fn, ": N = ", w->N, " must be a multiple of ",
+              out_kind == 2 ? 16 : 8);
     SXB_CHECK(aligned16(w->q) && aligned16(x) && aligned16(y), fn, ": codes, x and y must be 16-byte aligned");
     SXB_CHECK(out_kind != 2 || w->N % 2 == 0, fn, ": [gate | up] rows: N = ", w->N, " must be even");
     const int64_t out_bytes = out_kind == 2 ? M * (w->N / 2) * 2 : M * w->N * (out_kind == 1 ? 4 : 2);

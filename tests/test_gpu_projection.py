@@ -228,6 +228,28 @@ def test_dense_tcgen05_partial_row_blocks(cuda, oracle, bits, G, M, N, K):
     assert torch.equal(ybf, y32[:M].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("way", ["staged", "captured"])
+@pytest.mark.parametrize("bits,G,M,N,K", [(4, 128, 64, 4104, 2048), (8, 64, 127, 4104, 512), (4, 64, 129, 24, 256), (8, 128, 1001, 136, 256)])
+def test_dense_tcgen05_rows_in_eights(cuda, oracle, monkeypatch, way, bits, G, M, N, K):
+    """Weights whose row count is a multiple of 8 and not of 16, on both kernels: the last row block ends inside a 16-row piece of
+    tensor memory; nothing is stored past the last row."""
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(M + N)
+    wq = oracle.quantize(random_weights(rng, N, K), G, bits)
+    xb = oracle.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w, x = upload(wq, cuda), bf16_tensor(xb, cuda)
+    y32 = torch.full((M + 1, N), 7.0, dtype=torch.float32, device=cuda)
+    ybf = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=cuda)
+    if way == "captured":
+        capture_calls(monkeypatch)
+    Kn.linear_qw_wmma(x, w, y32, M, Kn.Act.BF16, Kn.Act.F32)
+    Kn.linear_qw_wmma(x, w, ybf, M, Kn.Act.BF16, Kn.Act.BF16)
+    torch.cuda.synchronize()
+    Kn.check_dense_status("rows in eights")
+    assert max_abs_over_rms(y32[:M].cpu().numpy(), oracle.linear_q(xb, wq, out_act=oracle.F32, w_f16=True)) <= 2e-5
+    assert torch.all(y32[M] == 7.0) and torch.all(ybf[M] == 7.0) and torch.equal(ybf[:M], y32[:M].to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("spread", [0, 6, 7, 9, 12])
 @pytest.mark.parametrize("bits,G,K", [(4, 128, 1024), (8, 64, 1024), (4, 32, 384), (8, 128, 640)])
 def test_dense_tcgen05_spread_scales(cuda, oracle, bits, G, K, spread):
