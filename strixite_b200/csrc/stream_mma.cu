@@ -935,7 +935,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
              ": reserving shared memory");
     // A dense projection of few units for the machine's warps: up to eight warps share one, as long as that gives a warp at most two and a half
     // parts in turn.  A warp alone walks K / (4 * kStepCodes) blocks one after another, each a round trip to memory (2048 x 4096
-    // Q8, one token: 39 us with 128 warps at work).
+    // Q8, one token: 28 us with 128 warps at work, 13.5 with eight warps a unit).
     const int64_t machine_warps = (int64_t)sm_count() * (kBigThreads / 32);
     StreamArgs args = a;
     args.chunks = SRC == kDense && geo::kStepsPerGroup == 1 && vector_scales(a, G) ? chunk_count(steps / kPrefetch) : 1, args.split = 1;
@@ -949,7 +949,9 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     // warps, two an SM where their shared memory allows, and never more CTAs than one per unit and warp.
     const bool big = est_units >= machine_warps * 2;
     const int threads = big ? kBigThreads : kThreads, warps = threads / 32;
-    const int per_sm = big || smem > 100 * 1024 ? 1 : 2;
+    // Two fit an SM's 228 KB with 1 KB of the system's and their static shared memory each, 25 KB in the dense form (with 100 KB as
+    // the line there too, 110 x 4096 x 5760 Q8 ran as two waves of one CTA an SM: 188 us, now 153; 100 x 4096 x 6144 Q4 84, now 50).
+    const int per_sm = big || smem > (SRC == kDense ? 88 : 100) * 1024 ? 1 : 2;
     int64_t grid = (int64_t)sm_count() * per_sm;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (est_units + warps - 1) / warps));
     kern<<<(unsigned)grid, threads, smem, st>>>(args);
