@@ -1,7 +1,8 @@
 // sxb_moe_layer: the call sequence of one MoE block as ONE entry point - what runtime/qwen4exp.cpp:3143-3217 issues
 // launcher by launcher: router top-k, grouping of the slots by expert, gate/up + SwiGLU, down + weighted combine, and the
 // always-on shared expert folded into the combine.  Everything goes to the caller's stream through the library's own
-// entry points; nothing is allocated, nothing synchronizes.
+// entry points, but for the shared expert's launches on the streaming kernels where the caller names a second stream for them;
+// nothing is allocated, nothing synchronizes.
 
 #include "experts.cuh"
 
@@ -95,6 +96,7 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
     const int64_t M = a->M, A = a->A, E = a->E, d = a->gate_up->K, I = a->gate_up->N / E / 2;
     SXB_CHECK(a->gate_up->N == E * 2 * I && a->down->N == E * d && a->down->K == I, fn, ": gate_up [", a->gate_up->N, ", ",
               a->gate_up->K, "] and down [", a->down->N, ", ", a->down->K, "] do not describe ", E, " experts");
+    // 256: what either side takes stands at MoeLayer.tc_min_tokens (layer.py)
     const int math = a->math >= 0 ? a->math : (M >= 256 ? SXB_MATH_WMMA_F16_F32_PARTIALS : SXB_MATH_F32);
     const bool tc = math >= SXB_MATH_WMMA_F16;
     SXB_CHECK(!tc || a->xs != nullptr, fn, ": the tcgen05 path needs the tile-blocked activation buffer xs (M * A * d F16)");

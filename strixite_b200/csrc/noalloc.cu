@@ -73,7 +73,9 @@ extern "C" int sxb_linear_q4_experts_combine_grouped_noalloc(const void *h, cons
               kNoAllocFloats, " floats (16 MiB); call linear_q4_experts_combine_grouped with caller-owned scratch instead");
     float *partial = nullptr;
     if (int rc = partial_scratch(&partial)) return rc;
-    // from here on the caller-scratch entry point's own code: the same checks (pointers, dtypes, overlaps), the same kernels
+    // from here on the caller-scratch entry point's own code and checks (pointers, dtypes, overlaps).  The kernels are the same but for
+    // the WMMA_F16 kinds with row-major h: those bring h into the tile-blocked form in scratch where they may allocate, and read it
+    // as it is here; a weight's one rounding to F16 may fall elsewhere where it is subnormal (strix_b200.h, "Ownership")
     const NoScratch no_scratch;
     return combine_grouped<4>(fn, h, w, E, ids, coef, ws, ws_bytes, partial, M, A, y, act, out_act, math, stream, shared, h_f16, E, 0);
 }

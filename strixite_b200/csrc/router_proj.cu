@@ -44,9 +44,10 @@ __device__ inline void load_w8(const uint16_t *p, float (&w)[8]) {
 }
 
 // y[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]).  A CTA stages the activations of 16 tokens in shared memory once and
-// streams four weight rows against them, four warps a row (one per quarter of the staged k range): the arithmetic of 16 tokens
-// is the bound, so all SMs have to share it (65 CTAs of eight rows -> 129 of four: 1 / 16 / 37
-// tokens 13.1 / 19.6 / 44.8 -> 10.3 / 16.8 / 37.6 us for 513 x 4096 FP32).  A lane issues ALL the
+// streams four weight rows against them, four warps a row (one per quarter of the staged k range): few rows a CTA, so that
+// nearly all SMs have one (65 CTAs of eight rows -> 129 of four: 1 / 16 / 37
+// tokens 13.1 / 19.6 / 44.8 -> 10.3 / 16.8 / 37.6 us for 513 x 4096 FP32, whose 8.4 MB are 1.3 us of HBM time: it is a chain of
+// staging, one round trip for the row and the sums of sixteen tokens, live or not).  A lane issues ALL the
 // loads of its part of the row before it consumes any of them - with a few dozen tokens the kernel is one memory round
 // trip plus arithmetic, so what counts is how many bytes are in flight.  The sum of a (token, row) pair is formed in a
 // fixed order: per lane ascending k, an xor butterfly in the warp, then the row's quarters in order.

@@ -74,13 +74,17 @@ class MoeLayer:
     """One MoE sublayer.  E_total / e_lo: expert-parallel ranks hold experts [e_lo, e_lo + E_local) of E_total in their
     weight views and return their partial sum of y (see `ep.ExpertParallelMoe`)."""
 
+    # From here on the tcgen05 kernels.  Layer of 512 experts, top-10, d = 4096, I = 1024, Q4 with a shared expert, us streaming /
+    # tcgen05: 128 tokens 714 / 919, 204 822 / 989, 256 880 / 1014, 320 1433 / 997, 400 1467 / 1009; Q8 down weights 256 1058 / 1208,
+    # 320 1530 / 1096.  The jump is the streaming kernels' second tile of eight slots an expert: the sides change between five and
+    # six slots an expert on average, i.e. between 256 and 320 tokens here.
     tc_min_tokens = 256
     # The tcgen05 path's numerics.  WmmaF16F32Partials keeps the combine's per-slot dots in FP32; WmmaF16 rounds them to
     # BF16 as the reference's served path does, which by itself moves an output by up to ~2e-2 of the output RMS
     # (measured on the Zipf-routed stack) - beyond the 1e-2 this path is held to - and measured no faster here.
     tc_math = MoeMath.WmmaF16F32Partials
-    stage_rows = False          # tcgen05 path: True = x converted once to F16 rows (sxb_stage_f16) and gathered per tile by the
-                                # kernel's copy warps; False = x gathered once into the tile-blocked form (sxb_stage_f16_tiles)
+    stage_rows = False          # tcgen05 path: False = x gathered once into the tile-blocked form (sxb_stage_f16_tiles); True = x
+                                # converted to F16 rows first (sxb_stage_f16), which the library then gathers: a pass more
     small_slots = SMALL_SLOTS   # up to this many slots the router and the pack are one call (sxb_moe_route_small)
 
     def __init__(self, weights: MoeWeights, n_experts: int, top_k: int, buffers: MoeBuffers, E_total: Optional[int] = None,

@@ -62,7 +62,7 @@ def run_both(lib, oracle, dev, M, A, E, I, d, seed, shared, math=None, out_dtype
 
 
 def test_noalloc_combine_matches_twice_in_a_row(cuda, oracle, lib):
-    # the same kernels run on both sides, so the outputs are equal bit for bit (the tolerance of the combine's own
+    # the same kernels run on both sides (MoeMath.F32), so the outputs are equal bit for bit (the tolerance of the combine's own
     # tests, 3e-5 of the output RMS, is the fallback bar should a future kernel reorder its sums)
     got1, want1 = run_both(lib, oracle, cuda, M=48, A=6, E=16, I=256, d=512, seed=1, shared=True)
     got2, want2 = run_both(lib, oracle, cuda, M=9, A=4, E=16, I=128, d=256, seed=2, shared=False, measure_memory=True)
@@ -75,7 +75,9 @@ def test_noalloc_combine_matches_twice_in_a_row(cuda, oracle, lib):
 
 def test_noalloc_combine_other_forms(cuda, oracle, lib):
     """The tcgen05 form of the down projection (BF16 per-slot dots in the built-in array) and a BF16 output, at small
-    shapes, each against the caller-scratch entry point; the second call of each also checks that no memory was taken."""
+    shapes, each against the caller-scratch entry point; the second call of each also checks that no memory was taken.  The
+    tcgen05 forms are two kernels (without scratch: the one that gathers rows); they are equal here because weights of this
+    size are exact or rounded alike in both, which weights that are subnormal in F16 need not be."""
     from strixite_b200 import kernels as K
     for kw in (dict(math=K.MoeMath.WmmaF16), dict(math=K.MoeMath.WmmaF16F32Partials), dict(out_dtype=torch.bfloat16)):
         for seed in (3, 4):
