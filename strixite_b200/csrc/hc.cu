@@ -7,15 +7,20 @@
 // a 32-code chunk is scale * sum(x * code) + min * sum(x) (kernels/hc.hip:117-123, 206-211): the weights are never
 // rounded to a dequantized value.
 //
-// Both are small-matrix, many-launch kernels (a few MB of weights, ~97 mixes per decoded token upstream): what matters is
-// that the weight matrix is read once per group of tokens and that enough CTAs exist to cover the SMs at T = 1..64.
-//   down: a CTA owns a group of weight rows and up to four tokens, whose streams it holds in shared memory; its sixteen warps
-//         take (row, eighth of the row) items, an eighth lying in one stream, and the parts meet in shared memory.
-//   up:   a thread owns one row s*d + j of W_up (consecutive threads' rows are adjacent in the chunk-major layout, so a
-//         warp's 16-byte loads are one contiguous run), dots it with the h of MT tokens held in shared memory, and the
+// Both are small-matrix, many-launch kernels (a few MB of weights, ~97 mixes per decoded token upstream): what bounds them is the round
+// trips of one launch, as long as the arithmetic stays out of the way.  As FP32 multiply-adds, one a code and token behind a conversion
+// of every code, it did not; on the tensor cores (skinny_mma.cuh: exact products of integer codes with BF16 activations, or with the three
+// BF16 planes of FP32 ones, FP32 sums) the same numbers are a few hundred MMAs a warp.  d = 4096, r = 320, Q8, as a CUDA graph, down and up:
+// 16 tokens 23.7 + 19.0 -> 8.6 + 7.9 us, one token 7.3 + 9.0 -> 6.7 + 6.2, 63 tokens 105 + 51 -> 20 + 21; against 64 bits, FP32 streams
+// of 16 tokens, h 4.0e-7 -> 1.4e-7 and u 5.7e-7 -> 1.0e-7 (2-norms).
+//   down: 16 weight rows by a cluster of eight CTAs, an eighth of the row each (an eighth lies in one stream), which a CTA's eight warps share;
+//         a lane's codes are all asked for at once, its activations come from L2 in fragment order as they lie; the parts meet in shared
+//         memory, then across the cluster.
+//   up:   a CTA owns 16 output columns, a warp their rows in one stream; h goes to shared memory once, as planes in fragment order; the
 //         H streams of a column meet in shared memory.
 
 #include "experts.cuh"
+#include "skinny_mma.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -23,280 +28,298 @@
 namespace sxb {
 namespace {
 
-constexpr int kHcThreads = 256;
 constexpr int kStreams = 4;
 constexpr int kChunk = 32;  // codes per chunk: 16 bytes of Q4, 32 of Q8
 constexpr int64_t kMaxRank = 1024;
+static_assert(kChunk == kMmaRun, "a chunk is a run of the MMA's k");
 
 __device__ inline float sigmoid_f32(float z) { return 1.0f / (1.0f + expf(-z)); }
-// 16 bytes of activations as FP32: four (FP32) or eight (BF16) values.
-__device__ inline void unpack16(const uint4 &u, float (&f)[4], const float *) {
-    f[0] = __uint_as_float(u.x), f[1] = __uint_as_float(u.y), f[2] = __uint_as_float(u.z), f[3] = __uint_as_float(u.w);
-}
-__device__ inline void unpack16(const uint4 &u, float (&f)[8], const uint16_t *) {
-    const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) f[2 * j] = __uint_as_float(w4[j] << 16), f[2 * j + 1] = __uint_as_float(w4[j] & 0xffff0000u);
-}
 
-// Eight consecutive codes of a chunk (k = 8 j .. 8 j + 7) as FP32, from the chunk's packed words.
+// A lane's eight codes of a chunk: 8 bytes (Q8) or 4 (Q4).
 template <int BITS>
-__device__ inline void codes8(const uint32_t *w, int j, float (&c)[8]) {
-    if (BITS == 8) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) c[i] = (float)((w[2 * j + (i >> 2)] >> (8 * (i & 3))) & 0xFFu);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) c[i] = (float)((w[j] >> (4 * i)) & 0xFu);
+struct Codes {
+    uint32_t w[BITS / 4];
+    __device__ inline void load(const uint8_t *p) {
+        if constexpr (BITS == 8) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+            w[0] = v.x, w[1] = v.y;
+        } else {
+            w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
+        }
     }
-}
-template <int BITS>
-__device__ inline void load_chunk_words(const uint8_t *p, uint32_t (&w)[BITS]) {
-#pragma unroll
-    for (int i = 0; i < BITS / 4; ++i) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p) + i);
-        w[4 * i] = u.x, w[4 * i + 1] = u.y, w[4 * i + 2] = u.z, w[4 * i + 3] = u.w;
-    }
-}
+    __device__ inline uint4 bf16() const { return codes_bf16<BITS>(w[0], w[BITS / 4 - 1]); }
+};
 
-// hc_mix_down.  grid = (row groups of RG rows, token groups of TT); one CTA of sixteen warps an SM.
-//   1. The TT tokens' streams go to shared memory once (chunk-interleaved: 16-byte piece p of chunk c of token tt at
-//      ((tt * P + p) * nc + c) * 16, so that lanes with consecutive chunks read consecutive 16 bytes), and each chunk's
-//      sum(x) and sum(x^2) - the same for every weight row - are computed once.
-//   2. The work items are (row, eighth of the row's chunks): an eighth lies in one stream (H = 4).  The warps take items in
-//      turn; a lane has only a few chunks of an item and all their loads are in flight together - with a warp walking a whole
-//      row, sixteen dependent rounds of loads made this kernel 57 us at T = 16.  An item's partial dot per token goes to
-//      shared memory.
-//   3. One thread per (row, token) adds the parts in order, applies the per-stream inverse RMS and the activation.
-constexpr int kDownThreads = 512, kParts = 8;
-constexpr int kMaxRowGroup = 32;
+// A lane's eight activations of a chunk of its token, as the BF16 planes they consist of.
+template <typename T>
+struct Acts;
+template <>
+struct Acts<uint16_t> {
+    static constexpr int kPlanes = 1;
+    uint4 v;
+    __device__ inline void load(const uint16_t *p) { v = __ldg(reinterpret_cast<const uint4 *>(p)); }
+    __device__ inline void clear() { v = make_uint4(0u, 0u, 0u, 0u); }
+    __device__ inline void planes(uint4 (&pl)[1]) const { pl[0] = v; }
+    __device__ inline float sum_sq(float s) const {
+        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float lo = __uint_as_float(w4[i] << 16), hi = __uint_as_float(w4[i] & 0xffff0000u);
+            s = fmaf(lo, lo, s), s = fmaf(hi, hi, s);
+        }
+        return s;
+    }
+};
+template <>
+struct Acts<float> {
+    static constexpr int kPlanes = 3;
+    float4 a, b;
+    __device__ inline void load(const float *p) { a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1); }
+    __device__ inline void clear() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ inline void planes(uint4 (&pl)[3]) const {
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        split_planes(f, pl);
+    }
+    __device__ inline float sum_sq(float s) const {
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = fmaf(f[i], f[i], s);
+        return s;
+    }
+};
 
-template <typename T, int BITS, int TT>
-__global__ void __launch_bounds__(kDownThreads, 1) hc_down_kernel(const T *__restrict__ x, const uint8_t *__restrict__ q,
-                                                                  const uint16_t *__restrict__ scale, const uint16_t *__restrict__ minv,
-                                                                  int64_t R, int64_t K, int64_t G, int64_t d, int r, float eps, int64_t Tn,
-                                                                  int RG, float *__restrict__ h, float *__restrict__ w_in,
-                                                                  float *__restrict__ inv) {
-    constexpr int P = kChunk * (int)sizeof(T) / 16;  // 16-byte pieces of a chunk of activations: 4 (BF16) or 8 (FP32)
-    constexpr int kWarps = kDownThreads / 32;
-    extern __shared__ __align__(16) unsigned char down_smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nc = (int)(K / kChunk);
-    uint4 *xs = reinterpret_cast<uint4 *>(down_smem);                                 // [TT][P][nc]
-    float2 *sums = reinterpret_cast<float2 *>(down_smem + (size_t)TT * P * nc * 16);  // [TT][nc]
-    float *part = reinterpret_cast<float *>(sums + (size_t)TT * nc);                  // [RG][kParts][TT]
-    float *ssq = part + (size_t)kMaxRowGroup * kParts * TT;                            // [TT][H]
-    const int64_t t0 = (int64_t)blockIdx.y * TT, n0 = (int64_t)blockIdx.x * RG;
-    const int nt = (int)min((int64_t)TT, Tn - t0), rows = (int)min((int64_t)RG, R - n0);
-    // 1. the activations, all loads of a thread in flight at once (batches of eight)
-    const int pieces_per_token = nc * P;
-    for (int base = threadIdx.x; base < nt * pieces_per_token; base += 8 * kDownThreads) {
-        uint4 v[8];
+// hc_mix_down.  grid = (8 x row tiles, token groups of 8 NT), clusters of eight CTAs along x.
+// A chunk's share of a dot is scale * sum(x * code) + min * sum(x), as the header of this file says; sum(x) comes from an MMA of its own with
+// a matrix of ones for weights, which leaves it in the lanes that need it.  sum(x^2), the same for every weight row, costs a few
+// instructions a chunk and is formed by every cluster for itself.
+constexpr int kDownWarps = 8, kParts = 8;
+constexpr int kCodesAhead = 8;  // chunks whose codes a lane has in flight: d = 4096 gives a warp eight
+template <typename T, int NT> constexpr int kActsAhead = sizeof(T) == 2 ? (NT == 4 ? 1 : 4) : (NT == 1 ? 4 : 1);  // ... whose activations
+
+template <typename T, int BITS, int NT>
+__global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__restrict__ x, const uint8_t *__restrict__ q,
+                                                                     const uint16_t *__restrict__ scale, const uint16_t *__restrict__ minv,
+                                                                     int64_t R, int64_t K, int64_t G, int64_t d, int r, float eps, int64_t Tn,
+                                                                     float *__restrict__ h, float *__restrict__ w_in, float *__restrict__ inv) {
+    constexpr int kTok = kMmaTokens * NT, kAhead = kActsAhead<T, NT>;
+    __shared__ float part[kDownWarps][kTok][kMmaRows + 1];  // + 1: the finishing threads of a token read different banks
+    __shared__ float part_sq[kDownWarps][kTok];
+    __shared__ float cta_part[kTok][kMmaRows], cta_sq[kTok];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const int rank = (int)cluster_rank();
+    const int64_t n0 = (int64_t)(blockIdx.x / kParts) * kMmaRows, t0 = (int64_t)blockIdx.y * kTok;
+    // rows past the end stream the last one; their sums are dropped
+    const int64_t row_bytes = K * BITS / 8, groups = K / G, ra = min(n0 + g, R - 1), rb = min(n0 + g + 8, R - 1);
+    const int per_part = (int)(K / kChunk) / kParts, lo = rank * per_part + per_part * warp / kDownWarps,
+              hi = rank * per_part + per_part * (warp + 1) / kDownWarps;
+    const uint8_t *qa = q + ra * row_bytes + c * BITS, *qb = q + rb * row_bytes + c * BITS;
+    float acc[NT][4], sq[NT];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int i = base + j * kDownThreads;
-            if (i < nt * pieces_per_token) {
-                const int tt = i / pieces_per_token, jj = i % pieces_per_token;
-                v[j] = __ldg(reinterpret_cast<const uint4 *>(x + (t0 + tt) * K) + jj);
-            }
+    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = sq[nt] = 0.f;
+    for (int c0 = lo; c0 < hi; c0 += kCodesAhead) {
+        Codes<BITS> wa[kCodesAhead], wb[kCodesAhead];
+        uint32_t sm_a[kCodesAhead / 4], sm_b[kCodesAhead / 4];  // (scale, min) of rows a and b for chunks c0 + 4 i + c: handed round by shuffles
+#pragma unroll
+        for (int e = 0; e < kCodesAhead; ++e) {
+            const int ch = min(c0 + e, hi - 1);
+            wa[e].load(qa + (int64_t)ch * (kChunk * BITS / 8)), wb[e].load(qb + (int64_t)ch * (kChunk * BITS / 8));
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int i = base + j * kDownThreads;
-            if (i < nt * pieces_per_token) {
-                const int tt = i / pieces_per_token, jj = i % pieces_per_token;
-                xs[(tt * P + jj % P) * nc + jj / P] = v[j];
-            }
+        for (int i = 0; i < kCodesAhead / 4; ++i) {
+            const int64_t gi = (int64_t)min(c0 + 4 * i + c, hi - 1) * kChunk / G;
+            sm_a[i] = __ldg(scale + ra * groups + gi) | (uint32_t)__ldg(minv + ra * groups + gi) << 16;
+            sm_b[i] = __ldg(scale + rb * groups + gi) | (uint32_t)__ldg(minv + rb * groups + gi) << 16;
         }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt * nc; i += kDownThreads) {
-        const int tt = i / nc, c = i % nc;
-        float sx = 0.f, sq = 0.f;
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const uint4 u = xs[(tt * P + p) * nc + c];
-            float f[16 / sizeof(T)];
-            unpack16(u, f, static_cast<const T *>(nullptr));
+        for (int e0 = 0; e0 < kCodesAhead; e0 += kAhead) {
+            if (c0 + e0 >= hi) break;
+            Acts<T> xv[kAhead][NT];
 #pragma unroll
-            for (int k = 0; k < (int)(16 / sizeof(T)); ++k) sx += f[k], sq = fmaf(f[k], f[k], sq);
-        }
-        sums[i] = make_float2(sx, sq);
-    }
-    __syncthreads();
-    // the sum of squares of every (token, stream): one thread each, chunks in order
-    if (threadIdx.x < nt * kStreams) {
-        const int tt = threadIdx.x / kStreams, st = threadIdx.x % kStreams, per = nc / kStreams;
-        float sq = 0.f;
-        for (int c = st * per; c < (st + 1) * per; ++c) sq += sums[tt * nc + c].y;
-        ssq[threadIdx.x] = sq;
-    }
-    // 2. items (row, part): chunks [part * nc / 8, (part + 1) * nc / 8) of row n0 + row
-    const int64_t row_bytes = K * BITS / 8, groups = K / G;
-    const int per_part = nc / kParts;
-    for (int item = warp; item < rows * kParts; item += kWarps) {
-        const int row = item / kParts, pt = item % kParts;
-        const int64_t n = n0 + row;
-        float acc[TT];
+            for (int e = 0; e < kAhead; ++e)
 #pragma unroll
-        for (int tt = 0; tt < TT; ++tt) acc[tt] = 0.f;
-        // a lane's chunks of the item two at a time, both chunks' loads issued before either is used
-        for (int c0 = pt * per_part + lane; c0 < (pt + 1) * per_part; c0 += 64) {
-            uint32_t w[2][BITS];
-            float sc[2], mn[2];
-            const bool two = c0 + 32 < (pt + 1) * per_part;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int c = e == 0 || two ? c0 + 32 * e : c0;
-                load_chunk_words<BITS>(q + n * row_bytes + (int64_t)c * (kChunk * BITS / 8), w[e]);
-                sc[e] = bf16_bits_to_f32(__ldg(scale + n * groups + c * kChunk / G));
-                mn[e] = bf16_bits_to_f32(__ldg(minv + n * groups + c * kChunk / G));
-            }
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (e == 1 && !two) break;
-                const int c = c0 + 32 * e;
-                float dsum[TT];
-#pragma unroll
-                for (int tt = 0; tt < TT; ++tt) dsum[tt] = 0.f;
-#pragma unroll
-                for (int j = 0; j < kChunk / 8; ++j) {  // eight codes at a time: converted once, met by every token
-                    float cf[8];
-                    codes8<BITS>(w[e], j, cf);
-#pragma unroll
-                    for (int tt = 0; tt < TT; ++tt) {
-                        if (tt >= nt) break;
-                        float f[8];
-                        if constexpr (sizeof(T) == 2) {
-                            unpack16(xs[(tt * P + j) * nc + c], f, static_cast<const T *>(nullptr));
-                        } else {
-                            float g4[4];
-                            unpack16(xs[(tt * P + 2 * j) * nc + c], g4, static_cast<const T *>(nullptr));
-                            f[0] = g4[0], f[1] = g4[1], f[2] = g4[2], f[3] = g4[3];
-                            unpack16(xs[(tt * P + 2 * j + 1) * nc + c], g4, static_cast<const T *>(nullptr));
-                            f[4] = g4[0], f[5] = g4[1], f[6] = g4[2], f[7] = g4[3];
-                        }
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) dsum[tt] = fmaf(f[k], cf[k], dsum[tt]);
-                    }
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int64_t t = t0 + nt * kMmaTokens + g;
+                    if (t < Tn && c0 + e0 + e < hi) xv[e][nt].load(x + t * K + (int64_t)(c0 + e0 + e) * kChunk + 8 * c);
+                    else xv[e][nt].clear();
                 }
 #pragma unroll
-                for (int tt = 0; tt < TT; ++tt)
-                    if (tt < nt) acc[tt] += fmaf(sc[e], dsum[tt], mn[e] * sums[tt * nc + c].x);
+            for (int e = 0; e < kAhead; ++e) {
+                const int i = e0 + e;
+                if (c0 + i >= hi) break;
+                const uint4 va = wa[i].bf16(), vb = wb[i].bf16(), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+                const uint32_t p_a = __shfl_sync(0xffffffffu, sm_a[i / 4], (lane & ~3) + i % 4), p_b = __shfl_sync(0xffffffffu, sm_b[i / 4], (lane & ~3) + i % 4);
+                const float s_a = __uint_as_float(p_a << 16), m_a = centered_min<BITS>(s_a, __uint_as_float(p_a & 0xffff0000u));
+                const float s_b = __uint_as_float(p_b << 16), m_b = centered_min<BITS>(s_b, __uint_as_float(p_b & 0xffff0000u));
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) {
+                    uint4 pl[Acts<T>::kPlanes];
+                    xv[e][nt].planes(pl);
+                    float dot[4] = {0.f, 0.f, 0.f, 0.f}, sx[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int p = Acts<T>::kPlanes - 1; p >= 0; --p) mma_run(dot, va, vb, pl[p]), mma_run(sx, ones, ones, pl[p]);
+                    acc[nt][0] = fmaf(s_a, dot[0], fmaf(m_a, sx[0], acc[nt][0])), acc[nt][1] = fmaf(s_a, dot[1], fmaf(m_a, sx[1], acc[nt][1]));
+                    acc[nt][2] = fmaf(s_b, dot[2], fmaf(m_b, sx[0], acc[nt][2])), acc[nt][3] = fmaf(s_b, dot[3], fmaf(m_b, sx[1], acc[nt][3]));
+                    sq[nt] = xv[e][nt].sum_sq(sq[nt]);
+                }
             }
         }
+    }
 #pragma unroll
-        for (int tt = 0; tt < TT; ++tt) {
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc[tt] += __shfl_xor_sync(0xffffffffu, acc[tt], off);
-            if (lane == 0) part[(row * kParts + pt) * TT + tt] = acc[tt];
-        }
+    for (int nt = 0; nt < NT; ++nt) {
+        const int t = nt * kMmaTokens + 2 * c;
+        part[warp][t][g] = acc[nt][0], part[warp][t + 1][g] = acc[nt][1];
+        part[warp][t][g + 8] = acc[nt][2], part[warp][t + 1][g + 8] = acc[nt][3];
+        sq[nt] += __shfl_xor_sync(0xffffffffu, sq[nt], 1);
+        sq[nt] += __shfl_xor_sync(0xffffffffu, sq[nt], 2);
+        if (c == 0) part_sq[warp][nt * kMmaTokens + g] = sq[nt];
     }
     __syncthreads();
-    // 3. one thread per (row, token)
-    for (int i = threadIdx.x; i < rows * nt; i += kDownThreads) {
-        const int row = i / nt, tt = i % nt;
-        const int64_t n = n0 + row, t = t0 + tt;
-        float a = 0.f;
+    for (int i = threadIdx.x; i < kTok * kMmaRows; i += 32 * kDownWarps) {
+        float sum = 0.f;
 #pragma unroll
-        for (int st = 0; st < kStreams; ++st) {
-            float dot = 0.f;
-#pragma unroll
-            for (int k = 0; k < kParts / kStreams; ++k) dot += part[(row * kParts + st * (kParts / kStreams) + k) * TT + tt];
-            a = fmaf(1.0f / sqrtf(ssq[tt * kStreams + st] / (float)d + eps), dot, a);
-        }
-        const float z = a / (float)kStreams;
-        if (n < r) h[t * r + n] = z * sigmoid_f32(z);
-        else w_in[t * kStreams + (n - r)] = 2.0f * sigmoid_f32(z);
+        for (int w = 0; w < kDownWarps; ++w) sum += part[w][i / kMmaRows][i % kMmaRows];
+        cta_part[i / kMmaRows][i % kMmaRows] = sum;
     }
-    if (n0 == 0 && threadIdx.x < nt * kStreams)
-        inv[(t0 + threadIdx.x / kStreams) * kStreams + threadIdx.x % kStreams] = 1.0f / sqrtf(ssq[threadIdx.x] / (float)d + eps);
+    if (threadIdx.x < kTok) {
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < kDownWarps; ++w) sum += part_sq[w][threadIdx.x];
+        cta_sq[threadIdx.x] = sum;
+    }
+    cluster_sync();
+    // A CTA of the cluster finishes every eighth token: its sixteen rows' dots, their streams' inverse RMS, the activation.
+    if (threadIdx.x < NT * kMmaRows) {
+        const int tt = rank + kParts * (threadIdx.x / kMmaRows), row = threadIdx.x % kMmaRows;
+        const int64_t n = n0 + row, t = t0 + tt;
+        if (n < R && t < Tn) {
+            float dots[kParts], sqs[kParts];
+#pragma unroll
+            for (int p = 0; p < kParts; ++p) dots[p] = ld_cluster(&cta_part[tt][row], p), sqs[p] = ld_cluster(&cta_sq[tt], p);
+            float a = 0.f;
+#pragma unroll
+            for (int st = 0; st < kStreams; ++st) {
+                const float rms = 1.0f / sqrtf((sqs[2 * st] + sqs[2 * st + 1]) / (float)d + eps);
+                a = fmaf(rms, dots[2 * st] + dots[2 * st + 1], a);
+                if (n == 0) inv[t * kStreams + st] = rms;
+            }
+            const float z = a / (float)kStreams;
+            if (n < r) h[t * r + n] = z * sigmoid_f32(z);
+            else w_in[t * kStreams + (n - r)] = 2.0f * sigmoid_f32(z);
+        }
+    }
+    cluster_sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// hc_mix_up.  grid = (d / 64, token groups of MT); thread (s, jl) owns row s*d + j of W_up.  Four chunks of packed codes are
-// in flight per thread (a thread has only r / 32 chunks, and one at a time made this kernel ten rounds of load latency).
-constexpr int kUpCols = kHcThreads / kStreams;  // 64 output columns per CTA
-constexpr int kUpAhead = 4;
+// hc_mix_up.  grid = (d / 16, token groups of 8 NT); warp s owns rows s * d + 16 blockIdx.x .. + 15 of W_up, whose chunks lie side by side in
+// the chunk-major layout.  h is an FP32 number and stays one: three BF16 planes.
+constexpr int kUpCols = kMmaRows;  // output columns per CTA
+constexpr int kUpAhead = 10;       // chunks of codes in flight per warp: r = 320 has ten
 
-template <typename T, int BITS, int MT>
-__global__ void __launch_bounds__(kHcThreads) hc_up_kernel(const float *__restrict__ h, const uint8_t *__restrict__ q,
-                                                           const uint16_t *__restrict__ scale, const uint16_t *__restrict__ minv, int64_t G,
-                                                           const T *__restrict__ x, const float *__restrict__ norm_w,
-                                                           const float *__restrict__ inv, int64_t d, int r, int64_t Tn, T *__restrict__ u) {
-    extern __shared__ float up_smem[];  // hs [MT][r], hsum [MT][r / 32], part [MT][H][64]
-    float *hs = up_smem, *hsum = hs + (size_t)MT * r, *part = hsum + (size_t)MT * (r / kChunk);
-    const int64_t t0 = (int64_t)blockIdx.y * MT, N = kStreams * d;
-    const int nt = (int)min((int64_t)MT, Tn - t0), chunks = r / kChunk;
-    const int s = threadIdx.x / kUpCols, jl = threadIdx.x % kUpCols;
-    const int64_t j = (int64_t)blockIdx.x * kUpCols + jl, row = s * d + min(j, d - 1);
+template <typename T, int BITS, int NT>
+__global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__restrict__ h, const uint8_t *__restrict__ q,
+                                                              const uint16_t *__restrict__ scale, const uint16_t *__restrict__ minv, int64_t G,
+                                                              const T *__restrict__ x, const float *__restrict__ norm_w,
+                                                              const float *__restrict__ inv, int64_t d, int r, int64_t Tn, bool vec_h, T *__restrict__ u) {
+    constexpr int kTok = kMmaTokens * NT;
+    extern __shared__ __align__(16) unsigned char up_smem[];
+    const int chunks = r / kChunk;
+    uint4 *planes = reinterpret_cast<uint4 *>(up_smem);                      // [chunk][nt][plane][lane]
+    float *hsum = reinterpret_cast<float *>(planes + (size_t)chunks * NT * 3 * 32);  // [chunk][token]
+    __shared__ float part[kStreams][kTok][kUpCols + 1];
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const int64_t N = kStreams * d, j0 = (int64_t)blockIdx.x * kUpCols, row = s * d + j0 + g, t0 = (int64_t)blockIdx.y * kTok;
     // the first chunks' codes are asked for before anything else
-    uint32_t wq[kUpAhead][BITS];
-    float sc[kUpAhead], mn[kUpAhead];
-    auto fetch = [&](int slot, int c) {
-        load_chunk_words<BITS>(q + ((int64_t)c * N + row) * (kChunk * BITS / 8), wq[slot]);
-        const int64_t gi = (int64_t)(c * kChunk / G) * N + row;
-        sc[slot] = bf16_bits_to_f32(__ldg(scale + gi)), mn[slot] = bf16_bits_to_f32(__ldg(minv + gi));
+    Codes<BITS> wa[kUpAhead], wb[kUpAhead];
+    uint16_t sa[kUpAhead], sb[kUpAhead], ma[kUpAhead], mb[kUpAhead];
+    auto fetch = [&](int slot, int ch) {
+        const uint8_t *p = q + ((int64_t)ch * N + row) * (kChunk * BITS / 8) + c * BITS;
+        wa[slot].load(p), wb[slot].load(p + 8 * (kChunk * BITS / 8));
+        const int64_t gi = (int64_t)ch * kChunk / G * N + row;
+        sa[slot] = __ldg(scale + gi), ma[slot] = __ldg(minv + gi), sb[slot] = __ldg(scale + gi + 8), mb[slot] = __ldg(minv + gi + 8);
     };
 #pragma unroll
     for (int a = 0; a < kUpAhead; ++a)
         if (a < chunks) fetch(a, a);
-    for (int i = threadIdx.x; i < nt * r; i += kHcThreads) hs[i] = h[t0 * r + i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt * chunks; i += kHcThreads) {
-        float sum = 0.f;
-        for (int k = 0; k < kChunk; ++k) sum += hs[(i / chunks) * r + (i % chunks) * kChunk + k];
-        hsum[i] = sum;
+    // what the tokens' terms take beside z: the lane's tokens are 2 c and 2 c + 1 of each eight, its columns g and g + 8
+    float xi[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t t = t0 + nt * kMmaTokens + 2 * c + (i & 1);
+            xi[nt][i] = t < Tn ? load_as_f32(x, t * N + row + 8 * (i >> 1)) * inv[t * kStreams + s] * (1.0f + norm_w[row + 8 * (i >> 1)]) : 0.f;
+        }
+    constexpr int kStage = 5;  // runs of h a warp has in flight: one at a time, each iteration was a round trip to L2
+    for (int i0 = s; i0 < chunks * NT; i0 += kStage * kStreams) {
+        float v[kStage][8];
+#pragma unroll
+        for (int b = 0; b < kStage; ++b) {
+            const int i = i0 + b * kStreams, ch = i / NT;
+            const int64_t t = t0 + i % NT * kMmaTokens + g;
+            const float *hp = h + t * r + ch * kChunk + 8 * c;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[b][k] = 0.f;
+            if (i < chunks * NT && t < Tn) {
+                if (vec_h) {
+                    const float4 p = reinterpret_cast<const float4 *>(hp)[0], q4 = reinterpret_cast<const float4 *>(hp)[1];
+                    v[b][0] = p.x, v[b][1] = p.y, v[b][2] = p.z, v[b][3] = p.w, v[b][4] = q4.x, v[b][5] = q4.y, v[b][6] = q4.z, v[b][7] = q4.w;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[b][k] = hp[k];
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < kStage; ++b) {
+            const int i = i0 + b * kStreams;
+            if (i >= chunks * NT) break;
+            uint4 pl[3];
+            split_planes(v[b], pl);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) planes[(i * 3 + p) * 32 + lane] = pl[p];
+            float sum = ((v[b][0] + v[b][1]) + (v[b][2] + v[b][3])) + ((v[b][4] + v[b][5]) + (v[b][6] + v[b][7]));
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            if (c == 0) hsum[i / NT * kTok + i % NT * kMmaTokens + g] = sum;
+        }
     }
     __syncthreads();
-    float acc[MT];
+    float acc[NT][4];
 #pragma unroll
-    for (int tt = 0; tt < MT; ++tt) acc[tt] = 0.f;
+    for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     for (int c0 = 0; c0 < chunks; c0 += kUpAhead) {
 #pragma unroll
         for (int a = 0; a < kUpAhead; ++a) {
-            const int c = c0 + a;
-            if (c >= chunks) break;
-            float dsum[MT];
+            const int ch = c0 + a;
+            if (ch >= chunks) break;
+            const uint4 va = wa[a].bf16(), vb = wb[a].bf16();
+            const float s_a = bf16_bits_to_f32(sa[a]), m_a = centered_min<BITS>(s_a, bf16_bits_to_f32(ma[a]));
+            const float s_b = bf16_bits_to_f32(sb[a]), m_b = centered_min<BITS>(s_b, bf16_bits_to_f32(mb[a]));
 #pragma unroll
-            for (int tt = 0; tt < MT; ++tt) dsum[tt] = 0.f;
+            for (int nt = 0; nt < NT; ++nt) {
+                float dot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int jj = 0; jj < kChunk / 8; ++jj) {
-                float cf[8];
-                codes8<BITS>(wq[a], jj, cf);
-#pragma unroll
-                for (int tt = 0; tt < MT; ++tt) {
-                    if (tt >= nt) break;
-                    // two 16-byte broadcasts instead of eight scalar ones: the shared-memory pipe was this kernel's limit
-                    const float4 *hv = reinterpret_cast<const float4 *>(hs + tt * r + c * kChunk + jj * 8);
-                    const float4 h0 = hv[0], h1 = hv[1];
-                    const float hf[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) dsum[tt] = fmaf(hf[k], cf[k], dsum[tt]);
-                }
+                for (int p = 2; p >= 0; --p) mma_run(dot, va, vb, planes[((ch * NT + nt) * 3 + p) * 32 + lane]);
+                const float2 hs = *reinterpret_cast<const float2 *>(hsum + ch * kTok + nt * kMmaTokens + 2 * c);
+                acc[nt][0] = fmaf(s_a, dot[0], fmaf(m_a, hs.x, acc[nt][0])), acc[nt][1] = fmaf(s_a, dot[1], fmaf(m_a, hs.y, acc[nt][1]));
+                acc[nt][2] = fmaf(s_b, dot[2], fmaf(m_b, hs.x, acc[nt][2])), acc[nt][3] = fmaf(s_b, dot[3], fmaf(m_b, hs.y, acc[nt][3]));
             }
-#pragma unroll
-            for (int tt = 0; tt < MT; ++tt)
-                if (tt < nt) acc[tt] = fmaf(sc[a], dsum[tt], fmaf(mn[a], hsum[tt * chunks + c], acc[tt]));
-            if (c + kUpAhead < chunks) fetch(a, c + kUpAhead);  // the slot's codes are spent: the chunk four ahead
+            if (ch + kUpAhead < chunks) fetch(a, ch + kUpAhead);  // the slot's codes are spent
         }
     }
-    if (j < d) {
-        const float nw = 1.0f + norm_w[row];
 #pragma unroll
-        for (int tt = 0; tt < MT; ++tt) {
-            if (tt >= nt) break;
-            const int64_t t = t0 + tt;
-            part[(tt * kStreams + s) * kUpCols + jl] = sigmoid_f32(acc[tt]) * (load_as_f32(x, t * N + row) * inv[t * kStreams + s] * nw);
-        }
-    }
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[s][nt * kMmaTokens + 2 * c + (i & 1)][g + 8 * (i >> 1)] = sigmoid_f32(acc[nt][i]) * xi[nt][i];
     __syncthreads();
-    if (s == 0 && j < d)
-        for (int tt = 0; tt < nt; ++tt) {
-            float sum = 0.f;
+    for (int i = threadIdx.x; i < kTok * kUpCols; i += 32 * kStreams) {
+        const int tt = i / kUpCols, j = i % kUpCols;
+        if (t0 + tt >= Tn) break;
+        float sum = 0.f;
 #pragma unroll
-            for (int k = 0; k < kStreams; ++k) sum += part[(tt * kStreams + k) * kUpCols + jl];
-            store_from_f32(u, (t0 + tt) * d + j, sum / (float)kStreams);
-        }
+        for (int k = 0; k < kStreams; ++k) sum += part[k][tt][j];
+        store_from_f32(u, (t0 + tt) * d + j0 + j, sum / (float)kStreams);
+    }
 }
 
 // Row-major Q4 / Q8 -> chunk-major (formats/q4.hpp:41-55): 32-code chunk c of row n at q[(c * N + n) * chunk bytes], group
@@ -314,6 +337,10 @@ __global__ void __launch_bounds__(256) chunk_major_kernel(const uint8_t *__restr
         so[g * N + n] = scale[i], mo[g * N + n] = minv[i];
     }
 }
+
+// Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Four where the last 32 are more than half
+// full (63 tokens, d = 4096 Q8, down + up: 41 us, 45 with two; 40 tokens: 39 and 32).
+int token_eights(int64_t T) { return T <= 8 ? 1 : T <= 16 || (T < 64 && (T - 1) % 32 < 16) ? 2 : 4; }
 
 int check_hc_shape(const char *fn, int64_t T, int64_t H, int64_t d) {
     SXB_CHECK(H == kStreams, fn, ": H = ", H, " streams, only ", kStreams, " is supported");
@@ -345,36 +372,26 @@ int mix_down(const void *x, const SxbQView *w, int64_t T, int64_t H, int64_t d, 
     SXB_CHECK(aligned16(x), fn, ": x ", x, " must be 16-byte aligned");
     SXB_CHECK(std::isfinite(eps) && eps > 0.f, fn, ": eps must be finite and > 0, got ", eps);
     SXB_CHECK((w->K / kChunk) % kParts == 0, fn, ": H*d = ", w->K, " must be a multiple of ", kChunk * kParts, " (eight parts of whole chunks a row)");
-    // Tokens per CTA: as many as shared memory holds (up to four); rows per CTA: so that the grid is one wave of CTAs.
-    const size_t es = act == SXB_ACT_F32 ? 4 : 2, per_token = (size_t)w->K * es + (size_t)(w->K / kChunk) * sizeof(float2);
-    const size_t fixed = (size_t)kMaxRowGroup * kParts * 4 * sizeof(float) + 64 * sizeof(float);
-    int TT = 4;
-    while (TT > 1 && (TT * per_token + fixed > 200 * 1024 || TT > T)) TT >>= 1;
-    SXB_CHECK(TT * per_token + fixed <= 200 * 1024, fn, ": H*d = ", w->K, " needs ", per_token, " bytes of shared memory a token");
-    const int64_t token_groups = (T + TT - 1) / TT;
-    int64_t row_groups = std::max<int64_t>(1, std::min<int64_t>(R, sm_count() / token_groups));
-    int RG = (int)std::min<int64_t>(kMaxRowGroup, (R + row_groups - 1) / row_groups);
-    row_groups = (R + RG - 1) / RG;
-    const size_t smem = TT * per_token + fixed;
-    auto st = static_cast<cudaStream_t>(stream);
-#define SXB_HC_DOWN(TYPE, TTV)                                                                                                         \
-    do {                                                                                                                               \
-        auto kern = hc_down_kernel<TYPE, BITS, TTV>;                                                                                   \
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory"); \
-        const dim3 grid((unsigned)row_groups, (unsigned)token_groups);                                                                 \
-        kern<<<grid, kDownThreads, smem, st>>>(static_cast<const TYPE *>(x), w->q, w->scale, w->minv, R, w->K, w->G, d, (int)r, eps, T, RG, h, \
-                                               w_in, inv);                                                                             \
-    } while (0)
-#define SXB_HC_DOWN_T(TYPE)                     \
-    do {                                        \
-        if (TT == 4) SXB_HC_DOWN(TYPE, 4);      \
-        else if (TT == 2) SXB_HC_DOWN(TYPE, 2); \
-        else SXB_HC_DOWN(TYPE, 1);              \
-    } while (0)
-    if (act == SXB_ACT_F32) SXB_HC_DOWN_T(float);
-    else SXB_HC_DOWN_T(uint16_t);
-#undef SXB_HC_DOWN_T
-#undef SXB_HC_DOWN
+    const size_t per_token = (size_t)w->K * act_bytes(act) + (size_t)(w->K / kChunk) * 8;  // the limit of a row of streams, 200 KB
+    SXB_CHECK(per_token + 4352 <= 200 * 1024, fn, ": H*d = ", w->K, " needs ", per_token, " bytes a token, limit ", 200 * 1024 - 4352);
+    const int NT = act == SXB_ACT_F32 ? std::min(2, token_eights(T)) : token_eights(T);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension, attr.val.clusterDim.x = kParts, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)((R + kMmaRows - 1) / kMmaRows * kParts), (unsigned)((T + NT * kMmaTokens - 1) / (NT * kMmaTokens)));
+    cfg.blockDim = dim3(32 * kDownWarps), cfg.stream = static_cast<cudaStream_t>(stream), cfg.attrs = &attr, cfg.numAttrs = 1;
+    auto launch = [&](auto kern, auto *xt) {
+        return cudaLaunchKernelEx(&cfg, kern, xt, w->q, w->scale, w->minv, R, w->K, w->G, d, (int)r, eps, T, h, w_in, inv);
+    };
+    cudaError_t e;
+    if (act == SXB_ACT_F32) {
+        auto xt = static_cast<const float *>(x);
+        e = NT == 1 ? launch(hc_down_kernel<float, BITS, 1>, xt) : launch(hc_down_kernel<float, BITS, 2>, xt);
+    } else {
+        auto xt = static_cast<const uint16_t *>(x);
+        e = NT == 1 ? launch(hc_down_kernel<uint16_t, BITS, 1>, xt) : NT == 2 ? launch(hc_down_kernel<uint16_t, BITS, 2>, xt) : launch(hc_down_kernel<uint16_t, BITS, 4>, xt);
+    }
+    SXB_CUDA(e, fn, ": launching T=", T, " R=", R, " K=", w->K);
     SXB_CHECK_LAUNCH(fn, " Q", BITS, " ", act_name(act), " T=", T, " R=", R, " K=", w->K, " G=", w->G);
     return SXB_OK;
 }
@@ -392,31 +409,30 @@ int mix_up(const float *h, const SxbQView *w, const void *x, const float *norm_w
     SXB_CHECK(w->K >= kChunk && w->K <= kMaxRank && w->K % kChunk == 0, fn, ": W_up K (the rank r) = ", w->K, ", expected a multiple of ",
               kChunk, " up to ", kMaxRank);
     SXB_CHECK(apart(u, T * d * act_bytes(act), x, T * H * d * act_bytes(act)), fn, ": u overlaps the streams x");
-    const int64_t r = w->K, col_groups = (d + kUpCols - 1) / kUpCols;
-    int MT = 8;
-    while (MT > 1 && (col_groups * ((T + MT - 1) / MT) < sm_count() || MT > T)) MT >>= 1;
-    const size_t smem = ((size_t)MT * r + (size_t)MT * (r / kChunk) + (size_t)MT * kStreams * kUpCols) * sizeof(float);
+    const int64_t r = w->K;
+    const int NT = token_eights(T);
+    const size_t smem = (size_t)(r / kChunk) * NT * (3 * 32 * sizeof(uint4) + kMmaTokens * sizeof(float));
+    const bool vec_h = aligned16(h);
     auto st = static_cast<cudaStream_t>(stream);
-#define SXB_HC_UP(TYPE, MTV)                                                                                                           \
+#define SXB_HC_UP(TYPE, NTV)                                                                                                           \
     do {                                                                                                                               \
-        auto kern = hc_up_kernel<TYPE, BITS, MTV>;                                                                                     \
+        auto kern = hc_up_kernel<TYPE, BITS, NTV>;                                                                                     \
         SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory"); \
-        const dim3 grid((unsigned)col_groups, (unsigned)((T + MTV - 1) / MTV));                                                        \
-        kern<<<grid, kHcThreads, smem, st>>>(h, w->q, w->scale, w->minv, w->G, static_cast<const TYPE *>(x), norm_w, inv, d, (int)r, T,    \
-                                             static_cast<TYPE *>(u));                                                                  \
+        const dim3 grid((unsigned)(d / kUpCols), (unsigned)((T + NTV * kMmaTokens - 1) / (NTV * kMmaTokens)));                          \
+        kern<<<grid, 32 * kStreams, smem, st>>>(h, w->q, w->scale, w->minv, w->G, static_cast<const TYPE *>(x), norm_w, inv, d, (int)r, T,  \
+                                                vec_h, static_cast<TYPE *>(u));                                                        \
     } while (0)
 #define SXB_HC_UP_T(TYPE)                    \
     do {                                     \
-        if (MT == 8) SXB_HC_UP(TYPE, 8);     \
-        else if (MT == 4) SXB_HC_UP(TYPE, 4);\
-        else if (MT == 2) SXB_HC_UP(TYPE, 2);\
+        if (NT == 4) SXB_HC_UP(TYPE, 4);     \
+        else if (NT == 2) SXB_HC_UP(TYPE, 2);\
         else SXB_HC_UP(TYPE, 1);             \
     } while (0)
     if (act == SXB_ACT_F32) SXB_HC_UP_T(float);
     else SXB_HC_UP_T(uint16_t);
 #undef SXB_HC_UP_T
 #undef SXB_HC_UP
-    SXB_CHECK_LAUNCH(fn, " Q", BITS, " ", act_name(act), " T=", T, " d=", d, " r=", r, " G=", w->G, " MT=", MT);
+    SXB_CHECK_LAUNCH(fn, " Q", BITS, " ", act_name(act), " T=", T, " d=", d, " r=", r, " G=", w->G, " NT=", NT);
     return SXB_OK;
 }
 

@@ -1,0 +1,94 @@
+// Warp-level MMA with FP32 arithmetic for skinny products: 16 weight rows x 8 tokens x 16 k of BF16 operands, exact products, FP32
+// sums.  An FP32 operand goes through as three BF16 planes, which together hold its 24 bits, each plane's products as exact.
+//
+// k inside a run of 32 is permuted the same way on both operands, which a dot product does not notice: lane (g = lane / 4, c = lane
+// % 4) holds elements 8 c .. 8 c + 7 of its weight rows g and g + 8 and of its token g, i.e. whole runs of eight consecutive
+// elements that a 16-byte load fetches; the run's first MMA takes elements 0 - 3, the second 4 - 7.
+// Results: d[0], d[1] = row g x tokens 2 c, 2 c + 1; d[2], d[3] = row g + 8 x the same.
+#pragma once
+
+#include "common.cuh"
+
+namespace sxb {
+
+constexpr int kMmaRows = 16, kMmaTokens = 8, kMmaRun = 32;  // weight rows, tokens and k of a step
+
+__device__ inline void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// d += a 32-k run: a, b = the lane's eight elements of rows g and g + 8, x = of its token, as BF16 pairs.
+__device__ inline void mma_run(float (&d)[4], const uint4 &a, const uint4 &b, const uint4 &x) {
+    mma_bf16(d, a.x, b.x, a.y, b.y, x.x, x.y);
+    mma_bf16(d, a.z, b.z, a.w, b.w, x.z, x.w);
+}
+
+// Two FP32 values that fit BF16 as a pair (the first in the lower half).
+__device__ inline uint32_t pack_bf16_exact(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+// The upper sixteen bits of an FP32 value: a BF16, and what is left of the value is an FP32 with eight bits fewer.
+__device__ inline float bf16_part(float v) { return __uint_as_float(__float_as_uint(v) & 0xffff0000u); }
+
+// Eight FP32 values as three BF16 planes whose sum they are, bit for bit (down to BF16's smallest exponent).
+__device__ inline void split_planes(const float (&v)[8], uint4 (&p)[3]) {
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float a = v[2 * i], b = v[2 * i + 1];
+        const float a1 = a - bf16_part(a), b1 = b - bf16_part(b);
+        w[0][i] = pack_bf16_exact(a, b), w[1][i] = pack_bf16_exact(a1, b1);
+        w[2][i] = pack_bf16_exact(a1 - bf16_part(a1), b1 - bf16_part(b1));
+    }
+#pragma unroll
+    for (int j = 0; j < 3; ++j) p[j] = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+}
+
+// The lane's eight codes of a row, less the middle of their range, as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).  What is taken
+// off goes to the group's min (centered_min); without it the sums carry the codes' mean times sum(x), which the min takes off again, and
+// the rounding of the larger sums stays.
+template <int BITS> constexpr float kCenter = BITS == 8 ? 128.f : 8.f;
+template <int BITS>
+__device__ inline float centered_min(float s, float m) { return fmaf(kCenter<BITS>, s, m); }
+template <int BITS>
+__device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1) {
+    constexpr float kOff = 0x1p23f + kCenter<BITS>;
+    uint32_t r[4];
+    if (BITS == 8) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t w = i < 2 ? w0 : w1;  // 2^23 + code, less 2^23 and the center: no conversion instruction, which runs at a quarter rate
+            const float lo = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7442 : 0x7440)) - kOff;
+            const float hi = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7443 : 0x7441)) - kOff;
+            r[i] = pack_bf16_exact(lo, hi);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float lo = __uint_as_float(0x4B000000u | ((w0 >> (8 * i)) & 15u)) - kOff;
+            const float hi = __uint_as_float(0x4B000000u | ((w0 >> (8 * i + 4)) & 15u)) - kOff;
+            r[i] = pack_bf16_exact(lo, hi);
+        }
+    }
+    return make_uint4(r[0], r[1], r[2], r[3]);
+}
+
+// ---- the CTAs of a cluster -------------------------------------------------------------------------------------------
+__device__ inline uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ inline void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// A float of another CTA's shared memory, at the place that `p` has in this CTA's.
+__device__ inline float ld_cluster(const float *p, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+    return v;
+}
+
+}  // namespace sxb

@@ -33,6 +33,7 @@
 // once per tile (once in total when an expert has <= 8 tokens, the decode case).
 
 #include "experts.cuh"
+#include "skinny_mma.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -125,13 +126,6 @@ __device__ inline void unit_mma(float (&d)[4], uint32_t a_w0, uint32_t a_w1, uin
 }
 
 __device__ inline float pow2f(int e) { return __int_as_float((e + 127) << 23); }  // e in -126 .. 127
-
-__device__ inline void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // What stage_tile finds out about a token of the tile.
 template <int BITS> constexpr bool kKeepLow = BITS == 8;  // see the head of this file

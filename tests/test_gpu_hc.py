@@ -63,6 +63,54 @@ def test_hc_mix(cuda, oracle, dt, bits, G, T, d, r, inject):
         assert np.all(np.abs(got - u_ref) <= 2.0 ** -8 * np.abs(u_ref) + 1e-5 * np.sqrt(np.mean(u_ref ** 2)))  # one BF16 rounding
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,G,T,d,r", [(8, 64, 8, 64, 32), (4, 32, 9, 192, 1024), (8, 32, 17, 320, 352), (4, 64, 33, 64, 64), (8, 64, 49, 2560, 320)])
+def test_hc_mix_edges(cuda, oracle, dt, bits, G, T, d, r):
+    """The edges of the tensor-core tiles: rows past a tile of 16, groups of 8 / 16 / 32 tokens that are full, one over, or partly filled, warps
+    without a chunk (d = 64), the longest rank, an h that 16-byte loads may not read; and a token's results do not depend on its batch.
+    FP32 sums of exact products: a dot of n terms, added in any order, is within n 2^-24 sum|terms| of 64 bits; the sums below are
+    chains of at most 256 (MMAs of a warp, groups, warps, CTAs), so 2^-16 sum|terms| with the activation functions' few ulp."""
+    from strixite_b200 import kernels as K
+    H, eps = 4, 1e-6
+    rng = np.random.default_rng(T * 3 + d + r)
+    R = r + H
+    wd = oracle.quantize(random_weights(rng, R, H * d, std=0.05), G, bits)
+    wu = oracle.quantize(random_weights(rng, H * d, r, std=0.2), 32 if r % G else G, bits)
+    norm_w = (rng.standard_normal(H * d) * 0.1).astype(np.float32)
+    x = (rng.standard_normal((T, H * d)) * np.repeat(rng.random((T, H)) * 3 + 0.2, d, axis=1)).astype(np.float32)
+    act = K.Act.F32
+    xd = torch.from_numpy(x).to(cuda)
+    if dt == torch.bfloat16:
+        xd, act = xd.to(torch.bfloat16), K.Act.BF16
+        x = xd.float().cpu().numpy()
+    wdd, wud, nw = upload(wd, cuda), K.to_chunk_major(upload(wu, cuda)), torch.from_numpy(norm_w).to(cuda)
+
+    def mix(xt):
+        n = xt.shape[0]
+        h = torch.full((n * r + 1,), float("nan"), dtype=torch.float32, device=cuda)[1:].view(n, r)  # 4-byte aligned
+        w_in, inv = (torch.full((n, H), float("nan"), dtype=torch.float32, device=cuda) for _ in range(2))
+        u = torch.empty((n, d), dtype=dt, device=cuda)
+        K.hc_mix_down(xt, wdd, n, H, d, r, True, eps, h, w_in, inv, act)
+        K.hc_mix_up(h, wud, xt, nw, inv, n, H, d, u, act)
+        return h, w_in, inv, u
+
+    h, w_in, inv, u = mix(xd)
+    h_ref, w_in_ref, inv_ref = oracle.hc_mix_down(x, wd, H, d, r, True, eps)
+    assert np.max(np.abs(inv.cpu().numpy() / inv_ref - 1)) <= 2.0 ** -20
+    terms = np.abs(x.reshape(T, H, d) * inv_ref[:, :, None]).reshape(T, H * d) @ np.abs(oracle.affine_weights(wd)).T / H
+    assert np.all(np.abs(h.cpu().numpy() - h_ref) <= 2.0 ** -16 * terms[:, :r])
+    assert np.all(np.abs(w_in.cpu().numpy() - w_in_ref) <= 2.0 ** -16 * terms[:, r:] + 2.0 ** -20)
+    hn = h.cpu().numpy()
+    u_ref = oracle.hc_mix_up(hn, wu, x, norm_w, inv.cpu().numpy(), H, d)
+    z_terms = np.abs(hn) @ np.abs(oracle.affine_weights(wu)).T  # sigmoid' <= 1/4
+    scale = np.abs(x * np.repeat(inv.cpu().numpy(), d, axis=1) * (1 + norm_w))
+    bound = ((2.0 ** -18 * z_terms + 2.0 ** -20) * scale).reshape(T, H, d).sum(axis=1) / H + (2.0 ** -8 * np.abs(u_ref) if dt == torch.bfloat16 else 0)
+    assert np.all(np.abs(u.float().cpu().numpy() - u_ref) <= bound)
+    for t in (0, T - 1):
+        one = mix(xd[t:t + 1])
+        assert all(torch.equal(a[0], b[t]) for a, b in zip(one, (h, w_in, inv, u)))
+
+
 def test_hc_mix_argument_checks(cuda, oracle):
     from strixite_b200 import kernels as K
     rng = np.random.default_rng(1)
