@@ -3,8 +3,8 @@
 // linear_bf16w_wmma), and the residual add that closes a sublayer.
 //
 // Two forms, by regime:
-//   * streaming (decode, a few dozen tokens): a warp owns one weight row and streams it once for all tokens; the row's
-//     bytes (FP32 or BF16) come by 16-byte loads, the tokens' activations from L2.  HBM-bound on the weight;
+//   * streaming (decode, a few dozen tokens): sixteen weight rows by a cluster of CTAs, each warp a part of their contraction against
+//     sixteen tokens at a time on the warp-level tensor-core path, FP32 weights as three BF16 planes split in registers;
 //   * tcgen05 (prefill, thousands of tokens): a plain tensor-core GEMM with both operands staged by tensor copies.  The
 //     weight is the reference's BF16 [N, K], or an FP32 one split once, at load time, into P BF16 "planes"
 //     W = W1 + W2 (+ W3) (each plane the BF16 rounding of what the planes before it left over), so that the products
@@ -16,6 +16,7 @@
 // sxb_check_dense_status) and the kernel returns.
 
 #include "experts.cuh"
+#include "skinny_mma.cuh"
 #include "tc_ptx.cuh"
 
 #include <algorithm>
@@ -25,97 +26,135 @@ namespace {
 
 // ---- streaming form ------------------------------------------------------------------------------------------
 
-constexpr int kStreamRows = 4;    // weight rows a CTA takes at a time: 513 rows are 129 CTAs, one an SM
-constexpr int kRowWarps = 4;      // warps per row, each streaming its part of the staged k range
-constexpr int kStreamWarps = kRowWarps * kStreamRows;
-constexpr int kTokChunk = 16;     // tokens whose activations sit in shared memory (and whose sums a lane keeps)
-constexpr int kStreamKTile = 4096;  // k range staged at a time: 16 tokens x 4096 x 2 bytes = 128 KB of shared memory
-constexpr int kRunsPerLane = kStreamKTile / kRowWarps / 8 / 32;  // runs of eight k a lane takes from its part of a full tile: 4
+constexpr int kStreamSplit = 8, kStreamWarps = 8;  // CTAs of a cluster, and warps of a CTA, that share 16 weight rows
 
-__device__ inline void load_w8(const float *p, float (&w)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
-    w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
-}
-__device__ inline void load_w8(const uint16_t *p, float (&w)[8]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p));
-    const uint32_t u[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[2 * i] = __uint_as_float(u[i] << 16), w[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+// A lane's eight consecutive weights of a row: the BF16 planes they consist of.
+template <typename TW>
+struct Weights;
+template <>
+struct Weights<uint16_t> {
+    static constexpr int kPlanes = 1, kAhead = 4;
+    uint4 v;
+    __device__ inline void load(const uint16_t *p) { v = __ldg(reinterpret_cast<const uint4 *>(p)); }
+    __device__ inline void clear() { v = make_uint4(0u, 0u, 0u, 0u); }
+    __device__ inline void planes(uint4 (&pl)[1]) const { pl[0] = v; }
+};
+template <>
+struct Weights<float> {
+    static constexpr int kPlanes = 3, kAhead = 2;
+    float4 a, b;
+    __device__ inline void load(const float *p) { a = __ldg(reinterpret_cast<const float4 *>(p)), b = __ldg(reinterpret_cast<const float4 *>(p) + 1); }
+    __device__ inline void clear() { a = b = make_float4(0.f, 0.f, 0.f, 0.f); }
+    __device__ inline void planes(uint4 (&pl)[3]) const {
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        split_planes(f, pl);
+    }
+};
+
+template <typename TW>
+__device__ __noinline__ float plain_dot(const uint16_t *x, const TW *w, int64_t K) {
+    float sum = 0.f;
+    for (int64_t k = 0; k < K; ++k) sum = fmaf(bf16_bits_to_f32(x[k]), load_as_f32(w, k), sum);
+    return sum;
 }
 
-// y[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]).  A CTA stages the activations of 16 tokens in shared memory once and
-// streams four weight rows against them, four warps a row (one per quarter of the staged k range): few rows a CTA, so that
-// nearly all SMs have one (65 CTAs of eight rows -> 129 of four: 1 / 16 / 37
-// tokens 13.1 / 19.6 / 44.8 -> 10.3 / 16.8 / 37.6 us for 513 x 4096 FP32, whose 8.4 MB are 1.3 us of HBM time: it is a chain of
-// staging, one round trip for the row and the sums of sixteen tokens, live or not).  A lane issues ALL the
-// loads of its part of the row before it consumes any of them - with a few dozen tokens the kernel is one memory round
-// trip plus arithmetic, so what counts is how many bytes are in flight.  The sum of a (token, row) pair is formed in a
-// fixed order: per lane ascending k, an xor butterfly in the warp, then the row's quarters in order.
-template <typename TW, typename TOUT>
-__global__ void __launch_bounds__(32 * kStreamWarps)
+// y[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]).  grid = (8 x tiles of 16 rows, groups of 8 NT tokens), clusters of eight CTAs along x:
+// the warps of a cluster take the row's runs of 32 k by turns of a 64th each, ask for all their weights at once (K = 4096 FP32: two
+// runs a warp), and the parts are added in order, across the warps in shared memory and then across the cluster.  FP32 weights go
+// through the tensor cores as three BF16 planes (skinny_mma.cuh): exact products, each plane's sum apart, so that the arithmetic is
+// no less than an FP32 multiply-add chain's (error against 64 bits 1.1e-7 -> 0.9e-7) and a token costs an MMA's column of it, not 16 dots
+// a CTA whether they live or not.  513 x 4096 FP32, as a CUDA graph: 1 token 8.1 -> 4.0 us, 16 11.7 -> 4.8, 37 29 -> 12, 127 82 -> 31.  What bounds
+// it: the launch, one round trip to memory, the meeting of the parts.
+template <typename TW, typename TOUT, int NT>
+__global__ void __launch_bounds__(32 * kStreamWarps, 2)
     logits_stream_kernel(const uint16_t *__restrict__ x, const TW *__restrict__ w, const float *__restrict__ bias, int64_t M,
                          int64_t N, int64_t K, TOUT *__restrict__ y, int64_t ld) {
-    extern __shared__ __align__(16) unsigned char xs_raw[];
-    uint4 *xs = reinterpret_cast<uint4 *>(xs_raw);  // [kTokChunk][kt / 8] chunks of eight BF16
-    __shared__ float part[kStreamWarps][kTokChunk];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, part_of = warp % kRowWarps;
-    const int64_t n = (int64_t)blockIdx.x * kStreamRows + warp / kRowWarps;
-    const bool row_ok = n < N;
-    const TW *wr = w + (row_ok ? n : 0) * K;
-    const float b = (row_ok && bias) ? bias[n] : 0.f;
-    for (int64_t m0 = 0; m0 < M; m0 += kTokChunk) {
-        const int live = (int)min((int64_t)kTokChunk, M - m0);
-        float acc[kTokChunk];
+    constexpr int kTok = kMmaTokens * NT, kAhead = Weights<TW>::kAhead, P = Weights<TW>::kPlanes;
+    __shared__ float part[kStreamWarps][kTok][kMmaRows + 1];
+    __shared__ float cta_part[kTok][kMmaRows];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const int rank = (int)cluster_rank();
+    const int64_t n0 = (int64_t)(blockIdx.x / kStreamSplit) * kMmaRows;
+    const TW *wa = w + min(n0 + g, N - 1) * K + 8 * c, *wb = w + min(n0 + g + 8, N - 1) * K + 8 * c;  // rows past the end: the last one
+    const int64_t runs = (K + kMmaRun - 1) / kMmaRun, at = rank * kStreamWarps + warp, parts = kStreamSplit * kStreamWarps;
+    const int64_t lo = runs * at / parts, hi = runs * (at + 1) / parts;
+    for (int64_t t0 = (int64_t)blockIdx.y * kTok; t0 < M; t0 += (int64_t)gridDim.y * kTok) {
+        float acc[NT][4];
 #pragma unroll
-        for (int t = 0; t < kTokChunk; ++t) acc[t] = 0.f;
-        for (int64_t k0 = 0; k0 < K; k0 += kStreamKTile) {
-            const int kt = (int)min((int64_t)kStreamKTile, K - k0), chunks = kt / 8;
-            // this warp's part of the tile, in runs of eight k: [c_lo, c_hi)
-            const int per = (chunks + kRowWarps - 1) / kRowWarps, c_lo = part_of * per, c_hi = min(chunks, c_lo + per);
-            float wv[kRunsPerLane][8];
+        for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+        for (int64_t r0 = lo; r0 < hi; r0 += kAhead) {
+            Weights<TW> va[kAhead], vb[kAhead];
+            uint4 xv[kAhead][NT];
+            bool in[kAhead];
 #pragma unroll
-            for (int j = 0; j < kRunsPerLane; ++j) {  // the row's bytes first: they come from HBM
-                const int c = c_lo + lane + 32 * j;
-                if (row_ok && c < c_hi) load_w8(wr + k0 + (int64_t)c * 8, wv[j]);
+            for (int e = 0; e < kAhead; ++e) {
+                const int64_t k = (r0 + e) * kMmaRun;
+                in[e] = r0 + e < hi && k + 8 * c < K;
+                if (in[e]) va[e].load(wa + k), vb[e].load(wb + k);
+                else va[e].clear(), vb[e].clear();
             }
-            __syncthreads();  // every warp is done with the previous tile
-            for (int i = threadIdx.x; i < kTokChunk * chunks; i += 32 * kStreamWarps) {
-                const int t = i / chunks, c = i % chunks;
-                xs[i] = t < live ? __ldg(reinterpret_cast<const uint4 *>(x + (m0 + t) * K + k0) + c) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            __syncthreads();
-            if (row_ok) {
 #pragma unroll
-                for (int j = 0; j < kRunsPerLane; ++j) {
-                    const int c = c_lo + lane + 32 * j;
-                    if (c >= c_hi) break;
+            for (int e = 0; e < kAhead; ++e)
 #pragma unroll
-                    for (int t = 0; t < kTokChunk; ++t) {
-                        const uint4 xv = xs[t * chunks + c];
-                        const uint32_t u[4] = {xv.x, xv.y, xv.z, xv.w};
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            acc[t] = fmaf(__uint_as_float(u[i] << 16), wv[j][2 * i], acc[t]);
-                            acc[t] = fmaf(__uint_as_float(u[i] & 0xffff0000u), wv[j][2 * i + 1], acc[t]);
-                        }
-                    }
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int64_t t = t0 + nt * kMmaTokens + g;
+                    xv[e][nt] = in[e] && t < M ? __ldg(reinterpret_cast<const uint4 *>(x + t * K + (r0 + e) * kMmaRun + 8 * c)) : make_uint4(0u, 0u, 0u, 0u);
                 }
+            float dot[P][NT][4];
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt) dot[p][nt][0] = dot[p][nt][1] = dot[p][nt][2] = dot[p][nt][3] = 0.f;
+#pragma unroll
+            for (int e = 0; e < kAhead; ++e) {
+                if (r0 + e >= hi) break;
+                uint4 pa[P], pb[P];
+                va[e].planes(pa), vb[e].planes(pb);
+#pragma unroll
+                for (int p = 0; p < P; ++p)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) mma_run(dot[p][nt], pa[p], pb[p], xv[e][nt]);
+            }
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float sum = dot[P - 1][nt][i];
+#pragma unroll
+                    for (int p = P - 2; p >= 0; --p) sum += dot[p][nt][i];
+                    acc[nt][i] += sum;
+                }
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const int t = nt * kMmaTokens + 2 * c;
+            part[warp][t][g] = acc[nt][0], part[warp][t + 1][g] = acc[nt][1];
+            part[warp][t][g + 8] = acc[nt][2], part[warp][t + 1][g + 8] = acc[nt][3];
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < kTok * kMmaRows; i += 32 * kStreamWarps) {
+            float sum = 0.f;
+#pragma unroll
+            for (int v = 0; v < kStreamWarps; ++v) sum += part[v][i / kMmaRows][i % kMmaRows];
+            cta_part[i / kMmaRows][i % kMmaRows] = sum;
+        }
+        cluster_sync();
+        // a CTA finishes every eighth token of the group
+        if (threadIdx.x < NT * kMmaRows) {
+            const int tt = rank + kStreamSplit * (threadIdx.x / kMmaRows), row = threadIdx.x % kMmaRows;
+            const int64_t n = n0 + row, t = t0 + tt;
+            if (n < N && t < M) {
+                float v[kStreamSplit], sum = 0.f;
+#pragma unroll
+                for (int p = 0; p < kStreamSplit; ++p) v[p] = ld_cluster(&cta_part[tt][row], p);
+#pragma unroll
+                for (int p = 0; p < kStreamSplit; ++p) sum += v[p];
+                // An infinity times a plane that is zero, or split into planes, is NaN: the plain sum says what it is.
+                if (P > 1 && isnan(sum)) sum = plain_dot(x + t * K, w + n * K, K);
+                store_from_f32(y, t * ld + n, sum + (bias != nullptr ? bias[n] : 0.f));
             }
         }
-#pragma unroll
-        for (int t = 0; t < kTokChunk; ++t) {
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], off);
-            if (lane == 0) part[warp][t] = acc[t];
-        }
-        __syncthreads();
-        if (part_of == 0 && lane < live && row_ok) {
-            float sum = part[warp][lane];
-#pragma unroll
-            for (int p = 1; p < kRowWarps; ++p) sum += part[warp + p][lane];
-            store_from_f32(y, (m0 + lane) * ld + n, sum + b);
-        }
-        __syncthreads();
+        cluster_sync();  // the parts have been read: the next group may overwrite them, or the CTA leave
     }
 }
 
@@ -369,17 +408,23 @@ int check_proj(const char *fn, const void *x, const void *w, const void *y, int6
 template <typename TOUT>
 int launch_stream_logits(const char *fn, const void *x, const void *w, int w_act, const float *bias, int64_t M, int64_t N, int64_t K,
                          TOUT *y, int64_t ld, cudaStream_t st) {
-    const unsigned blocks = (unsigned)((N + kStreamRows - 1) / kStreamRows);
-    const size_t smem = (size_t)kTokChunk * std::min<int64_t>(K, kStreamKTile) * 2;
+    const int NT = M <= kMmaTokens ? 1 : 2;  // eights of tokens a CTA takes; a second group's weights come from L2
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension, attr.val.clusterDim.x = kStreamSplit, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)((N + kMmaRows - 1) / kMmaRows * kStreamSplit), (unsigned)std::min<int64_t>((M + NT * kMmaTokens - 1) / (NT * kMmaTokens), 65535));
+    cfg.blockDim = dim3(32 * kStreamWarps), cfg.stream = st, cfg.attrs = &attr, cfg.numAttrs = 1;
+    auto xb = static_cast<const uint16_t *>(x);
+    auto launch = [&](auto kern, auto *wt) { return cudaLaunchKernelEx(&cfg, kern, xb, wt, bias, M, N, K, y, ld); };
+    cudaError_t e;
     if (w_act == SXB_ACT_F32) {
-        auto kern = logits_stream_kernel<float, TOUT>;
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
-        kern<<<blocks, 32 * kStreamWarps, smem, st>>>((const uint16_t *)x, (const float *)w, bias, M, N, K, y, ld);
+        auto wt = static_cast<const float *>(w);
+        e = NT == 1 ? launch(logits_stream_kernel<float, TOUT, 1>, wt) : launch(logits_stream_kernel<float, TOUT, 2>, wt);
     } else {
-        auto kern = logits_stream_kernel<uint16_t, TOUT>;
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
-        kern<<<blocks, 32 * kStreamWarps, smem, st>>>((const uint16_t *)x, (const uint16_t *)w, bias, M, N, K, y, ld);
+        auto wt = static_cast<const uint16_t *>(w);
+        e = NT == 1 ? launch(logits_stream_kernel<uint16_t, TOUT, 1>, wt) : launch(logits_stream_kernel<uint16_t, TOUT, 2>, wt);
     }
+    SXB_CUDA(e, fn, ": launching M=", M, " N=", N, " K=", K);
     SXB_CHECK_LAUNCH(fn, " M=", M, " N=", N, " K=", K);
     return SXB_OK;
 }

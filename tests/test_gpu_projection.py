@@ -48,6 +48,41 @@ def test_router_logits_streaming(cuda, oracle, M, N, K, w_bf16):
         assert torch.equal(ybf, y32.to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("w_bf16", [False, True])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 8), (8, 15, 40), (9, 16, 2048), (16, 17, 4104), (33, 130, 4096), (127, 513, 1000)])
+def test_router_logits_streaming_edges(cuda, oracle, M, N, K, w_bf16):
+    """Groups of 8 and 16 tokens full, one over or partly filled, rows past a tile of 16, contractions that end inside a run of 32 or leave
+    warps without one.  Exact products added in chains of at most 128 (K <= 4104: a warp's runs, 16 products an MMA, 64 parts): within
+    2^-17 sum|terms| of 64 bits.  Infinities keep their sign, NaN stays, and a row does not notice its batch."""
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(M + 31 * N + K)
+    xb = oracle.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w = (rng.standard_normal((N, K)) * 0.02).astype(np.float32)
+    if w_bf16:
+        w = oracle.bf16_to_f32(oracle.f32_to_bf16(w))
+    w_dev = torch.from_numpy(w).to(cuda)
+    w_dev = w_dev.to(torch.bfloat16) if w_bf16 else w_dev
+    bias = torch.from_numpy(rng.standard_normal(N).astype(np.float32)).to(cuda)
+    x, out = bf16_tensor(xb, cuda), torch.empty((M, N), dtype=torch.float32, device=cuda)
+    Kn.router_logits(x, w_dev, bias, out)
+    xf, b = oracle.bf16_to_f32(xb).astype(np.float64), bias.cpu().numpy().astype(np.float64)
+    want = xf @ w.astype(np.float64).T + b
+    assert np.all(np.abs(out.cpu().numpy() - want) <= 2.0 ** -17 * (np.abs(xf) @ np.abs(w).T.astype(np.float64) + np.abs(b)))
+    one = torch.empty((1, N), dtype=torch.float32, device=cuda)
+    Kn.router_logits(x[M - 1:].clone(), w_dev, bias, one)
+    assert torch.equal(one[0], out[M - 1])
+    x2, w2 = x.clone(), w_dev.clone()
+    x2[0, K - 1] = float("-inf")
+    w2[N - 1, K - 2] = float("inf")
+    out2 = torch.empty_like(out)
+    Kn.router_logits(x2, w2, bias, out2)
+    with np.errstate(invalid="ignore"):
+        want2 = x2.double().cpu().numpy() @ w2.double().cpu().numpy().T
+    got2 = out2.cpu().numpy()
+    bad = ~np.isfinite(want2)
+    assert np.array_equal(got2[bad], want2[bad], equal_nan=True) and np.array_equal(got2[~bad], out.cpu().numpy()[~bad])
+
+
 @pytest.mark.parametrize("M,N,K,planes,w_bf16", [(4096, 513, 4096, 3, False), (300, 513, 1024, 2, False), (1000, 129, 512, 1, True),
                                                    (128, 64, 256, 3, False)])
 def test_router_logits_tcgen05(cuda, oracle, M, N, K, planes, w_bf16):
