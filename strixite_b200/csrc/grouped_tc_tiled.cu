@@ -10,9 +10,11 @@
 // tokens reading the A operand bounds them); dequantizing 128 x 128 codes and storing them to tensor memory takes the sixteen
 // producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 660 a step for 15 tokens
 // and 840 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions.
-//   * One thread issues everything tensor-core: its loop runs under ONE elect.sync, with the base of tensor memory a constant
-//     (all of it is allocated).  12 cycles an MMA; with elect.sync inside each MMA's instruction group and the base read from
-//     shared memory an MMA cost its warp 90, which was the bound of the loop this one replaces (1400 a step).
+//   * One lane's MMAs and commits count, but its whole warp runs the loop, under control flow that the compiler can see to be uniform: addresses
+//     and descriptors then live in uniform registers.  Run by one lane of a diverged warp the MMAs took no longer to issue, but the loop
+//     around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps that showed it,
+//     which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 542 us at 777 tokens, 817 -> 760 at
+//     4096, dense 1001 x 8192 x 4096 64 -> 56, 4000 tokens Q8 234 -> 217.
 //   * A commit and the next stage's wait cost ~250 whatever lies between: steps of 128 k, eight MMAs.
 //   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 162 instructions a warp and step, not 290.
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
@@ -89,6 +91,17 @@ struct Item {
     int rb;                  // row block
 };
 
+// A role's place in a ring of N barriers and the parity of the phase it is in; steps of at most a turn.
+template <int N>
+struct Turn {
+    int at;
+    uint32_t phase;
+    __device__ inline void advance(int by) {
+        at += by;
+        if (at >= N) at -= N, phase ^= 1u;
+    }
+};
+
 // A row's common power of two is set by its largest group, and weights far below that one's lose bits (dequant_q4_scaled).  With e
 // the largest exponent among a row's groups (of the scale, or of the min less 8) and every other group's at most kScaleSpread
 // below, nothing is lost: a code's step is a BF16 of eight bits and at least 2^-16, so its last bit is at least 2^-23, above the
@@ -117,26 +130,58 @@ __device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
     return it;
 }
 
-// The sixteen BF16 halves' g-th, of eight groups.
-__device__ inline uint16_t pick16(const uint4 &v, int g) {
-    const uint32_t w = (g & 4) ? ((g & 2) ? v.w : v.z) : ((g & 2) ? v.y : v.x);
-    return (uint16_t)((g & 1) ? (w >> 16) : (w & 0xffffu));
+// Scales and mins (BF16 bits) of N consecutive groups of a row.
+template <int N>
+struct Scales {
+    static constexpr int kWords = (N + 1) / 2;
+    uint32_t s[kWords], m[kWords];
+    __device__ inline float scale(int g) const { return value(s, g); }
+    __device__ inline float min(int g) const { return value(m, g); }
+    static __device__ inline float value(const uint32_t (&v)[kWords], int g) {
+        uint32_t w = v[0];
+#pragma unroll
+        for (int i = 1; i < kWords; ++i) w = (g >> 1) == i ? v[i] : w;
+        return __uint_as_float((g & 1) ? (w & 0xffff0000u) : (w << 16));
+    }
+};
+template <int N>
+__device__ inline void load_groups(uint32_t (&v)[Scales<N>::kWords], const uint16_t *p) {
+    if constexpr (N == 1) {
+        v[0] = __ldg(p);
+    } else if constexpr (N == 2) {
+        v[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
+    } else {
+        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+        v[0] = u.x, v[1] = u.y;
+    }
+}
+// The same one by one: rows that N does not divide, or that do not start on a vector's boundary.
+template <int N>
+__device__ __noinline__ Scales<N> load_scales_each(const uint16_t *sp, const uint16_t *mp, int n) {
+    Scales<N> c{};
+    for (int i = 0; i < N; ++i)
+        if (i < n) {
+#pragma unroll
+            for (int w = 0; w < Scales<N>::kWords; ++w)
+                if (w == i >> 1) c.s[w] |= (uint32_t)__ldg(sp + i) << (16 * (i & 1)), c.m[w] |= (uint32_t)__ldg(mp + i) << (16 * (i & 1));
+        }
+    return c;
 }
 
-// A producer lane's step of a quadrant at natural magnitude (kScaleSpread): its row's codes at `src` of shared memory (16-byte chunks
-// swizzled by sw) with the groups from g0 on of s and m -> tensor memory.  Rare, so it is short rather than fast: a quarter at a time,
+// A producer lane's step of a quadrant at natural magnitude (kScaleSpread): its row's codes, 16-byte chunk c at `src` ^ 16 c of shared
+// memory, with its groups sc -> tensor memory.  Rare, so it is short rather than fast: a quarter at a time,
 // read again from shared memory (as a call, or unrolled, it cost the common step registers: 2000 x 8192 x 4096 Q8 133 us, not 129).
-template <int BITS, int G>
-__device__ __forceinline__ void natural_step(uint32_t src, uint32_t sw, uint32_t a_addr, uint4 s, uint4 m, int g0) {
+template <int BITS, int G, int N>
+__device__ __forceinline__ void natural_step(uint32_t src, uint32_t a_addr, const Scales<N> &sc) {
     constexpr int kChunkCodes = BITS == 4 ? 32 : 16, kChunks = 32 / kChunkCodes;
 #pragma unroll 1
     for (int hc = 0; hc < 4; ++hc) {
         uint4 d[4];
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) {
-            const uint4 v = ld_shared_v4(src + ((uint32_t)(hc * kChunks + c) ^ sw) * 16u);
-            const int g = (g0 + hc * 32 / G) & 7;  // 32 codes lie in one group
-            const __half2 s2 = __float2half2_rn(bf16_bits_to_f32(pick16(s, g))), m2 = __float2half2_rn(bf16_bits_to_f32(pick16(m, g)));
+            const uint4 v = ld_shared_v4(src ^ ((uint32_t)(hc * kChunks + c) * 16u));
+            const int g = hc * 32 / G;  // 32 codes lie in one group
+            const __half2 s2 = __float2half2_rn(sc.scale(g)), m2 = __float2half2_rn(sc.min(g));
             if (BITS == 4) {
                 d[0] = dequant_q4_word(v.x, s2, m2), d[1] = dequant_q4_word(v.y, s2, m2);
                 d[2] = dequant_q4_word(v.z, s2, m2), d[3] = dequant_q4_word(v.w, s2, m2);
@@ -251,80 +296,67 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         const int p0 = a_quad * 32 + lane;  // tensor-memory lane = row of the item
         // row of the ring slot that holds this lane's codes: the SwiGLU form's slot is [64 gate rows | 64 up rows]
         const int srow = MODE == kTcSwiglu ? (lane >> 4) * (kRows / 2) + a_quad * 16 + (lane & 15) : p0;
-        constexpr int kStepsPerChunk = 8 * G / kBK;  // steps covered by eight scale groups (one 16-byte load)
-        constexpr int kGroupsPerStep = kBK / G;
+        constexpr int kGroups = kBK / G;             // of a step
+        constexpr int kRowBytes = kBK * BITS / 8;    // of a row of a ring slot: 64 or 128
         constexpr int kCodeRegs = kBK * BITS / 128;  // 16-byte chunks of codes per row and step
         constexpr int kWordsPerChunk = BITS == 4 ? 4 : 2;  // runs of eight codes in one of them
-        constexpr int kSlotsPerSet = kWSlots / kWays;
-        const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
-        // this thread's row inside the set's first slot; its 16-byte chunks are swizzled (64-byte mode for Q4's 64-byte rows,
-        // 128-byte for Q8's)
-        const uint32_t my_w = w_base + (uint32_t)(set * kSlotBytes + srow * (kBK * BITS / 8)), my_sw = (uint32_t)(BITS == 4 ? (srow >> 1) & 3 : srow & 7);
+        const bool vec_scales = groups % kGroups == 0 &&
+                                ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & (2 * kGroups - 1)) == 0;
+        // this thread's row inside the first slot; its chunks are swizzled (128-byte mode, 64-byte for rows of 64 bytes), so that chunk c
+        // lies at my_w ^ 16 c
+        const uint32_t my_w = w_base + (uint32_t)(srow * kRowBytes) + (uint32_t)(kRowBytes == 64 ? (srow >> 1) & 3 : srow & 7) * 16u;
         const uint32_t a_addr = ((uint32_t)(a_quad * 32) << 16) + (uint32_t)(kAccs * kTile + set * kAStageCols);
 
-        // Scales and mins of eight consecutive groups of a row (BF16 bits), fetched one chunk ahead of use.  A row past the
-        // end of the expert gets zeros: its operand row is then zero whatever codes its lane reads.
-        struct ScaleChunk {
-            uint4 s, m;
-        };
-        auto load_scales = [&](int64_t wrow, int chunk) {
-            ScaleChunk c{make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+        // Scales and mins of a step's groups, fetched one step of the set ahead of use (fetched eight groups at a time, of which a set used a
+        // quarter or half, and picked out by selects, they were 5 % of the Q8 forms).  A row past the end of the expert gets zeros: its
+        // operand row is then zero whatever codes its lane reads.
+        auto load_scales = [&](int wrow, int step) {
+            Scales<kGroups> c{};
             if (wrow < 0) return c;
-            const int g0 = chunk * 8;
-            const uint16_t *sp = a.scale + wrow * groups + g0, *mp = a.minv + wrow * groups + g0;
-            if (vec_scales) {
-                c.s = __ldg(reinterpret_cast<const uint4 *>(sp)), c.m = __ldg(reinterpret_cast<const uint4 *>(mp));
-            } else {
-                uint32_t sw[4] = {0u, 0u, 0u, 0u}, mw[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    if (g0 + i < groups) sw[i >> 1] |= (uint32_t)__ldg(sp + i) << (16 * (i & 1)), mw[i >> 1] |= (uint32_t)__ldg(mp + i) << (16 * (i & 1));
-                c.s = make_uint4(sw[0], sw[1], sw[2], sw[3]), c.m = make_uint4(mw[0], mw[1], mw[2], mw[3]);
-            }
+            const int64_t at = (int64_t)wrow * groups + step * kGroups;
+            if (vec_scales) load_groups<kGroups>(c.s, a.scale + at), load_groups<kGroups>(c.m, a.minv + at);
+            else c = load_scales_each<kGroups>(a.scale + at, a.minv + at, groups - step * kGroups);
             return c;
         };
-        ScaleChunk sc_cur = {}, sc_nxt = {};
-        int nxt_item = -1, nxt_chunk = -1;  // what sc_nxt holds
-        uint32_t j = 0;                     // steps this set has done
-        int st = set;                       // the set's next step, relative to the item at hand
+        uint32_t free_phase = 1u;  // parity of the phase that leaves the stage to the set's next step: there is none before the first
+        Turn<kWSlots> slot{set, 0u};
+        int st = set;  // the set's next step, relative to the item at hand
         bool live = true;
         float nxt_scale = 1.f;
         Item nxt = read_item(0, p0, nxt_scale);
+        int row = -1;
+        Scales<kGroups> sc_nxt{};
+        bool have = false;  // sc_nxt is of the set's next step
+        if (nxt.bucket >= 0 && nxt.bucket < a.E) row = (int)row_of(nxt, p0);
         for (int i = 0; nxt.bucket >= 0 && live; ++i) {
             const Item it = nxt;
             const float scale = nxt_scale, scale_min = scale * 0x1p-24f;
             nxt = read_item(i + 1, p0, nxt_scale);
-            if (it.bucket >= a.E) continue;
-            int cur_chunk = -1;
-            for (; st < n_steps; st += kWays, ++j) {
-                const int chunk = st / kStepsPerChunk;
-                if (chunk != cur_chunk) {
-                    if (nxt_item == i && nxt_chunk == chunk) sc_cur = sc_nxt;
-                    else sc_cur = load_scales(row_of(it, p0), chunk);
-                    cur_chunk = chunk;
-                    // the set's first step past this chunk: in this item, or in the next one
-                    int nst = st + ((min((chunk + 1) * kStepsPerChunk, n_steps) - st + kWays - 1) & ~(kWays - 1));
-                    if (nst < n_steps) {
-                        nxt_item = i, nxt_chunk = nst / kStepsPerChunk;
-                        sc_nxt = load_scales(row_of(it, p0), nxt_chunk);
-                    } else if (nst -= n_steps; nxt.bucket >= 0 && nxt.bucket < a.E && nst < n_steps) {
-                        nxt_item = i + 1, nxt_chunk = nst / kStepsPerChunk;
-                        sc_nxt = load_scales(row_of(nxt, p0), nxt_chunk);
-                    }
+            const bool more = nxt.bucket >= 0 && nxt.bucket < a.E;
+            const int nxt_row = more ? (int)row_of(nxt, p0) : -1;
+            if (it.bucket >= a.E) {
+                row = nxt_row;
+                continue;
+            }
+            for (; st < n_steps; st += kWays, slot.advance(kWays)) {
+                if (!have) sc_nxt = load_scales(row, st);
+                const Scales<kGroups> sc = sc_nxt;
+                const int nst = st + kWays;  // in this item, or in the next one
+                have = nst < n_steps || (more && nst - n_steps < n_steps);
+                if (have) sc_nxt = nst < n_steps ? load_scales(row, nst) : load_scales(nxt_row, nst - n_steps);
+                bool ok = true;
+                if (!mbar_wait(&w_full[slot.at], slot.phase, abort_v, a.wait_limit_ns)) {
+                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 7);
+                    ok = false;
                 }
-                const uint32_t slot = set + (kSlotsPerSet > 1 ? (j % kSlotsPerSet) * kWays : 0);
-                bool ok = mbar_wait(&w_full[slot], (j / kSlotsPerSet) & 1u, abort_v, a.wait_limit_ns);
-                if (!ok && lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 7);
-                const uint32_t src = my_w + (slot - set) * (uint32_t)kSlotBytes;
+                const uint32_t src = my_w + slot.at * (uint32_t)kSlotBytes;
                 uint4 code[kCodeRegs];
 #pragma unroll
-                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(src + (((uint32_t)c ^ my_sw) << 4));
-                __half2 s2[kGroupsPerStep], s16[kGroupsPerStep], m2[kGroupsPerStep];
+                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(src ^ ((uint32_t)c << 4));
+                __half2 s2[kGroups], s16[kGroups], m2[kGroups];
 #pragma unroll
-                for (int gi = 0; gi < kGroupsPerStep; ++gi) {
-                    const int g = (st * kGroupsPerStep + gi) & 7;  // group inside the chunk of eight
-                    const float sf = bf16_bits_to_f32(pick16(sc_cur.s, g)), mf = bf16_bits_to_f32(pick16(sc_cur.m, g));
-                    s2[gi] = __float2half2_rn(sf * scale), m2[gi] = __float2half2_rn(mf * scale_min);
+                for (int gi = 0; gi < kGroups; ++gi) {
+                    s2[gi] = __float2half2_rn(sc.scale(gi) * scale), m2[gi] = __float2half2_rn(sc.min(gi) * scale_min);
                     s16[gi] = __hmul2(s2[gi], __float2half2_rn(0.0625f));
                 }
                 // 32 codes of the row -> 32 F16 = 16 tensor-memory columns of this lane
@@ -339,7 +371,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 };
                 uint4 d[4];
                 quarter(0, d);
-                if (ok && !mbar_wait(&empty_bar[set], (j & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                if (ok && !mbar_wait(&empty_bar[set], free_phase, abort_v, a.wait_limit_ns)) {
                     if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 1);
                     ok = false;
                 }
@@ -350,7 +382,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 }
                 tc_fence_after();  // the stores below come after the MMAs that freed the stage
                 if (scale > 0.f) {
-                    if (lane == 0) mbar_arrive(&w_empty[slot]);  // the codes are in registers: the slot may be refilled
+                    if (lane == 0) mbar_arrive(&w_empty[slot.at]);  // the codes are in registers: the slot may be refilled
                     tc_st16(a_addr, d);
 #pragma unroll
                     for (int hc = 1; hc < 4; ++hc) {
@@ -358,15 +390,16 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                         tc_st16(a_addr + hc * 16, d);
                     }
                 } else {
-                    natural_step<BITS, G>(src, my_sw, a_addr, sc_cur.s, sc_cur.m, (st * kGroupsPerStep) & 7);
-                    if (lane == 0) mbar_arrive(&w_empty[slot]);
+                    natural_step<BITS, G>(src, a_addr, sc);
+                    if (lane == 0) mbar_arrive(&w_empty[slot.at]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full_bar[set]);
+                free_phase ^= 1u;
             }
-            st -= n_steps;
+            st -= n_steps, row = nxt_row;
         }
     } else if (warp == kItemWarp) {
         // ===================== the item ring =====================
@@ -448,6 +481,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         // gate rows and, I rows further, their up rows; otherwise 128 consecutive rows).
         if (elect_one()) {
             bool ok = true;
+            Turn<kWSlots> turn{0, 0u};
             for (int i = 0; ok; ++i) {
                 const Item it = read_item_one(i);
                 if (it.bucket < 0) break;
@@ -456,13 +490,13 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 if (MODE == kTcSwiglu) y0 = (int)(it.bucket * a.N + it.rb * (kRows / 2)), y1 = y0 + (int)(a.N / 2);
                 else y0 = (int)(it.bucket * a.N + (int64_t)it.rb * kRows), y1 = y0 + kRows / 2;
                 for (int step = 0; step < n_steps; ++step) {
-                    const uint32_t slot = issued % kWSlots;
-                    if (issued >= (uint32_t)kWSlots && !mbar_wait(&w_empty[slot], ((issued / kWSlots) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                    const int slot = turn.at;
+                    if (!mbar_wait(&w_empty[slot], turn.phase ^ 1u, abort_v, a.wait_limit_ns)) {
                         raise_abort(blockIdx.x + i * gridDim.x, 6);
                         ok = false;
                         break;
                     }
-                    const uint32_t dst = w_base + slot * (uint32_t)kSlotBytes;
+                    const uint32_t dst = w_base + (uint32_t)(slot * kSlotBytes);
                     // test hook: CTA 0 leaves one slot unfilled (neither the byte count nor the copies), so that its consumers'
                     // wait runs out at the launch's limit and the abort path is exercised without anything faulting
                     if (!(blockIdx.x == 0 && (int)issued == a.test_skip_slot)) {
@@ -470,7 +504,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                         tma_load_2d(dst, &wmap, step * (kBK * BITS / 8), y0, &w_full[slot]);
                         tma_load_2d(dst + kSlotBytes / 2, &wmap, step * (kBK * BITS / 8), y1, &w_full[slot]);
                     }
-                    ++issued;
+                    ++issued, turn.advance(1);
                 }
             }
         }
@@ -506,44 +540,56 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         __syncwarp();
     } else if (warp == kMmaWarp) {
         // ===================== MMA issue =====================
-        if (elect_one()) {
-            uint32_t count = 0, acc_count = 0;
-            bool ok = true;
-            for (int i = 0; ok; ++i) {
-                const Item it = read_item_one(i);
-                if (it.bucket < 0) break;
-                if (it.bucket >= a.E) continue;
-                const uint32_t idesc = instr_desc((it.cnt + 15) & ~15);
-                const uint32_t half = acc_count & 1u;  // the accumulators take turns
-                if (!mbar_wait(&acc_empty[half], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
-                    raise_abort(blockIdx.x + i * gridDim.x, 2);
-                    break;
-                }
-                ++acc_count;
-                tc_fence_after();
-                const uint32_t d = half * (uint32_t)kTile;
-                for (int st = 0; st < n_steps; ++st, ++count) {
-                    const uint32_t stage = count % kStages;
-                    if (!mbar_wait(&full_bar[stage], (count / kStages) & 1u, abort_v, a.wait_limit_ns)) {
-                        raise_abort(blockIdx.x + i * gridDim.x, 3);
-                        ok = false;
+        // The whole warp runs the loop under control flow that is known to be uniform (votes and a reduction of what came through shared
+        // memory), so that addresses and descriptors stay in uniform registers; one lane's MMAs and commits count.  Whether the next
+        // step's operands are there is asked before this step's MMAs are issued: the answer comes under them.
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        const uint64_t desc0 = smem_desc(b_base);
+        const uint32_t b_lo0 = (uint32_t)desc0, b_hi = (uint32_t)(desc0 >> 32), at0 = (uint32_t)(kAccs * kTile);
+        uint32_t b_lo = b_lo0, at = at0;
+        Turn<kStages> turn{0, 0u};
+        int done = 0;  // the stage of the step at hand
+        uint32_t acc_count = 0;
+        bool ok = true;
+        for (int i = 0; ok; ++i) {
+            float unused;
+            const Item it = read_item(i, lane, unused);
+            if (__any_sync(0xffffffffu, it.bucket < 0)) break;
+            if (__any_sync(0xffffffffu, it.bucket >= a.E)) continue;
+            const uint32_t idesc = __reduce_max_sync(0xffffffffu, instr_desc((it.cnt + 15) & ~15));
+            const uint32_t half = acc_count & 1u;  // the accumulators take turns
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[half], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns));
+            if (!ok) {
+                if (leader) raise_abort(blockIdx.x + i * gridDim.x, 2);
+                break;
+            }
+            ++acc_count;
+            tc_fence_after();
+            const uint32_t d = half * (uint32_t)kTile;
+            bool ready = false;
+            for (int st = 0; st < n_steps; ++st) {
+                if (!__all_sync(0xffffffffu, ready)) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[turn.at], turn.phase, abort_v, a.wait_limit_ns));
+                    if (!ok) {
+                        if (leader) raise_abort(blockIdx.x + i * gridDim.x, 3);
                         break;
                     }
-                    tc_fence_after();
-                    const uint64_t b_desc = smem_desc(b_base + stage * (uint32_t)kStageBytes);
-                    const uint32_t at = (uint32_t)(kAccs * kTile) + stage * (uint32_t)kAStageCols;
-#pragma unroll
-                    for (int j = 0; j < kBK / 16; ++j)  // k = 16 an instruction: 8 columns of A, 32 bytes along B's swizzled line
-                        tc_mma_f16_ts_one(d, at + 8 * j, b_desc + (j >> 2) * (kSubBytes >> 4) + 2 * (j & 3), idesc, (st | j) != 0);
-                    tc_commit_one(&empty_bar[stage]);  // the stage is free when these MMAs have read it
                 }
-                if (ok) tc_commit_one(&acc_full[half]);
+                tc_fence_after();
+                turn.advance(1);
+                ready = mbar_test(&full_bar[turn.at], turn.phase);
+                tc_step_ts<kSubBytes>(leader, d, at, b_lo, b_hi, idesc, st != 0);
+                tc_commit_if(leader, &empty_bar[done]);  // the stage is free when these MMAs have read it
+                done = (done + 1) % kStages;
+                at += kAStageCols, b_lo += kStageBytes / 16;
+                if (turn.at == 0) at = at0, b_lo = b_lo0;
             }
-            // Drain: every MMA issued by this CTA has completed before tensor memory is released.
-            // (this wait does not give up when the CTA is aborting: tensor memory must not be released under an MMA)
-            tc_commit_one(&drain_bar);
-            mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
+            if (ok) tc_commit_if(leader, &acc_full[half]);
         }
+        // Drain: every MMA issued by this CTA has completed before tensor memory is released.
+        // (this wait does not give up when the CTA is aborting: tensor memory must not be released under an MMA)
+        tc_commit_if(leader, &drain_bar);
+        mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
         __syncwarp();
     } else if (MODE == kTcHcUp && warp < kEpiWarps) {
         // ===================== epilogue of the hyper-connection up mix =====================

@@ -37,6 +37,18 @@ __device__ inline bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+// Whether the phase has completed, at once.
+__device__ inline bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ inline unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
@@ -128,20 +140,45 @@ __device__ inline void tc_st16(uint32_t taddr, const uint4 (&d)[4]) {
         "r"(d[2].y), "r"(d[2].z), "r"(d[2].w), "r"(d[3].x), "r"(d[3].y), "r"(d[3].z), "r"(d[3].w)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem], the A operand (128 rows x 16 k of F16, two per 32-bit column) read from tensor memory, for
-// a loop that runs under ONE election: elect_one() picks a lane of the converged warp, and that lane alone runs the loop with
-// these.  An MMA then costs its issuer 12 cycles; with the election inside each instruction group, 40 to 90.
+// 1 in one lane of a converged warp.
 __device__ inline bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
     return p != 0;
 }
-__device__ inline void tc_mma_f16_ts_one(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+// D[tmem] (+)= A[tmem] * B[smem], the A operand (128 rows x 16 k of F16, two per 32-bit column) read from tensor memory, for a loop
+// that a whole warp runs: `leader` is 1 in the one lane (of elect_one) whose MMAs and commits count.  A step of
+// 128 k at once: eight MMAs, A's columns advance by 8, B's descriptor (b_hi : b_lo) by 32 bytes along the swizzled line, from the
+// fifth on in the next 64-k sub-tile, SUB bytes further.
+template <int SUB>
+__device__ inline void tc_step_ts(uint32_t leader, uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n\t.reg .pred p, q, one;\n\t.reg .b32 a1, a2, a3, a4, a5, a6, a7, l1, l2, l3, l4, l5, l6, l7;\n\t"
+        ".reg .b64 b0, b1, b2, b3, b4, b5, b6, b7;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tsetp.eq.b32 one, 0, 0;\n\t"
+        "mov.b64 b0, {%2, %3};\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 l1, %2, 2;\n\tmov.b64 b1, {l1, %3};\n\t"
+        "add.u32 a2, %1, 16;\n\tadd.u32 l2, %2, 4;\n\tmov.b64 b2, {l2, %3};\n\t"
+        "add.u32 a3, %1, 24;\n\tadd.u32 l3, %2, 6;\n\tmov.b64 b3, {l3, %3};\n\t"
+        "add.u32 a4, %1, 32;\n\tadd.u32 l4, %2, %7;\n\tmov.b64 b4, {l4, %3};\n\t"
+        "add.u32 a5, %1, 40;\n\tadd.u32 l5, %2, %8;\n\tmov.b64 b5, {l5, %3};\n\t"
+        "add.u32 a6, %1, 48;\n\tadd.u32 l6, %2, %9;\n\tmov.b64 b6, {l6, %3};\n\t"
+        "add.u32 a7, %1, 56;\n\tadd.u32 l7, %2, %10;\n\tmov.b64 b7, {l7, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %4, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a4], b4, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a5], b5, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a6], b6, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a7], b7, %4, one;\n\t}" ::"r"(d),
+        "r"(a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(leader), "n"(SUB / 16), "n"(SUB / 16 + 2), "n"(SUB / 16 + 4), "n"(SUB / 16 + 6)
+        : "memory");
+}
+__device__ inline void tc_commit_if(uint32_t leader, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
         : "memory");
 }
 __device__ inline void tc_commit_one(uint64_t *bar) {

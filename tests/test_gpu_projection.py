@@ -263,6 +263,31 @@ def test_dense_tcgen05_partial_row_blocks(cuda, oracle, bits, G, M, N, K):
     assert torch.equal(ybf, y32[:M].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("bits,G", [(4, 32), (4, 64), (4, 128), (8, 32), (8, 64), (8, 128)])
+@pytest.mark.parametrize("K", [128, 384, 1152])
+def test_dense_tcgen05_scale_alignment(cuda, oracle, bits, G, K):
+    """Contractions of 1, 3 and 9 steps of 128 - fewer than the producers' sets, and no multiple of them - with scales and mins that start
+    on any 2-byte boundary: the vector loads' groups and those read one by one give the same bits."""
+    from dataclasses import replace
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(bits + G + K)
+    M, N = 140, 200
+    wq = oracle.quantize(random_weights(rng, N, K), G, bits)
+    xb = oracle.f32_to_bf16(rng.standard_normal((M, K)).astype(np.float32))
+    w, x = upload(wq, cuda), bf16_tensor(xb, cuda)
+    want = oracle.linear_q(xb, wq, out_act=oracle.F32, w_f16=True)
+    ys = []
+    for off in (0, 1, 2):
+        moved = [torch.cat([v.new_zeros(8 + off), v.reshape(-1)])[8 + off:] for v in (w.scale, w.minv)]
+        y = torch.empty((M, N), dtype=torch.float32, device=cuda)
+        Kn.linear_qw_wmma(x, replace(w, scale=moved[0], minv=moved[1]), y, M, Kn.Act.BF16, Kn.Act.F32)
+        ys.append(y)
+    torch.cuda.synchronize()
+    Kn.check_dense_status("scale alignment")
+    assert max_abs_over_rms(ys[0].cpu().numpy(), want) <= 2e-5
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+
+
 @pytest.mark.parametrize("way", ["staged", "captured"])
 @pytest.mark.parametrize("bits,G,M,N,K", [(4, 128, 64, 4104, 2048), (8, 64, 127, 4104, 512), (4, 64, 129, 24, 256), (8, 128, 1001, 136, 256)])
 def test_dense_tcgen05_rows_in_eights(cuda, oracle, monkeypatch, way, bits, G, M, N, K):
