@@ -35,21 +35,6 @@ static_assert(kChunk == kMmaRun, "a chunk is a run of the MMA's k");
 
 __device__ inline float sigmoid_f32(float z) { return 1.0f / (1.0f + expf(-z)); }
 
-// A lane's eight codes of a chunk: 8 bytes (Q8) or 4 (Q4).
-template <int BITS>
-struct Codes {
-    uint32_t w[BITS / 4];
-    __device__ inline void load(const uint8_t *p) {
-        if constexpr (BITS == 8) {
-            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
-            w[0] = v.x, w[1] = v.y;
-        } else {
-            w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
-        }
-    }
-    __device__ inline uint4 bf16() const { return codes_bf16<BITS>(w[0], w[BITS / 4 - 1]); }
-};
-
 // A lane's eight activations of a chunk of its token, as the BF16 planes they consist of.
 template <typename T>
 struct Acts;
@@ -146,7 +131,7 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
             for (int e = 0; e < kAhead; ++e) {
                 const int i = e0 + e;
                 if (c0 + i >= hi) break;
-                const uint4 va = wa[i].bf16(), vb = wb[i].bf16(), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+                const uint4 va = wa[i].template bf16<true>(), vb = wb[i].template bf16<true>(), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
                 const uint32_t p_a = __shfl_sync(0xffffffffu, sm_a[i / 4], (lane & ~3) + i % 4), p_b = __shfl_sync(0xffffffffu, sm_b[i / 4], (lane & ~3) + i % 4);
                 const float s_a = __uint_as_float(p_a << 16), m_a = centered_min<BITS>(s_a, __uint_as_float(p_a & 0xffff0000u));
                 const float s_b = __uint_as_float(p_b << 16), m_b = centered_min<BITS>(s_b, __uint_as_float(p_b & 0xffff0000u));
@@ -292,7 +277,7 @@ __global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__res
         for (int a = 0; a < kUpAhead; ++a) {
             const int ch = c0 + a;
             if (ch >= chunks) break;
-            const uint4 va = wa[a].bf16(), vb = wb[a].bf16();
+            const uint4 va = wa[a].template bf16<true>(), vb = wb[a].template bf16<true>();
             const float s_a = bf16_bits_to_f32(sa[a]), m_a = centered_min<BITS>(s_a, bf16_bits_to_f32(ma[a]));
             const float s_b = bf16_bits_to_f32(sb[a]), m_b = centered_min<BITS>(s_b, bf16_bits_to_f32(mb[a]));
 #pragma unroll
@@ -337,10 +322,6 @@ __global__ void __launch_bounds__(256) chunk_major_kernel(const uint8_t *__restr
         so[g * N + n] = scale[i], mo[g * N + n] = minv[i];
     }
 }
-
-// Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Four where the last 32 are more than half
-// full (63 tokens, d = 4096 Q8, down + up: 41 us, 45 with two; 40 tokens: 39 and 32).
-int token_eights(int64_t T) { return T <= 8 ? 1 : T <= 16 || (T < 64 && (T - 1) % 32 < 16) ? 2 : 4; }
 
 int check_hc_shape(const char *fn, int64_t T, int64_t H, int64_t d) {
     SXB_CHECK(H == kStreams, fn, ": H = ", H, " streams, only ", kStreams, " is supported");

@@ -44,15 +44,15 @@ __device__ inline void split_planes(const float (&v)[8], uint4 (&p)[3]) {
     for (int j = 0; j < 3; ++j) p[j] = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
 }
 
-// The lane's eight codes of a row, less the middle of their range, as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).  What is taken
-// off goes to the group's min (centered_min); without it the sums carry the codes' mean times sum(x), which the min takes off again, and
-// the rounding of the larger sums stays.
+// The lane's eight codes of a row as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).  CENTER: less the middle of their range, which
+// goes to the group's min instead (centered_min): without it the sums carry the codes' mean times sum(x), which the min takes off again,
+// and the rounding of the larger sums stays.  Not where a weight of zero (code and min) must take nothing from the rest of its dot.
 template <int BITS> constexpr float kCenter = BITS == 8 ? 128.f : 8.f;
 template <int BITS>
 __device__ inline float centered_min(float s, float m) { return fmaf(kCenter<BITS>, s, m); }
-template <int BITS>
+template <int BITS, bool CENTER>
 __device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1) {
-    constexpr float kOff = 0x1p23f + kCenter<BITS>;
+    constexpr float kOff = 0x1p23f + (CENTER ? kCenter<BITS> : 0.f);
     uint32_t r[4];
     if (BITS == 8) {
 #pragma unroll
@@ -72,6 +72,26 @@ __device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1) {
     }
     return make_uint4(r[0], r[1], r[2], r[3]);
 }
+
+// A lane's eight codes of a run: 8 bytes (Q8) or 4 (Q4).
+template <int BITS>
+struct Codes {
+    uint32_t w[BITS / 4];
+    __device__ inline void load(const uint8_t *p) {
+        if constexpr (BITS == 8) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+            w[0] = v.x, w[1] = v.y;
+        } else {
+            w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
+        }
+    }
+    template <bool CENTER>
+    __device__ inline uint4 bf16() const { return codes_bf16<BITS, CENTER>(w[0], w[BITS / 4 - 1]); }
+};
+
+// Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Four where the last 32 are more than half
+// full (the hyper-connection mix of 63 tokens, d = 4096 Q8: 41 us, 45 with two; of 40 tokens: 39 and 32).
+inline int token_eights(int64_t T) { return T <= 8 ? 1 : T <= 16 || (T < 64 && (T - 1) % 32 < 16) ? 2 : 4; }
 
 // ---- the CTAs of a cluster -------------------------------------------------------------------------------------------
 __device__ inline uint32_t cluster_rank() {

@@ -1,5 +1,5 @@
-// Streaming expert / dense kernels for the HBM-bound regime (decode and small ragged batches; also the exact-product
-// path at any size).  C ABI twins of the launchers in kernels/linear_q4.hpp, kernels/linear_q8.hpp and of the
+// Streaming expert kernels, and dense ones of Q4 weights (Q8: dense_mma.cu), for the HBM-bound regime (decode and small ragged batches;
+// also the exact-product path at any size).  C ABI twins of the launchers in kernels/linear_q4.hpp, kernels/linear_q8.hpp and of the
 // MoeMath::F32 / WmmaBf16 forms of kernels/moe_grouped.hpp.
 //
 // What the reference does (kernels/linear_q4.hip:175-199): a wave walks one weight row, every lane takes 32 codes per
@@ -985,16 +985,24 @@ int linear_impl(const char *fn, const void *x, const SxbQView *w, void *y, int64
     if (int rc = need_bf16(fn, act)) return rc;
     SXB_CHECK(apart(x, M * w->K * 2, y, M * w->N * act_bytes(out_act)), fn, ": output y [", y, ", +",
               M * w->N * act_bytes(out_act), " B) overlaps input x [", x, ", +", M * w->K * 2, " B)");
-    StreamArgs a{};
-    a.x = static_cast<const uint16_t *>(x), a.q = w->q, a.scale = w->scale, a.minv = w->minv;
-    a.N = w->N, a.K = w->K, a.M = M, a.A = 1, a.E = 1, a.out = y;
-    const int64_t units = ((M + 7) / 8) * ((w->N + 15) / 16);
-    auto st = static_cast<cudaStream_t>(stream);
-    int rc = out_act == SXB_ACT_F32 ? launch_by_group<BITS, kGather, kDense, float>(fn, a, w->G, units, st)
-                                    : launch_by_group<BITS, kGather, kDense, uint16_t>(fn, a, w->G, units, st);
-    if (rc) return rc;
-    SXB_CHECK_LAUNCH(fn, " ", act_name(act), "->", act_name(out_act), " M=", M, " N=", w->N, " K=", w->K, " G=", w->G);
-    return SXB_OK;
+    if constexpr (BITS == 8) {
+        // the longest row: what a tile of eight tokens of one takes of shared memory in the routed forms of the same projection
+        const int64_t smem = w->K * 16 + w->K / std::min<int64_t>(64, w->G) * kTileTokens * 4;
+        SXB_CHECK(smem <= (int64_t)kMaxDynSmem, fn, ": K = ", w->K, " needs ", smem, " bytes of shared memory for one tile's activations, more than ",
+                  kMaxDynSmem, " (K * 16)");
+        return dense_mma<BITS>(fn, x, w, y, M, out_act, static_cast<cudaStream_t>(stream));
+    } else {
+        StreamArgs a{};
+        a.x = static_cast<const uint16_t *>(x), a.q = w->q, a.scale = w->scale, a.minv = w->minv;
+        a.N = w->N, a.K = w->K, a.M = M, a.A = 1, a.E = 1, a.out = y;
+        const int64_t units = ((M + 7) / 8) * ((w->N + 15) / 16);
+        auto st = static_cast<cudaStream_t>(stream);
+        int rc = out_act == SXB_ACT_F32 ? launch_by_group<BITS, kGather, kDense, float>(fn, a, w->G, units, st)
+                                        : launch_by_group<BITS, kGather, kDense, uint16_t>(fn, a, w->G, units, st);
+        if (rc) return rc;
+        SXB_CHECK_LAUNCH(fn, " ", act_name(act), "->", act_name(out_act), " M=", M, " N=", w->N, " K=", w->K, " G=", w->G);
+        return SXB_OK;
+    }
 }
 
 int check_experts(const char *fn, const void *x, const SxbQView *w, int64_t E, int64_t M, int64_t A, const void *y) {

@@ -96,6 +96,28 @@ def test_linear_activation_range(cuda, oracle, bits, G, Kd):
     assert np.all(np.abs(got[:10] - want) <= bound), np.max(np.abs(got[:10] - want) / bound, axis=1)
 
 
+@pytest.mark.parametrize("G,M,N,Kd", [(32, 8, 31, 32), (64, 9, 33, 192), (128, 17, 4740, 256), (64, 33, 2400, 576), (32, 49, 16, 2080), (64, 150, 4808, 128)])
+def test_linear_q8_edges(cuda, oracle, G, M, N, Kd):
+    """The edges of the Q8 dense form's tiles: groups of 8, 16 and 32 tokens that are full, one over or partly filled, rows past a tile of
+    16 and of 32, contractions of fewer runs than warps or none of their multiples; and activations whose products with the codes
+    leave FP32's range while the result does not.  Bound: as in test_linear_activation_range, the groups being runs of 32."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(M + N + Kd)
+    x = rng.standard_normal((M, Kd))
+    x[M - 1] = np.where(np.arange(Kd) % 2, 1.0, -1.0) * 2.0 ** 124
+    xb = oracle.f32_to_bf16(x.astype(np.float32))
+    w = oracle.quantize(random_weights(rng, N, Kd), G, 8)
+    y = torch.empty((M, N), dtype=torch.float32, device=cuda)
+    K.linear_qw(bf16_tensor(xb, cuda), upload(w, cuda), y, M, K.Act.BF16, out_act=K.Act.F32)
+    torch.cuda.synchronize()
+    xf = oracle.bf16_to_f32(xb).astype(np.float64)
+    s, m = (np.repeat(oracle.bf16_to_f32(v).astype(np.float64).reshape(N, Kd // G), G, axis=1) for v in (w.scale, w.minv))
+    codes = oracle.codes_of(w).astype(np.float64)
+    want = xf @ (codes * s + m).T
+    bound = (Kd / 8 + 3 * Kd / 32 + 12) * 2.0 ** -23 * (np.abs(xf) @ (codes * np.abs(s) + np.abs(m)).T)
+    assert np.all(np.abs(y.cpu().numpy().astype(np.float64) - want) <= bound)
+
+
 @pytest.mark.parametrize("far", [28, 31, 40, 80])
 @pytest.mark.parametrize("bits,G,Kd", [(8, 64, 1024), (8, 128, 384), (8, 32, 160)])
 def test_large_activation_against_zero_weights(cuda, oracle, bits, G, Kd, far):
