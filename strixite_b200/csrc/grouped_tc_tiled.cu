@@ -8,21 +8,22 @@
 //
 // What bounds it (B200, SM cycles per step, the pieces measured alone): the MMAs take max(305, 4 n) for n tokens (below 76
 // tokens reading the A operand bounds them); dequantizing 128 x 128 codes and storing them to tensor memory takes the sixteen
-// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 660 a step for 15 tokens
-// and 840 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions.
-//   * One lane's MMAs and commits count, but its whole warp runs the loop, under control flow that the compiler can see to be uniform: addresses
-//     and descriptors then live in uniform registers.  Run by one lane of a diverged warp the MMAs took no longer to issue, but the loop
-//     around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps that showed it,
-//     which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 542 us at 777 tokens, 817 -> 760 at
-//     4096, dense 1001 x 8192 x 4096 64 -> 56, 4000 tokens Q8 234 -> 217.
+// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 545 a step for 15 tokens
+// and 730 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions
+// (1400 to 1450 a step, 584 of them the dequantization, at 61 to 66 % of the slots).
+//   * One lane's MMAs and commits count, but its whole warp runs the loop, under control flow that the compiler can see to be uniform:
+//     addresses and descriptors then live in uniform registers.  Run by one lane of a diverged warp the MMAs took no longer to issue, but
+//     the loop around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps
+//     that showed it, which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 540 us at 777
+//     tokens, 789 -> 728 at 4096, dense 1001 x 8192 x 4096 64.7 -> 57.1, 4000 tokens Q8 232 -> 216.
 //   * A commit and the next stage's wait cost ~250 whatever lies between: steps of 128 k, eight MMAs.
 //   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 162 instructions a warp and step, not 290.
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
 // A wider token tile would not be cheaper: it shares a dequantization that is no longer the bound, and 128 columns leave tensor
 // memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column stages of A.
-// Measured, 512 experts, d = 4096, I = 1024, Q4: gate/up + SwiGLU 1052 -> 579 us at 777 tokens (15 an expert), 1132 -> 771 at
-// 4096 (80 an expert), 3034 -> 2477 at 16384 (Zipf-popular experts); down 820 -> 330, 861 -> 460, 1997 -> 1750 (Q8).
+// Measured, 512 experts, d = 4096, I = 1024, Q4: gate/up + SwiGLU 540 us at 777 tokens (15 an expert), 728 at
+// 4096 (80 an expert); down 304 and 435 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
 //
 // SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up
