@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
                     for (int i = 0; i < 2 * MT; ++i) {
                         const uint32_t p = __shfl_sync(0xffffffffu, sm[i][at / 4], (lane & ~3) + at % 4);
                         s[i] = __uint_as_float(p << 16), mn[i] = __uint_as_float(p & 0xffff0000u);
-                        a[i] = w[i][at].template bf16<false>();
+                        a[i] = w[i][at].bf16();
                     }
                     const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
 #pragma unroll

@@ -103,7 +103,8 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = sq[nt] = 0.f;
     for (int c0 = lo; c0 < hi; c0 += kCodesAhead) {
         Codes<BITS> wa[kCodesAhead], wb[kCodesAhead];
-        uint32_t sm_a[kCodesAhead / 4], sm_b[kCodesAhead / 4];  // (scale, min) of rows a and b for chunks c0 + 4 i + c: handed round by shuffles
+        uint32_t sm_a[kCodesAhead / 4], sm_b[kCodesAhead / 4];  // (scale, min) of rows a and b for chunks c0 + 4 i + c: handed round by shuffles,
+        float zc_a[kCodesAhead / 4], zc_b[kCodesAhead / 4];     // and the codes that mean zero
 #pragma unroll
         for (int e = 0; e < kCodesAhead; ++e) {
             const int ch = min(c0 + e, hi - 1);
@@ -114,6 +115,8 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
             const int64_t gi = (int64_t)min(c0 + 4 * i + c, hi - 1) * kChunk / G;
             sm_a[i] = __ldg(scale + ra * groups + gi) | (uint32_t)__ldg(minv + ra * groups + gi) << 16;
             sm_b[i] = __ldg(scale + rb * groups + gi) | (uint32_t)__ldg(minv + rb * groups + gi) << 16;
+            zc_a[i] = zero_code<BITS>(__uint_as_float(sm_a[i] << 16), __uint_as_float(sm_a[i] & 0xffff0000u));
+            zc_b[i] = zero_code<BITS>(__uint_as_float(sm_b[i] << 16), __uint_as_float(sm_b[i] & 0xffff0000u));
         }
 #pragma unroll
         for (int e0 = 0; e0 < kCodesAhead; e0 += kAhead) {
@@ -131,10 +134,12 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
             for (int e = 0; e < kAhead; ++e) {
                 const int i = e0 + e;
                 if (c0 + i >= hi) break;
-                const uint4 va = wa[i].template bf16<true>(), vb = wb[i].template bf16<true>(), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-                const uint32_t p_a = __shfl_sync(0xffffffffu, sm_a[i / 4], (lane & ~3) + i % 4), p_b = __shfl_sync(0xffffffffu, sm_b[i / 4], (lane & ~3) + i % 4);
-                const float s_a = __uint_as_float(p_a << 16), m_a = centered_min<BITS>(s_a, __uint_as_float(p_a & 0xffff0000u));
-                const float s_b = __uint_as_float(p_b << 16), m_b = centered_min<BITS>(s_b, __uint_as_float(p_b & 0xffff0000u));
+                const int from = (lane & ~3) + i % 4;
+                const uint32_t p_a = __shfl_sync(0xffffffffu, sm_a[i / 4], from), p_b = __shfl_sync(0xffffffffu, sm_b[i / 4], from);
+                const float z_a = __shfl_sync(0xffffffffu, zc_a[i / 4], from), z_b = __shfl_sync(0xffffffffu, zc_b[i / 4], from);
+                const float s_a = __uint_as_float(p_a << 16), m_a = shifted_min(s_a, __uint_as_float(p_a & 0xffff0000u), z_a);
+                const float s_b = __uint_as_float(p_b << 16), m_b = shifted_min(s_b, __uint_as_float(p_b & 0xffff0000u), z_b);
+                const uint4 va = wa[i].bf16(z_a), vb = wb[i].bf16(z_b), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     uint4 pl[Acts<T>::kPlanes];
@@ -277,9 +282,10 @@ __global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__res
         for (int a = 0; a < kUpAhead; ++a) {
             const int ch = c0 + a;
             if (ch >= chunks) break;
-            const uint4 va = wa[a].template bf16<true>(), vb = wb[a].template bf16<true>();
-            const float s_a = bf16_bits_to_f32(sa[a]), m_a = centered_min<BITS>(s_a, bf16_bits_to_f32(ma[a]));
-            const float s_b = bf16_bits_to_f32(sb[a]), m_b = centered_min<BITS>(s_b, bf16_bits_to_f32(mb[a]));
+            const float s_a = bf16_bits_to_f32(sa[a]), s_b = bf16_bits_to_f32(sb[a]);
+            const float z_a = zero_code<BITS>(s_a, bf16_bits_to_f32(ma[a])), z_b = zero_code<BITS>(s_b, bf16_bits_to_f32(mb[a]));
+            const float m_a = shifted_min(s_a, bf16_bits_to_f32(ma[a]), z_a), m_b = shifted_min(s_b, bf16_bits_to_f32(mb[a]), z_b);
+            const uint4 va = wa[a].bf16(z_a), vb = wb[a].bf16(z_b);
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float dot[4] = {0.f, 0.f, 0.f, 0.f};

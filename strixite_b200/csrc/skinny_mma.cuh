@@ -44,29 +44,34 @@ __device__ inline void split_planes(const float (&v)[8], uint4 (&p)[3]) {
     for (int j = 0; j < 3; ++j) p[j] = make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
 }
 
-// The lane's eight codes of a row as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).  CENTER: less the middle of their range, which
-// goes to the group's min instead (centered_min): without it the sums carry the codes' mean times sum(x), which the min takes off again,
-// and the rounding of the larger sums stays.  Not where a weight of zero (code and min) must take nothing from the rest of its dot.
-template <int BITS> constexpr float kCenter = BITS == 8 ? 128.f : 8.f;
+// 2^23 plus the code whose weight scale * code + min comes nearest to zero.  Codes less that one, with the rest in the min (shifted_min), are
+// as large as their weights: sums of codes as they are carry that code times sum(x), which the min takes off again, and the rounding of the larger
+// sums stays; and less the middle of their range a weight of zero takes bits from the rest of its dot when its activation is large.
+constexpr float kCodeBias = 0x1p23f;
 template <int BITS>
-__device__ inline float centered_min(float s, float m) { return fmaf(kCenter<BITS>, s, m); }
-template <int BITS, bool CENTER>
-__device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1) {
-    constexpr float kOff = 0x1p23f + (CENTER ? kCenter<BITS> : 0.f);
+__device__ inline float zero_code(float s, float m) { return fminf(fmaxf(__fdividef(-m, s), 0.f), (float)((1 << BITS) - 1)) + kCodeBias; }  // NaN: 0
+__device__ inline float shifted_min(float s, float m, float zero) {
+    const float z = zero - kCodeBias;
+    return z > 0.f ? fmaf(z, s, m) : m;
+}
+
+// The lane's eight codes of a row, less zero - 2^23, as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).
+template <int BITS>
+__device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1, float zero) {
     uint32_t r[4];
     if (BITS == 8) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint32_t w = i < 2 ? w0 : w1;  // 2^23 + code, less 2^23 and the center: no conversion instruction, which runs at a quarter rate
-            const float lo = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7442 : 0x7440)) - kOff;
-            const float hi = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7443 : 0x7441)) - kOff;
+            const uint32_t w = i < 2 ? w0 : w1;  // 2^23 + code, less `zero`: no conversion instruction, which runs at a quarter rate
+            const float lo = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7442 : 0x7440)) - zero;
+            const float hi = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7443 : 0x7441)) - zero;
             r[i] = pack_bf16_exact(lo, hi);
         }
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float lo = __uint_as_float(0x4B000000u | ((w0 >> (8 * i)) & 15u)) - kOff;
-            const float hi = __uint_as_float(0x4B000000u | ((w0 >> (8 * i + 4)) & 15u)) - kOff;
+            const float lo = __uint_as_float(0x4B000000u | ((w0 >> (8 * i)) & 15u)) - zero;
+            const float hi = __uint_as_float(0x4B000000u | ((w0 >> (8 * i + 4)) & 15u)) - zero;
             r[i] = pack_bf16_exact(lo, hi);
         }
     }
@@ -85,8 +90,7 @@ struct Codes {
             w[0] = __ldg(reinterpret_cast<const uint32_t *>(p));
         }
     }
-    template <bool CENTER>
-    __device__ inline uint4 bf16() const { return codes_bf16<BITS, CENTER>(w[0], w[BITS / 4 - 1]); }
+    __device__ inline uint4 bf16(float zero = kCodeBias) const { return codes_bf16<BITS>(w[0], w[BITS / 4 - 1], zero); }
 };
 
 // Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Four where the last 32 are more than half

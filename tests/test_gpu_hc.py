@@ -111,6 +111,56 @@ def test_hc_mix_edges(cuda, oracle, dt, bits, G, T, d, r):
         assert all(torch.equal(a[0], b[t]) for a, b in zip(one, (h, w_in, inv, u)))
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,zero,far", [(8, 0, 20), (8, 3, 40), (8, 255, 28), (4, 0, 28), (4, 2, 20), (4, 15, 40)])
+def test_hc_mix_large_value_against_zero_weights(cuda, oracle, dt, bits, zero, far):
+    """An activation, and an h, 2^far times the others meets weights that are exactly zero (code `zero`, min -zero * scale): the dots are
+    those of the small values, and none of their bits may go.  Bounds as in test_hc_mix_edges."""
+    from strixite_b200 import kernels as K
+    H, eps, T, d, r, G, at = 4, 1e-6, 17, 256, 64, 32, 37
+    rng = np.random.default_rng(bits + zero + far)
+
+    def weight(rows, cols, std):
+        w = oracle.quantize(random_weights(rng, rows, cols, std=std), G, bits)
+        s = np.float32(2.0 ** -9)
+        w.scale[:, at // G], w.minv[:, at // G] = oracle.f32_to_bf16(s[None])[0], oracle.f32_to_bf16((-zero * s)[None])[0]
+        if bits == 8:
+            w.q[:, at] = zero
+        else:
+            low = w.q[:, at // 2] & 0x0F if at % 2 else zero
+            w.q[:, at // 2] = low | ((zero if at % 2 else w.q[:, at // 2] >> 4) << 4)
+        assert np.all(oracle.affine_weights(w)[:, at] == 0)
+        return w
+
+    wd, wu = weight(r + H, H * d, 0.05), weight(H * d, r, 0.2)
+    x = rng.standard_normal((T, H * d)).astype(np.float32)
+    x[::2, at] = 2.0 ** far
+    xd, act = torch.from_numpy(x).to(cuda), K.Act.F32
+    if dt == torch.bfloat16:
+        xd, act = xd.to(torch.bfloat16), K.Act.BF16
+        x = xd.float().cpu().numpy()
+    h, w_in, inv = (torch.full((T, n), float("nan"), dtype=torch.float32, device=cuda) for n in (r, H, H))
+    K.hc_mix_down(xd, upload(wd, cuda), T, H, d, r, True, eps, h, w_in, inv, act)
+    h_ref, w_in_ref, inv_ref = oracle.hc_mix_down(x, wd, H, d, r, True, eps)
+    terms = np.abs(x.reshape(T, H, d) * inv_ref[:, :, None]).reshape(T, H * d) @ np.abs(oracle.affine_weights(wd)).T / H
+    assert np.all(np.abs(h.cpu().numpy() - h_ref) <= 2.0 ** -16 * terms[:, :r])
+    assert np.all(np.abs(w_in.cpu().numpy() - w_in_ref) <= 2.0 ** -16 * terms[:, r:] + 2.0 ** -20)
+    hn = rng.standard_normal((T, r)).astype(np.float32)
+    hn[::2, at] = 2.0 ** far
+    norm_w = (rng.standard_normal(H * d) * 0.1).astype(np.float32)
+    inv1 = torch.ones((T, H), dtype=torch.float32, device=cuda)
+    u = torch.empty((T, d), dtype=dt, device=cuda)
+    xs = rng.standard_normal((T, H * d)).astype(np.float32)
+    xsd = torch.from_numpy(xs).to(cuda).to(dt)
+    xs = xsd.float().cpu().numpy()
+    K.hc_mix_up(torch.from_numpy(hn).to(cuda), K.to_chunk_major(upload(wu, cuda)), xsd, torch.from_numpy(norm_w).to(cuda), inv1, T, H, d, u, act)
+    u_ref = oracle.hc_mix_up(hn, wu, xs, norm_w, np.ones((T, H), dtype=np.float32), H, d)
+    z_terms = np.abs(hn).astype(np.float64) @ np.abs(oracle.affine_weights(wu)).T
+    bound = ((2.0 ** -18 * z_terms + 2.0 ** -20) * np.abs(xs * (1 + norm_w))).reshape(T, H, d).sum(axis=1) / H
+    bound += 2.0 ** -8 * np.abs(u_ref) if dt == torch.bfloat16 else 0
+    assert np.all(np.abs(u.float().cpu().numpy() - u_ref) <= bound)
+
+
 def test_hc_mix_argument_checks(cuda, oracle):
     from strixite_b200 import kernels as K
     rng = np.random.default_rng(1)
