@@ -383,6 +383,11 @@ int mix_down(const void *x, const SxbQView *w, int64_t T, int64_t H, int64_t d, 
     return SXB_OK;
 }
 
+// Shared memory of hc_up_kernel.  The limit that a launch asks for is the function's, one for all threads of the process: it is always that of the
+// longest rank, or a call of a short one would lower it between another thread's request and launch.
+constexpr size_t up_smem_bytes(int64_t r, int NT) { return (size_t)(r / kChunk) * NT * (3 * 32 * sizeof(uint4) + kMmaTokens * sizeof(float)); }
+static_assert(up_smem_bytes(kMaxRank, 4) <= 200 * 1024, "with its static shared memory an SM has it");
+
 template <int BITS>
 int mix_up(const float *h, const SxbQView *w, const void *x, const float *norm_w, const float *inv, int64_t T, int64_t H, int64_t d,
            void *u, int act, sxb_stream_t stream) {
@@ -398,13 +403,13 @@ int mix_up(const float *h, const SxbQView *w, const void *x, const float *norm_w
     SXB_CHECK(apart(u, T * d * act_bytes(act), x, T * H * d * act_bytes(act)), fn, ": u overlaps the streams x");
     const int64_t r = w->K;
     const int NT = token_eights(T);
-    const size_t smem = (size_t)(r / kChunk) * NT * (3 * 32 * sizeof(uint4) + kMmaTokens * sizeof(float));
+    const size_t smem = up_smem_bytes(r, NT);
     const bool vec_h = aligned16(h);
     auto st = static_cast<cudaStream_t>(stream);
 #define SXB_HC_UP(TYPE, NTV)                                                                                                           \
     do {                                                                                                                               \
         auto kern = hc_up_kernel<TYPE, BITS, NTV>;                                                                                     \
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory"); \
+        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)up_smem_bytes(kMaxRank, NTV)), fn, ": reserving shared memory"); \
         const dim3 grid((unsigned)(d / kUpCols), (unsigned)((T + NTV * kMmaTokens - 1) / (NTV * kMmaTokens)));                          \
         kern<<<grid, 32 * kStreams, smem, st>>>(h, w->q, w->scale, w->minv, w->G, static_cast<const TYPE *>(x), norm_w, inv, d, (int)r, T,  \
                                                 vec_h, static_cast<TYPE *>(u));                                                        \

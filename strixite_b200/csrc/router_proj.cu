@@ -506,7 +506,9 @@ int sxb_router_logits_wmma(const void *x, const void *planes_in, int planes, con
                                kGemmBK, kTile, CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
         return rc;
     const size_t smem = (size_t)a.stages * (1 + planes) * kOperandBytes + 1024;
-    SXB_CUDA(cudaFuncSetAttribute(logits_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
+    // the function's limit is one for all threads of the process: always the largest (three planes), not this call's
+    SXB_CUDA(cudaFuncSetAttribute(logits_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kOperandBytes + 1024), fn,
+             ": reserving shared memory");
     const int64_t items = (a.Npad / kTile) * ((M + kTile - 1) / kTile);
     const unsigned grid = (unsigned)std::min<int64_t>(items, sm_count());
     logits_gemm_kernel<<<grid, kGemmThreads, smem, static_cast<cudaStream_t>(stream)>>>(a, xmap, wmap);

@@ -925,7 +925,8 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
               " bytes of shared memory for one tile's activations, more than ", kMaxDynSmem,
               " (K * 16 * ceil(A / 8) bytes for the per-slot combine, K * 16 otherwise; use the grouped form)");
     auto kern = stream_kernel<BITS, G, MODE, SRC, TOUT>;
-    SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn,
+    // the function's limit is one for all threads of the process: always the largest, not this call's, which would take it from another thread's
+    SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn,
              ": reserving shared memory");
     // A dense projection of few units for the machine's warps: up to eight warps share one, as long as that gives a warp at most two and a half
     // parts in turn.  A warp alone walks K / (4 * kStepCodes) blocks one after another, each a round trip to memory (2048 x 4096

@@ -178,6 +178,60 @@ def test_hc_mix_argument_checks(cuda, oracle):
         K.hc_mix_down(x, wd, T, H, d, r, True, 0.0, h, w_in, inv, K.Act.BF16)
 
 
+def test_concurrent_calls_of_different_shared_memory(cuda, oracle):
+    """Threads with a stream each may call the library at the same time.  A kernel's shared-memory limit is one for the whole process, and
+    these calls of one kernel need different amounts (an up mix of rank 1024 beside one of rank 32; a dense Q4 projection of a long row
+    beside a short one; a router projection of three planes beside one): every call must go through, with the results it has alone."""
+    import threading
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(3)
+    H, d, T = 4, 64, 25
+
+    def up(r):
+        wu = K.to_chunk_major(upload(oracle.quantize(random_weights(rng, H * d, r, std=0.2), 32, 8), cuda))
+        h, inv = torch.randn((T, r), device=cuda), torch.rand((T, H), device=cuda)
+        x, nw, u = torch.randn((T, H * d), device=cuda), torch.randn(H * d, device=cuda), torch.empty((T, d), device=cuda)
+        return u, lambda: K.hc_mix_up(h, wu, x, nw, inv, T, H, d, u, K.Act.F32)
+
+    def dense(k):
+        w = upload(oracle.quantize(random_weights(rng, 64, k), 64, 4), cuda)
+        x, y = torch.randn((4, k), device=cuda).to(torch.bfloat16), torch.empty((4, 64), dtype=torch.bfloat16, device=cuda)
+        return y, lambda: K.linear_qw(x, w, y, 4, K.Act.BF16)
+
+    def router(planes):
+        w = K.router_prepare(torch.randn((64, 128), device=cuda), planes)
+        x, out = torch.randn((130, 128), device=cuda).to(torch.bfloat16), torch.empty((130, 64), device=cuda)
+        return out, lambda: K.router_logits_wmma(x, w, None, out)
+
+    for make, sizes in ((up, (1024, 32)), (dense, (11008, 256)), (router, (3, 1))):
+        calls = [make(n) for n in sizes]
+        want = []
+        for out, call in calls:
+            call()
+            torch.cuda.synchronize()
+            want.append(out.clone())
+            out.zero_()
+        failed = []
+
+        def loop(call):
+            try:
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    for _ in range(3000):
+                        call()
+            except K.Error as e:
+                failed.append(str(e))
+
+        threads = [threading.Thread(target=loop, args=(call,)) for _, call in calls]
+        torch.cuda.synchronize()
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert not failed, failed[0]
+        assert all(torch.equal(out, w) for (out, _), w in zip(calls, want))
+
+
 def _ws(nbytes, device):
     return torch.empty(nbytes, dtype=torch.uint8, device=device)  # the caching allocator hands out 512-byte aligned blocks
 
