@@ -181,55 +181,67 @@ def test_hc_mix_argument_checks(cuda, oracle):
 def test_concurrent_calls_of_different_shared_memory(cuda, oracle):
     """Threads with a stream each may call the library at the same time.  A kernel's shared-memory limit is one for the whole process, and
     these calls of one kernel need different amounts (an up mix of rank 1024 beside one of rank 32; a dense Q4 projection of a long row
-    beside a short one; a router projection of three planes beside one): every call must go through, with the results it has alone."""
+    beside a short one; a router projection of three planes beside one): every call must go through, with the result it has alone.  A
+    call's own limit, set before its launch, let one up mix in 300 fail."""
+    import ctypes as C
     import threading
+    import time
+    from strixite_b200 import _lib
     from strixite_b200 import kernels as K
     rng = np.random.default_rng(3)
+    lib = _lib.load()
     H, d, T = 4, 64, 25
 
-    def up(r):
+    def p(t):
+        return C.c_void_p(t.data_ptr())
+
+    def up(r, st):
         wu = K.to_chunk_major(upload(oracle.quantize(random_weights(rng, H * d, r, std=0.2), 32, 8), cuda))
         h, inv = torch.randn((T, r), device=cuda), torch.rand((T, H), device=cuda)
         x, nw, u = torch.randn((T, H * d), device=cuda), torch.randn(H * d, device=cuda), torch.empty((T, d), device=cuda)
-        return u, lambda: K.hc_mix_up(h, wu, x, nw, inv, T, H, d, u, K.Act.F32)
+        args = (p(h), C.byref(wu.c()), p(x), p(nw), p(inv), T, H, d, p(u), int(K.Act.F32), st)
+        return u, (wu, h, inv, x, nw), lambda: lib.sxb_hc_mix_up_q8(*args)
 
-    def dense(k):
+    def dense(k, st):
         w = upload(oracle.quantize(random_weights(rng, 64, k), 64, 4), cuda)
         x, y = torch.randn((4, k), device=cuda).to(torch.bfloat16), torch.empty((4, 64), dtype=torch.bfloat16, device=cuda)
-        return y, lambda: K.linear_qw(x, w, y, 4, K.Act.BF16)
+        args = (p(x), C.byref(w.c()), p(y), 4, int(K.Act.BF16), int(K.Act.BF16), st)
+        return y, (w, x), lambda: lib.sxb_linear_q4(*args)
 
-    def router(planes):
+    def router(planes, st):
         w = K.router_prepare(torch.randn((64, 128), device=cuda), planes)
         x, out = torch.randn((130, 128), device=cuda).to(torch.bfloat16), torch.empty((130, 64), device=cuda)
-        return out, lambda: K.router_logits_wmma(x, w, None, out)
+        args = (p(x), p(w.data), planes, None, 130, 64, 128, p(out), 64, st)
+        return out, (w, x), lambda: lib.sxb_router_logits_wmma(*args)
 
     for make, sizes in ((up, (1024, 32)), (dense, (11008, 256)), (router, (3, 1))):
-        calls = [make(n) for n in sizes]
-        want = []
-        for out, call in calls:
-            call()
+        streams = [torch.cuda.Stream() for _ in sizes]
+        calls = [make(n, C.c_void_p(s.cuda_stream)) for n, s in zip(sizes, streams)]
+        want, failed = [], []
+        torch.cuda.synchronize()
+        for out, _, call in calls:
+            assert call() == 0
             torch.cuda.synchronize()
             want.append(out.clone())
             out.zero_()
-        failed = []
-
-        def loop(call):
-            try:
-                with torch.cuda.stream(torch.cuda.Stream()):
-                    for _ in range(3000):
-                        call()
-            except K.Error as e:
-                failed.append(str(e))
-
-        threads = [threading.Thread(target=loop, args=(call,)) for _, call in calls]
         torch.cuda.synchronize()
+        stop = time.monotonic() + 1.0
+
+        def loop(call, stream):
+            while time.monotonic() < stop:
+                for _ in range(200):
+                    if call() != 0:
+                        failed.append(lib.sxb_last_error().decode())
+                stream.synchronize()
+
+        threads = [threading.Thread(target=loop, args=(call, s)) for (_, _, call), s in zip(calls, streams)]
         for t in threads:
             t.start()
         for t in threads:
             t.join()
         torch.cuda.synchronize()
-        assert not failed, failed[0]
-        assert all(torch.equal(out, w) for (out, _), w in zip(calls, want))
+        assert not failed, (len(failed), failed[0])
+        assert all(torch.equal(out, w) for (out, _, _), w in zip(calls, want))
 
 
 def _ws(nbytes, device):
