@@ -51,10 +51,48 @@ struct Weights<float> {
     }
 };
 
-template <typename TW>
-__device__ __noinline__ float plain_dot(const uint16_t *x, const TW *w, int64_t K) {
-    float sum = 0.f;
-    for (int64_t k = 0; k < K; ++k) sum = fmaf(bf16_bits_to_f32(x[k]), load_as_f32(w, k), sum);
+// Whether a token's activations hold a NaN, and its dot with an FP32 weight row; by a whole warp.
+__device__ __noinline__ bool row_has_nan(const uint16_t *x, int64_t K) {
+    uint32_t nan = 0;
+#pragma unroll 4
+    for (int64_t e = threadIdx.x & 31; e < K / 8; e += 32) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x) + e);
+        const uint32_t xs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) nan |= ((xs[i] & 0x7fffu) > 0x7f80u) | ((xs[i] & 0x7fff0000u) > 0x7f800000u);
+    }
+    return __any_sync(0xffffffffu, nan != 0);
+}
+__device__ __noinline__ float plain_dot(const uint16_t *x, const float *w, int64_t K) {
+    double sum = 0.0;
+#pragma unroll 2
+    for (int64_t e = threadIdx.x & 31; e < K / 8; e += 32) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(x) + e);
+        const float4 a = __ldg(reinterpret_cast<const float4 *>(w) + 2 * e), b = __ldg(reinterpret_cast<const float4 *>(w) + 2 * e + 1);
+        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        const uint32_t xs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sum += (double)f[i] * (double)__uint_as_float((i & 1) ? (xs[i / 2] & 0xffff0000u) : (xs[i / 2] << 16));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    return (float)sum;
+}
+// The sum of a lane whose result came out NaN, formed again by its whole converged warp.  An infinity times a plane that is zero, or split into planes, is NaN:
+// the plain sum says what it is; a NaN among the token's activations, looked at once for all its rows, leaves nothing to say.  (One thread
+// walking the contraction for each such result, as it stood here before: 128 x 513 x 4096 with NaN in every token 885 us, now 71; 32 without.)
+__device__ inline float formed_again(bool bad, float sum, int64_t t, int64_t n, const uint16_t *x, const float *w, int64_t K) {
+    const int lane = threadIdx.x & 31;
+    int64_t seen = -1;
+    bool nan = false;
+    for (uint32_t todo = __ballot_sync(0xffffffffu, bad); todo != 0; todo &= todo - 1) {
+        const int from = __ffs(todo) - 1;
+        const int64_t t_of = __shfl_sync(0xffffffffu, t, from), n_of = __shfl_sync(0xffffffffu, n, from);
+        if (t_of != seen) seen = t_of, nan = row_has_nan(x + t_of * K, K);
+        if (nan) continue;
+        const float plain = plain_dot(x + t_of * K, w + n_of * K, K);
+        if (lane == from) sum = plain;
+    }
     return sum;
 }
 
@@ -140,19 +178,20 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 2)
         }
         cluster_sync();
         // a CTA finishes every eighth token of the group
-        if (threadIdx.x < NT * kMmaRows) {
-            const int tt = rank + kStreamSplit * (threadIdx.x / kMmaRows), row = threadIdx.x % kMmaRows;
+        if (warp == 0) {
+            const int tt = rank + kStreamSplit * (lane / kMmaRows), row = lane % kMmaRows;
             const int64_t n = n0 + row, t = t0 + tt;
-            if (n < N && t < M) {
-                float v[kStreamSplit], sum = 0.f;
+            const bool out = lane < NT * kMmaRows && n < N && t < M;
+            float sum = 0.f;
+            if (out) {
+                float v[kStreamSplit];
 #pragma unroll
                 for (int p = 0; p < kStreamSplit; ++p) v[p] = ld_cluster(&cta_part[tt][row], p);
 #pragma unroll
                 for (int p = 0; p < kStreamSplit; ++p) sum += v[p];
-                // An infinity times a plane that is zero, or split into planes, is NaN: the plain sum says what it is.
-                if (P > 1 && isnan(sum)) sum = plain_dot(x + t * K, w + n * K, K);
-                store_from_f32(y, t * ld + n, sum + (bias != nullptr ? bias[n] : 0.f));
             }
+            if constexpr (P > 1) sum = formed_again(out && isnan(sum), sum, t, n, x, w, K);
+            if (out) store_from_f32(y, t * ld + n, sum + (bias != nullptr ? bias[n] : 0.f));
         }
         cluster_sync();  // the parts have been read: the next group may overwrite them, or the CTA leave
     }

@@ -83,6 +83,51 @@ def test_router_logits_streaming_edges(cuda, oracle, M, N, K, w_bf16):
     assert np.array_equal(got2[bad], want2[bad], equal_nan=True) and np.array_equal(got2[~bad], out.cpu().numpy()[~bad])
 
 
+@pytest.mark.parametrize("form", ["dense", "router"])
+def test_non_finite_rows(cuda, oracle, form):
+    """NaN and infinities in some tokens' activations and, for the router, weights: the results are what 64 bits give, and the other
+    tokens keep their bits.  Nor does a token of NaN hold the call up: forming every one of its results again, one thread each, took 20 times
+    the call's time; looking at its activations once is a small part of it.  (x 5: the clock and the first launch.)"""
+    from strixite_b200 import kernels as Kn
+    M, N, K = 8, 4096, 4096
+    rng = np.random.default_rng(5)
+    x = torch.randn((M, K), device=cuda).to(torch.bfloat16)
+    if form == "dense":
+        wq = oracle.quantize(np.abs(rng.standard_normal((N, K)).astype(np.float32)), 64, 8)
+        wq.q[3, 7], wq.minv[3, 0] = 0, 0  # a weight of zero against an infinity
+        wd, w64 = upload(wq, cuda), torch.from_numpy(oracle.affine_weights(wq)).to(cuda)
+        call = lambda xs, out: Kn.linear_qw(xs, wd, out, M, Kn.Act.BF16, out_act=Kn.Act.F32)
+    else:
+        wd = torch.randn((N, K), device=cuda) * 0.02
+        wd[3, 7] = 0.0
+        wd[5, 9], wd[6, 9] = float("-inf"), float("nan")
+        w64 = wd.double()
+        call = lambda xs, out: Kn.router_logits(xs, wd, None, out)
+    bad = x.clone()
+    bad[1, 4000], bad[2, 7], bad[4, 7], bad[4, 8] = float("nan"), float("inf"), float("inf"), float("-inf")
+    y, yb = (torch.empty((M, N), dtype=torch.float32, device=cuda) for _ in range(2))
+    call(x, y)
+    call(bad, yb)
+    want = torch.stack([(row * w64).sum(dim=1) for row in bad.double()])
+    odd = ~torch.isfinite(want)
+    assert torch.equal(torch.isnan(yb), torch.isnan(want)) and torch.equal(yb[odd].nan_to_num(), want[odd].float().nan_to_num())
+    assert torch.equal(yb[[0, 3, 5, 6, 7]].nan_to_num(), y[[0, 3, 5, 6, 7]].nan_to_num())
+
+    def us(xs):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        best = float("inf")
+        for _ in range(5):
+            e[0].record()
+            for _ in range(10):
+                call(xs, y)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]) * 100)
+        return best
+    plain, all_nan = us(x), us(torch.full_like(x, float("nan")))
+    assert all_nan <= 5 * plain, (plain, all_nan)
+
+
 @pytest.mark.parametrize("M,N,K,planes,w_bf16", [(4096, 513, 4096, 3, False), (300, 513, 1024, 2, False), (1000, 129, 512, 1, True),
                                                    (128, 64, 256, 3, False)])
 def test_router_logits_tcgen05(cuda, oracle, M, N, K, planes, w_bf16):
