@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = sq[nt] = 0.f;
     for (int c0 = lo; c0 < hi; c0 += kCodesAhead) {
         Codes<BITS> wa[kCodesAhead], wb[kCodesAhead];
-        uint32_t sm_a[kCodesAhead / 4], sm_b[kCodesAhead / 4];  // (scale, min) of rows a and b for chunks c0 + 4 i + c: handed round by shuffles,
-        float zc_a[kCodesAhead / 4], zc_b[kCodesAhead / 4];     // and the codes that mean zero
+        uint32_t sz_a[kCodesAhead / 4], sz_b[kCodesAhead / 4];  // scales, zero codes and mins of rows a and b for chunks c0 + 4 i + c:
+        float mn_a[kCodesAhead / 4], mn_b[kCodesAhead / 4];     // handed round by shuffles
 #pragma unroll
         for (int e = 0; e < kCodesAhead; ++e) {
             const int ch = min(c0 + e, hi - 1);
@@ -113,10 +113,8 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
 #pragma unroll
         for (int i = 0; i < kCodesAhead / 4; ++i) {
             const int64_t gi = (int64_t)min(c0 + 4 * i + c, hi - 1) * kChunk / G;
-            sm_a[i] = __ldg(scale + ra * groups + gi) | (uint32_t)__ldg(minv + ra * groups + gi) << 16;
-            sm_b[i] = __ldg(scale + rb * groups + gi) | (uint32_t)__ldg(minv + rb * groups + gi) << 16;
-            zc_a[i] = zero_code<BITS>(__uint_as_float(sm_a[i] << 16), __uint_as_float(sm_a[i] & 0xffff0000u));
-            zc_b[i] = zero_code<BITS>(__uint_as_float(sm_b[i] << 16), __uint_as_float(sm_b[i] & 0xffff0000u));
+            pack_group<BITS>(__ldg(scale + ra * groups + gi), __ldg(minv + ra * groups + gi), sz_a[i], mn_a[i]);
+            pack_group<BITS>(__ldg(scale + rb * groups + gi), __ldg(minv + rb * groups + gi), sz_b[i], mn_b[i]);
         }
 #pragma unroll
         for (int e0 = 0; e0 < kCodesAhead; e0 += kAhead) {
@@ -135,11 +133,10 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
                 const int i = e0 + e;
                 if (c0 + i >= hi) break;
                 const int from = (lane & ~3) + i % 4;
-                const uint32_t p_a = __shfl_sync(0xffffffffu, sm_a[i / 4], from), p_b = __shfl_sync(0xffffffffu, sm_b[i / 4], from);
-                const float z_a = __shfl_sync(0xffffffffu, zc_a[i / 4], from), z_b = __shfl_sync(0xffffffffu, zc_b[i / 4], from);
-                const float s_a = __uint_as_float(p_a << 16), m_a = shifted_min(s_a, __uint_as_float(p_a & 0xffff0000u), z_a);
-                const float s_b = __uint_as_float(p_b << 16), m_b = shifted_min(s_b, __uint_as_float(p_b & 0xffff0000u), z_b);
-                const uint4 va = wa[i].bf16(z_a), vb = wb[i].bf16(z_b), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+                const uint32_t w_a = __shfl_sync(0xffffffffu, sz_a[i / 4], from), w_b = __shfl_sync(0xffffffffu, sz_b[i / 4], from);
+                const float m_a = __shfl_sync(0xffffffffu, mn_a[i / 4], from), m_b = __shfl_sync(0xffffffffu, mn_b[i / 4], from);
+                const float s_a = group_scale(w_a), s_b = group_scale(w_b);
+                const uint4 va = wa[i].bf16(group_zero(w_a)), vb = wb[i].bf16(group_zero(w_b)), ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
                     uint4 pl[Acts<T>::kPlanes];
@@ -203,7 +200,7 @@ __global__ void __launch_bounds__(32 * kDownWarps, 2) hc_down_kernel(const T *__
 // hc_mix_up.  grid = (d / 16, token groups of 8 NT); warp s owns rows s * d + 16 blockIdx.x .. + 15 of W_up, whose chunks lie side by side in
 // the chunk-major layout.  h is an FP32 number and stays one: three BF16 planes.
 constexpr int kUpCols = kMmaRows;  // output columns per CTA
-constexpr int kUpAhead = 10;       // chunks of codes in flight per warp: r = 320 has ten
+constexpr int kUpAhead = 12;       // chunks of codes in flight per warp: r = 320 has ten
 
 template <typename T, int BITS, int NT>
 __global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__restrict__ h, const uint8_t *__restrict__ q,
@@ -220,16 +217,21 @@ __global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__res
     const int64_t N = kStreams * d, j0 = (int64_t)blockIdx.x * kUpCols, row = s * d + j0 + g, t0 = (int64_t)blockIdx.y * kTok;
     // the first chunks' codes are asked for before anything else
     Codes<BITS> wa[kUpAhead], wb[kUpAhead];
-    uint16_t sa[kUpAhead], sb[kUpAhead], ma[kUpAhead], mb[kUpAhead];
+    uint16_t sa[kUpAhead / 4], sb[kUpAhead / 4], ma[kUpAhead / 4], mb[kUpAhead / 4];  // of chunk 4 i + c: the four lanes of a row share it
     auto fetch = [&](int slot, int ch) {
         const uint8_t *p = q + ((int64_t)ch * N + row) * (kChunk * BITS / 8) + c * BITS;
         wa[slot].load(p), wb[slot].load(p + 8 * (kChunk * BITS / 8));
-        const int64_t gi = (int64_t)ch * kChunk / G * N + row;
+    };
+    auto fetch_scales = [&](int slot, int ch) {
+        const int64_t gi = (int64_t)min(ch + c, chunks - 1) * kChunk / G * N + row;
         sa[slot] = __ldg(scale + gi), ma[slot] = __ldg(minv + gi), sb[slot] = __ldg(scale + gi + 8), mb[slot] = __ldg(minv + gi + 8);
     };
 #pragma unroll
     for (int a = 0; a < kUpAhead; ++a)
         if (a < chunks) fetch(a, a);
+#pragma unroll
+    for (int i = 0; i < kUpAhead / 4; ++i)
+        if (4 * i < chunks) fetch_scales(i, 4 * i);
     // what the tokens' terms take beside z: the lane's tokens are 2 c and 2 c + 1 of each eight, its columns g and g + 8
     float xi[NT][4];
 #pragma unroll
@@ -278,14 +280,21 @@ __global__ void __launch_bounds__(32 * kStreams) hc_up_kernel(const float *__res
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
     for (int c0 = 0; c0 < chunks; c0 += kUpAhead) {
+        uint32_t sz_a = 0, sz_b = 0;
+        float mn_a = 0.f, mn_b = 0.f;
 #pragma unroll
         for (int a = 0; a < kUpAhead; ++a) {
             const int ch = c0 + a;
             if (ch >= chunks) break;
-            const float s_a = bf16_bits_to_f32(sa[a]), s_b = bf16_bits_to_f32(sb[a]);
-            const float z_a = zero_code<BITS>(s_a, bf16_bits_to_f32(ma[a])), z_b = zero_code<BITS>(s_b, bf16_bits_to_f32(mb[a]));
-            const float m_a = shifted_min(s_a, bf16_bits_to_f32(ma[a]), z_a), m_b = shifted_min(s_b, bf16_bits_to_f32(mb[a]), z_b);
-            const uint4 va = wa[a].bf16(z_a), vb = wb[a].bf16(z_b);
+            if (a % 4 == 0) {
+                pack_group<BITS>(sa[a / 4], ma[a / 4], sz_a, mn_a), pack_group<BITS>(sb[a / 4], mb[a / 4], sz_b, mn_b);
+                if (ch + kUpAhead < chunks) fetch_scales(a / 4, ch + kUpAhead);
+            }
+            const int from = (lane & ~3) + a % 4;
+            const uint32_t w_a = __shfl_sync(0xffffffffu, sz_a, from), w_b = __shfl_sync(0xffffffffu, sz_b, from);
+            const float m_a = __shfl_sync(0xffffffffu, mn_a, from), m_b = __shfl_sync(0xffffffffu, mn_b, from);
+            const float s_a = group_scale(w_a), s_b = group_scale(w_b);
+            const uint4 va = wa[a].bf16(group_zero(w_a)), vb = wb[a].bf16(group_zero(w_b));
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 float dot[4] = {0.f, 0.f, 0.f, 0.f};

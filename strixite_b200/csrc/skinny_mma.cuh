@@ -49,11 +49,24 @@ __device__ inline void split_planes(const float (&v)[8], uint4 (&p)[3]) {
 // sums stays; and less the middle of their range a weight of zero takes bits from the rest of its dot when its activation is large.
 constexpr float kCodeBias = 0x1p23f;
 template <int BITS>
-__device__ inline float zero_code(float s, float m) { return fminf(fmaxf(__fdividef(-m, s), 0.f), (float)((1 << BITS) - 1)) + kCodeBias; }  // NaN: 0
+__device__ inline float zero_code(float s, float m) {
+    constexpr float kTop = (1 << BITS) - 1;
+    float inv;  // any code is right, if not as good: an approximate reciprocal will do
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(s));
+    return fmaf(__saturatef(inv * (m * (-1.f / kTop))), kTop, kCodeBias);  // NaN saturates to 0
+}
 __device__ inline float shifted_min(float s, float m, float zero) {
     const float z = zero - kCodeBias;
     return z > 0.f ? fmaf(z, s, m) : m;
 }
+// A row group's scale and zero code in a word, for the lanes that share the row.
+template <int BITS>
+__device__ inline void pack_group(uint16_t s, uint16_t m, uint32_t &word, float &min) {
+    const float zero = zero_code<BITS>(bf16_bits_to_f32(s), bf16_bits_to_f32(m));
+    word = (uint32_t)s << 16 | (__float_as_uint(zero) & 0xffu), min = shifted_min(bf16_bits_to_f32(s), bf16_bits_to_f32(m), zero);
+}
+__device__ inline float group_scale(uint32_t word) { return __uint_as_float(word & 0xffff0000u); }
+__device__ inline float group_zero(uint32_t word) { return __uint_as_float((word & 0xffu) | 0x4B000000u); }
 
 // The lane's eight codes of a row, less zero - 2^23, as BF16 pairs: Q8 from two words, Q4 from one (w1 unused).
 template <int BITS>
