@@ -8,9 +8,10 @@
 // order in shared memory.  Which runs a warp takes follows from K alone, so a row's bits depend neither on the batch nor on the tile.
 //
 // What bounds it: for few tokens a launch, the round trips to memory and the parts' meeting; for more the code conversions, once per
-// 32 tokens.  The form before it (stream_mma.cu, which keeps Q4) staged a tile of 8 tokens as scaled F16 in every CTA and converted every
-// code again for the next 8.  As CUDA graphs, us before -> now: 2048 x 4096, 1 / 16 / 37 / 150 tokens 9.5 -> 6.7, 12.0 -> 7.9,
-// 21.7 -> 16.9, 41.4 -> 34.6; 4096 x 1024 7.3 -> 4.1, 8.2 -> 4.9, 13.5 -> 9.5, 23.9 -> 21.9; 8192 x 4096, 8 / 63 tokens 16.4 -> 13.7, 58.5 -> 48.0.
+// 32 tokens, and the activations' way through L1, once per 16 rows; for many rows of x see dense_rows_kernel.  The form before it (stream_mma.cu,
+// which keeps Q4) staged a tile of 8 tokens as scaled F16 in every CTA and converted every code again for the next 8.  As CUDA graphs on weights that lie in L2,
+// us before -> now: 2048 x 4096, 1 / 16 / 40 / 300 tokens 9.6 -> 6.4, 12.2 -> 7.7, 21.7 -> 15.3, 70 -> 55; 4096 x 1024 7.4 -> 4.0, 8.3 -> 4.7, 13.7 -> 8.6,
+// 35.5 -> 37.2; 8192 x 4096, 8 / 63 / 300 tokens 16.5 -> 12.7, 56.7 -> 45.0, 205 -> 205; weights from HBM 8 tokens 24.6 -> 20.4, 63 67.6 -> 55.3.
 // Error against 64 bits (2-norms) 1.15e-7 .. 2.3e-7 -> 0.95e-7 .. 1.2e-7.  Q4, whose nibbles take more instructions to BF16 than to F16,
 // was slower this way (8192 x 4096, 8 tokens: 13 -> 17) and stays there.
 
@@ -104,6 +105,41 @@ __device__ __noinline__ void form_again(const float (&sums)[TOKENS][ROWS + 1], c
         }
 }
 
+// sum(x) over a run, of the lane's tokens 2 c and 2 c + 1.
+__device__ inline uint64_t run_sums(const uint4 &x) {
+    const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+    float sx[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_run(sx, ones, ones, x);
+    return pair(sx[0], sx[1]);
+}
+// acc += a run's share of the dots with P eights of tokens: a, s, mn = codes, scales and mins of the lane's rows, x = its tokens' activations, sx =
+// the sums of its tokens 2 c and 2 c + 1.  An MMA's result is some 35 cycles away: the runs' second halves come after all of the first ones.
+template <int P, int MT>
+__device__ inline void add_runs(uint64_t (*acc)[MT][2], const uint4 (&a)[2 * MT], const float (&s)[2 * MT], const float (&mn)[2 * MT], const uint4 *x, const uint64_t *sx) {
+    float dot[P][MT][4];
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+            dot[p][m][0] = dot[p][m][1] = dot[p][m][2] = dot[p][m][3] = 0.f;
+            mma_bf16(dot[p][m], a[2 * m].x, a[2 * m + 1].x, a[2 * m].y, a[2 * m + 1].y, x[p].x, x[p].y);
+        }
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) mma_bf16(dot[p][m], a[2 * m].z, a[2 * m + 1].z, a[2 * m].w, a[2 * m + 1].w, x[p].z, x[p].w);
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int r = 2 * m + i;
+                // the two terms meet before the sum does: they cancel by and large, and what they round is theirs alone
+                acc[p][m][i] = add_pair(acc[p][m][i], fma_pair(pair(s[r], s[r]), pair(dot[p][m][2 * i], dot[p][m][2 * i + 1]), mul_pair(pair(mn[r], mn[r]), sx[p])));
+            }
+}
+
 template <int BITS, int MT, int NT, typename TOUT>
 __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     dense_mma_kernel(const uint16_t *__restrict__ x, const uint8_t *__restrict__ q, const uint16_t *__restrict__ scale,
@@ -119,91 +155,247 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     int64_t row[2 * MT];  // rows past the end stream the last one; their sums are dropped
 #pragma unroll
     for (int i = 0; i < 2 * MT; ++i) row[i] = min(n0 + 8 * i + g, N - 1);
-    for (int64_t t0 = (int64_t)blockIdx.y * kTok; t0 < M; t0 += (int64_t)gridDim.y * kTok) {
-        float acc[MT][NT][4];
+    const int64_t t0 = (int64_t)blockIdx.y * kTok;
+    uint64_t acc[NT][MT][2];  // rows g + 16 m (+ 8), tokens 2 c and 2 c + 1 of each eight
 #pragma unroll
-        for (int m = 0; m < MT; ++m)
+    for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) acc[m][nt][0] = acc[m][nt][1] = acc[m][nt][2] = acc[m][nt][3] = 0.f;
-        for (int r0 = lo; r0 < hi; r0 += kAhead) {
-            Codes<BITS> w[2 * MT][kAhead];
-            uint32_t sm[2 * MT][kAhead / 4];  // (scale, min) for run r0 + 4 i + c: handed round by shuffles
+        for (int nt = 0; nt < NT; ++nt) acc[nt][m][0] = acc[nt][m][1] = 0;
+    for (int r0 = lo; r0 < hi; r0 += kAhead) {
+        Codes<BITS> w[2 * MT][kAhead];
+        uint32_t sm[2 * MT][kAhead / 4];  // (scale, min) for run r0 + 4 i + c: handed round by shuffles
 #pragma unroll
-            for (int e = 0; e < kAhead; ++e) {
-                const int64_t r = min(r0 + e, hi - 1);
+        for (int e = 0; e < kAhead; ++e) {
+            const int64_t r = min(r0 + e, hi - 1);
 #pragma unroll
-                for (int i = 0; i < 2 * MT; ++i) w[i][e].load(q + row[i] * row_bytes + r * kRunBytes + c * BITS);
-            }
+            for (int i = 0; i < 2 * MT; ++i) w[i][e].load(q + row[i] * row_bytes + r * kRunBytes + c * BITS);
+        }
 #pragma unroll
-            for (int e = 0; e < kAhead / 4; ++e) {
-                const int gi = min(r0 + 4 * e + c, hi - 1) / per_group;
+        for (int e = 0; e < kAhead / 4; ++e) {
+            const int gi = min(r0 + 4 * e + c, hi - 1) / per_group;
 #pragma unroll
-                for (int i = 0; i < 2 * MT; ++i)
-                    sm[i][e] = __ldg(scale + row[i] * groups + gi) | (uint32_t)__ldg(minv + row[i] * groups + gi) << 16;
-            }
+            for (int i = 0; i < 2 * MT; ++i)
+                sm[i][e] = __ldg(scale + row[i] * groups + gi) | (uint32_t)__ldg(minv + row[i] * groups + gi) << 16;
+        }
 #pragma unroll
-            for (int e0 = 0; e0 < kAhead; e0 += kActs) {
-                if (r0 + e0 >= hi) break;
-                uint4 xv[kActs][NT];
+        for (int e0 = 0; e0 < kAhead; e0 += kActs) {
+            if (r0 + e0 >= hi) break;
+            uint4 xv[kActs][NT];
 #pragma unroll
-                for (int e = 0; e < kActs; ++e)
+            for (int e = 0; e < kActs; ++e)
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) {
-                        const int64_t t = t0 + nt * kMmaTokens + g;
-                        xv[e][nt] = t < M && r0 + e0 + e < hi ? __ldg(reinterpret_cast<const uint4 *>(x + t * K + (int64_t)(r0 + e0 + e) * kMmaRun + 8 * c))
-                                                              : make_uint4(0u, 0u, 0u, 0u);
-                    }
+                for (int nt = 0; nt < NT; ++nt) {
+                    const int64_t t = t0 + nt * kMmaTokens + g;
+                    xv[e][nt] = t < M && r0 + e0 + e < hi ? __ldg(reinterpret_cast<const uint4 *>(x + t * K + (int64_t)(r0 + e0 + e) * kMmaRun + 8 * c))
+                                                          : make_uint4(0u, 0u, 0u, 0u);
+                }
 #pragma unroll
-                for (int e = 0; e < kActs; ++e) {
-                    const int at = e0 + e;
-                    if (r0 + at >= hi) break;
-                    uint4 a[2 * MT];
-                    float s[2 * MT], mn[2 * MT];
+            for (int e = 0; e < kActs; ++e) {
+                const int at = e0 + e;
+                if (r0 + at >= hi) break;
+                uint4 a[2 * MT];
+                float s[2 * MT], mn[2 * MT];
 #pragma unroll
-                    for (int i = 0; i < 2 * MT; ++i) {
-                        const uint32_t p = __shfl_sync(0xffffffffu, sm[i][at / 4], (lane & ~3) + at % 4);
-                        s[i] = __uint_as_float(p << 16), mn[i] = __uint_as_float(p & 0xffff0000u);
-                        a[i] = w[i][at].bf16();
-                    }
-                    const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+                for (int i = 0; i < 2 * MT; ++i) {
+                    const uint32_t p = __shfl_sync(0xffffffffu, sm[i][at / 4], (lane & ~3) + at % 4);
+                    s[i] = __uint_as_float(p << 16), mn[i] = __uint_as_float(p & 0xffff0000u);
+                    a[i] = w[i][at].bf16();
+                }
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) {
-                        float sx[4] = {0.f, 0.f, 0.f, 0.f};
-                        mma_run(sx, ones, ones, xv[e][nt]);
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-                            float dot[4] = {0.f, 0.f, 0.f, 0.f};
-                            mma_run(dot, a[2 * m], a[2 * m + 1], xv[e][nt]);
-                            float(&o)[4] = acc[m][nt];
-                            // the two terms meet before the sum does: they cancel by and large, and what they round is theirs alone
-                            o[0] += fmaf(s[2 * m], dot[0], mn[2 * m] * sx[0]), o[1] += fmaf(s[2 * m], dot[1], mn[2 * m] * sx[1]);
-                            o[2] += fmaf(s[2 * m + 1], dot[2], mn[2 * m + 1] * sx[0]), o[3] += fmaf(s[2 * m + 1], dot[3], mn[2 * m + 1] * sx[1]);
-                        }
-                    }
+                for (int nt = 0; nt < NT; ++nt) {
+                    const uint64_t sx = run_sums(xv[e][nt]);
+                    add_runs<1, MT>(&acc[nt], a, s, mn, &xv[e][nt], &sx);
                 }
             }
         }
-        __syncthreads();  // the previous group's parts have been read
+    }
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int t = nt * kMmaTokens + 2 * c, r = m * kMmaRows + g + 8 * i;
+                unpair(acc[nt][m][i], part[warp][t][r], part[warp][t + 1][r]);
+            }
+    __syncthreads();
+    bool bad = false;
+    for (int i = threadIdx.x; i < kTok * kRowsCta; i += 32 * kDenseWarps) {
+        const int tt = i / kRowsCta, r = i % kRowsCta;
+        const int64_t t = t0 + tt, n = n0 + r;
+        if (t >= M || n >= N) continue;
+        float sum = part[0][tt][r];
+#pragma unroll
+        for (int v = 1; v < kDenseWarps; ++v) sum += part[v][tt][r];
+        store_from_f32(y, t * N + n, sum);
+        part[0][tt][r] = sum, bad |= !isfinite(sum);
+    }
+    if (__syncthreads_or(bad)) form_again<kTok, kRowsCta, kDenseWarps>(part[0], x, q, scale, minv, t0, n0, M, N, K, G, y);
+}
+
+// ---- many rows of x: the same sums, bit for bit ------------------------------------------------------------------------
+// A CTA takes 256 weight rows x 32 tokens, a warp 32 of the rows over the whole contraction, one of its eight parts after another.  The
+// activations of 1024 k at a time lie in shared memory in fragment order with the sums of their runs, formed once for all rows; a warp's codes
+// come straight from memory, four runs ahead, and nothing is waited for in between.
+//
+// What bounds it: the L1 pipe, at 75 % (codes 32 of a run's 100 wavefronts, activations 16, scales), and the latencies between MMAs and sums with
+// four warps a scheduler (issue slots 48 %).  dense_mma_kernel reads the activations again for every 16 rows and converts a code for 32 tokens
+// as this does.  us, that -> this: 1024 x 8192 x 4096 648 -> 481, 4096 rows 2580 -> 1879, 4096 x 2048 x 4096 650 -> 480, 4096 x 4096 x 1024 447 -> 332
+// (eight parts of four runs each: closing them, and the start of a CTA, are a third; the form before these, stream_mma.cu, takes 292).  Activations copied 64 k at a time by cp.async with a barrier
+// a block: 1024 x 8192 x 4096 583.
+constexpr int kRowsMT = 2, kRowsNT = 4;  // of a warp
+constexpr int kRowsTile = kDenseWarps * kMmaRows * kRowsMT, kRowsTok = kMmaTokens * kRowsNT, kRowsChunk = 32;  // weight rows, tokens; runs in shared memory
+constexpr size_t kRowsSmem = (size_t)kRowsChunk * kRowsTok * (kMmaRun * 2 + sizeof(float)) + (size_t)kRowsTok * (kRowsTile + 1) * sizeof(float);
+
+template <typename TOUT>
+__global__ void __launch_bounds__(32 * kDenseWarps, 2)
+    dense_rows_kernel(const uint16_t *__restrict__ x, const uint8_t *__restrict__ q, const uint16_t *__restrict__ scale,
+                      const uint16_t *__restrict__ minv, int64_t M, int64_t N, int64_t K, int64_t G, TOUT *__restrict__ y) {
+    constexpr int MT = kRowsMT, NT = kRowsNT, kAhead = 4, kP = 2;
+    extern __shared__ __align__(16) unsigned char rows_smem[];
+    uint4 *acts = reinterpret_cast<uint4 *>(rows_smem);                           // [run][nt][lane]
+    uint64_t *sums = reinterpret_cast<uint64_t *>(acts + kRowsChunk * NT * 32);   // [run][nt][c]: of tokens 2 c and 2 c + 1
+    using Total = float[kRowsTok][kRowsTile + 1];
+    Total &total = *reinterpret_cast<Total *>(sums + kRowsChunk * NT * 4);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, wr = kMmaRows * MT * warp;
+    const int64_t n0 = (int64_t)blockIdx.x * kRowsTile, t0 = (int64_t)blockIdx.y * kRowsTok, groups = K / G;
+    const int runs = (int)(K / kMmaRun), per_group = (int)(G / kMmaRun);
+    const uint8_t *const tq = q + n0 * K + 8 * c;
+    const uint16_t *const ts = scale + n0 * groups, *const tm = minv + n0 * groups;
+    uint32_t q_at[2 * MT], s_at[2 * MT];  // rows past the end stream the last one; their sums are dropped
+#pragma unroll
+    for (int i = 0; i < 2 * MT; ++i) {
+        const uint32_t row = (uint32_t)min((int64_t)(wr + 8 * i + g), N - 1 - n0);
+        q_at[i] = row * (uint32_t)K, s_at[i] = row * (uint32_t)groups;
+    }
+    Codes<8> w[2 * MT][kAhead];
+    uint16_t ns[2 * MT], nm[2 * MT];  // scale and min of every fourth group, of the next four: handed round by shuffles
+    auto fetch = [&](int e, int r) {
+#pragma unroll
+        for (int i = 0; i < 2 * MT; ++i) w[i][e].load(tq + (q_at[i] + (uint32_t)(min(r, runs - 1) * kMmaRun)));
+    };
+    auto fetch_scales = [&](int g0) {
+        const uint32_t gi = min(g0 + c, (int)groups - 1);
+#pragma unroll
+        for (int i = 0; i < 2 * MT; ++i) ns[i] = __ldg(ts + (s_at[i] + gi)), nm[i] = __ldg(tm + (s_at[i] + gi));
+    };
+#pragma unroll
+    for (int e = 0; e < kAhead; ++e) fetch(e, e);
+    fetch_scales(0);
+    uint32_t sm[2 * MT];
+    const int lg_group = per_group == 1 ? 0 : per_group == 2 ? 1 : 2;
+    uint64_t acc[NT][MT][2];
+    auto clear = [&]() {
 #pragma unroll
         for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
+            for (int nt = 0; nt < NT; ++nt) acc[nt][m][0] = acc[nt][m][1] = 0;
+    };
+    clear();
+    int part = 0, part_end = runs / kDenseWarps;
+    auto close_parts = [&](int r) {  // the parts that end before run r
+        while (part < kDenseWarps && r == part_end) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) part[warp][nt * kMmaTokens + 2 * c + (i & 1)][m * kMmaRows + g + 8 * (i >> 1)] = acc[m][nt][i];
-        __syncthreads();
-        bool bad = false;
-        for (int i = threadIdx.x; i < kTok * kRowsCta; i += 32 * kDenseWarps) {
-            const int tt = i / kRowsCta, r = i % kRowsCta;
-            const int64_t t = t0 + tt, n = n0 + r;
-            if (t >= M || n >= N) continue;
-            float sum = part[0][tt][r];
+            for (int m = 0; m < MT; ++m) {  // all of a half's sums are read before any is written: one after another they cost 32 round trips
+                float before[NT][2][2];
+                auto at = [&](int nt, int i) { return &total[nt * kMmaTokens + 2 * c][wr + m * kMmaRows + g + 8 * i]; };
 #pragma unroll
-            for (int v = 1; v < kDenseWarps; ++v) sum += part[v][tt][r];
-            store_from_f32(y, t * N + n, sum);
-            part[0][tt][r] = sum, bad |= !isfinite(sum);
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (part > 0) before[nt][i][0] = at(nt, i)[0], before[nt][i][1] = at(nt, i)[kRowsTile + 1];
+                        else before[nt][i][0] = before[nt][i][1] = 0.f;
+                    }
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float p0, p1;
+                        unpair(acc[nt][m][i], p0, p1);
+                        at(nt, i)[0] = before[nt][i][0] + p0, at(nt, i)[kRowsTile + 1] = before[nt][i][1] + p1;
+                    }
+            }
+            clear();
+            ++part, part_end = runs * (part + 1) / kDenseWarps;
         }
-        if (__syncthreads_or(bad)) form_again<kTok, kRowsCta, kDenseWarps>(part[0], x, q, scale, minv, t0, n0, M, N, K, G, y);
+    };
+    close_parts(0);
+    for (int c0 = 0; c0 < runs; c0 += kRowsChunk) {
+        const int here = min(kRowsChunk, runs - c0);
+        __syncthreads();  // the chunk before has been read
+        // a warp has four tokens, whose 16-byte pieces it loads two tokens at a time, all in flight at once
+        const uint16_t *xc = x + (int64_t)c0 * kMmaRun;
+#pragma unroll
+        for (int j0 = 0; j0 < kRowsTok / kDenseWarps; j0 += 2) {
+            constexpr int kPieces = kRowsChunk * 4 / 32;
+            uint4 v[2][kPieces];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int m = 0; m < kPieces; ++m) {
+                    const int64_t t = t0 + warp * (kRowsTok / kDenseWarps) + j0 + j;
+                    v[j][m] = t < M && lane + 32 * m < here * 4 ? __ldg(reinterpret_cast<const uint4 *>(xc + t * K) + lane + 32 * m) : make_uint4(0u, 0u, 0u, 0u);
+                }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int m = 0; m < kPieces; ++m) {
+                    const int t = warp * (kRowsTok / kDenseWarps) + j0 + j, e = lane + 32 * m;
+                    acts[(((e >> 2) * NT + (t >> 3)) << 5) + ((t & 7) << 2) + (e & 3)] = v[j][m];
+                }
+        }
+        __syncthreads();
+        for (int i = warp; i < here * NT; i += kDenseWarps) {
+            const uint64_t sx = run_sums(acts[i * 32 + lane]);
+            if (g == 0) sums[i * 4 + c] = sx;
+        }
+        __syncthreads();
+        for (int r0 = c0; r0 < c0 + here; r0 += kAhead) {
+            if ((r0 >> lg_group) % 4 == 0 && (r0 & (per_group - 1)) == 0) {
+#pragma unroll
+                for (int i = 0; i < 2 * MT; ++i) sm[i] = ns[i] | (uint32_t)nm[i] << 16;
+                fetch_scales((r0 >> lg_group) + 4);
+            }
+#pragma unroll
+            for (int e = 0; e < kAhead; ++e) {
+                const int r = r0 + e;
+                if (r >= runs) break;
+                uint4 a[2 * MT];
+                float s[2 * MT], mn[2 * MT];
+#pragma unroll
+                for (int i = 0; i < 2 * MT; ++i) {
+                    const uint32_t p = __shfl_sync(0xffffffffu, sm[i], (lane & ~3) + ((r >> lg_group) & 3));
+                    s[i] = __uint_as_float(p << 16), mn[i] = __uint_as_float(p & 0xffff0000u);
+                    a[i] = w[i][e].bf16();
+                }
+                fetch(e, r + kAhead);
+#pragma unroll
+                for (int nt = 0; nt < NT; nt += kP) {
+                    uint4 xv[kP];
+                    uint64_t sx[kP];
+#pragma unroll
+                    for (int p = 0; p < kP; ++p) {
+                        const int at = (r - c0) * NT + nt + p;
+                        xv[p] = acts[at * 32 + lane], sx[p] = sums[at * 4 + c];
+                    }
+                    add_runs<kP, MT>(&acc[nt], a, s, mn, xv, sx);
+                }
+                close_parts(r + 1);
+            }
+        }
     }
+    __syncthreads();
+    bool bad = false;
+    static_assert(kRowsTile == 32 * kDenseWarps, "a thread has a weight row");
+    const int64_t n = n0 + threadIdx.x;
+#pragma unroll 8
+    for (int tt = 0; tt < kRowsTok; ++tt)
+        if (t0 + tt < M && n < N) {
+            const float sum = total[tt][threadIdx.x];
+            store_from_f32(y, (t0 + tt) * N + n, sum);
+            bad |= !isfinite(sum);
+        }
+    if (__syncthreads_or(bad)) form_again<kRowsTok, kRowsTile, kDenseWarps>(total, x, q, scale, minv, t0, n0, M, N, K, G, y);
 }
 
 }  // namespace
@@ -211,13 +403,28 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
 // x [M, K] BF16, y [M, N] BF16 or FP32; arguments checked by the caller.
 template <int BITS>
 int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st) {
+    auto xb = static_cast<const uint16_t *>(x);
+    // Two CTAs of dense_rows_kernel an SM: it is taken where its waves are at least three quarters full and the other form would take tokens by 32
+    // too.  As measured, us (dense_mma_kernel / this one):
+    // 128 CTAs 85.8 / 84.2, 160 37 / 50, 256 166 / 140 (1024 x 2048 x 4096), 320 205 / 214, 512 114 / 100.
+    const dim3 rows_grid((unsigned)((w->N + kRowsTile - 1) / kRowsTile), (unsigned)((M + kRowsTok - 1) / kRowsTok));
+    const int64_t rows_ctas = (int64_t)rows_grid.x * rows_grid.y, at_once = 2 * (int64_t)sm_count();
+    if (M >= 64 && rows_ctas * 4 >= (rows_ctas + at_once - 1) / at_once * at_once * 3) {
+        auto go_rows = [&](auto *yt) -> int {
+            auto kern = dense_rows_kernel<std::remove_pointer_t<decltype(yt)>>;
+            SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem), fn, ": reserving shared memory");
+            kern<<<rows_grid, 32 * kDenseWarps, kRowsSmem, st>>>(xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt);
+            SXB_CHECK_LAUNCH(fn, " BF16->", act_name(out_act), " M=", M, " N=", w->N, " K=", w->K, " G=", w->G);
+            return SXB_OK;
+        };
+        return out_act == SXB_ACT_F32 ? go_rows(static_cast<float *>(y)) : go_rows(static_cast<uint16_t *>(y));
+    }
     const int NT = token_eights(M);
     const int64_t token_groups = (M + NT * kMmaTokens - 1) / (NT * kMmaTokens);
     // 32 rows a CTA where that leaves every SM one: half the reading of activations, and as many CTAs as are resident at once
     // (8 x 8192 x 4096: 14.1 us, 16.7 with 16); with 32 tokens the registers are better spent on those
     const int MT = NT < 4 && (w->N + 31) / 32 * token_groups >= sm_count() ? 2 : 1;
-    const dim3 grid((unsigned)((w->N + kMmaRows * MT - 1) / (kMmaRows * MT)), (unsigned)std::min<int64_t>(token_groups, 65535));
-    auto xb = static_cast<const uint16_t *>(x);
+    const dim3 grid((unsigned)((w->N + kMmaRows * MT - 1) / (kMmaRows * MT)), (unsigned)token_groups);  // at most 16384: 524280 rows of x, 32 a CTA
     auto go = [&](auto *yt) {
         using T = std::remove_pointer_t<decltype(yt)>;
 #define SXB_DENSE(MTV, NTV) dense_mma_kernel<BITS, MTV, NTV, T><<<grid, 32 * kDenseWarps, 0, st>>>(xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt)

@@ -25,6 +25,29 @@ __device__ inline void mma_run(float (&d)[4], const uint4 &a, const uint4 &b, co
     mma_bf16(d, a.z, b.z, a.w, b.w, x.z, x.w);
 }
 
+// Pairs of FP32 values in one instruction, each rounded as on its own.
+__device__ inline uint64_t pair(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ inline void unpair(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ inline uint64_t mul_pair(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ inline uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ inline uint64_t add_pair(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Two FP32 values that fit BF16 as a pair (the first in the lower half).
 __device__ inline uint32_t pack_bf16_exact(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
 // The upper sixteen bits of an FP32 value: a BF16, and what is left of the value is an FP32 with eight bits fewer.
@@ -72,21 +95,18 @@ __device__ inline float group_zero(uint32_t word) { return __uint_as_float((word
 template <int BITS>
 __device__ inline uint4 codes_bf16(uint32_t w0, uint32_t w1, float zero) {
     uint32_t r[4];
-    if (BITS == 8) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t w = i < 2 ? w0 : w1;  // 2^23 + code, less `zero`: no conversion instruction, which runs at a quarter rate
-            const float lo = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7442 : 0x7440)) - zero;
-            const float hi = __uint_as_float(__byte_perm(w, 0x4B000000u, (i & 1) ? 0x7443 : 0x7441)) - zero;
-            r[i] = pack_bf16_exact(lo, hi);
+    for (int i = 0; i < 4; ++i) {
+        uint32_t lo, hi;  // 2^23 + code, less `zero`: no conversion instruction, which runs at a quarter rate
+        if (BITS == 8) {
+            const uint32_t w = i < 2 ? w0 : w1;
+            lo = __byte_perm(w, 0x4B000000u, (i & 1) ? 0x7442 : 0x7440), hi = __byte_perm(w, 0x4B000000u, (i & 1) ? 0x7443 : 0x7441);
+        } else {
+            lo = 0x4B000000u | ((w0 >> (8 * i)) & 15u), hi = 0x4B000000u | ((w0 >> (8 * i + 4)) & 15u);
         }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float lo = __uint_as_float(0x4B000000u | ((w0 >> (8 * i)) & 15u)) - zero;
-            const float hi = __uint_as_float(0x4B000000u | ((w0 >> (8 * i + 4)) & 15u)) - zero;
-            r[i] = pack_bf16_exact(lo, hi);
-        }
+        float a, b;
+        unpair(add_pair(pair(__uint_as_float(lo), __uint_as_float(hi)), pair(-zero, -zero)), a, b);
+        r[i] = pack_bf16_exact(a, b);
     }
     return make_uint4(r[0], r[1], r[2], r[3]);
 }

@@ -118,6 +118,27 @@ def test_linear_q8_edges(cuda, oracle, G, M, N, Kd):
     assert np.all(np.abs(y.cpu().numpy().astype(np.float64) - want) <= bound)
 
 
+@pytest.mark.parametrize("G,M,N,Kd", [(32, 2369, 513, 32), (32, 370, 4737, 288), (64, 2400, 700, 576), (128, 214, 8200, 1152), (32, 7200, 31, 96)])
+def test_linear_q8_many_rows(cuda, oracle, G, M, N, Kd):
+    """The Q8 dense form for many rows of x: tokens past a tile of 32, weight rows past 32 and 256, fewer runs than parts, parts of unequal
+    length, more runs than lie in shared memory at once.  Row by row the bits of a call of one row - NaN, infinities and products past FP32's range among them - and in
+    BF16 the rounded values."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(M + N + Kd)
+    x = torch.from_numpy(rng.standard_normal((M, Kd)).astype(np.float32)).to(cuda).to(torch.bfloat16)
+    x[M - 2] = torch.where(torch.arange(Kd, device=cuda) % 2 > 0, 1.0, -1.0) * 2.0 ** 124
+    x[3, 5], x[M // 2, Kd - 1] = float("nan"), float("inf")
+    w = upload(oracle.quantize(random_weights(rng, N, Kd), G, 8), cuda)
+    y, yb = (torch.empty((M, N), dtype=t, device=cuda) for t in (torch.float32, torch.bfloat16))
+    K.linear_qw(x, w, y, M, K.Act.BF16, out_act=K.Act.F32)
+    K.linear_qw(x, w, yb, M, K.Act.BF16)
+    one = torch.empty((1, N), dtype=torch.float32, device=cuda)
+    for t in sorted({0, 3, 31, 32, M // 2, M - 2, M - 1} | set(rng.integers(0, M, 12).tolist())):
+        K.linear_qw(x[t:t + 1].clone(), w, one, 1, K.Act.BF16, out_act=K.Act.F32)
+        assert torch.equal(one[0].view(torch.int32), y[t].view(torch.int32)), t
+    assert torch.equal(yb.nan_to_num(), y.to(torch.bfloat16).nan_to_num()) and torch.equal(yb.isnan(), y.isnan())
+
+
 @pytest.mark.parametrize("far", [28, 31, 40, 80])
 @pytest.mark.parametrize("bits,G,Kd", [(8, 64, 1024), (8, 128, 384), (8, 32, 160)])
 def test_large_activation_against_zero_weights(cuda, oracle, bits, G, Kd, far):
