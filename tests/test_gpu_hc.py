@@ -161,6 +161,50 @@ def test_hc_mix_large_value_against_zero_weights(cuda, oracle, dt, bits, zero, f
     assert np.all(np.abs(u.float().cpu().numpy() - u_ref) <= bound)
 
 
+@pytest.mark.parametrize("bits,T,d,r", [(8, 1, 64, 64), (8, 17, 256, 320), (4, 33, 128, 96)])
+def test_hc_mix_third_plane(cuda, oracle, bits, T, d, r):
+    """FP32 streams, and an FP32 h, whose last bits are all that is left of a dot: pairs 1 + 2^-8 + k 2^-23 and -(1 + 2^-8) against equal
+    weights, 1 to 12 times a power of two.  With two BF16 planes (16 bits) of the pairs, every dot is zero.  Bound: the products of an MMA are
+    added at its largest one's exponent, at most 3, 24 bits deep; two MMAs of 16 for each of three planes, 96 2^-21 = 5e-5 where a run of 32
+    keeps 16 x 64 x 6 2^-23 = 7e-4 in the mean: an eighth of the dot."""
+    from strixite_b200 import kernels as K
+    H, eps, G = 4, 1e-6, 32
+    rng = np.random.default_rng(T + d + r)
+
+    def pairs(rows, cols):
+        v = np.empty((rows, cols), dtype=np.float32)
+        v[:, 0::2] = 1 + 2.0 ** -8 + rng.integers(1, 128, (rows, cols // 2)) * 2.0 ** -23
+        v[:, 1::2] = -(1 + 2.0 ** -8)
+        return v
+
+    def weight(rows, cols, scale):
+        w = oracle.quantize(random_weights(rng, rows, cols), G, bits)
+        codes = np.repeat(rng.integers(4, 16, (rows, cols // 2)), 2, axis=1).astype(np.uint8)
+        w.q[:] = codes if bits == 8 else codes[:, 0::2] | (codes[:, 1::2] << 4)
+        w.scale[:], w.minv[:] = oracle.f32_to_bf16(np.float32([scale]))[0], oracle.f32_to_bf16(np.float32([-3 * scale]))[0]
+        return w
+
+    def cut(v):
+        return (v.view(np.uint32) & 0xFFFFFF00).view(np.float32)
+
+    wd, wu, x, hn = weight(r + H, H * d, 2.0 ** -4), weight(H * d, r, 2.0 ** 7), pairs(T, H * d), pairs(T, r)
+    assert not np.any(cut(x).astype(np.float64) @ oracle.affine_weights(wd).T) and not np.any(cut(hn).astype(np.float64) @ oracle.affine_weights(wu).T)
+    xd = torch.from_numpy(x).to(cuda)
+    h, w_in, inv = (torch.full((T, n), float("nan"), dtype=torch.float32, device=cuda) for n in (r, H, H))
+    K.hc_mix_down(xd, upload(wd, cuda), T, H, d, r, True, eps, h, w_in, inv, K.Act.F32)
+    h_ref, _, inv_ref = oracle.hc_mix_down(x, wd, H, d, r, True, eps)
+    assert np.all(h_ref > 0) and np.all(np.abs(h.cpu().numpy() - h_ref) <= h_ref / 8)
+    ones = torch.ones((T, H), dtype=torch.float32, device=cuda)
+    xs, nw, u = torch.rand((T, H * d), device=cuda) + 0.5, torch.zeros(H * d, device=cuda), torch.empty((T, d), device=cuda)
+    K.hc_mix_up(torch.from_numpy(hn).to(cuda), K.to_chunk_major(upload(wu, cuda)), xs, nw, ones, T, H, d, u, K.Act.F32)
+    u_ref = oracle.hc_mix_up(hn, wu, xs.cpu().numpy(), np.zeros(H * d, dtype=np.float32), np.ones((T, H), dtype=np.float32), H, d)
+    z = hn.astype(np.float64) @ oracle.affine_weights(wu).T  # sigmoid' <= 1/4
+    xn = xs.double().cpu().numpy()
+    bound = (xn * (np.abs(z) / 32 + 2.0 ** -20)).reshape(T, H, d).sum(axis=1) / H
+    assert np.all(np.abs(u.cpu().numpy() - u_ref) <= bound)
+    assert np.all(np.abs(xn.reshape(T, H, d).sum(axis=1) / (2 * H) - u_ref) > bound)  # what dots of zero would give
+
+
 def test_hc_mix_argument_checks(cuda, oracle):
     from strixite_b200 import kernels as K
     rng = np.random.default_rng(1)

@@ -83,6 +83,24 @@ def test_router_logits_streaming_edges(cuda, oracle, M, N, K, w_bf16):
     assert np.array_equal(got2[bad], want2[bad], equal_nan=True) and np.array_equal(got2[~bad], out.cpu().numpy()[~bad])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 17, 64), (16, 513, 4096), (37, 33, 1000)])
+def test_router_logits_streaming_third_plane(cuda, oracle, M, N, K):
+    """FP32 weights whose last bits are all that is left of a logit: pairs 1 + 2^-8 + k 2^-23 and -(1 + 2^-8) against the same activation, a
+    small whole number, so that every sum is exact in FP32 whatever its order.  The logits are the 64-bit ones, bit for bit; cut to two
+    BF16 planes (16 bits) the weights give zeros."""
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(M + N)
+    w = np.empty((N, K), dtype=np.float32)
+    w[:, 0::2] = 1 + 2.0 ** -8 + rng.integers(1, 128, (N, K // 2)) * 2.0 ** -23
+    w[:, 1::2] = -(1 + 2.0 ** -8)
+    x = np.repeat(rng.integers(-3, 4, (M, K // 2)), 2, axis=1).astype(np.float32)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    assert not np.any(x.astype(np.float64) @ (w.view(np.uint32) & 0xFFFFFF00).view(np.float32).astype(np.float64).T)
+    out = torch.empty((M, N), dtype=torch.float32, device=cuda)
+    Kn.router_logits(torch.from_numpy(x).to(cuda).to(torch.bfloat16), torch.from_numpy(w).to(cuda), None, out)
+    assert np.any(want) and np.array_equal(out.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("form", ["dense", "router"])
 def test_non_finite_rows(cuda, oracle, form):
     """NaN and infinities in some tokens' activations and, for the router, weights: the results are what 64 bits give, and the other
