@@ -10,8 +10,8 @@
 // What bounds it: for few tokens a launch, the round trips to memory and the parts' meeting; for more the code conversions, once per
 // 32 tokens, and the activations' way through L1, once per 16 rows; for many rows of x see dense_rows_kernel.  The form before it (stream_mma.cu,
 // which keeps Q4) staged a tile of 8 tokens as scaled F16 in every CTA and converted every code again for the next 8.  As CUDA graphs on weights that lie in L2,
-// us before -> now: 2048 x 4096, 1 / 16 / 40 / 300 tokens 9.6 -> 6.4, 12.2 -> 7.7, 21.7 -> 15.3, 70 -> 55; 4096 x 1024 7.4 -> 4.0, 8.3 -> 4.7, 13.7 -> 8.6,
-// 35.5 -> 37.2; 8192 x 4096, 8 / 63 / 300 tokens 16.5 -> 12.7, 56.7 -> 45.0, 205 -> 205; weights from HBM 8 tokens 24.6 -> 20.4, 63 67.6 -> 55.3.
+// us before -> now: 2048 x 4096, 1 / 16 / 40 / 300 tokens 9.6 -> 6.4, 12.2 -> 7.7, 21.8 -> 15.1, 70 -> 55; 4096 x 1024 7.4 -> 4.1, 8.2 -> 4.7, 13.6 -> 8.4,
+// 35.4 -> 36.0; 8192 x 4096, 8 / 63 / 300 tokens 16.4 -> 12.6, 56.8 -> 44.5, 205 -> 202; weights from HBM, 8 tokens 24.6 -> 20.5, 63 67.6 -> 55.3.
 // Error against 64 bits (2-norms) 1.15e-7 .. 2.3e-7 -> 0.95e-7 .. 1.2e-7.  Q4, whose nibbles take more instructions to BF16 than to F16,
 // was slower this way (8192 x 4096, 8 tokens: 13 -> 17) and stays there.
 
@@ -25,6 +25,9 @@ namespace sxb {
 namespace {
 
 constexpr int kDenseWarps = 8;
+// Sums in shared memory lie [token][weight row], rows of four more: a fragment's lanes (tokens 2 c, rows g) meet every bank once, with one more
+// four lanes met in one (dense_rows_kernel, 4096 x 4096 x 1024: 332 us, now 261).
+constexpr int kPad = 4;
 
 // What a token with one or more results that are not finite holds: infinities, NaN, or neither.
 constexpr uint32_t kHoldsInf = 1u, kHoldsNan = 2u;
@@ -79,13 +82,13 @@ __device__ __noinline__ float wide_dot(const uint16_t *x, const uint8_t *q, cons
     return (float)sum;
 }
 
-// The results of a CTA's tile - sums [tokens][rows + 1] of tokens t0 .., weight rows n0 .. - that are not finite, formed again by all of its WARPS
+// The results of a CTA's tile - sums [tokens][rows] of tokens t0 .., weight rows n0 .. - that are not finite, formed again by all of its WARPS
 // and stored: each token's activations are looked at once (a NaN among them: every result is NaN, as it is), then the warps share the
 // weight rows.
 // One thread walking the contraction for each such result, as it stood here before: 8 x 8192 x 4096 with a NaN or an infinity in one token 922 us,
 // now 20 and 34; NaN in all tokens 3270, now 22; 128 rows with an infinity each 23500, now 1790; 16 and 88 us without.
 template <int TOKENS, int ROWS, int WARPS, typename TOUT>
-__device__ __noinline__ void form_again(const float (&sums)[TOKENS][ROWS + 1], const uint16_t *x, const uint8_t *q, const uint16_t *scale,
+__device__ __noinline__ void form_again(const float (&sums)[TOKENS][ROWS + kPad], const uint16_t *x, const uint8_t *q, const uint16_t *scale,
                                         const uint16_t *minv, int64_t t0, int64_t n0, int64_t M, int64_t N, int64_t K, int64_t G, TOUT *y) {
     __shared__ uint32_t holds[TOKENS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     constexpr int kAhead = MT == 2 || NT == 4 ? 4 : 8;           // runs whose codes a lane has in flight
     constexpr int kActs = NT == 4 ? 1 : (NT == 2 ? 2 : 4) / MT;  // ... whose activations
     constexpr int kRunBytes = kMmaRun * BITS / 8;
-    __shared__ float part[kDenseWarps][kTok][kRowsCta + 1];
+    __shared__ float part[kDenseWarps][kTok][kRowsCta + kPad];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
     const int64_t n0 = (int64_t)blockIdx.x * kRowsCta, row_bytes = K * BITS / 8, groups = K / G;
     const int runs = (int)(K / kMmaRun), lo = runs * warp / kDenseWarps, hi = runs * (warp + 1) / kDenseWarps, per_group = (int)(G / kMmaRun);
@@ -238,14 +241,14 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
 // activations of 1024 k at a time lie in shared memory in fragment order with the sums of their runs, formed once for all rows; a warp's codes
 // come straight from memory, four runs ahead, and nothing is waited for in between.
 //
-// What bounds it: the L1 pipe, at 75 % (codes 32 of a run's 100 wavefronts, activations 16, scales), and the latencies between MMAs and sums with
-// four warps a scheduler (issue slots 48 %).  dense_mma_kernel reads the activations again for every 16 rows and converts a code for 32 tokens
-// as this does.  us, that -> this: 1024 x 8192 x 4096 648 -> 481, 4096 rows 2580 -> 1879, 4096 x 2048 x 4096 650 -> 480, 4096 x 4096 x 1024 447 -> 332
-// (eight parts of four runs each: closing them, and the start of a CTA, are a third; the form before these, stream_mma.cu, takes 292).  Activations copied 64 k at a time by cp.async with a barrier
-// a block: 1024 x 8192 x 4096 583.
+// What bounds it: the L1 pipe, at four fifths (codes 32 of a run's 90 wavefronts - eight rows, eight lines a load -, activations 16, scales), and the
+// latencies between MMAs and sums with four warps a scheduler (issue slots 50 %).  dense_mma_kernel reads the activations again for every 16
+// rows and converts a code for 32 tokens as this does.  us, that -> this: 1024 x 8192 x 4096 648 -> 443, 4096 rows 2580 -> 1726, 4096 x 2048 x 4096
+// 650 -> 443, 4096 x 4096 x 1024 447 -> 261; the form before these (stream_mma.cu) takes 593, 2390, 621 and 291.  Activations copied 64 k at
+// a time by cp.async with a barrier a block: 1024 x 8192 x 4096 583.
 constexpr int kRowsMT = 2, kRowsNT = 4;  // of a warp
 constexpr int kRowsTile = kDenseWarps * kMmaRows * kRowsMT, kRowsTok = kMmaTokens * kRowsNT, kRowsChunk = 32;  // weight rows, tokens; runs in shared memory
-constexpr size_t kRowsSmem = (size_t)kRowsChunk * kRowsTok * (kMmaRun * 2 + sizeof(float)) + (size_t)kRowsTok * (kRowsTile + 1) * sizeof(float);
+constexpr size_t kRowsSmem = (size_t)kRowsChunk * kRowsTok * (kMmaRun * 2 + sizeof(float)) + (size_t)kRowsTok * (kRowsTile + kPad) * sizeof(float);
 
 template <typename TOUT>
 __global__ void __launch_bounds__(32 * kDenseWarps, 2)
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     extern __shared__ __align__(16) unsigned char rows_smem[];
     uint4 *acts = reinterpret_cast<uint4 *>(rows_smem);                           // [run][nt][lane]
     uint64_t *sums = reinterpret_cast<uint64_t *>(acts + kRowsChunk * NT * 32);   // [run][nt][c]: of tokens 2 c and 2 c + 1
-    using Total = float[kRowsTok][kRowsTile + 1];
+    using Total = float[kRowsTok][kRowsTile + kPad];
     Total &total = *reinterpret_cast<Total *>(sums + kRowsChunk * NT * 4);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, wr = kMmaRows * MT * warp;
     const int64_t n0 = (int64_t)blockIdx.x * kRowsTile, t0 = (int64_t)blockIdx.y * kRowsTok, groups = K / G;
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
                 for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
-                        if (part > 0) before[nt][i][0] = at(nt, i)[0], before[nt][i][1] = at(nt, i)[kRowsTile + 1];
+                        if (part > 0) before[nt][i][0] = at(nt, i)[0], before[nt][i][1] = at(nt, i)[kRowsTile + kPad];
                         else before[nt][i][0] = before[nt][i][1] = 0.f;
                     }
 #pragma unroll
@@ -312,7 +315,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
                     for (int i = 0; i < 2; ++i) {
                         float p0, p1;
                         unpair(acc[nt][m][i], p0, p1);
-                        at(nt, i)[0] = before[nt][i][0] + p0, at(nt, i)[kRowsTile + 1] = before[nt][i][1] + p1;
+                        at(nt, i)[0] = before[nt][i][0] + p0, at(nt, i)[kRowsTile + kPad] = before[nt][i][1] + p1;
                     }
             }
             clear();
@@ -405,8 +408,8 @@ template <int BITS>
 int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st) {
     auto xb = static_cast<const uint16_t *>(x);
     // Two CTAs of dense_rows_kernel an SM: it is taken where its waves are at least three quarters full and the other form would take tokens by 32
-    // too.  As measured, us (dense_mma_kernel / this one):
-    // 128 CTAs 85.8 / 84.2, 160 37 / 50, 256 166 / 140 (1024 x 2048 x 4096), 320 205 / 214, 512 114 / 100.
+    // too.  As measured, us (dense_mma_kernel / this one): 80 CTAs 55 / 84 (300 x 2048 x 4096), 160 37 / 50 (300 x 4096 x 1024), 256 166 / 130
+    // (1024 x 2048 x 4096), 320 205 / 214, 512 114 / 78 (1024 x 4096 x 1024).
     const dim3 rows_grid((unsigned)((w->N + kRowsTile - 1) / kRowsTile), (unsigned)((M + kRowsTok - 1) / kRowsTok));
     const int64_t rows_ctas = (int64_t)rows_grid.x * rows_grid.y, at_once = 2 * (int64_t)sm_count();
     if (M >= 64 && rows_ctas * 4 >= (rows_ctas + at_once - 1) / at_once * at_once * 3) {
