@@ -143,17 +143,16 @@ __device__ inline void add_runs(uint64_t (*acc)[MT][2], const uint4 (&a)[2 * MT]
             }
 }
 
-template <int BITS, int MT, int NT, typename TOUT>
+template <int MT, int NT, typename TOUT>
 __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     dense_mma_kernel(const uint16_t *__restrict__ x, const uint8_t *__restrict__ q, const uint16_t *__restrict__ scale,
                      const uint16_t *__restrict__ minv, int64_t M, int64_t N, int64_t K, int64_t G, TOUT *__restrict__ y) {
     constexpr int kTok = kMmaTokens * NT, kRowsCta = kMmaRows * MT;
     constexpr int kAhead = MT == 2 || NT == 4 ? 4 : 8;           // runs whose codes a lane has in flight
     constexpr int kActs = NT == 4 ? 1 : (NT == 2 ? 2 : 4) / MT;  // ... whose activations
-    constexpr int kRunBytes = kMmaRun * BITS / 8;
     __shared__ float part[kDenseWarps][kTok][kRowsCta + kPad];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-    const int64_t n0 = (int64_t)blockIdx.x * kRowsCta, row_bytes = K * BITS / 8, groups = K / G;
+    const int64_t n0 = (int64_t)blockIdx.x * kRowsCta, groups = K / G;
     const int runs = (int)(K / kMmaRun), lo = runs * warp / kDenseWarps, hi = runs * (warp + 1) / kDenseWarps, per_group = (int)(G / kMmaRun);
     int64_t row[2 * MT];  // rows past the end stream the last one; their sums are dropped
 #pragma unroll
@@ -165,13 +164,13 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) acc[nt][m][0] = acc[nt][m][1] = 0;
     for (int r0 = lo; r0 < hi; r0 += kAhead) {
-        Codes<BITS> w[2 * MT][kAhead];
+        Codes<8> w[2 * MT][kAhead];
         uint32_t sm[2 * MT][kAhead / 4];  // (scale, min) for run r0 + 4 i + c: handed round by shuffles
 #pragma unroll
         for (int e = 0; e < kAhead; ++e) {
             const int64_t r = min(r0 + e, hi - 1);
 #pragma unroll
-            for (int i = 0; i < 2 * MT; ++i) w[i][e].load(q + row[i] * row_bytes + r * kRunBytes + c * BITS);
+            for (int i = 0; i < 2 * MT; ++i) w[i][e].load(q + row[i] * K + r * kMmaRun + 8 * c);
         }
 #pragma unroll
         for (int e = 0; e < kAhead / 4; ++e) {
@@ -404,8 +403,7 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
 }  // namespace
 
 // x [M, K] BF16, y [M, N] BF16 or FP32; arguments checked by the caller.
-template <int BITS>
-int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st) {
+int dense_q8(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st) {
     auto xb = static_cast<const uint16_t *>(x);
     // Two CTAs of dense_rows_kernel an SM: it is taken where its waves are at least three quarters full and the other form would take tokens by 32
     // too.  As measured, us (dense_mma_kernel / this one): 80 CTAs 55 / 84 (300 x 2048 x 4096), 160 37 / 50 (300 x 4096 x 1024), 256 166 / 130
@@ -430,7 +428,7 @@ int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t
     const dim3 grid((unsigned)((w->N + kMmaRows * MT - 1) / (kMmaRows * MT)), (unsigned)token_groups);  // at most 16384: 524280 rows of x, 32 a CTA
     auto go = [&](auto *yt) {
         using T = std::remove_pointer_t<decltype(yt)>;
-#define SXB_DENSE(MTV, NTV) dense_mma_kernel<BITS, MTV, NTV, T><<<grid, 32 * kDenseWarps, 0, st>>>(xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt)
+#define SXB_DENSE(MTV, NTV) dense_mma_kernel<MTV, NTV, T><<<grid, 32 * kDenseWarps, 0, st>>>(xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt)
         if (NT == 4) SXB_DENSE(1, 4);
         else if (NT == 2 && MT == 1) SXB_DENSE(1, 2);
         else if (NT == 2) SXB_DENSE(2, 2);
@@ -443,7 +441,5 @@ int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t
     SXB_CHECK_LAUNCH(fn, " BF16->", act_name(out_act), " M=", M, " N=", w->N, " K=", w->K, " G=", w->G);
     return SXB_OK;
 }
-
-template int dense_mma<8>(const char *, const void *, const SxbQView *, void *, int64_t, int, cudaStream_t);
 
 }  // namespace sxb

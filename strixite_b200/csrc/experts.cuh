@@ -27,8 +27,7 @@ int stream_combine_slots(const char *fn, const void *h, const SxbQView *w, int64
                          const float *coef, int64_t M, int64_t A, void *y, int act, int out_act, uint32_t *err,
                          sxb_stream_t stream);
 // dense_mma.cu - dense projections of Q8 weights with exact products, any M.
-template <int BITS>
-int dense_mma(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st);
+int dense_q8(const char *fn, const void *x, const SxbQView *w, void *y, int64_t M, int out_act, cudaStream_t st);
 int combine_reduce(const char *fn, const float *partial, const int32_t *ids, const float *coef, int64_t M, int64_t A,
                    int64_t E_total, int64_t e_lo, int64_t E_local, int64_t N, void *y, int out_act,
                    const SxbMoeSharedAdd *shared, int s_act, bool partial_bf16, sxb_stream_t stream,

@@ -16,7 +16,7 @@
 //     the loop around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps
 //     that showed it, which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 540 us at 777
 //     tokens, 789 -> 728 at 4096, dense 1001 x 8192 x 4096 64.7 -> 57.1, 4000 tokens Q8 232 -> 216.
-//   * A commit and the next stage's wait cost ~250 whatever lies between: steps of 128 k, eight MMAs.
+//   * Steps of 128 k, eight MMAs a commit: with the loop of one lane a commit and the next stage's wait cost ~250 cycles whatever lay between.
 //   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 162 instructions a warp and step, not 290.
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
@@ -156,16 +156,12 @@ __device__ inline void load_groups(uint32_t (&v)[Scales<N>::kWords], const uint1
         v[0] = u.x, v[1] = u.y;
     }
 }
-// The same one by one: rows that N does not divide, or that do not start on a vector's boundary.
+// The same one by one: arrays that do not start on a vector's boundary.
 template <int N>
-__device__ __noinline__ Scales<N> load_scales_each(const uint16_t *sp, const uint16_t *mp, int n) {
+__device__ __noinline__ Scales<N> load_scales_each(const uint16_t *sp, const uint16_t *mp) {
     Scales<N> c{};
-    for (int i = 0; i < N; ++i)
-        if (i < n) {
 #pragma unroll
-            for (int w = 0; w < Scales<N>::kWords; ++w)
-                if (w == i >> 1) c.s[w] |= (uint32_t)__ldg(sp + i) << (16 * (i & 1)), c.m[w] |= (uint32_t)__ldg(mp + i) << (16 * (i & 1));
-        }
+    for (int i = 0; i < N; ++i) c.s[i >> 1] |= (uint32_t)__ldg(sp + i) << (16 * (i & 1)), c.m[i >> 1] |= (uint32_t)__ldg(mp + i) << (16 * (i & 1));
     return c;
 }
 
@@ -301,8 +297,8 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         constexpr int kRowBytes = kBK * BITS / 8;    // of a row of a ring slot: 64 or 128
         constexpr int kCodeRegs = kBK * BITS / 128;  // 16-byte chunks of codes per row and step
         constexpr int kWordsPerChunk = BITS == 4 ? 4 : 2;  // runs of eight codes in one of them
-        const bool vec_scales = groups % kGroups == 0 &&
-                                ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & (2 * kGroups - 1)) == 0;
+        // K is a multiple of 128 and so a row's groups of a step's: where the arrays start decides
+        const bool vec_scales = ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & (2 * kGroups - 1)) == 0;
         // this thread's row inside the first slot; its chunks are swizzled (128-byte mode, 64-byte for rows of 64 bytes), so that chunk c
         // lies at my_w ^ 16 c
         const uint32_t my_w = w_base + (uint32_t)(srow * kRowBytes) + (uint32_t)(kRowBytes == 64 ? (srow >> 1) & 3 : srow & 7) * 16u;
@@ -316,7 +312,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
             if (wrow < 0) return c;
             const int64_t at = (int64_t)wrow * groups + step * kGroups;
             if (vec_scales) load_groups<kGroups>(c.s, a.scale + at), load_groups<kGroups>(c.m, a.minv + at);
-            else c = load_scales_each<kGroups>(a.scale + at, a.minv + at, groups - step * kGroups);
+            else c = load_scales_each<kGroups>(a.scale + at, a.minv + at);
             return c;
         };
         uint32_t free_phase = 1u;  // parity of the phase that leaves the stage to the set's next step: there is none before the first

@@ -368,8 +368,10 @@ int mix_down(const void *x, const SxbQView *w, int64_t T, int64_t H, int64_t d, 
     SXB_CHECK(aligned16(x), fn, ": x ", x, " must be 16-byte aligned");
     SXB_CHECK(std::isfinite(eps) && eps > 0.f, fn, ": eps must be finite and > 0, got ", eps);
     SXB_CHECK((w->K / kChunk) % kParts == 0, fn, ": H*d = ", w->K, " must be a multiple of ", kChunk * kParts, " (eight parts of whole chunks a row)");
-    const size_t per_token = (size_t)w->K * act_bytes(act) + (size_t)(w->K / kChunk) * 8;  // the limit of a row of streams, 200 KB
-    SXB_CHECK(per_token + 4352 <= 200 * 1024, fn, ": H*d = ", w->K, " needs ", per_token, " bytes a token, limit ", 200 * 1024 - 4352);
+    // The longest row of streams is part of the interface (a token's streams and its chunks' sums in 196 KB); the kernel itself would take a longer one.
+    const size_t per_token = (size_t)w->K * act_bytes(act) + (size_t)(w->K / kChunk) * 8;
+    SXB_CHECK(per_token <= 200 * 1024 - 4352, fn, ": H*d = ", w->K, " is longer than the mix takes (", act_name(act), ": at most ",
+              (200 * 1024 - 4352) / (4 * act_bytes(act) + 1) * 4 / (kChunk * kParts) * (kChunk * kParts), ")");
     const int NT = act == SXB_ACT_F32 ? std::min(2, token_eights(T)) : token_eights(T);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};

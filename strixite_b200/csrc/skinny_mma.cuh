@@ -126,8 +126,9 @@ struct Codes {
     __device__ inline uint4 bf16(float zero = kCodeBias) const { return codes_bf16<BITS>(w[0], w[BITS / 4 - 1], zero); }
 };
 
-// Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Four where the last 32 are more than half
-// full (the hyper-connection mix of 63 tokens, d = 4096 Q8: 41 us, 45 with two; of 40 tokens: 39 and 32).
+// Eights of tokens a CTA takes, 1, 2 or 4; the weights of a second group of tokens come from L2.  Two for 9 to 16 tokens, and below 64 where the last
+// 32 would be at most half full (the hyper-connection mix of 40 tokens, d = 4096 Q8: 32 us, 39 with four; of 63 tokens: 45 and 41); from 64
+// tokens on a group that is not full weighs little.
 inline int token_eights(int64_t T) { return T <= 8 ? 1 : T <= 16 || (T < 64 && (T - 1) % 32 < 16) ? 2 : 4; }
 
 // ---- the CTAs of a cluster -------------------------------------------------------------------------------------------

@@ -930,7 +930,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
              ": reserving shared memory");
     // A dense projection of few units for the machine's warps: up to eight warps share one, as long as that gives a warp at most two and a half
     // parts in turn.  A warp alone walks K / (4 * kStepCodes) blocks one after another, each a round trip to memory (2048 x 4096
-    // Q8, one token: 28 us with 128 warps at work, 13.5 with eight warps a unit).
+    // Q4, one token: 16.4 us with 128 warps at work, 9.1 with eight warps a unit).
     const int64_t machine_warps = (int64_t)sm_count() * (kBigThreads / 32);
     StreamArgs args = a;
     args.chunks = SRC == kDense && geo::kStepsPerGroup == 1 && vector_scales(a, G) ? chunk_count(steps / kPrefetch) : 1, args.split = 1;
@@ -945,7 +945,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     const bool big = est_units >= machine_warps * 2;
     const int threads = big ? kBigThreads : kThreads, warps = threads / 32;
     // Two fit an SM's 228 KB with 1 KB of the system's and their static shared memory each, 25 KB in the dense form (with 100 KB as
-    // the line there too, 110 x 4096 x 5760 Q8 ran as two waves of one CTA an SM: 188 us, now 153; 100 x 4096 x 6144 Q4 84, now 50).
+    // the line there too, 100 x 4096 x 6144 Q4 ran as two waves of one CTA an SM: 84 us, now 50).
     const int per_sm = big || smem > (SRC == kDense ? 88 : 100) * 1024 ? 1 : 2;
     int64_t grid = (int64_t)sm_count() * per_sm;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (est_units + warps - 1) / warps));
@@ -987,11 +987,12 @@ int linear_impl(const char *fn, const void *x, const SxbQView *w, void *y, int64
     SXB_CHECK(apart(x, M * w->K * 2, y, M * w->N * act_bytes(out_act)), fn, ": output y [", y, ", +",
               M * w->N * act_bytes(out_act), " B) overlaps input x [", x, ", +", M * w->K * 2, " B)");
     if constexpr (BITS == 8) {
-        // the longest row: what a tile of eight tokens of one takes of shared memory in the routed forms of the same projection
-        const int64_t smem = w->K * 16 + w->K / std::min<int64_t>(64, w->G) * kTileTokens * 4;
-        SXB_CHECK(smem <= (int64_t)kMaxDynSmem, fn, ": K = ", w->K, " needs ", smem, " bytes of shared memory for one tile's activations, more than ",
-                  kMaxDynSmem, " (K * 16)");
-        return dense_mma<BITS>(fn, x, w, y, M, out_act, static_cast<cudaStream_t>(stream));
+        // The longest row is part of the interface, the same as in the routed forms of the projection, whose tile of eight tokens it comes from;
+        // this kernel itself would take a longer one.
+        const int64_t tile_bytes = w->K * 16 + w->K / std::min<int64_t>(64, w->G) * kTileTokens * 4;
+        SXB_CHECK(tile_bytes <= (int64_t)kMaxDynSmem, fn, ": K = ", w->K, " is longer than the exact-product projections take (G = ", w->G,
+                  ": at most ", (int64_t)kMaxDynSmem / (w->G == 32 ? 34 : 33) * 2 / w->G * w->G, ")");
+        return dense_q8(fn, x, w, y, M, out_act, static_cast<cudaStream_t>(stream));
     } else {
         StreamArgs a{};
         a.x = static_cast<const uint16_t *>(x), a.q = w->q, a.scale = w->scale, a.minv = w->minv;
