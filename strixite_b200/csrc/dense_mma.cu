@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(32 * kDenseWarps, 2)
 // activations of 1024 k at a time lie in shared memory in fragment order with the sums of their runs, formed once for all rows; a warp's codes
 // come straight from memory, four runs ahead, and nothing is waited for in between.
 //
-// What bounds it: the L1 pipe, at four fifths (codes 32 of a run's 90 wavefronts - eight rows, eight lines a load -, activations 16, scales), and the
-// latencies between MMAs and sums with four warps a scheduler (issue slots 50 %).  dense_mma_kernel reads the activations again for every 16
+// What bounds it: the L1 pipe, at 79 % (codes 32 of a run's 90 wavefronts - eight rows, eight lines a load -, activations 16, scales), and the
+// latencies between MMAs and sums with four warps a scheduler (issue slots 54 %, tensor pipe 30).  dense_mma_kernel reads the activations again for every 16
 // rows and converts a code for 32 tokens as this does.  us, that -> this: 1024 x 8192 x 4096 648 -> 443, 4096 rows 2580 -> 1726, 4096 x 2048 x 4096
 // 650 -> 443, 4096 x 4096 x 1024 447 -> 261; the form before these (stream_mma.cu) takes 593, 2390, 621 and 291.  Activations copied 64 k at
 // a time by cp.async with a barrier a block: 1024 x 8192 x 4096 583.

@@ -10,9 +10,10 @@
 // Both are small-matrix, many-launch kernels (a few MB of weights, ~97 mixes per decoded token upstream): what bounds them is the round
 // trips of one launch, as long as the arithmetic stays out of the way.  As FP32 multiply-adds, one a code and token behind a conversion
 // of every code, it did not; on the tensor cores (skinny_mma.cuh: exact products of integer codes with BF16 activations, or with the three
-// BF16 planes of FP32 ones, FP32 sums) the same numbers are a few hundred MMAs a warp.  d = 4096, r = 320, Q8, as a CUDA graph, down and up:
-// 16 tokens 23.7 + 19.0 -> 8.6 + 7.9 us, one token 7.3 + 9.0 -> 6.7 + 6.2, 63 tokens 105 + 51 -> 20 + 21; against 64 bits, FP32 streams
-// of 16 tokens, h 4.0e-7 -> 1.4e-7 and u 5.7e-7 -> 1.0e-7 (2-norms).
+// BF16 planes of FP32 ones, FP32 sums) the same numbers are a few hundred MMAs a warp.  Both halves as a CUDA graph, d = 4096, Q8, us before ->
+// now: r = 320, one token 16.9 -> 12.6, 16 tokens 42.2 -> 15.7, 64 158 -> 40, 300 525 -> 136; r = 32, 16 tokens 17.9 -> 10.7; r = 1024, 99.5 -> 31.9.
+// Against 64 bits, FP32 streams of 16 tokens, h 4.0e-7 -> 1.4e-7 and u 5.7e-7 -> 0.9e-7 (2-norms).  ncu, 16 tokens from HBM: issue slots 25 and
+// 32 %, tensor pipe 9 and 13 %, DRAM 6 and 7 %; the warps wait for loads (long scoreboard) and, in the down half, for the cluster.
 //   down: 16 weight rows by a cluster of eight CTAs, an eighth of the row each (an eighth lies in one stream), which a CTA's eight warps share;
 //         a lane's codes are all asked for at once, its activations come from L2 in fragment order as they lie; the parts meet in shared
 //         memory, then across the cluster.
