@@ -227,6 +227,22 @@ def test_route_small_reports_a_bad_logit(cuda):
     assert e2.tolist()[0] == 1  # the pack sees the token's ids of -1 as out of range
 
 
+@pytest.mark.parametrize("M,K,bits", [(19000, 64 * 17, 8), (19000, 64 * 17, 4), (10001, 64 * 32, 8), (33, 64 * 40, 4), (32, 64, 8)])
+def test_staged_tiles_cut_by_k(cuda, M, K, bits):
+    """Tile-blocked activations of a dense projection, word for word, where the launch cuts k into ranges: one block past a range, two
+    whole ranges, and few rows."""
+    from strixite_b200 import kernels as Kn
+    x = torch.randn((M, K), generator=torch.Generator(device="cpu").manual_seed(K)).to(torch.bfloat16).to(cuda)
+    xs = torch.full((M, K), -1, dtype=torch.int16, device=cuda)
+    Kn.stage_f16_tiles(x, None, 0, M, 1, 1, K, bits, xs)
+    v = x.to(torch.float16).view(M, K // 64, 8, 8)  # [row, 64-k block, 16-byte chunk, element]
+    if bits == 4:
+        v = v[..., [0, 4, 1, 5, 2, 6, 3, 7]]
+    chunk = torch.arange(8, device=cuda)[None, :] ^ (torch.arange(M, device=cuda)[:, None] & 7)  # chunk c of row r lies at place c ^ r % 8
+    v = torch.gather(v, 2, chunk[:, None, :, None].expand(M, K // 64, 8, 8))
+    assert torch.equal(xs.view(K // 64, M, 64), v.permute(1, 0, 2, 3).reshape(K // 64, M, 64).contiguous().view(torch.int16))
+
+
 @pytest.mark.parametrize("ydt", [torch.float32, torch.bfloat16])
 def test_residual_add(cuda, ydt):
     from strixite_b200 import kernels as Kn
