@@ -17,7 +17,10 @@
 //     that showed it, which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 540 us at 777
 //     tokens, 789 -> 728 at 4096, dense 1001 x 8192 x 4096 64.7 -> 57.1, 4000 tokens Q8 232 -> 216.
 //   * Steps of 128 k, eight MMAs a commit: with the loop of one lane a commit and the next stage's wait cost ~250 cycles whatever lay between.
-//   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 162 instructions a warp and step, not 290.
+//   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 146 instructions a warp and step.  With neither copies nor MMAs the producers'
+//     own loop took 464 of the 548 us at 777 tokens: another 140 instructions a warp and step.  Now scales come through pointers that advance, the next item's
+//     first ones are asked for at the item's start, and arrivals are predicated, not branched to: 410 alone, gate/up 548 -> 506 us.  Asking for barriers a
+//     phase ahead, a deeper item ring or a second quarter dequantized before the stage is free: no faster (+0 to +1 %).
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
 // A wider token tile would not be cheaper: it shares a dequantization that is no longer the bound, and 128 columns leave tensor
@@ -298,22 +301,30 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         constexpr int kCodeRegs = kBK * BITS / 128;  // 16-byte chunks of codes per row and step
         constexpr int kWordsPerChunk = BITS == 4 ? 4 : 2;  // runs of eight codes in one of them
         // K is a multiple of 128 and so a row's groups of a step's: where the arrays start decides
-        const bool vec_scales = ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & (2 * kGroups - 1)) == 0;
+        const bool vec_scales = kGroups == 1 || ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & (2 * kGroups - 1)) == 0;
         // this thread's row inside the first slot; its chunks are swizzled (128-byte mode, 64-byte for rows of 64 bytes), so that chunk c
         // lies at my_w ^ 16 c
         const uint32_t my_w = w_base + (uint32_t)(srow * kRowBytes) + (uint32_t)(kRowBytes == 64 ? (srow >> 1) & 3 : srow & 7) * 16u;
         const uint32_t a_addr = ((uint32_t)(a_quad * 32) << 16) + (uint32_t)(kAccs * kTile + set * kAStageCols);
+        const uint32_t signals = lane == 0 ? 1u : 0u;
 
         // Scales and mins of a step's groups, fetched one step of the set ahead of use (fetched eight groups at a time, of which a set used a
         // quarter or half, and picked out by selects, they were 5 % of the Q8 forms).  A row past the end of the expert gets zeros: its
         // operand row is then zero whatever codes its lane reads.
-        auto load_scales = [&](int wrow, int step) {
+        auto load_scales = [&](const uint16_t *sp, const uint16_t *mp) {
             Scales<kGroups> c{};
-            if (wrow < 0) return c;
-            const int64_t at = (int64_t)wrow * groups + step * kGroups;
-            if (vec_scales) load_groups<kGroups>(c.s, a.scale + at), load_groups<kGroups>(c.m, a.minv + at);
-            else c = load_scales_each<kGroups>(a.scale + at, a.minv + at);
+            if (vec_scales) load_groups<kGroups>(c.s, sp), load_groups<kGroups>(c.m, mp);
+            else c = load_scales_each<kGroups>(sp, mp);
             return c;
+        };
+        auto scales_at = [&](int wrow, int step) {
+            const int64_t at = (int64_t)wrow * groups + step * kGroups;
+            return wrow < 0 ? Scales<kGroups>{} : load_scales(a.scale + at, a.minv + at);
+        };
+        auto wait = [&](uint64_t *bar, uint32_t parity, int i, int role) {
+            if (mbar_wait(bar, parity, abort_v, a.wait_limit_ns)) return true;
+            raise_abort(blockIdx.x + i * gridDim.x, role);
+            return false;
         };
         uint32_t free_phase = 1u;  // parity of the phase that leaves the stage to the set's next step: there is none before the first
         Turn<kWSlots> slot{set, 0u};
@@ -321,31 +332,27 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         bool live = true;
         float nxt_scale = 1.f;
         Item nxt = read_item(0, p0, nxt_scale);
-        int row = -1;
-        Scales<kGroups> sc_nxt{};
-        bool have = false;  // sc_nxt is of the set's next step
-        if (nxt.bucket >= 0 && nxt.bucket < a.E) row = (int)row_of(nxt, p0);
+        int row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
+        Scales<kGroups> sc_nxt = scales_at(st < n_steps ? row : -1, st);  // of the set's next step
         for (int i = 0; nxt.bucket >= 0 && live; ++i) {
             const Item it = nxt;
             const float scale = nxt_scale, scale_min = scale * 0x1p-24f;
             nxt = read_item(i + 1, p0, nxt_scale);
-            const bool more = nxt.bucket >= 0 && nxt.bucket < a.E;
-            const int nxt_row = more ? (int)row_of(nxt, p0) : -1;
+            const int nxt_row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
             if (it.bucket >= a.E) {
-                row = nxt_row;
+                row = nxt_row, sc_nxt = scales_at(st < n_steps ? row : -1, st);
                 continue;
             }
-            for (; st < n_steps; st += kWays, slot.advance(kWays)) {
-                if (!have) sc_nxt = load_scales(row, st);
+            const bool natural = __any_sync(0xffffffffu, scale < 0.f);  // the quadrant's rows share it
+            // the set's first step of the next item, if it has one there
+            const int after = st + (max(n_steps - st, 0) + kWays - 1) / kWays * kWays - n_steps;
+            Scales<kGroups> sc_item{};
+            if (kGroups < 4) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
+            const uint16_t *sp = a.scale + (int64_t)max(row, 0) * groups + (st + kWays) * kGroups, *mp = a.minv + (sp - a.scale);
+            for (; st < n_steps; st += kWays, slot.advance(kWays), sp += kWays * kGroups, mp += kWays * kGroups) {
                 const Scales<kGroups> sc = sc_nxt;
-                const int nst = st + kWays;  // in this item, or in the next one
-                have = nst < n_steps || (more && nst - n_steps < n_steps);
-                if (have) sc_nxt = nst < n_steps ? load_scales(row, nst) : load_scales(nxt_row, nst - n_steps);
-                bool ok = true;
-                if (!mbar_wait(&w_full[slot.at], slot.phase, abort_v, a.wait_limit_ns)) {
-                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 7);
-                    ok = false;
-                }
+                if (row >= 0 && st + kWays < n_steps) sc_nxt = load_scales(sp, mp);
+                bool ok = wait(&w_full[slot.at], slot.phase, i, 7);
                 const uint32_t src = my_w + slot.at * (uint32_t)kSlotBytes;
                 uint4 code[kCodeRegs];
 #pragma unroll
@@ -368,18 +375,15 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 };
                 uint4 d[4];
                 quarter(0, d);
-                if (ok && !mbar_wait(&empty_bar[set], free_phase, abort_v, a.wait_limit_ns)) {
-                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 1);
-                    ok = false;
-                }
+                ok = wait(&empty_bar[set], free_phase, i, 1) && ok;
                 // reconverges the warp; a wait that gave up in any lane ends the warp's work
                 if (!__all_sync(0xffffffffu, ok)) {
                     live = false;
                     break;
                 }
                 tc_fence_after();  // the stores below come after the MMAs that freed the stage
-                if (scale > 0.f) {
-                    if (lane == 0) mbar_arrive(&w_empty[slot.at]);  // the codes are in registers: the slot may be refilled
+                if (!natural) {
+                    mbar_arrive_if(signals, &w_empty[slot.at]);  // the codes are in registers: the slot may be refilled
                     tc_st16(a_addr, d);
 #pragma unroll
                     for (int hc = 1; hc < 4; ++hc) {
@@ -388,15 +392,16 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                     }
                 } else {
                     natural_step<BITS, G>(src, a_addr, sc);
-                    if (lane == 0) mbar_arrive(&w_empty[slot.at]);
+                    mbar_arrive_if(signals, &w_empty[slot.at]);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&full_bar[set]);
+                mbar_arrive_if(signals, &full_bar[set]);
                 free_phase ^= 1u;
             }
-            st -= n_steps, row = nxt_row;
+            if (kGroups == 4) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);  // four groups are too many registers to hold over an item
+            st -= n_steps, row = nxt_row, sc_nxt = sc_item;
         }
     } else if (warp == kItemWarp) {
         // ===================== the item ring =====================

@@ -26,6 +26,13 @@ __device__ inline void mbar_init(uint64_t *bar, uint32_t count) {
 __device__ inline void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// The same in the lanes whose `pred` is not zero, without a branch around it.
+__device__ inline void mbar_arrive_if(uint32_t pred, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(pred)
+        : "memory");
+}
 __device__ inline bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
