@@ -9,9 +9,8 @@
 //     weight is the reference's BF16 [N, K], or an FP32 one split once, at load time, into P BF16 "planes"
 //     W = W1 + W2 (+ W3) (each plane the BF16 rounding of what the planes before it left over), so that the products
 //     x * Wp are exact BF16 x BF16 products and their FP32 sum carries 16 (P = 2) or 24 (P = 3) bits of the weight.
-//     The weight rows sit on the MMA's M (128 a tile), the tokens on its N (128), accumulators double-buffered in
-//     tensor memory; warp 0 issues the copies, warp 1 the MMAs, warps 2-5 are the epilogue (bias add, FP32 store,
-//     a token's 32 experts of a warp are 128 contiguous bytes).
+//     The tokens sit on the MMA's M (128 a tile), the weight rows on its N, as many as suit the launch (gemm_shape); accumulators
+//     double-buffered in tensor memory; warp 0 issues the copies, warp 1 the MMAs, warps 2-5 are the epilogue (bias add, FP32 store).
 // Every device-side wait is bounded; one that runs out is recorded in the library's status words (see
 // sxb_check_dense_status) and the kernel returns.
 
@@ -20,6 +19,7 @@
 #include "tc_ptx.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace sxb {
 namespace {
@@ -229,18 +229,22 @@ __global__ void __launch_bounds__(256) residual_add_kernel(const uint4 *__restri
 // ---- tcgen05 form ----------------------------------------------------------------------------------------------
 
 constexpr int kGemmThreads = 192;      // warp 0 copies, warp 1 MMA issue, warps 2-5 epilogue
-constexpr int kTile = 128;             // weight rows (MMA M) and tokens (MMA N) of a tile
+constexpr int kTile = 128;             // tokens of a tile (MMA M); the planes' rows are padded to as many
 constexpr int kGemmBK = 64;            // k per stage: one 128-byte swizzle line of BF16
-constexpr int kOperandBytes = kTile * kGemmBK * 2;  // 16 KB: one operand tile of one k-block
-constexpr int kMaxStages = 4;
+constexpr int kXBytes = kTile * kGemmBK * 2;  // 16 KB: a stage's activations; a plane's part is 128 bytes a weight row
+constexpr int kMaxStages = 8;
 constexpr int kMaxPlanes = 3;
-constexpr int kGemmTmemCols = 256;     // two accumulators of 128 token columns
+constexpr int kMaxRows = 256;          // weight rows of a tile (MMA N), a multiple of 16: two accumulators fill tensor memory
+constexpr int kGemmTmemCols = 512;
+constexpr int kEpiCols = 16, kEpiPitch = kEpiCols + 1;  // the epilogue's transpose: 32 tokens x 16 rows a warp
+constexpr int kEpiBytes = 4 * 32 * kEpiPitch * 4;
+constexpr size_t kGemmSmem = 230400;   // of 232448 bytes; the rest is for the barriers
 
 struct GemmArgs {
     const float *bias;
     float *logits;
     int64_t M, N, Npad, K, ld;
-    int planes, stages;
+    int planes, stages, rows;  // rows: of a tile
     uint32_t *status;
     unsigned long long wait_limit_ns;
 };
@@ -250,13 +254,20 @@ struct GemmArgs {
 __device__ inline uint32_t instr_desc_bf16(int n_cols) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n_cols >> 3) << 17) | ((128u >> 4) << 24);
 }
-// D[tmem] (+)= A[smem] * B[smem], issued by one thread.
-__device__ inline void tc_mma_f16_ss_one(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+// D[tmem] (+)= A[smem] * B[smem] over 64 k, both 128-byte-swizzled: four MMAs, issued by the lane with leader = 1 of a whole warp under uniform
+// control flow, so that descriptors stay in uniform registers.
+__device__ inline void tc_kblock_ss(uint32_t leader, uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n\t.reg .pred p, q, one;\n\t.reg .b32 x1, x2, x3, y1, y2, y3;\n\t.reg .b64 a0, a1, a2, a3, b0, b1, b2, b3;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tsetp.eq.b32 one, 0, 0;\n\t"
+        "add.u32 x1, %1, 2;\n\tadd.u32 x2, %1, 4;\n\tadd.u32 x3, %1, 6;\n\tadd.u32 y1, %2, 2;\n\tadd.u32 y2, %2, 4;\n\tadd.u32 y3, %2, 6;\n\t"
+        "mov.b64 a0, {%1, %3};\n\tmov.b64 a1, {x1, %3};\n\tmov.b64 a2, {x2, %3};\n\tmov.b64 a3, {x3, %3};\n\t"
+        "mov.b64 b0, {%2, %3};\n\tmov.b64 b1, {y1, %3};\n\tmov.b64 b2, {y2, %3};\n\tmov.b64 b3, {y3, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a0, b0, %4, p;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %4, one;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %4, one;\n\t}" ::"r"(d),
+        "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(leader)
         : "memory");
 }
 __device__ inline void tc_ld16(uint32_t taddr, float (&v)[16]) {
@@ -270,6 +281,14 @@ __device__ inline void tc_ld16(uint32_t taddr, float (&v)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+// A place in a ring of n barriers and the parity of the phase it is in.
+struct RingTurn {
+    int at;
+    uint32_t phase;
+    __device__ inline void advance(int n) {
+        if (++at == n) at = 0, phase ^= 1u;
+    }
+};
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
     logits_gemm_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap) {
@@ -279,10 +298,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_kb = (int)(a.K / kGemmBK), n_rb = (int)(a.Npad / kTile), n_tt = (int)((a.M + kTile - 1) / kTile);
-    const int n_items = n_rb * n_tt;
-    const int stage_bytes = (1 + a.planes) * kOperandBytes;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int n_kb = (int)(a.K / kGemmBK), n_rb = (int)((a.N + a.rows - 1) / a.rows), n_tt = (int)((a.M + kTile - 1) / kTile);
+    const int64_t n_items = (int64_t)n_rb * n_tt;
+    const int plane_bytes = a.rows * kGemmBK * 2, stage_bytes = kXBytes + a.planes * plane_bytes;
     volatile int *abort_v = &abort_flag;
 
     if (threadIdx.x == 0) {
@@ -301,7 +320,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
 
-    auto raise_abort = [&](int item, int role) {
+    auto raise_abort = [&](int64_t item, int role) {
         if (atomicExch(&abort_flag, 1) == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) {
             a.status[1] = (uint32_t)item;
             a.status[2] = (uint32_t)role;
@@ -312,93 +331,98 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     if (warp == 0) {
         // ===================== copies: one thread, as far ahead as free stages allow =====================
         if (lane == 0) {
-            for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x) {
-                const int tile = item / n_rb, rb = item % n_rb;
-                for (int kb = 0; kb < n_kb; ++kb, ++issued) {
-                    const int stage = issued % a.stages;
-                    if (issued >= (uint32_t)a.stages &&
-                        !mbar_wait(&empty_bar[stage], ((issued / a.stages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+            RingTurn turn{0, 1u};  // the phase before the first leaves every stage free
+            for (int64_t item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x) {
+                const int tile = (int)(item / n_rb), rb = (int)(item % n_rb);
+                for (int kb = 0; kb < n_kb; ++kb, ++issued, turn.advance(a.stages)) {
+                    if (!mbar_wait(&empty_bar[turn.at], turn.phase, abort_v, a.wait_limit_ns)) {
                         raise_abort(item, 5);
                         break;
                     }
-                    const uint32_t dst = smem_u32(smem + stage * stage_bytes);
-                    mbar_expect_tx(&full_bar[stage], (uint32_t)stage_bytes);
-                    tma_load_2d(dst, &xmap, kb * kGemmBK, tile * kTile, &full_bar[stage]);
+                    const uint32_t dst = smem_u32(smem + turn.at * stage_bytes);
+                    mbar_expect_tx(&full_bar[turn.at], (uint32_t)stage_bytes);
+                    tma_load_2d(dst, &xmap, kb * kGemmBK, tile * kTile, &full_bar[turn.at]);
                     for (int p = 0; p < a.planes; ++p)
-                        tma_load_2d(dst + (1 + p) * kOperandBytes, &wmap, kb * kGemmBK, (int)(p * a.Npad) + rb * kTile, &full_bar[stage]);
+                        tma_load_2d(dst + kXBytes + p * plane_bytes, &wmap, kb * kGemmBK, (int)(p * a.Npad) + rb * a.rows, &full_bar[turn.at]);
                 }
             }
         }
     } else if (warp == 1) {
         // ===================== MMA issue =====================
-        // One thread runs the whole loop: an MMA costs it 12 cycles, against 40 to 90 with the election inside each MMA's
-        // instruction group, which at twelve MMAs a k-block (three planes) was more than their time on the tensor cores.
-        if (elect_one()) {
-            uint32_t count = 0, acc_count = 0;
-            const uint32_t idesc = instr_desc_bf16(kTile);
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++acc_count) {
-                const uint32_t buf = acc_count & 1u;
-                if (!mbar_wait(&acc_empty[buf], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
-                    raise_abort(item, 2);
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t d = tmem_base + buf * (uint32_t)kTile;
-                for (int kb = 0; kb < n_kb; ++kb, ++count) {
-                    const int stage = count % a.stages;
-                    if (!mbar_wait(&full_bar[stage], (count / a.stages) & 1u, abort_v, a.wait_limit_ns)) {
-                        raise_abort(item, 3);
-                        ok = false;
+        const uint32_t leader = elect_one() ? 1u : 0u, idesc = instr_desc_bf16(a.rows);
+        const uint64_t desc0 = smem_desc(smem_u32(smem));
+        const uint32_t hi = (uint32_t)(desc0 >> 32), plane_lo = (uint32_t)plane_bytes / 16, stage_lo = (uint32_t)stage_bytes / 16;
+        uint32_t lo = (uint32_t)desc0, acc_count = 0;
+        RingTurn turn{0, 0u};
+        bool ok = true;
+        for (int64_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++acc_count) {
+            const uint32_t buf = acc_count & 1u;
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns));
+            if (!ok) {
+                if (leader) raise_abort(item, 2);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem_base + buf * (uint32_t)kMaxRows;
+            bool ready = false;
+            for (int kb = 0; kb < n_kb; ++kb) {
+                if (!__all_sync(0xffffffffu, ready)) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[turn.at], turn.phase, abort_v, a.wait_limit_ns));
+                    if (!ok) {
+                        if (leader) raise_abort(item, 3);
                         break;
                     }
-                    tc_fence_after();
-                    const uint32_t base = smem_u32(smem + stage * stage_bytes);
-                    const uint64_t b_desc = smem_desc(base);
-                    for (int p = 0; p < a.planes; ++p) {
-                        const uint64_t a_desc = smem_desc(base + (uint32_t)((1 + p) * kOperandBytes));
-#pragma unroll
-                        for (int j = 0; j < kGemmBK / 16; ++j)  // k = 16 an instruction: 32 bytes further along the swizzled line
-                            tc_mma_f16_ss_one(d, a_desc + 2 * j, b_desc + 2 * j, idesc, (kb | p | j) != 0);
-                    }
-                    tc_commit_one(&empty_bar[stage]);  // the stage is free once these MMAs have read it
                 }
-                if (ok) tc_commit_one(&acc_full[buf]);
+                tc_fence_after();
+                uint64_t *const done = &empty_bar[turn.at];
+                const uint32_t b_lo = lo + kXBytes / 16;
+                const uint32_t lo_nxt = turn.at + 1 == a.stages ? (uint32_t)desc0 : lo + stage_lo;
+                turn.advance(a.stages);
+                ready = mbar_test(&full_bar[turn.at], turn.phase);  // asked for under the MMAs
+                for (int p = 0; p < a.planes; ++p) tc_kblock_ss(leader, d, lo, b_lo + p * plane_lo, hi, idesc, (kb | p) != 0);
+                tc_commit_if(leader, done);  // the stage is free once these MMAs have read it
+                lo = lo_nxt;
             }
-            // every MMA of this CTA has completed before tensor memory is released (not given up while aborting)
-            tc_commit_one(&drain_bar);
-            mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
+            if (ok) tc_commit_if(leader, &acc_full[buf]);
         }
+        // every MMA of this CTA has completed before tensor memory is released (not given up while aborting)
+        tc_commit_if(leader, &drain_bar);
+        mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
         __syncwarp();
     } else {
         // ===================== epilogue =====================
+        // Lane = token: sixteen weight rows at a time go through shared memory, so that a store writes 64 neighbouring bytes of two tokens.
         const int quad = warp & 3;  // the tensor-memory lanes a warp may read: 32 (warp % 4) ..
+        float *turned = reinterpret_cast<float *>(smem + a.stages * stage_bytes) + (warp - 2) * 32 * kEpiPitch;
         uint32_t acc_count = 0;
-        for (int item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x, ++acc_count) {
-            const int tile = item / n_rb, rb = item % n_rb;
+        for (int64_t item = blockIdx.x; item < n_items && !*abort_v; item += gridDim.x, ++acc_count) {
+            const int tile = (int)(item / n_rb), rb = (int)(item % n_rb);
             const uint32_t buf = acc_count & 1u;
             if (lane == 0 && !mbar_wait(&acc_full[buf], (acc_count >> 1) & 1u, abort_v, a.wait_limit_ns)) raise_abort(item, 4);
             __syncwarp();
             if (*abort_v) break;
             tc_fence_after();
-            const int64_t e = (int64_t)rb * kTile + quad * 32 + lane;
-            const bool row_ok = e < a.N;
-            const float b = (row_ok && a.bias) ? a.bias[e] : 0.f;
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (uint32_t)kTile;
-            const int64_t t0 = (int64_t)tile * kTile;
-            for (int c0 = 0; c0 < kTile; c0 += 16) {
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + buf * (uint32_t)kMaxRows;
+            const int64_t t0 = (int64_t)tile * kTile + quad * 32, e0 = (int64_t)rb * a.rows;
+            for (int c0 = 0; c0 < a.rows; c0 += kEpiCols) {
                 float v[16];
                 tc_ld16(taddr + (uint32_t)c0, v);
-                if (c0 + 16 == kTile) {  // the last columns are in registers: the accumulator may be overwritten
+                if (c0 + kEpiCols == a.rows) {  // the last columns are in registers: the accumulator may be overwritten
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&acc_empty[buf]);
                 }
 #pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    const int64_t tok = t0 + c0 + t;
-                    if (row_ok && tok < a.M) a.logits[tok * a.ld + e] = v[t] + b;
+                for (int c = 0; c < kEpiCols; ++c) turned[lane * kEpiPitch + c] = v[c];
+                __syncwarp();
+                const int64_t e = e0 + c0 + (lane & 15);
+                const float b = (e < a.N && a.bias) ? a.bias[e] : 0.f;
+#pragma unroll
+                for (int t = 0; t < 32; t += 2) {
+                    const int64_t tok = t0 + t + (lane >> 4);
+                    if (e < a.N && tok < a.M) a.logits[tok * a.ld + e] = turned[(t + (lane >> 4)) * kEpiPitch + (lane & 15)] + b;
                 }
+                __syncwarp();
             }
         }
     }
@@ -416,6 +440,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kGemmTmemCols) : "memory");
     }
+}
+
+// The weight rows of a tile: those for which the launch's estimate is least.  In SM cycles a k-block takes the longest of its copies (50 bytes a
+// cycle and SM, measured with every SM at it), its MMAs (66 at least: reading 4 KB of activations from shared memory bounds them) and what one stage
+// less than there are hides of a copy's latency; an item, its epilogue.  Few tokens want narrow tiles, so that the k-blocks' chain of MMAs is
+// shared by the machine (128 weight rows a tile, the weights on the M side: 10 CTAs at 150 tokens); many want wide ones, for less traffic.
+// 513 x 4096 FP32, the sums' order and bits as before: 150 tokens 48 -> 29 us (16 rows), 777 48 -> 30 (32), 1200 48 -> 32 (48), 4096 91 -> 52 (144),
+// 16384 230 -> 227.  What bounds it: the MMAs' operand reads, from 4096 tokens on the copies.
+struct GemmShape {
+    int rows, stages;
+};
+GemmShape gemm_shape(int64_t M, int64_t N, int64_t n_kb, int planes, int sms) {
+    GemmShape best{16, 2};
+    double least = 0;
+    for (int rows = 16; rows <= kMaxRows && (rows == 16 || rows < N + 16); rows += 16) {
+        const int bytes = kXBytes + planes * rows * kGemmBK * 2;
+        const int stages = (int)std::min<size_t>(kMaxStages, (kGemmSmem - 1024 - kEpiBytes) / bytes);
+        if (stages < 2) break;
+        const double copies = bytes / 50.0, mmas = planes * 4 * std::max(66.0, 32 + rows / 4.0), latency = (1500 + mmas) / stages;
+        const double items = (double)((M + kTile - 1) / kTile) * (double)((N + rows - 1) / rows);
+        const double cost = std::ceil(items / sms) * ((double)n_kb * std::max(copies, std::max(mmas, latency)) + 20.0 * rows + 3000);
+        if (least == 0 || cost <= least) least = cost, best = GemmShape{rows, stages};
+    }
+    return best;
 }
 
 // W [N, K] (FP32 or BF16) -> P BF16 planes [P][Npad][K]: plane p holds the BF16 rounding of what the planes before it left
@@ -533,7 +581,8 @@ int sxb_router_logits_wmma(const void *x, const void *planes_in, int planes, con
     SXB_CHECK(apart(x, M * K * 2, logits, M * ld * 4), fn, ": logits overlap x");
     GemmArgs a{};
     a.bias = bias, a.logits = logits, a.M = M, a.N = N, a.Npad = pad_rows(N), a.K = K, a.ld = ld, a.planes = planes;
-    a.stages = planes == 3 ? 3 : 4;
+    const GemmShape shape = gemm_shape(M, N, K / kGemmBK, planes, sm_count());
+    a.rows = shape.rows, a.stages = shape.stages;
     a.wait_limit_ns = wait_limit_ns();
     if (int rc = library_status_words(fn, &a.status)) return rc;
     CUtensorMap xmap, wmap;
@@ -542,13 +591,12 @@ int sxb_router_logits_wmma(const void *x, const void *planes_in, int planes, con
         return rc;
     // one plane may be the raw BF16 weight [N, K] itself: its rows past N read as zero instead of being stored as zeros
     if (int rc = tensor_map_2d(fn, planes_in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)K, (uint64_t)(planes == 1 ? N : planes * a.Npad), (uint64_t)K * 2,
-                               kGemmBK, kTile, CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
+                               kGemmBK, (uint32_t)a.rows, CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
         return rc;
-    const size_t smem = (size_t)a.stages * (1 + planes) * kOperandBytes + 1024;
-    // the function's limit is one for all threads of the process: always the largest (three planes), not this call's
-    SXB_CUDA(cudaFuncSetAttribute(logits_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * kOperandBytes + 1024), fn,
-             ": reserving shared memory");
-    const int64_t items = (a.Npad / kTile) * ((M + kTile - 1) / kTile);
+    const size_t smem = (size_t)a.stages * (kXBytes + planes * a.rows * kGemmBK * 2) + kEpiBytes + 1024;
+    // the function's limit is one for all threads of the process: always the largest, not this call's
+    SXB_CUDA(cudaFuncSetAttribute(logits_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem), fn, ": reserving shared memory");
+    const int64_t items = ((N + a.rows - 1) / a.rows) * ((M + kTile - 1) / kTile);
     const unsigned grid = (unsigned)std::min<int64_t>(items, sm_count());
     logits_gemm_kernel<<<grid, kGemmThreads, smem, static_cast<cudaStream_t>(stream)>>>(a, xmap, wmap);
     SXB_CHECK_LAUNCH(fn, " M=", M, " N=", N, " K=", K, " planes=", planes);

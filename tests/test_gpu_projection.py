@@ -227,6 +227,28 @@ def test_route_small_reports_a_bad_logit(cuda):
     assert e2.tolist()[0] == 1  # the pack sees the token's ids of -1 as out of range
 
 
+@pytest.mark.parametrize("M,N,K,planes", [(1, 1, 64, 3), (129, 17, 128, 2), (150, 513, 256, 3), (640, 255, 192, 1), (777, 513, 512, 3), (1200, 513, 128, 3),
+                                           (4096, 513, 64, 3), (60001, 16, 64, 2), (40000, 300, 64, 1)])
+def test_router_logits_tcgen05_tiles(cuda, M, N, K, planes):
+    """Tiles of every width that the launch picks, ragged last tiles on both sides, several tiles a CTA (both accumulators, several turns).
+    FP32 sums of exact products: K P of them, each off by 2^-23 of the largest partial sum at most; two planes hold 16 bits of a weight."""
+    from strixite_b200 import kernels as Kn
+    g = torch.Generator(device="cpu").manual_seed(M + N)
+    x = torch.randn((M, K), generator=g).to(torch.bfloat16).to(cuda)
+    w = (torch.randn((N, K), generator=g) * 0.02).to(cuda)
+    if planes == 1:
+        w = w.to(torch.bfloat16)
+    bias = torch.randn(N, generator=g).to(cuda)
+    out = torch.full((M, N + 3), float("nan"), device=cuda)
+    Kn.router_logits_wmma(x, Kn.router_prepare(w, planes), bias, out)
+    torch.cuda.synchronize()
+    Kn.check_dense_status("router_logits_wmma")
+    want = x.double() @ w.double().T + bias.double()
+    size = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    bound = size * (K * planes * 2.0 ** -23 + (2.0 ** -16 if planes == 2 else 0)) + 1e-7
+    assert torch.isnan(out[:, N:]).all() and ((out[:, :N].double() - want).abs() <= bound).all()
+
+
 @pytest.mark.parametrize("M,K,bits", [(19000, 64 * 17, 8), (19000, 64 * 17, 4), (10001, 64 * 32, 8), (33, 64 * 40, 4), (32, 64, 8)])
 def test_staged_tiles_cut_by_k(cuda, M, K, bits):
     """Tile-blocked activations of a dense projection, word for word, where the launch cuts k into ranges: one block past a range, two
