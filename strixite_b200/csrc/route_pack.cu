@@ -20,7 +20,7 @@ namespace {
 
 constexpr int kPackThreads = 1024;
 constexpr int kSmallSlots = 2048;
-constexpr int kSegWarps = 4;  // warps (segments) per CTA in the histogram / scatter launches
+constexpr int kSegWarps = 8, kSegRounds = kSegSlots / (32 * kSegWarps);  // of the CTA that takes a segment in the histogram / scatter launches
 
 __device__ inline int bucket_of(int32_t id, int e_lo, int E_local) {
     const int b = id - e_lo;
@@ -112,25 +112,21 @@ __device__ void emit_tiles(const RouteWords &L, int32_t *ws, const Layout &sm, i
     }
 }
 
-// One warp places the slots [s0, s1), at most kSegSlots of them, in order: rank inside a round from match.any, bucket cursors
-// in shared memory.  All ids are asked for before the first is used (with a load a round a round took 1100 cycles).
-__device__ inline void warp_place(const int32_t *ids, int s0, int s1, int e_lo, int E_local, int *cursor, int32_t *slots) {
-    constexpr int kRounds = kSegSlots / 32;
+// Ranks of a warp's slots s0 + 32 r + lane (ids id[r], below S) among its slots of the same bucket: match.any in a round, the warp's own
+// counts (zero at first) across rounds.  bucket < 0: past the end.
+template <int ROUNDS>
+__device__ inline void rank_slots(const int32_t (&id)[ROUNDS], int s0, int S, int e_lo, int E, uint16_t *counts, int (&bucket)[ROUNDS], int (&rank)[ROUNDS]) {
     const int lane = threadIdx.x & 31;
-    int id[kRounds];
 #pragma unroll
-    for (int r = 0; r < kRounds; ++r) id[r] = s0 + r * 32 + lane < s1 ? ids[s0 + r * 32 + lane] : 0;
-#pragma unroll
-    for (int r = 0; r < kRounds; ++r) {
-        const int s = s0 + r * 32 + lane;
-        if (s0 + r * 32 >= s1) break;
-        const bool live = s < s1;
-        const int b = live ? bucket_of(id[r], e_lo, E_local) : -1 - lane;  // dead lanes match nobody
-        const unsigned peers = __match_any_sync(0xffffffffu, b);
-        const int rank = __popc(peers & ((1u << lane) - 1u)), at = live ? cursor[b] : 0;
-        if (live) slots[at + rank] = s;
+    for (int r = 0; r < ROUNDS; ++r) {
+        const bool live = s0 + r * 32 + lane < S;
+        bucket[r] = live ? bucket_of(id[r], e_lo, E) : -1 - lane;  // dead lanes match nobody
+        if (s0 + r * 32 >= S) continue;
+        const unsigned peers = __match_any_sync(0xffffffffu, bucket[r]);
+        const int before = live ? counts[bucket[r]] : 0, mine = __popc(peers & ((1u << lane) - 1u));
+        rank[r] = before + mine;
         __syncwarp();  // of the whole warp: one per group of peers ran them one after another
-        if (live && rank == 0) cursor[b] = at + __popc(peers);
+        if (live && mine == 0) counts[bucket[r]] = (uint16_t)(before + __popc(peers));
         __syncwarp();
     }
 }
@@ -161,17 +157,9 @@ __device__ void pack_small_body(const int32_t *__restrict__ ids, const RouteWord
 #pragma unroll
         for (int r = 0; r < kPlaceRounds; ++r) {
             const int s = (warp * rounds + r) * 32 + lane;
-            const bool live = r < rounds && s < S;
-            bucket[r] = live ? bucket_of(id[r], e_lo, E) : -1 - lane;  // dead lanes match nobody
-            if (live && (id[r] < 0 || id[r] >= E_total)) atomicMin(&first_bad, s);
-            if (r >= rounds) continue;
-            const unsigned peers = __match_any_sync(0xffffffffu, bucket[r]);
-            const int before = live ? counts[warp][bucket[r]] : 0, mine = __popc(peers & ((1u << lane) - 1u));
-            rank[r] = before + mine;
-            __syncwarp();
-            if (live && mine == 0) counts[warp][bucket[r]] = (uint16_t)(before + __popc(peers));
-            __syncwarp();
+            if (r < rounds && s < S && (id[r] < 0 || id[r] >= E_total)) atomicMin(&first_bad, s);
         }
+        rank_slots<kPlaceRounds>(id, warp * rounds * 32, min(S, (warp + 1) * rounds * 32), e_lo, E, counts[warp], bucket, rank);
     }
     __syncthreads();
     if (t == 0 && first_bad != 0x7fffffff) raise_error(err, (uint32_t)ids[first_bad], (uint32_t)first_bad);
@@ -215,28 +203,29 @@ __global__ void __launch_bounds__(kPackThreads)
     pack_small_body(ids, L, E_total, e_lo, ep, ws, expert_err);
 }
 
-// Large S, launch 1: histogram of every 1024-slot segment (one warp each) into scratch [nseg][E + 1], and the
+// Large S, launch 1: histogram of every 1024-slot segment (one CTA each) into scratch [nseg][E + 1], and the
 // segment's first invalid slot into segbad [nseg].
 __global__ void __launch_bounds__(32 * kSegWarps)
     pack_hist_kernel(const int32_t *__restrict__ ids, RouteWords L, int E_total, int e_lo, int32_t *ws) {
-    __shared__ int hist[kSegWarps][1024];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, E = (int)L.E, S = (int)L.S;
-    const int seg = blockIdx.x * kSegWarps + warp;
-    if (seg >= L.nseg) return;
-    for (int b = lane; b <= E; b += 32) hist[warp][b] = 0;
-    __syncwarp();
-    const int s0 = seg * kSegSlots, s1 = min(S, s0 + kSegSlots);
-    int bad = 0x7fffffff;
-    for (int s = s0 + lane; s < s1; s += 32) {
-        const int32_t id = ids[s];
-        atomicAdd(&hist[warp][bucket_of(id, e_lo, E)], 1);
-        if (id < 0 || id >= E_total) bad = min(bad, s);
+    __shared__ int hist[kMoeMaxExperts + 1], first_bad;
+    const int t = threadIdx.x, E = (int)L.E, S = (int)L.S, s0 = (int)blockIdx.x * kSegSlots;
+    int32_t id[kSegRounds];
+#pragma unroll
+    for (int r = 0; r < kSegRounds; ++r) id[r] = s0 + r * 32 * kSegWarps + t < S ? ids[s0 + r * 32 * kSegWarps + t] : 0;
+    for (int b = t; b <= E; b += 32 * kSegWarps) hist[b] = 0;
+    if (t == 0) first_bad = 0x7fffffff;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSegRounds; ++r) {
+        const int s = s0 + r * 32 * kSegWarps + t;
+        if (s >= S) break;
+        atomicAdd(&hist[bucket_of(id[r], e_lo, E)], 1);
+        if (id[r] < 0 || id[r] >= E_total) atomicMin(&first_bad, s);
     }
-    bad = __reduce_min_sync(0xffffffffu, bad);
-    __syncwarp();
-    int32_t *out = ws + L.scratch + (int64_t)seg * (E + 1);
-    for (int b = lane; b <= E; b += 32) out[b] = hist[warp][b];
-    if (lane == 0) ws[L.segbad + seg] = bad;
+    __syncthreads();
+    int32_t *out = ws + L.scratch + (int64_t)blockIdx.x * (E + 1);
+    for (int b = t; b <= E; b += 32 * kSegWarps) out[b] = hist[b];
+    if (t == 0) ws[L.segbad + blockIdx.x] = first_bad;
 }
 
 // Launch 2 (one CTA): per bucket, turn the segments' counts into their exclusive prefix (the segment's base inside
@@ -283,26 +272,40 @@ __global__ void __launch_bounds__(kPackThreads)
     for (int i = b; i < kTileLists * (E + 2); i += kPackThreads) ws[L.first + i] = sm.first[i / (E + 2)][i % (E + 2)];
 }
 
-// Launch 3: every warp places its segment, starting each bucket at offsets[b] + the segment's base; the CTAs then share the
-// tile lists, whose length grows with the slots (written by the one CTA of launch 2 they were most of its 39 us at 16384
-// tokens).
+// Launch 3: a CTA places its segment, each bucket from offsets[b] + the segment's base on; the CTAs then share the tile lists, whose
+// length grows with the slots (written by the one CTA of launch 2 they were most of its 39 us at 16384 tokens).  The segment's warps
+// take 128 slots each, as in the small pack: no warp waits for another (a warp a segment, 32 rounds one after another, was most of the
+// launch: 15.5 us at 777 to 16384 tokens x 10 slots).
 __global__ void __launch_bounds__(32 * kSegWarps)
     pack_scatter_kernel(const int32_t *__restrict__ ids, RouteWords L, int e_lo, int32_t *ws) {
-    __shared__ int cursor[kSegWarps][1024];
+    __shared__ __align__(4) uint16_t counts[kSegWarps][kMoeMaxExperts + 1];
     __shared__ Layout sm;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, E = (int)L.E, S = (int)L.S;
-    const int seg = blockIdx.x * kSegWarps + warp;
-    for (int b = threadIdx.x; b <= E; b += 32 * kSegWarps) sm.start[b] = ws[L.offsets + b];
-    for (int i = threadIdx.x; i < kTileLists * (E + 2); i += 32 * kSegWarps) sm.first[i / (E + 2)][i % (E + 2)] = ws[L.first + i];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, E = (int)L.E, S = (int)L.S, s0 = (int)blockIdx.x * kSegSlots + warp * kSegRounds * 32;
+    int32_t id[kSegRounds];
+#pragma unroll
+    for (int r = 0; r < kSegRounds; ++r) id[r] = s0 + r * 32 + lane < S ? ids[s0 + r * 32 + lane] : 0;
+    const int32_t *base = ws + L.scratch + (int64_t)blockIdx.x * (E + 1);
+    for (int i = t; i < kSegWarps * (kMoeMaxExperts + 1) / 2; i += 32 * kSegWarps) reinterpret_cast<uint32_t *>(counts)[i] = 0u;
+    for (int i = t; i < kTileLists * (E + 2); i += 32 * kSegWarps) sm.first[i / (E + 2)][i % (E + 2)] = ws[L.first + i];
+    for (int b = t; b <= E; b += 32 * kSegWarps) sm.start[b] = ws[L.offsets + b];
     __syncthreads();
-    if (seg < L.nseg) {
-        const int32_t *base = ws + L.scratch + (int64_t)seg * (E + 1);
-        for (int b = lane; b <= E; b += 32) cursor[warp][b] = sm.start[b] + base[b];
-        __syncwarp();
-        const int s0 = seg * kSegSlots;
-        warp_place(ids, s0, min(S, s0 + kSegSlots), e_lo, E, cursor[warp], ws + L.slots);
+    int bucket[kSegRounds], rank[kSegRounds];
+    rank_slots<kSegRounds>(id, s0, S, e_lo, E, counts[warp], bucket, rank);
+    __syncthreads();
+    for (int b = t; b <= E; b += 32 * kSegWarps) {
+        int at = 0;
+#pragma unroll
+        for (int w = 0; w < kSegWarps; ++w) {
+            const int c = counts[w][b];
+            counts[w][b] = (uint16_t)at;  // the warp's base inside the segment's run of the bucket
+            at += c;
+        }
     }
-    emit_tiles(L, ws, sm, blockIdx.x * 32 * kSegWarps + threadIdx.x, gridDim.x * 32 * kSegWarps);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSegRounds; ++r)
+        if (bucket[r] >= 0) ws[L.slots + sm.start[bucket[r]] + base[bucket[r]] + counts[warp][bucket[r]] + rank[r]] = s0 + r * 32 + lane;
+    emit_tiles(L, ws, sm, blockIdx.x * 32 * kSegWarps + t, gridDim.x * 32 * kSegWarps);
 }
 
 int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo,
@@ -321,7 +324,7 @@ int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64
     if (L.S <= kSmallSlots) {
         pack_small_kernel<<<1, kPackThreads, 0, st>>>(ids, L, (int)E_total, (int)e_lo, ep, w, err);
     } else {
-        const unsigned ctas = (unsigned)((L.nseg + kSegWarps - 1) / kSegWarps);
+        const unsigned ctas = (unsigned)L.nseg;
         pack_hist_kernel<<<ctas, 32 * kSegWarps, 0, st>>>(ids, L, (int)E_total, (int)e_lo, w);
         pack_scan_kernel<<<1, kPackThreads, 0, st>>>(ids, L, ep, w, err);
         pack_scatter_kernel<<<ctas, 32 * kSegWarps, 0, st>>>(ids, L, (int)e_lo, w);
