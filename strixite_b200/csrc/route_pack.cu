@@ -194,10 +194,11 @@ __global__ void __launch_bounds__(kPackThreads)
     route_small_kernel(const float *__restrict__ logits, int64_t ld, int M, int E_total, int k, int32_t *__restrict__ ids,
                        float *__restrict__ coef, RouteWords L, int e_lo, bool ep, int32_t *ws, uint32_t *router_err,
                        uint32_t *expert_err) {
+    __shared__ unsigned long long cand[kPackThreads / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int m = warp; m < M; m += kPackThreads / 32)
         route_token<float, NV>(logits + (int64_t)m * ld, lane, m, E_total, k, nullptr, 1, 0, ids + (int64_t)m * k,
-                               coef + (int64_t)m * k, k, router_err);
+                               coef + (int64_t)m * k, k, router_err, cand[warp]);
     __threadfence_block();
     __syncthreads();  // the ids written above are read by other threads of this CTA below
     pack_small_body(ids, L, E_total, e_lo, ep, ws, expert_err);

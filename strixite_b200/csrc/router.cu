@@ -71,10 +71,11 @@ __global__ void __launch_bounds__(kLanes *kTokensPerCta)
     router_kernel(const T *__restrict__ logits, int64_t ld, int64_t M, int E, int k, const T *__restrict__ shared,
                   int64_t shared_ld, int32_t shared_id, int32_t *__restrict__ ids, float *__restrict__ coef, int A,
                   uint32_t *err) {
+    __shared__ unsigned long long cand[kTokensPerCta][kLanes];
     const int lane = threadIdx.x % kLanes;
     const int64_t m = (int64_t)blockIdx.x * kTokensPerCta + threadIdx.x / kLanes;
     if (m >= M) return;  // whole warps leave together
-    route_token<T, NV>(logits + m * ld, lane, m, E, k, shared, shared_ld, shared_id, ids + m * A, coef + m * A, A, err);
+    route_token<T, NV>(logits + m * ld, lane, m, E, k, shared, shared_ld, shared_id, ids + m * A, coef + m * A, A, err, cand[threadIdx.x / kLanes]);
 }
 
 constexpr int kAddThreads = 256;

@@ -57,6 +57,25 @@ def test_router_ids_bit_exact(cuda, oracle, M, E, k):
     np.testing.assert_allclose(coef_b, ref_coef_b, rtol=2e-6, atol=1e-30)
 
 
+@pytest.mark.parametrize("E,k", [(1, 1), (16, 16), (31, 9), (33, 16), (512, 16), (512, 17), (1024, 16), (1000, 10)])
+@pytest.mark.parametrize("tied", [0, 31, 32, 33, 200])
+def test_router_ties_at_the_bound(cuda, oracle, E, k, tied):
+    """Picks by sorted candidates: as many logits tied at the lowest pick's value as fit the candidates beside the larger ones, one more
+    and fewer (the round-by-round picks), and signed zeros, which tie."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(E * 31 + tied)
+    logits = -rng.random((6, E + 1)).astype(np.float32) - 1
+    at = rng.permutation(E)
+    logits[:, at[: min(tied, E)]] = 0.25
+    logits[3:, at[: min(tied, E)]] = np.where(rng.random((3, min(tied, E))) < 0.5, np.float32(0.0), np.float32(-0.0))
+    top = at[min(tied, E): min(tied, E) + min(3, k - 1)]
+    logits[:, top] = 0.5 + rng.random((6, len(top))).astype(np.float32)
+    ids, coef, err = run_router(K, logits, E, k, False, cuda)
+    ref_ids, ref_coef = oracle.moe_router(logits, E, k)
+    assert err[0] == 0 and np.array_equal(ids, ref_ids)
+    np.testing.assert_allclose(coef, ref_coef, rtol=2e-6, atol=1e-30)
+
+
 def test_router_mutation_is_caught(cuda, oracle):
     """A deliberately wrong expectation must fail: guards against a comparison that passes vacuously."""
     from strixite_b200 import kernels as K
