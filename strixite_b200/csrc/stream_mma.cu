@@ -34,6 +34,7 @@
 
 #include "experts.cuh"
 #include "skinny_mma.cuh"
+#include "tc_ptx.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -166,6 +167,8 @@ struct StreamArgs {
     const float *coef;   // kPerToken
     void *out;
     uint32_t *err;
+    uint32_t *status;    // kFromWs: {2, tile, role} of a wait that ran out, in the workspace's header
+    unsigned long long wait_limit_ns;
     int chunks, split;   // see chunk_count: chunks of a contraction; warps that share a unit (1 .. chunks)
 };
 
@@ -196,23 +199,21 @@ __device__ inline void tree_push(float4 *level, int i, float (&v)[4]) {
 
 template <typename T> __device__ inline void store_out(T *p, int64_t i, float v) { store_from_f32(p, i, v); }
 
-// Stages up to 8 activation rows (rows[n] < 0 = none) as F16 in fragment order at xs, every row times its power of two
-// 2^e (token_exponent), and at xsum the sums of every (step, token) times 2^(e - 9), the factor that the dots with the codes carry.
-// kKeepLow: activations that would be subnormal are staged as zeros and listed in tok[n], which comes in cleared; *any_low = 1 where
-// there are any.  All threads of the CTA; the caller synchronizes before it reads those.
-template <int BITS, int G>
-__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok, int *any_low) {
+// Stages activation row `row` as token n of a tile: F16 in fragment order at xs, times the row's power of two 2^e (token_exponent), and at xsum the
+// sums of every step times 2^(e - 9), the factor that the dots with the codes carry.  kKeepLow: activations that would be subnormal are staged as
+// zeros and listed in tok, which comes in cleared; *any_low = 1 where there are any.  By `warps` whole warps, of which this is number `share`;
+// `meet` is the barrier between the first pass over the row and the second, and is called by every one of them (row == nullptr: no token).
+// BATCH loads in flight a lane: under a streaming kernel's load an L2 round trip is thousands of cycles.
+template <int BITS, int G, int BATCH, typename Meet>
+__device__ __forceinline__ void stage_row(const uint16_t *__restrict__ row, int K, int n, int share, int warps, uint4 *xs, float *xsum, Token &tok,
+                                          int *any_low, Meet meet) {
     using geo = Geo<BITS, G>;
     constexpr int UNITS = geo::kUnits, KI = geo::kStepCodes, CPL = geo::kCodesPerLane;
     constexpr int kStepLanes = KI / 8;  // lanes that hold one step of one token: 4, 8 or 16
-    constexpr int kBatch = 8;           // 16-byte loads a lane has in flight
-    // A token is staged by every eighth warp, so that what belongs to the token is the same for a whole warp (dealing 16-byte
-    // units out over the CTA cost two divisions a unit and an atomic a step: 150 tokens x 10 experts, 4096 x 2048 Q4, 415 ->
-    // 442 us).  Eight loads in flight: under a streaming kernel's load an L2 round trip is thousands of cycles.
-    const int lane = threadIdx.x & 31, n = (threadIdx.x >> 5) & (kTileTokens - 1), share = threadIdx.x >> 8, stride = (int)blockDim.x / kTileTokens;
+    constexpr int kBatch = BATCH;
+    const int lane = threadIdx.x & 31, stride = 32 * warps;
     const int units = K / 8;
-    const int64_t row = rows[n];
-    const uint4 *src = reinterpret_cast<const uint4 *>(x + row * K);
+    const uint4 *src = reinterpret_cast<const uint4 *>(row);
     uint4 v[kBatch];
     auto load = [&](int base) {
 #pragma unroll
@@ -220,7 +221,7 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             if (base + j * stride < units) v[j] = src[base + j * stride];
     };
     uint32_t top = 0u, low2 = 0x7fff7fffu;
-    if (row >= 0) {
+    if (row != nullptr) {
         // sum(x) of every step: eight values a lane, then a butterfly over the step's lanes
         for (int base = share * 32 + lane; base - lane < units; base += kBatch * stride) {
             load(base);
@@ -245,20 +246,20 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
             }
         }
         top = __reduce_max_sync(0xffffffffu, max(top >> 16, top & 0xffffu));
-        if (lane == 0) atomicMax(&tok[n].top, top);
+        if (lane == 0) atomicMax(&tok.top, top);
         if (kKeepLow<BITS>) {
             const int low = __reduce_min_sync(0xffffffffu, min((int)low2 >> 16, (int)(int16_t)low2));
-            if (lane == 0) atomicMin(&tok[n].low, low);
+            if (lane == 0) atomicMin(&tok.low, low);
         }
     }
-    __syncthreads();
+    meet();
     // absent tokens' columns keep whatever the memory held: a column of the products depends on its own token only, and theirs
     // are dropped
-    if (row < 0) return;
-    const int e = token_exponent(tok[n].top), smallest = kKeepLow<BITS> ? tok[n].low : 0x7fff;
+    if (row == nullptr) return;
+    const int e = token_exponent(tok.top), smallest = kKeepLow<BITS> ? tok.low : 0x7fff;
     const float f = pow2f(e);
     const bool low = smallest != 0x7fff && too_small(__uint_as_float((uint32_t)((smallest - 0x7fff) & 0xffff) << 16) * f);
-    if (lane == 0 && share == 0) tok[n].exp = e;
+    if (lane == 0 && share == 0) tok.exp = e;
     if (low) {
         int found = 0;
         for (int first = share * 32; first < units; first += stride) {
@@ -279,14 +280,14 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
                         if (((mine >> i) & 1u) && at < kLowMax)
-                            tok[n].list[share][at++] = Low{u * 8 + i, __uint_as_float((i & 1) ? w4[i >> 1] & 0xffff0000u : w4[i >> 1] << 16)};
+                            tok.list[share][at++] = Low{u * 8 + i, __uint_as_float((i & 1) ? w4[i >> 1] & 0xffff0000u : w4[i >> 1] << 16)};
                 }
                 found += __popc(theirs);
             }
         }
-        if (lane == 0 && found > 0) tok[n].n_list[share] = min(found, kLowMax), atomicAdd(&tok[n].n_low, found), *any_low = 1;
+        if (lane == 0 && found > 0) tok.n_list[share] = min(found, kLowMax), atomicAdd(&tok.n_low, found), *any_low = 1;
     }
-    // One batch holds the row up to 4096 k at 512 threads; a longer one is read again.
+    // One batch holds a row up to 256 k a load and warp; a longer one is read again.
     const bool held = units <= kBatch * stride;
     for (int base = share * 32 + lane; base < units; base += kBatch * stride) {
         if (!held) load(base);
@@ -316,32 +317,40 @@ __device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const i
     }
 }
 
-// Stages the tile's tokens with more than kLowMax small activations again, as BF16 in natural order, and their sums as they are.
+
+// Stages up to 8 activation rows (rows[n] < 0 = none), a token by every eighth warp, so that what belongs to the token is the same for a whole
+// warp (dealing 16-byte units out over the CTA cost two divisions a unit and an atomic a step: 150 tokens x 10 experts, 4096 x 2048 Q4,
+// 415 -> 442 us).  All threads of the CTA; the caller synchronizes before it reads what is staged.
 template <int BITS, int G>
-__device__ __noinline__ void stage_wide(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok) {
+__device__ inline void stage_tile(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok, int *any_low) {
+    const int n = (threadIdx.x >> 5) & (kTileTokens - 1);
+    stage_row<BITS, G, 8>(rows[n] >= 0 ? x + rows[n] * K : nullptr, K, n, threadIdx.x >> 8, (int)blockDim.x / (32 * kTileTokens), xs, xsum, tok[n], any_low,
+                       [] { __syncthreads(); });
+}
+
+// A token with more than kLowMax small activations staged again, as BF16 in natural order, and its sums as they are; by `threads` threads, of
+// which this is number t.
+template <int BITS, int G>
+__device__ __noinline__ void stage_wide(const uint16_t *__restrict__ row, int K, int n, uint4 *xs, float *xsum, Token &tok, int t, int threads) {
     using geo = Geo<BITS, G>;
     constexpr int KI = geo::kStepCodes;
-    for (int n = 0; n < kTileTokens; ++n) {
-        if (tok[n].n_low <= kLowMax) continue;
-        const uint4 *src = reinterpret_cast<const uint4 *>(x + rows[n] * K);
-        if (threadIdx.x == 0) tok[n].exp = 9;
-        for (int u = threadIdx.x; u < K / 8; u += blockDim.x) {
-            const int step = u * 8 / KI, rem = u * 8 % KI;
-            xs[(step * geo::kUnits + rem % geo::kCodesPerLane / 8) * 32 + n * 4 + rem / geo::kCodesPerLane] = src[u];
-        }
-        for (int step = threadIdx.x; step < K / KI; step += blockDim.x) {
-            float sum = 0.f;
-            for (int i = 0; i < KI; ++i) sum += bf16_bits_to_f32(x[rows[n] * K + (int64_t)step * KI + i]);
-            xsum[step * kTileTokens + n] = sum;
-        }
+    const uint4 *src = reinterpret_cast<const uint4 *>(row);
+    if (t == 0) tok.exp = 9;
+    for (int u = t; u < K / 8; u += threads) {
+        const int step = u * 8 / KI, rem = u * 8 % KI;
+        xs[(step * geo::kUnits + rem % geo::kCodesPerLane / 8) * 32 + n * 4 + rem / geo::kCodesPerLane] = src[u];
+    }
+    for (int step = t; step < K / KI; step += threads) {
+        float sum = 0.f;
+        for (int i = 0; i < KI; ++i) sum += bf16_bits_to_f32(row[(int64_t)step * KI + i]);
+        xsum[step * kTileTokens + n] = sum;
     }
 }
 // After stage_tile and a barrier, where some token has small activations.
 template <int BITS, int G>
 __device__ inline void finish_staging(const uint16_t *__restrict__ x, int K, const int64_t *rows, uint4 *xs, float *xsum, Token *tok) {
-    bool again = false;
-    for (int n = 0; n < kTileTokens; ++n) again = again || tok[n].n_low > kLowMax;
-    if (again) stage_wide<BITS, G>(x, K, rows, xs, xsum, tok);
+    for (int n = 0; n < kTileTokens; ++n)
+        if (tok[n].n_low > kLowMax) stage_wide<BITS, G>(x + rows[n] * K, K, n, xs, xsum, tok[n], threadIdx.x, blockDim.x);
     __syncthreads();
 }
 
@@ -544,6 +553,48 @@ __device__ inline void rows_dot(float (&acc)[4], const StreamArgs &a, int64_t ro
         rows_dot_fast<BITS, G, TREE>(acc, a, va ? rowa : any, vb ? rowb : any, xs, xsum, lane, part, tree);
     } else {
         rows_dot_impl<BITS, G>(acc, a, rowa, rowb, va, vb, xs, xsum, lane);
+    }
+}
+
+// A unit's dots acc -> results.  Lane (g, c) holds rows ra and rb of the expert for tokens 2c and 2c + 1 of the tile; low: some of its tokens have
+// activations too small for F16.
+template <int BITS, int G, int MODE, typename TOUT>
+__device__ __forceinline__ void finish_unit(const StreamArgs &a, TOUT *out, float (&acc)[4], int bucket, int cnt, int64_t ra, int64_t rb, bool va, bool vb,
+                                            const uint4 *xs, const float *xsum, const Token *tok, const int64_t *orows, int low) {
+    const int K = (int)a.K, c = threadIdx.x & 3;
+    const int64_t I = a.N / 2;
+    const bool valid = bucket < a.E;  // bucket E: slots with an id outside [0, E) - their outputs become NaN
+    const int64_t row0 = (int64_t)bucket * a.N;
+    const bool any_low = kKeepLow<BITS> && valid && low != 0;
+    if (any_low) {
+        bool wide[2] = {tok[2 * c].n_low > kLowMax, tok[2 * c + 1].n_low > kLowMax};
+        if (__any_sync(0xffffffffu, wide[0] || wide[1])) {
+            const float4 w = rows_dot_wide<BITS, G>(a.q, a.scale, a.minv, K, row0 + ra, row0 + rb, va, vb, xs, xsum);
+            if (wide[0]) acc[0] = w.x, acc[2] = w.z;
+            if (wide[1]) acc[1] = w.y, acc[3] = w.w;
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int n = 2 * c + t;
+        if (n >= cnt) continue;
+        const int64_t orow = orows[n];
+        const Token &token = tok[n];
+        float dot_a = unscaled(acc[t], token.exp), dot_b = unscaled(acc[2 + t], token.exp);
+        if (any_low && token.n_low > 0 && token.n_low <= kLowMax) {
+            if (va) dot_a += low_dot<BITS, G>(a.q, a.scale, K, row0 + ra, token);
+            if (vb) dot_b += low_dot<BITS, G>(a.q, a.scale, K, row0 + rb, token);
+        }
+        if (MODE == kSwiglu) {
+            if (!va) continue;
+            // kernels/linear_q4.hip:272-274: g, u as stored, h = stored(stored(silu(g)) * u)
+            const float gg = as_stored_bf16(dot_a), uu = as_stored_bf16(dot_b);
+            const float hv = as_stored_bf16(silu_f32(gg)) * uu;
+            store_out(out, orow * I + ra, valid ? hv : qnan_f32());
+        } else {
+            if (va) store_out(out, orow * a.N + ra, valid ? dot_a : qnan_f32());
+            if (vb) store_out(out, orow * a.N + rb, valid ? dot_b : qnan_f32());
+        }
     }
 }
 
@@ -765,41 +816,115 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
                 group_sync();
                 if (part != 0) continue;
             }
-            const int64_t row0 = (int64_t)bucket * a.N;
-            const bool any_low = kKeepLow<BITS> && valid && s_low[0] != 0;
-            if (any_low) {
-                bool wide[2] = {s_tok[0][2 * c].n_low > kLowMax, s_tok[0][2 * c + 1].n_low > kLowMax};
-                if (__any_sync(0xffffffffu, wide[0] || wide[1])) {
-                    const float4 w = rows_dot_wide<BITS, G>(a.q, a.scale, a.minv, K, row0 + ra, row0 + rb, va, vb, xs, xsum);
-                    if (wide[0]) acc[0] = w.x, acc[2] = w.z;
-                    if (wide[1]) acc[1] = w.y, acc[3] = w.w;
-                }
-            }
-            // Epilogue.  Lane (g, c) holds rows ra / rb for tokens 2c and 2c + 1.
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                const int n = 2 * c + t;
-                if (n >= cnt) continue;
-                const int64_t orow = s_out[n];
-                const Token &tok = s_tok[0][n];
-                float dot_a = unscaled(acc[t], tok.exp), dot_b = unscaled(acc[2 + t], tok.exp);
-                if (any_low && tok.n_low > 0 && tok.n_low <= kLowMax) {
-                    if (va) dot_a += low_dot<BITS, G>(a.q, a.scale, K, row0 + ra, tok);
-                    if (vb) dot_b += low_dot<BITS, G>(a.q, a.scale, K, row0 + rb, tok);
-                }
-                if (MODE == kSwiglu) {
-                    if (!va) continue;
-                    // kernels/linear_q4.hip:272-274: g, u as stored, h = stored(stored(silu(g)) * u)
-                    const float gg = as_stored_bf16(dot_a), uu = as_stored_bf16(dot_b);
-                    const float hv = as_stored_bf16(silu_f32(gg)) * uu;
-                    store_out(out, orow * I + ra, valid ? hv : qnan_f32());
-                } else {
-                    if (va) store_out(out, orow * a.N + ra, valid ? dot_a : qnan_f32());
-                    if (vb) store_out(out, orow * a.N + rb, valid ? dot_b : qnan_f32());
-                }
-            }
+            finish_unit<BITS, G, MODE>(a, out, acc, bucket, cnt, ra, rb, va, vb, xs, xsum, s_tok[0], s_out, s_low[0]);
         }
     }
+    }
+}
+
+// The routed forms: one CTA of sixteen warps an SM, the tiles' activations in two buffers of shared memory.  The next tile's are staged under the
+// streaming, a token by a warp - at once where the buffer is free, else after its next unit - and a warp that finds no unit left goes on to the
+// next tile by itself: no barrier of the CTA stands between two tiles.  So a CTA may begin and end inside a tile, and the units are dealt evenly.
+// Results as stream_kernel's, bit for bit: a unit's sums do not depend on who forms them.
+// What bounds it: HBM while it streams, 22 bytes a cycle and SM, 6.2 TB/s, whatever the tile; launch and first staging (8000 cycles), the last
+// units.  With one buffer and a barrier on either side of the staging, tile-aligned runs and, in small launches, CTAs of eight warps two an SM, it
+// streamed 76 to 87 % of the time.  4096 x 2048 + 1024 x 4096, 512 experts, top-10, gate/up and down us, before -> now: 16 tokens Q4 130 + 70 -> 121 + 63,
+// 37 tokens (Q8 down) 207 + 167 -> 184 + 158, 150 tokens 424 + 234 -> 384 + 211; the layer as a graph, 2 tokens 83.5 -> 67.5, 4 109 -> 90, 64 552 -> 495.
+// The staging's loads are four at a time and inline: with eight or sixteen in flight, or as a call, the loop over a unit's codes lost registers to
+// them (16 tokens 126 + 65; as a call 200 + 89).
+// Every wait is bounded; one that runs out is recorded in the grouping workspace's status words and ends the warp.
+constexpr int kTileBufs = 2, kBigWarps = kBigThreads / 32;
+struct TileBuf {
+    int64_t row[kTileTokens], out[kTileTokens];  // activation and output row of each token, -1 = none
+    Token tok[kTileTokens];
+    int bucket, cnt, next;  // next: the next unit of the CTA's run that no warp has taken yet
+};
+// A token of the next tile, by one warp.
+template <int BITS, int G>
+__device__ __forceinline__ void stage_token(const uint16_t *row, int K, int n, uint4 *xs, float *xsum, Token *tok) {
+    int any_low = 0;
+    stage_row<BITS, G, 4>(row, K, n, 0, 1, xs, xsum, *tok, &any_low, [] { __syncwarp(); });
+    __syncwarp();
+    if (kKeepLow<BITS> && tok->n_low > kLowMax) stage_wide<BITS, G>(row, K, n, xs, xsum, *tok, threadIdx.x & 31, 32);
+}
+template <int BITS, int G, int MODE, typename TOUT>
+__global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const StreamArgs a) {
+    using geo = Geo<BITS, G>;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ TileBuf bufs[kTileBufs];
+    __shared__ int s_low;  // some token of the first tile has activations too small for F16
+    __shared__ uint64_t staged[kTileBufs], left[kTileBufs];  // a buffer's tile is staged (a warp a token) / every warp has left it
+    const int K = (int)a.K, steps = K / geo::kStepCodes, xs_bytes = steps * geo::kUnits * 512, pass_bytes = xs_bytes + steps * kTileTokens * 4;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2;
+    const int I = (int)(a.N / 2), units_per_tile = MODE == kSwiglu ? (I + 7) / 8 : (int)((a.N + 15) / 16);
+    TOUT *out = static_cast<TOUT *>(a.out);
+    // the CTA's run of units: from unit u0 of tile0 to before unit u1 of tile1
+    const int64_t total = (int64_t)a.ws[0] * units_per_tile, begin = total * blockIdx.x / gridDim.x, end = total * (blockIdx.x + 1) / gridDim.x;
+    if (begin >= end) return;
+    const int tile0 = (int)(begin / units_per_tile), tile1 = (int)((end - 1) / units_per_tile);
+    const int u0 = (int)(begin - (int64_t)tile0 * units_per_tile), u1 = (int)(end - (int64_t)tile1 * units_per_tile);
+
+    auto xs_of = [&](int b) { return reinterpret_cast<uint4 *>(smem + b * pass_bytes); };
+    auto xsum_of = [&](int b) { return reinterpret_cast<float *>(smem + b * pass_bytes + xs_bytes); };
+    // Token n of tile `tile`; n == 0 also describes the tile.
+    auto describe = [&](TileBuf &t, int tile, int n) {
+        const int bucket = a.ws[a.L.t8_bucket + tile], start = a.ws[a.L.t8_start + tile];
+        const int cnt = min(kTileTokens, a.ws[a.L.offsets + bucket + 1] - start);
+        int64_t row = -1, orow = -1;
+        if (n < cnt) orow = a.ws[a.L.slots + start + n], row = MODE == kPartial ? orow : orow / a.A;
+        t.row[n] = bucket < a.E ? row : -1, t.out[n] = orow, clear_token(t.tok[n]);
+        if (n == 0) t.bucket = bucket, t.cnt = cnt, t.next = tile == tile0 ? u0 : 0;
+    };
+    if (threadIdx.x < kTileTokens) describe(bufs[0], tile0, threadIdx.x);
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < kTileBufs; ++b) mbar_init(&staged[b], kTileTokens), mbar_init(&left[b], kBigWarps);
+        s_low = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    stage_tile<BITS, G>(a.x, K, bufs[0].row, xs_of(0), xsum_of(0), bufs[0].tok, &s_low);
+    __syncthreads();
+    if (kKeepLow<BITS> && s_low) finish_staging<BITS, G>(a.x, K, bufs[0].row, xs_of(0), xsum_of(0), bufs[0].tok);
+
+    auto wait = [&](uint64_t *bar, uint32_t parity, int tile) {
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, nullptr, a.wait_limit_ns));
+        if (!ok && lane == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) a.status[1] = (uint32_t)tile, a.status[2] = 8u;
+        return ok;
+    };
+    for (int tile = tile0; tile <= tile1; ++tile) {
+        const int j = tile - tile0, b = j & 1;
+        const uint32_t turn = (uint32_t)((j - 1) >> 1) & 1u;  // of this tile's `staged` and of the last one's `left`
+        TileBuf &t = bufs[b];
+        if (j > 0 && !wait(&staged[b], turn, tile)) return;
+        const int low = kKeepLow<BITS> && __any_sync(0xffffffffu, t.tok[lane & (kTileTokens - 1)].n_low != 0);
+        const int hi = tile == tile1 ? u1 : units_per_tile;
+        bool to_stage = tile < tile1 && warp < kTileTokens;
+        for (bool again = false;; again = true) {
+            if (to_stage && (again || j == 0 || __all_sync(0xffffffffu, mbar_test(&left[b ^ 1], turn)))) {
+                to_stage = false;
+                TileBuf &n = bufs[b ^ 1];
+                if (j > 0 && !wait(&left[b ^ 1], turn, tile)) return;
+                if (lane == 0) describe(n, tile + 1, warp);
+                __syncwarp();
+                if (n.row[warp] >= 0) stage_token<BITS, G>(a.x + n.row[warp] * K, K, warp, xs_of(b ^ 1), xsum_of(b ^ 1), &n.tok[warp]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&staged[b ^ 1]);
+            }
+            int u = 0;
+            if (lane == 0) u = atomicAdd(&t.next, 1);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if (u < hi) {
+                const int bucket = t.bucket, ra = MODE == kSwiglu ? u * 8 + g : u * 16 + g, rb = MODE == kSwiglu ? I + ra : ra + 8;
+                const bool va = MODE == kSwiglu ? ra < I : ra < (int)a.N, vb = MODE == kSwiglu ? va : ra < (int)a.N - 8;
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+                if (bucket < a.E)
+                    rows_dot<BITS, G, false>(acc, a, (int64_t)bucket * a.N + ra, (int64_t)bucket * a.N + rb, va, vb, xs_of(b), xsum_of(b), lane, 0, nullptr);
+                finish_unit<BITS, G, MODE>(a, out, acc, bucket, t.cnt, ra, rb, va, vb, xs_of(b), xsum_of(b), t.tok, t.out, low);
+            }
+            if (u >= hi && !to_stage) break;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&left[b]);
     }
 }
 
@@ -939,6 +1064,16 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     if (args.split > 1) {
         kern<<<(unsigned)std::min<int64_t>(sm_count(), est_units), kBigThreads, smem, st>>>(args);
         return SXB_OK;
+    }
+    // Routed tiles of a grouping workspace; rows too long for two buffers go on below.
+    if constexpr (SRC == kFromWs) {
+        if (kTileBufs * smem <= kMaxDynSmem) {
+            auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
+            SXB_CUDA(cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
+            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = wait_limit_ns();
+            tiles<<<(unsigned)sm_count(), kBigThreads, kTileBufs * smem, st>>>(args);
+            return SXB_OK;
+        }
     }
     // One CTA of sixteen warps an SM when there are several units for every warp of the machine; otherwise CTAs of eight
     // warps, two an SM where their shared memory allows, and never more CTAs than one per unit and warp.

@@ -293,6 +293,37 @@ def test_per_slot_experts(cuda, oracle, bits, G, M, A, E, N, Kd):
             K.check_expert_error(err, "combine")
 
 
+@pytest.mark.parametrize("bits,G,E,N,Kd", [(4, 128, 5, 48, 512), (8, 64, 7, 272, 256), (4, 32, 3, 2064, 128), (8, 128, 40, 16, 1024), (4, 128, 6, 64, 8192),
+                                           (8, 64, 3, 400, 5760)])
+@pytest.mark.parametrize("M,A", [(1, 2), (17, 3), (200, 2), (900, 1)])
+def test_grouped_tiles_equal_slots(cuda, oracle, bits, G, E, N, Kd, M, A):
+    """The grouped exact forms against the per-slot ones, bit for bit: runs of units that begin and end inside tiles, tiles of 1 to 8 tokens,
+    experts without any and with an id out of range, fewer units than CTAs, rows too long for two buffers, a token with small activations."""
+    from strixite_b200 import kernels as Kn
+    rng = np.random.default_rng(M * 7 + N)
+    w = upload(oracle.quantize(random_weights(rng, E * N, Kd), G, bits), cuda)
+    x = rng.standard_normal((M, Kd)).astype(np.float32)
+    x[M // 2, :3] = 2.0 ** -34   # beside the largest too small for F16: kept apart
+    x[M // 3, :9] = 2.0 ** -36   # more of them than are
+    xd = bf16_tensor(oracle.f32_to_bf16(x), cuda)
+    ids = torch.from_numpy(np.minimum(rng.geometric(0.4, (M, A)) - 1, E - 1).astype(np.int32)).to(cuda)
+    if M > 1:
+        ids[M - 1, 0] = E
+    err = torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = Kn.moe_route_workspace_bytes(M, A, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    Kn.moe_group_routes(ids, M, A, E, ws, nbytes, err)
+    for swiglu in (False, True):
+        out = [torch.zeros((M * A, N // 2 if swiglu else N), dtype=torch.bfloat16, device=cuda) for _ in range(2)]
+        slots, grouped = ((Kn.linear_qw_experts_gather_swiglu, Kn.linear_qw_experts_gather_grouped_swiglu) if swiglu
+                          else (Kn.linear_qw_experts_gather, Kn.linear_qw_experts_gather_grouped))
+        slots(xd, w, E, ids, M, A, out[0], Kn.Act.BF16, err)
+        grouped(xd, w, E, ws, nbytes, M, A, out[1], Kn.Act.BF16, Kn.MoeMath.F32)
+        torch.cuda.synchronize()
+        Kn.check_grouped_status(ws, "grouped tiles")
+        assert torch.equal(out[0].view(torch.int16), out[1].view(torch.int16))
+
+
 @pytest.mark.parametrize("bits,G", [(4, 128), (8, 64)])
 @pytest.mark.parametrize("M,A,E,I,d", [(16, 10, 64, 128, 512), (37, 4, 16, 64, 256), (300, 2, 8, 64, 256)])
 def test_grouped_experts_exact_math(cuda, oracle, bits, G, M, A, E, I, d):
