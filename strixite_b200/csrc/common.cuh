@@ -61,6 +61,22 @@ inline bool aligned16(const void *p) { return reinterpret_cast<uintptr_t>(p) % 1
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// A launch whose CTAs may take their places, and wait there, while the kernel ahead of it in the stream still runs: the gap between two
+// dependent kernels, one to two microseconds, is most of some of the decode chain's.  The kernel calls behind_grid() before it touches memory.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_behind(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, Args &&...args) {
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension, attr[1].val.clusterDim.x = (unsigned)cluster, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+
+// First statement of a kernel that is launched by launch_behind (by any launch: with nothing ahead it passes): the grid ahead has ended and its
+// results, and with it those of every grid ahead of it, are visible; and the next one may come in behind this one's CTAs, all of which run.
+__device__ inline void behind_grid() { asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- device helpers ---------------------------------------------------------------------------------------------
 __host__ __device__ inline float bf16_bits_to_f32(uint16_t b) {
 #ifdef __CUDA_ARCH__

@@ -147,6 +147,7 @@ template <int MT, int NT, typename TOUT>
 __global__ void __launch_bounds__(32 * kDenseWarps, 2)
     dense_mma_kernel(const uint16_t *__restrict__ x, const uint8_t *__restrict__ q, const uint16_t *__restrict__ scale,
                      const uint16_t *__restrict__ minv, int64_t M, int64_t N, int64_t K, int64_t G, TOUT *__restrict__ y) {
+    behind_grid();
     constexpr int kTok = kMmaTokens * NT, kRowsCta = kMmaRows * MT;
     constexpr int kAhead = MT == 2 || NT == 4 ? 4 : 8;           // runs whose codes a lane has in flight
     constexpr int kActs = NT == 4 ? 1 : (NT == 2 ? 2 : 4) / MT;  // ... whose activations
@@ -428,7 +429,7 @@ int dense_q8(const char *fn, const void *x, const SxbQView *w, void *y, int64_t 
     const dim3 grid((unsigned)((w->N + kMmaRows * MT - 1) / (kMmaRows * MT)), (unsigned)token_groups);  // at most 16384: 524280 rows of x, 32 a CTA
     auto go = [&](auto *yt) {
         using T = std::remove_pointer_t<decltype(yt)>;
-#define SXB_DENSE(MTV, NTV) dense_mma_kernel<MTV, NTV, T><<<grid, 32 * kDenseWarps, 0, st>>>(xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt)
+#define SXB_DENSE(MTV, NTV) launch_behind(dense_mma_kernel<MTV, NTV, T>, grid, 32 * kDenseWarps, 0, st, 1, xb, w->q, w->scale, w->minv, M, w->N, w->K, w->G, yt)
         if (NT == 4) SXB_DENSE(1, 4);
         else if (NT == 2 && MT == 1) SXB_DENSE(1, 2);
         else if (NT == 2) SXB_DENSE(2, 2);

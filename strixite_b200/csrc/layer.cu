@@ -102,6 +102,17 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
     SXB_CHECK(!tc || a->xs != nullptr, fn, ": the tcgen05 path needs the tile-blocked activation buffer xs (M * A * d F16)");
     auto st = static_cast<cudaStream_t>(stream);
 
+    // The shared expert as dense projections (runtime/qwen4exp.cpp:3163-3168), in y's dtype.  On the streaming kernels its stream goes its own way from
+    // before the router, which it does not need and whose one CTA leaves the machine to it; its launches are issued after the router's, on which the
+    // rest of the layer waits.
+    SideWork beside(st, static_cast<cudaStream_t>(side));
+    if (shared) {
+        SXB_CHECK(a->sh_h != nullptr && a->sh_y != nullptr, fn, ": null shared-expert buffer");
+        SXB_CHECK(tc || a->sh_gu != nullptr, fn, ": null shared-expert buffer sh_gu");
+        SXB_CHECK(!tc || a->sh_xs != nullptr, fn, ": null shared-expert buffer sh_xs for the tcgen05 path");
+    }
+    if (shared && !tc && side != stream) SXB_CUDA(beside.fork(), fn, ": starting the shared expert's stream");
+
     // router (kernels/moe_router.hpp:38-40): top-k of the first E_total logits; a shared expert's gate is column E_total.
     // logits == NULL: ids and coef already hold the routes (an expert-parallel rank receives them from the tokens' owners)
     // A small batch (decode) routes and packs in one launch.
@@ -117,32 +128,25 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
             return rc;
     }
 
-    // the shared expert as dense projections (runtime/qwen4exp.cpp:3163-3168), in y's dtype
-    SideWork beside(st, static_cast<cudaStream_t>(side));
-    if (shared) {
-        SXB_CHECK(a->sh_h != nullptr && a->sh_y != nullptr, fn, ": null shared-expert buffer");
-        if (!tc) {
-            SXB_CHECK(a->sh_gu != nullptr, fn, ": null shared-expert buffer sh_gu");
-            if (side != stream) SXB_CUDA(beside.fork(), fn, ": starting the shared expert's stream");
-            if (int rc = linear_dense(a->shared_bits, a->x, a->shared_gate_up, a->sh_gu, M, SXB_ACT_BF16, SXB_ACT_BF16, side)) return rc;
-            if (int rc = sxb_swiglu(a->sh_gu, a->sh_h, M, I, SXB_ACT_BF16, side)) return rc;
-            if (int rc = linear_dense(a->shared_bits, a->sh_h, a->shared_down, a->sh_y, M, SXB_ACT_BF16, a->out_act, side)) return rc;
-        } else {
-            // dense projections on the tcgen05 kernel (kernels/linear_wmma.hip:69-113), SwiGLU fused into the first;
-            // a wait that ran out is recorded in the routed experts' workspace header, like theirs
-            SXB_CHECK(a->sh_xs != nullptr, fn, ": null shared-expert buffer sh_xs for the tcgen05 path");
-            uint32_t *status = reinterpret_cast<uint32_t *>(a->ws) + 5;
-            if (int rc = sxb_stage_f16_tiles(a->x, nullptr, 0, M, 1, 1, d, a->shared_bits, a->sh_xs, stream)) return rc;
-            const int hf = a->shared_bits == 4 ? 3 : 4;
-            const int of = a->out_act == SXB_ACT_F32 ? 1 : 0;
-            int rc = a->shared_bits == 4
-                         ? tc_dense<4>(fn, a->sh_xs, a->shared_gate_up, a->sh_h, M, 3, 2, hf, status, stream)
-                         : tc_dense<8>(fn, a->sh_xs, a->shared_gate_up, a->sh_h, M, 3, 2, hf, status, stream);
-            if (rc) return rc;
-            rc = a->shared_bits == 4 ? tc_dense<4>(fn, a->sh_h, a->shared_down, a->sh_y, M, 3, of, 0, status, stream)
-                                     : tc_dense<8>(fn, a->sh_h, a->shared_down, a->sh_y, M, 3, of, 0, status, stream);
-            if (rc) return rc;
-        }
+    if (shared && !tc) {
+        if (int rc = linear_dense(a->shared_bits, a->x, a->shared_gate_up, a->sh_gu, M, SXB_ACT_BF16, SXB_ACT_BF16, side)) return rc;
+        if (int rc = sxb_swiglu(a->sh_gu, a->sh_h, M, I, SXB_ACT_BF16, side)) return rc;
+        if (int rc = linear_dense(a->shared_bits, a->sh_h, a->shared_down, a->sh_y, M, SXB_ACT_BF16, a->out_act, side)) return rc;
+    }
+    if (shared && tc) {
+        // dense projections on the tcgen05 kernel (kernels/linear_wmma.hip:69-113), SwiGLU fused into the first;
+        // a wait that ran out is recorded in the routed experts' workspace header, like theirs
+        uint32_t *status = reinterpret_cast<uint32_t *>(a->ws) + 5;
+        if (int rc = sxb_stage_f16_tiles(a->x, nullptr, 0, M, 1, 1, d, a->shared_bits, a->sh_xs, stream)) return rc;
+        const int hf = a->shared_bits == 4 ? 3 : 4;
+        const int of = a->out_act == SXB_ACT_F32 ? 1 : 0;
+        int rc = a->shared_bits == 4
+                     ? tc_dense<4>(fn, a->sh_xs, a->shared_gate_up, a->sh_h, M, 3, 2, hf, status, stream)
+                     : tc_dense<8>(fn, a->sh_xs, a->shared_gate_up, a->sh_h, M, 3, 2, hf, status, stream);
+        if (rc) return rc;
+        rc = a->shared_bits == 4 ? tc_dense<4>(fn, a->sh_h, a->shared_down, a->sh_y, M, 3, of, 0, status, stream)
+                                 : tc_dense<8>(fn, a->sh_h, a->shared_down, a->sh_y, M, 3, of, 0, status, stream);
+        if (rc) return rc;
     }
 
     // pack (kernels/moe_grouped.hpp:53-54)

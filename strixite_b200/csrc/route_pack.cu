@@ -184,6 +184,7 @@ __device__ void pack_small_body(const int32_t *__restrict__ ids, const RouteWord
 __global__ void __launch_bounds__(kPackThreads)
     pack_small_kernel(const int32_t *__restrict__ ids, RouteWords L, int E_total, int e_lo, bool ep, int32_t *ws,
                       uint32_t *err) {
+    behind_grid();
     pack_small_body(ids, L, E_total, e_lo, ep, ws, err);
 }
 
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(kPackThreads)
     route_small_kernel(const float *__restrict__ logits, int64_t ld, int M, int E_total, int k, int32_t *__restrict__ ids,
                        float *__restrict__ coef, RouteWords L, int e_lo, bool ep, int32_t *ws, uint32_t *router_err,
                        uint32_t *expert_err) {
+    behind_grid();
     __shared__ unsigned long long cand[kPackThreads / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int m = warp; m < M; m += kPackThreads / 32)
@@ -323,7 +325,7 @@ int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64
     auto st = static_cast<cudaStream_t>(stream);
     auto *w = static_cast<int32_t *>(ws);
     if (L.S <= kSmallSlots) {
-        pack_small_kernel<<<1, kPackThreads, 0, st>>>(ids, L, (int)E_total, (int)e_lo, ep, w, err);
+        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, err);
     } else {
         const unsigned ctas = (unsigned)L.nseg;
         pack_hist_kernel<<<ctas, 32 * kSegWarps, 0, st>>>(ids, L, (int)E_total, (int)e_lo, w);
@@ -461,12 +463,12 @@ int sxb_moe_route_small(const float *logits, int64_t ld, int64_t M, int64_t E_to
     // machine (150 tokens x 512 experts, top-10: 87 us as one launch).
     if (M > kPackThreads / 32) {
         if (int rc = sxb_moe_router(logits, ld, M, E_total, k, nullptr, 1, 0, ids, coef, SXB_ACT_F32, router_err, stream)) return rc;
-        pack_small_kernel<<<1, kPackThreads, 0, st>>>(ids, L, (int)E_total, (int)e_lo, ep, w, expert_err);
+        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, expert_err);
         SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
         return SXB_OK;
     }
 #define SXB_ROUTE_SMALL(NV) \
-    route_small_kernel<NV><<<1, kPackThreads, 0, st>>>(logits, ld, (int)M, (int)E_total, (int)k, ids, coef, L, (int)e_lo, ep, w, router_err, expert_err)
+    launch_behind(route_small_kernel<NV>, 1, kPackThreads, 0, st, 1, logits, ld, (int)M, (int)E_total, (int)k, ids, coef, L, (int)e_lo, ep, w, router_err, expert_err)
     if (E_total <= 128) SXB_ROUTE_SMALL(4);
     else if (E_total <= 256) SXB_ROUTE_SMALL(8);
     else if (E_total <= 512) SXB_ROUTE_SMALL(16);

@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kLanes *kTokensPerCta)
     router_kernel(const T *__restrict__ logits, int64_t ld, int64_t M, int E, int k, const T *__restrict__ shared,
                   int64_t shared_ld, int32_t shared_id, int32_t *__restrict__ ids, float *__restrict__ coef, int A,
                   uint32_t *err) {
+    behind_grid();
     __shared__ unsigned long long cand[kTokensPerCta][kLanes];
     const int lane = threadIdx.x % kLanes;
     const int64_t m = (int64_t)blockIdx.x * kTokensPerCta + threadIdx.x / kLanes;
@@ -154,7 +155,7 @@ int sxb_moe_router(const void *logits, int64_t ld, int64_t M, int64_t E, int64_t
     const dim3 grid((unsigned)((M + kTokensPerCta - 1) / kTokensPerCta)), block(kLanes * kTokensPerCta);
     auto st = static_cast<cudaStream_t>(stream);
 #define SXB_ROUTER(T, NV)                                                                                         \
-    router_kernel<T, NV><<<grid, block, 0, st>>>(static_cast<const T *>(logits), ld, M, (int)E, (int)k,            \
+    launch_behind(router_kernel<T, NV>, grid, block, 0, st, 1, static_cast<const T *>(logits), ld, M, (int)E, (int)k,            \
                                                  static_cast<const T *>(shared_logit), shared_ld, shared_id, ids, \
                                                  coef, A, err)
 #define SXB_ROUTER_NV(T)                 \

@@ -107,6 +107,7 @@ template <typename TW, typename TOUT, int NT>
 __global__ void __launch_bounds__(32 * kStreamWarps, 2)
     logits_stream_kernel(const uint16_t *__restrict__ x, const TW *__restrict__ w, const float *__restrict__ bias, int64_t M,
                          int64_t N, int64_t K, TOUT *__restrict__ y, int64_t ld) {
+    behind_grid();
     constexpr int kTok = kMmaTokens * NT, kAhead = Weights<TW>::kAhead, P = Weights<TW>::kPlanes;
     __shared__ float part[kStreamWarps][kTok][kMmaRows + 1];
     __shared__ float cta_part[kTok][kMmaRows];
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 2)
 template <typename TY>
 __global__ void __launch_bounds__(256) residual_add_kernel(const uint4 *__restrict__ x, const TY *__restrict__ y, uint4 *__restrict__ out,
                                                            int64_t chunks) {
+    behind_grid();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < chunks; i += (int64_t)gridDim.x * blockDim.x) {
         const uint4 xv = x[i];
         const uint32_t u[4] = {xv.x, xv.y, xv.z, xv.w};
@@ -496,13 +498,9 @@ template <typename TOUT>
 int launch_stream_logits(const char *fn, const void *x, const void *w, int w_act, const float *bias, int64_t M, int64_t N, int64_t K,
                          TOUT *y, int64_t ld, cudaStream_t st) {
     const int NT = M <= kMmaTokens ? 1 : 2;  // eights of tokens a CTA takes; a second group's weights come from L2
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension, attr.val.clusterDim.x = kStreamSplit, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)((N + kMmaRows - 1) / kMmaRows * kStreamSplit), (unsigned)std::min<int64_t>((M + NT * kMmaTokens - 1) / (NT * kMmaTokens), 65535));
-    cfg.blockDim = dim3(32 * kStreamWarps), cfg.stream = st, cfg.attrs = &attr, cfg.numAttrs = 1;
+    const dim3 grid((unsigned)((N + kMmaRows - 1) / kMmaRows * kStreamSplit), (unsigned)std::min<int64_t>((M + NT * kMmaTokens - 1) / (NT * kMmaTokens), 65535));
     auto xb = static_cast<const uint16_t *>(x);
-    auto launch = [&](auto kern, auto *wt) { return cudaLaunchKernelEx(&cfg, kern, xb, wt, bias, M, N, K, y, ld); };
+    auto launch = [&](auto kern, auto *wt) { return launch_behind(kern, grid, dim3(32 * kStreamWarps), 0, st, kStreamSplit, xb, wt, bias, M, N, K, y, ld); };
     cudaError_t e;
     if (w_act == SXB_ACT_F32) {
         auto wt = static_cast<const float *>(w);
@@ -613,8 +611,8 @@ int sxb_residual_add(const void *x, const void *y, int y_act, void *out, int64_t
     const int64_t chunks = n / 8;
     const unsigned blocks = (unsigned)std::min<int64_t>((chunks + 255) / 256, (int64_t)sm_count() * 8);
     auto st = static_cast<cudaStream_t>(stream);
-    if (y_act == SXB_ACT_F32) residual_add_kernel<float><<<blocks, 256, 0, st>>>((const uint4 *)x, (const float *)y, (uint4 *)out, chunks);
-    else residual_add_kernel<uint16_t><<<blocks, 256, 0, st>>>((const uint4 *)x, (const uint16_t *)y, (uint4 *)out, chunks);
+    if (y_act == SXB_ACT_F32) launch_behind(residual_add_kernel<float>, blocks, 256, 0, st, 1, (const uint4 *)x, (const float *)y, (uint4 *)out, chunks);
+    else launch_behind(residual_add_kernel<uint16_t>, blocks, 256, 0, st, 1, (const uint4 *)x, (const uint16_t *)y, (uint4 *)out, chunks);
     SXB_CHECK_LAUNCH(fn, " n=", n);
     return SXB_OK;
 }

@@ -600,6 +600,7 @@ __device__ __forceinline__ void finish_unit(const StreamArgs &a, TOUT *out, floa
 
 template <int BITS, int G, int MODE, int SRC, typename TOUT>
 __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs a) {
+    behind_grid();
     using geo = Geo<BITS, G>;
     const int kWarps = (int)blockDim.x >> 5;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -849,6 +850,7 @@ __device__ __forceinline__ void stage_token(const uint16_t *row, int K, int n, u
 }
 template <int BITS, int G, int MODE, typename TOUT>
 __global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const StreamArgs a) {
+    behind_grid();
     using geo = Geo<BITS, G>;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ TileBuf bufs[kTileBufs];
@@ -982,6 +984,7 @@ __global__ void __launch_bounds__(256)
                           int64_t M, int64_t A, int64_t E_total, int64_t e_lo, int64_t E_local, int64_t N,
                           TOUT *__restrict__ y, const TS *__restrict__ s, const float *__restrict__ gate_logit,
                           int64_t gate_ld, uint32_t gate_index, uint32_t *err) {
+    behind_grid();
     const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (i >= M * N) return;
     const int64_t m = i / N, n = i % N;  // N % 4 == 0: the four columns lie in one row
@@ -1062,7 +1065,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     if (SRC == kDense)
         while (args.split * 2 <= args.chunks && est_units * args.split * 4 <= machine_warps * 5) args.split *= 2;
     if (args.split > 1) {
-        kern<<<(unsigned)std::min<int64_t>(sm_count(), est_units), kBigThreads, smem, st>>>(args);
+        launch_behind(kern, (unsigned)std::min<int64_t>(sm_count(), est_units), kBigThreads, smem, st, 1, args);
         return SXB_OK;
     }
     // Routed tiles of a grouping workspace; rows too long for two buffers go on below.
@@ -1071,7 +1074,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
             auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
             SXB_CUDA(cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
             args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = wait_limit_ns();
-            tiles<<<(unsigned)sm_count(), kBigThreads, kTileBufs * smem, st>>>(args);
+            launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
             return SXB_OK;
         }
     }
@@ -1084,7 +1087,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     const int per_sm = big || smem > (SRC == kDense ? 88 : 100) * 1024 ? 1 : 2;
     int64_t grid = (int64_t)sm_count() * per_sm;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (est_units + warps - 1) / warps));
-    kern<<<(unsigned)grid, threads, smem, st>>>(args);
+    launch_behind(kern, (unsigned)grid, threads, smem, st, 1, args);
     return SXB_OK;
 }
 

@@ -17,6 +17,7 @@ template <> struct Vec<uint16_t> { static constexpr int n = 8; };
 
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(kThreads) swiglu_kernel(const T *__restrict__ gu, T *__restrict__ h, int64_t n, int64_t I) {
+    behind_grid();
     constexpr int V = VEC ? Vec<T>::n : 1;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * V; i < n; i += (int64_t)gridDim.x * blockDim.x * V) {
         const int64_t r = i / I, j = i % I;
@@ -57,11 +58,11 @@ extern "C" int sxb_swiglu(const void *gu, void *h, int64_t rows, int64_t I, int 
     auto st = static_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)std::max<int64_t>(blocks, 1));
     if (act == SXB_ACT_F32) {
-        if (vec) swiglu_kernel<float, true><<<grid, kThreads, 0, st>>>((const float *)gu, (float *)h, n, I);
-        else swiglu_kernel<float, false><<<grid, kThreads, 0, st>>>((const float *)gu, (float *)h, n, I);
+        if (vec) launch_behind(swiglu_kernel<float, true>, grid, kThreads, 0, st, 1, (const float *)gu, (float *)h, n, I);
+        else launch_behind(swiglu_kernel<float, false>, grid, kThreads, 0, st, 1, (const float *)gu, (float *)h, n, I);
     } else {
-        if (vec) swiglu_kernel<uint16_t, true><<<grid, kThreads, 0, st>>>((const uint16_t *)gu, (uint16_t *)h, n, I);
-        else swiglu_kernel<uint16_t, false><<<grid, kThreads, 0, st>>>((const uint16_t *)gu, (uint16_t *)h, n, I);
+        if (vec) launch_behind(swiglu_kernel<uint16_t, true>, grid, kThreads, 0, st, 1, (const uint16_t *)gu, (uint16_t *)h, n, I);
+        else launch_behind(swiglu_kernel<uint16_t, false>, grid, kThreads, 0, st, 1, (const uint16_t *)gu, (uint16_t *)h, n, I);
     }
     SXB_CHECK_LAUNCH("swiglu ", act_name(act), " rows=", rows, " I=", I);
     return SXB_OK;

@@ -289,3 +289,52 @@ def test_one_call_layer_equals_the_launch_sequence(cuda, name, T, tc, shared):
         assert torch.equal(b2.ids, buf.ids)
         assert torch.equal(got.view(torch.int32 if dt == torch.float32 else torch.int16),
                            want.view(torch.int32 if dt == torch.float32 else torch.int16)), f"{cfg.name} {dt}"
+
+
+@pytest.mark.parametrize("T", [1, 16, 40])
+@pytest.mark.parametrize("captured", [False, True])
+def test_inputs_written_just_before(cuda, T, captured):
+    """A decode step whose activations the work right ahead of it writes, late: launches that come in behind their predecessors wait for their
+    results, on the second stream of the shared expert too, and pass after pass without a host in between."""
+    from strixite_b200 import kernels as K
+    from strixite_b200.layer import MoeBuffers, MoeLayer, MoeWeights
+    E, A, d, I = 16, 4, 1024, 256
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q = lambda rows, cols, bits: K.quantize(torch.randn((rows, cols), generator=g, device=cuda) * 0.05, 64, bits)
+    w = MoeWeights(q(E * 2 * I, d, 4), q(E * d, I, 4), q(2 * I, d, 8), q(d, I, 8))
+    wr = torch.randn((E + 1, d), generator=g, device=cuda) * 0.05
+    x, x_out = torch.zeros((T, d), dtype=torch.bfloat16, device=cuda), torch.zeros((T, d), dtype=torch.bfloat16, device=cuda)
+    logits, y = torch.zeros((T, E + 1), device=cuda), torch.zeros((T, d), device=cuda)
+    layer = MoeLayer(w, E, A, MoeBuffers(T, d, I, E, A, cuda, True))
+    big = torch.randn((4096, 4096), generator=g, device=cuda)
+    inputs = [torch.randn((T, d), generator=g, device=cuda).to(torch.bfloat16) for _ in range(6)]
+    src = torch.zeros_like(x)
+
+    def step():
+        late = (big @ big)[0, 0] * 0           # some hundred microseconds ahead of the write
+        x.copy_(src + late.to(torch.bfloat16))
+        K.router_logits(x, wr, None, logits)
+        layer.forward(x, logits, y)
+        K.residual_add(x, y, x_out)
+
+    want = []
+    for i in inputs:
+        src.copy_(i)
+        step()
+        torch.cuda.synchronize()
+        want.append((x_out.clone(), y.clone()))
+    run = step
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            step()
+        run = graph.replay
+    got = []
+    for i in inputs:
+        src.copy_(i)
+        run()
+        got.append((x_out.clone(), y.clone()))
+    torch.cuda.synchronize()
+    layer.check_errors()
+    for (a, b), (c, e) in zip(want, got):
+        assert torch.equal(a, c) and torch.equal(b, e)
