@@ -18,12 +18,11 @@
 // The re-layouts of the two weights (a few MB) are done per call into the caller's workspace: the views an engine holds
 // stay the reference's (row-major folded down weight, chunk-major up weight), shared with the per-token kernels.
 
-#include "experts.cuh"
-#include "route_pack.cuh"
-#include "tc_ptx.cuh"
+#include "grouped_tc.cuh"
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace sxb {
 namespace {
@@ -216,6 +215,302 @@ __global__ void __launch_bounds__(256) hc_stage_h_kernel(const float *__restrict
     }
 }
 
+// ---- up, ranks up to 512: a kernel of its own ------------------------------------------------------------------------
+
+// z = h W_up^T and the stream combine for 128 rows of W_up - 32 output columns, their four streams in neighbouring tensor-memory lanes (up_source_row) -
+// against up to 128 tokens an item.  The contraction is short (r = 320: three steps of 128 k), so what an item costs is everything but its products: on
+// the general kernel, whose items dequantize their rows again for every 128 tokens, look for their powers of two and pass through its rings,
+// 11200 SM cycles, of which the MMAs take 1500.  Here a CTA takes neighbouring items, the tokens of a row block one after another, and the
+// block's weights stay in tensor memory: dequantized once or twice a CTA, straight from the chunk-major codes.
+// Warps: sixteen for the epilogue (a lane quadrant and 32 of an item's tokens each), four producers, MMA issue, activation copies.  Waits are
+// bounded; one that runs out raises the CTA's abort flag and is recorded in the library's status words.
+constexpr int kUpTile = 128, kUpSubBytes = kUpTile * 128, kUpStageBytes = 2 * kUpSubBytes, kUpSteps = 4;  // steps of 128 k at most
+constexpr int kUpEpiWarps = 16, kUpProducer = kUpEpiWarps, kUpMma = kUpEpiWarps + 4, kUpCopy = kUpEpiWarps + 5, kUpThreads = 32 * (kUpEpiWarps + 6);
+constexpr int kUpACols = 256;   // first tensor-memory column of the weights, behind two accumulators of 128
+constexpr int kUpScaleBufs = 4; // row blocks whose powers of two are kept: the epilogue is two accumulators behind at most
+template <typename TX> constexpr int kUpBuf = 128 * 8 * (int)sizeof(TX) + 32 * 16;  // an epilogue warp's pass: 32 tokens x 4 streams x 8 columns of X, inv
+template <typename TX> constexpr int kUpStages = sizeof(TX) == 2 ? 4 : 2;           // what shared memory holds beside them
+
+struct HcUpArgs {
+    const unsigned char *hs;  // h, tile-blocked F16 [M, Kp]
+    const uint8_t *q;         // chunk-major W_up
+    const uint16_t *scale, *minv;
+    const void *x;
+    const float *inv, *norm_w;
+    void *u;
+    int64_t M, d;
+    int r, G, steps;
+    uint32_t *status;
+    unsigned long long wait_limit_ns;
+};
+
+template <int BITS, typename TX>
+__global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs a) {
+    constexpr int kStages = kUpStages<TX>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t b_full[kStages], b_empty[kStages], acc_full[2], acc_empty[2], w_full, w_free, drain_bar;
+    __shared__ float row_scale[kUpScaleBufs][128];
+    __shared__ uint32_t tmem_base_smem;
+    __shared__ int abort_flag;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31, quad = warp & 3;
+    const int tiles = (int)((a.M + kUpTile - 1) / kUpTile);
+    const int64_t items = (a.d / 32) * tiles;
+    const int64_t i0 = items * blockIdx.x / gridDim.x, i1 = items * (blockIdx.x + 1) / gridDim.x;  // item i: row block i / tiles, tokens of tile i % tiles
+    volatile int *abort_v = &abort_flag;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) mbar_init(&b_full[s], 1), mbar_init(&b_empty[s], 1);
+        for (int h = 0; h < 2; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kUpEpiWarps);
+        mbar_init(&w_full, 4), mbar_init(&w_free, 1), mbar_init(&drain_bar, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kUpMma) {  // all 512 columns: one CTA per SM
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_smem)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_smem;
+    auto raise_abort = [&](int64_t item, int role) {
+        if (atomicExch(&abort_flag, 1) == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) a.status[1] = (uint32_t)item, a.status[2] = (uint32_t)role;
+    };
+    auto cnt_of = [&](int tile) { return (int)min((int64_t)kUpTile, a.M - (int64_t)tile * kUpTile); };
+    bool copied = false;  // this thread has issued bulk copies
+
+    if (warp >= kUpProducer && warp < kUpMma) {
+        // ===================== weights: a lane a row =====================
+        const int64_t N = kStreams * a.d;
+        const int chunks = a.r / kChunk, groups = a.r / a.G;
+        int block = 0;
+        for (int64_t rb = i0 / tiles; rb * tiles < i1; ++rb, ++block) {
+            const int64_t n = up_source_row(rb * 128 + quad * 32 + lane, a.d);
+            // The row's power of two, or none for the quadrant, as the general kernel chooses it (kScaleSpread in grouped_tc_tiled.cu).
+            int hi = 0x400, lo = 0x7fff;  // over v = max(|scale| 2^8, |min|) as BF16 bits; 0x400 = an empty group
+            for (int g = 0; g < groups; ++g) {
+                const int v = max(((int)__ldg(a.scale + g * N + n) & 0x7fff) + 0x400, (int)__ldg(a.minv + g * N + n) & 0x7fff);
+                hi = max(hi, v);
+                if (v != 0x400) lo = min(lo, v);
+            }
+            const int e = min(max((hi >> 7) - 8, 127 - 24), 127 + 15);
+            const bool natural = __any_sync(0xffffffffu, e > 127 - 10 && lo != 0x7fff && (lo >> 7) - 8 < e - 6);
+            const float scale = __int_as_float((127 + 14 + 127 - e) << 23), scale_min = scale * 0x1p-24f;
+            row_scale[block % kUpScaleBufs][quad * 32 + lane] = natural ? 1.f : __uint_as_float(((127u + 24u + 127u) << 23) - __float_as_uint(scale));  // undoes it: 2^(24 - k)
+            if (block > 0) {  // the MMAs of the block before have read their weights
+                const bool ok = mbar_wait(&w_free, (uint32_t)(block - 1) & 1u, abort_v, a.wait_limit_ns);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) raise_abort(rb * tiles, 1);
+                    break;
+                }
+            }
+            tc_fence_after();
+            const uint32_t to = tmem + ((uint32_t)(quad * 32) << 16) + kUpACols;
+#pragma unroll 2
+            for (int c = 0; c < a.steps * 4; ++c) {  // 32 codes -> 16 columns
+                uint4 dq[4];
+                const bool in = c < chunks;
+                const int64_t at = (int64_t)(in ? c : 0) * N + n, gi = (int64_t)((in ? c : 0) * kChunk / a.G) * N + n;
+                const float sc = in ? bf16_bits_to_f32(__ldg(a.scale + gi)) : 0.f, mn = in ? bf16_bits_to_f32(__ldg(a.minv + gi)) : 0.f;
+                const uint4 *src = reinterpret_cast<const uint4 *>(a.q) + at * (BITS / 4);
+                const uint4 v0 = __ldg(src), v1 = BITS == 8 ? __ldg(src + (BITS / 8)) : v0;
+                if (natural) {
+                    const __half2 s2 = __float2half2_rn(sc), m2 = __float2half2_rn(mn);
+                    if (BITS == 4) dq[0] = dequant_q4_word(v0.x, s2, m2), dq[1] = dequant_q4_word(v0.y, s2, m2), dq[2] = dequant_q4_word(v0.z, s2, m2), dq[3] = dequant_q4_word(v0.w, s2, m2);
+                    else dq[0] = dequant_q8_words(v0.x, v0.y, s2, m2), dq[1] = dequant_q8_words(v0.z, v0.w, s2, m2), dq[2] = dequant_q8_words(v1.x, v1.y, s2, m2), dq[3] = dequant_q8_words(v1.z, v1.w, s2, m2);
+                } else {
+                    const __half2 s2 = __float2half2_rn(sc * scale), m2 = __float2half2_rn(mn * scale_min), s16 = __hmul2(s2, __float2half2_rn(0.0625f));
+                    if (BITS == 4) dq[0] = dequant_q4_scaled(v0.x, s2, s16, m2), dq[1] = dequant_q4_scaled(v0.y, s2, s16, m2), dq[2] = dequant_q4_scaled(v0.z, s2, s16, m2), dq[3] = dequant_q4_scaled(v0.w, s2, s16, m2);
+                    else dq[0] = dequant_q8_scaled(v0.x, v0.y, s2, m2), dq[1] = dequant_q8_scaled(v0.z, v0.w, s2, m2), dq[2] = dequant_q8_scaled(v1.x, v1.y, s2, m2), dq[3] = dequant_q8_scaled(v1.z, v1.w, s2, m2);
+                }
+                __syncwarp();
+                tc_st16(to + (uint32_t)c * 16u, dq);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&w_full);
+        }
+    } else if (warp == kUpCopy) {
+        // ===================== activations: two bulk copies a step =====================
+        if (elect_one()) {
+            const int64_t line = a.M * 128;  // bytes from one 64-k sub-tile to the next
+            uint32_t count = 0;
+            for (int64_t i = i0; i < i1 && !*abort_v; ++i) {
+                const int tile = (int)(i % tiles);
+                const uint32_t bytes = (uint32_t)cnt_of(tile) * 128u;
+                const unsigned char *src = a.hs + (int64_t)tile * kUpTile * 128;
+                for (int st = 0; st < a.steps; ++st, ++count, src += 2 * line) {
+                    const uint32_t stage = count % kStages;
+                    if (!mbar_wait(&b_empty[stage], ((count / kStages) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                        raise_abort(i, 5);
+                        break;
+                    }
+                    const uint32_t dst = smem_u32(smem) + stage * (uint32_t)kUpStageBytes;
+                    mbar_expect_tx(&b_full[stage], 2 * bytes);
+                    bulk_g2s(dst, src, bytes, &b_full[stage]);
+                    bulk_g2s(dst + kUpSubBytes, src + line, bytes, &b_full[stage]);
+                    copied = true;
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == kUpMma) {
+        // ===================== MMA issue: the whole warp, uniform control flow =====================
+        const uint32_t leader = elect_one() ? 1u : 0u;
+        const uint64_t desc0 = smem_desc(smem_u32(smem));
+        uint32_t count = 0, acc_count = 0;
+        int block = -1;
+        int64_t rb_at = -1;
+        bool ok = true;
+        for (int64_t i = i0; i < i1 && ok; ++i, ++acc_count) {
+            const int64_t rb = i / tiles;
+            if (rb != rb_at) {
+                rb_at = rb, ++block;
+                ok = __all_sync(0xffffffffu, mbar_wait(&w_full, (uint32_t)block & 1u, abort_v, a.wait_limit_ns));
+                if (!ok) {
+                    if (leader) raise_abort(i, 3);
+                    break;
+                }
+            }
+            const uint32_t half = acc_count & 1u;
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[half], ((acc_count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns));
+            if (!ok) {
+                if (leader) raise_abort(i, 2);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t idesc = __reduce_max_sync(0xffffffffu, instr_desc((cnt_of((int)(i % tiles)) + 15) & ~15));
+            for (int st = 0; st < a.steps; ++st, ++count) {
+                const uint32_t stage = count % kStages;
+                ok = __all_sync(0xffffffffu, mbar_wait(&b_full[stage], (count / kStages) & 1u, abort_v, a.wait_limit_ns));
+                if (!ok) {
+                    if (leader) raise_abort(i, 3);
+                    break;
+                }
+                tc_fence_after();
+                tc_step_ts<kUpSubBytes>(leader, tmem + half * (uint32_t)kUpTile, tmem + (uint32_t)(kUpACols + st * 64), (uint32_t)desc0 + stage * (uint32_t)(kUpStageBytes / 16),
+                                        (uint32_t)(desc0 >> 32), idesc, st != 0);
+                tc_commit_if(leader, &b_empty[stage]);
+            }
+            if (ok) tc_commit_if(leader, &acc_full[half]);
+            if (ok && (i + 1) / tiles != rb) tc_commit_if(leader, &w_free);  // the last item of the block: its weights have been read
+        }
+        tc_commit_if(leader, &drain_bar);  // not given up while aborting: tensor memory must not be released under an MMA
+        mbar_wait(&drain_bar, 0u, nullptr, a.wait_limit_ns);
+        __syncwarp();
+    } else if (warp < kUpEpiWarps) {
+        // ===================== epilogue: the stream combine (TcHcUp) =====================
+        // Lane = (stream s = lane & 3, output column j).  X and inv of the warp's 32 tokens come through shared memory by 16-byte asynchronous
+        // copies an item ahead: a load into registers would stall the in-order issue once a token.
+        constexpr int es = sizeof(TX), seg = 8 * es, kParts = seg / 16, kTokStep = 8 / kParts, kPieces = 128 * seg / 16 / 32;
+        const int s = lane & 3, jj = lane >> 2, tok0 = (warp >> 2) * 32;
+        const int64_t row_bytes = 4 * a.d * es;
+        unsigned char *my_buf = smem + kStages * kUpStageBytes + warp * (2 * kUpBuf<TX>);
+        const int part_l = lane % kParts, str_l = (lane / kParts) & 3, tok_l = lane / (4 * kParts);
+        auto issue = [&](int64_t i, unsigned char *buf) {
+            if (i < i1) {
+                const int64_t rb = i / tiles;
+                const int tile = (int)(i % tiles), live = cnt_of(tile) - tok0;
+                const int64_t t0 = (int64_t)tile * kUpTile + tok0;
+                const unsigned char *src = static_cast<const unsigned char *>(a.x) + (rb * 32 + quad * 8 + (int64_t)str_l * a.d) * es + part_l * 16 + (t0 + tok_l) * row_bytes;
+                const uint32_t dst = smem_u32(buf) + (uint32_t)lane * 16u;
+#pragma unroll
+                for (int k = 0; k < kPieces; ++k)
+                    if (k * kTokStep + tok_l < live) cp_async16(dst + (uint32_t)k * 512u, src + (int64_t)(k * kTokStep) * row_bytes);
+                if (lane < live) cp_async16(smem_u32(buf) + 128 * seg + (uint32_t)lane * 16u, a.inv + (t0 + lane) * 4);
+            }
+            cp_async_commit();
+        };
+        issue(i0, my_buf);
+        uint32_t acc_count = 0;
+        int block = -1;
+        int64_t rb_at = -1;
+        float nwp = 0.f, nz = 0.f;
+        for (int64_t i = i0; i < i1; ++i, ++acc_count) {
+            const int64_t rb = i / tiles, j = rb * 32 + quad * 8 + jj;
+            const int tile = (int)(i % tiles), live = cnt_of(tile) - tok0;
+            const bool fresh = rb != rb_at;
+            if (fresh) rb_at = rb, ++block, nwp = 1.0f + __ldg(a.norm_w + (int64_t)s * a.d + j);
+            unsigned char *buf = my_buf + (acc_count & 1u) * kUpBuf<TX>;
+            __syncwarp();  // every lane has finished reading the buffer that the next copies overwrite
+            issue(i + 1, my_buf + ((acc_count + 1) & 1u) * kUpBuf<TX>);
+            const uint32_t half = acc_count & 1u;
+            const bool ok = mbar_wait(&acc_full[half], (acc_count >> 1) & 1u, abort_v, a.wait_limit_ns);
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) raise_abort(i, 4);
+                break;
+            }
+            tc_fence_after();
+            // sigmoid(z) = 1 / (1 + 2^(-z log2 e)), with the row's power of two taken out of z on the way
+            if (fresh) nz = -1.44269504f * row_scale[block % kUpScaleBufs][quad * 32 + lane];
+            float va[16], vb[16];
+            const uint32_t tcol = tmem + ((uint32_t)(quad * 32) << 16) + half * (uint32_t)kUpTile + (uint32_t)tok0;
+            if (live > 0) tc_ld16x2(tcol, tcol + 16u, va, vb);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[half]);
+            cp_async_wait<1>();  // this item's copies have landed (the next one's may still be in flight)
+            __syncwarp();
+            if (live <= 0) continue;
+            const TX *xs_ = reinterpret_cast<const TX *>(buf + s * seg) + jj;  // token tt: + tt * 32 elements
+            const float *ivs = reinterpret_cast<const float *>(buf + 128 * seg) + s;
+            // First every token's term of this lane's stream, in place of its accumulator (shared-memory reads and arithmetic only: a store
+            // to u in between would fence the next token's reads behind it, both being generic addresses).  Then the four streams of a
+            // column - lanes l, l ^ 1, l ^ 2, l ^ 3 - four tokens at a time by a reduce-scatter: three shuffles instead of the eight of
+            // four butterflies, and it leaves each of the four lanes with the sum of one token, which that lane stores.
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int tt = t + 16 * hf;
+                    const float z = hf ? vb[t] : va[t];
+                    const float c = __fdividef(load_as_f32(xs_, tt * 32) * ivs[tt * 4] * nwp, 1.0f + exp2_fast(z * nz));
+                    if (hf) vb[t] = c;
+                    else va[t] = c;
+                }
+            }
+            const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+            const int mine = (b0 ? 2 : 0) + (b1 ? 1 : 0);  // which of a group's four tokens this lane ends up with
+            TX *up = static_cast<TX *>(a.u) + ((int64_t)tile * kUpTile + tok0 + mine) * a.d + j;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float ta = k < 4 ? va[4 * k] : vb[4 * k - 16], tb = k < 4 ? va[4 * k + 1] : vb[4 * k - 15];
+                const float tc = k < 4 ? va[4 * k + 2] : vb[4 * k - 14], td = k < 4 ? va[4 * k + 3] : vb[4 * k - 13];
+                // lanes with bit 0 clear keep tokens a, b and send c, d; the others the reverse
+                const float k0 = (b0 ? tc : ta) + __shfl_xor_sync(0xffffffffu, b0 ? ta : tc, 1);
+                const float k1 = (b0 ? td : tb) + __shfl_xor_sync(0xffffffffu, b0 ? tb : td, 1);
+                // lanes with bit 1 clear keep the first of the two and send the second; the others the reverse
+                const float sum = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+                if (4 * k + mine < live) store_from_f32(up, (int64_t)(4 * k) * a.d, sum * 0.25f);
+            }
+        }
+        cp_async_wait<0>();
+    }
+
+    // An aborting CTA must not return under copies into its own shared memory: their issuer lets a generous time pass.
+    if (*abort_v && copied)
+        for (const unsigned long long t0 = global_ns(); global_ns() - t0 < 50000ull;) {}
+    tc_fence_before();
+    __syncthreads();
+    if (warp == kUpMma) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+template <int BITS, typename TX>
+int launch_hc_up(const char *fn, const HcUpArgs &a, cudaStream_t st) {
+    const size_t smem = (size_t)kUpStages<TX> * kUpStageBytes + (size_t)kUpEpiWarps * 2 * kUpBuf<TX> + 1024;
+    auto kern = hc_up_tc_kernel<BITS, TX>;
+    SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
+    const int64_t items = a.d / 32 * ((a.M + kUpTile - 1) / kUpTile);
+    kern<<<(unsigned)std::min<int64_t>(items, sm_count()), kUpThreads, smem, st>>>(a);
+    SXB_CHECK_LAUNCH(fn, " T=", a.M, " d=", a.d, " r=", a.r);
+    return SXB_OK;
+}
+
 // ---- hosts ---------------------------------------------------------------------------------------------------------
 
 int check_shape(const char *fn, int64_t T, int64_t H, int64_t d, const SxbQView *w, int act) {
@@ -324,14 +619,19 @@ int mix_up_tc(const float *h, const SxbQView *w, const void *x, const float *nor
     auto st = static_cast<cudaStream_t>(stream);
     SxbQView rows{base + L.wq, reinterpret_cast<uint16_t *>(base + L.wscale), reinterpret_cast<uint16_t *>(base + L.wmin), N, Kp, w->G};
 
+    const unsigned stage_blocks = (unsigned)std::min<int64_t>((T * (Kp / 8) + 255) / 256, (int64_t)sm_count() * 8);
+    hc_stage_h_kernel<BITS><<<stage_blocks, 256, 0, st>>>(h, T, r, Kp, base + L.hs);
+    SXB_CHECK_LAUNCH(fn, " staging h, T=", T, " r=", r);
+    if (Kp <= kUpSteps * 128) {
+        HcUpArgs a{base + L.hs, w->q, w->scale, w->minv, x, inv, norm_w, u, T, d, (int)r, (int)w->G, (int)(Kp / 128), nullptr, wait_limit_ns()};
+        if (int rc = library_status_words(fn, &a.status)) return rc;
+        return act == SXB_ACT_F32 ? launch_hc_up<BITS, float>(fn, a, st) : launch_hc_up<BITS, uint16_t>(fn, a, st);
+    }
     const int64_t vecs = N * Kp * BITS / 128;
     hc_unchunk_up_kernel<<<(unsigned)std::min<int64_t>((vecs + 255) / 256, (int64_t)sm_count() * 8), 256, 0, st>>>(
         w->q, w->scale, w->minv, d, r, Kp, w->G, BITS, reinterpret_cast<uint32_t *>(base + L.wq), reinterpret_cast<uint16_t *>(base + L.wscale),
         reinterpret_cast<uint16_t *>(base + L.wmin));
     SXB_CHECK_LAUNCH(fn, " un-chunking the weight, N=", N, " r=", r);
-    const unsigned stage_blocks = (unsigned)std::min<int64_t>((T * (Kp / 8) + 255) / 256, (int64_t)sm_count() * 8);
-    hc_stage_h_kernel<BITS><<<stage_blocks, 256, 0, st>>>(h, T, r, Kp, base + L.hs);
-    SXB_CHECK_LAUNCH(fn, " staging h, T=", T, " r=", r);
     return tc_hc_up<BITS>(fn, base + L.hs, &rows, x, inv, norm_w, u, T, d, act == SXB_ACT_F32, stream);
 }
 
