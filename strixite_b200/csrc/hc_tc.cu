@@ -225,17 +225,18 @@ __global__ void __launch_bounds__(256) hc_stage_h_kernel(const float *__restrict
 // Warps: sixteen for the epilogue (a lane quadrant and 32 of an item's tokens each), four producers, MMA issue, activation copies.  Waits are
 // bounded; one that runs out raises the CTA's abort flag and is recorded in the library's status words.
 constexpr int kUpTile = 128, kUpSubBytes = kUpTile * 128, kUpStageBytes = 2 * kUpSubBytes, kUpSteps = 4;  // steps of 128 k at most
-constexpr int kUpEpiWarps = 16, kUpProducer = kUpEpiWarps, kUpMma = kUpEpiWarps + 4, kUpCopy = kUpEpiWarps + 5, kUpThreads = 32 * (kUpEpiWarps + 6);
+constexpr int kUpEpiWarps = 16, kUpProducer = kUpEpiWarps, kUpMma = kUpEpiWarps + 4, kUpCopy = kUpEpiWarps + 5, kUpXCopy = kUpEpiWarps + 6,
+              kUpThreads = 32 * (kUpEpiWarps + 7);
 constexpr int kUpACols = 256;   // first tensor-memory column of the weights, behind two accumulators of 128
 constexpr int kUpScaleBufs = 4; // row blocks whose powers of two are kept: the epilogue is two accumulators behind at most
-template <typename TX> constexpr int kUpBuf = 128 * 8 * (int)sizeof(TX) + 32 * 16;  // an epilogue warp's pass: 32 tokens x 4 streams x 8 columns of X, inv
-template <typename TX> constexpr int kUpStages = sizeof(TX) == 2 ? 4 : 2;           // what shared memory holds beside them
+template <typename TX> constexpr int kUpXBytes = 4 * kUpTile * 32 * (int)sizeof(TX);  // an item's X: 128 tokens x 4 streams x 32 columns
+template <typename TX> constexpr int kUpBuf = kUpXBytes<TX> + kUpTile * 16;           // and inv
+template <typename TX> constexpr int kUpStages = sizeof(TX) == 2 ? 4 : 2;             // what shared memory holds beside two of them
 
 struct HcUpArgs {
     const unsigned char *hs;  // h, tile-blocked F16 [M, Kp]
     const uint8_t *q;         // chunk-major W_up
     const uint16_t *scale, *minv;
-    const void *x;
     const float *inv, *norm_w;
     void *u;
     int64_t M, d;
@@ -244,12 +245,19 @@ struct HcUpArgs {
     unsigned long long wait_limit_ns;
 };
 
+// 2^v on the special-function unit, results below 2^-126 as zero: what is added to one.
+__device__ inline float exp2_ftz(float v) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 template <int BITS, typename TX>
-__global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs a) {
+__global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs a, const __grid_constant__ CUtensorMap xmap) {
     constexpr int kStages = kUpStages<TX>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ uint64_t b_full[kStages], b_empty[kStages], acc_full[2], acc_empty[2], w_full, w_free, drain_bar;
+    __shared__ uint64_t b_full[kStages], b_empty[kStages], acc_full[2], acc_empty[2], x_full[2], x_empty[2], w_full, w_free, drain_bar;
     __shared__ float row_scale[kUpScaleBufs][128];
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
@@ -261,7 +269,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&b_full[s], 1), mbar_init(&b_empty[s], 1);
-        for (int h = 0; h < 2; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kUpEpiWarps);
+        for (int h = 0; h < 2; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kUpEpiWarps), mbar_init(&x_full[h], 1), mbar_init(&x_empty[h], kUpEpiWarps);
         mbar_init(&w_full, 4), mbar_init(&w_free, 1), mbar_init(&drain_bar, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -277,6 +285,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
     auto raise_abort = [&](int64_t item, int role) {
         if (atomicExch(&abort_flag, 1) == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) a.status[1] = (uint32_t)item, a.status[2] = (uint32_t)role;
     };
+    unsigned char *const x_bufs = smem + kStages * kUpStageBytes;
     auto cnt_of = [&](int tile) { return (int)min((int64_t)kUpTile, a.M - (int64_t)tile * kUpTile); };
     bool copied = false;  // this thread has issued bulk copies
 
@@ -356,6 +365,27 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
             }
         }
         __syncwarp();
+    } else if (warp == kUpXCopy) {
+        // ===================== X and inv, an item ahead: a row is a stream of a token, 16-byte chunks swizzled =====================
+        // (by 16-byte asynchronous copies of the epilogue's lanes, each to a row of its own, X took a third of the epilogue's time)
+        if (elect_one()) {
+            uint32_t count = 0;
+            for (int64_t i = i0; i < i1 && !*abort_v; ++i, ++count) {
+                const uint32_t half = count & 1u;
+                if (!mbar_wait(&x_empty[half], ((count >> 1) & 1u) ^ 1u, abort_v, a.wait_limit_ns)) {
+                    raise_abort(i, 5);
+                    break;
+                }
+                const int tile = (int)(i % tiles), x0 = (int)(i / tiles) * 32, y0 = tile * 4 * kUpTile;
+                const uint32_t dst = smem_u32(x_bufs) + half * (uint32_t)kUpBuf<TX>, inv_bytes = (uint32_t)cnt_of(tile) * 16u;
+                mbar_expect_tx(&x_full[half], (uint32_t)kUpXBytes<TX> + inv_bytes);
+                tma_load_2d(dst, &xmap, x0, y0, &x_full[half]);  // rows past the last token read as zeros
+                tma_load_2d(dst + kUpXBytes<TX> / 2, &xmap, x0, y0 + 2 * kUpTile, &x_full[half]);
+                bulk_g2s(dst + kUpXBytes<TX>, a.inv + (int64_t)tile * kUpTile * 4, inv_bytes, &x_full[half]);
+                copied = true;
+            }
+        }
+        __syncwarp();
     } else if (warp == kUpMma) {
         // ===================== MMA issue: the whole warp, uniform control flow =====================
         const uint32_t leader = elect_one() ? 1u : 0u;
@@ -402,28 +432,17 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
         __syncwarp();
     } else if (warp < kUpEpiWarps) {
         // ===================== epilogue: the stream combine (TcHcUp) =====================
-        // Lane = (stream s = lane & 3, output column j).  X and inv of the warp's 32 tokens come through shared memory by 16-byte asynchronous
-        // copies an item ahead: a load into registers would stall the in-order issue once a token.
-        constexpr int es = sizeof(TX), seg = 8 * es, kParts = seg / 16, kTokStep = 8 / kParts, kPieces = 128 * seg / 16 / 32;
+        // Lane = (stream s = lane & 3, output column j).
+        constexpr int es = sizeof(TX), kRowBytes = 32 * es;
         const int s = lane & 3, jj = lane >> 2, tok0 = (warp >> 2) * 32;
-        const int64_t row_bytes = 4 * a.d * es;
-        unsigned char *my_buf = smem + kStages * kUpStageBytes + warp * (2 * kUpBuf<TX>);
-        const int part_l = lane % kParts, str_l = (lane / kParts) & 3, tok_l = lane / (4 * kParts);
-        auto issue = [&](int64_t i, unsigned char *buf) {
-            if (i < i1) {
-                const int64_t rb = i / tiles;
-                const int tile = (int)(i % tiles), live = cnt_of(tile) - tok0;
-                const int64_t t0 = (int64_t)tile * kUpTile + tok0;
-                const unsigned char *src = static_cast<const unsigned char *>(a.x) + (rb * 32 + quad * 8 + (int64_t)str_l * a.d) * es + part_l * 16 + (t0 + tok_l) * row_bytes;
-                const uint32_t dst = smem_u32(buf) + (uint32_t)lane * 16u;
+        // this lane's element of a token at even / odd place: row 4 tok + s, column quad * 8 + jj, its chunk swizzled (64-byte rows by row >> 1 & 3,
+        // 128-byte rows by row & 7)
+        int x_at[2];
 #pragma unroll
-                for (int k = 0; k < kPieces; ++k)
-                    if (k * kTokStep + tok_l < live) cp_async16(dst + (uint32_t)k * 512u, src + (int64_t)(k * kTokStep) * row_bytes);
-                if (lane < live) cp_async16(smem_u32(buf) + 128 * seg + (uint32_t)lane * 16u, a.inv + (t0 + lane) * 4);
-            }
-            cp_async_commit();
-        };
-        issue(i0, my_buf);
+        for (int p = 0; p < 2; ++p) {
+            const int chunk = (quad * 8 + jj) * es / 16, swz = es == 2 ? p * 2 + (s >> 1) : p * 4 + s;
+            x_at[p] = (4 * (tok0 + p) + s) * kRowBytes + ((chunk ^ swz) << 4) + (jj * es) % 16;
+        }
         uint32_t acc_count = 0;
         int block = -1;
         int64_t rb_at = -1;
@@ -433,11 +452,9 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
             const int tile = (int)(i % tiles), live = cnt_of(tile) - tok0;
             const bool fresh = rb != rb_at;
             if (fresh) rb_at = rb, ++block, nwp = 1.0f + __ldg(a.norm_w + (int64_t)s * a.d + j);
-            unsigned char *buf = my_buf + (acc_count & 1u) * kUpBuf<TX>;
-            __syncwarp();  // every lane has finished reading the buffer that the next copies overwrite
-            issue(i + 1, my_buf + ((acc_count + 1) & 1u) * kUpBuf<TX>);
-            const uint32_t half = acc_count & 1u;
-            const bool ok = mbar_wait(&acc_full[half], (acc_count >> 1) & 1u, abort_v, a.wait_limit_ns);
+            const uint32_t half = acc_count & 1u, phase = (acc_count >> 1) & 1u;
+            const unsigned char *buf = x_bufs + half * (uint32_t)kUpBuf<TX>;
+            const bool ok = mbar_wait(&x_full[half], phase, abort_v, a.wait_limit_ns) && mbar_wait(&acc_full[half], phase, abort_v, a.wait_limit_ns);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) raise_abort(i, 4);
                 break;
@@ -451,11 +468,12 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[half]);
-            cp_async_wait<1>();  // this item's copies have landed (the next one's may still be in flight)
-            __syncwarp();
-            if (live <= 0) continue;
-            const TX *xs_ = reinterpret_cast<const TX *>(buf + s * seg) + jj;  // token tt: + tt * 32 elements
-            const float *ivs = reinterpret_cast<const float *>(buf + 128 * seg) + s;
+            if (live <= 0) {
+                if (lane == 0) mbar_arrive(&x_empty[half]);
+                continue;
+            }
+            const TX *xs_[2] = {reinterpret_cast<const TX *>(buf + x_at[0]), reinterpret_cast<const TX *>(buf + x_at[1])};
+            const float *ivs = reinterpret_cast<const float *>(buf + kUpXBytes<TX>) + tok0 * 4 + s;
             // First every token's term of this lane's stream, in place of its accumulator (shared-memory reads and arithmetic only: a store
             // to u in between would fence the next token's reads behind it, both being generic addresses).  Then the four streams of a
             // column - lanes l, l ^ 1, l ^ 2, l ^ 3 - four tokens at a time by a reduce-scatter: three shuffles instead of the eight of
@@ -466,11 +484,13 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
                 for (int hf = 0; hf < 2; ++hf) {
                     const int tt = t + 16 * hf;
                     const float z = hf ? vb[t] : va[t];
-                    const float c = __fdividef(load_as_f32(xs_, tt * 32) * ivs[tt * 4] * nwp, 1.0f + exp2_fast(z * nz));
+                    const float c = __fdividef(load_as_f32(xs_[tt & 1], (tt >> 1) * 256) * ivs[tt * 4] * nwp, 1.0f + exp2_ftz(z * nz));
                     if (hf) vb[t] = c;
                     else va[t] = c;
                 }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&x_empty[half]);
             const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
             const int mine = (b0 ? 2 : 0) + (b1 ? 1 : 0);  // which of a group's four tokens this lane ends up with
             TX *up = static_cast<TX *>(a.u) + ((int64_t)tile * kUpTile + tok0 + mine) * a.d + j;
@@ -486,7 +506,6 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
                 if (4 * k + mine < live) store_from_f32(up, (int64_t)(4 * k) * a.d, sum * 0.25f);
             }
         }
-        cp_async_wait<0>();
     }
 
     // An aborting CTA must not return under copies into its own shared memory: their issuer lets a generous time pass.
@@ -501,12 +520,17 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
 }
 
 template <int BITS, typename TX>
-int launch_hc_up(const char *fn, const HcUpArgs &a, cudaStream_t st) {
-    const size_t smem = (size_t)kUpStages<TX> * kUpStageBytes + (size_t)kUpEpiWarps * 2 * kUpBuf<TX> + 1024;
+int launch_hc_up(const char *fn, const HcUpArgs &a, const void *x, cudaStream_t st) {
+    const size_t smem = (size_t)kUpStages<TX> * kUpStageBytes + (size_t)2 * kUpBuf<TX> + 1024;
+    // X as [4 T, d], boxes of 32 columns x 256 rows
+    CUtensorMap xmap;
+    if (int rc = tensor_map_2d(fn, x, sizeof(TX) == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, sizeof(TX), (uint64_t)a.d, (uint64_t)(kStreams * a.M),
+                               (uint64_t)a.d * sizeof(TX), 32u, 256u, sizeof(TX) == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, &xmap))
+        return rc;
     auto kern = hc_up_tc_kernel<BITS, TX>;
     SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
     const int64_t items = a.d / 32 * ((a.M + kUpTile - 1) / kUpTile);
-    kern<<<(unsigned)std::min<int64_t>(items, sm_count()), kUpThreads, smem, st>>>(a);
+    kern<<<(unsigned)std::min<int64_t>(items, sm_count()), kUpThreads, smem, st>>>(a, xmap);
     SXB_CHECK_LAUNCH(fn, " T=", a.M, " d=", a.d, " r=", a.r);
     return SXB_OK;
 }
@@ -623,9 +647,9 @@ int mix_up_tc(const float *h, const SxbQView *w, const void *x, const float *nor
     hc_stage_h_kernel<BITS><<<stage_blocks, 256, 0, st>>>(h, T, r, Kp, base + L.hs);
     SXB_CHECK_LAUNCH(fn, " staging h, T=", T, " r=", r);
     if (Kp <= kUpSteps * 128) {
-        HcUpArgs a{base + L.hs, w->q, w->scale, w->minv, x, inv, norm_w, u, T, d, (int)r, (int)w->G, (int)(Kp / 128), nullptr, wait_limit_ns()};
+        HcUpArgs a{base + L.hs, w->q, w->scale, w->minv, inv, norm_w, u, T, d, (int)r, (int)w->G, (int)(Kp / 128), nullptr, wait_limit_ns()};
         if (int rc = library_status_words(fn, &a.status)) return rc;
-        return act == SXB_ACT_F32 ? launch_hc_up<BITS, float>(fn, a, st) : launch_hc_up<BITS, uint16_t>(fn, a, st);
+        return act == SXB_ACT_F32 ? launch_hc_up<BITS, float>(fn, a, x, st) : launch_hc_up<BITS, uint16_t>(fn, a, x, st);
     }
     const int64_t vecs = N * Kp * BITS / 128;
     hc_unchunk_up_kernel<<<(unsigned)std::min<int64_t>((vecs + 255) / 256, (int64_t)sm_count() * 8), 256, 0, st>>>(
