@@ -62,38 +62,52 @@ __device__ inline void load8(const uint16_t *p, int64_t i, float (&f)[8]) {
 
 // ---- down ----------------------------------------------------------------------------------------------------------
 
+struct DownStack {
+    const uint8_t *q;  // the folded down weight [R, H*d]
+    const uint16_t *scale, *minv;
+    int64_t R, Rp, G;
+    uint32_t *qo;      // its per-stream stacks [H * Rp, d]
+    uint16_t *so, *mo;
+    RouteWords L;      // the grouping workspace of T slots a stream
+    int32_t *ws;
+};
+
 // The folded down weight [R, H*d] -> per-stream stacks [H * Rp, d]: codes, scales and mins of columns [s d, (s + 1) d) of
-// row n become row s * Rp + n; rows n >= R are zero codes with zero scale and min.
-__global__ void __launch_bounds__(256) hc_stack_down_kernel(const uint8_t *__restrict__ q, const uint16_t *__restrict__ scale,
-                                                            const uint16_t *__restrict__ minv, int64_t R, int64_t Rp, int64_t d, int64_t G,
-                                                            int bits, uint32_t *__restrict__ qo, uint16_t *__restrict__ so,
-                                                            uint16_t *__restrict__ mo) {
-    const int64_t row_vecs = d * bits / 128, row_groups = d / G, stride = (int64_t)gridDim.x * blockDim.x;  // 16-byte pieces a stream's row
-    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint4 *qi = reinterpret_cast<const uint4 *>(q);
-    uint4 *qv = reinterpret_cast<uint4 *>(qo);
-    for (int64_t i = first; i < kStreams * Rp * row_vecs; i += stride) {
-        const int64_t w = i % row_vecs, sn = i / row_vecs, n = sn % Rp, s = sn / Rp;
-        qv[i] = n < R ? __ldg(qi + (n * kStreams + s) * row_vecs + w) : make_uint4(0u, 0u, 0u, 0u);
+// row n become row s * Rp + n; rows n >= R are zero codes with zero scale and min.  And the grouping workspace.
+__device__ __noinline__ void prepare_down(const DownStack &k, int64_t T, int64_t d, int bits, int64_t first, int64_t stride) {
+    const int64_t row_vecs = d * bits / 128, row_groups = d / k.G;  // 16-byte pieces a stream's row
+    const uint4 *qi = reinterpret_cast<const uint4 *>(k.q);
+    uint4 *qv = reinterpret_cast<uint4 *>(k.qo);
+    for (int64_t i = first; i < kStreams * k.Rp * row_vecs; i += stride) {
+        const int64_t w = i % row_vecs, sn = i / row_vecs, n = sn % k.Rp, s = sn / k.Rp;
+        qv[i] = n < k.R ? __ldg(qi + (n * kStreams + s) * row_vecs + w) : make_uint4(0u, 0u, 0u, 0u);
     }
-    for (int64_t i = first; i < kStreams * Rp * row_groups; i += stride) {
-        const int64_t g = i % row_groups, sn = i / row_groups, n = sn % Rp, s = sn / Rp;
+    for (int64_t i = first; i < kStreams * k.Rp * row_groups; i += stride) {
+        const int64_t g = i % row_groups, sn = i / row_groups, n = sn % k.Rp, s = sn / k.Rp;
         const int64_t at = (n * kStreams + s) * row_groups + g;
-        so[i] = n < R ? scale[at] : (uint16_t)0, mo[i] = n < R ? minv[at] : (uint16_t)0;
+        k.so[i] = n < k.R ? k.scale[at] : (uint16_t)0, k.mo[i] = n < k.R ? k.minv[at] : (uint16_t)0;
     }
+    write_regular_routes(k.L, T, k.ws, first, stride);
 }
 
 // One pass over X [T, H*d]: inv[t, s] = 1 / sqrt(mean(X_s[t]^2) + eps) (kernels/hc_wmma.hip:25-45; skipped when the caller
 // has it), and the row X_s[t] as F16 in the tile-blocked form at the position the pack gives slot t * H + s: bucket s
 // starts at s * T and holds its slots in ascending order, and a row's swizzle depends on its place in its tile modulo 8
 // only, which is t modulo 8 for every tile size in use.  A warp per row, rows in position order.
+// The launch's first `stack_blocks` CTAs meanwhile restack the weight and write the grouping workspace (as launches of their own those took 10 us
+// of a 4096-token mix, which the pass over X now hides).
 template <typename TX, int BITS>
 __global__ void __launch_bounds__(256) hc_stage_down_kernel(const TX *__restrict__ x, int64_t T, int64_t d, float eps, bool want_inv,
-                                                            float *__restrict__ inv, unsigned char *__restrict__ xs) {
+                                                            float *__restrict__ inv, unsigned char *__restrict__ xs, const __grid_constant__ DownStack k,
+                                                            int stack_blocks) {
+    if ((int)blockIdx.x < stack_blocks) {
+        prepare_down(k, T, d, BITS, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)stack_blocks * blockDim.x);
+        return;
+    }
     const int lane = threadIdx.x & 31;
-    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5), S = T * kStreams;
+    const int64_t warps = (int64_t)((int)gridDim.x - stack_blocks) * (blockDim.x >> 5), S = T * kStreams;
     const int chunks = (int)(d / 8);
-    for (int64_t pos = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); pos < S; pos += warps) {
+    for (int64_t pos = (int64_t)((int)blockIdx.x - stack_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5); pos < S; pos += warps) {
         const int64_t s = pos / T, t = pos % T;
         const TX *row = x + (t * kStreams + s) * d;
         float ssq = 0.f;
@@ -588,17 +602,17 @@ int mix_down_tc(const void *x, const SxbQView *w, int64_t T, int64_t H, int64_t 
     auto *partial = reinterpret_cast<float *>(base + L.partial);
     SxbQView stacked{base + L.wq, reinterpret_cast<uint16_t *>(base + L.wscale), reinterpret_cast<uint16_t *>(base + L.wmin), kStreams * Rp, d, w->G};
 
+    const DownStack stack{w->q, w->scale, w->minv, R, Rp, w->G, reinterpret_cast<uint32_t *>(base + L.wq), reinterpret_cast<uint16_t *>(base + L.wscale),
+                          reinterpret_cast<uint16_t *>(base + L.wmin), route_words(S, 1, kStreams), reinterpret_cast<int32_t *>(base + L.route)};
     const int64_t stack_vecs = kStreams * Rp * d * BITS / 128;
-    hc_stack_down_kernel<<<(unsigned)std::min<int64_t>((stack_vecs + 255) / 256, (int64_t)sm_count() * 8), 256, 0, st>>>(
-        w->q, w->scale, w->minv, R, Rp, d, w->G, BITS, reinterpret_cast<uint32_t *>(base + L.wq), reinterpret_cast<uint16_t *>(base + L.wscale),
-        reinterpret_cast<uint16_t *>(base + L.wmin));
-    SXB_CHECK_LAUNCH(fn, " restacking the weight, R=", R, " d=", d);
-    if (int rc = regular_routes(fn, T, kStreams, base + L.route, L.route_bytes, stream)) return rc;
     const unsigned stage_blocks = (unsigned)std::min<int64_t>((S + 7) / 8, (int64_t)sm_count() * 8);
+    const int stack_blocks = (int)std::min<int64_t>((stack_vecs + 255) / 256, (int64_t)sm_count() * 2);
     if (act == SXB_ACT_F32)
-        hc_stage_down_kernel<float, BITS><<<stage_blocks, 256, 0, st>>>(static_cast<const float *>(x), T, d, eps, inv_ready == 0, inv, base + L.xs);
+        hc_stage_down_kernel<float, BITS><<<stage_blocks + stack_blocks, 256, 0, st>>>(static_cast<const float *>(x), T, d, eps, inv_ready == 0, inv, base + L.xs,
+                                                                                       stack, stack_blocks);
     else
-        hc_stage_down_kernel<uint16_t, BITS><<<stage_blocks, 256, 0, st>>>(static_cast<const uint16_t *>(x), T, d, eps, inv_ready == 0, inv, base + L.xs);
+        hc_stage_down_kernel<uint16_t, BITS><<<stage_blocks + stack_blocks, 256, 0, st>>>(static_cast<const uint16_t *>(x), T, d, eps, inv_ready == 0, inv,
+                                                                                          base + L.xs, stack, stack_blocks);
     SXB_CHECK_LAUNCH(fn, " staging the streams, T=", T, " d=", d);
     if (int rc = tc_partial_grouped<BITS>(fn, base + L.xs, &stacked, kStreams, base + L.route, L.route_bytes, S, 1, partial, SXB_ACT_F16_TILED,
                                           BITS == 4 ? 3 : 4, false, stream))

@@ -22,8 +22,16 @@ struct RouteWords {
     int64_t offsets, slots, t8_bucket, t8_start, t128_bucket, t128_start, segbad, scratch, first, total;
 };
 RouteWords route_words(int64_t M, int64_t A, int64_t E);
-// The workspace (route_words(M * E, 1, E)) of the grouping in which slot m * E + b belongs to bucket b, for all m < M: what
-// sxb_moe_group_routes writes for ids[m * E + b] = b, without the ids or the sort.
-int regular_routes(const char *fn, int64_t M, int64_t E, void *ws, size_t ws_bytes, sxb_stream_t stream);
+
+// The workspace of the grouping in which slot m * E + b belongs to bucket b, for all m < per_bucket: what sxb_moe_group_routes writes for
+// ids[m * E + b] = b, without the ids or the sort.  L = route_words(per_bucket * E, 1, E); by threads first, first + stride, ...
+__device__ inline void write_regular_routes(const RouteWords &L, int64_t per_bucket, int32_t *ws, int64_t first, int64_t stride) {
+    const int64_t E = L.E, n8 = (per_bucket + 7) / 8, n128 = (per_bucket + 127) / 128;
+    for (int64_t i = first; i < L.S; i += stride) ws[L.slots + i] = (int32_t)((i % per_bucket) * E + i / per_bucket);
+    for (int64_t i = first; i < E * n8; i += stride) ws[L.t8_bucket + i] = (int32_t)(i / n8), ws[L.t8_start + i] = (int32_t)(i / n8 * per_bucket + i % n8 * 8);
+    for (int64_t i = first; i < E * n128; i += stride) ws[L.t128_bucket + i] = (int32_t)(i / n128), ws[L.t128_start + i] = (int32_t)(i / n128 * per_bucket + i % n128 * 128);
+    for (int64_t i = first; i < E + 2; i += stride) ws[L.offsets + i] = (int32_t)(min(i, E) * per_bucket);
+    for (int64_t i = first; i < 8; i += stride) ws[i] = i == 0 ? (int32_t)(E * n8) : i == 1 ? (int32_t)L.S : i == 2 ? (int32_t)E : i == 3 ? (int32_t)(E * n128) : 0;
+}
 
 }  // namespace sxb

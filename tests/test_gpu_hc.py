@@ -415,3 +415,24 @@ def test_hc_mix_wmma_argument_checks(cuda, oracle):
         K.hc_mix_up_wmma(h, wu, x, nw, inv, T, H, d, u, _ws(256, cuda), K.Act.BF16)
     with pytest.raises(K.Error, match="u overlaps"):
         K.hc_mix_up_wmma(h, wu, x, nw, inv, T, H, d, x, _ws(K.hc_mix_up_wmma_workspace_bytes(T, H, d, r, 8, 32), cuda), K.Act.BF16)
+
+
+@pytest.mark.parametrize("T", [1, 7, 128, 129, 1000])
+def test_down_mix_grouping_workspace(cuda, T):
+    """The grouping workspace that the tensor-core down mix writes by formula is the pack's for the same slots."""
+    from strixite_b200 import kernels as K
+    d, r, H, G = 128, 16, 4, 32
+    g = torch.Generator(device="cpu").manual_seed(T)
+    w = K.quantize((torch.randn((r + H, H * d), generator=g) * 0.1).to(cuda), G, 8)
+    x = torch.randn((T, H * d), generator=g).to(torch.bfloat16).to(cuda)
+    h, w_in, inv = (torch.empty((T, n), device=cuda) for n in (r, H, H))
+    ws = torch.full((K.hc_wmma_workspace_bytes(T, H, d, r + H, 8, G),), 255, dtype=torch.uint8, device=cuda)
+    K.hc_mix_down_wmma(x, w, T, H, d, r, True, 1e-6, h, w_in, inv, ws, K.Act.BF16)
+    S, nbytes = T * H, K.moe_route_workspace_bytes(T * H, 1, H)
+    ref, err = torch.full((nbytes // 4,), -1, dtype=torch.int32, device=cuda), torch.zeros(4, dtype=torch.int32, device=cuda)
+    K.moe_group_routes((torch.arange(S, device=cuda) % H).to(torch.int32), S, 1, H, ref, nbytes, err)
+    got = ws[:nbytes].view(torch.int32)
+    at = K.route_layout(S, 1, H)
+    n8, n128 = int(ref[0]), int(ref[3])
+    for lo, n in ((0, 8), (at["offsets"], H + 2), (at["slots"], S), (at["tile8_bucket"], n8), (at["tile8_start"], n8), (at["tile128_bucket"], n128), (at["tile128_start"], n128)):
+        assert torch.equal(got[lo:lo + n], ref[lo:lo + n]), (lo, n)
