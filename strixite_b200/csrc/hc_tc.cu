@@ -242,6 +242,7 @@ constexpr int kUpTile = 128, kUpSubBytes = kUpTile * 128, kUpStageBytes = 2 * kU
 constexpr int kUpEpiWarps = 16, kUpProducer = kUpEpiWarps, kUpMma = kUpEpiWarps + 4, kUpCopy = kUpEpiWarps + 5, kUpXCopy = kUpEpiWarps + 6,
               kUpThreads = 32 * (kUpEpiWarps + 7);
 constexpr int kUpACols = 256;   // first tensor-memory column of the weights, behind two accumulators of 128
+constexpr int kUpGroup = kUpEpiWarps / 2;  // epilogue warps that share an item; the two groups take items by turns
 constexpr int kUpScaleBufs = 4; // row blocks whose powers of two are kept: the epilogue is two accumulators behind at most
 template <typename TX> constexpr int kUpXBytes = 4 * kUpTile * 32 * (int)sizeof(TX);  // an item's X: 128 tokens x 4 streams x 32 columns
 template <typename TX> constexpr int kUpBuf = kUpXBytes<TX> + kUpTile * 16;           // and inv
@@ -259,12 +260,19 @@ struct HcUpArgs {
     unsigned long long wait_limit_ns;
 };
 
-// 2^v on the special-function unit, results below 2^-126 as zero: what is added to one.
+// 2^v and 1 / v on the special-function unit, results below 2^-126 as zero: the one is added to one, the other is of a sum of one or more.
 __device__ inline float exp2_ftz(float v) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
     return r;
 }
+__device__ inline float rcp_ftz(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ inline void store_rounded(float *p, float v) { *p = v; }
+__device__ inline void store_rounded(uint16_t *p, float v) { *p = __bfloat16_as_ushort(__float2bfloat16_rn(v)); }
 
 template <int BITS, typename TX>
 __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs a, const __grid_constant__ CUtensorMap xmap) {
@@ -283,7 +291,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&b_full[s], 1), mbar_init(&b_empty[s], 1);
-        for (int h = 0; h < 2; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kUpEpiWarps), mbar_init(&x_full[h], 1), mbar_init(&x_empty[h], kUpEpiWarps);
+        for (int h = 0; h < 2; ++h) mbar_init(&acc_full[h], 1), mbar_init(&acc_empty[h], kUpGroup), mbar_init(&x_full[h], 1), mbar_init(&x_empty[h], kUpGroup);
         mbar_init(&w_full, 4), mbar_init(&w_free, 1), mbar_init(&drain_bar, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -446,28 +454,27 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
         __syncwarp();
     } else if (warp < kUpEpiWarps) {
         // ===================== epilogue: the stream combine (TcHcUp) =====================
-        // Lane = (stream s = lane & 3, output column j).
+        // Lane = (stream s = lane & 3, output column j); a warp has 64 of the item's tokens, 32 a pass and every other 32.  One accumulator and one buffer of X belong to
+        // a group, and while one group's warps are at the special-function unit, which bounds the terms, the other's are at shuffles and stores.
         constexpr int es = sizeof(TX), kRowBytes = 32 * es;
-        const int s = lane & 3, jj = lane >> 2, tok0 = (warp >> 2) * 32;
+        const int s = lane & 3, jj = lane >> 2, tok0 = ((warp >> 2) & 1) * 32;
+        const uint32_t half = (uint32_t)(warp / kUpGroup);
         // this lane's element of a token at even / odd place: row 4 tok + s, column quad * 8 + jj, its chunk swizzled (64-byte rows by row >> 1 & 3,
         // 128-byte rows by row & 7)
-        int x_at[2];
+        const TX *xs_[2];
 #pragma unroll
         for (int p = 0; p < 2; ++p) {
             const int chunk = (quad * 8 + jj) * es / 16, swz = es == 2 ? p * 2 + (s >> 1) : p * 4 + s;
-            x_at[p] = (4 * (tok0 + p) + s) * kRowBytes + ((chunk ^ swz) << 4) + (jj * es) % 16;
+            xs_[p] = reinterpret_cast<const TX *>(x_bufs + half * (uint32_t)kUpBuf<TX> + (4 * (tok0 + p) + s) * kRowBytes + ((chunk ^ swz) << 4) + (jj * es) % 16);
         }
-        uint32_t acc_count = 0;
-        int block = -1;
-        int64_t rb_at = -1;
-        float nwp = 0.f, nz = 0.f;
-        for (int64_t i = i0; i < i1; ++i, ++acc_count) {
+        const float *ivs = reinterpret_cast<const float *>(x_bufs + half * (uint32_t)kUpBuf<TX> + kUpXBytes<TX>) + tok0 * 4 + s;
+        const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+        const int mine = (b0 ? 2 : 0) + (b1 ? 1 : 0);  // which of a group's four tokens this lane ends up with
+        uint32_t phase = 0;
+        for (int64_t i = i0 + half; i < i1; i += 2, phase ^= 1u) {
             const int64_t rb = i / tiles, j = rb * 32 + quad * 8 + jj;
             const int tile = (int)(i % tiles), live = cnt_of(tile) - tok0;
-            const bool fresh = rb != rb_at;
-            if (fresh) rb_at = rb, ++block, nwp = 1.0f + __ldg(a.norm_w + (int64_t)s * a.d + j);
-            const uint32_t half = acc_count & 1u, phase = (acc_count >> 1) & 1u;
-            const unsigned char *buf = x_bufs + half * (uint32_t)kUpBuf<TX>;
+            const float nwp = 1.0f + __ldg(a.norm_w + (int64_t)s * a.d + j);
             const bool ok = mbar_wait(&x_full[half], phase, abort_v, a.wait_limit_ns) && mbar_wait(&acc_full[half], phase, abort_v, a.wait_limit_ns);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) raise_abort(i, 4);
@@ -475,49 +482,53 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
             }
             tc_fence_after();
             // sigmoid(z) = 1 / (1 + 2^(-z log2 e)), with the row's power of two taken out of z on the way
-            if (fresh) nz = -1.44269504f * row_scale[block % kUpScaleBufs][quad * 32 + lane];
-            float va[16], vb[16];
-            const uint32_t tcol = tmem + ((uint32_t)(quad * 32) << 16) + half * (uint32_t)kUpTile + (uint32_t)tok0;
-            if (live > 0) tc_ld16x2(tcol, tcol + 16u, va, vb);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[half]);
-            if (live <= 0) {
-                if (lane == 0) mbar_arrive(&x_empty[half]);
-                continue;
-            }
-            const TX *xs_[2] = {reinterpret_cast<const TX *>(buf + x_at[0]), reinterpret_cast<const TX *>(buf + x_at[1])};
-            const float *ivs = reinterpret_cast<const float *>(buf + kUpXBytes<TX>) + tok0 * 4 + s;
-            // First every token's term of this lane's stream, in place of its accumulator (shared-memory reads and arithmetic only: a store
-            // to u in between would fence the next token's reads behind it, both being generic addresses).  Then the four streams of a
-            // column - lanes l, l ^ 1, l ^ 2, l ^ 3 - four tokens at a time by a reduce-scatter: three shuffles instead of the eight of
-            // four butterflies, and it leaves each of the four lanes with the sum of one token, which that lane stores.
-#pragma unroll
-            for (int t = 0; t < 16; ++t) {
-#pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {
-                    const int tt = t + 16 * hf;
-                    const float z = hf ? vb[t] : va[t];
-                    const float c = __fdividef(load_as_f32(xs_[tt & 1], (tt >> 1) * 256) * ivs[tt * 4] * nwp, 1.0f + exp2_ftz(z * nz));
-                    if (hf) vb[t] = c;
-                    else va[t] = c;
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&x_empty[half]);
-            const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
-            const int mine = (b0 ? 2 : 0) + (b1 ? 1 : 0);  // which of a group's four tokens this lane ends up with
+            const float nz = -1.44269504f * row_scale[(int)(rb - i0 / tiles) % kUpScaleBufs][quad * 32 + lane];
             TX *up = static_cast<TX *>(a.u) + ((int64_t)tile * kUpTile + tok0 + mine) * a.d + j;
+#pragma unroll 1
+            for (int p = 0; p < 2; ++p, up += 64 * a.d) {
+                const int left = live - 64 * p;
+                float va[16], vb[16];
+                const uint32_t tcol = tmem + ((uint32_t)(quad * 32) << 16) + half * (uint32_t)kUpTile + (uint32_t)(tok0 + 64 * p);
+                if (left > 0) tc_ld16x2(tcol, tcol + 16u, va, vb);
+                if (p == 1) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[half]);
+                }
+                // First every token's term of this lane's stream, in place of its accumulator (shared-memory reads and arithmetic only: a store
+                // to u in between would fence the next token's reads behind it, both being generic addresses).  Then the four streams of a
+                // column - lanes l, l ^ 1, l ^ 2, l ^ 3 - four tokens at a time by a reduce-scatter: three shuffles instead of the eight of
+                // four butterflies, and it leaves each of the four lanes with the sum of one token, which that lane stores.
+                if (left > 0) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const float ta = k < 4 ? va[4 * k] : vb[4 * k - 16], tb = k < 4 ? va[4 * k + 1] : vb[4 * k - 15];
-                const float tc = k < 4 ? va[4 * k + 2] : vb[4 * k - 14], td = k < 4 ? va[4 * k + 3] : vb[4 * k - 13];
-                // lanes with bit 0 clear keep tokens a, b and send c, d; the others the reverse
-                const float k0 = (b0 ? tc : ta) + __shfl_xor_sync(0xffffffffu, b0 ? ta : tc, 1);
-                const float k1 = (b0 ? td : tb) + __shfl_xor_sync(0xffffffffu, b0 ? tb : td, 1);
-                // lanes with bit 1 clear keep the first of the two and send the second; the others the reverse
-                const float sum = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
-                if (4 * k + mine < live) store_from_f32(up, (int64_t)(4 * k) * a.d, sum * 0.25f);
+                    for (int t = 0; t < 16; ++t) {
+#pragma unroll
+                        for (int hf = 0; hf < 2; ++hf) {
+                            const int tt = t + 16 * hf;
+                            const float z = hf ? vb[t] : va[t];
+                            const float c = load_as_f32(xs_[tt & 1], p * 8192 + (tt >> 1) * 256) * ivs[p * 256 + tt * 4] * nwp * rcp_ftz(1.0f + exp2_ftz(z * nz));
+                            if (hf) vb[t] = c;
+                            else va[t] = c;
+                        }
+                    }
+                }
+                if (p == 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&x_empty[half]);
+                }
+                if (left > 0) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float ta = k < 4 ? va[4 * k] : vb[4 * k - 16], tb = k < 4 ? va[4 * k + 1] : vb[4 * k - 15];
+                        const float tc = k < 4 ? va[4 * k + 2] : vb[4 * k - 14], td = k < 4 ? va[4 * k + 3] : vb[4 * k - 13];
+                        // lanes with bit 0 clear keep tokens a, b and send c, d; the others the reverse
+                        const float k0 = (b0 ? tc : ta) + __shfl_xor_sync(0xffffffffu, b0 ? ta : tc, 1);
+                        const float k1 = (b0 ? td : tb) + __shfl_xor_sync(0xffffffffu, b0 ? tb : td, 1);
+                        // lanes with bit 1 clear keep the first of the two and send the second; the others the reverse
+                        const float sum = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 2);
+                        if (4 * k + mine < left) store_rounded(up + (int64_t)(4 * k) * a.d, sum * 0.25f);
+                    }
+                }
             }
         }
     }
