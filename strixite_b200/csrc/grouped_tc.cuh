@@ -41,6 +41,7 @@ struct TcArgs {
                   // 3 / 4 tile-blocked for a Q4 / Q8 down operand
     uint32_t *status;  // >= 3 words: {2, item, role} on a wait that ran out
     int64_t dense_M;   // > 0: a dense projection - no grouping workspace, one group holding rows 0 .. dense_M - 1 in order
+    int dense_tile;    // its rows a tile (the kernel for tile-blocked activations), a multiple of 16
     unsigned long long wait_limit_ns;  // bound of every device-side wait
     int test_skip_slot;  // >= 0: CTA 0 never issues ring slot number test_skip_slot, so a wait runs out (tests only)
     TcHcUp hc;           // kTcHcUp only

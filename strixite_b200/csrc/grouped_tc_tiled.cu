@@ -47,6 +47,7 @@
 
 #include "grouped_tc.cuh"
 
+#include <cmath>
 #include <type_traits>
 
 namespace sxb {
@@ -123,9 +124,9 @@ __device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
     Item it;
     const int tile = item / rbs;
     it.rb = item % rbs;
-    if (a.dense_M > 0) {  // dense projection: tile t holds rows kTile * t .. of the one group
-        it.bucket = 0, it.start = tile * kTile;
-        it.cnt = (int)min((int64_t)kTile, a.dense_M - it.start);
+    if (a.dense_M > 0) {  // dense projection: tile t holds rows dense_tile * t .. of the one group
+        it.bucket = 0, it.start = tile * a.dense_tile;
+        it.cnt = (int)min((int64_t)a.dense_tile, a.dense_M - it.start);
         return it;
     }
     it.bucket = a.ws[a.L.t128_bucket + tile];
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int n_steps = (int)a.K / kBK, groups = (int)a.K / G;
     const int rbs = row_blocks<MODE>(a);
-    const int n_items = (a.dense_M > 0 ? (int)((a.dense_M + kTile - 1) / kTile) : a.ws[3]) * rbs;
+    const int n_items = (a.dense_M > 0 ? (int)((a.dense_M + a.dense_tile - 1) / a.dense_tile) : a.ws[3]) * rbs;
     // slot (row of the output / of h) at position pos of the slot order; a dense projection's rows are in their own order
     auto slot_at = [&](int pos) -> int { return a.dense_M > 0 ? pos : a.ws[a.L.slots + pos]; };
     volatile int *abort_v = &abort_flag;
@@ -841,12 +842,28 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
 
 }  // namespace
 
+// Rows a tile of a dense projection has: 128 unless fewer fill the last wave of items better.  A step of 128 k takes about 450 + 3 n SM cycles for n
+// rows with Q4 codes and 650 + 3 n with Q8.  Tiles of 128 -> as chosen, us: 300 x 2048 x 4096 Q8 + SwiGLU 26.2 -> 22.6 (80 rows), 200 x 2560 x 4096 Q4
+// 20.5 -> 16.5 (64), 150 x 4096 x 4096 19.7 -> 17.9 (64), 777 x 4096 x 1024 Q8 18.5 -> 16.5 (96), 1001 x 8192 x 4096 Q4 53.4 -> 52.3 (112).
+int dense_tile_rows(int64_t M, int64_t row_blocks, int64_t steps, int bits, int sms) {
+    int best = kTile;
+    double least = 0;
+    for (int n = kTile; n >= 64; n -= 16) {
+        const double items = (double)((M + n - 1) / n) * (double)row_blocks, cost = std::ceil(items / sms) * (steps * ((bits == 4 ? 450 : 650) + 3.0 * n) + 1000);
+        if (least == 0 || cost < least) least = cost, best = n;
+    }
+    return best;
+}
+
 // Two boxes of 128 codes x 64 rows fill a ring slot; 16-byte chunks swizzled in the mode of the box's row length so that the
 // producers' 16-byte reads of consecutive rows hit every bank once.
 template <int BITS, int MODE>
 int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     SXB_CHECK(a.x_kind == 3, fn, ": the tiled tcgen05 kernel takes tile-blocked activations only");
     using S = Shape<BITS, MODE == kTcHcUp>;
+    a.dense_tile = kTile;
+    if (a.dense_M > 0 && MODE != kTcHcUp)
+        a.dense_tile = dense_tile_rows(a.dense_M, MODE == kTcSwiglu ? (a.N / 2 + kRows / 2 - 1) / (kRows / 2) : (a.N + kRows - 1) / kRows, a.K / kBK, BITS, sm_count());
     const uint64_t row_bytes = (uint64_t)(BITS == 4 ? a.K / 2 : a.K);
     CUtensorMap wmap;
     if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)(a.E * a.N), row_bytes, (uint32_t)(kBK * BITS / 8),
