@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kPackThreads)
 // segment's first invalid slot into segbad [nseg].
 __global__ void __launch_bounds__(32 * kSegWarps)
     pack_hist_kernel(const int32_t *__restrict__ ids, RouteWords L, int E_total, int e_lo, int32_t *ws) {
+    behind_grid();
     __shared__ int hist[kMoeMaxExperts + 1], first_bad;
     const int t = threadIdx.x, E = (int)L.E, S = (int)L.S, s0 = (int)blockIdx.x * kSegSlots;
     int32_t id[kSegRounds];
@@ -235,6 +236,7 @@ __global__ void __launch_bounds__(32 * kSegWarps)
 // the bucket); totals -> offsets, header, tile lists; the first invalid slot -> err.
 __global__ void __launch_bounds__(kPackThreads)
     pack_scan_kernel(const int32_t *__restrict__ ids, RouteWords L, bool ep, int32_t *ws, uint32_t *err) {
+    behind_grid();
     __shared__ Layout sm;
     const int b = threadIdx.x, E = (int)L.E;
     int total = 0;
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(kPackThreads)
 // launch: 15.5 us at 777 to 16384 tokens x 10 slots).
 __global__ void __launch_bounds__(32 * kSegWarps)
     pack_scatter_kernel(const int32_t *__restrict__ ids, RouteWords L, int e_lo, int32_t *ws) {
+    behind_grid();
     __shared__ __align__(4) uint16_t counts[kSegWarps][kMoeMaxExperts + 1];
     __shared__ Layout sm;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, E = (int)L.E, S = (int)L.S, s0 = (int)blockIdx.x * kSegSlots + warp * kSegRounds * 32;
@@ -328,9 +331,9 @@ int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64
         launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, err);
     } else {
         const unsigned ctas = (unsigned)L.nseg;
-        pack_hist_kernel<<<ctas, 32 * kSegWarps, 0, st>>>(ids, L, (int)E_total, (int)e_lo, w);
-        pack_scan_kernel<<<1, kPackThreads, 0, st>>>(ids, L, ep, w, err);
-        pack_scatter_kernel<<<ctas, 32 * kSegWarps, 0, st>>>(ids, L, (int)e_lo, w);
+        launch_behind(pack_hist_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)E_total, (int)e_lo, w);
+        launch_behind(pack_scan_kernel, 1, kPackThreads, 0, st, 1, ids, L, ep, w, err);
+        launch_behind(pack_scatter_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)e_lo, w);
     }
     SXB_CHECK_LAUNCH(fn, " M=", M, " A=", A, " E=", E_local);
     return SXB_OK;
