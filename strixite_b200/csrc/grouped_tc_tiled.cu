@@ -8,9 +8,9 @@
 //
 // What bounds it (B200, SM cycles per step, the pieces measured alone): the MMAs take max(305, 4 n) for n tokens (below 76
 // tokens reading the A operand bounds them); dequantizing 128 x 128 codes and storing them to tensor memory takes the sixteen
-// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 545 a step for 15 tokens
-// and 730 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions
-// (1400 to 1450 a step, 584 of them the dequantization, at 61 to 66 % of the slots).
+// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 510 a step for 15 tokens
+// and 700 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions (584 a step
+// of them the dequantization).  From some 80 tokens an expert on launches in a row run at the card's power limit, 1000 W at 1.3 to 1.4 GHz.
 //   * One lane's MMAs and commits count, but its whole warp runs the loop, under control flow that the compiler can see to be uniform:
 //     addresses and descriptors then live in uniform registers.  Run by one lane of a diverged warp the MMAs took no longer to issue, but
 //     the loop around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps
@@ -25,8 +25,8 @@
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
 // A wider token tile would not be cheaper: it shares a dequantization that is no longer the bound, and 128 columns leave tensor
 // memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column stages of A.
-// Measured, 512 experts, d = 4096, I = 1024, Q4: gate/up + SwiGLU 540 us at 777 tokens (15 an expert), 728 at
-// 4096 (80 an expert); down 304 and 435 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
+// Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 506 us at 777 tokens (15 an expert), 685 at
+// 4096 (80 an expert); down 291 and 480 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
 //
 // SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up

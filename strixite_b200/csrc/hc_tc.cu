@@ -3,19 +3,17 @@
 // x and h rounded once to F16, the weights dequantized to F16 (code * scale + min, one rounding), FP32 accumulation over
 // each product's whole K range; norms, gates and the stream combine in FP32.
 //
-// Both halves run on this library's tcgen05 expert kernels rather than on kernels of their own:
-//   down  a = sum_s inv[t, s] * (W'_s . X_s[t]) is a grouped projection with the H streams as H "experts": slot t * H + s
+//   down  runs on this library's tcgen05 expert kernel: a = sum_s inv[t, s] * (W'_s . X_s[t]) is a grouped projection with the H streams as H "experts": slot t * H + s
 //         holds the row X_s[t] (X [T, H*d] read as [T*H, d] IS that slot-major matrix), expert s the weight's column range
 //         [s d, (s + 1) d) restacked as rows [s Rp, (s + 1) Rp) of a [H * Rp, d] view (Rp = R rounded up to 16, the padding
 //         rows zero).  One pass over X computes inv and writes the tile-blocked F16 operand; the grouping workspace of that
-//         regular pattern is written directly (no ids, no sort); the grouped kernel leaves FP32 per-slot dots; a last pass folds them with
-//         inv, in stream order (kernels/hc_wmma.hip:136-150), into h and w_in.
-//   up    z = h W_up^T is a dense projection of h [T, r] on W_up [H*d, r], un-chunked to row-major with r padded to a
-//         multiple of 128 by zero groups and its rows put in the order that makes the four streams of an output column
-//         neighbours in tensor memory; the kernel's epilogue is the stream combine itself,
+//         regular pattern is written by formula under that pass (no ids, no sort); the grouped kernel leaves FP32 per-slot dots; a last pass
+//         folds them with inv, in stream order (kernels/hc_wmma.hip:136-150), into h and w_in.
+//   up    z = h W_up^T is a dense projection of h [T, r] on W_up [H*d, r], r padded to a multiple of 128 by zero groups, its rows in the order
+//         that makes the four streams of an output column neighbours in tensor memory; the kernel's epilogue is the stream combine itself,
 //         u = (1/H) sum_s sigmoid(z_s) * X_s * inv_s * (1 + norm_w_s) (kernels/hc_wmma.hip:244-272), so z never exists
-//         in memory.
-// The re-layouts of the two weights (a few MB) are done per call into the caller's workspace: the views an engine holds
+//         in memory.  Ranks up to 512: a kernel of its own (hc_up_tc_kernel).  Above: the general kernel, on W_up un-chunked to row-major.
+// The re-layouts of weights (a few MB) are done per call into the caller's workspace: the views an engine holds
 // stay the reference's (row-major folded down weight, chunk-major up weight), shared with the per-token kernels.
 
 #include "grouped_tc.cuh"
@@ -236,8 +234,9 @@ __global__ void __launch_bounds__(256) hc_stage_h_kernel(const float *__restrict
 // the general kernel, whose items dequantize their rows again for every 128 tokens, look for their powers of two and pass through its rings,
 // 11200 SM cycles, of which the MMAs take 1500.  Here a CTA takes neighbouring items, the tokens of a row block one after another, and the
 // block's weights stay in tensor memory: dequantized once or twice a CTA, straight from the chunk-major codes.
-// Warps: sixteen for the epilogue (a lane quadrant and 32 of an item's tokens each), four producers, MMA issue, activation copies.  Waits are
-// bounded; one that runs out raises the CTA's abort flag and is recorded in the library's status words.
+// Warps: sixteen for the epilogue, four producers, MMA issue, copies of h, copies of X.  Waits are bounded; one that runs out raises the CTA's abort
+// flag and is recorded in the library's status words.  4096 tokens, d = 4096, r = 320, Q8: 169 us and 6 for the re-layout -> 97, 6500 SM cycles an
+// item.  What bounds it: the epilogue's warps - latencies of shared memory and the special-function unit (33 % busy), issue slots 46 %.
 constexpr int kUpTile = 128, kUpSubBytes = kUpTile * 128, kUpStageBytes = 2 * kUpSubBytes, kUpSteps = 4;  // steps of 128 k at most
 constexpr int kUpEpiWarps = 16, kUpProducer = kUpEpiWarps, kUpMma = kUpEpiWarps + 4, kUpCopy = kUpEpiWarps + 5, kUpXCopy = kUpEpiWarps + 6,
               kUpThreads = 32 * (kUpEpiWarps + 7);

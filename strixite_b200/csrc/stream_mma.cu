@@ -28,9 +28,10 @@
 //     operands, which a dot product does not notice;
 //   * per step: D = sum over the quad's codes of q * x on the tensor cores (exact products, FP32 sums), then
 //     acc += s * D + m * sum(x) in FP32; the token's power of two comes off the finished dot.
-// Work is cut into units of 16 rows x one tile of <= 8 tokens of one expert; CTAs take contiguous ranges of units so
-// a CTA restages activations only when it crosses into another tile, and every touched expert's weights are read
-// once per tile (once in total when an expert has <= 8 tokens, the decode case).
+// Work is cut into units of 16 rows x one tile of <= 8 tokens of one expert; CTAs take contiguous ranges of units, and every touched
+// expert's weights are read once per tile (once in total when an expert has <= 8 tokens, the decode case).  The routed forms of a
+// grouping workspace run as stream_tiles_kernel, the next tile's activations staged under the streaming; the others, and rows too long for its
+// two buffers, as stream_kernel, which stages between tiles.
 
 #include "experts.cuh"
 #include "skinny_mma.cuh"

@@ -436,3 +436,31 @@ def test_down_mix_grouping_workspace(cuda, T):
     n8, n128 = int(ref[0]), int(ref[3])
     for lo, n in ((0, 8), (at["offsets"], H + 2), (at["slots"], S), (at["tile8_bucket"], n8), (at["tile8_start"], n8), (at["tile128_bucket"], n128), (at["tile128_start"], n128)):
         assert torch.equal(got[lo:lo + n], ref[lo:lo + n]), (lo, n)
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,G,T,d,r,spread", [(8, 64, 129, 128, 512, 0), (4, 32, 300, 1280, 416, 0), (8, 128, 700, 256, 384, 9), (4, 64, 65, 384, 192, 9), (8, 32, 1, 128, 32, 0),
+                                                 (4, 128, 260, 128, 512, 9), (8, 32, 200, 256, 544, 0), (4, 64, 130, 128, 1024, 9)])
+def test_hc_mix_up_wmma_ranks(cuda, oracle, dt, bits, G, T, d, r, spread):
+    """The up mix by rank: the kernel that keeps a row block's weights in tensor memory up to 512 (one to four steps, several tokens tiles and row blocks a
+    CTA, rows whose groups' scales lie 2^spread apart) and the general one above it."""
+    from strixite_b200 import kernels as K
+    rng, H = np.random.default_rng(T + r), 4
+    w, h = random_weights(rng, H * d, r, std=0.2), (rng.standard_normal((T, r)) * 0.5).astype(np.float32)
+    w[:, :G] *= 2.0 ** spread
+    h[:, :G] *= 2.0 ** -spread
+    wu = oracle.quantize(w, G, bits)
+    x, norm_w = rng.standard_normal((T, H * d)).astype(np.float32), (rng.standard_normal(H * d) * 0.1).astype(np.float32)
+    inv = (0.5 + rng.random((T, H))).astype(np.float32)
+    xd = torch.from_numpy(x).to(cuda).to(dt)
+    x = xd.float().cpu().numpy()
+    act = K.Act.BF16 if dt == torch.bfloat16 else K.Act.F32
+    u = torch.full((T, d), float("nan"), dtype=dt, device=cuda)
+    ws = _ws(K.hc_mix_up_wmma_workspace_bytes(T, H, d, r, bits, G), cuda)
+    K.hc_mix_up_wmma(torch.from_numpy(h).to(cuda), K.to_chunk_major(upload(wu, cuda)), xd, torch.from_numpy(norm_w).to(cuda), torch.from_numpy(inv).to(cuda), T, H, d, u,
+                     ws, act)
+    K.check_dense_status("hc_mix_up_wmma")
+    ref = oracle.hc_mix_up(h, wu, x, norm_w, inv, H, d, f16_operands=True)
+    got = u.float().cpu().numpy().astype(np.float64)
+    step = 2.0 ** -8 if dt == torch.bfloat16 else 0.0
+    assert np.all(np.abs(got - ref) <= step * np.abs(ref) + 2e-4 * np.sqrt(np.mean(np.square(ref))))
