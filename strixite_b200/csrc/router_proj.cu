@@ -4,7 +4,7 @@
 //
 // Two forms, by regime:
 //   * streaming (decode, a few dozen tokens): sixteen weight rows by a cluster of CTAs, each warp a part of their contraction against
-//     sixteen tokens at a time on the warp-level tensor-core path, FP32 weights as three BF16 planes split in registers;
+//     sixteen tokens at a time, up to 64 a CTA, on the warp-level tensor-core path, FP32 weights as three BF16 planes split in registers;
 //   * tcgen05 (prefill, thousands of tokens): a plain tensor-core GEMM with both operands staged by tensor copies.  The
 //     weight is the reference's BF16 [N, K], or an FP32 one split once, at load time, into P BF16 "planes"
 //     W = W1 + W2 (+ W3) (each plane the BF16 rounding of what the planes before it left over), so that the products
@@ -27,6 +27,7 @@ namespace {
 // ---- streaming form ------------------------------------------------------------------------------------------
 
 constexpr int kStreamSplit = 8, kStreamWarps = 8;  // CTAs of a cluster, and warps of a CTA, that share 16 weight rows
+constexpr int kStreamEights = 8;                   // eights of tokens a CTA takes at most
 
 // A lane's eight consecutive weights of a row: the BF16 planes they consist of.
 template <typename TW>
@@ -101,14 +102,16 @@ __device__ inline float formed_again(bool bad, float sum, int64_t t, int64_t n, 
 // runs a warp), and the parts are added in order, across the warps in shared memory and then across the cluster.  FP32 weights go
 // through the tensor cores as three BF16 planes (skinny_mma.cuh): exact products, each plane's sum apart, so that the arithmetic is
 // no less than an FP32 multiply-add chain's (error against 64 bits 1.1e-7 -> 0.9e-7) and a token costs an MMA's column of it, not 16 dots
-// a CTA whether they live or not.  513 x 4096 FP32, as a CUDA graph: 1 token 8.1 -> 4.0 us, 16 11.7 -> 4.8, 37 29 -> 12, 127 82 -> 31.  What bounds
-// it: the launch, one round trip to memory, the meeting of the parts.
+// a CTA whether they live or not.  513 x 4096 FP32, as a CUDA graph: 1 token 8.1 -> 4.1 us, 16 11.7 -> 4.5, 37 29 -> 6.1, 127 82 -> 14.
+// Above sixteen tokens a warp keeps its weights, split, for one pair of eights after another: the same sums, FP32 8192 x 4096, 300 tokens 1230 -> 513 us
+// (with groups of sixteen each was another CTA, which loaded and split them again).  What bounds it: the launch, one round trip to memory, the meeting of the parts.
 template <typename TW, typename TOUT, int NT>
 __global__ void __launch_bounds__(32 * kStreamWarps, 2)
     logits_stream_kernel(const uint16_t *__restrict__ x, const TW *__restrict__ w, const float *__restrict__ bias, int64_t M,
                          int64_t N, int64_t K, TOUT *__restrict__ y, int64_t ld) {
     behind_grid();
-    constexpr int kTok = kMmaTokens * NT, kAhead = Weights<TW>::kAhead, P = Weights<TW>::kPlanes;
+    constexpr int kTok = kMmaTokens * NT, kBatch = NT < 2 ? NT : 2, kAhead = Weights<TW>::kAhead, P = Weights<TW>::kPlanes;
+    constexpr bool kKept = NT > kBatch;  // the split weights stay in registers for one batch of tokens after another
     __shared__ float part[kStreamWarps][kTok][kMmaRows + 1];
     __shared__ float cta_part[kTok][kMmaRows];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
@@ -118,12 +121,12 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 2)
     const int64_t runs = (K + kMmaRun - 1) / kMmaRun, at = rank * kStreamWarps + warp, parts = kStreamSplit * kStreamWarps;
     const int64_t lo = runs * at / parts, hi = runs * (at + 1) / parts;
     for (int64_t t0 = (int64_t)blockIdx.y * kTok; t0 < M; t0 += (int64_t)gridDim.y * kTok) {
-        float acc[NT][4];
+        const int live = (int)min((int64_t)NT, (M - t0 + kMmaTokens - 1) / kMmaTokens);  // eights of tokens in this group
+        float acc[kBatch][4];  // of up to kBatch eights; more have their sums in `part` itself
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-        for (int64_t r0 = lo; r0 < hi; r0 += kAhead) {
+        for (int b = 0; b < kBatch; ++b) acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.f;
+        for (int64_t r0 = lo; (kKept && r0 == lo) || r0 < hi; r0 += kAhead) {  // a warp without runs: parts of zero
             Weights<TW> va[kAhead], vb[kAhead];
-            uint4 xv[kAhead][NT];
             bool in[kAhead];
 #pragma unroll
             for (int e = 0; e < kAhead; ++e) {
@@ -132,46 +135,62 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 2)
                 if (in[e]) va[e].load(wa + k), vb[e].load(wb + k);
                 else va[e].clear(), vb[e].clear();
             }
+            uint4 xv[kBatch][kAhead], pa[kAhead][P], pb[kAhead][P];
+            auto fetch = [&](int nt0) {
 #pragma unroll
-            for (int e = 0; e < kAhead; ++e)
+                for (int b = 0; b < kBatch; ++b)
 #pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-                    const int64_t t = t0 + nt * kMmaTokens + g;
-                    xv[e][nt] = in[e] && t < M ? __ldg(reinterpret_cast<const uint4 *>(x + t * K + (r0 + e) * kMmaRun + 8 * c)) : make_uint4(0u, 0u, 0u, 0u);
-                }
-            float dot[P][NT][4];
+                    for (int e = 0; e < kAhead; ++e) {
+                        const int64_t t = t0 + (nt0 + b) * kMmaTokens + g;
+                        xv[b][e] = in[e] && t < M ? __ldg(reinterpret_cast<const uint4 *>(x + t * K + (r0 + e) * kMmaRun + 8 * c)) : make_uint4(0u, 0u, 0u, 0u);
+                    }
+            };
+            fetch(0);
+            if constexpr (kKept) {
 #pragma unroll
-            for (int p = 0; p < P; ++p)
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) dot[p][nt][0] = dot[p][nt][1] = dot[p][nt][2] = dot[p][nt][3] = 0.f;
-#pragma unroll
-            for (int e = 0; e < kAhead; ++e) {
-                if (r0 + e >= hi) break;
-                uint4 pa[P], pb[P];
-                va[e].planes(pa), vb[e].planes(pb);
-#pragma unroll
-                for (int p = 0; p < P; ++p)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) mma_run(dot[p][nt], pa[p], pb[p], xv[e][nt]);
+                for (int e = 0; e < kAhead; ++e) va[e].planes(pa[e]), vb[e].planes(pb[e]);
             }
+#pragma unroll 1
+            for (int nt0 = 0; nt0 < (kKept ? live : 1); nt0 += kBatch) {
+                float dot[kBatch][P][4];
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
+                for (int b = 0; b < kBatch; ++b)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float sum = dot[P - 1][nt][i];
+                    for (int p = 0; p < P; ++p) dot[b][p][0] = dot[b][p][1] = dot[b][p][2] = dot[b][p][3] = 0.f;
 #pragma unroll
-                    for (int p = P - 2; p >= 0; --p) sum += dot[p][nt][i];
-                    acc[nt][i] += sum;
+                for (int e = 0; e < kAhead; ++e) {
+                    if (r0 + e >= hi) break;
+                    if constexpr (!kKept) va[e].planes(pa[e]), vb[e].planes(pb[e]);
+#pragma unroll
+                    for (int p = 0; p < P; ++p)
+#pragma unroll
+                        for (int b = 0; b < kBatch; ++b) mma_run(dot[b][p], pa[e][p], pb[e][p], xv[b][e]);
                 }
-        }
+                if (kKept && nt0 + kBatch < live) fetch(nt0 + kBatch);
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            const int t = nt * kMmaTokens + 2 * c;
-            part[warp][t][g] = acc[nt][0], part[warp][t + 1][g] = acc[nt][1];
-            part[warp][t][g + 8] = acc[nt][2], part[warp][t + 1][g + 8] = acc[nt][3];
+                for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float sum = dot[b][P - 1][i];
+#pragma unroll
+                        for (int p = P - 2; p >= 0; --p) sum += dot[b][p][i];
+                        if constexpr (kKept) {
+                            float &to = part[warp][(nt0 + b) * kMmaTokens + 2 * c + (i & 1)][g + 8 * (i >> 1)];
+                            to = r0 == lo ? sum : to + sum;
+                        } else {
+                            acc[b][i] += sum;
+                        }
+                    }
+            }
+        }
+        if constexpr (!kKept) {
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) part[warp][b * kMmaTokens + 2 * c + (i & 1)][g + 8 * (i >> 1)] = acc[b][i];
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < kTok * kMmaRows; i += 32 * kStreamWarps) {
+        for (int i = threadIdx.x; i < (kKept ? live * kMmaTokens : kTok) * kMmaRows; i += 32 * kStreamWarps) {
             float sum = 0.f;
 #pragma unroll
             for (int v = 0; v < kStreamWarps; ++v) sum += part[v][i / kMmaRows][i % kMmaRows];
@@ -179,10 +198,10 @@ __global__ void __launch_bounds__(32 * kStreamWarps, 2)
         }
         cluster_sync();
         // a CTA finishes every eighth token of the group
-        if (warp == 0) {
-            const int tt = rank + kStreamSplit * (lane / kMmaRows), row = lane % kMmaRows;
+        if (warp < (NT * kMmaRows + 31) / 32) {
+            const int tt = rank + kStreamSplit * ((int)threadIdx.x / kMmaRows), row = lane % kMmaRows;
             const int64_t n = n0 + row, t = t0 + tt;
-            const bool out = lane < NT * kMmaRows && n < N && t < M;
+            const bool out = threadIdx.x < NT * kMmaRows && n < N && t < M;
             float sum = 0.f;
             if (out) {
                 float v[kStreamSplit];
@@ -497,17 +516,24 @@ int check_proj(const char *fn, const void *x, const void *w, const void *y, int6
 template <typename TOUT>
 int launch_stream_logits(const char *fn, const void *x, const void *w, int w_act, const float *bias, int64_t M, int64_t N, int64_t K,
                          TOUT *y, int64_t ld, cudaStream_t st) {
-    const int NT = M <= kMmaTokens ? 1 : 2;  // eights of tokens a CTA takes; a second group's weights come from L2
-    const dim3 grid((unsigned)((N + kMmaRows - 1) / kMmaRows * kStreamSplit), (unsigned)std::min<int64_t>((M + NT * kMmaTokens - 1) / (NT * kMmaTokens), 65535));
+    // Eights of tokens a CTA takes: two while the launch then fits the machine at two CTAs an SM (65 rows, 37 tokens: 3.6 us against 4.6), else eight,
+    // for which the weights are loaded and split once (513 rows, 17 / 37 / 127 tokens: 8.0 -> 5.2, 12.1 -> 6.1, 30.6 -> 14).
+    const int64_t by_row = (N + kMmaRows - 1) / kMmaRows * kStreamSplit;
+    const int NT = M <= kMmaTokens ? 1 : M <= 2 * kMmaTokens || by_row * ((M + 2 * kMmaTokens - 1) / (2 * kMmaTokens)) <= 2 * sm_count() ? 2 : kStreamEights;
+    const dim3 grid((unsigned)by_row, (unsigned)std::min<int64_t>((M + NT * kMmaTokens - 1) / (NT * kMmaTokens), 65535));
     auto xb = static_cast<const uint16_t *>(x);
     auto launch = [&](auto kern, auto *wt) { return launch_behind(kern, grid, dim3(32 * kStreamWarps), 0, st, kStreamSplit, xb, wt, bias, M, N, K, y, ld); };
     cudaError_t e;
     if (w_act == SXB_ACT_F32) {
         auto wt = static_cast<const float *>(w);
-        e = NT == 1 ? launch(logits_stream_kernel<float, TOUT, 1>, wt) : launch(logits_stream_kernel<float, TOUT, 2>, wt);
+        e = NT == 1   ? launch(logits_stream_kernel<float, TOUT, 1>, wt)
+            : NT == 2 ? launch(logits_stream_kernel<float, TOUT, 2>, wt)
+                      : launch(logits_stream_kernel<float, TOUT, kStreamEights>, wt);
     } else {
         auto wt = static_cast<const uint16_t *>(w);
-        e = NT == 1 ? launch(logits_stream_kernel<uint16_t, TOUT, 1>, wt) : launch(logits_stream_kernel<uint16_t, TOUT, 2>, wt);
+        e = NT == 1   ? launch(logits_stream_kernel<uint16_t, TOUT, 1>, wt)
+            : NT == 2 ? launch(logits_stream_kernel<uint16_t, TOUT, 2>, wt)
+                      : launch(logits_stream_kernel<uint16_t, TOUT, kStreamEights>, wt);
     }
     SXB_CUDA(e, fn, ": launching M=", M, " N=", N, " K=", K);
     SXB_CHECK_LAUNCH(fn, " M=", M, " N=", N, " K=", K);

@@ -83,6 +83,25 @@ def test_router_logits_streaming_edges(cuda, oracle, M, N, K, w_bf16):
     assert np.array_equal(got2[bad], want2[bad], equal_nan=True) and np.array_equal(got2[~bad], out.cpu().numpy()[~bad])
 
 
+@pytest.mark.parametrize("w_bf16", [False, True])
+@pytest.mark.parametrize("M,N,K", [(17, 513, 4096), (24, 600, 8), (63, 530, 4128), (64, 513, 8192), (65, 514, 1000), (129, 520, 12296), (37, 65, 4096)])
+def test_router_logits_streaming_eights(cuda, M, N, K, w_bf16):
+    """Above sixteen tokens and a machine full of CTAs, a CTA keeps its weights for eight eights of tokens: groups full, partly filled and one over,
+    an odd number of eights, contractions of one pass of a warp's registers, several, and none.  A token's sums do not depend on its group: every row has the
+    bits of the call for that token by itself."""
+    from strixite_b200 import kernels as Kn
+    gen = torch.Generator(device="cpu").manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=gen).to(cuda).to(torch.bfloat16)
+    w = (torch.randn(N, K, generator=gen) * 0.02).to(cuda).to(torch.bfloat16 if w_bf16 else torch.float32)
+    bias = torch.randn(N, generator=gen).to(cuda)
+    out = torch.full((M, N + 2), float("nan"), device=cuda)
+    Kn.router_logits(x, w, bias, out)
+    one = torch.empty((M, N), device=cuda)
+    for m in range(M):
+        Kn.router_logits(x[m:m + 1], w, bias, one[m:m + 1])
+    assert torch.equal(out[:, :N], one) and bool(torch.isnan(out[:, N:]).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 17, 64), (16, 513, 4096), (37, 33, 1000)])
 def test_router_logits_streaming_third_plane(cuda, oracle, M, N, K):
     """FP32 weights whose last bits are all that is left of a logit: pairs 1 + 2^-8 + k 2^-23 and -(1 + 2^-8) against the same activation, a
