@@ -656,8 +656,9 @@ int mix_up_tc(const float *h, const SxbQView *w, const void *x, const float *nor
     SXB_CHECK(w->N == H * d, fn, ": W_up has ", w->N, " rows, expected H*d = ", H * d);
     SXB_CHECK(w->K >= kChunk && w->K <= kMaxRank && w->K % kChunk == 0, fn, ": W_up K (the rank r) = ", w->K, ", expected a multiple of ", kChunk,
               " up to ", kMaxRank);
-    SXB_CHECK(aligned16(h) && aligned16(x) && aligned16(norm_w) && aligned16(u) && reinterpret_cast<uintptr_t>(ws) % 256 == 0, fn,
-              ": h, x, norm_w and u must be 16-byte and the workspace 256-byte aligned");
+    // inv: both kernels fetch a token's four of it as one 16-byte piece
+    SXB_CHECK(aligned16(h) && aligned16(x) && aligned16(norm_w) && aligned16(inv) && aligned16(u) && reinterpret_cast<uintptr_t>(ws) % 256 == 0, fn,
+              ": h, x, norm_w, inv and u must be 16-byte and the workspace 256-byte aligned");
     SXB_CHECK(w->K % 8 == 0, fn, ": r = ", w->K, " must be a multiple of 8");
     SXB_CHECK(apart(u, T * d * act_bytes(act), x, T * H * d * act_bytes(act)), fn, ": u overlaps the streams x");
     const int64_t r = w->K, Kp = up128(r), N = H * d;

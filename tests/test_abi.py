@@ -167,3 +167,17 @@ def test_hc_wmma_workspace_sizes_and_preconditions(lib):
         K.hc_inject_inv(1 << 20, 4096, 8192, 4, 4, 64, 0.0, 16384, K.Act.BF16, stream=0)
     with pytest.raises(K.Error, match="y overlaps the streams"):
         K.hc_inject_inv(1 << 20, 4096, (1 << 20) + 64, 4, 4, 64, 1e-6, 16384, K.Act.BF16, stream=0)
+
+
+@pytest.mark.parametrize("r", [64, 512, 544, 1024])
+@pytest.mark.parametrize("bits", [4, 8])
+def test_up_mix_refuses_an_unaligned_inv(lib, bits, r):
+    """Both tensor-core forms of the up mix fetch a token's four inv at once (16 bytes, from 16-byte boundaries): an array that starts between
+    two is refused on the host, before anything is enqueued."""
+    from strixite_b200 import _lib
+    T, H, d, G = 130, 4, 256, 32
+    w = _lib.SxbQView(1 << 20, 2 << 20, 3 << 20, H * d, r, G)
+    need = lib.sxb_hc_mix_up_wmma_workspace_bytes(T, H, d, r, bits, G)
+    for off in (4, 8, 12):
+        rc = getattr(lib, f"sxb_hc_mix_up_wmma_q{bits}")(4 << 20, C.byref(w), 5 << 20, 6 << 20, (7 << 20) + off, T, H, d, 8 << 20, 16 << 20, need, 1, None)
+        assert rc == 1 and "inv" in lib.sxb_last_error().decode() and "16-byte" in lib.sxb_last_error().decode()
