@@ -252,7 +252,9 @@ int sxb_moe_group_routes_ep(const int32_t *ids, int64_t M, int64_t A, int64_t E_
 int sxb_route_layout(int64_t M, int64_t A, int64_t E, int64_t out[8]);
 
 /* No counterpart in the reference.  Bound of every device-side wait of the tcgen05 kernels for the launches that follow
- * (process-wide; default 2 s, minimum 1 us).  A wait that runs out ends its kernel with the status words set. */
+ * (process-wide; default 2 s, minimum 1 us).  A wait that runs out ends its kernel with the status words set.  The exact grouped
+ * forms (SXB_MATH_F32, SXB_MATH_WMMA_BF16) wait inside a CTA too, for another warp's share of the work: their bound is this one or
+ * 2 s, whichever is longer. */
 int sxb_set_wait_limit(uint64_t nanoseconds);
 /* Test hook, no counterpart in the reference: slot >= 0 makes CTA 0 of the following tcgen05 launches leave that fill of
  * its weight-code ring out, so a bounded wait runs out and the kernel's give-up path runs; -1 (the default) = off. */

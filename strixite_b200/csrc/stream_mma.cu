@@ -1074,7 +1074,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
         if (kTileBufs * smem <= kMaxDynSmem) {
             auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
             SXB_CUDA(cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
-            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = wait_limit_ns();
+            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns();
             launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
             return SXB_OK;
         }

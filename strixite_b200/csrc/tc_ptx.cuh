@@ -17,6 +17,9 @@ int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, i
                   uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map);
 int library_status_words(const char *fn, uint32_t **out);
 unsigned long long wait_limit_ns();
+// ... of the streaming expert kernel's, which wait for a whole unit of another warp as a matter of course: never below the default, whatever a
+// host allows the tcgen05 kernels.
+unsigned long long stream_wait_limit_ns();
 
 // ---- PTX wrappers ----------------------------------------------------------------------------------------------
 __device__ inline uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

@@ -631,3 +631,32 @@ def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
     torch.cuda.synchronize()
     K.check_dense_status("two streams")
     assert not bad and lib.sxb_release_scratch() == 0
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_a_short_wait_limit_leaves_the_exact_forms_whole(cuda, oracle, swiglu):
+    """sxb_set_wait_limit is for the tcgen05 kernels: in the exact grouped forms a warp waits for another's unit or row as a matter of course, longer
+    than a host may allow those.  A unit a tile, long rows, and tokens that take the slow way for small activations: every tile waits for one warp."""
+    from strixite_b200 import kernels as Kn
+    M, A, E, N, Kd, G = 4000, 2, 40, 16, 6144, 64
+    g = torch.Generator(device="cuda").manual_seed(3)
+    w = Kn.quantize(torch.randn((E * N, Kd), generator=g, device=cuda) * 0.02, G, 8)
+    x = torch.randn((M, Kd), generator=g, device=cuda).to(torch.bfloat16)
+    x[:, :9] = 2.0 ** -36
+    ids = torch.rand((M, E), generator=g, device=cuda).topk(A, dim=1).indices.to(torch.int32)
+    err = torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = Kn.moe_route_workspace_bytes(M, A, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    Kn.moe_group_routes(ids, M, A, E, ws, nbytes, err)
+    grouped = Kn.linear_qw_experts_gather_grouped_swiglu if swiglu else Kn.linear_qw_experts_gather_grouped
+    out = [torch.full((M * A, N // 2 if swiglu else N), float("nan"), dtype=torch.bfloat16, device=cuda) for _ in range(2)]
+    grouped(x, w, E, ws, nbytes, M, A, out[0], Kn.Act.BF16, Kn.MoeMath.F32)
+    torch.cuda.synchronize()
+    try:
+        Kn.set_wait_limit(1000)
+        grouped(x, w, E, ws, nbytes, M, A, out[1], Kn.Act.BF16, Kn.MoeMath.F32)
+        torch.cuda.synchronize()
+    finally:
+        Kn.set_wait_limit(2_000_000_000)
+    Kn.check_grouped_status(ws, "a limit of 1 us")
+    assert torch.equal(out[0], out[1]) and not bool(torch.isnan(out[0]).any())
