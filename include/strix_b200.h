@@ -237,9 +237,10 @@ int sxb_moe_group_routes(const int32_t *ids, int64_t M, int64_t A, int64_t E, vo
 int sxb_moe_route_small(const float *logits, int64_t ld, int64_t M, int64_t E_total, int64_t k, int64_t e_lo, int64_t E_local,
                         int32_t *ids, float *coef, void *ws, size_t ws_bytes, uint32_t *router_err, uint32_t *expert_err,
                         sxb_stream_t stream);
-/* No counterpart in the reference.  The tcgen05 grouped kernels bound every device-side wait; one that runs out writes
- * {2, work item, role} into words 5..7 of the workspace header (zeroed by every pack) and the kernel returns.  This
- * reads the header back (it synchronizes, like sxb_check_expert_error) and returns SXB_ERR_DATA if that happened. */
+/* No counterpart in the reference.  The grouped kernels, the tcgen05 ones and those of the exact forms (SXB_MATH_F32,
+ * SXB_MATH_WMMA_BF16), bound every device-side wait; one that runs out writes {2, work item, role} into words 5..7 of the
+ * workspace header (zeroed by every pack) and ends the kernel, whose outputs are then incomplete.  This reads the header
+ * back (it synchronizes, like sxb_check_expert_error) and returns SXB_ERR_DATA if that happened. */
 int sxb_check_grouped_status(const void *ws, const char *what);
 /* No counterpart in the reference (which has one GPU).  The expert-parallel form: this rank owns experts
  * [e_lo, e_lo + E_local) of E_total; bucket b = expert e_lo + b; slots of other ranks' experts and invalid ids go to

@@ -364,7 +364,8 @@ RouteWords route_words(int64_t M, int64_t A, int64_t E) {
 using namespace sxb;
 
 namespace sxb {
-// {2, work item, role}: the record of a device-side wait of the tcgen05 kernels that ran out (grouped_tc.cu).
+// {2, work item, role}: the record of a device-side wait that ran out, of the tcgen05 kernels (grouped_tc.cu) or of the exact grouped forms
+// (kRoleStaged and kRoleLeft, the item being a tile of eight tokens).
 int tc_status_error(const char *what, const uint32_t e[3]) {
     static const char *roles[] = {"an unknown role",
                                   "a weight producer waiting for a free operand stage",
@@ -375,9 +376,13 @@ int tc_status_error(const char *what, const uint32_t e[3]) {
                                   "the weight-code copy thread waiting for a free ring slot",
                                   "a weight producer waiting for its packed codes",
                                   "a warp waiting for the description of its next work item",
-                                  "the work-item thread waiting for room in its ring"};
-    last_error() = cat(what ? what : "", ": a tcgen05 kernel gave up a wait at work item ", e[1], " (",
-                       roles[e[2] >= 1 && e[2] <= 9 ? e[2] : 0], "); its outputs are incomplete");
+                                  "the work-item thread waiting for room in its ring",
+                                  "a warp waiting for the tile's staged activations",
+                                  "a staging warp waiting for the last warp to leave its buffer"};
+    static_assert(sizeof(roles) / sizeof(roles[0]) == kRoleLeft + 1, "a text for each role");
+    const bool streaming = e[2] == kRoleStaged || e[2] == kRoleLeft;
+    last_error() = cat(what ? what : "", streaming ? ": the streaming expert kernel gave up a wait at tile " : ": a tcgen05 kernel gave up a wait at work item ",
+                       e[1], " (", roles[e[2] >= 1 && e[2] <= kRoleLeft ? e[2] : 0], "); its outputs are incomplete");
     return SXB_ERR_DATA;
 }
 }  // namespace sxb

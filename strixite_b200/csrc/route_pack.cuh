@@ -23,6 +23,10 @@ struct RouteWords {
 };
 RouteWords route_words(int64_t M, int64_t A, int64_t E);
 
+// Roles of the exact grouped forms in the status words (header words 5 .. 7), behind those of the tcgen05 kernels: a warp that waits for a tile's
+// staged activations, a staging warp that waits for the last warp to leave the buffer.
+constexpr int kRoleStaged = 10, kRoleLeft = 11;
+
 // The workspace of the grouping in which slot m * E + b belongs to bucket b, for all m < per_bucket: what sxb_moe_group_routes writes for
 // ids[m * E + b] = b, without the ids or the sort.  L = route_words(per_bucket * E, 1, E); by threads first, first + stride, ...
 __device__ inline void write_regular_routes(const RouteWords &L, int64_t per_bucket, int32_t *ws, int64_t first, int64_t stride) {

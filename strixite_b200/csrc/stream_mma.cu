@@ -889,16 +889,16 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const Stre
     __syncthreads();
     if (kKeepLow<BITS> && s_low) finish_staging<BITS, G>(a.x, K, bufs[0].row, xs_of(0), xsum_of(0), bufs[0].tok);
 
-    auto wait = [&](uint64_t *bar, uint32_t parity, int tile) {
+    auto wait = [&](uint64_t *bar, uint32_t parity, int tile, int role) {
         const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, nullptr, a.wait_limit_ns));
-        if (!ok && lane == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) a.status[1] = (uint32_t)tile, a.status[2] = 8u;
+        if (!ok && lane == 0 && atomicCAS(&a.status[0], 0u, 2u) == 0u) a.status[1] = (uint32_t)tile, a.status[2] = (uint32_t)role;
         return ok;
     };
     for (int tile = tile0; tile <= tile1; ++tile) {
         const int j = tile - tile0, b = j & 1;
         const uint32_t turn = (uint32_t)((j - 1) >> 1) & 1u;  // of this tile's `staged` and of the last one's `left`
         TileBuf &t = bufs[b];
-        if (j > 0 && !wait(&staged[b], turn, tile)) return;
+        if (j > 0 && !wait(&staged[b], turn, tile, kRoleStaged)) return;
         const int low = kKeepLow<BITS> && __any_sync(0xffffffffu, t.tok[lane & (kTileTokens - 1)].n_low != 0);
         const int hi = tile == tile1 ? u1 : units_per_tile;
         bool to_stage = tile < tile1 && warp < kTileTokens;
@@ -906,7 +906,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const Stre
             if (to_stage && (again || j == 0 || __all_sync(0xffffffffu, mbar_test(&left[b ^ 1], turn)))) {
                 to_stage = false;
                 TileBuf &n = bufs[b ^ 1];
-                if (j > 0 && !wait(&left[b ^ 1], turn, tile)) return;
+                if (j > 0 && !wait(&left[b ^ 1], turn, tile, kRoleLeft)) return;
                 if (lane == 0) describe(n, tile + 1, warp);
                 __syncwarp();
                 if (n.row[warp] >= 0) stage_token<BITS, G>(a.x + n.row[warp] * K, K, warp, xs_of(b ^ 1), xsum_of(b ^ 1), &n.tok[warp]);

@@ -660,3 +660,19 @@ def test_a_short_wait_limit_leaves_the_exact_forms_whole(cuda, oracle, swiglu):
         Kn.set_wait_limit(2_000_000_000)
     Kn.check_grouped_status(ws, "a limit of 1 us")
     assert torch.equal(out[0], out[1]) and not bool(torch.isnan(out[0]).any())
+
+
+def test_status_words_name_the_kernel_that_gave_up(cuda):
+    """The record of a wait that ran out, as words: the exact grouped forms have roles of their own, and a message that names them and their tile."""
+    from strixite_b200 import kernels as Kn
+    ws = torch.zeros(8, dtype=torch.int32, device=cuda)
+    for words, text in (((0, 0, 0), None), ((2, 7, 8), r"a tcgen05 kernel gave up a wait at work item 7 \(a warp waiting for the description of its next work item\)"),
+                        ((2, 5, 9), r"a tcgen05 kernel gave up a wait at work item 5 \(the work-item thread"), ((2, 3, 12), "a tcgen05 kernel .* unknown role"),
+                        ((2, 41, 10), r"the streaming expert kernel gave up a wait at tile 41 \(a warp waiting for the tile's staged activations\); its outputs are incomplete"),
+                        ((2, 42, 11), r"the streaming expert kernel gave up a wait at tile 42 \(a staging warp waiting")):
+        ws[5:8] = torch.tensor(words, dtype=torch.int32)
+        if text is None:
+            Kn.check_grouped_status(ws, "clean")
+        else:
+            with pytest.raises(Kn.Error, match="L0: " + text):
+                Kn.check_grouped_status(ws, "L0")
