@@ -787,6 +787,7 @@ int launch_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
 }  // namespace
 
 unsigned long long wait_limit_ns() { return g_wait_limit_ns; }
+int test_skip_slot() { return g_test_skip_slot; }
 unsigned long long stream_wait_limit_ns() { return std::max(g_wait_limit_ns, kWaitLimitNs); }
 
 int library_status_words(const char *fn, uint32_t **out) {

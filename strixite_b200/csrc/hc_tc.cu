@@ -257,6 +257,7 @@ struct HcUpArgs {
     int r, G, steps;
     uint32_t *status;
     unsigned long long wait_limit_ns;
+    int test_skip_slot;  // >= 0: CTA 0 never issues the copies of that stage fill of h, so that a wait runs out (tests only)
 };
 
 // 2^v and 1 / v on the special-function unit, results below 2^-126 as zero: the one is added to one, the other is of a sum of one or more.
@@ -377,6 +378,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
                         raise_abort(i, 5);
                         break;
                     }
+                    if (blockIdx.x == 0 && (int)count == a.test_skip_slot) continue;
                     const uint32_t dst = smem_u32(smem) + stage * (uint32_t)kUpStageBytes;
                     mbar_expect_tx(&b_full[stage], 2 * bytes);
                     bulk_g2s(dst, src, bytes, &b_full[stage]);
@@ -672,7 +674,7 @@ int mix_up_tc(const float *h, const SxbQView *w, const void *x, const float *nor
     hc_stage_h_kernel<BITS><<<stage_blocks, 256, 0, st>>>(h, T, r, Kp, base + L.hs);
     SXB_CHECK_LAUNCH(fn, " staging h, T=", T, " r=", r);
     if (Kp <= kUpSteps * 128) {
-        HcUpArgs a{base + L.hs, w->q, w->scale, w->minv, inv, norm_w, u, T, d, (int)r, (int)w->G, (int)(Kp / 128), nullptr, wait_limit_ns()};
+        HcUpArgs a{base + L.hs, w->q, w->scale, w->minv, inv, norm_w, u, T, d, (int)r, (int)w->G, (int)(Kp / 128), nullptr, wait_limit_ns(), test_skip_slot()};
         if (int rc = library_status_words(fn, &a.status)) return rc;
         return act == SXB_ACT_F32 ? launch_hc_up<BITS, float>(fn, a, x, st) : launch_hc_up<BITS, uint16_t>(fn, a, x, st);
     }

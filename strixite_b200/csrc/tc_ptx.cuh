@@ -20,6 +20,7 @@ unsigned long long wait_limit_ns();
 // ... of the streaming expert kernel's, which wait for a whole unit of another warp as a matter of course: never below the default, whatever a
 // host allows the tcgen05 kernels.
 unsigned long long stream_wait_limit_ns();
+int test_skip_slot();  // sxb_test_skip_ring_slot: the fill that CTA 0 leaves out, -1 = none
 
 // ---- PTX wrappers ----------------------------------------------------------------------------------------------
 __device__ inline uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }

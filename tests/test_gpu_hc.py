@@ -464,3 +464,34 @@ def test_hc_mix_up_wmma_ranks(cuda, oracle, dt, bits, G, T, d, r, spread):
     got = u.float().cpu().numpy().astype(np.float64)
     step = 2.0 ** -8 if dt == torch.bfloat16 else 0.0
     assert np.all(np.abs(got - ref) <= step * np.abs(ref) + 2e-4 * np.sqrt(np.mean(np.square(ref))))
+
+
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("bits,T,d,r,slot", [(8, 200, 256, 512, 0), (4, 130, 128, 320, 2), (8, 700, 4096, 320, 7), (4, 130, 128, 1024, 3)])
+def test_up_mix_gives_up_a_wait(cuda, oracle, lib, dt, bits, T, d, r, slot):
+    """Both kernels of the tensor-core up mix (the line is rank 512) with CTA 0 told to leave one fill of its operand ring out: in the first item or in a
+    later one, whose predecessors' copies, products and epilogues are under way.  The kernel returns, the status names it, the next call is right."""
+    from strixite_b200 import kernels as K
+    rng, H, G = np.random.default_rng(T + r), 4, 32
+    w, h = random_weights(rng, H * d, r, std=0.2), (rng.standard_normal((T, r)) * 0.5).astype(np.float32)
+    wu = oracle.quantize(w, G, bits)
+    x, norm_w = rng.standard_normal((T, H * d)).astype(np.float32), (rng.standard_normal(H * d) * 0.1).astype(np.float32)
+    inv = (0.5 + rng.random((T, H))).astype(np.float32)
+    xd, act = torch.from_numpy(x).to(cuda).to(dt), K.Act.BF16 if dt == torch.bfloat16 else K.Act.F32
+    args = [torch.from_numpy(h).to(cuda), K.to_chunk_major(upload(wu, cuda)), xd, torch.from_numpy(norm_w).to(cuda), torch.from_numpy(inv).to(cuda), T, H, d]
+    ws, u = _ws(K.hc_mix_up_wmma_workspace_bytes(T, H, d, r, bits, G), cuda), [torch.full((T, d), float("nan"), dtype=dt, device=cuda) for _ in range(3)]
+    K.hc_mix_up_wmma(*args, u[0], ws, act)
+    K.check_dense_status("warm-up")
+    try:
+        K.set_wait_limit(2_000_000)
+        assert lib.sxb_test_skip_ring_slot(slot) == 0
+        K.hc_mix_up_wmma(*args, u[1], ws, act)
+        torch.cuda.synchronize()
+    finally:
+        lib.sxb_test_skip_ring_slot(-1)
+        K.set_wait_limit(2_000_000_000)
+    with pytest.raises(K.Error, match=r"skipped fill: a tcgen05 kernel gave up a wait at work item \d+ \((a weight producer|an MMA warp|the epilogue|the activation copy|the weight-code copy)"):
+        K.check_dense_status("skipped fill")
+    K.hc_mix_up_wmma(*args, u[2], ws, act)
+    K.check_dense_status("after")
+    assert torch.equal(u[2], u[0]) and not bool(torch.isnan(u[2]).any())
