@@ -257,9 +257,10 @@ int sxb_route_layout(int64_t M, int64_t A, int64_t E, int64_t out[8]);
  * forms (SXB_MATH_F32, SXB_MATH_WMMA_BF16) wait inside a CTA too, for another warp's share of the work: their bound is this one or
  * 2 s, whichever is longer. */
 int sxb_set_wait_limit(uint64_t nanoseconds);
-/* Test hook, no counterpart in the reference: slot >= 0 makes CTA 0 of the following launches leave one fill out - of the
- * weight-code ring in the expert kernels and the dense projections, of the h stages in the up mix up to rank 512 - so a
- * bounded wait runs out and the kernel's give-up path runs; -1 (the default) = off. */
+/* Test hook, no counterpart in the reference: slot >= 0 makes CTA 0 of the following launches leave that fill out - of the
+ * weight-code ring in the tcgen05 expert kernels and dense projections, of the h stages in the up mix up to rank 512 - or, in
+ * the exact grouped forms, an arrival of its second (even slot) or third tile (odd), so a bounded wait runs out and the
+ * kernel's give-up path runs; -1 (the default) = off. */
 int sxb_test_skip_ring_slot(int slot);
 
 /* ---- Dense quantized linear --------------------------------------------------------------------------------- */

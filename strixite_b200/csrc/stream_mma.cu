@@ -170,6 +170,7 @@ struct StreamArgs {
     uint32_t *err;
     uint32_t *status;    // kFromWs: {2, tile, role} of a wait that ran out, in the workspace's header
     unsigned long long wait_limit_ns;
+    int test_skip_slot;  // >= 0: CTA 0's second (even) or third (odd) tile waits for one arrival more than its warps make (tests only)
     int chunks, split;   // see chunk_count: chunks of a contraction; warps that share a unit (1 .. chunks)
 };
 
@@ -880,7 +881,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const Stre
     };
     if (threadIdx.x < kTileTokens) describe(bufs[0], tile0, threadIdx.x);
     if (threadIdx.x == 0) {
-        for (int b = 0; b < kTileBufs; ++b) mbar_init(&staged[b], kTileTokens), mbar_init(&left[b], kBigWarps);
+        for (int b = 0; b < kTileBufs; ++b) mbar_init(&staged[b], kTileTokens + (blockIdx.x == 0 && a.test_skip_slot >= 0 && b != (a.test_skip_slot & 1))), mbar_init(&left[b], kBigWarps);
         s_low = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1074,7 +1075,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
         if (kTileBufs * smem <= kMaxDynSmem) {
             auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
             SXB_CUDA(cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
-            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns();
+            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns(), args.test_skip_slot = test_skip_slot();
             launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
             return SXB_OK;
         }

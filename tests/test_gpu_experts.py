@@ -676,3 +676,45 @@ def test_status_words_name_the_kernel_that_gave_up(cuda):
         else:
             with pytest.raises(Kn.Error, match="L0: " + text):
                 Kn.check_grouped_status(ws, "L0")
+
+
+@pytest.mark.parametrize("slot", [0, 1])
+@pytest.mark.parametrize("bits,form", [(4, "gather"), (8, "swiglu"), (8, "combine")])
+def test_exact_grouped_forms_give_up_a_wait(cuda, lib, bits, form, slot):
+    """The exact grouped forms where CTA 0's second tile, or its third (a buffer's second turn), never counts as staged: the wait runs out after 2 s, warp by
+    warp, the status names kernel, tile and role, and the next calls on the context are right."""
+    from strixite_b200 import kernels as Kn
+    M, A, E, N, Kd, G = 4000, 2, 40, 16, 512, 64
+    g = torch.Generator(device="cuda").manual_seed(slot)
+    w = Kn.quantize(torch.randn((E * N, Kd), generator=g, device=cuda) * 0.05, G, bits)
+    x = torch.randn((M * A if form == "combine" else M, Kd), generator=g, device=cuda).to(torch.bfloat16)
+    ids = torch.rand((M, E), generator=g, device=cuda).topk(A, dim=1).indices.to(torch.int32)
+    coef = torch.rand((M, A), generator=g, device=cuda)
+    err = torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = Kn.moe_route_workspace_bytes(M, A, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    partial = torch.empty((M * A, N), device=cuda)
+
+    def run():
+        Kn.moe_group_routes(ids, M, A, E, ws, nbytes, err)
+        if form == "combine":
+            y = torch.full((M, N), float("nan"), device=cuda)
+            Kn.linear_qw_experts_combine_grouped(x, w, E, ids, coef, ws, nbytes, partial, M, A, y, Kn.Act.BF16, Kn.MoeMath.F32, out_act=Kn.Act.F32)
+        else:
+            y = torch.full((M * A, N // 2 if form == "swiglu" else N), float("nan"), dtype=torch.bfloat16, device=cuda)
+            (Kn.linear_qw_experts_gather_grouped_swiglu if form == "swiglu" else Kn.linear_qw_experts_gather_grouped)(x, w, E, ws, nbytes, M, A, y, Kn.Act.BF16, Kn.MoeMath.F32)
+        torch.cuda.synchronize()
+        return y
+
+    want = run()
+    Kn.check_grouped_status(ws, "warm-up")
+    try:
+        assert lib.sxb_test_skip_ring_slot(slot) == 0
+        run()
+    finally:
+        lib.sxb_test_skip_ring_slot(-1)
+    with pytest.raises(Kn.Error, match=rf"skipped: the streaming expert kernel gave up a wait at tile {slot + 1} \(a (warp waiting for the tile's staged|staging warp waiting)"):
+        Kn.check_grouped_status(ws, "skipped")
+    got = run()
+    Kn.check_grouped_status(ws, "after")
+    assert torch.equal(got, want) and not bool(torch.isnan(got).any())
