@@ -1054,31 +1054,35 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     SXB_CHECK(smem <= kMaxDynSmem, fn, ": K = ", a.K, SRC == kPerToken ? " x A = " : "", SRC == kPerToken ? a.A : 0, " needs ", smem,
               " bytes of shared memory for one tile's activations, more than ", kMaxDynSmem,
               " (K * 16 * ceil(A / 8) bytes for the per-slot combine, K * 16 otherwise; use the grouped form)");
-    auto kern = stream_kernel<BITS, G, MODE, SRC, TOUT>;
+    StreamArgs args = a;
     // the function's limit is one for all threads of the process: always the largest, not this call's, which would take it from another thread's
-    SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn,
-             ": reserving shared memory");
+    auto reserve = [&](auto k) -> int {
+        SXB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
+        return SXB_OK;
+    };
+    // Routed tiles of a grouping workspace; rows too long for two buffers go on below.
+    if constexpr (SRC == kFromWs) {
+        if (kTileBufs * smem <= kMaxDynSmem) {
+            auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
+            if (int rc = reserve(tiles)) return rc;
+            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns(), args.test_skip_slot = test_skip_slot();
+            args.chunks = args.split = 1;
+            launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
+            return SXB_OK;
+        }
+    }
+    auto kern = stream_kernel<BITS, G, MODE, SRC, TOUT>;
+    if (int rc = reserve(kern)) return rc;
     // A dense projection of few units for the machine's warps: up to eight warps share one, as long as that gives a warp at most two and a half
     // parts in turn.  A warp alone walks K / (4 * kStepCodes) blocks one after another, each a round trip to memory (2048 x 4096
     // Q4, one token: 16.4 us with 128 warps at work, 9.1 with eight warps a unit).
     const int64_t machine_warps = (int64_t)sm_count() * (kBigThreads / 32);
-    StreamArgs args = a;
     args.chunks = SRC == kDense && geo::kStepsPerGroup == 1 && vector_scales(a, G) ? chunk_count(steps / kPrefetch) : 1, args.split = 1;
     if (SRC == kDense)
         while (args.split * 2 <= args.chunks && est_units * args.split * 4 <= machine_warps * 5) args.split *= 2;
     if (args.split > 1) {
         launch_behind(kern, (unsigned)std::min<int64_t>(sm_count(), est_units), kBigThreads, smem, st, 1, args);
         return SXB_OK;
-    }
-    // Routed tiles of a grouping workspace; rows too long for two buffers go on below.
-    if constexpr (SRC == kFromWs) {
-        if (kTileBufs * smem <= kMaxDynSmem) {
-            auto tiles = stream_tiles_kernel<BITS, G, MODE, TOUT>;
-            SXB_CUDA(cudaFuncSetAttribute(tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem), fn, ": reserving shared memory");
-            args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns(), args.test_skip_slot = test_skip_slot();
-            launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
-            return SXB_OK;
-        }
     }
     // One CTA of sixteen warps an SM when there are several units for every warp of the machine; otherwise CTAs of eight
     // warps, two an SM where their shared memory allows, and never more CTAs than one per unit and warp.
