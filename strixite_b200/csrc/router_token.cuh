@@ -34,7 +34,11 @@ __device__ inline V sorted_down(V v, int lane) {
     return v;
 }
 
-constexpr int kPickSort = 16;  // top-k up to which the candidates are few enough to be sorted (picked_by_sort)
+// The k of the picks by sort (picked_by_sort).  Above 16 the candidates are too many to be sorted; below the other line a few rounds cost less than the
+// two sorts: us of rounds and of the sort, 16384 tokens, E = 128 k = 4 8.7 and 9.2, k = 6 11.0 and 9.2; E = 256 k = 3 9.9 and 11.5, k = 4 13.1 and 11.6;
+// E = 512 k = 1 15.7 and 18.0, k = 3 21.3 and 18.0; E = 1000 k = 1 37 and 40, k = 3 46 and 40.
+constexpr int kPickSort = 16;
+template <int NV> constexpr int kPickSortMin = NV <= 4 ? 6 : NV <= 8 ? 4 : 3;
 
 // The top k of the warp's keys (0 = no key), pick r in lane r as {key, ~index}, k <= kPickSort.  The k-th largest of the lanes' own largest keys
 // bounds the k-th pick from below: k different keys reach it.  What reaches it - a dozen of 512 for a top-10 - is gathered in shared memory (cand,
@@ -94,7 +98,7 @@ __device__ inline void route_token(const T *__restrict__ row, int lane, int64_t 
     float my_v = 0.f, top = 0.f;
     int my_i = -1;
     unsigned long long pick;
-    if (k <= kPickSort && picked_by_sort<NV>(key, lane, k, cand, pick)) {
+    if (k >= kPickSortMin<NV> && k <= kPickSort && picked_by_sort<NV>(key, lane, k, cand, pick)) {
         my_v = key_value((uint32_t)(pick >> 32)), my_i = (int)~(uint32_t)pick;
         top = __shfl_sync(0xffffffffu, my_v, 0);
     } else {

@@ -76,6 +76,20 @@ def test_router_ties_at_the_bound(cuda, oracle, E, k, tied):
     np.testing.assert_allclose(coef, ref_coef, rtol=2e-6, atol=1e-30)
 
 
+@pytest.mark.parametrize("E", [7, 128, 129, 256, 257, 512, 513, 1024])
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 6, 7])
+def test_router_few_picks(cuda, oracle, E, k):
+    """Few picks are made round by round, more by sorted candidates; the line moves with the number of experts: both sides of it, ties on every token."""
+    from strixite_b200 import kernels as K
+    rng = np.random.default_rng(E * 8 + k)
+    logits = np.round(rng.standard_normal((40, E + 1)) * 4).astype(np.float32) / 4
+    logits[0], logits[1, : E // 2] = 0.0, -0.0
+    ids, coef, err = run_router(K, logits, E, k, False, cuda)
+    ref_ids, ref_coef = oracle.moe_router(logits, E, k)
+    assert err[0] == 0 and np.array_equal(ids, ref_ids)
+    np.testing.assert_allclose(coef, ref_coef, rtol=2e-6, atol=1e-30)
+
+
 def test_router_mutation_is_caught(cuda, oracle):
     """A deliberately wrong expectation must fail: guards against a comparison that passes vacuously."""
     from strixite_b200 import kernels as K
