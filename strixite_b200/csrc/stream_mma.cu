@@ -36,6 +36,7 @@
 #include "experts.cuh"
 #include "skinny_mma.cuh"
 #include "tc_ptx.cuh"
+#include "unit_runs.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -827,7 +828,8 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
 
 // The routed forms: one CTA of sixteen warps an SM, the tiles' activations in two buffers of shared memory.  The next tile's are staged under the
 // streaming, a token by a warp - at once where the buffer is free, else after its next unit - and a warp that finds no unit left goes on to the
-// next tile by itself: no barrier of the CTA stands between two tiles.  So a CTA may begin and end inside a tile, and the units are dealt evenly.
+// next tile by itself: no barrier of the CTA stands between two tiles.  So a CTA may begin and end inside a tile, and the units are dealt evenly, unless
+// whole tiles a group of CTAs suit the launch better (unit_runs.cuh).
 // Results as stream_kernel's, bit for bit: a unit's sums do not depend on who forms them.
 // What bounds it: HBM while it streams, 22 bytes a cycle and SM, 6.2 TB/s, whatever the tile; launch and first staging (8000 cycles), the last
 // units.  With one buffer and a barrier on either side of the staging, tile-aligned runs and, in small launches, CTAs of eight warps two an SM, it
@@ -862,11 +864,9 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_tiles_kernel(const Stre
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2;
     const int I = (int)(a.N / 2), units_per_tile = MODE == kSwiglu ? (I + 7) / 8 : (int)((a.N + 15) / 16);
     TOUT *out = static_cast<TOUT *>(a.out);
-    // the CTA's run of units: from unit u0 of tile0 to before unit u1 of tile1
-    const int64_t total = (int64_t)a.ws[0] * units_per_tile, begin = total * blockIdx.x / gridDim.x, end = total * (blockIdx.x + 1) / gridDim.x;
-    if (begin >= end) return;
-    const int tile0 = (int)(begin / units_per_tile), tile1 = (int)((end - 1) / units_per_tile);
-    const int u0 = (int)(begin - (int64_t)tile0 * units_per_tile), u1 = (int)(end - (int64_t)tile1 * units_per_tile);
+    const UnitRun run = unit_run((uint32_t)a.ws[0], (uint32_t)units_per_tile, blockIdx.x, gridDim.x, kBigWarps);
+    const int tile0 = run.tile0, tile1 = run.tile1, u0 = run.u0, u1 = run.u1;
+    if (tile0 > tile1) return;
 
     auto xs_of = [&](int b) { return reinterpret_cast<uint4 *>(smem + b * pass_bytes); };
     auto xsum_of = [&](int b) { return reinterpret_cast<float *>(smem + b * pass_bytes + xs_bytes); };

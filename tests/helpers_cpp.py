@@ -28,3 +28,10 @@ def build_scratch_fake(out_dir: pathlib.Path) -> pathlib.Path:
     subprocess.run(["g++", "-std=c++17", "-x", "c++", "-w", f"-I{ROOT / 'include'}", f"-I{ROOT / 'strixite_b200' / 'csrc'}",
                     f"-I{cuda_home() / 'include'}", str(ROOT / "tests" / "cpp" / "scratch_fake.cpp"), "-pthread", "-o", str(exe)], check=True)
     return exe
+
+
+def build_unit_runs(out_dir: pathlib.Path) -> pathlib.Path:
+    exe = pathlib.Path(out_dir) / "unit_runs"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", f"-I{ROOT / 'strixite_b200' / 'csrc'}", str(ROOT / "tests" / "cpp" / "unit_runs.cpp"), "-o", str(exe)],
+                   check=True)
+    return exe

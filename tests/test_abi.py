@@ -58,6 +58,13 @@ def test_scratch_pool_against_a_fake_runtime(tmp_path):
     assert res.returncode == 0 and "FAIL" not in res.stdout, res.stdout + res.stderr
 
 
+def test_unit_runs_hold_every_unit_once(tmp_path):
+    """csrc/unit_runs.cuh, the deal of the streaming kernel's units to CTAs, compiled for the host (tests/cpp/unit_runs.cpp)."""
+    from helpers_cpp import build_unit_runs
+    res = subprocess.run([str(build_unit_runs(tmp_path))], capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and "FAIL" not in res.stdout, res.stdout[:2000]
+
+
 def test_preconditions_fail_before_any_launch(lib):
     from strixite_b200 import kernels as K
     with pytest.raises(K.Error, match="null pointer"):

@@ -633,6 +633,32 @@ def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
     assert not bad and lib.sxb_release_scratch() == 0
 
 
+@pytest.mark.parametrize("tiles,N", [(1, 16), (3, 1040), (5, 2064), (49, 512), (74, 1024), (75, 512), (140, 1536), (148, 32), (149, 64)])
+def test_exact_grouped_runs_of_units(cuda, tiles, N):
+    """Tiles of units dealt inside tiles and evenly: one unit a warp or fewer, several rounds, CTAs left over, both sides of as many tiles as CTAs; bit for
+    bit the per-slot forms, with FP32 dots through the combine of one slot a token."""
+    from strixite_b200 import kernels as Kn
+    Kd, G, M = 256, 64, tiles * 8 - 3
+    g = torch.Generator(device="cuda").manual_seed(tiles)
+    w = Kn.quantize(torch.randn((2 * N, Kd), generator=g, device=cuda) * 0.05, G, 8)
+    x = torch.randn((M, Kd), generator=g, device=cuda).to(torch.bfloat16)
+    ids = (torch.arange(M, device=cuda)[:, None] >= (tiles + 1) // 2 * 8).to(torch.int32) if tiles > 1 else torch.zeros((M, 1), dtype=torch.int32, device=cuda)
+    coef, err = torch.ones((M, 1), device=cuda), torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = Kn.moe_route_workspace_bytes(M, 1, 2)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    Kn.moe_group_routes(ids, M, 1, 2, ws, nbytes, err)
+    assert int(ws[0]) == tiles
+    y = [torch.full((M, N), float("nan"), device=cuda) for _ in range(2)]
+    Kn.linear_qw_experts_combine(x[:, None], w, 2, ids, coef, M, 1, y[0], Kn.Act.BF16, err, out_act=Kn.Act.F32)
+    Kn.linear_qw_experts_combine_grouped(x, w, 2, ids, coef, ws, nbytes, torch.empty((M, N), device=cuda), M, 1, y[1], Kn.Act.BF16, Kn.MoeMath.F32, out_act=Kn.Act.F32)
+    h = [torch.full((M, N // 2), float("nan"), dtype=torch.bfloat16, device=cuda) for _ in range(2)]
+    Kn.linear_qw_experts_gather_swiglu(x, w, 2, ids, M, 1, h[0], Kn.Act.BF16, err)
+    Kn.linear_qw_experts_gather_grouped_swiglu(x, w, 2, ws, nbytes, M, 1, h[1], Kn.Act.BF16, Kn.MoeMath.F32)
+    torch.cuda.synchronize()
+    Kn.check_grouped_status(ws, "runs")
+    assert torch.equal(h[0], h[1]) and torch.equal(y[0], y[1]) and not bool(torch.isnan(y[1]).any() | torch.isnan(h[1]).any())
+
+
 @pytest.mark.parametrize("swiglu", [False, True])
 def test_a_short_wait_limit_leaves_the_exact_forms_whole(cuda, oracle, swiglu):
     """sxb_set_wait_limit is for the tcgen05 kernels: in the exact grouped forms a warp waits for another's unit or row as a matter of course, longer
