@@ -345,10 +345,12 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 continue;
             }
             const bool natural = __any_sync(0xffffffffu, scale < 0.f);  // the quadrant's rows share it
-            // the set's first step of the next item, if it has one there
+            // The set's first step of the next item, if it has one there: its scales are asked for at this item's start, but for four groups (registers)
+            // and for gate/up of Q8, which HBM bounds: 512 experts x 4096 x 2048, 256 tokens 929 us so and 889 at the end, 500 940 and 899.
+            constexpr bool kEarly = kGroups < 4 && !(BITS == 8 && MODE == kTcSwiglu);
             const int after = st + (max(n_steps - st, 0) + kWays - 1) / kWays * kWays - n_steps;
             Scales<kGroups> sc_item{};
-            if (kGroups < 4) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
+            if (kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
             const uint16_t *sp = a.scale + (int64_t)max(row, 0) * groups + (st + kWays) * kGroups, *mp = a.minv + (sp - a.scale);
             for (; st < n_steps; st += kWays, slot.advance(kWays), sp += kWays * kGroups, mp += kWays * kGroups) {
                 const Scales<kGroups> sc = sc_nxt;
@@ -401,7 +403,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 mbar_arrive_if(signals, &full_bar[set]);
                 free_phase ^= 1u;
             }
-            if (kGroups == 4) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);  // four groups are too many registers to hold over an item
+            if (!kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
             st -= n_steps, row = nxt_row, sc_nxt = sc_item;
         }
     } else if (warp == kItemWarp) {
