@@ -206,9 +206,9 @@ int sxb_hc_inject_inv(void *x, const float *w_in, const void *y, int64_t T, int6
                       sxb_stream_t stream);
 /* kernels/hc_wmma.hpp:45-49  hc_mix_up_wmma (Q4ChunkMajorView / Q8ChunkMajorView overloads): hc_mix_up on the tensor cores -
  * h rounded once to F16, weights f16(code * scale + min), FP32 accumulation; sigmoid and the stream combine in FP32.
- * Same arguments as sxb_hc_mix_up_q*, plus a workspace (the reference's launcher needs none; this one un-chunks W_up to
- * row-major and keeps the FP32 logits z of one block of 1024 tokens there): sxb_hc_mix_up_wmma_workspace_bytes, device,
- * 256-byte aligned.  h, x, norm_w, inv, u 16-byte aligned; d % 128 == 0.  A device-side wait that ran out is reported by
+ * Same arguments as sxb_hc_mix_up_q*, plus a workspace (the reference's launcher needs none; this one keeps h as
+ * tile-blocked F16 there and, for ranks above 512, W_up un-chunked to row-major; the size asked for holds both at any
+ * rank): sxb_hc_mix_up_wmma_workspace_bytes, device, 256-byte aligned.  h, x, norm_w, inv, u 16-byte aligned; d % 128 == 0.  A device-side wait that ran out is reported by
  * sxb_check_dense_status. */
 size_t sxb_hc_mix_up_wmma_workspace_bytes(int64_t T, int64_t H, int64_t d, int64_t r, int bits, int64_t G);
 int sxb_hc_mix_up_wmma_q4(const float *h, const SxbQView *w_up, const void *x, const float *norm_w, const float *inv, int64_t T, int64_t H,

@@ -23,8 +23,9 @@
 //     phase ahead, a deeper item ring or a second quarter dequantized before the stage is free: no faster (+0 to +1 %).
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
-// A wider token tile would not be cheaper: it shares a dequantization that is no longer the bound, and 128 columns leave tensor
-// memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column stages of A.
+// Why 128 tokens: that leaves tensor memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column
+// stages of A.  An expert of more tokens has its rows dequantized again for every 128 of them; a wider tile, which would share that at the price of an
+// accumulator or of stages, has not been built.
 // Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 506 us at 777 tokens (15 an expert), 685 at
 // 4096 (80 an expert); down 291 and 480 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
 //

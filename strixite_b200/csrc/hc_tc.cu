@@ -20,7 +20,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <type_traits>
 
 namespace sxb {
 namespace {
@@ -634,6 +633,8 @@ int mix_down_tc(const void *x, const SxbQView *w, int64_t T, int64_t H, int64_t 
     return SXB_OK;
 }
 
+// Parts of the up mix's workspace.  The un-chunked weight is the general kernel's: up to rank 512 its place stays unused (the size is part of the
+// interface, which a host may have stored).
 struct UpWs {
     size_t wq, wscale, wmin, hs, total;
 };

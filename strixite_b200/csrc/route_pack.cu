@@ -7,8 +7,8 @@
 // be compared word for word with a CPU counting sort.  Ranks inside a bucket come from `match.any` warp votes, never
 // from the arrival order of atomics.
 //   S <= kSmallSlots: one CTA does everything, eight of its warps a run of slots each.
-//   larger S: three launches - per-warp-segment histograms, one CTA that scans them into bucket offsets and per-segment
-//   bases, and a scatter in which every warp places its own segment in order and the CTAs share the tile lists.
+//   larger S: three launches - histograms of segments, a CTA each, one CTA that scans them into bucket offsets and per-segment
+//   bases, and a scatter in which a CTA places its segment in order, a run of it a warp, and the CTAs share the tile lists.
 
 #include "route_pack.cuh"
 

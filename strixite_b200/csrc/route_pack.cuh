@@ -7,7 +7,7 @@ namespace sxb {
 
 constexpr int64_t kMoeMaxExperts = 1023;   // E + 1 buckets fit one 1024-thread CTA (kernels/moe_grouped.hpp:43)
 constexpr int64_t kMoeMaxSlots = 1 << 20;  // kernels/moe_grouped.hpp:44
-constexpr int kSegSlots = 1024;            // slots one warp places in the multi-CTA pack
+constexpr int kSegSlots = 1024;            // slots one CTA places in the multi-CTA pack
 
 // Word (int32) offsets into the workspace.
 //   header [8]: n_tiles8, S, E, n_tiles128, ep_mode, 0, 0, 0

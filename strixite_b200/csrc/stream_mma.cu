@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
 // What bounds it: HBM while it streams, 22 bytes a cycle and SM, 6.2 TB/s, whatever the tile; launch and first staging (8000 cycles), the last
 // units.  With one buffer and a barrier on either side of the staging, tile-aligned runs and, in small launches, CTAs of eight warps two an SM, it
 // streamed 76 to 87 % of the time.  4096 x 2048 + 1024 x 4096, 512 experts, top-10, gate/up and down us, before -> now: 16 tokens Q4 130 + 70 -> 121 + 63,
-// 37 tokens (Q8 down) 207 + 167 -> 184 + 158, 150 tokens 424 + 234 -> 384 + 211; the layer as a graph, 2 tokens 83.5 -> 67.5, 4 109 -> 90, 64 552 -> 495.
+// 37 tokens (Q8 down) 207 + 167 -> 184 + 158, 150 tokens 424 + 234 -> 384 + 211; the layer as a graph, 2 tokens 82 -> 65, 4 107 -> 87, 64 599 -> 523.
 // The staging's loads are four at a time and inline: with eight or sixteen in flight, or as a call, the loop over a unit's codes lost registers to
 // them (16 tokens 126 + 65; as a call 200 + 89).
 // Every wait is bounded; one that runs out is recorded in the grouping workspace's status words and ends the warp.

@@ -192,9 +192,6 @@ __device__ inline void tc_commit_if(uint32_t leader, uint64_t *bar) {
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
         : "memory");
 }
-__device__ inline void tc_commit_one(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // One k-block of an accumulator as one instruction group: a non-blocking probe of the NEXT k-block's "operands ready"
 // barrier first, then the four MMAs (k = 16 each; the A columns advance by 8, the B descriptor by 32 bytes), the commit
