@@ -258,9 +258,9 @@ int sxb_route_layout(int64_t M, int64_t A, int64_t E, int64_t out[8]);
  * 2 s, whichever is longer. */
 int sxb_set_wait_limit(uint64_t nanoseconds);
 /* Test hook, no counterpart in the reference: slot >= 0 makes CTA 0 of the following launches leave that fill out - of the
- * weight-code ring in the tcgen05 expert kernels and dense projections, of the h stages in the up mix up to rank 512 - or, in
- * the exact grouped forms, an arrival of its second (even slot) or third tile (odd), so a bounded wait runs out and the
- * kernel's give-up path runs; -1 (the default) = off. */
+ * weight-code ring in the tcgen05 expert kernels and dense projections, of the h stages in the up mix up to rank 512, of the
+ * stages in the router-logits GEMM - or, in the exact grouped forms, an arrival of its second (even slot) or third tile
+ * (odd), so a bounded wait runs out and the kernel's give-up path runs; -1 (the default) = off. */
 int sxb_test_skip_ring_slot(int slot);
 
 /* ---- Dense quantized linear --------------------------------------------------------------------------------- */

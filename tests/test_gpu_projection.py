@@ -598,6 +598,32 @@ def test_a_wait_that_runs_out_ends_the_kernel_with_a_status(cuda, oracle, lib, t
     assert max_abs_over_rms(y2.cpu().numpy(), want) <= 2e-5
 
 
+@pytest.mark.parametrize("M,N,K,planes,slot", [(150, 513, 512, 3, 0), (150, 513, 512, 3, 6), (40000, 300, 64, 1, 1), (1200, 513, 2048, 2, 9)])
+def test_router_gemm_gives_up_a_wait(cuda, lib, M, N, K, planes, slot):
+    """The router-logits GEMM with CTA 0 told to leave one stage fill out: in its first item, behind a full turn of the stages and in its second item.
+    The kernel returns, the status names the role, the next call has the bits of the call before."""
+    from strixite_b200 import kernels as Kn
+    g = torch.Generator(device="cpu").manual_seed(M)
+    x, w = torch.randn((M, K), generator=g).to(torch.bfloat16).to(cuda), (torch.randn((N, K), generator=g) * 0.02).to(cuda)
+    planes_ = Kn.router_prepare(w.to(torch.bfloat16) if planes == 1 else w, planes)
+    out = [torch.full((M, N), float("nan"), device=cuda) for _ in range(3)]
+    Kn.router_logits_wmma(x, planes_, None, out[0])
+    Kn.check_dense_status("warm-up")
+    try:
+        Kn.set_wait_limit(2_000_000)
+        assert lib.sxb_test_skip_ring_slot(slot) == 0
+        Kn.router_logits_wmma(x, planes_, None, out[1])
+        torch.cuda.synchronize()
+    finally:
+        lib.sxb_test_skip_ring_slot(-1)
+        Kn.set_wait_limit(2_000_000_000)
+    with pytest.raises(Kn.Error, match=r"skipped fill: a tcgen05 kernel gave up a wait at work item \d+ \((an MMA warp|the epilogue|the activation copy)"):
+        Kn.check_dense_status("skipped fill")
+    Kn.router_logits_wmma(x, planes_, None, out[2])
+    Kn.check_dense_status("after")
+    assert torch.equal(out[2], out[0]) and not bool(torch.isnan(out[2]).any())
+
+
 def test_dense_tcgen05_captured(cuda, oracle, lib, monkeypatch):
     """The dense forms, spread scales and a wait that runs out, on the kernel that captured calls take (no scratch)."""
     graphs = capture_calls(monkeypatch)
