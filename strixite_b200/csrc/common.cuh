@@ -76,6 +76,11 @@ inline cudaError_t launch_behind(void (*kern)(Params...), dim3 grid, dim3 block,
 // First statement of a kernel that is launched by launch_behind (by any launch: with nothing ahead it passes): the grid ahead has ended and its
 // results, and with it those of every grid ahead of it, are visible; and the next one may come in behind this one's CTAs, all of which run.
 __device__ inline void behind_grid() { asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory"); }
+// The same; let_in = false: the next one comes in when this one's CTAs leave.
+__device__ inline void behind_grid(bool let_in) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (let_in) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ---- device helpers ---------------------------------------------------------------------------------------------
 __host__ __device__ inline float bf16_bits_to_f32(uint16_t b) {

@@ -111,15 +111,16 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
         SXB_CHECK(tc || a->sh_gu != nullptr, fn, ": null shared-expert buffer sh_gu");
         SXB_CHECK(!tc || a->sh_xs != nullptr, fn, ": null shared-expert buffer sh_xs for the tcgen05 path");
     }
-    if (shared && !tc && side != stream) SXB_CUDA(beside.fork(), fn, ": starting the shared expert's stream");
+    const bool two = shared && !tc && side != stream;  // then the experts' first kernel must not take its places ahead of the shared expert's
+    if (two) SXB_CUDA(beside.fork(), fn, ": starting the shared expert's stream");
 
     // router (kernels/moe_router.hpp:38-40): top-k of the first E_total logits; a shared expert's gate is column E_total.
     // logits == NULL: ids and coef already hold the routes (an expert-parallel rank receives them from the tokens' owners)
     // A small batch (decode) routes and packs in one launch.
     bool packed = false;
     if (a->logits != nullptr && !ep && M * A <= 2048) {
-        if (int rc = sxb_moe_route_small(a->logits, a->logits_ld, M, a->E_total, A, 0, E, a->ids, a->coef, a->ws, a->ws_bytes,
-                                         a->router_err, a->expert_err, stream))
+        if (int rc = route_small("moe_route_small", a->logits, a->logits_ld, M, a->E_total, A, 0, E, a->ids, a->coef, a->ws, a->ws_bytes,
+                                 a->router_err, a->expert_err, !two, stream))
             return rc;
         packed = true;
     } else if (a->logits != nullptr) {
@@ -154,7 +155,7 @@ int moe_layer_impl(const SxbMoeLayerArgs *a, sxb_stream_t stream, const PeerOut 
     } else if (ep) {
         if (int rc = sxb_moe_group_routes_ep(a->ids, M, A, a->E_total, a->e_lo, E, a->ws, a->ws_bytes, a->expert_err, stream)) return rc;
     } else {
-        if (int rc = sxb_moe_group_routes(a->ids, M, A, E, a->ws, a->ws_bytes, a->expert_err, stream)) return rc;
+        if (int rc = group_routes("moe_group_routes", a->ids, M, A, E, 0, E, false, a->ws, a->ws_bytes, a->expert_err, !two, stream)) return rc;
     }
     // gate/up + SwiGLU (kernels/moe_grouped.hpp:67-69)
     const int hf = tc ? (a->down_bits == 4 ? 3 : 4) : 0;

@@ -183,8 +183,8 @@ __device__ void pack_small_body(const int32_t *__restrict__ ids, const RouteWord
 
 __global__ void __launch_bounds__(kPackThreads)
     pack_small_kernel(const int32_t *__restrict__ ids, RouteWords L, int E_total, int e_lo, bool ep, int32_t *ws,
-                      uint32_t *err) {
-    behind_grid();
+                      uint32_t *err, bool let_in) {
+    behind_grid(let_in);
     pack_small_body(ids, L, E_total, e_lo, ep, ws, err);
 }
 
@@ -194,8 +194,8 @@ template <int NV>
 __global__ void __launch_bounds__(kPackThreads)
     route_small_kernel(const float *__restrict__ logits, int64_t ld, int M, int E_total, int k, int32_t *__restrict__ ids,
                        float *__restrict__ coef, RouteWords L, int e_lo, bool ep, int32_t *ws, uint32_t *router_err,
-                       uint32_t *expert_err) {
-    behind_grid();
+                       uint32_t *expert_err, bool let_in) {
+    behind_grid(let_in);
     __shared__ unsigned long long cand[kPackThreads / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int m = warp; m < M; m += kPackThreads / 32)
@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(kPackThreads)
 // take 128 slots each, as in the small pack: no warp waits for another (a warp a segment, 32 rounds one after another, was most of the
 // launch: 15.5 us at 777 to 16384 tokens x 10 slots).
 __global__ void __launch_bounds__(32 * kSegWarps)
-    pack_scatter_kernel(const int32_t *__restrict__ ids, RouteWords L, int e_lo, int32_t *ws) {
-    behind_grid();
+    pack_scatter_kernel(const int32_t *__restrict__ ids, RouteWords L, int e_lo, int32_t *ws, bool let_in) {
+    behind_grid(let_in);
     __shared__ __align__(4) uint16_t counts[kSegWarps][kMoeMaxExperts + 1];
     __shared__ Layout sm;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, E = (int)L.E, S = (int)L.S, s0 = (int)blockIdx.x * kSegSlots + warp * kSegRounds * 32;
@@ -314,31 +314,6 @@ __global__ void __launch_bounds__(32 * kSegWarps)
     emit_tiles(L, ws, sm, blockIdx.x * 32 * kSegWarps + t, gridDim.x * 32 * kSegWarps);
 }
 
-int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo,
-                 int64_t E_local, bool ep, void *ws, size_t ws_bytes, uint32_t *err, sxb_stream_t stream) {
-    SXB_CHECK(ids != nullptr && ws != nullptr && err != nullptr, fn, ": null pointer (ids=", (const void *)ids, ", ws=", ws,
-              ", err=", (const void *)err, ")");
-    SXB_CHECK(M >= 1 && A >= 1 && A <= 64 && E_local >= 1 && E_local <= kMoeMaxExperts && M * A <= kMoeMaxSlots, fn,
-              ": M = ", M, ", A = ", A, ", E = ", E_local, " (A 1..64, E 1..", kMoeMaxExperts, ", M*A <= ", kMoeMaxSlots, ")");
-    SXB_CHECK(e_lo >= 0 && e_lo + E_local <= E_total, fn, ": experts [", e_lo, ", ", e_lo + E_local, ") outside [0, ",
-              E_total, ")");
-    const RouteWords L = route_words(M, A, E_local);
-    SXB_CHECK(ws_bytes >= (size_t)L.total * 4, fn, ": workspace of ", ws_bytes, " bytes, needs ", L.total * 4);
-    SXB_CHECK(reinterpret_cast<uintptr_t>(ws) % 4 == 0, fn, ": workspace ", ws, " must be 4-byte aligned");
-    auto st = static_cast<cudaStream_t>(stream);
-    auto *w = static_cast<int32_t *>(ws);
-    if (L.S <= kSmallSlots) {
-        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, err);
-    } else {
-        const unsigned ctas = (unsigned)L.nseg;
-        launch_behind(pack_hist_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)E_total, (int)e_lo, w);
-        launch_behind(pack_scan_kernel, 1, kPackThreads, 0, st, 1, ids, L, ep, w, err);
-        launch_behind(pack_scatter_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)e_lo, w);
-    }
-    SXB_CHECK_LAUNCH(fn, " M=", M, " A=", A, " E=", E_local);
-    return SXB_OK;
-}
-
 }  // namespace
 
 RouteWords route_words(int64_t M, int64_t A, int64_t E) {
@@ -357,6 +332,65 @@ RouteWords route_words(int64_t M, int64_t A, int64_t E) {
     L.first = L.scratch + L.nseg * (E + 1);
     L.total = L.first + (L.nseg ? kTileLists * (E + 2) : 0);
     return L;
+}
+
+int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo,
+                 int64_t E_local, bool ep, void *ws, size_t ws_bytes, uint32_t *err, bool let_in, sxb_stream_t stream) {
+    SXB_CHECK(ids != nullptr && ws != nullptr && err != nullptr, fn, ": null pointer (ids=", (const void *)ids, ", ws=", ws,
+              ", err=", (const void *)err, ")");
+    SXB_CHECK(M >= 1 && A >= 1 && A <= 64 && E_local >= 1 && E_local <= kMoeMaxExperts && M * A <= kMoeMaxSlots, fn,
+              ": M = ", M, ", A = ", A, ", E = ", E_local, " (A 1..64, E 1..", kMoeMaxExperts, ", M*A <= ", kMoeMaxSlots, ")");
+    SXB_CHECK(e_lo >= 0 && e_lo + E_local <= E_total, fn, ": experts [", e_lo, ", ", e_lo + E_local, ") outside [0, ",
+              E_total, ")");
+    const RouteWords L = route_words(M, A, E_local);
+    SXB_CHECK(ws_bytes >= (size_t)L.total * 4, fn, ": workspace of ", ws_bytes, " bytes, needs ", L.total * 4);
+    SXB_CHECK(reinterpret_cast<uintptr_t>(ws) % 4 == 0, fn, ": workspace ", ws, " must be 4-byte aligned");
+    auto st = static_cast<cudaStream_t>(stream);
+    auto *w = static_cast<int32_t *>(ws);
+    if (L.S <= kSmallSlots) {
+        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, err, let_in);
+    } else {
+        const unsigned ctas = (unsigned)L.nseg;
+        launch_behind(pack_hist_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)E_total, (int)e_lo, w);
+        launch_behind(pack_scan_kernel, 1, kPackThreads, 0, st, 1, ids, L, ep, w, err);
+        launch_behind(pack_scatter_kernel, ctas, 32 * kSegWarps, 0, st, 1, ids, L, (int)e_lo, w, let_in);
+    }
+    SXB_CHECK_LAUNCH(fn, " M=", M, " A=", A, " E=", E_local);
+    return SXB_OK;
+}
+
+int route_small(const char *fn, const float *logits, int64_t ld, int64_t M, int64_t E_total, int64_t k, int64_t e_lo, int64_t E_local, int32_t *ids, float *coef,
+                void *ws, size_t ws_bytes, uint32_t *router_err, uint32_t *expert_err, bool let_in, sxb_stream_t stream) {
+    SXB_CHECK(logits != nullptr && ids != nullptr && coef != nullptr && ws != nullptr && router_err != nullptr && expert_err != nullptr,
+              fn, ": null pointer");
+    SXB_CHECK(E_total >= 1 && E_total <= 1024 && k >= 1 && k <= E_total && k <= 32 && ld >= E_total, fn, ": E = ", E_total, ", k = ", k,
+              ", ld = ", ld, " (E 1..1024, k 1..min(E, 32), ld >= E)");
+    SXB_CHECK(M >= 1 && M * k <= kSmallSlots, fn, ": M * k = ", M * k, " slots, this one-CTA form takes at most ", kSmallSlots,
+              " (use moe_router + moe_group_routes)");
+    SXB_CHECK(E_local >= 1 && E_local <= kMoeMaxExperts && e_lo >= 0 && e_lo + E_local <= E_total, fn, ": experts [", e_lo, ", ",
+              e_lo + E_local, ") outside [0, ", E_total, ")");
+    const bool ep = E_local != E_total;
+    const RouteWords L = route_words(M, k, E_local);
+    SXB_CHECK(ws_bytes >= (size_t)L.total * 4, fn, ": workspace of ", ws_bytes, " bytes, needs ", L.total * 4);
+    auto st = static_cast<cudaStream_t>(stream);
+    auto *w = static_cast<int32_t *>(ws);
+    // One CTA routes 32 tokens at a time, so from there on the router has a launch of its own, with a warp a token over the
+    // machine (150 tokens x 512 experts, top-10: 87 us as one launch).
+    if (M > kPackThreads / 32) {
+        if (int rc = sxb_moe_router(logits, ld, M, E_total, k, nullptr, 1, 0, ids, coef, SXB_ACT_F32, router_err, stream)) return rc;
+        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, expert_err, let_in);
+        SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
+        return SXB_OK;
+    }
+#define SXB_ROUTE_SMALL(NV) \
+    launch_behind(route_small_kernel<NV>, 1, kPackThreads, 0, st, 1, logits, ld, (int)M, (int)E_total, (int)k, ids, coef, L, (int)e_lo, ep, w, router_err, expert_err, let_in)
+    if (E_total <= 128) SXB_ROUTE_SMALL(4);
+    else if (E_total <= 256) SXB_ROUTE_SMALL(8);
+    else if (E_total <= 512) SXB_ROUTE_SMALL(16);
+    else SXB_ROUTE_SMALL(32);
+#undef SXB_ROUTE_SMALL
+    SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
+    return SXB_OK;
 }
 
 }  // namespace sxb
@@ -418,48 +452,18 @@ int sxb_check_grouped_status(const void *ws, const char *what) {
 
 int sxb_moe_group_routes(const int32_t *ids, int64_t M, int64_t A, int64_t E, void *ws, size_t ws_bytes, uint32_t *err,
                          sxb_stream_t stream) {
-    return group_routes("moe_group_routes", ids, M, A, E, 0, E, false, ws, ws_bytes, err, stream);
+    return group_routes("moe_group_routes", ids, M, A, E, 0, E, false, ws, ws_bytes, err, true, stream);
 }
 
 int sxb_moe_group_routes_ep(const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo, int64_t E_local,
                             void *ws, size_t ws_bytes, uint32_t *err, sxb_stream_t stream) {
-    return group_routes("moe_group_routes_ep", ids, M, A, E_total, e_lo, E_local, true, ws, ws_bytes, err, stream);
+    return group_routes("moe_group_routes_ep", ids, M, A, E_total, e_lo, E_local, true, ws, ws_bytes, err, true, stream);
 }
 
 int sxb_moe_route_small(const float *logits, int64_t ld, int64_t M, int64_t E_total, int64_t k, int64_t e_lo, int64_t E_local,
                         int32_t *ids, float *coef, void *ws, size_t ws_bytes, uint32_t *router_err, uint32_t *expert_err,
                         sxb_stream_t stream) {
-    const char *fn = "moe_route_small";
-    SXB_CHECK(logits != nullptr && ids != nullptr && coef != nullptr && ws != nullptr && router_err != nullptr && expert_err != nullptr,
-              fn, ": null pointer");
-    SXB_CHECK(E_total >= 1 && E_total <= 1024 && k >= 1 && k <= E_total && k <= 32 && ld >= E_total, fn, ": E = ", E_total, ", k = ", k,
-              ", ld = ", ld, " (E 1..1024, k 1..min(E, 32), ld >= E)");
-    SXB_CHECK(M >= 1 && M * k <= kSmallSlots, fn, ": M * k = ", M * k, " slots, this one-CTA form takes at most ", kSmallSlots,
-              " (use moe_router + moe_group_routes)");
-    SXB_CHECK(E_local >= 1 && E_local <= kMoeMaxExperts && e_lo >= 0 && e_lo + E_local <= E_total, fn, ": experts [", e_lo, ", ",
-              e_lo + E_local, ") outside [0, ", E_total, ")");
-    const bool ep = E_local != E_total;
-    const RouteWords L = route_words(M, k, E_local);
-    SXB_CHECK(ws_bytes >= (size_t)L.total * 4, fn, ": workspace of ", ws_bytes, " bytes, needs ", L.total * 4);
-    auto st = static_cast<cudaStream_t>(stream);
-    auto *w = static_cast<int32_t *>(ws);
-    // One CTA routes 32 tokens at a time, so from there on the router has a launch of its own, with a warp a token over the
-    // machine (150 tokens x 512 experts, top-10: 87 us as one launch).
-    if (M > kPackThreads / 32) {
-        if (int rc = sxb_moe_router(logits, ld, M, E_total, k, nullptr, 1, 0, ids, coef, SXB_ACT_F32, router_err, stream)) return rc;
-        launch_behind(pack_small_kernel, 1, kPackThreads, 0, st, 1, ids, L, (int)E_total, (int)e_lo, ep, w, expert_err);
-        SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
-        return SXB_OK;
-    }
-#define SXB_ROUTE_SMALL(NV) \
-    launch_behind(route_small_kernel<NV>, 1, kPackThreads, 0, st, 1, logits, ld, (int)M, (int)E_total, (int)k, ids, coef, L, (int)e_lo, ep, w, router_err, expert_err)
-    if (E_total <= 128) SXB_ROUTE_SMALL(4);
-    else if (E_total <= 256) SXB_ROUTE_SMALL(8);
-    else if (E_total <= 512) SXB_ROUTE_SMALL(16);
-    else SXB_ROUTE_SMALL(32);
-#undef SXB_ROUTE_SMALL
-    SXB_CHECK_LAUNCH(fn, " M=", M, " E=", E_total, " k=", k);
-    return SXB_OK;
+    return route_small("moe_route_small", logits, ld, M, E_total, k, e_lo, E_local, ids, coef, ws, ws_bytes, router_err, expert_err, true, stream);
 }
 
 }  // extern "C"

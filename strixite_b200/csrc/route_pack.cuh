@@ -23,6 +23,15 @@ struct RouteWords {
 };
 RouteWords route_words(int64_t M, int64_t A, int64_t E);
 
+// sxb_moe_route_small and sxb_moe_group_routes[_ep] (route_pack.cu).  let_in: whether the next launch of the stream may take its places while these few CTAs run.  In
+// front of the streaming expert kernel, which takes all registers of an SM and waits there, not where a second stream has work for the SMs:
+// one-token layer with the shared expert beside it, issued call by call, 64.8 us let in at once and 55.1 at the end; without a second
+// stream a layer of 512 x 128, one token, 18.8 and 19.9.
+int route_small(const char *fn, const float *logits, int64_t ld, int64_t M, int64_t E_total, int64_t k, int64_t e_lo, int64_t E_local, int32_t *ids, float *coef,
+                void *ws, size_t ws_bytes, uint32_t *router_err, uint32_t *expert_err, bool let_in, sxb_stream_t stream);
+int group_routes(const char *fn, const int32_t *ids, int64_t M, int64_t A, int64_t E_total, int64_t e_lo, int64_t E_local, bool ep, void *ws, size_t ws_bytes,
+                 uint32_t *err, bool let_in, sxb_stream_t stream);
+
 // Roles of the exact grouped forms in the status words (header words 5 .. 7), behind those of the tcgen05 kernels: a warp that waits for a tile's
 // staged activations, a staging warp that waits for the last warp to leave the buffer.
 constexpr int kRoleStaged = 10, kRoleLeft = 11;

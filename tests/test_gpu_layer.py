@@ -338,3 +338,45 @@ def test_inputs_written_just_before(cuda, T, captured):
     layer.check_errors()
     for (a, b), (c, e) in zip(want, got):
         assert torch.equal(a, c) and torch.equal(b, e)
+
+
+@pytest.mark.parametrize("T", [1, 32, 33, 204, 205, 255])
+@pytest.mark.parametrize("captured", [False, True])
+def test_second_stream_of_the_shared_expert(cuda, T, captured):
+    """One call with the shared expert on a stream of its own, where the routing lets the experts' first kernel in at its end, against the same call in order:
+    routing in one launch, with a router of its own, and of more slots than the one-CTA pack takes.  Same bits, pass after pass."""
+    from strixite_b200 import kernels as K
+    from strixite_b200.layer import MoeBuffers
+    E, A, d, I = 24, 10, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q = lambda rows, cols, bits: K.quantize(torch.randn((rows, cols), generator=g, device=cuda) * 0.05, 64, bits)
+    gu, dn, sgu, sdn = q(E * 2 * I, d, 4), q(E * d, I, 4), q(2 * I, d, 8), q(d, I, 8)
+    b, side = MoeBuffers(T, d, I, E, A, cuda, True), torch.cuda.Stream()
+    x, logits = torch.zeros((T, d), dtype=torch.bfloat16, device=cuda), torch.zeros((T, E + 1), device=cuda)
+    inputs = [(torch.randn((T, d), generator=g, device=cuda).to(torch.bfloat16), torch.randn((T, E + 1), generator=g, device=cuda)) for _ in range(4)]
+
+    def call(y, side):
+        K.moe_layer(x, logits, y, gu, dn, E, A, b.ids, b.coef, b.ws, b.ws_bytes, b.h, b.partial, b.router_err, b.expert_err, math=K.MoeMath.F32, side=side,
+                    shared_gate_up=sgu, shared_down=sdn, sh_gu=b.sh_gu, sh_h=b.sh_h, sh_y=b.sh_y32)
+
+    want, got, y = [], [], torch.empty((T, d), device=cuda)
+    for xi, li in inputs:
+        x.copy_(xi), logits.copy_(li)
+        call(y, None)
+        torch.cuda.synchronize()
+        want.append(y.clone())
+    run = lambda: call(y, side)
+    run()
+    if captured:
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            run()
+        run = graph.replay
+    for xi, li in inputs:
+        x.copy_(xi), logits.copy_(li)
+        run()
+        got.append(y.clone())
+    torch.cuda.synchronize()
+    K.check_grouped_status(b.ws, "two streams")
+    assert all(torch.equal(p, r) for p, r in zip(want, got))
