@@ -23,16 +23,21 @@
 //     phase ahead, a deeper item ring or a second quarter dequantized before the stage is free: no faster (+0 to +1 %).
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
+//   * Where contractions are short the item counts: eight steps of down against 4500 instructions of epilogue at 80 tokens, 230 a warp and pass, which
+//     made it the bound (it worked 6700 of an item's 7300 cycles), and the producers waited for it in an item ring of two.  Output rows through the item
+//     ring, shared memory in place of a shuffle a token, gate and up in one thread: down 1900 instructions an item fewer; scan loops that do not unroll: 72 KB of
+//     code, now 50.  Under load, us: down with its combine 654 -> 600 at 4096 tokens, 2449 -> 2281 at 16384 (Q8), 353 at 777 either way; gate/up 847 -> 838,
+//     2669 -> 2620 and 598 -> 586.  The next item's scales asked into L2 ahead of the scan: gate/up 2 % slower, down no faster.
 // Why 128 tokens: that leaves tensor memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column
 // stages of A.  An expert of more tokens has its rows dequantized again for every 128 of them; a wider tile, which would share that at the price of an
 // accumulator or of stages, has not been built.
-// Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 506 us at 777 tokens (15 an expert), 685 at
-// 4096 (80 an expert); down 291 and 480 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
+// Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 505 us at 777 tokens (15 an expert), 685 at
+// 4096 (80 an expert); down 283 and 430 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
 //
 // SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up
-// rows of the same h columns, and the epilogue pairs them with one shuffle per value: of the 16 tokens of a pass the gate
-// lane finishes the first 8, the up lane the other 8.
+// rows of the same h columns, and the epilogue reads both in the sixteen-lane form of tcgen05.ld, which gives a thread a gate value
+// and its up value.
 //
 // Operands as in grouped_tc.cu: A (weights) dequantized in registers and stored to tensor memory by the producer warps
 // (the [tmem] form of tcgen05.mma), B (activations) two cp.async.bulk per step (one per 64-k sub-tile) into
@@ -82,14 +87,16 @@ struct Shape {
     static_assert(kAccs * kTile + kStages * kAStageCols <= kTmemCols, "tensor memory");
     static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
-constexpr int kItemRing = 2;
+constexpr int kItemRing = 4;
 // kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
 constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
-// The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).  Rows at natural magnitude: scale = -2^24.
+// The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).  Rows at natural magnitude: scale = -2^24.  The item
+// ring holds a scale's biased exponent, 0 for kNatural.
 constexpr float kNatural = -0x1p24f;
 __host__ __device__ constexpr uint32_t unscale_bits(uint32_t scale_bits) { return ((127u + 24u + 127u) << 23) - scale_bits; }  // past int
 static_assert(unscale_bits((127u + 24u) << 23) == 127u << 23 && unscale_bits((127u - 1u) << 23) == (127u + 25u) << 23, "2^(24 - k)");
+__device__ inline float scale_of(uint8_t exponent) { return exponent != 0 ? __uint_as_float((uint32_t)exponent << 23) : kNatural; }
 __device__ inline float unscale(float scale) { return __uint_as_float(unscale_bits(__float_as_uint(fabsf(scale)))); }
 
 struct Item {
@@ -121,21 +128,6 @@ template <int MODE>
 __device__ inline int row_blocks(const TcArgs &a) {
     return MODE == kTcSwiglu ? (int)((a.N / 2 + kRows / 2 - 1) / (kRows / 2)) : (int)((a.N + kRows - 1) / kRows);
 }
-__device__ inline Item item_info(const TcArgs &a, int item, int rbs) {
-    Item it;
-    const int tile = item / rbs;
-    it.rb = item % rbs;
-    if (a.dense_M > 0) {  // dense projection: tile t holds rows dense_tile * t .. of the one group
-        it.bucket = 0, it.start = tile * a.dense_tile;
-        it.cnt = (int)min((int64_t)a.dense_tile, a.dense_M - it.start);
-        return it;
-    }
-    it.bucket = a.ws[a.L.t128_bucket + tile];
-    it.start = a.ws[a.L.t128_start + tile];
-    it.cnt = min(kTile, a.ws[a.L.offsets + it.bucket + 1] - it.start);
-    return it;
-}
-
 // Scales and mins (BF16 bits) of N consecutive groups of a row.
 template <int N>
 struct Scales {
@@ -204,13 +196,13 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                   kEpiWarps = S::kEpiWarps, kMmaWarp = S::kMmaWarp, kBCopyWarp = S::kBCopyWarp, kWCopyWarp = S::kWCopyWarp,
                   kItemWarp = S::kItemWarp, kFirstAWarp = S::kFirstAWarp;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    // 1024-byte alignment of the operand tiles (the swizzle pattern repeats every 1024 bytes).
-    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char *const smem = smem_raw;  // 1024-byte aligned, as the operand tiles want it (the swizzle pattern repeats every 1024 bytes)
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[kAccs], acc_empty[kAccs], drain_bar;
     __shared__ uint64_t w_full[kWSlots], w_empty[kWSlots];
     __shared__ uint64_t item_full[kItemRing], item_empty[kItemRing];
     __shared__ __align__(16) Item item_ring[kItemRing];
-    __shared__ float row_scale[kItemRing][kRows];
+    __shared__ uint8_t row_scale[kItemRing][kRows];
+    __shared__ __align__(16) uint32_t out_row[kItemRing][kTile];  // where a token's output row starts, in 16-byte units
     __shared__ uint32_t tmem_base_smem;
     __shared__ int abort_flag;
 
@@ -246,9 +238,9 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         }
     };
     // All 512 columns are this CTA's, so they start at column 0, and the code below says so with constants.
-    if (tmem_base_smem != 0 && threadIdx.x == 0) raise_abort(0, 0);
+    const bool run = tmem_base_smem == 0 && (smem_u32(smem) & 1023u) == 0;
+    if (!run && threadIdx.x == 0) raise_abort(0, 0);
     __syncthreads();
-    const bool run = tmem_base_smem == 0;
 
     const uint32_t b_base = smem_u32(smem), w_base = b_base + (uint32_t)(kStages * kStageBytes);
     uint32_t issued = 0;  // ring slots issued by this thread (the ring's thread only)
@@ -271,7 +263,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
             return no_item;
         }
         const Item it = item_ring[i % kItemRing];
-        scale = row_scale[i % kItemRing][p];
+        scale = scale_of(row_scale[i % kItemRing][p]);
         __syncwarp();
         if (lane == 0) mbar_arrive(&item_empty[i % kItemRing]);
         return it;
@@ -416,11 +408,35 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         // contractions are short this is the longest chain of an item: its instructions count.
         const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
         const bool pair_scales = groups % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 3) == 0;
-        Item nxt = blockIdx.x < n_items ? item_info(a, blockIdx.x, rbs) : no_item;
+        // What it needs to know of an item takes two loads, the second from where the first says: the first one for the next item is under way while
+        // this one's scales are looked at.
+        const int tiles_by = (int)gridDim.x / rbs, rbs_by = (int)gridDim.x % rbs;
+        int tile = (int)blockIdx.x / rbs, rb = (int)blockIdx.x % rbs;
+        auto look_up = [&](Item &x) {
+            x.rb = rb;
+            if (a.dense_M > 0) x.bucket = 0, x.start = tile * a.dense_tile;  // dense projection: tile t holds rows dense_tile * t .. of the one group
+            else x.bucket = a.ws[a.L.t128_bucket + tile], x.start = a.ws[a.L.t128_start + tile];
+            tile += tiles_by, rb += rbs_by;
+            if (rb >= rbs) rb -= rbs, ++tile;
+        };
+        auto count_of = [&](const Item &x) {
+            return a.dense_M > 0 ? (int)min((int64_t)a.dense_tile, a.dense_M - x.start) : min(kTile, a.ws[a.L.offsets + x.bucket + 1] - x.start);
+        };
+        const int64_t row_bytes = MODE == kTcSwiglu ? a.N : a.N * (MODE == kTcPartial ? 4 : 2);  // of the output
+        const bool rows_wanted = MODE != kTcHcUp && !(MODE == kTcSwiglu && a.out_f16 >= 3);  // the tile-blocked h follows from the positions
+        Item nxt = no_item;
+        if ((int)blockIdx.x < n_items) look_up(nxt), nxt.cnt = count_of(nxt);
         for (int i = 0;; ++i) {
             const Item it = nxt;
             const int item = blockIdx.x + i * gridDim.x;
-            nxt = item + (int)gridDim.x < n_items ? item_info(a, item + gridDim.x, rbs) : no_item;
+            const bool more = item + (int)gridDim.x < n_items;
+            nxt = no_item;
+            if (more) look_up(nxt);
+            int slot[4] = {0, 0, 0, 0};
+            if (rows_wanted && it.bucket >= 0) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) slot[r] = r * 32 + lane < it.cnt ? slot_at(it.start + r * 32 + lane) : 0;
+            }
             // Of every group v = max(|scale| * 2^8, |min|) as BF16 bits, 0x400 = an empty group; two 16-bit maxima of v, and signed
             // minima of v + 0x7bff, in which an empty group's is the largest.  Five instructions for two groups.
             uint32_t top[4] = {0u, 0u, 0u, 0u}, low[4] = {0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu};
@@ -436,7 +452,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                     at[r] = (wrow < 0 ? row_of(it, 0) : wrow) * groups;  // lanes past the expert's end look at a row that exists
                 }
                 if (vec_scales) {
-#pragma unroll 2
+#pragma unroll 1
                     for (int g = 0; g < groups; g += 8) {
                         uint4 sv[4], mv[4];
 #pragma unroll
@@ -449,17 +465,19 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                             take(r, sv[r].x, mv[r].x), take(r, sv[r].y, mv[r].y), take(r, sv[r].z, mv[r].z), take(r, sv[r].w, mv[r].w);
                     }
                 } else if (pair_scales) {
-#pragma unroll 2
+#pragma unroll 1
                     for (int g = 0; g < groups; g += 2)
 #pragma unroll
                         for (int r = 0; r < 4; ++r)
                             take(r, __ldg(reinterpret_cast<const uint32_t *>(a.scale + at[r] + g)), __ldg(reinterpret_cast<const uint32_t *>(a.minv + at[r] + g)));
                 } else {
+#pragma unroll 1
                     for (int g = 0; g < groups; ++g)
 #pragma unroll
                         for (int r = 0; r < 4; ++r) take(r, __ldg(a.scale + at[r] + g), __ldg(a.minv + at[r] + g));
                 }
             }
+            if (more) nxt.cnt = count_of(nxt);
             if (i >= kItemRing) {
                 const bool ok = mbar_wait(&item_empty[i % kItemRing], ((uint32_t)(i / kItemRing) & 1u) ^ 1u, abort_v, a.wait_limit_ns);
                 if (!__all_sync(0xffffffffu, ok)) {
@@ -474,7 +492,8 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 const int hi = (int)max(top[r] >> 16, top[r] & 0xffffu), lo = min((int)low[r] >> 16, (int)(int16_t)low[r]);
                 const int e = min(max((hi >> 7) - 8, 127 - 24), 127 + 15), e_low = (((lo - 0x7bff) & 0xffff) >> 7) - 8;
                 const bool spread = __any_sync(0xffffffffu, e > 127 - 10 && lo != 0x7fff && e_low < e - kScaleSpread);
-                row_scale[i % kItemRing][r * 32 + lane] = spread ? kNatural : __int_as_float((127 + 14 + 127 - e) << 23);
+                row_scale[i % kItemRing][r * 32 + lane] = spread ? 0 : (uint8_t)(127 + 14 + 127 - e);
+                if (rows_wanted) out_row[i % kItemRing][r * 32 + lane] = (uint32_t)(((int64_t)slot[r] * row_bytes) >> 4);
             }
             if (lane == 0) item_ring[i % kItemRing] = it;
             __syncwarp();
@@ -720,50 +739,27 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         }
     } else if (warp < kEpiWarps) {
         // ===================== epilogue =====================
-        // Lane = weight row: 16 tokens at a time from tensor memory into registers (two loads of 8 columns: a longer pass
-        // would be more code than the instruction caches hold beside the producers'), then one store per token straight
-        // to global memory - for a fixed token a warp's rows are contiguous bytes.  Tensor memory goes back to the MMA
-        // thread as soon as the item's last columns are in registers.  What depends on the token - the output row of its slot - is
-        // computed by lane t for token t of the pass and handed round by shuffles; a line of the tile-blocked h follows from
-        // the token's position.
+        // 16 tokens at a time from tensor memory into registers, stored straight to global memory: for a fixed token a warp's rows are
+        // contiguous bytes.  Tensor memory goes back to the MMA warp as soon as the item's last columns are in registers.  Where a token's
+        // output row starts comes through the item ring; a line of the tile-blocked h follows from the token's position.  A pass runs as
+        // straight code that the warp has to itself, at about eight cycles an instruction beside the producers: instructions count.
         uint32_t acc_count = 0;
         const int64_t I = a.N / 2;
-        const bool tiled_out = MODE == kTcSwiglu && a.out_f16 >= 3;
-        const bool h_as_f16 = a.out_f16 != 0, q4_order = a.out_f16 == 2 || a.out_f16 == 3;
         const uint32_t lane_addr = (uint32_t)(warp * 32) << 16;  // warp = the lane quadrant it may read
-        const int up_lane = lane >> 4;  // SwiGLU: lanes 16-31 hold the up rows of the h columns of lanes 0-15
         for (int i = 0;; ++i) {
-            float scale = 1.f;
-            const Item it = read_item(i, warp * 32 + lane, scale);
-            if (it.bucket < 0) break;
-            const float back = unscale(scale);  // undoes the row's power of two
-            const bool valid = it.bucket < a.E;
-            // per-thread constants of the item: byte offset of this thread's element inside a token's output row / line
-            int64_t elem_off;
-            uint32_t xor_chunk = 0;  // tile-blocked h: 16-byte chunk of the line, before the per-token swizzle
-            bool row_ok;
-            if (MODE == kTcSwiglu) {
-                const int64_t j = (int64_t)it.rb * (kRows / 2) + warp * 16 + (lane & 15);  // h column
-                const int j7 = (int)(j & 7), pos = q4_order ? (((j7 & 3) << 1) | (j7 >> 2)) : j7;  // [0 4 1 5 2 6 3 7]
-                row_ok = j < I;
-                if (tiled_out) elem_off = (j >> 6) * a.L.S * 128 + pos * 2 + (int64_t)(it.start + 8 * up_lane) * 128, xor_chunk = (uint32_t)((j & 63) >> 3);
-                else elem_off = ((j & ~(int64_t)7) + pos) * 2;
-            } else {
-                const int64_t r = (int64_t)it.rb * kRows + warp * 32 + lane;
-                row_ok = r < a.N;
-                elem_off = r * (MODE == kTcPartial ? 4 : 2);
+            const int ring = i % kItemRing;
+            {
+                const bool ok = mbar_wait(&item_full[ring], (uint32_t)(i / kItemRing) & 1u, abort_v, a.wait_limit_ns);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 8);
+                    break;
+                }
             }
-            // Slot of token n of the item (lanes 0-15 and again 16-31; fetched one pass ahead: nothing may depend on the loaded
-            // value before the next pass, or the in-order issue would stall this pass's stores behind it).
-            auto token_slot = [&](int n) -> int { return (tiled_out || n >= it.cnt) ? 0 : slot_at(it.start + n); };
-            // Offset of a token's output row, in 16-byte units.
-            auto token_off = [&](int slot) -> uint32_t {
-                return (uint32_t)(((int64_t)slot * (MODE == kTcSwiglu ? I * 2 : a.N * (MODE == kTcPartial ? 4 : 2))) >> 4);
-            };
-            int slot_nxt = token_slot(lane & 15);
-            uint32_t half = 0;
+            const Item it = item_ring[ring];
+            if (it.bucket < 0) break;
+            const bool valid = it.bucket < a.E;
+            const uint32_t half = acc_count & 1u, acc = lane_addr + half * (uint32_t)kTile;
             if (valid) {
-                half = acc_count & 1u;
                 const uint32_t acc_phase = (acc_count >> 1) & 1u;
                 ++acc_count;
                 const bool ok = mbar_wait(&acc_full[half], acc_phase, abort_v, a.wait_limit_ns);
@@ -773,52 +769,81 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 }
                 tc_fence_after();
             }
-            unsigned char *out = static_cast<unsigned char *>(a.out) + elem_off;
-            for (int c0 = 0; c0 < it.cnt; c0 += 16) {
-                float va[8], vb[8];  // this row's accumulators of tokens c0 .. c0 + 7 and c0 + 8 .. c0 + 15
-                if (valid) {
-                    tc_ld8x2(lane_addr + half * (uint32_t)kTile + (uint32_t)c0, va, vb);
-                    if (c0 + 16 >= it.cnt) {  // the last columns are out: this warp's share of the accumulator is free
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&acc_empty[half]);
-                    }
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) va[t] *= back, vb[t] *= back;
-                } else {
-#pragma unroll
-                    for (int t = 0; t < 8; ++t) va[t] = vb[t] = qnan_f32();
+            // What undoes a row's power of two.  Slots with an id outside [0, E) have no products: their rows become NaN.
+            auto back_of = [&](int p) { return valid ? unscale(scale_of(row_scale[ring][warp * 32 + p])) : qnan_f32(); };
+            auto columns_read = [&](int c0) {  // the last columns are out: this warp's share of the accumulator is free
+                if (valid && c0 + 16 >= it.cnt) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[half]);
                 }
-                const uint32_t off_cur = token_off(slot_nxt);
-                if (c0 + 16 < it.cnt) slot_nxt = token_slot(c0 + 16 + (lane & 15));
-                const int live = row_ok ? it.cnt - c0 : 0;  // tokens of this pass; the columns past them are computed and dropped
+            };
+            if constexpr (MODE == kTcSwiglu) {
+                // Gate rows are the quadrant's lanes 0-15, the up rows of the same h columns its lanes 16-31.  Read in the form of sixteen
+                // lanes by eight columns, both give a thread the same places: h columns r0 and r0 + 8 of tokens t and t + 1, and of
+                // t + 8 and t + 9.  From the FP32 accumulators, rounded once (kernels/moe_grouped.hip:508-524).
+                const int r0 = lane >> 2, t0 = (lane & 3) * 2;
+                const float g0 = back_of(r0), g1 = back_of(r0 + 8), u0 = back_of(r0 + 16), u1 = back_of(r0 + 24);
+                const bool h_as_f16 = a.out_f16 != 0, q4_order = a.out_f16 == 2 || a.out_f16 == 3, tiled_out = a.out_f16 >= 3;
+                const int64_t j0 = (int64_t)it.rb * (kRows / 2) + warp * 16 + r0;  // h column; j0 + 8 is the other
+                const bool ok0 = j0 < I, ok1 = j0 + 8 < I;
+                const int pos = q4_order ? (((r0 & 3) << 1) | (r0 >> 2)) : r0;  // [0 4 1 5 2 6 3 7]
+                // tile-blocked h: the token's line, its 16-byte chunks swizzled by the token; token t + 1 is the odd one of the pair
+                const uint32_t in0 = (uint32_t)(t0 * 128 + (((2 * warp) ^ t0) << 4) + pos * 2), in1 = in0 ^ 16u;
+                unsigned char *const out = static_cast<unsigned char *>(a.out) +
+                                           (tiled_out ? ((int64_t)it.rb * a.L.S + it.start) * 128 : ((j0 & ~(int64_t)7) + pos) * 2);
+                for (int c0 = 0; c0 < it.cnt; c0 += 16) {
+                    float g[8] = {}, u[8] = {};
+                    if (valid) tc_ld16lanes_x2(acc + (uint32_t)c0, acc + (16u << 16) + (uint32_t)c0, g, u);
+                    columns_read(c0);
+                    uint16_t h[8];
 #pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    if (MODE == kTcSwiglu) {
-                        // the gate lane finishes token c0 + t, its up lane token c0 + 8 + t: each sends the other the
-                        // value that one needs (kernels/moe_grouped.hip:508-524: from the FP32 accumulators, rounded once)
-                        const float theirs = __shfl_xor_sync(0xffffffffu, up_lane ? va[t] : vb[t], 16);
-                        const float g = up_lane ? theirs : va[t], u = up_lane ? vb[t] : theirs;
-                        const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(silu_fast(g) * u));
-                        const uint16_t hv = h_as_f16 ? __half_as_ushort(__float2half_rn(bf16_bits_to_f32(b))) : b;
-                        unsigned char *p = out;
-                        if (tiled_out) p += t * 128 + ((xor_chunk ^ (uint32_t)t) << 4);
-                        else p += (int64_t)__shfl_sync(0xffffffffu, off_cur, t + 8 * up_lane) << 4;
-                        if (t + 8 * up_lane < live) *reinterpret_cast<uint16_t *>(p) = hv;
+                    for (int t = 0; t < 8; ++t) {
+                        const float gv = g[t] * ((t & 2) ? g1 : g0), uv = u[t] * ((t & 2) ? u1 : u0);
+                        const uint16_t b = __bfloat16_as_ushort(__float2bfloat16_rn(silu_fast(gv) * uv));
+                        h[t] = h_as_f16 ? __half_as_ushort(__float2half_rn(bf16_bits_to_f32(b))) : b;
+                    }
+                    const int live = it.cnt - c0 - t0;  // of this thread's tokens: 0, 1, 8, 9 from t0 on
+                    auto put = [&](unsigned char *p, int t, int token, bool ok) { st_global_if(ok && token < live, p, h[t]); };
+                    if (tiled_out) {
+                        unsigned char *const p0 = out + (int64_t)c0 * 128 + in0, *const p1 = out + (int64_t)c0 * 128 + in1;
+                        put(p0, 0, 0, ok0), put(p1, 2, 0, ok1), put(p1 + 128, 1, 1, ok0), put(p0 + 128, 3, 1, ok1);
+                        put(p0 + 1024, 4, 8, ok0), put(p1 + 1024, 6, 8, ok1), put(p1 + 1152, 5, 9, ok0), put(p0 + 1152, 7, 9, ok1);
                     } else {
-                        const int64_t off_a = (int64_t)__shfl_sync(0xffffffffu, off_cur, t) << 4;
-                        const int64_t off_b = (int64_t)__shfl_sync(0xffffffffu, off_cur, t + 8) << 4;
-                        if (MODE == kTcPartial) {
-                            if (t < live) *reinterpret_cast<float *>(out + off_a) = va[t];
-                            if (t + 8 < live) *reinterpret_cast<float *>(out + off_b) = vb[t];
-                        } else {  // BF16 rows: the plain gather's y, or the per-slot dots as kernels/moe_grouped.hip:47-57 stores them
-                            if (t < live) *reinterpret_cast<uint16_t *>(out + off_a) = __bfloat16_as_ushort(__float2bfloat16_rn(va[t]));
-                            if (t + 8 < live) *reinterpret_cast<uint16_t *>(out + off_b) = __bfloat16_as_ushort(__float2bfloat16_rn(vb[t]));
-                        }
+                        const uint2 a_b = *reinterpret_cast<const uint2 *>(&out_row[ring][c0 + t0]), c_d = *reinterpret_cast<const uint2 *>(&out_row[ring][c0 + t0 + 8]);
+                        unsigned char *const pa = out + (uint64_t)a_b.x * 16, *const pb = out + (uint64_t)a_b.y * 16, *const pc = out + (uint64_t)c_d.x * 16,
+                                             *const pd = out + (uint64_t)c_d.y * 16;
+                        put(pa, 0, 0, ok0), put(pa + 16, 2, 0, ok1), put(pb, 1, 1, ok0), put(pb + 16, 3, 1, ok1);
+                        put(pc, 4, 8, ok0), put(pc + 16, 6, 8, ok1), put(pd, 5, 9, ok0), put(pd + 16, 7, 9, ok1);
                     }
                 }
-                if (tiled_out) out += 16 * 128;
+            } else {
+                // Lane = weight row; FP32 rows, or BF16 rows: the plain gather's y, or the per-slot dots as kernels/moe_grouped.hip:47-57 stores them.
+                const float back = back_of(lane);
+                const int64_t r = (int64_t)it.rb * kRows + warp * 32 + lane;
+                const int rows_live = r < a.N ? it.cnt : 0;
+                unsigned char *const out = static_cast<unsigned char *>(a.out) + r * (MODE == kTcPartial ? 4 : 2);
+                for (int c0 = 0; c0 < it.cnt; c0 += 16) {
+                    float v[16] = {};
+                    if (valid) tc_ld16(acc + (uint32_t)c0, v);
+                    columns_read(c0);
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) v[t] *= back;
+                    const int live = rows_live - c0;  // tokens of this pass; the columns past them are computed and dropped
+#pragma unroll
+                    for (int t = 0; t < 16; t += 4) {
+                        const uint4 row = *reinterpret_cast<const uint4 *>(&out_row[ring][c0 + t]);
+                        auto put = [&](uint32_t at, int k) {
+                            unsigned char *const p = out + (uint64_t)at * 16;
+                            if (MODE == kTcPartial) st_global_if(k < live, p, v[k]);
+                            else st_global_if(k < live, p, __bfloat16_as_ushort(__float2bfloat16_rn(v[k])));
+                        };
+                        put(row.x, t), put(row.y, t + 1), put(row.z, t + 2), put(row.w, t + 3);
+                    }
+                }
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&item_empty[ring]);
         }
     }
 
@@ -826,6 +851,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     // the thread that ran the ring of weight codes waits, bounded, for the last fill of every slot; the activation copies
     // complete on barriers that also count thread arrivals, so their issuer lets a generous time pass instead.
     if (*abort_v) {
+#pragma unroll 1
         for (int sl = 0; sl < kWSlots && issued > 0; ++sl) {
             if (issued <= (uint32_t)sl) continue;
             const uint32_t last = ((issued - 1 - (uint32_t)sl) / kWSlots) * kWSlots + (uint32_t)sl;
@@ -872,7 +898,7 @@ int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)(a.E * a.N), row_bytes, (uint32_t)(kBK * BITS / 8),
                                (uint32_t)(kRows / 2), BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
         return rc;
-    const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + 1024 +
+    const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes +
                         (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
     auto go = [&](auto kern) -> int {
         SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");

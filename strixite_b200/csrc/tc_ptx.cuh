@@ -121,18 +121,26 @@ __device__ inline void tc_ld16x2(uint32_t taddr0, uint32_t taddr1, float (&v0)[1
 #pragma unroll
     for (int i = 0; i < 16; ++i) v0[i] = __uint_as_float(r[i]), v1[i] = __uint_as_float(q[i]);
 }
-// 2 x 8 consecutive columns of this thread's TMEM lane.
-__device__ inline void tc_ld8x2(uint32_t taddr, float (&v0)[8], float (&v1)[8]) {
-    uint32_t r[8], q[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
-                 : "r"(taddr + 8));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v0[i] = __uint_as_float(r[i]), v1[i] = __uint_as_float(q[i]);
+// 16 consecutive columns of this thread's TMEM lane.
+__device__ inline void tc_ld16(uint32_t taddr, float (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]),
+          "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+// 16 lanes x 16 columns from each of two addresses: of every eight columns a thread gets those 2 (lane % 4) and the next one of TMEM lanes
+// lane / 4 (two values) and lane / 4 + 8 (two values).
+__device__ inline void tc_ld16lanes_x2(uint32_t taddr0, uint32_t taddr1, float (&v0)[8], float (&v1)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+        "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v0[0]), "=f"(v0[1]), "=f"(v0[2]), "=f"(v0[3]), "=f"(v0[4]), "=f"(v0[5]), "=f"(v0[6]), "=f"(v0[7]), "=f"(v1[0]), "=f"(v1[1]), "=f"(v1[2]),
+          "=f"(v1[3]), "=f"(v1[4]), "=f"(v1[5]), "=f"(v1[6]), "=f"(v1[7])
+        : "r"(taddr0), "r"(taddr1)
+        : "memory");
 }
 // 2^v on the special-function unit.
 __device__ inline float exp2_fast(float v) {
@@ -262,6 +270,13 @@ __device__ inline void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, 
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
+}
+// Stores where `pred` holds, without a branch around them.
+__device__ inline void st_global_if(bool pred, void *p, float v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v), "r"((uint32_t)pred) : "memory");
+}
+__device__ inline void st_global_if(bool pred, void *p, uint16_t v) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.global.u16 [%0], %1;\n\t}" ::"l"(p), "h"(v), "r"((uint32_t)pred) : "memory");
 }
 // 16 bytes global -> shared without passing through registers (both addresses 16-byte aligned); complete, for the
 // issuing thread, after cp_async_wait<N> has let at most N of its later groups remain in flight.

@@ -633,6 +633,53 @@ def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
     assert not bad and lib.sxb_release_scratch() == 0
 
 
+@pytest.mark.parametrize("bits,G", [(4, 128), (8, 32)])
+@pytest.mark.parametrize("N,Kd", [(16, 128), (48, 384), (144, 256), (272, 128)])
+def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd):
+    """Tiles of one token, around eight, sixteen and thirty-two and around a full tile, one and several steps of the contraction, rows that end inside
+    a row block, slots without an expert: every output form of the kernel for tile-blocked activations, bit for bit the general kernel's (which a captured
+    call runs on): the same operands, summed in the same order."""
+    from strixite_b200 import kernels as K
+    counts = [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 128, 129]
+    E, g = len(counts), torch.Generator(device="cuda").manual_seed(N + bits)
+    ids = torch.cat([torch.repeat_interleave(torch.arange(E), torch.tensor(counts)), torch.full((19,), E + 3)]).to(torch.int32)
+    M = ids.numel()
+    ids = ids[torch.randperm(M, generator=torch.Generator().manual_seed(N))].to(cuda)[:, None].contiguous()
+    w = K.quantize(torch.randn((E * N, Kd), generator=g, device=cuda) * 0.05, G, bits)
+    x = torch.randn((M, Kd), generator=g, device=cuda).to(torch.bfloat16)
+    coef, err = torch.rand((M, 1), generator=g, device=cuda), torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = K.moe_route_workspace_bytes(M, 1, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    K.moe_group_routes(ids, M, 1, E, ws, nbytes, err)
+    partial, f32 = torch.empty((M, N), device=cuda), K.Act.F32
+
+    def combine(y, math, out):
+        K.linear_qw_experts_combine_grouped(x, w, E, ids, coef, ws, nbytes, partial, M, 1, y, K.Act.BF16, math, out_act=out)
+
+    def gate_up(y, h_f16):
+        K.linear_qw_experts_gather_grouped_swiglu(x, w, E, ws, nbytes, M, 1, y, K.Act.BF16, K.MoeMath.WmmaF16, h_f16=h_f16)
+
+    forms = [("rows", torch.bfloat16, N, lambda y: K.linear_qw_experts_gather_grouped(x, w, E, ws, nbytes, M, 1, y, K.Act.BF16, K.MoeMath.WmmaF16)),
+             ("gate/up", torch.bfloat16, N // 2, lambda y: gate_up(y, 0)), ("gate/up F16", torch.float16, N // 2, lambda y: gate_up(y, 1)),
+             ("gate/up F16, Q4 order", torch.float16, N // 2, lambda y: gate_up(y, 2)),
+             ("FP32 dots", torch.float32, N, lambda y: combine(y, K.MoeMath.WmmaF16F32Partials, f32)),
+             ("BF16 dots", torch.float32, N, lambda y: combine(y, K.MoeMath.WmmaF16, f32))]
+    live = (ids[:, 0] < E).cpu()
+    for name, dtype, cols, call in forms:
+        y = [torch.full((M + 1, cols), 77.0, dtype=dtype, device=cuda) for _ in range(2)]
+        call(y[0])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call(y[1])
+        graph.replay()
+        torch.cuda.synchronize()
+        K.check_grouped_status(ws, name)
+        got, want = (v.cpu() for v in y)
+        assert torch.equal(got[:M][live].view(torch.uint8), want[:M][live].view(torch.uint8)), name
+        assert bool(torch.isnan(got[:M][~live]).all()) and not bool(torch.isnan(got[:M][live]).any()), name
+        assert bool((got[M] == 77.0).all()), name  # nothing past the last row
+
+
 @pytest.mark.parametrize("tiles,N", [(1, 16), (3, 1040), (5, 2064), (49, 512), (74, 1024), (75, 512), (140, 1536), (148, 32), (149, 64)])
 def test_exact_grouped_runs_of_units(cuda, tiles, N):
     """Tiles of units dealt inside tiles and evenly: one unit a warp or fewer, several rounds, CTAs left over, both sides of as many tiles as CTAs; bit for
