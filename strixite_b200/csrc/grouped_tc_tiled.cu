@@ -28,11 +28,18 @@
 //     ring, shared memory in place of a shuffle a token, gate and up in one thread: down 1900 instructions an item fewer; scan loops that do not unroll: 72 KB of
 //     code, now 50.  Under load, us: down with its combine 654 -> 600 at 4096 tokens, 2449 -> 2281 at 16384 (Q8), 353 at 777 either way; gate/up 847 -> 838,
 //     2669 -> 2620 and 598 -> 586.  The next item's scales asked into L2 ahead of the scan: gate/up 2 % slower, down no faster.
+//   * Scales and mins lie in shared memory where two items' fit, up to 32 groups a row (SS): the item warp reads them anyway.  Producers that each ask for their
+//     own row's groups (what is left for longer rows) fetch two bytes from each of 32 sectors a load, as many bytes from L2 as the codes are, and
+//     carry pointers and the next item's rows along: 1330 instructions a step against 1140 (gate/up, 15 tokens an expert), for twelve ring slots of Q4 codes
+//     against eight.  Under load, us: gate/up 609 -> 582 at 777 tokens, 881 -> 847 at 4096, 2650 -> 2566 at 16384; down with its combine 363 -> 345, 627 -> 613,
+//     2348 -> 2309 (Q8); dense 1001 x 8192 x 4096 Q4 61.5 -> 59.0, 4096 x 4096 x 1024 Q8 43.4 -> 38.6.
+//   * In down the item warp is the longest chain, 4500 cycles an item: so it asks for the next item's scales, in HBM, before it has published this one (down 361 ->
+//     345 at 777 tokens).  A second item warp leaves 72 registers a thread: down 350 -> 336, gate/up 550 -> 562.
 // Why 128 tokens: that leaves tensor memory for two accumulators (an item's epilogue runs under the next item's mainloop) and four 64-column
 // stages of A.  An expert of more tokens has its rows dequantized again for every 128 of them; a wider tile, which would share that at the price of an
 // accumulator or of stages, has not been built.
-// Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 505 us at 777 tokens (15 an expert), 685 at
-// 4096 (80 an expert); down 283 and 430 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
+// Measured, 512 experts, d = 4096, I = 1024, Q4, a few launches at a time: gate/up + SwiGLU 495 us at 777 tokens (15 an expert), 670 at
+// 4096 (80 an expert); down 275 and 425 (gathering row-major activations the same products took 1052, 1132, 820 and 861).
 //
 // SwiGLU: gate row j and up row j are rows of the same accumulator, so they cannot share a lane.  An item holds 64
 // gate rows and their 64 up rows; inside every tensor-memory lane quadrant lanes 0-15 are gate rows and lanes 16-31 the up
@@ -71,14 +78,15 @@ constexpr int kTmemCols = 512;
 
 // HC: the hyper-connection up mix (kTcHcUp), whose contraction is short and whose epilogue needs registers and shared memory:
 // half the producers, stages and ring slots.
+// SS: the scales of the items at hand lie in shared memory.
 // A set of four producer warps (one per lane quadrant) owns one stage, and its own ring slots: it meets every barrier it
 // waits on again only after it has seen that barrier's previous phase end, so watching the parity is enough.
-template <int BITS, bool HC>
+template <int BITS, bool HC, bool SS>
 struct Shape {
     static constexpr int kWays = HC ? 2 : 4;  // producer sets
     static constexpr int kStages = kWays;
     static constexpr int kSlotBytes = kRows * kBK * BITS / 8;  // a ring slot: the packed codes of a step, 8 or 16 KB
-    static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 4 ? 3 : 1);  // what shared memory holds beside the stages (Q4, 8 -> 12 slots: 583 -> 572 us at 777 tokens)
+    static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 8 ? 1 : SS ? 2 : 3);  // what shared memory holds beside the stages and the scales (Q4, 8 -> 12 slots: 583 -> 572 us at 777 tokens)
     static constexpr int kEpiSets = HC ? 2 : 1;  // epilogue warps per lane quadrant
     static constexpr int kEpiWarps = 4 * kEpiSets, kMmaWarp = kEpiWarps, kBCopyWarp = kEpiWarps + 1, kWCopyWarp = kEpiWarps + 2,
                          kItemWarp = kEpiWarps + 3, kFirstAWarp = kEpiWarps + 4;
@@ -88,6 +96,10 @@ struct Shape {
     static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
 constexpr int kItemRing = 4;
+constexpr int kScaleGroups = 32;  // SS: groups of a row at most
+// ... items whose scales lie in shared memory, as a power of two
+__host__ __device__ constexpr int scale_bufs_log(int groups) { return groups <= kScaleGroups / 2 ? 2 : 1; }
+constexpr int kScaleBufs = 4;
 // kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
 constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
@@ -128,6 +140,20 @@ template <int MODE>
 __device__ inline int row_blocks(const TcArgs &a) {
     return MODE == kTcSwiglu ? (int)((a.N / 2 + kRows / 2 - 1) / (kRows / 2)) : (int)((a.N + kRows - 1) / kRows);
 }
+// Scales and mins of N groups of a row as the item warp leaves them in shared memory: a word a group, the min above.
+template <int N>
+struct ScaleWords {
+    uint32_t w[N];
+    __device__ inline float scale(int g) const { return __uint_as_float(value(g) << 16); }
+    __device__ inline float min(int g) const { return __uint_as_float(value(g) & 0xffff0000u); }
+    __device__ inline uint32_t value(int g) const {
+        uint32_t v = w[0];
+#pragma unroll
+        for (int i = 1; i < N; ++i) v = g == i ? w[i] : v;
+        return v;
+    }
+};
+
 // Scales and mins (BF16 bits) of N consecutive groups of a row.
 template <int N>
 struct Scales {
@@ -165,8 +191,8 @@ __device__ __noinline__ Scales<N> load_scales_each(const uint16_t *sp, const uin
 // A producer lane's step of a quadrant at natural magnitude (kScaleSpread): its row's codes, 16-byte chunk c at `src` ^ 16 c of shared
 // memory, with its groups sc -> tensor memory.  Rare, so it is short rather than fast: a quarter at a time,
 // read again from shared memory (as a call, or unrolled, it cost the common step registers: 2000 x 8192 x 4096 Q8 133 us, not 129).
-template <int BITS, int G, int N>
-__device__ __forceinline__ void natural_step(uint32_t src, uint32_t a_addr, const Scales<N> &sc) {
+template <int BITS, int G, typename SCALES>
+__device__ __forceinline__ void natural_step(uint32_t src, uint32_t a_addr, const SCALES &sc) {
     constexpr int kChunkCodes = BITS == 4 ? 32 : 16, kChunks = 32 / kChunkCodes;
 #pragma unroll 1
     for (int hc = 0; hc < 4; ++hc) {
@@ -188,10 +214,10 @@ __device__ __forceinline__ void natural_step(uint32_t src, uint32_t a_addr, cons
     __syncwarp();
 }
 
-template <int BITS, int G, int MODE>
-__global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
+template <int BITS, int G, int MODE, bool SS>
+__global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 1)
     tiled_tc_kernel(const TcArgs a, const __grid_constant__ CUtensorMap wmap) {
-    using S = Shape<BITS, MODE == kTcHcUp>;
+    using S = Shape<BITS, MODE == kTcHcUp, SS>;
     constexpr int kStages = S::kStages, kWSlots = S::kWSlots, kSlotBytes = S::kSlotBytes, kWays = S::kWays, kEpiSets = S::kEpiSets,
                   kEpiWarps = S::kEpiWarps, kMmaWarp = S::kMmaWarp, kBCopyWarp = S::kBCopyWarp, kWCopyWarp = S::kWCopyWarp,
                   kItemWarp = S::kItemWarp, kFirstAWarp = S::kFirstAWarp;
@@ -199,7 +225,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     unsigned char *const smem = smem_raw;  // 1024-byte aligned, as the operand tiles want it (the swizzle pattern repeats every 1024 bytes)
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[kAccs], acc_empty[kAccs], drain_bar;
     __shared__ uint64_t w_full[kWSlots], w_empty[kWSlots];
-    __shared__ uint64_t item_full[kItemRing], item_empty[kItemRing];
+    __shared__ uint64_t item_full[kItemRing], item_empty[kItemRing], scales_empty[kScaleBufs];
     __shared__ __align__(16) Item item_ring[kItemRing];
     __shared__ uint8_t row_scale[kItemRing][kRows];
     __shared__ __align__(16) uint32_t out_row[kItemRing][kTile];  // where a token's output row starts, in 16-byte units
@@ -207,7 +233,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     __shared__ int abort_flag;
 
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int n_steps = (int)a.K / kBK, groups = (int)a.K / G;
+    const int n_steps = (int)a.K / kBK, groups = (int)a.K / G, sb_log = scale_bufs_log(groups), sb_mask = (1 << sb_log) - 1;
     const int rbs = row_blocks<MODE>(a);
     const int n_items = (a.dense_M > 0 ? (int)((a.dense_M + a.dense_tile - 1) / a.dense_tile) : a.ws[3]) * rbs;
     // slot (row of the output / of h) at position pos of the slot order; a dense projection's rows are in their own order
@@ -220,6 +246,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         mbar_init(&drain_bar, 1);
         for (int s = 0; s < kWSlots; ++s) mbar_init(&w_full[s], 1), mbar_init(&w_empty[s], 4);
         for (int s = 0; s < kItemRing; ++s) mbar_init(&item_full[s], 1), mbar_init(&item_empty[s], S::kItemReaders);
+        for (int s = 0; s < kScaleBufs; ++s) mbar_init(&scales_empty[s], 4 * kWays);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -242,7 +269,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
     if (!run && threadIdx.x == 0) raise_abort(0, 0);
     __syncthreads();
 
-    const uint32_t b_base = smem_u32(smem), w_base = b_base + (uint32_t)(kStages * kStageBytes);
+    const uint32_t b_base = smem_u32(smem), w_base = b_base + (uint32_t)(kStages * kStageBytes), s_base = w_base + (uint32_t)(kWSlots * kSlotBytes);
     uint32_t issued = 0;  // ring slots issued by this thread (the ring's thread only)
 
     // Item number i of this CTA, from the item ring.  read_item: a whole warp; read_item_one: a single thread.
@@ -302,7 +329,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         const uint32_t a_addr = ((uint32_t)(a_quad * 32) << 16) + (uint32_t)(kAccs * kTile + set * kAStageCols);
         const uint32_t signals = lane == 0 ? 1u : 0u;
 
-        // Scales and mins of a step's groups, fetched one step of the set ahead of use (fetched eight groups at a time, of which a set used a
+        // Not SS: scales and mins of a step's groups, fetched one step of the set ahead of use (fetched eight groups at a time, of which a set used a
         // quarter or half, and picked out by selects, they were 5 % of the Q8 forms).  A row past the end of the expert gets zeros: its
         // operand row is then zero whatever codes its lane reads.
         auto load_scales = [&](const uint16_t *sp, const uint16_t *mp) {
@@ -324,88 +351,116 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         Turn<kWSlots> slot{set, 0u};
         int st = set;  // the set's next step, relative to the item at hand
         bool live = true;
-        float nxt_scale = 1.f;
-        Item nxt = read_item(0, p0, nxt_scale);
-        int row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
-        Scales<kGroups> sc_nxt = scales_at(st < n_steps ? row : -1, st);  // of the set's next step
-        for (int i = 0; nxt.bucket >= 0 && live; ++i) {
-            const Item it = nxt;
-            const float scale = nxt_scale, scale_min = scale * 0x1p-24f;
-            nxt = read_item(i + 1, p0, nxt_scale);
-            const int nxt_row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
-            if (it.bucket >= a.E) {
-                row = nxt_row, sc_nxt = scales_at(st < n_steps ? row : -1, st);
-                continue;
+        // The step whose codes come into slot.at next, of item number i: sc its groups, scale and scale_min the row's power of two.
+        auto fill_stage = [&](const auto &sc, float scale, float scale_min, bool natural, int i) {
+            bool ok = wait(&w_full[slot.at], slot.phase, i, 7);
+            const uint32_t src = my_w + slot.at * (uint32_t)kSlotBytes;
+            uint4 code[kCodeRegs];
+#pragma unroll
+            for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(src ^ ((uint32_t)c << 4));
+            __half2 s2[kGroups], s16[kGroups], m2[kGroups];
+#pragma unroll
+            for (int gi = 0; gi < kGroups; ++gi) {
+                s2[gi] = __float2half2_rn(sc.scale(gi) * scale), m2[gi] = __float2half2_rn(sc.min(gi) * scale_min);
+                s16[gi] = __hmul2(s2[gi], __float2half2_rn(0.0625f));
             }
-            const bool natural = __any_sync(0xffffffffu, scale < 0.f);  // the quadrant's rows share it
-            // The set's first step of the next item, if it has one there: its scales are asked for at this item's start, but for four groups (registers)
-            // and for gate/up of Q8, which HBM bounds: 512 experts x 4096 x 2048, 256 tokens 929 us so and 889 at the end, 500 940 and 899.
-            constexpr bool kEarly = kGroups < 4 && !(BITS == 8 && MODE == kTcSwiglu);
-            const int after = st + (max(n_steps - st, 0) + kWays - 1) / kWays * kWays - n_steps;
-            Scales<kGroups> sc_item{};
-            if (kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
-            const uint16_t *sp = a.scale + (int64_t)max(row, 0) * groups + (st + kWays) * kGroups, *mp = a.minv + (sp - a.scale);
-            for (; st < n_steps; st += kWays, slot.advance(kWays), sp += kWays * kGroups, mp += kWays * kGroups) {
-                const Scales<kGroups> sc = sc_nxt;
-                if (row >= 0 && st + kWays < n_steps) sc_nxt = load_scales(sp, mp);
-                bool ok = wait(&w_full[slot.at], slot.phase, i, 7);
-                const uint32_t src = my_w + slot.at * (uint32_t)kSlotBytes;
-                uint4 code[kCodeRegs];
+            // 32 codes of the row -> 32 F16 = 16 tensor-memory columns of this lane
+            auto quarter = [&](int hc, uint4 (&d)[4]) {
 #pragma unroll
-                for (int c = 0; c < kCodeRegs; ++c) code[c] = ld_shared_v4(src ^ ((uint32_t)c << 4));
-                __half2 s2[kGroups], s16[kGroups], m2[kGroups];
-#pragma unroll
-                for (int gi = 0; gi < kGroups; ++gi) {
-                    s2[gi] = __float2half2_rn(sc.scale(gi) * scale), m2[gi] = __float2half2_rn(sc.min(gi) * scale_min);
-                    s16[gi] = __hmul2(s2[gi], __float2half2_rn(0.0625f));
+                for (int cc = 0; cc < 4; ++cc) {
+                    const int gi = ((hc * 4 + cc) * 8) / G;
+                    const uint4 v = code[(hc * 4 + cc) / kWordsPerChunk];
+                    if (BITS == 4) d[cc] = dequant_q4_scaled(cc == 0 ? v.x : cc == 1 ? v.y : cc == 2 ? v.z : v.w, s2[gi], s16[gi], m2[gi]);
+                    else d[cc] = (cc & 1) ? dequant_q8_scaled(v.z, v.w, s2[gi], m2[gi]) : dequant_q8_scaled(v.x, v.y, s2[gi], m2[gi]);
                 }
-                // 32 codes of the row -> 32 F16 = 16 tensor-memory columns of this lane
-                auto quarter = [&](int hc, uint4 (&d)[4]) {
+            };
+            uint4 d[4];
+            quarter(0, d);
+            ok = wait(&empty_bar[set], free_phase, i, 1) && ok;
+            // reconverges the warp; a wait that gave up in any lane ends the warp's work
+            if (!__all_sync(0xffffffffu, ok)) {
+                live = false;
+                return;
+            }
+            tc_fence_after();  // the stores below come after the MMAs that freed the stage
+            if (!natural) {
+                mbar_arrive_if(signals, &w_empty[slot.at]);  // the codes are in registers: the slot may be refilled
+                tc_st16(a_addr, d);
 #pragma unroll
-                    for (int cc = 0; cc < 4; ++cc) {
-                        const int gi = ((hc * 4 + cc) * 8) / G;
-                        const uint4 v = code[(hc * 4 + cc) / kWordsPerChunk];
-                        if (BITS == 4) d[cc] = dequant_q4_scaled(cc == 0 ? v.x : cc == 1 ? v.y : cc == 2 ? v.z : v.w, s2[gi], s16[gi], m2[gi]);
-                        else d[cc] = (cc & 1) ? dequant_q8_scaled(v.z, v.w, s2[gi], m2[gi]) : dequant_q8_scaled(v.x, v.y, s2[gi], m2[gi]);
+                for (int hc = 1; hc < 4; ++hc) {
+                    quarter(hc, d);
+                    tc_st16(a_addr + hc * 16, d);
+                }
+            } else {
+                natural_step<BITS, G>(src, a_addr, sc);
+                mbar_arrive_if(signals, &w_empty[slot.at]);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
+            __syncwarp();
+            mbar_arrive_if(signals, &full_bar[set]);
+            free_phase ^= 1u;
+        };
+        if constexpr (SS) {
+            // A row's scales come from shared memory; rows past the end of the expert have some other row's: their sums are dropped.
+            for (int i = 0; live; ++i) {
+                float scale = 1.f;
+                const Item it = read_item(i, p0, scale);
+                if (it.bucket < 0) break;
+                if (it.bucket < a.E) {
+                    const float scale_min = scale * 0x1p-24f;
+                    const bool natural = __any_sync(0xffffffffu, scale < 0.f);  // the quadrant's rows share it
+                    uint32_t at = s_base + (uint32_t)(((i & sb_mask) * groups + st * kGroups) * kRows + p0) * 4u;
+                    for (; st < n_steps && live; st += kWays, slot.advance(kWays), at += kWays * kGroups * kRows * 4) {
+                        ScaleWords<kGroups> sc;
+#pragma unroll
+                        for (int g = 0; g < kGroups; ++g) sc.w[g] = ld_shared_u32(at + g * kRows * 4);
+                        fill_stage(sc, scale, scale_min, natural, i);
                     }
-                };
-                uint4 d[4];
-                quarter(0, d);
-                ok = wait(&empty_bar[set], free_phase, i, 1) && ok;
-                // reconverges the warp; a wait that gave up in any lane ends the warp's work
-                if (!__all_sync(0xffffffffu, ok)) {
-                    live = false;
-                    break;
+                    st -= n_steps;
                 }
-                tc_fence_after();  // the stores below come after the MMAs that freed the stage
-                if (!natural) {
-                    mbar_arrive_if(signals, &w_empty[slot.at]);  // the codes are in registers: the slot may be refilled
-                    tc_st16(a_addr, d);
-#pragma unroll
-                    for (int hc = 1; hc < 4; ++hc) {
-                        quarter(hc, d);
-                        tc_st16(a_addr + hc * 16, d);
-                    }
-                } else {
-                    natural_step<BITS, G>(src, a_addr, sc);
-                    mbar_arrive_if(signals, &w_empty[slot.at]);
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                tc_fence_before();  // orders the stores before the MMAs that read them across the barrier
                 __syncwarp();
-                mbar_arrive_if(signals, &full_bar[set]);
-                free_phase ^= 1u;
+                mbar_arrive_if(signals, &scales_empty[i & sb_mask]);
             }
-            if (!kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
-            st -= n_steps, row = nxt_row, sc_nxt = sc_item;
+        } else {
+            float nxt_scale = 1.f;
+            Item nxt = read_item(0, p0, nxt_scale);
+            int row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
+            Scales<kGroups> sc_nxt = scales_at(st < n_steps ? row : -1, st);  // of the set's next step
+            for (int i = 0; nxt.bucket >= 0 && live; ++i) {
+                const Item it = nxt;
+                const float scale = nxt_scale, scale_min = scale * 0x1p-24f;
+                nxt = read_item(i + 1, p0, nxt_scale);
+                const int nxt_row = nxt.bucket >= 0 && nxt.bucket < a.E ? (int)row_of(nxt, p0) : -1;
+                if (it.bucket >= a.E) {
+                    row = nxt_row, sc_nxt = scales_at(st < n_steps ? row : -1, st);
+                    continue;
+                }
+                const bool natural = __any_sync(0xffffffffu, scale < 0.f);  // the quadrant's rows share it
+                // The set's first step of the next item, if it has one there: its scales are asked for at this item's start, but for four groups (registers)
+                // and for gate/up of Q8, which HBM bounds: 512 experts x 4096 x 2048, 256 tokens 929 us so and 889 at the end, 500 940 and 899.
+                constexpr bool kEarly = kGroups < 4 && !(BITS == 8 && MODE == kTcSwiglu);
+                const int after = st + (max(n_steps - st, 0) + kWays - 1) / kWays * kWays - n_steps;
+                Scales<kGroups> sc_item{};
+                if (kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
+                const uint16_t *sp = a.scale + (int64_t)max(row, 0) * groups + (st + kWays) * kGroups, *mp = a.minv + (sp - a.scale);
+                for (; st < n_steps; st += kWays, slot.advance(kWays), sp += kWays * kGroups, mp += kWays * kGroups) {
+                    const Scales<kGroups> sc = sc_nxt;
+                    if (row >= 0 && st + kWays < n_steps) sc_nxt = load_scales(sp, mp);
+                    fill_stage(sc, scale, scale_min, natural, i);
+                    if (!live) break;
+                }
+                if (!kEarly) sc_item = scales_at(after < n_steps ? nxt_row : -1, after);
+                st -= n_steps, row = nxt_row, sc_nxt = sc_item;
+            }
         }
     } else if (warp == kItemWarp) {
         // ===================== the item ring =====================
         // One warp looks the CTA's items up ahead of everyone else: the other roles read an item's description from shared
         // memory instead of each walking two dependent loads of the grouping workspace per item.  It also finds each
         // row's power of two (dequant_q4_scaled) from the row's scales and mins, four rows a lane, and whether one suits the rows of
-        // a tensor-memory quadrant at all (kScaleSpread); those lines are then in L2 when the producers want them.  Where
-        // contractions are short this is the longest chain of an item: its instructions count.
+        // a tensor-memory quadrant at all (kScaleSpread); the scales go to shared memory on the way (SS), or are in L2 when the producers want
+        // them.  Where contractions are short this is the longest chain of an item: its instructions count.
         const bool vec_scales = groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0;
         const bool pair_scales = groups % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 3) == 0;
         // What it needs to know of an item takes two loads, the second from where the first says: the first one for the next item is under way while
@@ -424,8 +479,33 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
         };
         const int64_t row_bytes = MODE == kTcSwiglu ? a.N : a.N * (MODE == kTcPartial ? 4 : 2);  // of the output
         const bool rows_wanted = MODE != kTcHcUp && !(MODE == kTcSwiglu && a.out_f16 >= 3);  // the tile-blocked h follows from the positions
+        // Waits until the producers are done with the item that had item i's place for scales.  Once an item, whether it needs the place or not: only then is
+        // watching the parity enough.
+        auto scales_free = [&](int i) {
+            const bool ok = i <= sb_mask || mbar_wait(&scales_empty[i & sb_mask], ((uint32_t)(i >> sb_log) & 1u) ^ 1u, abort_v, a.wait_limit_ns);
+            if (__all_sync(0xffffffffu, ok)) return true;
+            if (lane == 0) raise_abort(blockIdx.x + i * gridDim.x, 9);
+            return false;
+        };
+        int64_t at[4];  // of an item's rows r * 32 + lane: where their scales start; lanes past the expert's end look at a row that exists
+        uint4 sv[4], mv[4];
+        auto find_rows = [&](const Item &x) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int64_t wrow = row_of(x, r * 32 + lane);
+                at[r] = (wrow < 0 ? row_of(x, 0) : wrow) * groups;
+            }
+        };
+        auto ask = [&](int g) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                sv[r] = __ldg(reinterpret_cast<const uint4 *>(a.scale + at[r] + g));
+                mv[r] = __ldg(reinterpret_cast<const uint4 *>(a.minv + at[r] + g));
+            }
+        };
         Item nxt = no_item;
         if ((int)blockIdx.x < n_items) look_up(nxt), nxt.cnt = count_of(nxt);
+        if (SS && nxt.bucket >= 0 && nxt.bucket < a.E) find_rows(nxt), ask(0);
         for (int i = 0;; ++i) {
             const Item it = nxt;
             const int item = blockIdx.x + i * gridDim.x;
@@ -445,21 +525,28 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
                 top[r] = __vmaxu2(top[r], v), low[r] = __viaddmin_s16x2(v, 0x7bff7bffu, low[r]);
             };
             if (it.bucket >= 0 && it.bucket < a.E) {
-                int64_t at[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int64_t wrow = row_of(it, r * 32 + lane);
-                    at[r] = (wrow < 0 ? row_of(it, 0) : wrow) * groups;  // lanes past the expert's end look at a row that exists
-                }
-                if (vec_scales) {
+                if (!SS) find_rows(it);
+                if (SS) {
+                    if (!scales_free(i)) break;
+                    uint32_t to = s_base + (uint32_t)((i & sb_mask) * groups * kRows + lane) * 4u;
 #pragma unroll 1
-                    for (int g = 0; g < groups; g += 8) {
-                        uint4 sv[4], mv[4];
+                    for (int g = 0;; to += 8 * kRows * 4) {
 #pragma unroll
                         for (int r = 0; r < 4; ++r) {
-                            sv[r] = __ldg(reinterpret_cast<const uint4 *>(a.scale + at[r] + g));
-                            mv[r] = __ldg(reinterpret_cast<const uint4 *>(a.minv + at[r] + g));
+                            auto two = [&](int k, uint32_t s, uint32_t m) {
+                                take(r, s, m);
+                                st_shared_u32(to + (2 * k * kRows + r * 32) * 4, __byte_perm(s, m, 0x5410));
+                                st_shared_u32(to + ((2 * k + 1) * kRows + r * 32) * 4, __byte_perm(s, m, 0x7632));
+                            };
+                            two(0, sv[r].x, mv[r].x), two(1, sv[r].y, mv[r].y), two(2, sv[r].z, mv[r].z), two(3, sv[r].w, mv[r].w);
                         }
+                        if ((g += 8) >= groups) break;
+                        ask(g);
+                    }
+                } else if (vec_scales) {
+#pragma unroll 2
+                    for (int g = 0; g < groups; g += 8) {
+                        ask(g);
 #pragma unroll
                         for (int r = 0; r < 4; ++r)
                             take(r, sv[r].x, mv[r].x), take(r, sv[r].y, mv[r].y), take(r, sv[r].z, mv[r].z), take(r, sv[r].w, mv[r].w);
@@ -476,8 +563,11 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp>::kThreads), 1)
 #pragma unroll
                         for (int r = 0; r < 4; ++r) take(r, __ldg(a.scale + at[r] + g), __ldg(a.minv + at[r] + g));
                 }
+            } else if (SS && it.bucket >= 0) {
+                if (!scales_free(i)) break;
             }
             if (more) nxt.cnt = count_of(nxt);
+            if (SS && nxt.bucket >= 0 && nxt.bucket < a.E) find_rows(nxt), ask(0);  // from HBM, under what is left to do here
             if (i >= kItemRing) {
                 const bool ok = mbar_wait(&item_empty[i % kItemRing], ((uint32_t)(i / kItemRing) & 1u) ^ 1u, abort_v, a.wait_limit_ns);
                 if (!__all_sync(0xffffffffu, ok)) {
@@ -889,7 +979,6 @@ int dense_tile_rows(int64_t M, int64_t row_blocks, int64_t steps, int bits, int 
 template <int BITS, int MODE>
 int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     SXB_CHECK(a.x_kind == 3, fn, ": the tiled tcgen05 kernel takes tile-blocked activations only");
-    using S = Shape<BITS, MODE == kTcHcUp>;
     a.dense_tile = kTile;
     if (a.dense_M > 0 && MODE != kTcHcUp)
         a.dense_tile = dense_tile_rows(a.dense_M, MODE == kTcSwiglu ? (a.N / 2 + kRows / 2 - 1) / (kRows / 2) : (a.N + kRows - 1) / kRows, a.K / kBK, BITS, sm_count());
@@ -898,17 +987,34 @@ int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
     if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)(a.E * a.N), row_bytes, (uint32_t)(kBK * BITS / 8),
                                (uint32_t)(kRows / 2), BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
         return rc;
-    const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes +
-                        (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
-    auto go = [&](auto kern) -> int {
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), fn, ": reserving shared memory");
+    auto go = [&](auto kern, auto shape, int64_t scale_bytes) -> int {
+        using S = decltype(shape);
+        const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + (size_t)scale_bytes +
+                            (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
+        constexpr size_t most = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
+        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most + (scale_bytes > 0 ? 2 * kScaleGroups * kRows * 4 : 0))), fn,
+                 ": reserving shared memory");
         kern<<<(unsigned)sm_count(), S::kThreads, smem, st>>>(a, wmap);
         return SXB_OK;
     };
+    if constexpr (MODE != kTcHcUp) {
+        // The scales of two items fit beside the rings up to 32 groups a row, of four up to 16; the item warp reads them by eights.
+        const int64_t groups = a.K / G;
+        if (groups <= kScaleGroups && groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0) {
+            const int64_t bytes = ((int64_t)groups << scale_bufs_log((int)groups)) * kRows * 4;
+            using S = Shape<BITS, false, true>;
+            switch (G) {
+                case 32: return go(tiled_tc_kernel<BITS, 32, MODE, true>, S{}, bytes);
+                case 64: return go(tiled_tc_kernel<BITS, 64, MODE, true>, S{}, bytes);
+                default: return go(tiled_tc_kernel<BITS, 128, MODE, true>, S{}, bytes);
+            }
+        }
+    }
+    using S = Shape<BITS, MODE == kTcHcUp, false>;
     switch (G) {
-        case 32: return go(tiled_tc_kernel<BITS, 32, MODE>);
-        case 64: return go(tiled_tc_kernel<BITS, 64, MODE>);
-        default: return go(tiled_tc_kernel<BITS, 128, MODE>);
+        case 32: return go(tiled_tc_kernel<BITS, 32, MODE, false>, S{}, 0);
+        case 64: return go(tiled_tc_kernel<BITS, 64, MODE, false>, S{}, 0);
+        default: return go(tiled_tc_kernel<BITS, 128, MODE, false>, S{}, 0);
     }
 }
 

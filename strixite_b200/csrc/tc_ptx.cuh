@@ -294,4 +294,11 @@ __device__ inline uint4 ld_shared_v4(uint32_t addr) {
     return v;
 }
 
+__device__ inline uint32_t ld_shared_u32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ inline void st_shared_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
 }  // namespace sxb

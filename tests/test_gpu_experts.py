@@ -633,12 +633,15 @@ def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
     assert not bad and lib.sxb_release_scratch() == 0
 
 
-@pytest.mark.parametrize("bits,G", [(4, 128), (8, 32)])
-@pytest.mark.parametrize("N,Kd", [(16, 128), (48, 384), (144, 256), (272, 128)])
-def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd):
+# (N, K, groups a row): no whole eight of groups; 8, 16, 24 and 32, the last that lie in shared memory; 40; and arrays that do not start on 16 bytes.
+# 8192 rows: several items a CTA, so that the places of scales and items come round.
+@pytest.mark.parametrize("bits,G,N,Kd,shift", [
+    (4, 128, 16, 128, 0), (8, 32, 48, 384, 0), (4, 128, 144, 1152, 0), (8, 32, 272, 128, 0), (4, 128, 8192, 1024, 0), (8, 64, 4096, 1024, 0), (8, 32, 144, 256, 0),
+    (4, 32, 48, 768, 0), (4, 128, 1040, 3072, 0), (8, 64, 1040, 2048, 0), (4, 128, 144, 4096, 0), (4, 128, 144, 5120, 0), (4, 128, 1040, 1024, 1), (8, 64, 272, 512, 3)])
+def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd, shift):
     """Tiles of one token, around eight, sixteen and thirty-two and around a full tile, one and several steps of the contraction, rows that end inside
-    a row block, slots without an expert: every output form of the kernel for tile-blocked activations, bit for bit the general kernel's (which a captured
-    call runs on): the same operands, summed in the same order."""
+    a row block, slots without an expert, scales from shared memory and by the producers: every output form of the kernel for tile-blocked activations, bit for
+    bit the general kernel's (which a captured call runs on): the same operands, summed in the same order."""
     from strixite_b200 import kernels as K
     counts = [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 128, 129]
     E, g = len(counts), torch.Generator(device="cuda").manual_seed(N + bits)
@@ -646,6 +649,9 @@ def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd):
     M = ids.numel()
     ids = ids[torch.randperm(M, generator=torch.Generator().manual_seed(N))].to(cuda)[:, None].contiguous()
     w = K.quantize(torch.randn((E * N, Kd), generator=g, device=cuda) * 0.05, G, bits)
+    if shift:
+        scale, minv = (torch.cat([torch.zeros(shift, dtype=torch.int16, device=cuda), t.reshape(-1)])[shift:].view(t.shape) for t in (w.scale, w.minv))
+        w = K.QDeviceView(w.q, scale, minv, w.N, w.K, w.G, w.bits)
     x = torch.randn((M, Kd), generator=g, device=cuda).to(torch.bfloat16)
     coef, err = torch.rand((M, 1), generator=g, device=cuda), torch.zeros(4, dtype=torch.int32, device=cuda)
     nbytes = K.moe_route_workspace_bytes(M, 1, E)
