@@ -800,8 +800,8 @@ int library_status_words(const char *fn, uint32_t **out) {
 // A 2-D tiled tensor map over row-major data [outer, inner] of `elem_bytes`-byte elements.  The encoder is a host-side
 // computation of the driver library, found through the runtime (nothing links libcuda).  Out-of-range parts of a box read
 // as zero.
-int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, int elem_bytes, uint64_t inner, uint64_t outer,
-                  uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
+static int encode_map(const char *fn, CUtensorMap *map, CUtensorMapDataType dtype, const void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                      const cuuint32_t *box, CUtensorMapSwizzle swizzle) {
     using TensorMapEncode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                          const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -814,13 +814,24 @@ int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, i
         return reinterpret_cast<TensorMapEncode>(p);
     }();
     SXB_CHECK(encode != nullptr, fn, ": the driver offers no cuTensorMapEncodeTiled");
+    const cuuint32_t elem[3] = {1u, 1u, 1u};
+    const CUresult rc = encode(map, dtype, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    SXB_CHECK(rc == CUDA_SUCCESS, fn, ": tensor map over ", dims[1], " rows of ", strides[0], " bytes refused (CUresult ", (int)rc, ")");
+    return SXB_OK;
+}
+int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, int elem_bytes, uint64_t inner, uint64_t outer,
+                  uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
     (void)elem_bytes;
     const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer}, strides[1] = {(cuuint64_t)row_stride_bytes};
-    const cuuint32_t box[2] = {box_inner, box_outer}, elem[2] = {1u, 1u};
-    const CUresult rc = encode(map, dtype, 2, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    SXB_CHECK(rc == CUDA_SUCCESS, fn, ": tensor map over ", outer, " rows of ", row_stride_bytes, " bytes refused (CUresult ", (int)rc, ")");
-    return SXB_OK;
+    const cuuint32_t box[2] = {box_inner, box_outer};
+    return encode_map(fn, map, dtype, base, 2, dims, strides, box, swizzle);
+}
+int tensor_map_3d_bytes(const char *fn, const void *base, uint64_t inner, uint64_t mid, uint64_t outer, uint64_t mid_stride, uint64_t outer_stride,
+                        uint32_t box_inner, uint32_t box_mid, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
+    const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)mid, (cuuint64_t)outer}, strides[2] = {(cuuint64_t)mid_stride, (cuuint64_t)outer_stride};
+    const cuuint32_t box[3] = {box_inner, box_mid, box_outer};
+    return encode_map(fn, map, CU_TENSOR_MAP_DATA_TYPE_UINT8, base, 3, dims, strides, box, swizzle);
 }
 
 template <int BITS>

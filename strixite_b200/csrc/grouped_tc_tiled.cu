@@ -48,7 +48,7 @@
 //
 // Operands as in grouped_tc.cu: A (weights) dequantized in registers and stored to tensor memory by the producer warps
 // (the [tmem] form of tcgen05.mma), B (activations) two cp.async.bulk per step (one per 64-k sub-tile) into
-// 128-byte-swizzled K-major tiles, packed codes by 2-D tensor copies (128 codes x 64 rows a box, two boxes a ring slot).
+// 128-byte-swizzled K-major tiles, packed codes by tensor copies (128 codes x 128 rows a box and ring slot).
 //
 // One persistent CTA per SM.  Warps: the epilogue first (one per lane quadrant; two in the hyper-connection up mix, whose
 // epilogue carries the arithmetic of the stream combine - see TcHcUp), then MMA issue, activation copies, the ring of weight
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
     __syncthreads();
 
     const uint32_t b_base = smem_u32(smem), w_base = b_base + (uint32_t)(kStages * kStageBytes), s_base = w_base + (uint32_t)(kWSlots * kSlotBytes);
-    uint32_t issued = 0;  // ring slots issued by this thread (the ring's thread only)
+    uint32_t issued = 0;  // ring slots issued by this thread (the ring's only)
 
     // Item number i of this CTA, from the item ring.  read_item: a whole warp; read_item_one: a single thread.
     const Item no_item{-1, 0, 0, 0};
@@ -592,38 +592,71 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
         }
     } else if (warp == kWCopyWarp) {
         // ===================== the ring of weight codes =====================
-        // One thread keeps the ring as far ahead as free slots allow: per slot two boxes of 64 rows (the SwiGLU form: the
-        // gate rows and, I rows further, their up rows; otherwise 128 consecutive rows).
-        if (elect_one()) {
-            bool ok = true;
+        // The ring is kept as far ahead as free slots allow, a box of codes a slot: 128 consecutive rows (the SwiGLU form: 64 gate rows and
+        // their 64 up rows).  Q4, whose steps are short: a whole warp's loop with one lane's copies, as the MMA warp's, and the next slot asked for under
+        // this one's copy.  One thread's loop took 400 of a step's 540 cycles; us under load, that -> this: gate/up 548 -> 532 at 777 tokens, 468 -> 450
+        // at 300, down with its combine 325 -> 320 and 265 -> 259.  Q8's step has twice the time, and its down went 442 -> 448: one thread.
+        // test hook: CTA 0 leaves one slot unfilled (neither the byte count nor the copy), so that its consumers' wait runs out at the launch's
+        // limit and the abort path is exercised without anything faulting
+        if constexpr (BITS == 4) {
+            const uint32_t leader = elect_one() ? 1u : 0u;
             Turn<kWSlots> turn{0, 0u};
+            bool ok = true, ready = false;
             for (int i = 0; ok; ++i) {
-                const Item it = read_item_one(i);
-                if (it.bucket < 0) break;
-                if (it.bucket >= a.E) continue;
-                int y0, y1;
-                if (MODE == kTcSwiglu) y0 = (int)(it.bucket * a.N + it.rb * (kRows / 2)), y1 = y0 + (int)(a.N / 2);
-                else y0 = (int)(it.bucket * a.N + (int64_t)it.rb * kRows), y1 = y0 + kRows / 2;
+                float unused;
+                const Item it = read_item(i, lane, unused);
+                if (__any_sync(0xffffffffu, it.bucket < 0)) break;
+                if (__any_sync(0xffffffffu, it.bucket >= a.E)) continue;
+                const int y = (int)__reduce_max_sync(0xffffffffu, (uint32_t)(MODE == kTcSwiglu ? it.rb * (kRows / 2) : (int)(it.bucket * a.N + (int64_t)it.rb * kRows)));
+                const int z = MODE == kTcSwiglu ? (int)__reduce_max_sync(0xffffffffu, (uint32_t)(2 * it.bucket)) : 0;
                 for (int step = 0; step < n_steps; ++step) {
-                    const int slot = turn.at;
-                    if (!mbar_wait(&w_empty[slot], turn.phase ^ 1u, abort_v, a.wait_limit_ns)) {
-                        raise_abort(blockIdx.x + i * gridDim.x, 6);
-                        ok = false;
-                        break;
+                    if (!__all_sync(0xffffffffu, ready)) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&w_empty[turn.at], turn.phase ^ 1u, abort_v, a.wait_limit_ns));
+                        if (!ok) {
+                            if (leader) raise_abort(blockIdx.x + i * gridDim.x, 6);
+                            break;
+                        }
                     }
-                    const uint32_t dst = w_base + (uint32_t)(slot * kSlotBytes);
-                    // test hook: CTA 0 leaves one slot unfilled (neither the byte count nor the copies), so that its consumers'
-                    // wait runs out at the launch's limit and the abort path is exercised without anything faulting
+                    uint64_t *full = &w_full[turn.at];
+                    const uint32_t dst = w_base + (uint32_t)(turn.at * kSlotBytes);
+                    turn.advance(1);
+                    ready = mbar_test(&w_empty[turn.at], turn.phase ^ 1u);
                     if (!(blockIdx.x == 0 && (int)issued == a.test_skip_slot)) {
-                        mbar_expect_tx(&w_full[slot], (uint32_t)kSlotBytes);
-                        tma_load_2d(dst, &wmap, step * (kBK * BITS / 8), y0, &w_full[slot]);
-                        tma_load_2d(dst + kSlotBytes / 2, &wmap, step * (kBK * BITS / 8), y1, &w_full[slot]);
+                        mbar_expect_tx_if(leader, full, (uint32_t)kSlotBytes);
+                        if (MODE == kTcSwiglu) tma_load_3d_if(leader, dst, &wmap, step * (kBK * BITS / 8), y, z, full);
+                        else tma_load_2d_if(leader, dst, &wmap, step * (kBK * BITS / 8), y, full);
                     }
-                    ++issued, turn.advance(1);
+                    ++issued;
                 }
             }
+        } else {
+            if (elect_one()) {
+                bool ok = true;
+                Turn<kWSlots> turn{0, 0u};
+                for (int i = 0; ok; ++i) {
+                    const Item it = read_item_one(i);
+                    if (it.bucket < 0) break;
+                    if (it.bucket >= a.E) continue;
+                    const int y = MODE == kTcSwiglu ? it.rb * (kRows / 2) : (int)(it.bucket * a.N + (int64_t)it.rb * kRows);
+                    for (int step = 0; step < n_steps; ++step) {
+                        const int slot = turn.at;
+                        if (!mbar_wait(&w_empty[slot], turn.phase ^ 1u, abort_v, a.wait_limit_ns)) {
+                            raise_abort(blockIdx.x + i * gridDim.x, 6);
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t dst = w_base + (uint32_t)(slot * kSlotBytes);
+                        if (!(blockIdx.x == 0 && (int)issued == a.test_skip_slot)) {
+                            mbar_expect_tx(&w_full[slot], (uint32_t)kSlotBytes);
+                            if (MODE == kTcSwiglu) tma_load_3d(dst, &wmap, step * (kBK * BITS / 8), y, 2 * it.bucket, &w_full[slot]);
+                            else tma_load_2d(dst, &wmap, step * (kBK * BITS / 8), y, &w_full[slot]);
+                        }
+                        ++issued, turn.advance(1);
+                    }
+                }
+            }
+            __syncwarp();
         }
-        __syncwarp();
     } else if (warp == kBCopyWarp) {
         // ===================== activations =====================
         // One thread, two bulk copies per step: the tile of (item, 64 k) is one contiguous run of cnt * 128 bytes;
@@ -974,7 +1007,7 @@ int dense_tile_rows(int64_t M, int64_t row_blocks, int64_t steps, int bits, int 
     return best;
 }
 
-// Two boxes of 128 codes x 64 rows fill a ring slot; 16-byte chunks swizzled in the mode of the box's row length so that the
+// One box of 128 codes x 128 rows (the SwiGLU form: of 64 rows of two matrices) fills a ring slot; 16-byte chunks swizzled in the mode of the box's row length so that the
 // producers' 16-byte reads of consecutive rows hit every bank once.
 template <int BITS, int MODE>
 int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
@@ -984,8 +1017,11 @@ int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
         a.dense_tile = dense_tile_rows(a.dense_M, MODE == kTcSwiglu ? (a.N / 2 + kRows / 2 - 1) / (kRows / 2) : (a.N + kRows - 1) / kRows, a.K / kBK, BITS, sm_count());
     const uint64_t row_bytes = (uint64_t)(BITS == 4 ? a.K / 2 : a.K);
     CUtensorMap wmap;
-    if (int rc = tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, (uint64_t)(a.E * a.N), row_bytes, (uint32_t)(kBK * BITS / 8),
-                               (uint32_t)(kRows / 2), BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, &wmap))
+    constexpr uint32_t box = kBK * BITS / 8;
+    constexpr CUtensorMapSwizzle swizzle = BITS == 4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
+    const uint64_t rows = (uint64_t)(a.E * a.N), I = (uint64_t)a.N / 2;
+    if (int rc = MODE == kTcSwiglu ? tensor_map_3d_bytes(fn, a.q, row_bytes, I, rows / I, row_bytes, I * row_bytes, box, (uint32_t)(kRows / 2), 2u, swizzle, &wmap)
+                                   : tensor_map_2d(fn, a.q, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, row_bytes, rows, row_bytes, box, (uint32_t)kRows, swizzle, &wmap))
         return rc;
     auto go = [&](auto kern, auto shape, int64_t scale_bytes) -> int {
         using S = decltype(shape);

@@ -15,6 +15,9 @@ namespace sxb {
 // grouped_tc.cu (host): tiled 2-D tensor map; the library's own status words; the current bound of device-side waits.
 int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, int elem_bytes, uint64_t inner, uint64_t outer,
                   uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map);
+// ... a 3-D one over bytes: [outer][mid][inner], `mid_stride` and `outer_stride` bytes apart.
+int tensor_map_3d_bytes(const char *fn, const void *base, uint64_t inner, uint64_t mid, uint64_t outer, uint64_t mid_stride, uint64_t outer_stride,
+                        uint32_t box_inner, uint32_t box_mid, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map);
 int library_status_words(const char *fn, uint32_t **out);
 unsigned long long wait_limit_ns();
 // ... of the streaming expert kernel's, which wait for a whole unit of another warp as a matter of course: never below the default, whatever a
@@ -277,6 +280,33 @@ __device__ inline void st_global_if(bool pred, void *p, float v) {
 }
 __device__ inline void st_global_if(bool pred, void *p, uint16_t v) {
     asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q st.global.u16 [%0], %1;\n\t}" ::"l"(p), "h"(v), "r"((uint32_t)pred) : "memory");
+}
+__device__ inline void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+                 "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
+// The copies and the expected byte count for a loop that a whole warp runs under uniform control flow: `leader` is 1 in the one lane (of
+// elect_one) whose instructions count, so that addresses, coordinates and barriers stay in uniform registers.
+__device__ inline void mbar_expect_tx_if(uint32_t leader, uint64_t *bar, uint32_t bytes) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+        "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(leader)
+        : "memory");
+}
+__device__ inline void tma_load_2d_if(uint32_t leader, uint32_t dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)), "r"(leader)
+        : "memory");
+}
+__device__ inline void tma_load_3d_if(uint32_t leader, uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+        "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "r"(leader)
+        : "memory");
 }
 // 16 bytes global -> shared without passing through registers (both addresses 16-byte aligned); complete, for the
 // issuing thread, after cp_async_wait<N> has let at most N of its later groups remain in flight.
