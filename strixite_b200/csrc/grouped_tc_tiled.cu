@@ -87,6 +87,9 @@ struct Shape {
     static constexpr int kStages = kWays;
     static constexpr int kSlotBytes = kRows * kBK * BITS / 8;  // a ring slot: the packed codes of a step, 8 or 16 KB
     static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 8 ? 1 : SS ? 2 : 3);  // what shared memory holds beside the stages and the scales (Q4, 8 -> 12 slots: 583 -> 572 us at 777 tokens)
+    // Items that the ring holds.  The epilogue keeps an item's place until it is done with it.  Without SS three: 4096 x 8192 x 4096 Q8 under load 283 us with
+    // two, 261 with three, 263 with four, which lets the item warp's look at a later item's scales push those that the producers want out of L1.
+    static constexpr int kItemRing = SS ? 4 : 3;
     static constexpr int kEpiSets = HC ? 2 : 1;  // epilogue warps per lane quadrant
     static constexpr int kEpiWarps = 4 * kEpiSets, kMmaWarp = kEpiWarps, kBCopyWarp = kEpiWarps + 1, kWCopyWarp = kEpiWarps + 2,
                          kItemWarp = kEpiWarps + 3, kFirstAWarp = kEpiWarps + 4;
@@ -95,7 +98,6 @@ struct Shape {
     static_assert(kAccs * kTile + kStages * kAStageCols <= kTmemCols, "tensor memory");
     static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
-constexpr int kItemRing = 4;
 constexpr int kScaleGroups = 32;  // SS: groups of a row at most
 // ... items whose scales lie in shared memory, as a power of two
 __host__ __device__ constexpr int scale_bufs_log(int groups) { return groups <= kScaleGroups / 2 ? 2 : 1; }
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
     using S = Shape<BITS, MODE == kTcHcUp, SS>;
     constexpr int kStages = S::kStages, kWSlots = S::kWSlots, kSlotBytes = S::kSlotBytes, kWays = S::kWays, kEpiSets = S::kEpiSets,
                   kEpiWarps = S::kEpiWarps, kMmaWarp = S::kMmaWarp, kBCopyWarp = S::kBCopyWarp, kWCopyWarp = S::kWCopyWarp,
-                  kItemWarp = S::kItemWarp, kFirstAWarp = S::kFirstAWarp;
+                  kItemWarp = S::kItemWarp, kFirstAWarp = S::kFirstAWarp, kItemRing = S::kItemRing;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *const smem = smem_raw;  // 1024-byte aligned, as the operand tiles want it (the swizzle pattern repeats every 1024 bytes)
     __shared__ uint64_t full_bar[kStages], empty_bar[kStages], acc_full[kAccs], acc_empty[kAccs], drain_bar;
