@@ -17,6 +17,7 @@
 // stay the reference's (row-major folded down weight, chunk-major up weight), shared with the per-token kernels.
 
 #include "grouped_tc.cuh"
+#include "skinny_mma.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -483,6 +484,7 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
             tc_fence_after();
             // sigmoid(z) = 1 / (1 + 2^(-z log2 e)), with the row's power of two taken out of z on the way
             const float nz = -1.44269504f * row_scale[(int)(rb - i0 / tiles) % kUpScaleBufs][quad * 32 + lane];
+            const uint64_t nz2 = pair(nz, nz), nwp2 = pair(nwp, nwp), one2 = pair(1.0f, 1.0f);
             TX *up = static_cast<TX *>(a.u) + ((int64_t)tile * kUpTile + tok0 + mine) * a.d + j;
 #pragma unroll 1
             for (int p = 0; p < 2; ++p, up += 64 * a.d) {
@@ -501,15 +503,15 @@ __global__ void __launch_bounds__(kUpThreads, 1) hc_up_tc_kernel(const HcUpArgs 
                 // four butterflies, and it leaves each of the four lanes with the sum of one token, which that lane stores.
                 if (left > 0) {
 #pragma unroll
-                    for (int t = 0; t < 16; ++t) {
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            const int tt = t + 16 * hf;
-                            const float z = hf ? vb[t] : va[t];
-                            const float c = load_as_f32(xs_[tt & 1], p * 8192 + (tt >> 1) * 256) * ivs[p * 256 + tt * 4] * nwp * rcp_ftz(1.0f + exp2_ftz(z * nz));
-                            if (hf) vb[t] = c;
-                            else va[t] = c;
-                        }
+                    for (int t = 0; t < 32; t += 2) {  // two tokens' factors in one instruction, each rounded as on its own (4096 tokens 104.8 -> 101.3 us under load, 1024 36.9 -> 34.8, 77 18.2 -> 16.4)
+                        float (&v)[16] = t < 16 ? va : vb;
+                        const int q = t & 15;
+                        float e0, e1;
+                        unpair(mul_pair(pair(v[q], v[q + 1]), nz2), e0, e1);
+                        unpair(add_pair(one2, pair(exp2_ftz(e0), exp2_ftz(e1))), e0, e1);
+                        const uint64_t x2 = pair(load_as_f32(xs_[0], p * 8192 + (t >> 1) * 256), load_as_f32(xs_[1], p * 8192 + (t >> 1) * 256));
+                        const uint64_t c2 = mul_pair(mul_pair(x2, pair(ivs[p * 256 + t * 4], ivs[p * 256 + t * 4 + 4])), nwp2);
+                        unpair(mul_pair(c2, pair(rcp_ftz(e0), rcp_ftz(e1))), v[q], v[q + 1]);
                     }
                 }
                 if (p == 1) {
