@@ -481,6 +481,10 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
         };
         const int64_t row_bytes = MODE == kTcSwiglu ? a.N : a.N * (MODE == kTcPartial ? 4 : 2);  // of the output
         const bool rows_wanted = MODE != kTcHcUp && !(MODE == kTcSwiglu && a.out_f16 >= 3);  // the tile-blocked h follows from the positions
+        // SwiGLU without SS: its four registers of slots are asked for behind the scan of the scales.  Held across it they made ptxas spill (Q8, groups of 64: 108
+        // bytes a thread), and local memory then took the L1 lines that the producers find their scales in: gate/up of 512 experts, d = 4096, I = 1024, Q8,
+        // 300 tokens 1004-1062 us under load, 839-916 so (853-917 before slots were looked up here); 4096 x 8192 x 4096 Q8 + SwiGLU 274 -> 261 (257).
+        constexpr bool kSlotsLate = !SS && MODE == kTcSwiglu;
         // Waits until the producers are done with the item that had item i's place for scales.  Once an item, whether it needs the place or not: only then is
         // watching the parity enough.
         auto scales_free = [&](int i) {
@@ -515,10 +519,12 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
             nxt = no_item;
             if (more) look_up(nxt);
             int slot[4] = {0, 0, 0, 0};
-            if (rows_wanted && it.bucket >= 0) {
+            auto find_slots = [&] {
+                if (!rows_wanted || it.bucket < 0) return;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) slot[r] = r * 32 + lane < it.cnt ? slot_at(it.start + r * 32 + lane) : 0;
-            }
+            };
+            if (!kSlotsLate) find_slots();
             // Of every group v = max(|scale| * 2^8, |min|) as BF16 bits, 0x400 = an empty group; two 16-bit maxima of v, and signed
             // minima of v + 0x7bff, in which an empty group's is the largest.  Five instructions for two groups.
             uint32_t top[4] = {0u, 0u, 0u, 0u}, low[4] = {0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu};
@@ -568,6 +574,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
             } else if (SS && it.bucket >= 0) {
                 if (!scales_free(i)) break;
             }
+            if (kSlotsLate) find_slots();
             if (more) nxt.cnt = count_of(nxt);
             if (SS && nxt.bucket >= 0 && nxt.bucket < a.E) find_rows(nxt), ask(0);  // from HBM, under what is left to do here
             if (i >= kItemRing) {
