@@ -485,6 +485,12 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
         // bytes a thread), and local memory then took the L1 lines that the producers find their scales in: gate/up of 512 experts, d = 4096, I = 1024, Q8,
         // 300 tokens 1004-1062 us under load, 839-916 so (853-917 before slots were looked up here); 4096 x 8192 x 4096 Q8 + SwiGLU 274 -> 261 (257).
         constexpr bool kSlotsLate = !SS && MODE == kTcSwiglu;
+        // How far the scan by eights unrolls without SS.  The rows of down that come here have groups that are no multiple of eight, or more than 32: rarely the
+        // latter, and that scan's code stands between.  Groups of 32 would spill.  A few launches at a time, us, 2 -> 1: 128 experts' 2560 x 768 Q8, 300 tokens
+        // 72.4 -> 69.9, 64 experts' 3584 x 1280 Q8 79.5 -> 78.7, 2048 x 1408 Q4 44.9 -> 43.4; dense 4096 x 8192 x 4096 Q8 under load 272 -> 283.
+        // The scans by two and one stand in front of a launch's first step: 2 and 4 at a time against one dense 1500 x 2048 x 2816 Q4 24.7 -> 23.8,
+        // 64 x 4096 x 1408 Q8 12.4 -> 11.6, 300 x 4096 x 1920 Q4 13.6 -> 12.5.
+        constexpr int kUnrollEights = (MODE == kTcPartial || MODE == kTcPartialBf16) && G > 32 ? 1 : 2;
         // Waits until the producers are done with the item that had item i's place for scales.  Once an item, whether it needs the place or not: only then is
         // watching the parity enough.
         auto scales_free = [&](int i) {
@@ -552,7 +558,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
                         ask(g);
                     }
                 } else if (vec_scales) {
-#pragma unroll 2
+#pragma unroll kUnrollEights
                     for (int g = 0; g < groups; g += 8) {
                         ask(g);
 #pragma unroll
@@ -560,13 +566,13 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
                             take(r, sv[r].x, mv[r].x), take(r, sv[r].y, mv[r].y), take(r, sv[r].z, mv[r].z), take(r, sv[r].w, mv[r].w);
                     }
                 } else if (pair_scales) {
-#pragma unroll 1
+#pragma unroll 2
                     for (int g = 0; g < groups; g += 2)
 #pragma unroll
                         for (int r = 0; r < 4; ++r)
                             take(r, __ldg(reinterpret_cast<const uint32_t *>(a.scale + at[r] + g)), __ldg(reinterpret_cast<const uint32_t *>(a.minv + at[r] + g)));
                 } else {
-#pragma unroll 1
+#pragma unroll 4
                     for (int g = 0; g < groups; ++g)
 #pragma unroll
                         for (int r = 0; r < 4; ++r) take(r, __ldg(a.scale + at[r] + g), __ldg(a.minv + at[r] + g));
