@@ -485,12 +485,9 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
         // bytes a thread), and local memory then took the L1 lines that the producers find their scales in: gate/up of 512 experts, d = 4096, I = 1024, Q8,
         // 300 tokens 1004-1062 us under load, 839-916 so (853-917 before slots were looked up here); 4096 x 8192 x 4096 Q8 + SwiGLU 274 -> 261 (257).
         constexpr bool kSlotsLate = !SS && MODE == kTcSwiglu;
-        // How far the scan by eights unrolls without SS.  The rows of down that come here have groups that are no multiple of eight, or more than 32: rarely the
-        // latter, and that scan's code stands between.  Groups of 32 would spill.  A few launches at a time, us, 2 -> 1: 128 experts' 2560 x 768 Q8, 300 tokens
-        // 72.4 -> 69.9, 64 experts' 3584 x 1280 Q8 79.5 -> 78.7, 2048 x 1408 Q4 44.9 -> 43.4; dense 4096 x 8192 x 4096 Q8 under load 272 -> 283.
-        // The scans by two and one stand in front of a launch's first step: 2 and 4 at a time against one dense 1500 x 2048 x 2816 Q4 24.7 -> 23.8,
-        // 64 x 4096 x 1408 Q8 12.4 -> 11.6, 300 x 4096 x 1920 Q4 13.6 -> 12.5.
-        constexpr int kUnrollEights = (MODE == kTcPartial || MODE == kTcPartialBf16) && G > 32 ? 1 : 2;
+        // The scans without SS stand in front of a launch's first step and unroll by 64 registers of loads.  A few launches at a time, us, one at a time -> so:
+        // by twos dense 1500 x 2048 x 2816 Q4 24.7 -> 23.8, by ones 64 x 4096 x 1408 Q8 12.4 -> 11.6, 300 x 4096 x 1920 Q4 13.6 -> 12.5; by eights the down half of
+        // the hyper-connection mix, 77 tokens, d = 4096, rank 320, 32.8 -> 30.8, dense 4096 x 8192 x 4096 Q8 under load 283 -> 272.
         // Waits until the producers are done with the item that had item i's place for scales.  Once an item, whether it needs the place or not: only then is
         // watching the parity enough.
         auto scales_free = [&](int i) {
@@ -558,7 +555,7 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
                         ask(g);
                     }
                 } else if (vec_scales) {
-#pragma unroll kUnrollEights
+#pragma unroll 2
                     for (int g = 0; g < groups; g += 8) {
                         ask(g);
 #pragma unroll
