@@ -140,7 +140,7 @@ __device__ inline void tc_ld16lanes_x2(uint32_t taddr0, uint32_t taddr1, float (
         "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
         "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
         "tcgen05.wait::ld.sync.aligned;"
-        : "=f"(v0[0]), "=f"(v0[1]), "=f"(v0[2]), "=f"(v0[3]), "=f"(v0[4]), "=f"(v0[5]), "=f"(v0[6]), "=f"(v0[7]), "=f"(v1[0]), "=f"(v1[1]), "=f"(v1[2]),
+        : "=&f"(v0[0]), "=&f"(v0[1]), "=&f"(v0[2]), "=&f"(v0[3]), "=&f"(v0[4]), "=&f"(v0[5]), "=&f"(v0[6]), "=&f"(v0[7]), "=f"(v1[0]), "=f"(v1[1]), "=f"(v1[2]),
           "=f"(v1[3]), "=f"(v1[4]), "=f"(v1[5]), "=f"(v1[6]), "=f"(v1[7])
         : "r"(taddr0), "r"(taddr1)
         : "memory");
