@@ -76,6 +76,15 @@ constexpr int kAStageCols = kBK / 2; // 128 F16 of one weight row per lane
 constexpr int kAccs = 2;
 constexpr int kTmemCols = 512;
 
+constexpr int kScaleGroups = 32;  // SS: groups of a row at most
+// ... items whose scales lie in shared memory, as a power of two
+__host__ __device__ constexpr int scale_bufs_log(int groups) { return groups <= kScaleGroups / 2 ? 2 : 1; }
+constexpr int kScaleBufs = 4;
+// kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
+constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
+constexpr int kSharedBytes = 227 * 1024;  // of a CTA
+constexpr int kStaticBytes = 3 * 1024;    // barriers, item ring and the like at most: the dynamic part starts on the next 1024 bytes behind them
+
 // HC: the hyper-connection up mix (kTcHcUp), whose contraction is short and whose epilogue needs registers and shared memory:
 // half the producers, stages and ring slots.
 // SS: the scales of the items at hand lie in shared memory.
@@ -95,15 +104,14 @@ struct Shape {
                          kItemWarp = kEpiWarps + 3, kFirstAWarp = kEpiWarps + 4;
     static constexpr int kThreads = 32 * (kFirstAWarp + 4 * kWays);
     static constexpr int kItemReaders = kEpiWarps + 3 + 4 * kWays;  // warps that read every item from the item ring
+    // The dynamic part: stages, ring slots, scales of a launch's longest rows, the up mix's buffers.  With scales of 32 groups the CTA's shared memory is full to
+    // the byte, and one more static word past kStaticBytes would have every launch of those forms refused.
+    static constexpr int kBufferBytes = kStages * kStageBytes + kWSlots * kSlotBytes + (HC ? kEpiWarps * 2 * kHcUpBufBytes : 0);
+    static constexpr int kMostDynamic = kBufferBytes + (SS ? 2 * kScaleGroups * kRows * 4 : 0);
+    static_assert(kMostDynamic + kStaticBytes <= kSharedBytes, "shared memory");
     static_assert(kAccs * kTile + kStages * kAStageCols <= kTmemCols, "tensor memory");
     static_assert((kWays & (kWays - 1)) == 0 && kWSlots % kWays == 0, "sets");
 };
-constexpr int kScaleGroups = 32;  // SS: groups of a row at most
-// ... items whose scales lie in shared memory, as a power of two
-__host__ __device__ constexpr int scale_bufs_log(int groups) { return groups <= kScaleGroups / 2 ? 2 : 1; }
-constexpr int kScaleBufs = 4;
-// kTcHcUp: one buffer of an epilogue warp - a pass's 128 (token, stream) segments of X, 32 bytes each at most, then inv
-constexpr int kHcUpBufBytes = 128 * 32 + 32 * 16;
 
 // The power of two that undoes a row's scale 2^k on its accumulators, 2^(24 - k).  Rows at natural magnitude: scale = -2^24.  The item
 // ring holds a scale's biased exponent, 0 for kNatural.
@@ -1037,12 +1045,8 @@ int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
         return rc;
     auto go = [&](auto kern, auto shape, int64_t scale_bytes) -> int {
         using S = decltype(shape);
-        const size_t smem = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + (size_t)scale_bytes +
-                            (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
-        constexpr size_t most = (size_t)S::kStages * kStageBytes + (size_t)S::kWSlots * S::kSlotBytes + (MODE == kTcHcUp ? (size_t)S::kEpiWarps * 2 * kHcUpBufBytes : 0);
-        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most + (scale_bytes > 0 ? 2 * kScaleGroups * kRows * 4 : 0))), fn,
-                 ": reserving shared memory");
-        kern<<<(unsigned)sm_count(), S::kThreads, smem, st>>>(a, wmap);
+        SXB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kMostDynamic), fn, ": reserving shared memory");
+        kern<<<(unsigned)sm_count(), S::kThreads, (size_t)(S::kBufferBytes + scale_bytes), st>>>(a, wmap);
         return SXB_OK;
     };
     if constexpr (MODE != kTcHcUp) {
