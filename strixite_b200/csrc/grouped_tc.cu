@@ -797,9 +797,8 @@ int library_status_words(const char *fn, uint32_t **out) {
     return SXB_OK;
 }
 
-// A 2-D tiled tensor map over row-major data [outer, inner] of `elem_bytes`-byte elements.  The encoder is a host-side
-// computation of the driver library, found through the runtime (nothing links libcuda).  Out-of-range parts of a box read
-// as zero.
+// A tiled tensor map of two or three dimensions, innermost first.  The encoder is a host-side computation of the driver
+// library, found through the runtime (nothing links libcuda).  Out-of-range parts of a box read as zero.
 static int encode_map(const char *fn, CUtensorMap *map, CUtensorMapDataType dtype, const void *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
                       const cuuint32_t *box, CUtensorMapSwizzle swizzle) {
     using TensorMapEncode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -817,9 +816,11 @@ static int encode_map(const char *fn, CUtensorMap *map, CUtensorMapDataType dtyp
     const cuuint32_t elem[3] = {1u, 1u, 1u};
     const CUresult rc = encode(map, dtype, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    SXB_CHECK(rc == CUDA_SUCCESS || rank == 2, fn, ": tensor map over ", dims[2], " x ", dims[1], " rows of ", strides[0], " bytes refused (CUresult ", (int)rc, ")");
     SXB_CHECK(rc == CUDA_SUCCESS, fn, ": tensor map over ", dims[1], " rows of ", strides[0], " bytes refused (CUresult ", (int)rc, ")");
     return SXB_OK;
 }
+// Row-major data [outer, inner] of `elem_bytes`-byte elements.
 int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, int elem_bytes, uint64_t inner, uint64_t outer,
                   uint64_t row_stride_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
     (void)elem_bytes;
@@ -827,6 +828,7 @@ int tensor_map_2d(const char *fn, const void *base, CUtensorMapDataType dtype, i
     const cuuint32_t box[2] = {box_inner, box_outer};
     return encode_map(fn, map, dtype, base, 2, dims, strides, box, swizzle);
 }
+// Bytes [outer][mid][inner], `mid_stride` and `outer_stride` bytes apart.
 int tensor_map_3d_bytes(const char *fn, const void *base, uint64_t inner, uint64_t mid, uint64_t outer, uint64_t mid_stride, uint64_t outer_stride,
                         uint32_t box_inner, uint32_t box_mid, uint32_t box_outer, CUtensorMapSwizzle swizzle, CUtensorMap *map) {
     const cuuint64_t dims[3] = {(cuuint64_t)inner, (cuuint64_t)mid, (cuuint64_t)outer}, strides[2] = {(cuuint64_t)mid_stride, (cuuint64_t)outer_stride};
