@@ -1,6 +1,7 @@
 """The steps either side of the expert kernels, and the boundary's remaining forms, on the GPU against the CPU oracle:
 the router-logits projection (streaming and tcgen05), router + pack as one launch, the residual add, the dense tcgen05
 projections (linear_q*_wmma), FP32 activations, and a C++ host that issues the reference's call block through the shim."""
+import re
 import subprocess
 
 import numpy as np
@@ -622,6 +623,63 @@ def test_router_gemm_gives_up_a_wait(cuda, lib, M, N, K, planes, slot):
     Kn.router_logits_wmma(x, planes_, None, out[2])
     Kn.check_dense_status("after")
     assert torch.equal(out[2], out[0]) and not bool(torch.isnan(out[2]).any())
+
+
+# (slot, item that it belongs to): in the first turn of the ring of codes, behind a full turn, and in a later item, so that the item warp stands at a place for scales.
+# Eight groups (four places for scales), thirty-two (two), forty (the producers load scales themselves).
+@pytest.mark.parametrize("bits,N,K,slot", [(4, 32768, 1024, 3), (4, 32768, 1024, 11), (4, 32768, 1024, 45), (4, 32768, 4096, 5), (4, 32768, 4096, 130), (8, 32768, 512, 22),
+                                           (8, 32768, 2048, 60), (4, 32768, 5120, 13), (4, 32768, 5120, 130)])
+def test_a_wait_that_runs_out_in_a_later_item(cuda, lib, bits, N, K, slot):
+    """The kernel for tile-blocked activations with several items a CTA and CTA 0 told to leave one fill of its ring of codes out.  The kernel returns, the status names item and
+    role, the next call has the bits of the call before."""
+    from strixite_b200 import kernels as Kn
+    M, g = 512, torch.Generator(device="cuda").manual_seed(slot)
+    w = Kn.quantize(torch.randn((N, K), generator=g, device=cuda) * 0.05, 128 if bits == 4 else 64, bits)
+    x = torch.randn((M, K), generator=g, device=cuda).to(torch.bfloat16)
+    xs, out = torch.empty((M, K), dtype=torch.float16, device=cuda), [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=cuda) for _ in range(3)]
+    Kn.stage_f16_tiles(x, None, 0, M, 1, 1, K, bits, xs)
+    Kn.linear_qw_wmma(xs, w, out[0], M, Kn.Act.F16_TILED)
+    Kn.check_dense_status("warm-up")
+    try:
+        Kn.set_wait_limit(2_000_000)
+        assert lib.sxb_test_skip_ring_slot(slot) == 0
+        Kn.linear_qw_wmma(xs, w, out[1], M, Kn.Act.F16_TILED)
+        torch.cuda.synchronize()
+    finally:
+        lib.sxb_test_skip_ring_slot(-1)
+        Kn.set_wait_limit(2_000_000_000)
+    # items of CTA 0, of which any role's wait may run out first: the skipped step's, one before it and up to four ahead
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    item = sms * (slot // (K // 128))
+    with pytest.raises(Kn.Error, match=r"skipped fill: a tcgen05 kernel gave up a wait at work item \d+ \((a weight producer|an MMA warp|the epilogue|the activation copy|the weight-code copy|a warp waiting for the description|the work-item)") as e:
+        Kn.check_dense_status("skipped fill")
+    at = int(re.search(r"work item (\d+)", str(e.value)).group(1))
+    assert at in range(max(item - sms, 0), item + 5 * sms, sms), (at, item)
+    Kn.linear_qw_wmma(xs, w, out[2], M, Kn.Act.F16_TILED)
+    Kn.check_dense_status("after")
+    assert torch.equal(out[2].view(torch.int16), out[0].view(torch.int16)) and not bool(torch.isnan(out[2]).any())
+
+
+@pytest.mark.parametrize("bits,G,M,N,K", [(8, 64, 777, 4096, 1024), (4, 128, 300, 2048, 4096), (4, 32, 150, 4096, 1024), (8, 64, 200, 2560, 1536), (8, 128, 129, 4112, 4096), (4, 128, 1001, 1040, 768)])
+def test_dense_tiles_of_fewer_rows(cuda, bits, G, M, N, K):
+    """Tiles of 64 to 112 rows, the last one ragged, with scales in shared memory (and, at six groups, without): FP32, BF16 and gate/up rows, bit for bit the general kernel's,
+    which a captured call runs on."""
+    from strixite_b200 import kernels as Kn
+    g = torch.Generator(device="cuda").manual_seed(M)
+    w = Kn.quantize(torch.randn((N, K), generator=g, device=cuda) * 0.05, G, bits)
+    x = torch.randn((M, K), generator=g, device=cuda).to(torch.bfloat16)
+    forms = [(torch.float32, N, lambda y: Kn.linear_qw_wmma(x, w, y, M, Kn.Act.BF16, Kn.Act.F32)), (torch.bfloat16, N, lambda y: Kn.linear_qw_wmma(x, w, y, M, Kn.Act.BF16))]
+    forms += [(torch.bfloat16, N // 2, lambda y: Kn.linear_qw_wmma_swiglu(x, w, y, M, Kn.Act.BF16))]
+    for dtype, cols, call in forms:
+        y = [torch.full((M + 1, cols), 77.0, dtype=dtype, device=cuda) for _ in range(2)]
+        call(y[0])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call(y[1])
+        graph.replay()
+        torch.cuda.synchronize()
+        Kn.check_dense_status("tiles of fewer rows")
+        assert torch.equal(y[0].view(torch.uint8), y[1].view(torch.uint8)) and not bool(torch.isnan(y[0]).any())
 
 
 def test_dense_tcgen05_captured(cuda, oracle, lib, monkeypatch):
