@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <sstream>
 #include <string>
@@ -70,6 +71,18 @@ inline cudaError_t launch_behind(void (*kern)(Params...), dim3 grid, dim3 block,
     attr[1].id = cudaLaunchAttributeClusterDimension, attr[1].val.clusterDim.x = (unsigned)cluster, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+// The same for a kernel whose loads need the L1: an SM gives shared memory `sm_bytes`, all that its CTAs of this kernel take, and no more.  Without the
+// wish an SM keeps the split that some small kernel ahead left it with, if that will do (stream_mma.cu).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_behind_l1(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, size_t sm_bytes, Args &&...args) {
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization, attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = (unsigned)std::min<size_t>(100, (sm_bytes * 100 + 228 * 1024 - 1) / (228 * 1024));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = st, cfg.attrs = attr, cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
 }
 

@@ -52,6 +52,7 @@ constexpr int kPrefetch = 4;  // steps of weights in flight per warp beyond the 
 constexpr int64_t kMaxK = 1 << 24;
 constexpr int64_t kMaxN = 0x7fffffff;
 constexpr size_t kMaxDynSmem = 200 * 1024;
+constexpr size_t kCtaExtra = 3 * 1024;  // shared memory of a routed CTA beside the dynamic part: static, and 1 KB of the system's
 
 enum Mode { kGather = 0, kSwiglu = 1, kPartial = 2 };
 enum Src { kFromWs = 0, kFromSlots = 1, kDense = 2, kPerToken = 3 };
@@ -837,6 +838,10 @@ __global__ void __launch_bounds__(kBigThreads, 1) stream_kernel(const StreamArgs
 // 37 tokens (Q8 down) 207 + 167 -> 184 + 158, 150 tokens 424 + 234 -> 384 + 211; the layer as a graph, 2 tokens 82 -> 65, 4 107 -> 87, 64 599 -> 523.
 // The staging's loads are four at a time and inline: with eight or sixteen in flight, or as a call, the loop over a unit's codes lost registers to
 // them (16 tokens 126 + 65; as a call 200 + 89).
+// The codes come through L1, some 32 KB of them on their way.  The pack of more than 2048 slots leaves the SMs of its last CTAs with all of their 256 KB
+// but 28 as shared memory, which is enough for a CTA of this kernel, and there its warps ran at half their speed: with runs dealt ahead of time the whole launch did.  So
+// the launch says how much shared memory it wants (launch_behind_l1): gate/up at 205 tokens 809 -> 405 us (Q8 down 334 -> 227), the layer of 230 tokens 1242 -> 847,
+// of 400 tokens 1575 -> 1170; up to 204 tokens the same as before.
 // Every wait is bounded; one that runs out is recorded in the grouping workspace's status words and ends the warp.
 constexpr int kTileBufs = 2, kBigWarps = kBigThreads / 32;
 struct TileBuf {
@@ -1067,7 +1072,7 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
             if (int rc = reserve(tiles)) return rc;
             args.status = reinterpret_cast<uint32_t *>(const_cast<int32_t *>(a.ws)) + 5, args.wait_limit_ns = stream_wait_limit_ns(), args.test_skip_slot = test_skip_slot();
             args.chunks = args.split = 1;
-            launch_behind(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, 1, args);
+            launch_behind_l1(tiles, (unsigned)sm_count(), kBigThreads, kTileBufs * smem, st, kTileBufs * smem + kCtaExtra, args);
             return SXB_OK;
         }
     }
@@ -1093,7 +1098,8 @@ int launch_stream(const char *fn, const StreamArgs &a, int64_t est_units, cudaSt
     const int per_sm = big || smem > (SRC == kDense ? 88 : 100) * 1024 ? 1 : 2;
     int64_t grid = (int64_t)sm_count() * per_sm;
     grid = std::max<int64_t>(1, std::min<int64_t>(grid, (est_units + warps - 1) / warps));
-    launch_behind(kern, (unsigned)grid, threads, smem, st, 1, args);
+    if (SRC == kFromWs) launch_behind_l1(kern, (unsigned)grid, threads, smem, st, per_sm * (smem + kCtaExtra), args);
+    else launch_behind(kern, (unsigned)grid, threads, smem, st, 1, args);
     return SXB_OK;
 }
 
