@@ -8,19 +8,19 @@
 //
 // What bounds it (B200, SM cycles per step, the pieces measured alone): the MMAs take max(305, 4 n) for n tokens (below 76
 // tokens reading the A operand bounds them); dequantizing 128 x 128 codes and storing them to tensor memory takes the sixteen
-// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at 510 a step for 15 tokens
-// and 700 for 80: every role shares the four schedulers' issue slots and instruction caches, so what counts is instructions (584 a step
-// of them the dequantization).  From some 80 tokens an expert on launches in a row run at the card's power limit, 1000 W at 1.3 to 1.4 GHz.
+// producer warps 202; the HBM time of the codes is 340 (Q4) or 680 (Q8).  All of it together runs at some 520 a step for 15 tokens
+// and 700 for 80 (the times below at 1.9 GHz): every role shares the four schedulers' issue slots and instruction caches, so what counts is
+// instructions (584 a step of them the dequantization).  Launches in a row run at the card's power limit, at 15 tokens an expert as at 300: then it is energy.
 //   * One lane's MMAs and commits count, but its whole warp runs the loop, under control flow that the compiler can see to be uniform:
 //     addresses and descriptors then live in uniform registers.  Run by one lane of a diverged warp the MMAs took no longer to issue, but
 //     the loop around them 490 cycles a step (the wait 140, commit and the way back 350): 650 a step at 15 tokens with the stamps
 //     that showed it, which bounded every shape.  The scales of the step's own groups and this loop: gate/up 563 -> 540 us at 777
 //     tokens, 789 -> 728 at 4096, dense 1001 x 8192 x 4096 64.7 -> 57.1, 4000 tokens Q8 232 -> 216.
 //   * Steps of 128 k, eight MMAs a commit: with the loop of one lane a commit and the next stage's wait cost ~250 cycles whatever lay between.
-//   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 146 instructions a warp and step.  With neither copies nor MMAs the producers'
-//     own loop took 464 of the 548 us at 777 tokens: another 140 instructions a warp and step.  Now scales come through pointers that advance, the next item's
-//     first ones are asked for at the item's start, and arrivals are predicated, not branched to: 410 alone, gate/up 548 -> 506 us.  Asking for barriers a
-//     phase ahead, a deeper item ring or a second quarter dequantized before the stage is free: no faster (+0 to +1 %).
+//   * Dequantization is a mask and a multiply-add (dequant_q4_scaled): 146 instructions a warp and step.  The rest of the producers' loop counts as much (with
+//     neither copies nor MMAs it took 464 of then 548 us at 777 tokens): arrivals are predicated, not branched to; without SS scales come through pointers that
+//     advance, the next item's first ones asked for at the item's start: 410 alone, gate/up 548 -> 506 us.  Asking for barriers a phase ahead or a
+//     second quarter dequantized before the stage is free: no faster (+0 to +1 %).
 //   * A wait suspends its warp instead of polling; item descriptions come through shared memory (the item ring); the
 //     epilogue's pass is 16 tokens, not 32 (shorter code: gate/up 2593 -> 2477 us at 16384 tokens).
 //   * Where contractions are short the item counts: eight steps of down against 4500 instructions of epilogue at 80 tokens, 230 a warp and pass, which
@@ -95,9 +95,13 @@ struct Shape {
     static constexpr int kWays = HC ? 2 : 4;  // producer sets
     static constexpr int kStages = kWays;
     static constexpr int kSlotBytes = kRows * kBK * BITS / 8;  // a ring slot: the packed codes of a step, 8 or 16 KB
-    static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 8 ? 1 : SS ? 2 : 3);  // what shared memory holds beside the stages and the scales (Q4, 8 -> 12 slots: 583 -> 572 us at 777 tokens)
-    // Items that the ring holds.  The epilogue keeps an item's place until it is done with it.  Without SS three: 4096 x 8192 x 4096 Q8 under load 283 us with
-    // two, 261 with three, 263 with four, which lets the item warp's look at a later item's scales push those that the producers want out of L1.
+    // What shared memory holds beside the stages and the scales.  Without SS Q4 has room for twelve slots (583 -> 572 us at 777 tokens against eight, before SS took
+    // that case to eight slots and 548).
+    static constexpr int kWSlots = kWays * (HC ? (BITS == 4 ? 4 : 2) : BITS == 8 ? 1 : SS ? 2 : 3);
+    // Items that the ring holds.  The epilogue keeps an item's place until it is done with it.  Without SS three, us under load with two / three / four: dense
+    // 4096 x 8192 x 4096 Q8 315 / 263 / 272; gate/up of 64 experts, d = 7168, I = 2048, Q4, 4000 tokens 2047 / 1735 / 1768; down of 128 experts,
+    // 2560 x 768 Q4, 4000 tokens - / 204 / 196.  A deeper one lets the item warp's look at a later item's scales push those that the producers want out of L1,
+    // where rows are long.
     static constexpr int kItemRing = SS ? 4 : 3;
     static constexpr int kEpiSets = HC ? 2 : 1;  // epilogue warps per lane quadrant
     static constexpr int kEpiWarps = 4 * kEpiSets, kMmaWarp = kEpiWarps, kBCopyWarp = kEpiWarps + 1, kWCopyWarp = kEpiWarps + 2,
@@ -493,7 +497,8 @@ __global__ void __launch_bounds__((Shape<BITS, MODE == kTcHcUp, SS>::kThreads), 
         // bytes a thread), and local memory then took the L1 lines that the producers find their scales in: gate/up of 512 experts, d = 4096, I = 1024, Q8,
         // 300 tokens 1004-1062 us under load, 839-916 so (853-917 before slots were looked up here); 4096 x 8192 x 4096 Q8 + SwiGLU 274 -> 261 (257).
         constexpr bool kSlotsLate = !SS && MODE == kTcSwiglu;
-        // The scans without SS stand in front of a launch's first step and unroll by 64 registers of loads.  A few launches at a time, us, one at a time -> so:
+        // The scans without SS stand in front of a launch's first step: two loads of eight groups, two of two or four of one are under way for each of four rows.  A few
+        // launches at a time, us, one load -> so:
         // by twos dense 1500 x 2048 x 2816 Q4 24.7 -> 23.8, by ones 64 x 4096 x 1408 Q8 12.4 -> 11.6, 300 x 4096 x 1920 Q4 13.6 -> 12.5; by eights the down half of
         // the hyper-connection mix, 77 tokens, d = 4096, rank 320, 32.8 -> 30.8, dense 4096 x 8192 x 4096 Q8 under load 283 -> 272.
         // Waits until the producers are done with the item that had item i's place for scales.  Once an item, whether it needs the place or not: only then is
@@ -1050,7 +1055,8 @@ int launch_tiled_tc(const char *fn, TcArgs a, int64_t G, cudaStream_t st) {
         return SXB_OK;
     };
     if constexpr (MODE != kTcHcUp) {
-        // The scales of two items fit beside the rings up to 32 groups a row, of four up to 16; the item warp reads them by eights.
+        // The scales of two items fit beside the rings up to 32 groups a row, of four up to 16.  The item warp reads them by eights, so rows of 6, 12, 20 or 28 groups, which
+        // would fit too, are left to the producers' own loads, as longer rows and arrays that start elsewhere are.  With / without SS: see the head of this file.
         const int64_t groups = a.K / G;
         if (groups <= kScaleGroups && groups % 8 == 0 && ((reinterpret_cast<uintptr_t>(a.scale) | reinterpret_cast<uintptr_t>(a.minv)) & 15) == 0) {
             const int64_t bytes = ((int64_t)groups << scale_bufs_log((int)groups)) * kRows * 4;

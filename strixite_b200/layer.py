@@ -74,10 +74,10 @@ class MoeLayer:
     """One MoE sublayer.  E_total / e_lo: expert-parallel ranks hold experts [e_lo, e_lo + E_local) of E_total in their
     weight views and return their partial sum of y (see `ep.ExpertParallelMoe`)."""
 
-    # From here on the tcgen05 kernels.  Layer of 512 experts, top-10, d = 4096, I = 1024, Q4 with a shared expert, us streaming /
-    # tcgen05: 128 tokens 714 / 919, 204 822 / 989, 256 880 / 1014, 320 1433 / 997, 400 1467 / 1009; Q8 down weights 256 1058 / 1208,
-    # 320 1530 / 1096.  The jump is the streaming kernels' second tile of eight slots an expert: the sides change between five and
-    # six slots an expert on average, i.e. between 256 and 320 tokens here.
+    # From here on the tcgen05 kernels.  Layer of 512 experts, top-10, d = 4096, I = 1024, Q4 with a shared expert, us under load streaming /
+    # tcgen05: level popularity 128 tokens 747 / 852, 204 835 / 919, 256 876 / 911, 288 936 / 934, 320 997 / 932, 400 1187 / 936; with Q8 down
+    # weights 204 985 / 1042, 256 1039 / 1074, 288 1102 / 1066; popularity of N(0, 0.5) on the logits 128 667 / 723, 204 844 / 806, 256 933 / 855.
+    # The sides change between 200 and 290 tokens, sooner the less level the experts are: a second tile of eight slots reads an expert's weights again.
     tc_min_tokens = 256
     # The tcgen05 path's numerics.  WmmaF16F32Partials keeps the combine's per-slot dots in FP32; WmmaF16 rounds them to
     # BF16 as the reference's served path does, which by itself moves an output by up to ~2e-2 of the output RMS
