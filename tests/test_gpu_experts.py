@@ -633,17 +633,15 @@ def test_scratch_from_two_threads_and_streams(cuda, oracle, lib):
     assert not bad and lib.sxb_release_scratch() == 0
 
 
-# Groups a row: no whole eight of them; 8, 16, 24 and 32, the last that lie in shared memory; 40; and arrays that do not start on 16 bytes.  8192 rows are six
-# or seven items a CTA, so that the places of items and of scales come round, four of each up to 16 groups, two of scales above and three of items without any.
+# (N, K, groups a row): no whole eight of groups; 8, 16, 24 and 32, the last that lie in shared memory; 40; and arrays that do not start on 16 bytes.
+# 8192 rows: several items a CTA, so that the places of scales and items come round.
 @pytest.mark.parametrize("bits,G,N,Kd,shift", [
     (4, 128, 16, 128, 0), (8, 32, 48, 384, 0), (4, 128, 144, 1152, 0), (8, 32, 272, 128, 0), (4, 128, 8192, 1024, 0), (8, 64, 4096, 1024, 0), (8, 32, 144, 256, 0),
-    (4, 32, 48, 768, 0), (4, 128, 1040, 3072, 0), (8, 64, 1040, 2048, 0), (4, 128, 144, 4096, 0), (4, 128, 144, 5120, 0), (4, 128, 1040, 1024, 1), (8, 64, 272, 512, 3),
-    (4, 32, 8192, 768, 0), (8, 32, 8192, 768, 0), (4, 32, 8192, 1024, 0), (8, 32, 8192, 1024, 0), (8, 64, 8192, 640, 0), (8, 32, 8192, 1280, 0), (4, 128, 8192, 1024, 1),
-    (4, 64, 1152, 1024, 0), (8, 128, 1152, 1024, 0)])
+    (4, 32, 48, 768, 0), (4, 128, 1040, 3072, 0), (8, 64, 1040, 2048, 0), (4, 128, 144, 4096, 0), (4, 128, 144, 5120, 0), (4, 128, 1040, 1024, 1), (8, 64, 272, 512, 3)])
 def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd, shift):
     """Tiles of one token, around eight, sixteen and thirty-two and around a full tile, one and several steps of the contraction, rows that end inside
-    a row block, slots without an expert, scales from shared memory and by the producers: every output form of the grouped kernel for tile-blocked activations (the
-    tile-blocked h where it is whole blocks of 64), bit for bit the general kernel's (which a captured call runs on): the same operands, summed in the same order."""
+    a row block, slots without an expert, scales from shared memory and by the producers: every output form of the kernel for tile-blocked activations, bit for
+    bit the general kernel's (which a captured call runs on): the same operands, summed in the same order."""
     from strixite_b200 import kernels as K
     counts = [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 128, 129]
     E, g = len(counts), torch.Generator(device="cuda").manual_seed(N + bits)
@@ -672,8 +670,56 @@ def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd, shift):
              ("gate/up F16, Q4 order", torch.float16, N // 2, lambda y: gate_up(y, 2)),
              ("FP32 dots", torch.float32, N, lambda y: combine(y, K.MoeMath.WmmaF16F32Partials, f32)),
              ("BF16 dots", torch.float32, N, lambda y: combine(y, K.MoeMath.WmmaF16, f32))]
-    blocks = [("tile-blocked gate/up, Q4 order", torch.float16, N // 2, lambda y: gate_up(y, 3)), ("tile-blocked gate/up", torch.float16, N // 2, lambda y: gate_up(y, 4))]
-    forms += blocks if N % 128 == 0 else []
+    live = (ids[:, 0] < E).cpu()
+    for name, dtype, cols, call in forms:
+        y = [torch.full((M + 1, cols), 77.0, dtype=dtype, device=cuda) for _ in range(2)]
+        call(y[0])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            call(y[1])
+        graph.replay()
+        torch.cuda.synchronize()
+        K.check_grouped_status(ws, name)
+        got, want = (v.cpu() for v in y)
+        assert torch.equal(got[:M][live].view(torch.uint8), want[:M][live].view(torch.uint8)), name
+        assert bool(torch.isnan(got[:M][~live]).all()) and not bool(torch.isnan(got[:M][live]).any()), name
+        assert bool((got[M] == 77.0).all()), name  # nothing past the last row
+
+
+# 8192 rows are six or seven items a CTA, so that the places of items and of scales come round, four of each up to 16 groups a row, two of scales above and three of
+# items where none lie in shared memory; and the shapes of the test before that have whole blocks of 64 h columns.
+@pytest.mark.parametrize("bits,G,N,Kd,shift", [
+    (4, 32, 8192, 768, 0), (8, 32, 8192, 768, 0), (4, 32, 8192, 1024, 0), (8, 32, 8192, 1024, 0), (8, 64, 8192, 640, 0), (8, 32, 8192, 1280, 0), (4, 128, 8192, 1024, 1),
+    (4, 64, 1152, 1024, 0), (8, 128, 1152, 1024, 0), (4, 128, 8192, 1024, 0), (8, 64, 4096, 1024, 0)])
+def test_tcgen05_places_come_round_and_tile_blocked_h(cuda, bits, G, N, Kd, shift):
+    """Every output form of the grouped kernel for tile-blocked activations, the tile-blocked h among them, over tiles of 1 to 128 tokens with several items a CTA: bit for bit
+    the general kernel's, which a captured call runs on."""
+    from strixite_b200 import kernels as K
+    counts = [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 128, 129]
+    E, g = len(counts), torch.Generator(device="cuda").manual_seed(N + bits)
+    ids = torch.cat([torch.repeat_interleave(torch.arange(E), torch.tensor(counts)), torch.full((19,), E + 3)]).to(torch.int32)
+    M = ids.numel()
+    ids = ids[torch.randperm(M, generator=torch.Generator().manual_seed(N))].to(cuda)[:, None].contiguous()
+    w = K.quantize(torch.randn((E * N, Kd), generator=g, device=cuda) * 0.05, G, bits)
+    if shift:  # arrays that do not start on 16 bytes
+        scale, minv = (torch.cat([torch.zeros(shift, dtype=torch.int16, device=cuda), t.reshape(-1)])[shift:].view(t.shape) for t in (w.scale, w.minv))
+        w = K.QDeviceView(w.q, scale, minv, w.N, w.K, w.G, w.bits)
+    x = torch.randn((M, Kd), generator=g, device=cuda).to(torch.bfloat16)
+    coef, err = torch.rand((M, 1), generator=g, device=cuda), torch.zeros(4, dtype=torch.int32, device=cuda)
+    nbytes = K.moe_route_workspace_bytes(M, 1, E)
+    ws = torch.empty(nbytes // 4, dtype=torch.int32, device=cuda)
+    K.moe_group_routes(ids, M, 1, E, ws, nbytes, err)
+    partial, f32 = torch.empty((M, N), device=cuda), K.Act.F32
+
+    def combine(math):
+        return lambda y: K.linear_qw_experts_combine_grouped(x, w, E, ids, coef, ws, nbytes, partial, M, 1, y, K.Act.BF16, math, out_act=f32)
+
+    def gate_up(h_f16):
+        return lambda y: K.linear_qw_experts_gather_grouped_swiglu(x, w, E, ws, nbytes, M, 1, y, K.Act.BF16, K.MoeMath.WmmaF16, h_f16=h_f16)
+
+    forms = [("rows", torch.bfloat16, N, lambda y: K.linear_qw_experts_gather_grouped(x, w, E, ws, nbytes, M, 1, y, K.Act.BF16, K.MoeMath.WmmaF16)),
+             ("FP32 dots", torch.float32, N, combine(K.MoeMath.WmmaF16F32Partials)), ("BF16 dots", torch.float32, N, combine(K.MoeMath.WmmaF16))]
+    forms += [(f"gate/up, h_f16 = {f}", torch.bfloat16 if f == 0 else torch.float16, N // 2, gate_up(f)) for f in range(5)]  # 3 and 4: tile-blocked
     in_slots, in_order = (ids[:, 0] < E).cpu(), torch.arange(M) < sum(counts)  # the tile-blocked h stands in the order of the experts
     for name, dtype, cols, call in forms:
         y = [torch.full((M + 1, cols), 77.0, dtype=dtype, device=cuda) for _ in range(2)]
@@ -684,7 +730,7 @@ def test_tcgen05_tiles_and_rows_at_their_edges(cuda, bits, G, N, Kd, shift):
         graph.replay()
         torch.cuda.synchronize()
         K.check_grouped_status(ws, name)
-        tiled = any(name == b[0] for b in blocks)
+        tiled = name in ("gate/up, h_f16 = 3", "gate/up, h_f16 = 4")
         live = in_order if tiled else in_slots
         got, want = (v[:M].reshape(cols // 64, M, 64).transpose(0, 1).cpu() if tiled else v[:M].cpu() for v in y)
         assert torch.equal(got[live].view(torch.uint8), want[live].view(torch.uint8)), name
